@@ -4,10 +4,11 @@ Same constructor, parameters (``qkvo_w [4, dim, dim]`` bf16, ``g_ve``), attribut
 ``AttentionProtocol`` entry points (models/daisy/attention_protocol.py:5-42).  ``forward`` and ``prefill``
 run on hand-written sm_100a kernels of ``libdaisy_b200.so`` only: the merged QKV projection with the RMS
 norm, RoPE and value-embedding gate in its epilogue, the windowed softmax attention, the output projection.
-The single-token ``step`` forms are three launches: the token's merged QKV projection (a weight-streaming
-kernel), the single-launch ring-cache decode (norm, RoPE, value-embedding gate, split-KV attention, merge, ring
-store) and the output projection.  There is no other code path and no switch that selects one: on a machine without the library
-or without a GPU the calls raise.
+The single-token ``step`` forms are one launch for up to ``dim`` 2048 and batch 16 (``csrc/swa_token.cu``; a
+``StepRunner`` puts all layers of its stack into it).  Larger ones are three: the token's merged QKV projection, the
+single-launch ring-cache decode (norm, RoPE, value-embedding gate, split-KV attention, merge, ring store) and the output
+projection.  There is no other code path and no switch that selects one: on a machine without the library or without a GPU
+the calls raise.
 
 Masking.  The kernels evaluate the reference's inference mask (models/daisy/daisy_core.py:53-69)
 analytically: key visible iff ``0 <= q - k < window`` and both tokens lie in one document.  ``attn_mask`` is
@@ -32,7 +33,8 @@ from torch import nn, Tensor
 import torch.nn.functional as F
 
 from . import ops
-from ._lib import NORM_Q, NORM_K, NORM_V, ROPE, QKV_DEFAULT
+from ._native import ext
+from ._lib import WRITE_RING, NORM_Q, NORM_K, NORM_V, ROPE, QKV_DEFAULT
 from .kv_cache import B200KVCache
 
 
@@ -308,13 +310,18 @@ class B200CausalSelfAttention(nn.Module):
         """One token against a chronological context ``[B,n,H,D]`` (models/daisy/attention.py:181-202).
         Returns ``(y [B,1,dim], k_new [B,1,H,D], v_new [B,1,H,D])``."""
         B = x.size(0)
-        q, k, v = self._project(x)
         n = 0 if k_ctx is None else k_ctx.size(1)
         kc = None if n == 0 else k_ctx.transpose(1, 2)        # logical [B,H,n,D]
         vc = None if n == 0 else v_ctx.transpose(1, 2)
         if kc is not None and kc.dtype != torch.bfloat16:     # reference casts the context to q's dtype
             kc, vc = kc.to(torch.bfloat16), vc.to(torch.bfloat16)
-        y, k_new, v_new = self._decode(q, k, v, kc, vc, n, n, pos, ve, window, write_ring=False)
+        if kc is None:                                        # no context yet: an empty one
+            kc = vc = x.new_empty((B, self.num_heads, 0, self.head_dim), dtype=torch.bfloat16)
+        res = self._step_one_launch(x, kc, vc, n, pos, ve, window, write_ring=False)
+        if res is not None:
+            return res
+        q, k, v = self._project(x)
+        y, k_new, v_new = self._decode(q, k, v, kc if n else None, vc if n else None, n, n, pos, ve, window, write_ring=False)
         y = self._linear(y.view(B, 1, self.m_dim), self.qkvo_w.detach()[3])
         return y, k_new, v_new
 
@@ -323,8 +330,12 @@ class B200CausalSelfAttention(nn.Module):
         (replaces ``cache.view(layer)`` + ``step`` + ``cache.write(layer, ...)`` of
         inference/generate.py:231-246).  The caller still calls ``cache.advance()`` once per token."""
         B = x.size(0)
-        q, k, v = self._project(x)
         kr, vr = cache.ring(layer)
+        res = self._step_one_launch(x, kr, vr, cache.t, pos, ve, window, write_ring=True)
+        if res is not None:
+            cache.mark_written(layer)
+            return res
+        q, k, v = self._project(x)
         y, k_new, v_new = self._decode(q, k, v, kr, vr, cache.t, cache.W, pos, ve, window, write_ring=True)
         cache.mark_written(layer)
         y = self._linear(y.view(B, 1, self.m_dim), self.qkvo_w.detach()[3])
@@ -334,13 +345,18 @@ class B200CausalSelfAttention(nn.Module):
                       ve: Optional[Tensor] = None):
         """``step_ring`` with the position read from ``cache.t_dev`` on the device: nothing in the launch
         sequence depends on the token index, so it can be captured once in a CUDA graph and replayed
-        (``StepRunner.capture_step``).  Position = tokens in the cache, as in ``Generator._step``.  Three launches,
-        all of this library: the merged QKV projection of the token (weight-streaming kernel), the single-launch
-        ring decode (norm, RoPE, value-embedding gate, split-KV attention, merge, ring store), the output
-        projection."""
+        (``StepRunner.capture_step``).  Position = tokens in the cache, as in ``Generator._step``.  The same one or
+        three launches as ``step_ring``."""
         self._no_autograd(x)
         B = x.size(0)
         H, D = self.num_heads, self.head_dim
+        if ext().token_step_supported(B, H, 1):
+            if getattr(self, "_token_ws_key", None) != (B, x.device):     # zeroed once, then the calls keep its tags
+                self._token_ws = torch.zeros(ext().token_workspace_bytes(B, H), dtype=torch.uint8, device=x.device)
+                self._token_ws_key = (B, x.device)
+            kr, vr = cache.ring(layer)
+            return self._token_call(x, kr, vr, 0, cache.t_dev, self.rotary.cos, self.rotary.sin, ve, window, write_ring,
+                                    None, None, self._token_ws)
         w = self.qkvo_w.detach()
         qkv = ops.gemm_skinny(x.detach().to(w.dtype).view(B, self.m_dim), w[:3].flatten(end_dim=1)).view(B, 1, 3 * H, D)
         q, k, v = qkv[:, :, :H], qkv[:, :, H:2 * H], qkv[:, :, 2 * H:]
@@ -359,6 +375,29 @@ class B200CausalSelfAttention(nn.Module):
                                       self.attn_scale, self.norm_eps, QKV_DEFAULT, write_ring=write_ring,
                                       splits=self._fused_splits, workspace=self._fused_ws, **ve_kw)
         return ops.gemm_skinny(y.view(B, self.m_dim), w[3]).view(B, 1, self.m_dim)
+
+    def _token_call(self, x, kc, vc, t, t_dev, cos, sin, ve, window, write_ring, k_new, v_new, workspace):
+        gate = None
+        if self.receives_ve:
+            torch._assert(ve is not None, "ve must be provided when receives_ve=True")
+            gate = self.g_ve.detach().float().reshape(1)
+        return ext().token_step(x.detach(), [self.qkvo_w.detach()], [cos], [sin], kc[None], vc[None], t, t_dev, None, int(window or 0),
+                                self.attn_scale, self.norm_eps, QKV_DEFAULT | (WRITE_RING if write_ring else 0),
+                                ve if self.receives_ve else None, gate, k_new, v_new, None, workspace)
+
+    def _step_one_launch(self, x, kc, vc, t: int, pos: int, ve, window, write_ring):
+        """``(y, k_new, v_new)`` of a step over ``t`` tokens in the ring (or context) kc, vc ``[B,H,cap,D]``, or None where the
+        single-launch kernel does not take the sizes."""
+        self._no_autograd(x)
+        B, H, D = x.size(0), self.num_heads, self.head_dim
+        cos, sin = self.rotary.tables(pos + 1)
+        if pos < t or not ext().token_step_supported(B, H, 1):
+            return None
+        if pos > t:                                                       # the kernel takes row `t` of the tables it is given
+            cos, sin = cos[pos - t:], sin[pos - t:]
+        k_new, v_new = (torch.empty(B, 1, H, D, dtype=torch.bfloat16, device=x.device) for _ in range(2))
+        y = self._token_call(x, kc, vc, int(t), None, cos, sin, ve, window, write_ring, k_new, v_new, None)
+        return y, k_new, v_new
 
     def _decode(self, q, k, v, kc, vc, t, cap, pos, ve, window, write_ring):
         cos, sin = self.rotary.tables(pos + 1)

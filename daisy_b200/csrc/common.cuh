@@ -507,6 +507,7 @@ namespace daisy_host {
 
 // Per-device host state (kernel attributes are per device; a process may drive several).
 constexpr int MAX_DEVICES = 64;
+constexpr int MAX_SMS = 192;                           // upper bound used to size per-SM workspaces
 // Index of the current device into such tables, or -1.
 int device_slot();
 // SM count of the current device, cached per device; 0 if there is none.

@@ -2,8 +2,8 @@
 
 Mirror of the reference ``Generator._prefill`` / ``Generator._step`` (inference/generate.py:220-248) for a
 stack of attention layers: prefill fills the ring layer by layer from inside the projection kernel (the rows
-``bulk_write_packed`` would write, no copy pass); each step hands every
-layer the ring itself (no per-layer chronological ``view`` copy, no separate ``write``) and advances once.
+``bulk_write_packed`` would write, no copy pass); each step is one launch that takes every layer's ring in place (no
+per-layer chronological ``view`` copy, no separate ``write``) and advances once.
 Sampling, embeddings and the MLPs are outside this path; the runner works on hidden states.
 """
 from __future__ import annotations
@@ -12,6 +12,8 @@ from typing import List, Optional, Sequence
 
 import torch
 
+from ._lib import QKV_DEFAULT, WRITE_RING
+from ._native import ext
 from .attention import B200CausalSelfAttention, WindowMask
 from .kv_cache import B200KVCache
 
@@ -42,14 +44,34 @@ class StepRunner:
         self.cache.set_position(T)
         return x
 
-    # ------------------------------------------------------------------ CUDA-graph step
+    # ------------------------------------------------------------------ all layers in one launch
+    def _one_launch(self, x: torch.Tensor) -> bool:
+        """Whether the whole stack fits the single-launch step: plain layers of one shape with the same constants."""
+        c, a = self.cache, self.layers[0]
+        return (x.size(0) == c.B and all(type(m) is B200CausalSelfAttention and not m.receives_ve and m.num_heads == a.num_heads
+                                         and m.attn_scale == a.attn_scale and m.norm_eps == a.norm_eps for m in self.layers)
+                and ext().token_step_supported(c.B, c.H, len(self.layers)))
+
+    def _token(self, x, t, t_dev, out=None, workspace=None):
+        c, a = self.cache, self.layers[0]
+        rot = [m._modules["rotary"]._buffers for m in self.layers]
+        return ext().token_step(x, [m._parameters["qkvo_w"] for m in self.layers], [r["cos"] for r in rot], [r["sin"] for r in rot],
+                                c.k, c.v, t, t_dev, c.t_dev, self.window, a.attn_scale, a.norm_eps, QKV_DEFAULT | WRITE_RING,
+                                None, None, None, None, out, workspace)
+
+    # ------------------------------------------------------------------ fixed-buffer step
     @torch.inference_mode()
     def capture_step(self, batch: int, dim: int) -> None:
-        """Record one token step of all layers into a CUDA graph.  The position lives in ``cache.t_dev`` and is
-        advanced inside the graph, the input and output are fixed buffers: ``_step_graph`` then costs one copy
-        and one graph launch per token instead of four launches per layer issued from Python."""
+        """Prepare ``_step_graph``: the position lives in ``cache.t_dev``, the output is a fixed buffer, nothing is allocated
+        per token.  Where the stack fits the single-launch kernel that launch is the whole step; otherwise one token step
+        of all layers is recorded into a CUDA graph, and ``_step_graph`` costs one copy and one graph launch per token."""
         dev = self.cache.device
         self._gx = torch.zeros(batch, 1, dim, device=dev, dtype=torch.bfloat16)
+        self._graph = None
+        if self._one_launch(self._gx):
+            self._gy = torch.zeros_like(self._gx)
+            self._gws = torch.zeros(ext().token_workspace_bytes(batch, self.cache.H), dtype=torch.uint8, device=dev)
+            return
         t_saved = self.cache.t_dev.clone()
         side = torch.cuda.Stream(device=dev)
         side.wait_stream(torch.cuda.current_stream(dev))
@@ -71,18 +93,27 @@ class StepRunner:
 
     @torch.inference_mode()
     def _step_graph(self, x: torch.Tensor) -> torch.Tensor:
-        """``_step`` through the captured graph.  Neither the warm-up run (made without the ring store) nor the
+        """``_step`` into the fixed buffer.  Neither the warm-up run (made without the ring store) nor the
         capture itself (which executes nothing) has touched the ring, so a capture is safe at any position, also
         with a window larger than the ring, where the slot of the next token is the oldest row still attended."""
-        self._gx.copy_(x)
-        self._graph.replay()
-        self.cache.t += 1                                          # host mirror; the device counter moved in the graph
+        if self._graph is None:
+            self._token(x, 0, self.cache.t_dev, self._gy, self._gws)
+        else:
+            self._gx.copy_(x)
+            self._graph.replay()
+        self.cache.t += 1                                          # host mirror; the device counter moved in the launch
         return self._gy
 
     @torch.inference_mode()
     def _step(self, x: torch.Tensor) -> torch.Tensor:
         """One token ``x [B,1,dim]``: every layer reads the ring in place and stores its new row; one advance."""
         pos = self.cache.t
+        if self._one_launch(x):
+            torch._assert(pos < self.layers[0].rotary.cos.shape[0], "Rotary buffers too small")
+            x = self._token(x, pos, None)
+            self.cache.t += 1                                      # its device counter moved in the launch
+            self.cache._staged = [False] * self.cache.L
+            return x
         for i, a in enumerate(self.layers):
             x, _, _ = a.step_ring(x, self.cache, i, pos, None, self.window)
         self.cache.advance()

@@ -9,6 +9,7 @@ from typing import Optional, Tuple
 import torch
 
 from . import _lib
+from ._native import ext
 from ._lib import (NORM_Q, NORM_K, NORM_V, ROPE, QKV_DEFAULT, WRITE_RING, OUT_BTHD, KV_BHTD, Q_IN_KERNEL, KDA_L2NORM_QK,
                    KDA_OUT_FP32)
 
@@ -26,8 +27,13 @@ def status_word(device) -> torch.Tensor:
     dev = torch.device(device)
     key = dev.index if dev.index is not None else torch.cuda.current_device()
     if key not in _status_words:
-        _status_words[key] = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", key))
+        _status_words[key] = ext().status_word(key)
     return _status_words[key]
+
+
+def release_workspaces() -> None:
+    """Give back the small workspaces kept per stream for the decode steps (they are made again when needed)."""
+    ext().release_workspaces()
 
 
 def check_device_status(device) -> None:

@@ -142,6 +142,29 @@ int daisy_b200_gemm_nt(const void* x, int64_t ldx, const void* w, int64_t ldw, v
 int daisy_b200_gemm_skinny(const void* x, int64_t ldx, const void* w, int64_t ldw, void* y, int64_t ldy,
                            int M, int N, int K, void* stream);
 
+/* One decoded token through n_layers attention layers in one launch: per layer the merged QKV projection, the new
+ * token's norm / RoPE / value-embedding gate, the windowed attention over the ring cache, the ring store and the output
+ * projection -- CausalSelfAttention.step for every layer of Generator._step (models/daisy/attention.py:181-202,
+ * inference/generate.py:231-248).  x [B, dim] (row stride x_sb elements), y [B, dim] contiguous, dim = H * 128 <= 2048,
+ * B <= 16, n_layers <= 16; qkvo_w [4, dim, dim] contiguous.  The rings share their strides (elements); t / t_dev, cap,
+ * window and flags (DAISY_QKV_DEFAULT bits, DAISY_WRITE_RING, DAISY_CACHE_FP16) as in daisy_b200_swa_decode_step_fused;
+ * t_advance: a counter in device memory that is incremented once the step is done, or NULL.  The kernel is a cooperative launch of one
+ * CTA per SM.  workspace: 256-byte aligned, zero before the first call, afterwards left to the calls.  Calls that may overlap on the device need workspaces of their own. */
+typedef struct daisy_b200_token_layer {
+  const void* qkvo_w;
+  void *kcache, *vcache;
+  const void* ve;                 /* value embedding [B, dim] (row stride ve_sb) or NULL */
+  const float* ve_gate_logit;
+  void *k_new_out, *v_new_out;    /* [B, H, 128] bf16 copies of the new rows, or NULL */
+  const float *cos, *sin;         /* whole RoPE tables [table_rows, 64] */
+} daisy_b200_token_layer;
+size_t daisy_b200_swa_token_workspace_bytes(int B, int H, int D);
+int daisy_b200_swa_token_step(const daisy_b200_token_layer* layers, int n_layers, const void* x, int64_t x_sb, void* y,
+                              int64_t c_sb, int64_t c_sh, int64_t c_sr, int64_t t, const int64_t* t_dev, int64_t* t_advance,
+                              int cap, int window, int table_rows, int64_t ve_sb,
+                              int B, int H, int D, float scale, float eps, unsigned flags,
+                              void* workspace, size_t workspace_bytes, int* status_word, void* stream);
+
 /* ---------------------------------------------------------------------------------------------
  * Sliding-window causal softmax attention, prefill form.
  * Replaces CausalSelfAttention._sdpa_common between the two projections

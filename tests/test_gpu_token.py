@@ -1,0 +1,66 @@
+"""The single-launch decode step (csrc/swa_token.cu) against the CPU oracle, at the edges of its partition: one and many
+layers, batch 1 to 16, one row tile or several, contexts of 0, 1, 15 .. 17 and many rows, a wrapped ring, fp16 rings."""
+import pytest
+import torch
+
+from gpu_util import assert_close_bf16
+from oracle import swa
+
+pytestmark = pytest.mark.gpu
+D = 128
+
+
+def _setup(B, H, L, cap, f16, seed=0):
+    g = torch.Generator().manual_seed(seed)
+    dim = H * D
+    w = [(torch.randn(4, dim, dim, generator=g) * dim ** -0.5).bfloat16() for _ in range(L)]
+    ring = [torch.randn(L, B, H, cap, D, generator=g).to(torch.float16 if f16 else torch.bfloat16) for _ in range(2)]
+    return w, ring, torch.randn(B, 1, dim, generator=g).bfloat16()
+
+
+def _oracle(w, rk, rv, x, t, cap, window, cos, sin, eps):
+    B, _, dim = x.shape
+    H = dim // D
+    qkv = (x.float() @ w[:3].flatten(end_dim=1).float().T).bfloat16().float().view(B, 1, 3 * H, D)
+    idx = torch.arange(t - min(t, cap), t) % cap
+    y, k, v = swa.decode_step(*qkv.chunk(3, dim=-2), rk[:, :, idx].transpose(1, 2).float(), rv[:, :, idx].transpose(1, 2).float(), t, window,
+                              cos, sin, eps=eps)
+    return (y.reshape(B, 1, dim).bfloat16().float() @ w[3].float().T).bfloat16(), k, v
+
+
+@pytest.mark.parametrize("B,H,L,t,cap,window,f16", [
+    (1, 1, 1, 0, 48, 16, False), (1, 3, 2, 1, 48, 16, False), (2, 2, 1, 16, 48, 17, True), (3, 5, 2, 100, 48, 100, False),
+    (1, 16, 2, 3000, 2048, 2048, False), (8, 6, 1, 700, 512, 300, True), (9, 4, 2, 77, 64, 18, False), (16, 16, 1, 130, 64, 64, False),
+    (1, 2, 17, 40, 32, 24, False),
+])
+def test_token_step_matches_oracle(B, H, L, t, cap, window, f16):
+    from daisy_b200 import ops
+    from daisy_b200._lib import QKV_DEFAULT, WRITE_RING
+    from daisy_b200._native import ext
+    w, (rk, rv), x = _setup(B, H, L, cap, f16)
+    eps = float(torch.finfo(torch.bfloat16).eps)
+    cos, sin = swa.rope_tables(D, t + 2)
+    dev = [a.cuda() for a in w], rk.cuda(), rv.cuda(), x.cuda(), cos.cuda(), sin.cuda()
+    assert ext().token_step_supported(B, H, L)
+    t_dev, adv = torch.tensor([t], device="cuda"), torch.tensor([t], device="cuda")
+    args = lambda k, v, pos, d, a: (dev[3], dev[0], [dev[4]] * L, [dev[5]] * L, k, v, pos, d, a, window, 0.12, eps, QKV_DEFAULT | WRITE_RING,
+                                    None, None, None, None, None, None)
+    k1, v1 = dev[1].clone(), dev[2].clone()
+    y = ext().token_step(*args(k1, v1, t, None, adv))
+    k2, v2 = dev[1].clone(), dev[2].clone()
+    y2 = ext().token_step(*args(k2, v2, 0, t_dev, None))
+    ops.check_device_status("cuda")
+    assert torch.equal(y, y2) and torch.equal(k1, k2) and torch.equal(v1, v2), "position on the device"
+    assert int(adv) == t + 1 and int(t_dev) == t
+    h = x
+    for l in range(L):
+        h, k, v = _oracle(w[l], rk[l], rv[l], h, t, cap, window, cos, sin, eps)
+        if l == 0:
+            got_k, got_v = k1[0, :, :, t % cap].float().cpu(), v1[0, :, :, t % cap].float().cpu()
+            assert_close_bf16(got_k, k[:, 0], "new k row")
+            assert_close_bf16(got_v, v[:, 0], "new v row")
+    rel = ((y.float().cpu() - h.float()).norm() / h.float().norm()).item()
+    assert rel < 1e-2 * max(1.0, L ** 0.5), rel
+    mask = torch.ones(cap, dtype=torch.bool)
+    mask[t % cap] = False
+    assert torch.equal(k1[:, :, :, mask].cpu(), rk[:, :, :, mask]) and torch.equal(v1[:, :, :, mask].cpu(), rv[:, :, :, mask])

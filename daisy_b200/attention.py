@@ -257,18 +257,14 @@ class B200CausalSelfAttention(nn.Module):
         self._no_autograd(x)
         window, doc_start = mask[0], mask[1]
         in_blocks = len(mask) > 2 and mask[2]
-        B, T = x.size(0), x.size(1)
-        cos, sin = self.rotary.tables(T)
-        w = self.qkvo_w.detach()
-        ve_kw = {}
+        cos, sin = self.rotary.tables(x.size(1))
+        gate = None
         if self.receives_ve:
             torch._assert(ve is not None, "ve must be provided when receives_ve=True")
-            ve_kw = dict(ve=ve.to(torch.bfloat16), ve_gate_logit=self.g_ve.detach().float().reshape(1))
-        qp, kp, vp = ops.qkv_gemm(x.detach().to(w.dtype), w[:3].flatten(end_dim=1), cos, sin, self.num_heads, self.norm_eps,
-                                  ring=ring, ring_first=ring_first, **ve_kw)
-        y = ops.swa_attend(qp, kp, vp, window, self.attn_scale, bounded_qk=True, doc_start=doc_start,   # q, k are RMS-normalised
-                           window_in_blocks=in_blocks)
-        y = ops.gemm_nt(y.view(B, T, self.m_dim), w[3])
+            ve, gate = ve.to(torch.bfloat16), self.g_ve.detach().float().reshape(1)
+        rk, rv = ring if ring is not None else (None, None)
+        y, kp, vp, qp = ext().attn_layer(x, self.qkvo_w, cos, sin, self.num_heads, self.norm_eps, self.attn_scale, int(window or 0), doc_start, in_blocks,
+                                         ve if self.receives_ve else None, gate, rk, rv, ring_first)
         return y, kp.transpose(1, 2), vp.transpose(1, 2), qp.transpose(1, 2)
 
     # ------------------------------------------------------------------ AttentionProtocol

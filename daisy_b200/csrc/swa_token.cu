@@ -25,21 +25,12 @@
 // fp32 precision: each is split into a high and a low 16-bit part that occupy two of the product's empty columns / rows.
 // All waits are bounded; a CTA that gives up keeps walking through its barriers (its waits return at once), so nobody is
 // left behind, and every warp waits for the copies it has in flight before it leaves.
-#include "common.cuh"
-#include <cuda_fp16.h>
+#include "token_common.cuh"
 
 namespace daisy {
 
-constexpr int TK_CW = 12;                             // warps
-constexpr int TK_CT = 32 * TK_CW;
-constexpr int TK_DEPTH = 2;                           // pieces of a warp in flight (one where the vectors of a large batch take the room)
-constexpr int TK_KW = 256;                            // weight columns of a piece
-// A piece is 16 weight rows x 256 columns, or 16 K rows + 16 V rows: blocks of 16 rows x 128 bytes, 128-byte swizzle
-constexpr int TK_PIECE = 8192, TK_BLK = 2048;
 constexpr int TK_MAX_SEG = 4;                         // (batch, head) segments of one CTA's range
-constexpr int TK_COPIES = 4;                          // of x and o: 148 CTAs reading the same 8 KB at once queue at its L2 slices
 constexpr int TK_MAX_LAYERS = 16;
-constexpr int TK_MAX_DIM = 2048, TK_MAX_B = 16;
 constexpr float TK_NEG = -1.0e30f;
 
 struct TokenLayer {
@@ -80,101 +71,6 @@ struct TokenBars {
 constexpr int TK_FIXED = TK_MAX_SEG * (512 + 1024 + 512);   // shared memory of the segments: q halves, k and v, own partial
 constexpr int TK_PART = 65;                           // uint4 words of a partial
 
-template <bool F16>
-__device__ __forceinline__ void tk_mma(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
-  if (F16)
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-  else
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void tk_ldm4(uint32_t* r, uint32_t addr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void tk_ldm4_t(uint32_t* r, uint32_t addr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void tk_tma3(uint32_t dst, const CUtensorMap* m, uint64_t* bar, int x, int y, int z) {
-  asm volatile("cp.async.bulk.tensor.3d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-               ::"r"(dst), "l"(m), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z) : "memory");
-}
-__device__ __forceinline__ void tk_tma5(uint32_t dst, const CUtensorMap* m, uint64_t* bar, int row, int h, int b) {
-  asm volatile("cp.async.bulk.tensor.5d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %3, %5, %6}], [%2];"
-               ::"r"(dst), "l"(m), "r"(smem_u32(bar)), "r"(0), "r"(row), "r"(h), "r"(b) : "memory");
-}
-__device__ __forceinline__ float tk_warp_sum(float x) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-  return x;
-}
-// high and low 16-bit halves of a value: h + l carries 16 (bf16) to 21 (fp16) bits of it
-template <bool F16>
-__device__ __forceinline__ void tk_split(float x, uint16_t& hi, uint16_t& lo) {
-  if (F16) {
-    const __half h = __float2half_rn(x);
-    hi = __half_as_ushort(h); lo = __half_as_ushort(__float2half_rn(x - __half2float(h)));
-  } else {
-    const __nv_bfloat16 h = __float2bfloat16_rn(x);
-    hi = __bfloat16_as_ushort(h); lo = __bfloat16_as_ushort(__float2bfloat16_rn(x - __bfloat162float(h)));
-  }
-}
-// Tagged words.  Each 8-byte half of a 16-byte access is written and read as one unit.
-__device__ __forceinline__ void tk_put2(uint2* p, uint32_t a, uint32_t tag) {
-  asm volatile("st.relaxed.gpu.global.v2.u32 [%0], {%1, %2};" ::"l"(p), "r"(a), "r"(tag) : "memory");
-}
-__device__ __forceinline__ void tk_put4(void* p, uint32_t a, uint32_t b, uint32_t tag) {
-  asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %3, %2, %3};" ::"l"(p), "r"(a), "r"(b), "r"(tag) : "memory");
-}
-__device__ __forceinline__ uint4 tk_peek(const void* p) {
-  uint4 r;
-  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p) : "memory");
-  return r;
-}
-constexpr long long TK_PATIENCE = 4000000000ll;      // cycles a wait lasts at most: about two seconds
-__device__ __noinline__ void tk_give_up(volatile int* abort_flag, int* status) {
-  *abort_flag = 9;
-  if (status) status[0] = DAISY_ETIMEOUT;
-}
-// N 16-byte words at p, p + step, .. once all of them carry the tag.  Bounded: the caller then gets whatever is there and
-// the launch reports it.
-template <int N>
-__device__ __forceinline__ void tk_get(const uint4* p, int step, uint4 (&r)[N], uint32_t tag, volatile int* abort_flag, int* status) {
-  const long long t0 = clock64();
-  while (true) {
-    bool ok = true;
-#pragma unroll
-    for (int i = 0; i < N; ++i) r[i] = tk_peek(p + i * step);
-#pragma unroll
-    for (int i = 0; i < N; ++i) ok = ok && r[i].y == tag && r[i].w == tag;
-    if (ok || *abort_flag) return;
-    if (clock64() - t0 > TK_PATIENCE) { tk_give_up(abort_flag, status); return; }
-  }
-}
-__device__ __forceinline__ bool tk_bar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const long long t0 = clock64();
-  while (!mbar_try_wait(bar, parity)) {
-    if (*abort_flag) return false;
-    if (clock64() - t0 > TK_PATIENCE) { tk_give_up(abort_flag, status); return false; }
-  }
-  return true;
-}
-// n tagged words of 4 bf16 each (two per 8-byte half) into a plain row in shared memory, by all threads
-__device__ __forceinline__ void tk_gather(uint8_t* dst, const uint2* src, int n, uint32_t tag, volatile int* abort_flag, int* status) {
-  const uint4* s = reinterpret_cast<const uint4*>(src);
-#pragma unroll 1
-  for (int i = threadIdx.x; i < n; i += 2 * TK_CT) {
-    const int d = i + TK_CT < n ? TK_CT : 0;                                    // (the same word twice at the end)
-    uint4 r[2];
-    tk_get(s + i, d, r, tag, abort_flag, status);
-    *reinterpret_cast<uint2*>(dst + i * 8) = make_uint2(r[0].x, r[0].z);
-    *reinterpret_cast<uint2*>(dst + (i + d) * 8) = make_uint2(r[1].x, r[1].z);
-  }
-}
-
 // Position-dependent geometry of the step, and this CTA's share of the tiles.
 struct TokenGeom {
   int start, n1, n2, t1, tpb;                         // context rows: n1 from slot `start`, n2 from slot 0; pieces: t1 + the rest = tpb
@@ -184,7 +80,6 @@ struct TokenGeom {
   long long pos;
 };
 // (the launcher keeps pieces x CTAs below 2^31)
-__device__ __noinline__ unsigned tk_div(unsigned a, unsigned b) { return a / b; }
 __device__ __forceinline__ int tk_lo(int c, int tot, int parts) { return (int)tk_div((unsigned)c * (unsigned)tot, (unsigned)parts); }
 __device__ __forceinline__ int tk_owner(int tile, int tot, int parts) { return (int)tk_div(((unsigned)tile + 1u) * (unsigned)parts - 1u, (unsigned)tot); }
 __device__ __forceinline__ TokenGeom tk_geom(const TokenParams& p) {
@@ -210,18 +105,15 @@ __device__ __forceinline__ TokenGeom tk_geom(const TokenParams& p) {
   return g;
 }
 
-// This warp's two ends in the CTA's stream of pieces: where it loads and where it consumes.
-struct TokenStream {
+// This warp's pieces of the CTA's stream: weight rows, cache rows, weight rows of each layer.
+struct TokenStream : TokenRing {
   const TokenParams& p;
   const TokenGeom& g;
-  uint64_t* full;                                     // this warp's barriers
-  uint32_t buf;                                       // and buffers
-  int na, nb, nc, ks_n, a0, c0;                       // pieces of the phases of a layer; weight slots of a row tile; first rows
+  int na, nb, nc, ks_n, a0, c0;                       // pieces of the phases of a layer; pieces of a row tile; first rows
   int l, i;                                           // next to load: layer, piece of the layer
-  int st, par;                                        // next to consume
-  int skip;                                           // pieces of the stream before the phase's first one of this warp
 
-  __device__ __forceinline__ void load(int at) {      // into buffer `at`; then step to the warp's next piece
+  __device__ TokenStream(const TokenParams& p_, const TokenGeom& g_) : p(p_), g(g_) {}
+  __device__ __forceinline__ void load(int at) {
     if (l >= p.L) return;
     const TokenLayer& ly = p.layer[l];
     const uint32_t dst = buf + at * TK_PIECE;
@@ -241,86 +133,7 @@ struct TokenStream {
     i += TK_CW;
     while (i >= na + nb + nc) { i -= na + nb + nc; ++l; }
   }
-  __device__ __forceinline__ uint32_t wait(volatile int* abort_flag) {         // -> shared address of the piece
-    (void)tk_bar_wait(&full[st], par, abort_flag, p.status);
-    __syncwarp();
-    return buf + st * TK_PIECE;
-  }
-  __device__ __forceinline__ void done(int lane, volatile int* abort_flag) {   // the piece is used up: refill its place
-    __syncwarp();
-    if (lane == 0 && !*abort_flag) load(st);
-    if (++st == p.depth) { st = 0; par ^= 1; }
-  }
-  // the warp's first piece among the next n of the stream, which then move on
-  __device__ __forceinline__ int phase(int n) {
-    const int first = skip;
-    int k = skip - n;
-    while (k < 0) k += TK_CW;
-    skip = k;
-    return first;
-  }
 };
-
-// Projection rows [n0, n1) of a weight: partial products per piece into psum, summed over the pieces of a row tile in a
-// fixed order, rounded to bf16: a tagged word for each pair of rows, or plain rows of y.
-// swz[j]: byte offset, inside a swizzled 16 x 128-byte block, of this lane's row and 16-byte piece 2 j (+ 1).
-template <int NB>
-__device__ __forceinline__ void tk_project(const TokenParams& p, TokenBars* bars, TokenStream& in, float* psum, uint32_t xs, int xs_ld, int count,
-                                           int n0, int n1, uint2* out, int out_ld, int copies, uint32_t tag, __nv_bfloat16* plain,
-                                           const uint32_t (&swz)[4], int lane) {
-  volatile int* abort_flag = &bars->abort_flag;
-  const int ks_n = in.ks_n, g8 = lane >> 2, t4 = lane & 3;
-  const int first = in.phase(count);
-  const uint32_t xrow0 = xs + min(lane & 7, p.B - 1) * xs_ld + 16 * (lane >> 3), xrow1 = xs + min(8 + (lane & 7), p.B - 1) * xs_ld + 16 * (lane >> 3);
-  int kb = first % ks_n;
-  named_bar(1, TK_CT);                                                          // the vector is in shared memory
-#pragma unroll 1
-  for (int i = first; i < count; i += TK_CW) {
-    uint32_t blk = in.wait(abort_flag), xo = kb * (TK_KW * 2);
-    float c[NB][2][4];
-#pragma unroll
-    for (int nb = 0; nb < NB; ++nb)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) c[nb][j >> 2][j & 3] = 0.f;
-    const int blocks = min(TK_KW, p.dim - kb * TK_KW) / 64;
-#pragma unroll 4
-    for (int k = 0; k < blocks; ++k, blk += TK_BLK, xo += 128) {                // a 16 x 64 block of the piece
-      uint32_t a[4][4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) tk_ldm4(a[j], blk + swz[j]);
-#pragma unroll
-      for (int nb = 0; nb < NB; ++nb) {
-        uint32_t b[2][4];
-        tk_ldm4(b[0], (nb ? xrow1 : xrow0) + xo); tk_ldm4(b[1], (nb ? xrow1 : xrow0) + xo + 64);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) tk_mma<false>(c[nb][j & 1], a[j], b[j >> 1][2 * (j & 1)], b[j >> 1][2 * (j & 1) + 1]);
-      }
-    }
-    in.done(lane, abort_flag);
-    float* ps = psum + i * (16 * 8 * NB) + g8 * (8 * NB) + 2 * t4;
-#pragma unroll
-    for (int nb = 0; nb < NB; ++nb) {
-      *reinterpret_cast<float2*>(ps + nb * 8) = make_float2(c[nb][0][0] + c[nb][1][0], c[nb][0][1] + c[nb][1][1]);
-      *reinterpret_cast<float2*>(ps + 8 * (8 * NB) + nb * 8) = make_float2(c[nb][0][2] + c[nb][1][2], c[nb][0][3] + c[nb][1][3]);
-    }
-    kb += TK_CW;
-    while (kb >= ks_n) kb -= ks_n;
-  }
-  named_bar(1, TK_CT);
-  const int pairs = (n1 - n0) >> 1;                                             // the rows come in pairs
-#pragma unroll 1
-  for (int i = threadIdx.x; i < pairs * p.B; i += TK_CT) {
-    const int b = p.B == 1 ? 0 : (int)tk_div(i, pairs), row = 2 * (i - b * pairs);
-    const float* ps = psum + (row >> 4) * ks_n * (16 * 8 * NB) + (row & 15) * (8 * NB) + b;
-    float s0 = 0.f, s1 = 0.f;
-#pragma unroll 8
-    for (int k = 0; k < ks_n; ++k, ps += 16 * 8 * NB) { s0 += ps[0]; s1 += ps[8 * NB]; }
-    const uint32_t v = pack_bf16(s0, s1);
-    if (plain) *reinterpret_cast<uint32_t*>(plain + (size_t)b * p.dim + n0 + row) = v;
-    else
-      for (int c = 0; c < copies; ++c) tk_put2(out + (size_t)(c * p.B + b) * out_ld + ((n0 + row) >> 1), v, tag);
-  }
-}
 
 // One warp: the raw q / k / v row (lane = 4 consecutive elements) -> normalised, rotated.
 __device__ __forceinline__ void tk_norm_rope(float (&x)[4], bool norm, bool rope, float eps, const float4 c, const float4 s, int lane) {
@@ -462,7 +275,10 @@ __global__ void __launch_bounds__(TK_CT, 1) swa_token_kernel(const __grid_consta
   __syncthreads();
 
   const int ks_n = (p.dim + TK_KW - 1) / TK_KW, na = (a1 - a0 + 15) / 16 * ks_n, nb = g.hi - g.lo, nc = (c1 - c0 + 15) / 16 * ks_n;
-  TokenStream in{p, g, bars->full + warp * TK_DEPTH, ring + warp * (p.depth * TK_PIECE), na, nb, nc, ks_n, a0, c0, 0, warp - TK_CW, 0, 0, warp};
+  TokenStream in(p, g);
+  in.full = bars->full + warp * TK_DEPTH; in.buf = ring + warp * (p.depth * TK_PIECE);
+  in.depth = p.depth; in.st = in.par = 0; in.skip = warp; in.abort_flag = abort_flag; in.status = p.status;
+  in.na = na; in.nb = nb; in.nc = nc; in.ks_n = ks_n; in.a0 = a0; in.c0 = c0; in.l = 0; in.i = warp - TK_CW;
   in.step();                                                                    // the warp's first piece
   if (lane == 0)
     for (int i = 0; i < p.depth; ++i) in.load(i);
@@ -496,8 +312,16 @@ __global__ void __launch_bounds__(TK_CT, 1) swa_token_kernel(const __grid_consta
         tk_gather(xs + b * xs_ld, (is_c ? p.o : p.xmid) + (size_t)(cta % TK_COPIES * p.B + b) * (p.dim / 2), p.dim / 4, is_c ? tag : tag - 1, abort_flag, p.status);
       }
     }
-    tk_project<NB>(p, bars, in, psum, smem_u32(xs), xs_ld, is_c ? nc : na, is_c ? c0 : a0, is_c ? c1 : a1, is_c ? p.xmid : p.qkv, (is_c ? 1 : 3) * (p.dim / 2),
-                   is_c ? TK_COPIES : 1, tag, ph == 2 * p.L - 1 ? p.y : nullptr, swz, lane);
+    const int n0 = is_c ? c0 : a0, out_ld = (is_c ? 1 : 3) * (p.dim / 2);
+    __nv_bfloat16* plain = ph == 2 * p.L - 1 ? p.y : nullptr;
+    tk_project<NB>(in, psum, smem_u32(xs), xs_ld, p.B, p.dim, is_c ? nc : na, (is_c ? c1 - c0 : a1 - a0) >> 1, swz, lane,
+                   [&](bool, int b, int row, float s0, float s1) {
+      const uint32_t v = pack_bf16(s0, s1);
+      if (plain) *reinterpret_cast<uint32_t*>(plain + (size_t)b * p.dim + n0 + row) = v;
+      else if (!is_c) tk_put2(p.qkv + (size_t)b * out_ld + ((n0 + row) >> 1), v, tag);
+      else
+        for (int c = 0; c < TK_COPIES; ++c) tk_put2(p.xmid + (size_t)(c * p.B + b) * out_ld + ((n0 + row) >> 1), v, tag);
+    });
     if (is_c) continue;
     // ---- phase B
 #pragma unroll 1
@@ -515,7 +339,7 @@ __global__ void __launch_bounds__(TK_CT, 1) swa_token_kernel(const __grid_consta
       if (sg == 0) named_bar(1, TK_CT);                                         // q is in shared memory
 #pragma unroll 1
       for (; piece < p_end; piece += TK_CW) {
-        const uint32_t blk = in.wait(abort_flag);
+        const uint32_t blk = in.wait();
         {
           const int j0 = piece - bh * g.tpb, valid = j0 < g.t1 ? g.n1 - 16 * j0 : g.n2 - 16 * (j0 - g.t1);
           float sc[4][4];
@@ -563,7 +387,7 @@ __global__ void __launch_bounds__(TK_CT, 1) swa_token_kernel(const __grid_consta
             tk_mma<F16>(acc[2 * j + 1], a, bv[2], bv[3]);
           }
         }
-        in.done(lane, abort_flag);
+        in.done(in, lane);
       }
       // the warps' shares of the segment
       lsum += __shfl_xor_sync(0xffffffffu, lsum, 4);
@@ -618,11 +442,7 @@ __global__ void __launch_bounds__(TK_CT, 1) swa_token_kernel(const __grid_consta
     for (int sg = warp; sg < merged; sg += TK_CW)
       tk_finish<F16>(p, g, ly, bars, kv, own, psum, any, others > 0 && sg == 0, bh_lo + sg * seg_step, sg, tag, lane);
   }
-  if (*abort_flag) {                                                            // leave only when no copy is in flight any more
-    const long long t0 = clock64();
-    for (int i = 0; i < p.depth; ++i)
-      while (!mbar_try_wait(&in.full[i], i < in.st ? in.par ^ 1 : in.par) && clock64() - t0 < TK_PATIENCE / 1000) {}
-  }
+  in.drain();
   // CTA 0 is done only when every CTA has contributed, hence read the position and the tag
   if (threadIdx.x == 0 && cta == 0) {
     *p.epoch = tag0 + p.L - 1;
@@ -643,21 +463,12 @@ extern "C" size_t daisy_b200_swa_token_workspace_bytes(int B, int H, int D) {
   return 256 + tk_align(B * 3 * dim * 4) + 2 * TK_COPIES * tk_align(B * dim * 4) + parts * TK_PART * 16;
 }
 
-// weights [4 dim rows][dim] as (64 columns, rows, blocks of 64 columns); a ring as (64 elements, slots, halves of a row, h, b)
-static int make_token_map(CUtensorMap* m, const void* base, int nd, const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box) {
-  daisy_host::EncodeTiledFn enc = daisy_host::get_encode_tiled();
-  if (!enc) return DAISY_ECUDA;
-  const cuuint32_t one[5] = {1, 1, 1, 1, 1};
-  return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, nd, const_cast<void*>(base), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? DAISY_OK : DAISY_ECUDA;
-}
-
 template <bool F16, int NB>
 static int launch_token(TokenParams& p, int sms, cudaStream_t st) {
   static bool attr[daisy_host::MAX_DEVICES] = {};
   const int dev = daisy_host::device_slot();
   if (dev < 0) return DAISY_ENODEV;
-  constexpr int limit = 232448;
+  constexpr int limit = TK_SMEM_LIMIT;
   if (!attr[dev]) {
     if (cudaFuncSetAttribute(swa_token_kernel<F16, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit) != cudaSuccess) {
       (void)cudaGetLastError();
@@ -665,8 +476,8 @@ static int launch_token(TokenParams& p, int sms, cudaStream_t st) {
     }
     attr[dev] = true;
   }
-  const int ks = (p.dim + TK_KW - 1) / TK_KW, tiles = ((3 * p.dim / 2 + sms - 1) / sms * 2 + 15) / 16;
-  const int psum = ks * tiles * 16 * 8 * NB * 4 > TK_CW * 512 ? ks * tiles * 16 * 8 * NB * 4 : TK_CW * 512;
+  int psum = tk_psum_bytes(p.dim, ((3 * p.dim / 2 + sms - 1) / sms * 2 + 15) / 16, NB);
+  if (psum < TK_CW * 512) psum = TK_CW * 512;                             // also the warps' attention accumulators
   const int fixed = 2048 + TK_FIXED + p.B * (p.dim + 8) * 2 + psum;
   p.depth = fixed + TK_CW * TK_DEPTH * TK_PIECE <= limit ? TK_DEPTH : 1;
   const int smem = fixed + TK_CW * p.depth * TK_PIECE;
@@ -715,17 +526,13 @@ extern "C" int daisy_b200_swa_token_step(const daisy_b200_token_layer* layers, i
       return DAISY_EALIGN;
     TokenLayer& ly = p.layer[l];
     int rc;
-    {
-      const cuuint64_t dims[3] = {64, 4 * (cuuint64_t)dim, (cuuint64_t)dim / 64}, st[2] = {(cuuint64_t)dim * 2, 128};
-      const cuuint32_t box[3] = {64, 16, TK_KW / 64};
-      if ((rc = make_token_map(&ly.tw, s.qkvo_w, 3, dims, st, box)) != DAISY_OK) return rc;
-    }
-    if (need_cache) {
+    if ((rc = tk_make_weight_map(&ly.tw, s.qkvo_w, 4 * dim, dim)) != DAISY_OK) return rc;
+    if (need_cache) {                                 // a ring as (64 elements, slots, halves of a row, h, b)
       const cuuint64_t dims[5] = {64, (cuuint64_t)cap, 2, (cuuint64_t)H, (cuuint64_t)B};
       const cuuint64_t st[4] = {(cuuint64_t)c_sr * 2, 128, (cuuint64_t)c_sh * 2, (cuuint64_t)c_sb * 2};
       const cuuint32_t box[5] = {64, 16, 2, 1, 1};
-      if ((rc = make_token_map(&ly.tk, s.kcache, 5, dims, st, box)) != DAISY_OK) return rc;
-      if ((rc = make_token_map(&ly.tv, s.vcache, 5, dims, st, box)) != DAISY_OK) return rc;
+      if ((rc = tk_make_map(&ly.tk, s.kcache, 5, dims, st, box)) != DAISY_OK) return rc;
+      if ((rc = tk_make_map(&ly.tv, s.vcache, 5, dims, st, box)) != DAISY_OK) return rc;
     }
     ly.kc = s.kcache; ly.vc = s.vcache; ly.ve = (const __nv_bfloat16*)s.ve; ly.ve_gate = s.ve_gate_logit;
     ly.k_new = (__nv_bfloat16*)s.k_new_out; ly.v_new = (__nv_bfloat16*)s.v_new_out; ly.cos = s.cos; ly.sin = s.sin;

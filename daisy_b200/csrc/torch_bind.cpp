@@ -83,7 +83,7 @@ void release_workspaces() {
   std::lock_guard<std::mutex> lock(g_mutex);
   g_pool.clear();
 }
-enum { WS_TOKEN = 0 };
+enum { WS_TOKEN = 0, WS_KDA_TOKEN = 1 };
 
 // ------------------------------------------------------------------ decode step
 void rope_table(const Tensor& t, const char* name) {
@@ -158,6 +158,156 @@ Tensor token_step(const Tensor& x_, const std::vector<Tensor>& weights, const st
   return y;
 }
 
+
+// ------------------------------------------------------------------ attention layer, whole sequences
+struct Doc { Tensor t; const int32_t* ptr = nullptr; int64_t sb = 0; };
+Doc doc_arg(const OptTensor& doc, int64_t B, int64_t T, const Tensor& like) {
+  Doc d;
+  if (!doc.has_value()) return d;
+  TORCH_CHECK_VALUE(doc->is_cuda(), "doc_start must be a CUDA tensor");
+  d.t = doc->to(like.device(), at::kInt).contiguous();
+  d.ptr = d.t.data_ptr<int32_t>();
+  if (d.t.dim() == 1 && d.t.size(0) == T) return d;
+  if (d.t.dim() == 2 && d.t.size(0) == B && d.t.size(1) == T) { d.sb = T; return d; }
+  TORCH_CHECK_VALUE(false, "doc_start must have shape [", T, "] or [", B, ",", T, "], got ", d.t.sizes());
+  return d;
+}
+
+Tensor rows_of(const Tensor& x, int64_t K) {
+  Tensor x2 = x.reshape({-1, K});
+  return x2.stride(1) == 1 ? x2 : x2.contiguous();
+}
+
+Tensor gemm_nt(const Tensor& x, const Tensor& w) {
+  req(x, "x"); req(w, "w");
+  const int64_t K = x.size(-1), N = w.size(0);
+  Tensor x2 = rows_of(x, K);
+  std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
+  shape.back() = N;
+  Tensor c = at::empty(shape, x.options());
+  check(daisy_b200_gemm_nt(x2.data_ptr(), x2.stride(0), w.data_ptr(), w.stride(0), c.data_ptr(), N, (int)x2.size(0), (int)N, (int)K, status_ptr(x), stream_of(x)),
+        "daisy_b200_gemm_nt");
+  return c;
+}
+
+// merged projection with the norm / RoPE / gate epilogue -> q', k', v' [B,T,H,128]
+std::vector<Tensor> qkv_gemm(const Tensor& x, const Tensor& w_qkv, const OptTensor& cos, const OptTensor& sin, int64_t H, double eps, int64_t flags,
+                             const OptTensor& ve, const OptTensor& ve_gate, const OptTensor& ring_k, const OptTensor& ring_v, int64_t ring_first) {
+  req(x, "x"); req(w_qkv, "w_qkv");
+  TORCH_CHECK_VALUE(x.dim() == 3, "x must be [B, T, dim]");
+  const int64_t B = x.size(0), T = x.size(1), dim = x.size(2);
+  TORCH_CHECK_VALUE(w_qkv.dim() == 2 && w_qkv.size(0) == 3 * H * 128 && w_qkv.size(1) == dim, "w_qkv must be [", 3 * H * 128, ", ", dim, "], got ", w_qkv.sizes());
+  Tensor x2 = rows_of(x, dim);
+  if (flags & DAISY_ROPE)
+    for (const OptTensor* t : {&cos, &sin})
+      TORCH_CHECK_VALUE(t->has_value() && (*t)->is_cuda() && (*t)->scalar_type() == at::kFloat && (*t)->is_contiguous() && (*t)->size(0) >= T && (*t)->size(1) == 64,
+                        "cos, sin must be contiguous float32 CUDA tensors of at least T rows");
+  Tensor ve2;
+  if (ve.has_value()) {
+    TORCH_CHECK_VALUE(ve_gate.has_value() && ve_gate->is_cuda() && ve_gate->scalar_type() == at::kFloat && ve_gate->numel() == 1,
+                      "ve needs ve_gate_logit, a float32 scalar CUDA tensor");
+    ve2 = ve->reshape({B * T, H * 128});
+    req(ve2, "ve");
+  }
+  int64_t sb = 0, sh = 0, sr = 0, cap = 0;
+  unsigned f = (unsigned)flags;
+  if (ring_k.has_value()) {
+    const Tensor &rk = *ring_k, &rv = *ring_v;
+    const bool f16 = rk.scalar_type() == at::kHalf;
+    req(rk, "ring k", f16 ? at::kHalf : at::kBFloat16); req(rv, "ring v", rk.scalar_type());
+    TORCH_CHECK_VALUE(rk.dim() == 4 && rk.sizes() == rv.sizes() && rk.strides() == rv.strides() && rk.size(0) == B && rk.size(1) == H && rk.size(3) == 128,
+                      "ring tensors must both be [", B, ", ", H, ", cap, 128] with equal strides");
+    sb = rk.stride(0); sh = rk.stride(1); sr = rk.stride(2); cap = rk.size(2);
+    f |= f16 ? DAISY_CACHE_FP16 : 0;
+  }
+  std::vector<Tensor> out;
+  for (int i = 0; i < 3; ++i) out.push_back(at::empty({B, T, H, 128}, x.options()));
+  check(daisy_b200_qkv_gemm_ring(x2.data_ptr(), x2.stride(0), w_qkv.data_ptr(), w_qkv.stride(0), cos.has_value() ? cos->data_ptr<float>() : nullptr,
+                                 sin.has_value() ? sin->data_ptr<float>() : nullptr, out[0].data_ptr(), out[1].data_ptr(), out[2].data_ptr(),
+                                 ve2.defined() ? ve2.data_ptr() : nullptr, ve2.defined() ? ve2.stride(0) : 0, ve2.defined() ? ve_gate->data_ptr<float>() : nullptr,
+                                 ring_k.has_value() ? ring_k->data_ptr() : nullptr, ring_k.has_value() ? ring_v->data_ptr() : nullptr, sb, sh, sr, (int)cap,
+                                 (int)ring_first, (int)B, (int)T, (int)H, 128, (int)dim, (float)eps, f, status_ptr(x), stream_of(x)),
+        "daisy_b200_qkv_gemm_ring");
+  return out;
+}
+
+// windowed attention on prepared [B,T,H,128] tensors -> (out, lse2 or undefined)
+std::pair<Tensor, Tensor> swa_attend(const Tensor& q, const Tensor& k, const Tensor& v, int64_t window, double scale, const OptTensor& out_, bool bounded,
+                                     const OptTensor& doc_start, bool in_blocks, bool want_lse) {
+  req(q, "q"); req(k, "k"); req(v, "v");
+  TORCH_CHECK_VALUE(q.dim() == 4 && k.sizes() == q.sizes() && v.sizes() == q.sizes(), "q, k, v must be [B,T,H,D] of one shape");
+  const int64_t B = q.size(0), T = q.size(1), H = q.size(2), D = q.size(3);
+  Tensor out = out_.has_value() ? *out_ : at::empty({B, T, H, D}, q.options());
+  Doc d = doc_arg(doc_start, B, T, q);
+  Tensor lse;
+  if (want_lse) lse = at::empty({B, H, T}, q.options().dtype(at::kFloat));
+  const unsigned flags = (bounded ? DAISY_BOUNDED_QK : 0) | (in_blocks ? DAISY_WINDOW_BLOCKS : 0);
+  auto call = [&](auto fn, auto... extra) {
+    return fn(q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), q.stride(1), q.stride(2), k.stride(0), k.stride(1), k.stride(2), v.stride(0), v.stride(1),
+              v.stride(2), out.data_ptr(), out.stride(0), out.stride(1), out.stride(2), extra..., (int)B, (int)T, (int)H, (int)D, (int)window, (float)scale, d.ptr,
+              d.sb, flags, status_ptr(q), stream_of(q));
+  };
+  if (want_lse) check(call(daisy_b200_swa_attend_lse, lse.data_ptr<float>()), "daisy_b200_swa_attend_lse");
+  else check(call(daisy_b200_swa_attend), "daisy_b200_swa_attend");
+  return {out, lse};
+}
+
+// One attention layer: projection, attention, output projection -> (y, k', v', q')
+std::vector<Tensor> attn_layer(const Tensor& x_, const Tensor& qkvo_w, const Tensor& cos, const Tensor& sin, int64_t H, double eps, double scale, int64_t window,
+                               const OptTensor& doc_start, bool in_blocks, const OptTensor& ve, const OptTensor& ve_gate, const OptTensor& ring_k,
+                               const OptTensor& ring_v, int64_t ring_first) {
+  Tensor w = qkvo_w.detach(), x = x_.detach().to(w.scalar_type());
+  TORCH_CHECK_VALUE(x.is_cuda(), "x must be a CUDA tensor (daisy_b200 has no CPU path)");
+  c10::cuda::CUDAGuard guard(x.device());
+  const int64_t B = x.size(0), T = x.size(1), dim = w.size(2);
+  auto p = qkv_gemm(x, w.narrow(0, 0, 3).view({3 * dim, dim}), cos, sin, H, eps, DAISY_QKV_DEFAULT, ve, ve_gate, ring_k, ring_v, ring_first);
+  Tensor y = swa_attend(p[0], p[1], p[2], window, scale, std::nullopt, true, doc_start, in_blocks, false).first;   // q, k are RMS-normalised
+  y = gemm_nt(y.view({B, T, dim}), w.select(0, 3));
+  return {y, p[1], p[2], p[0]};
+}
+
+// ------------------------------------------------------------------ Kimi layer, one token
+bool kda_token_supported(int64_t H) { return H >= 1 && daisy_b200_kda_token_workspace_bytes(1, (int)H, 128) != 0; }
+int64_t kda_token_workspace_bytes(int64_t B, int64_t H) { return (int64_t)daisy_b200_kda_token_workspace_bytes((int)std::min<int64_t>(B, 16), (int)H, 128); }
+
+// weights: q, k, v, f0, f1, g0, g1, b, o; conv: q, k, v weights (and biases); the states are updated in place
+Tensor kda_token_step(const Tensor& x_, const std::vector<Tensor>& w, const OptTensor& g1_bias, const OptTensor& norm_w, const std::vector<Tensor>& conv_w,
+                      const std::vector<OptTensor>& conv_b, const Tensor& a_log, const Tensor& dt_bias, Tensor state, const std::vector<Tensor>& conv_s,
+                      bool silu, double eps, const OptTensor& out, const OptTensor& workspace) {
+  TORCH_CHECK_VALUE(w.size() == 9 && conv_w.size() == 3 && conv_b.size() == 3 && conv_s.size() == 3, "nine weights, three convolutions");
+  const int64_t B = state.size(0), H = state.size(1), dim = H * 128;
+  TORCH_CHECK_VALUE(x_.is_cuda() && x_.numel() == B * dim && x_.size(-1) == dim, "x must be a CUDA tensor [", B, ", 1, ", dim, "]");
+  c10::cuda::CUDAGuard guard(x_.device());
+  Tensor x = x_.to(at::kBFloat16).reshape({B, dim}).contiguous();
+  for (const Tensor& t : w) { req(t, "weight"); TORCH_CHECK_VALUE(t.is_contiguous(), "weights must be contiguous"); }
+  daisy_b200_kda_layer ly{};
+  ly.q_w = w[0].data_ptr(); ly.k_w = w[1].data_ptr(); ly.v_w = w[2].data_ptr(); ly.f0_w = w[3].data_ptr(); ly.f1_w = w[4].data_ptr();
+  ly.g0_w = w[5].data_ptr(); ly.g1_w = w[6].data_ptr(); ly.b_w = w[7].data_ptr(); ly.o_w = w[8].data_ptr();
+  if (g1_bias.has_value()) { req(*g1_bias, "g_proj bias"); ly.g1_bias = g1_bias->data_ptr(); }
+  if (norm_w.has_value()) { req(*norm_w, "norm weight"); ly.norm_w = norm_w->data_ptr(); }
+  req(a_log, "A_log", at::kFloat); req(dt_bias, "dt_bias", at::kFloat); req(state, "state", at::kFloat);
+  TORCH_CHECK_VALUE(a_log.numel() == H && dt_bias.numel() == dim && a_log.is_contiguous() && state.is_contiguous() && state.numel() == B * H * 128 * 128,
+                    "state must be a contiguous [B, H, 128, 128]");
+  for (int i = 0; i < 3; ++i) {
+    req(conv_w[i], "conv weight"); req(conv_s[i], "conv state");
+    TORCH_CHECK_VALUE(conv_w[i].numel() == dim * 4 && conv_w[i].is_contiguous() && conv_s[i].is_contiguous() && conv_s[i].numel() == B * dim * 4,
+                      "four taps, states [B, dim, 4]");
+    ly.conv_w[i] = conv_w[i].data_ptr();
+    if (conv_b[i].has_value()) { req(*conv_b[i], "conv bias"); ly.conv_bias[i] = conv_b[i]->data_ptr(); }
+  }
+  ly.a_log = a_log.data_ptr<float>(); ly.dt_bias = dt_bias.data_ptr<float>();
+  Tensor y = out.has_value() ? *out : at::empty({B, 1, dim}, x.options());
+  Tensor ws = workspace.has_value() ? *workspace : stream_workspace(x, WS_KDA_TOKEN, kda_token_workspace_bytes(B, H));
+  for (int64_t b0 = 0; b0 < B; b0 += 16) {                               // larger batches: 16 rows a launch, the weights come from L2 again
+    const int64_t n = std::min<int64_t>(16, B - b0);
+    check(daisy_b200_kda_token_step(&ly, (char*)x.data_ptr() + b0 * dim * 2, dim, (char*)y.data_ptr() + b0 * dim * 2, state.data_ptr<float>() + b0 * H * 128 * 128,
+                                    (char*)conv_s[0].data_ptr() + b0 * dim * 8, (char*)conv_s[1].data_ptr() + b0 * dim * 8, (char*)conv_s[2].data_ptr() + b0 * dim * 8,
+                                    (int)n, (int)H, 128, (float)eps, silu ? DAISY_KDA_CONV_SILU : 0, ws.data_ptr(), (size_t)ws.numel(), status_ptr(x), stream_of(x)),
+          "daisy_b200_kda_token_step");
+  }
+  return y;
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -174,4 +324,18 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("token_workspace_bytes", [](int64_t B, int64_t H) { return (int64_t)daisy_b200_swa_token_workspace_bytes((int)B, (int)H, 128); });
   m.def("token_step_supported", &token_step_supported);
   m.def("token_step", &token_step);
+  m.def("gemm_nt", &gemm_nt);
+  m.def("qkv_gemm", &qkv_gemm);
+  m.def("swa_attend", [](const Tensor& q, const Tensor& k, const Tensor& v, int64_t window, double scale, const OptTensor& out, bool bounded,
+                         const OptTensor& doc_start, bool in_blocks) {
+    return swa_attend(q, k, v, window, scale, out, bounded, doc_start, in_blocks, false).first;
+  });
+  m.def("swa_attend_lse", [](const Tensor& q, const Tensor& k, const Tensor& v, int64_t window, double scale, const OptTensor& out, bool bounded,
+                             const OptTensor& doc_start, bool in_blocks) {
+    return swa_attend(q, k, v, window, scale, out, bounded, doc_start, in_blocks, true);
+  });
+  m.def("attn_layer", &attn_layer);
+  m.def("kda_token_supported", &kda_token_supported);
+  m.def("kda_token_workspace_bytes", &kda_token_workspace_bytes);
+  m.def("kda_token_step", &kda_token_step);
 }

@@ -15,7 +15,7 @@ chunked pair.
 
 ``B200ShortConvolution``, ``B200FusedRMSNormGated`` and ``B200KimiLinearSelfAttention`` mirror the rest of the
 layer (attention_kimi.py:41-62, 65-211): same constructors, parameter names and call protocol, on the kernels of
-``csrc/kda_layer.cu``; the layer adds ``capture_step`` / ``step_graph`` (one CUDA-graph replay per decoded token).
+``csrc/kda_layer.cu``; the layer adds ``capture_step`` / ``step_graph`` (the decode step into fixed buffers).
 """
 from __future__ import annotations
 
@@ -24,6 +24,7 @@ from typing import Optional
 import torch
 
 from . import ops
+from ._native import ext
 
 RECURRENT_MAX_T = 4      # up to this many tokens the state is carried token by token in registers
 
@@ -184,12 +185,41 @@ class B200KimiLinearSelfAttention(torch.nn.Module):
     def reset_history(self):
         self._recurrent_state, self._conv_state, self._seen = None, None, 0
 
+    def _token_step(self, x, out=None, workspace=None):
+        """The decode step as one launch (``csrc/kda_token.cu``; 16 batch rows at a time), states updated in place; None
+        where the layer or its states are not of the form that kernel takes."""
+        rec, conv = self._recurrent_state, self._conv_state
+        if (rec is None or conv is None or x.shape[1] != 1 or not x.is_cuda or self.conv_size != 4 or self.head_dim != 128
+                or self.head_v_dim != 128 or self.hidden_size != self.key_dim or not ext().kda_token_supported(self.num_heads)
+                or rec.dtype != torch.float32 or rec.shape[0] != x.shape[0] or not rec.is_contiguous() or not rec.is_cuda
+                or any(c.dtype != torch.bfloat16 or not c.is_contiguous() for c in conv)):
+            return None
+        m, p = self._modules, self._parameters
+        lin = lambda name: m[name]._parameters["weight"]
+        seq = lambda name, i: m[name]._modules[i]._parameters["weight"]
+        w = [lin("q_proj"), lin("k_proj"), lin("v_proj"), seq("f_proj", "0"), seq("f_proj", "1"), seq("g_proj", "0"), seq("g_proj", "1"),
+             lin("b_proj"), lin("o_proj")]
+        cv = [m["q_conv1d"], m["k_conv1d"], m["v_conv1d"]]
+        act = cv[0].activation
+        fp32 = (p["A_log"], p["dt_bias"])
+        if (any(t.dtype != torch.bfloat16 for t in w) or any(t.dtype != torch.float32 for t in fp32)
+                or any(c.activation != act or c._parameters["weight"].dtype != torch.bfloat16 for c in cv)):
+            return None
+        return ext().kda_token_step(x, w, m["g_proj"]._modules["1"]._parameters["bias"], m["o_norm"]._parameters["weight"],
+                                    [c._parameters["weight"] for c in cv], [c._parameters["bias"] for c in cv], p["A_log"], p["dt_bias"],
+                                    rec, list(conv), act is not None, 1e-6, out, workspace)
+
     def _forward_core(self, x, ve, sa_lambdas, attn_mask, use_cache: bool):
         if torch.is_grad_enabled() and (x.requires_grad or any(p.requires_grad for p in self.parameters())):
             # the kernels return tensors without a grad_fn: autograd would treat the layer as a constant
             raise NotImplementedError("daisy_b200 implements the forward pass only: call under torch.no_grad() / "
                                       "inference_mode(), or detach the input and freeze the parameters")
         B0, T0, _ = x.shape
+        if use_cache and T0 == 1 and attn_mask is None and (ve is None or sa_lambdas is None):
+            y = self._token_step(x)
+            if y is not None:
+                self._seen += 1
+                return y
         indices = tabs = None
         if attn_mask is not None:                                          # attention_kimi.py:150-154
             indices, cu_seqlens, _ = get_unpad_data(attn_mask[:, -T0:])
@@ -237,13 +267,16 @@ class B200KimiLinearSelfAttention(torch.nn.Module):
     # ------------------------------------------------------------------ CUDA-graph decode step
     @torch.inference_mode()
     def capture_step(self, batch: int = 1) -> None:
-        """Record one single-token ``step`` (no value embedding) into a CUDA graph.  Needs the states a ``prefill``
-        leaves; they are updated in place by the replayed kernels, input and output are fixed buffers.
-        ``step_graph(x)`` then costs one copy and one graph launch instead of ~17 launches issued from Python."""
+        """Prepare ``step_graph``: a single-token ``step`` (no value embedding) into a fixed output buffer.  Needs the states a
+        ``prefill`` leaves; they are updated in place.  Where the layer takes the single-launch step that launch is all of it;
+        otherwise the step is recorded into a CUDA graph, and ``step_graph(x)`` costs one copy and one graph launch."""
         if self._recurrent_state is None or (self.use_short_conv and self._conv_state is None):
             raise RuntimeError("capture_step needs the cached states of a prefill")
         dev = self._recurrent_state.device
         self._gx = torch.zeros(batch, 1, self.hidden_size, device=dev, dtype=torch.bfloat16)
+        self._graph, self._gy = None, torch.zeros_like(self._gx)
+        if ext().kda_token_supported(self.num_heads):
+            self._gws = torch.zeros(ext().kda_token_workspace_bytes(batch, self.num_heads), dtype=torch.uint8, device=dev)
         saved = [self._recurrent_state.clone()] + [c.clone() for c in (self._conv_state or ())]
         seen = self._seen
 
@@ -256,9 +289,13 @@ class B200KimiLinearSelfAttention(torch.nn.Module):
         side = torch.cuda.Stream(device=dev)
         side.wait_stream(torch.cuda.current_stream(dev))
         with torch.cuda.stream(side):                              # warm-up outside the capture (lazy initialisation)
-            self._forward_core(self._gx, None, None, None, use_cache=True)
+            one_launch = ext().kda_token_supported(self.num_heads) and self._token_step(self._gx, self._gy, self._gws) is not None
+            if not one_launch:
+                self._forward_core(self._gx, None, None, None, use_cache=True)
         torch.cuda.current_stream(dev).wait_stream(side)
         restore()
+        if one_launch:
+            return
         self._graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(self._graph):
             self._gy = self._forward_core(self._gx, None, None, None, use_cache=True)
@@ -266,9 +303,12 @@ class B200KimiLinearSelfAttention(torch.nn.Module):
 
     @torch.inference_mode()
     def step_graph(self, x):
-        """``step`` through the captured graph: ``x [batch, 1, dim]`` -> ``y`` (a fixed buffer, overwritten by the next call)."""
-        self._gx.copy_(x)
-        self._graph.replay()
+        """``step`` into the fixed buffer: ``x [batch, 1, dim]`` -> ``y`` (overwritten by the next call)."""
+        if self._graph is None:
+            self._token_step(x, self._gy, self._gws)
+        else:
+            self._gx.copy_(x)
+            self._graph.replay()
         self._seen += 1
         return self._gy
 

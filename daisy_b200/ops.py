@@ -103,56 +103,13 @@ def qkv_gemm(x, w_qkv, cos, sin, num_heads: int, eps: float, flags: int = QKV_DE
     the normalised v: ``v' = g * norm(v) + (1 - g) * ve``.  ``ring = (k_ring, v_ring)``, one layer of a KV ring
     ``[B,H,cap,128]`` (bf16 or float16): the epilogue also stores rows ``t >= ring_first`` of k', v' into slot
     ``t % cap`` -- the rows ``KVCache.bulk_write_packed`` keeps when ``ring_first = T - min(T, cap - 1)``."""
-    _req(x, "x"); _req(w_qkv, "w_qkv")
-    B, T, dim = x.shape
-    H, D = int(num_heads), 128
-    if w_qkv.shape != (3 * H * D, dim):
-        raise ValueError(f"w_qkv must be [{3 * H * D}, {dim}], got {tuple(w_qkv.shape)}")
-    x2 = x.reshape(B * T, dim)
-    if x2.stride(1) != 1:
-        x2 = x2.contiguous()
-    if flags & ROPE:
-        cos, sin = _f32c(cos, "cos"), _f32c(sin, "sin")
-        assert cos.shape[0] >= T and cos.shape[1] == D // 2
-    ve_args = (None, 0, None)
-    if ve is not None:
-        if ve_gate_logit is None or not (ve_gate_logit.is_cuda and ve_gate_logit.dtype == torch.float32 and ve_gate_logit.numel() == 1):
-            raise ValueError("ve needs ve_gate_logit, a float32 scalar CUDA tensor")
-        ve2 = ve.reshape(B * T, H * D)
-        _req(ve2, "ve")
-        ve_args = (ve2.data_ptr(), ve2.stride(0), ve_gate_logit.data_ptr())
-    outs = [torch.empty(B, T, H, D, dtype=torch.bfloat16, device=x.device) for _ in range(3)]
-    ring_args = (None, None, 0, 0, 0, 0, 0)
-    if ring is not None:
-        rk, rv = ring
-        f16 = rk.dtype == torch.float16
-        _req(rk, "ring k", rk.dtype if f16 else torch.bfloat16); _req(rv, "ring v", rk.dtype)
-        if rk.shape != rv.shape or rk.stride() != rv.stride() or rk.shape[0] != B or rk.shape[1] != H or rk.shape[3] != D:
-            raise ValueError(f"ring tensors must both be [{B}, {H}, cap, {D}] with equal strides")
-        ring_args = (rk.data_ptr(), rv.data_ptr(), rk.stride(0), rk.stride(1), rk.stride(2), rk.shape[2], int(ring_first))
-        flags = flags | (_lib.CACHE_FP16 if f16 else 0)
-    rc = _lib.lib().daisy_b200_qkv_gemm_ring(
-        x2.data_ptr(), x2.stride(0), w_qkv.data_ptr(), w_qkv.stride(0),
-        cos.data_ptr() if cos is not None else None, sin.data_ptr() if sin is not None else None,
-        outs[0].data_ptr(), outs[1].data_ptr(), outs[2].data_ptr(), *ve_args, *ring_args, B, T, H, D, dim, eps, flags,
-        status_word(x.device).data_ptr(), _stream(x))
-    _lib.check(rc, "daisy_b200_qkv_gemm_ring")
-    return tuple(outs)
+    rk, rv = ring if ring is not None else (None, None)
+    return tuple(ext().qkv_gemm(x, w_qkv, cos, sin, int(num_heads), eps, flags, ve, ve_gate_logit, rk, rv, int(ring_first)))
 
 
 def gemm_nt(x, w):
     """``x [..., K] @ w[N, K]^T`` in bf16 with fp32 accumulation (``F.linear(x, w)``) on the tcgen05 GEMM kernel."""
-    _req(x, "x"); _req(w, "w")
-    K = x.shape[-1]
-    x2 = x.reshape(-1, K)
-    if x2.stride(1) != 1:
-        x2 = x2.contiguous()
-    M, N = x2.shape[0], w.shape[0]
-    c = torch.empty(M, N, dtype=torch.bfloat16, device=x.device)
-    rc = _lib.lib().daisy_b200_gemm_nt(x2.data_ptr(), x2.stride(0), w.data_ptr(), w.stride(0), c.data_ptr(), c.stride(0),
-                                       M, N, K, status_word(x.device).data_ptr(), _stream(x))
-    _lib.check(rc, "daisy_b200_gemm_nt")
-    return c.view(*x.shape[:-1], N)
+    return ext().gemm_nt(x, w)
 
 
 def gemm_skinny(x, w, out: Optional[torch.Tensor] = None):
@@ -196,33 +153,9 @@ def swa_attend(q, k, v, window: Optional[int], scale: float = ATTN_SCALE,
     ``window`` counts blocks of 128 tokens (key block >= query block - window + 1), the training-form mask.
     ``return_lse``: also return ``lse2 [B,H,T]`` float32 (base-2 log of each row's softmax denominator), what
     :func:`swa_attend_bwd` needs."""
-    for n, t in (("q", q), ("k", k), ("v", v)):
-        _req(t, n)
-    B, T, H, D = q.shape
-    assert k.shape == q.shape and v.shape == q.shape
-    if out is None:
-        out = torch.empty(B, T, H, D, dtype=torch.bfloat16, device=q.device)
-    _doc, doc_ptr, doc_sb = _doc_arg(doc_start, B, T, q.device)
     if return_lse:
-        lse = torch.empty(B, H, T, dtype=torch.float32, device=q.device)
-        rc = _lib.lib().daisy_b200_swa_attend_lse(
-            q.data_ptr(), k.data_ptr(), v.data_ptr(),
-            q.stride(0), q.stride(1), q.stride(2), k.stride(0), k.stride(1), k.stride(2),
-            v.stride(0), v.stride(1), v.stride(2), out.data_ptr(),
-            out.stride(0), out.stride(1), out.stride(2), lse.data_ptr(), B, T, H, D, int(window or 0), scale, doc_ptr, doc_sb,
-            (_lib.BOUNDED_QK if bounded_qk else 0) | (_lib.WINDOW_BLOCKS if window_in_blocks else 0),
-            status_word(q.device).data_ptr(), _stream(q))
-        _lib.check(rc, "daisy_b200_swa_attend_lse")
-        return out, lse
-    rc = _lib.lib().daisy_b200_swa_attend(
-        q.data_ptr(), k.data_ptr(), v.data_ptr(),
-        q.stride(0), q.stride(1), q.stride(2), k.stride(0), k.stride(1), k.stride(2),
-        v.stride(0), v.stride(1), v.stride(2), out.data_ptr(),
-        out.stride(0), out.stride(1), out.stride(2), B, T, H, D, int(window or 0), scale, doc_ptr, doc_sb,
-        (_lib.BOUNDED_QK if bounded_qk else 0) | (_lib.WINDOW_BLOCKS if window_in_blocks else 0),
-        status_word(q.device).data_ptr(), _stream(q))
-    _lib.check(rc, "daisy_b200_swa_attend")
-    return out
+        return ext().swa_attend_lse(q, k, v, int(window or 0), scale, out, bounded_qk, doc_start, window_in_blocks)
+    return ext().swa_attend(q, k, v, int(window or 0), scale, out, bounded_qk, doc_start, window_in_blocks)
 
 
 def swa_attend_bwd(q, k, v, o, d_o, lse2, window: Optional[int], scale: float = ATTN_SCALE,

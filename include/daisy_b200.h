@@ -458,6 +458,27 @@ int daisy_b200_kda_out_norm(const void* o, int o_is_fp32, const void* gate, cons
 int daisy_b200_selftest_umma(const void* a, const void* b, float* c, int K, int mode,
                              int* status_word, void* stream);
 
+/* One decoded token through a Kimi-delta-attention layer in one launch (KimiLinearSelfAttention.step,
+ * models/daisy/attention_kimi.py:128-211): projections, short convolutions (four taps, SiLU with DAISY_KDA_CONV_SILU), decay
+ * gate, recurrent update, gated norm, output projection.  dim = H * 128 <= 2048, B <= 16.  Weights bf16, row-major as their
+ * Linear layers hold them; a_log [H] and dt_bias [dim] fp32.  state [B,H,128,128] fp32 and conv_q / conv_k / conv_v
+ * [B,dim,4] bf16 are updated in place.  x [B,dim] (row stride x_sb elements), y [B,dim].  Cooperative launch; workspace as
+ * in daisy_b200_swa_token_step. */
+typedef struct daisy_b200_kda_layer {
+  const void *q_w, *k_w, *v_w;               /* [dim, dim] */
+  const void *f0_w, *g0_w;                   /* [128, dim] */
+  const void *b_w;                           /* [H, dim] */
+  const void *o_w;                           /* [dim, dim] */
+  const void *f1_w, *g1_w;                   /* [dim, 128] */
+  const void *g1_bias, *norm_w;              /* [dim], [128]; each may be NULL */
+  const void *conv_w[3], *conv_bias[3];      /* q, k, v: [dim, 4]; [dim] or NULL */
+  const float *a_log, *dt_bias;
+} daisy_b200_kda_layer;
+size_t daisy_b200_kda_token_workspace_bytes(int B, int H, int D);
+int daisy_b200_kda_token_step(const daisy_b200_kda_layer* layer, const void* x, int64_t x_sb, void* y, float* state,
+                              void* conv_q, void* conv_k, void* conv_v, int B, int H, int D, float eps, unsigned flags,
+                              void* workspace, size_t workspace_bytes, int* status_word, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

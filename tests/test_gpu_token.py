@@ -64,3 +64,29 @@ def test_token_step_matches_oracle(B, H, L, t, cap, window, f16):
     mask = torch.ones(cap, dtype=torch.bool)
     mask[t % cap] = False
     assert torch.equal(k1[:, :, :, mask].cpu(), rk[:, :, :, mask]) and torch.equal(v1[:, :, :, mask].cpu(), rv[:, :, :, mask])
+
+
+@pytest.mark.parametrize("B,H,bias", [(1, 1, False), (3, 6, True), (8, 16, False), (9, 5, True), (17, 2, False)])
+def test_kimi_token_step_continues_a_prefill(B, H, bias):
+    """The single-launch Kimi step (csrc/kda_token.cu) after a prefill of T tokens against a prefill of T + 1: the output,
+    the recurrent state and the convolution states; batches that are one, several and more than sixteen rows."""
+    from daisy_b200 import B200KimiLinearSelfAttention, ops
+    torch.manual_seed(B * 100 + H)
+    layer = B200KimiLinearSelfAttention(H * D, H, 4096, D, conv_bias=bias).cuda()
+    T = 70
+    x = torch.randn(B, T + 1, H * D, device="cuda", dtype=torch.bfloat16)
+    with torch.inference_mode():
+        ref, _, _ = layer.prefill(x)
+        rec, conv = layer._recurrent_state.clone(), [c.clone() for c in layer._conv_state]
+        layer.reset_history()
+        layer.prefill(x[:, :T])
+        assert layer._token_step(x[:, T:], torch.empty(B, 1, H * D, device="cuda", dtype=torch.bfloat16)) is not None
+        layer.reset_history()
+        layer.prefill(x[:, :T])
+        y, _, _ = layer.step(x[:, T:])
+    ops.check_device_status("cuda")
+    assert_close_bf16(y, ref[:, T:], "y", max_tol=3e-2, mean_tol=3e-3)
+    assert ((layer._recurrent_state - rec).norm() / rec.norm()).item() < 5e-3
+    for a, b in zip(layer._conv_state, conv):
+        assert torch.equal(a[..., :3], b[..., :3]), "the carried inputs move up"
+        assert_close_bf16(a, b, "the new input")

@@ -17,10 +17,10 @@ a ``WindowMask(window[, doc_start])``, an int, ``None`` (plain causal) -- or the
 (:func:`band_of_dense_mask`) and rejected if it is not such a band.
 
 Training.  When a call needs gradients (grad mode on and the input or a parameter requires them) ``forward``
-takes the differentiable route: ``F.linear`` projections (autograd supplies their gradients) around
-``daisy_b200.autograd.swa_attention``, whose backward is this library's tcgen05 backward kernels.  In a layer that
-receives a value embedding the norm of v and the gate are torch operations on that route, so the gate parameter and
-``ve`` get their gradients too.  The cache-writing ``prefill`` / ``step`` forms have no backward and raise.
+takes the differentiable route: one autograd function for the layer (``AttnFunction`` of ``csrc/torch_bind.cpp``) on the
+same forward kernels, this library's tcgen05 attention backward, one pass that undoes norms, RoPE and the value-embedding
+gate (the gate parameter and ``ve`` get their gradients too), and library products for the projections' gradients.  The
+cache-writing ``prefill`` / ``step`` forms have no backward and raise.
 """
 from __future__ import annotations
 
@@ -228,8 +228,8 @@ class B200CausalSelfAttention(nn.Module):
                                       "it under torch.no_grad() / inference_mode(), or detach the input and freeze the parameters")
 
     def _attend_autograd(self, x: Tensor, ve: Optional[Tensor], mask):
-        """The differentiable forward: same arithmetic as ``_attend`` with the norm / RoPE as their own pass.  In a layer
-        with a value embedding the norm of v and the gate ``v = s(g_ve) norm(v) + (1 - s(g_ve)) ve``
+        """The differentiable forward: ``_attend``'s kernels under one autograd function for the whole layer.  Only a value
+        embedding that is not bf16 takes the composed route: norm / RoPE as their own pass, and the norm of v and the gate ``v = s(g_ve) norm(v) + (1 - s(g_ve)) ve``
         (models/daisy/attention.py:125,132-135) are torch operations, so autograd supplies the gradients of ``g_ve`` and
         ``ve`` as well, and the kernels get a v they must not normalise again."""
         from .autograd import swa_attention
@@ -238,16 +238,16 @@ class B200CausalSelfAttention(nn.Module):
         B, T = x.size(0), x.size(1)
         cos, sin = self.rotary.tables(T)
         w = self.qkvo_w
+        torch._assert(ve is not None or not self.receives_ve, "ve must be provided when receives_ve=True")
+        if not self.receives_ve or ve.dtype == torch.bfloat16:
+            return ext().attn_train(x, w, ve if self.receives_ve else None, self.g_ve, cos, sin, self.num_heads, self.norm_eps, self.attn_scale,
+                                    int(window or 0), doc_start, in_blocks)
         qkv = F.linear(x.to(w.dtype), w[:3].flatten(end_dim=1)).view(B, T, 3 * self.num_heads, self.head_dim)
         q, k, v = qkv.chunk(3, dim=-2)
-        flags = QKV_DEFAULT
-        if self.receives_ve:
-            torch._assert(ve is not None, "ve must be provided when receives_ve=True")
-            vn = F.rms_norm(v.float(), (self.head_dim,), eps=self.norm_eps)
-            g = torch.sigmoid(self.g_ve.float())
-            v = (g * vn + (1.0 - g) * ve.view_as(v).float()).to(q.dtype)
-            flags = QKV_DEFAULT & ~NORM_V
-        y = swa_attention(q, k, v, cos, sin, window, self.attn_scale, self.norm_eps, flags, doc_start, in_blocks)
+        vn = F.rms_norm(v.float(), (self.head_dim,), eps=self.norm_eps)
+        g = torch.sigmoid(self.g_ve.float())
+        v = (g * vn + (1.0 - g) * ve.view_as(v).float()).to(q.dtype)
+        y = swa_attention(q, k, v, cos, sin, window, self.attn_scale, self.norm_eps, QKV_DEFAULT & ~NORM_V, doc_start, in_blocks)
         return F.linear(y.view(B, T, self.m_dim), w[3])
 
     def _attend(self, x: Tensor, ve: Optional[Tensor], mask, ring=None, ring_first: int = 0):

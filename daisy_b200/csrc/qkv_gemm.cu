@@ -59,6 +59,9 @@ struct GemmParams {
   void* ring[2];
   int64_t r_sb, r_sh, r_sr;
   int cap, ring_first, ring_f16;
+  // training: 1 / rms of every row and head slot, [M][3 H], and v as normalised before the gate, [M, H, 128]; or null
+  float* rstd;
+  __nv_bfloat16* vn;
 };
 
 struct GemmBars {
@@ -196,6 +199,7 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
 #pragma unroll
             for (int i = 0; i < 128; ++i) { const float x = __uint_as_float(r[i]); ss = fmaf(x, x, ss); }
             const float rs = rsqrtf(ss * (1.0f / 128.0f) + p.eps);
+            if (p.rstd && m < p.M) p.rstd[(size_t)m * (3 * p.H) + nh] = rs;
 #pragma unroll
             for (int i = 0; i < 128; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * rs);
           }
@@ -215,6 +219,13 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
                 r[i + 64] = __float_as_uint(b2 * cc[e] - a * sn[e]);
               }
             }
+          }
+          if (which == 2 && p.vn && m < p.M) {                      // (thread = row: the gated layers of a model are few)
+            uint4* vd = reinterpret_cast<uint4*>(p.vn + ((size_t)m * p.H + h) * 128);
+#pragma unroll
+            for (int c = 0; c < 16; ++c)
+              vd[c] = make_uint4(pack_bf16(__uint_as_float(r[8 * c]), __uint_as_float(r[8 * c + 1])), pack_bf16(__uint_as_float(r[8 * c + 2]), __uint_as_float(r[8 * c + 3])),
+                                 pack_bf16(__uint_as_float(r[8 * c + 4]), __uint_as_float(r[8 * c + 5])), pack_bf16(__uint_as_float(r[8 * c + 6]), __uint_as_float(r[8 * c + 7])));
           }
           if (which == 2 && p.ve) {                                // value-embedding gate on the normalised v
             const float gte = 1.0f / (1.0f + __expf(-*p.ve_gate_logit));
@@ -365,24 +376,11 @@ extern "C" int daisy_b200_gemm_nt(const void* x, int64_t ldx, const void* w, int
   return gemm_common(x, ldx, w, ldw, p, stream);
 }
 
-extern "C" int daisy_b200_qkv_gemm(const void* x, int64_t ldx, const void* w_qkv, int64_t ldw,
-                                   const float* cos, const float* sin,
-                                   void* q_out, void* k_out, void* v_out,
-                                   const void* ve, int64_t ve_ld, const float* ve_gate_logit,
-                                   int B, int T, int H, int D, int dim, float eps, unsigned flags,
-                                   int* status_word, void* stream) {
-  return daisy_b200_qkv_gemm_ring(x, ldx, w_qkv, ldw, cos, sin, q_out, k_out, v_out, ve, ve_ld, ve_gate_logit,
-                                  nullptr, nullptr, 0, 0, 0, 0, 0, B, T, H, D, dim, eps, flags, status_word, stream);
-}
-
-extern "C" int daisy_b200_qkv_gemm_ring(const void* x, int64_t ldx, const void* w_qkv, int64_t ldw,
-                                        const float* cos, const float* sin,
-                                        void* q_out, void* k_out, void* v_out,
-                                        const void* ve, int64_t ve_ld, const float* ve_gate_logit,
-                                        void* ring_k, void* ring_v, int64_t r_sb, int64_t r_sh, int64_t r_sr,
-                                        int cap, int ring_first,
-                                        int B, int T, int H, int D, int dim, float eps, unsigned flags,
-                                        int* status_word, void* stream) {
+static int qkv_gemm_launch(const void* x, int64_t ldx, const void* w_qkv, int64_t ldw, const float* cos, const float* sin,
+                           void* q_out, void* k_out, void* v_out, const void* ve, int64_t ve_ld, const float* ve_gate_logit,
+                           void* ring_k, void* ring_v, int64_t r_sb, int64_t r_sh, int64_t r_sr, int cap, int ring_first,
+                           float* rstd, void* vn, int B, int T, int H, int D, int dim, float eps, unsigned flags,
+                           int* status_word, void* stream) {
   if (!q_out || !k_out || !v_out || B <= 0 || T <= 0 || H <= 0) return DAISY_EINVAL;
   if (D != DAISY_HEAD_DIM) return DAISY_EUNSUPPORTED;
   if ((int64_t)B * T >= (int64_t)1 << 31) return DAISY_EUNSUPPORTED;
@@ -402,6 +400,41 @@ extern "C" int daisy_b200_qkv_gemm_ring(const void* x, int64_t ldx, const void* 
   p.out[0] = (__nv_bfloat16*)q_out; p.out[1] = (__nv_bfloat16*)k_out; p.out[2] = (__nv_bfloat16*)v_out;
   p.cos = cos; p.sin = sin; p.T = T; p.H = H; p.eps = eps; p.flags = flags & DAISY_QKV_DEFAULT; p.status = status_word;
   p.ring[0] = ring_k; p.ring[1] = ring_v; p.r_sb = r_sb; p.r_sh = r_sh; p.r_sr = r_sr;
+  p.rstd = rstd; p.vn = (__nv_bfloat16*)vn;
   p.cap = cap; p.ring_first = ring_first; p.ring_f16 = (flags & DAISY_CACHE_FP16) ? 1 : 0;
   return gemm_common(x, ldx, w_qkv, ldw, p, stream);
+}
+
+extern "C" int daisy_b200_qkv_gemm(const void* x, int64_t ldx, const void* w_qkv, int64_t ldw,
+                                   const float* cos, const float* sin,
+                                   void* q_out, void* k_out, void* v_out,
+                                   const void* ve, int64_t ve_ld, const float* ve_gate_logit,
+                                   int B, int T, int H, int D, int dim, float eps, unsigned flags,
+                                   int* status_word, void* stream) {
+  return qkv_gemm_launch(x, ldx, w_qkv, ldw, cos, sin, q_out, k_out, v_out, ve, ve_ld, ve_gate_logit,
+                         nullptr, nullptr, 0, 0, 0, 0, 0, nullptr, nullptr, B, T, H, D, dim, eps, flags, status_word, stream);
+}
+
+extern "C" int daisy_b200_qkv_gemm_ring(const void* x, int64_t ldx, const void* w_qkv, int64_t ldw,
+                                        const float* cos, const float* sin,
+                                        void* q_out, void* k_out, void* v_out,
+                                        const void* ve, int64_t ve_ld, const float* ve_gate_logit,
+                                        void* ring_k, void* ring_v, int64_t r_sb, int64_t r_sh, int64_t r_sr,
+                                        int cap, int ring_first,
+                                        int B, int T, int H, int D, int dim, float eps, unsigned flags,
+                                        int* status_word, void* stream) {
+  return qkv_gemm_launch(x, ldx, w_qkv, ldw, cos, sin, q_out, k_out, v_out, ve, ve_ld, ve_gate_logit,
+                         ring_k, ring_v, r_sb, r_sh, r_sr, cap, ring_first, nullptr, nullptr, B, T, H, D, dim, eps, flags, status_word, stream);
+}
+
+extern "C" int daisy_b200_qkv_gemm_train(const void* x, int64_t ldx, const void* w_qkv, int64_t ldw,
+                                         const float* cos, const float* sin,
+                                         void* q_out, void* k_out, void* v_out, float* rstd, void* vn_out,
+                                         const void* ve, int64_t ve_ld, const float* ve_gate_logit,
+                                         int B, int T, int H, int D, int dim, float eps, unsigned flags,
+                                         int* status_word, void* stream) {
+  if (!rstd || (ve != nullptr) != (vn_out != nullptr) || (flags & DAISY_QKV_DEFAULT) != DAISY_QKV_DEFAULT) return DAISY_EINVAL;
+  if (!daisy_aligned16(vn_out)) return DAISY_EALIGN;
+  return qkv_gemm_launch(x, ldx, w_qkv, ldw, cos, sin, q_out, k_out, v_out, ve, ve_ld, ve_gate_logit,
+                         nullptr, nullptr, 0, 0, 0, 0, 0, rstd, vn_out, B, T, H, D, dim, eps, flags, status_word, stream);
 }

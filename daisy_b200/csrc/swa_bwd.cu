@@ -57,6 +57,17 @@ __device__ __forceinline__ void bwd_range(int blk, int nblk, int T, int window, 
     hi = nblk - 1;
     if (window_blocks > 0) hi = min(hi, blk + window_blocks - 1);
     else if (window > 0) hi = min(hi, (blk * WB + WB - 1 + window - 1) / WB);
+    if (doc_row && hi > lo && doc_row[hi * WB] > blk * WB + WB - 1) {
+      // later documents see none of these keys: doc_start does not decrease, so the last query block whose first row's
+      // document begins at or before the last key is found by bisection (six documents of 8192 tokens under a
+      // 2048-token window: the kernel 3.48 -> 2.24 ms at 8 x 8192 tokens, 16 heads)
+      int a = lo, c = hi;                                  // a: visible (its own block), c: not
+      while (c - a > 1) {
+        const int m = (a + c) >> 1;
+        if (doc_row[m * WB] > blk * WB + WB - 1) c = m; else a = m;
+      }
+      hi = a;
+    }
   } else {                                                 // query block blk: key blocks inside its window
     hi = blk;
     int klo = 0;
@@ -448,6 +459,112 @@ __global__ void __launch_bounds__(256) qkv_prep_bwd_kernel(const PrepBwdParams p
   }
 }
 
+// ---------------------------------------------------------------------------------------------
+// The same backward from what the fused projection leaves: the prepared rows y' and 1 / rms.  With y' = R xh (R the
+// rotation, orthogonal) the mean in the norm's backward is mean(g_y y') and
+//     g_x = R^T ( r (g_y - y' mean(g_y y')) )
+// so the raw projections need not be kept or read.  A gated v (v' = g vn + (1 - g) ve) takes vn in place of y' and g g_y in
+// place of g_y, and leaves d ve = (1 - g) g_y and the block's share of d g = sum g_y (vn - ve).  The three gradients go
+// straight into the merged [M, 3 H 128] matrix that the two projection gradients read.  HBM-bound: 3 x 256 bytes a row.
+struct PrepGradParams {
+  const __nv_bfloat16* y[3];      // q', k', and v' or vn: [M, H, 128]
+  const __nv_bfloat16* gy[3];     // their gradients (of v' where v is gated)
+  const float* rstd;              // [M, 3 H]
+  __nv_bfloat16* gx;              // [M, 3 H 128]
+  const float *cos, *sin;
+  const __nv_bfloat16* ve;        // [M, H, 128] or null
+  const float* gate_logit;
+  __nv_bfloat16* g_ve;            // [M, H, 128]
+  float* partial;                 // one per block of the v part
+  int M, T, H;
+};
+
+__global__ void __launch_bounds__(256) qkv_prep_grad_kernel(const PrepGradParams p) {
+  const int which = blockIdx.y;
+  const int64_t rows = (int64_t)p.M * p.H;
+  const int64_t r = ((int64_t)blockIdx.x * 256 + threadIdx.x) >> 3;
+  const int sub = threadIdx.x & 7;
+  const int64_t rc = r < rows ? r : rows - 1;
+  const int m = (int)(rc / p.H), h = (int)(rc - (int64_t)m * p.H);
+  float x1[8], x2[8], g1[8], g2[8];
+  const int64_t off = rc * DAISY_HEAD_DIM + 8 * sub;
+  unpack8(ld_stream16(p.y[which] + off), x1); unpack8(ld_stream16(p.y[which] + off + 64), x2);
+  unpack8(ld_stream16(p.gy[which] + off), g1); unpack8(ld_stream16(p.gy[which] + off + 64), g2);
+  const float rr = __ldg(p.rstd + ((int64_t)m * 3 + which) * p.H + h);
+  float share = 0.f;
+  if (which == 2 && p.ve) {
+    const float gate = 1.0f / (1.0f + __expf(-*p.gate_logit));
+    float e1[8], e2[8], d1[8], d2[8];
+    unpack8(ld_stream16(p.ve + off), e1); unpack8(ld_stream16(p.ve + off + 64), e2);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      share = fmaf(g1[e], x1[e] - e1[e], share); share = fmaf(g2[e], x2[e] - e2[e], share);
+      d1[e] = (1.0f - gate) * g1[e]; d2[e] = (1.0f - gate) * g2[e];
+      g1[e] *= gate; g2[e] *= gate;
+    }
+    if (r < rows) {
+      *reinterpret_cast<uint4*>(p.g_ve + off) = pack8(d1);
+      *reinterpret_cast<uint4*>(p.g_ve + off + 64) = pack8(d2);
+    } else {
+      share = 0.f;
+    }
+  }
+  float gd = 0.f;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) gd += g1[e] * x1[e] + g2[e] * x2[e];
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) gd += __shfl_xor_sync(0xffffffffu, gd, o);
+  const float mean = gd * (1.0f / DAISY_HEAD_DIM);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) { g1[e] = rr * (g1[e] - x1[e] * mean); g2[e] = rr * (g2[e] - x2[e] * mean); }
+  if (which < 2) {
+    const int t = m % p.T;
+    const float4* cr = reinterpret_cast<const float4*>(p.cos + (int64_t)t * 64 + 8 * sub);
+    const float4* sr = reinterpret_cast<const float4*>(p.sin + (int64_t)t * 64 + 8 * sub);
+    const float4 c0 = cr[0], c1 = cr[1], s0 = sr[0], s1 = sr[1];
+    const float c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w}, s[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float a = g1[e], b2 = g2[e];
+      g1[e] = a * c[e] - b2 * s[e];
+      g2[e] = a * s[e] + b2 * c[e];
+    }
+  }
+  if (r < rows) {
+    __nv_bfloat16* dst = p.gx + ((int64_t)m * 3 + which) * p.H * DAISY_HEAD_DIM + h * DAISY_HEAD_DIM + 8 * sub;
+    *reinterpret_cast<uint4*>(dst) = pack8(g1);
+    *reinterpret_cast<uint4*>(dst + 64) = pack8(g2);
+  }
+  if (which == 2 && p.ve) {
+    __shared__ float red[8];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) share += __shfl_xor_sync(0xffffffffu, share, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = share;
+    __syncthreads();
+    if (threadIdx.x == 0) p.partial[blockIdx.x] = ((red[0] + red[1]) + (red[2] + red[3])) + ((red[4] + red[5]) + (red[6] + red[7]));
+  }
+}
+
+// The gate's gradient from the blocks' shares, in a fixed order: d logit = g (1 - g) sum.
+__global__ void __launch_bounds__(1024) gate_grad_kernel(const float* partial, int n, const float* gate_logit, float* out) {
+  __shared__ float red[32];
+  float s = 0.f;
+  for (int i = threadIdx.x; i < n; i += 1024) s += partial[i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    s = red[threadIdx.x];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (threadIdx.x == 0) {
+      const float g = 1.0f / (1.0f + __expf(-*gate_logit));
+      *out = g * (1.0f - g) * s;
+    }
+  }
+}
+
 }  // namespace daisy
 
 using namespace daisy;
@@ -555,5 +672,33 @@ extern "C" int daisy_b200_qkv_prep_bwd(const void* q, const void* k, const void*
   dim3 grid((unsigned)((rows * 8 + 255) / 256), 3, 1);
   qkv_prep_bwd_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(p);
   DAISY_CHECK_LAUNCH();
+  return DAISY_OK;
+}
+
+extern "C" int64_t daisy_b200_qkv_prep_grad_blocks(int M, int H) { return M > 0 && H > 0 ? ((int64_t)M * H * 8 + 255) / 256 : 0; }
+
+extern "C" int daisy_b200_qkv_prep_grad(const void* q_p, const void* k_p, const void* v_n, const void* dq_p, const void* dk_p, const void* dv_p,
+                                        const float* rstd, const float* cos, const float* sin, void* dqkv,
+                                        const void* ve, const float* ve_gate_logit, void* d_ve, float* d_logit, float* partial,
+                                        int M, int T, int H, int D, void* stream) {
+  if (!q_p || !k_p || !v_n || !dq_p || !dk_p || !dv_p || !rstd || !cos || !sin || !dqkv || M <= 0 || T <= 0 || H <= 0) return DAISY_EINVAL;
+  if (D != DAISY_HEAD_DIM) return DAISY_EUNSUPPORTED;
+  if (ve && (!ve_gate_logit || !d_ve || !d_logit || !partial)) return DAISY_EINVAL;
+  const void* ptrs[] = {q_p, k_p, v_n, dq_p, dk_p, dv_p, cos, sin, dqkv, ve, d_ve};
+  for (const void* x : ptrs) if (!daisy_aligned16(x)) return DAISY_EALIGN;
+  if ((int64_t)M * H >= (int64_t)1 << 31) return DAISY_EUNSUPPORTED;
+  PrepGradParams p{};
+  p.y[0] = (const __nv_bfloat16*)q_p; p.y[1] = (const __nv_bfloat16*)k_p; p.y[2] = (const __nv_bfloat16*)v_n;
+  p.gy[0] = (const __nv_bfloat16*)dq_p; p.gy[1] = (const __nv_bfloat16*)dk_p; p.gy[2] = (const __nv_bfloat16*)dv_p;
+  p.rstd = rstd; p.gx = (__nv_bfloat16*)dqkv; p.cos = cos; p.sin = sin;
+  p.ve = (const __nv_bfloat16*)ve; p.gate_logit = ve_gate_logit; p.g_ve = (__nv_bfloat16*)d_ve; p.partial = partial;
+  p.M = M; p.T = T; p.H = H;
+  const int64_t blocks = daisy_b200_qkv_prep_grad_blocks(M, H);
+  qkv_prep_grad_kernel<<<dim3((unsigned)blocks, 3, 1), 256, 0, (cudaStream_t)stream>>>(p);
+  DAISY_CHECK_LAUNCH();
+  if (ve) {
+    gate_grad_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(partial, (int)blocks, ve_gate_logit, d_logit);
+    DAISY_CHECK_LAUNCH();
+  }
   return DAISY_OK;
 }

@@ -266,6 +266,107 @@ std::vector<Tensor> attn_layer(const Tensor& x_, const Tensor& qkvo_w, const Ten
   return {y, p[1], p[2], p[0]};
 }
 
+// ------------------------------------------------------------------ attention layer under autograd
+// Forward: the fused projection (which also leaves 1 / rms of every head row), attention with its log-sum-exp, output
+// projection.  Backward: two library products for each projection, the attention backward, and one row-wise pass that undoes
+// norms, RoPE and gate into the merged gradient matrix.  As F.linear calls around the attention core this took a copy of the
+// merged gradient (concatenation of three), zero fills and an addition for the two slices of the weight's gradient, a separate
+// norm / RoPE pass and its raw inputs.
+struct AttnFunction : public torch::autograd::Function<AttnFunction> {
+  static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& x, const Tensor& w, const OptTensor& ve, const OptTensor& logit, const Tensor& cos,
+                        const Tensor& sin, int64_t H, double eps, double scale, int64_t window, const OptTensor& doc_start, bool in_blocks) {
+    at::AutoDispatchBelowADInplaceOrView guard;
+    req(x, "x"); req(w, "qkvo_w");
+    const int64_t B = x.size(0), T = x.size(1), dim = w.size(2), M = B * T;
+    TORCH_CHECK_VALUE(w.dim() == 3 && w.size(0) == 4 && w.is_contiguous() && dim == H * 128 && x.size(2) == dim, "qkvo_w must be a contiguous [4, dim, dim]");
+    rope_table(cos, "cos"); rope_table(sin, "sin");
+    Tensor x2 = rows_of(x, dim);
+    auto q = at::empty({B, T, H, 128}, x.options()), k = at::empty_like(q), v = at::empty_like(q);
+    Tensor rstd = at::empty({M, 3 * H}, x.options().dtype(at::kFloat)), vn = v, ve2, g32;
+    if (ve.has_value()) {
+      req(*ve, "ve");
+      ve2 = ve->reshape({M, dim});
+      if (!ve2.is_contiguous()) ve2 = ve2.contiguous();
+      g32 = logit->to(at::kFloat).reshape({1});
+      vn = at::empty_like(q);
+    }
+    check(daisy_b200_qkv_gemm_train(x2.data_ptr(), x2.stride(0), w.data_ptr(), dim, cos.data_ptr<float>(), sin.data_ptr<float>(), q.data_ptr(), k.data_ptr(),
+                                    v.data_ptr(), rstd.data_ptr<float>(), ve2.defined() ? vn.data_ptr() : nullptr, ve2.defined() ? ve2.data_ptr() : nullptr,
+                                    ve2.defined() ? dim : 0, ve2.defined() ? g32.data_ptr<float>() : nullptr, (int)B, (int)T, (int)H, 128, (int)dim, (float)eps,
+                                    DAISY_QKV_DEFAULT, status_ptr(x), stream_of(x)),
+          "daisy_b200_qkv_gemm_train");
+    auto [o, lse] = swa_attend(q, k, v, window, scale, std::nullopt, true, doc_start, in_blocks, true);
+    Tensor y = gemm_nt(o.view({B, T, dim}), w.select(0, 3));
+    ctx->save_for_backward({x2, w, q, k, v, o, lse, rstd, cos, sin, ve2, g32, vn, doc_start.has_value() ? *doc_start : Tensor()});
+    ctx->saved_data["dims"] = std::vector<int64_t>{B, T, H, window, in_blocks ? 1 : 0};
+    ctx->saved_data["scale"] = scale;
+    if (ve.has_value()) {
+      ctx->saved_data["ve_shape"] = ve->sizes().vec();
+      ctx->saved_data["logit_shape"] = logit->sizes().vec();
+      ctx->saved_data["logit_type"] = (int64_t)logit->scalar_type();
+    }
+    return y;
+  }
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
+    at::AutoDispatchBelowADInplaceOrView guard;
+    auto s = ctx->get_saved_variables();
+    const Tensor &x2 = s[0], &w = s[1], &q = s[2], &k = s[3], &v = s[4], &o = s[5], &lse = s[6], &rstd = s[7], &cos = s[8], &sin = s[9], &ve2 = s[10], &g32 = s[11],
+                 &vn = s[12], &doc = s[13];
+    auto d = ctx->saved_data["dims"].toIntVector();
+    const int64_t B = d[0], T = d[1], H = d[2], window = d[3], dim = H * 128, M = B * T;
+    const float scale = (float)ctx->saved_data["scale"].toDouble();
+    const bool need_x = ctx->needs_input_grad(0), need_w = ctx->needs_input_grad(1);
+    Tensor dy = grads[0].to(at::kBFloat16).reshape({M, dim});
+    if (dy.stride(1) != 1) dy = dy.contiguous();
+    Tensor dw, dx;
+    if (need_w) {
+      dw = at::empty_like(w);
+      Tensor dwo = dw.select(0, 3);
+      at::mm_out(dwo, dy.t(), o.view({M, dim}));
+    }
+    Tensor d_o = at::mm(dy, w.select(0, 3)).view({B, T, H, 128});
+    auto dq = at::empty_like(q), dk = at::empty_like(q), dv = at::empty_like(q);
+    Tensor ws = at::empty({(int64_t)daisy_b200_swa_attend_bwd_workspace_bytes((int)B, (int)T, (int)H)}, q.options().dtype(at::kByte));
+    Doc dc = doc_arg(doc.defined() ? OptTensor(doc) : std::nullopt, B, T, q);
+    const int64_t sb = T * H * 128, st = H * 128, sh = 128;
+    check(daisy_b200_swa_attend_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), d_o.data_ptr(), sb, st, sh, sb, st, sh, sb, st, sh, sb, st, sh, sb, st, sh,
+                                    lse.data_ptr<float>(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), (int)B, (int)T, (int)H, 128, (int)window, scale, dc.ptr, dc.sb,
+                                    d[4] ? DAISY_WINDOW_BLOCKS : 0, ws.data_ptr(), (size_t)ws.numel(), status_ptr(q), stream_of(q)),
+          "daisy_b200_swa_attend_bwd");
+    Tensor dqkv = at::empty({M, 3 * dim}, q.options()), d_ve, d_logit, part;
+    if (ve2.defined()) {
+      d_ve = at::empty({M, dim}, q.options());
+      d_logit = at::empty({1}, q.options().dtype(at::kFloat));
+      part = at::empty({daisy_b200_qkv_prep_grad_blocks((int)M, (int)H)}, q.options().dtype(at::kFloat));
+    }
+    auto ptr = [](const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; };
+    check(daisy_b200_qkv_prep_grad(q.data_ptr(), k.data_ptr(), vn.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), rstd.data_ptr<float>(), cos.data_ptr<float>(),
+                                   sin.data_ptr<float>(), dqkv.data_ptr(), ptr(ve2), (const float*)ptr(g32), ptr(d_ve), (float*)ptr(d_logit), (float*)ptr(part), (int)M,
+                                   (int)T, (int)H, 128, stream_of(q)),
+          "daisy_b200_qkv_prep_grad");
+    const Tensor wqkv = w.narrow(0, 0, 3).view({3 * dim, dim});
+    if (need_w) {
+      Tensor dwq = dw.narrow(0, 0, 3).view({3 * dim, dim});
+      at::mm_out(dwq, dqkv.t(), x2);
+    }
+    if (need_x) dx = at::mm(dqkv, wqkv).view({B, T, dim});
+    torch::autograd::variable_list out(12);
+    out[0] = dx; out[1] = dw;
+    if (ve2.defined()) {
+      out[2] = d_ve.view(ctx->saved_data["ve_shape"].toIntVector());
+      out[3] = d_logit.to((at::ScalarType)ctx->saved_data["logit_type"].toInt()).view(ctx->saved_data["logit_shape"].toIntVector());
+    }
+    return out;
+  }
+};
+
+Tensor attn_train(const Tensor& x, const Tensor& w, const OptTensor& ve, const OptTensor& logit, const Tensor& cos, const Tensor& sin, int64_t H, double eps,
+                  double scale, int64_t window, const OptTensor& doc_start, bool in_blocks) {
+  TORCH_CHECK_VALUE(x.is_cuda(), "x must be a CUDA tensor (daisy_b200 has no CPU path)");
+  c10::cuda::CUDAGuard guard(x.device());
+  return AttnFunction::apply(x.scalar_type() == w.scalar_type() ? x : x.to(w.scalar_type()), w, ve, logit, cos, sin, H, eps, scale, window, doc_start, in_blocks);
+}
+
 // ------------------------------------------------------------------ Kimi layer, one token
 bool kda_token_supported(int64_t H) { return H >= 1 && daisy_b200_kda_token_workspace_bytes(1, (int)H, 128) != 0; }
 int64_t kda_token_workspace_bytes(int64_t B, int64_t H) { return (int64_t)daisy_b200_kda_token_workspace_bytes((int)std::min<int64_t>(B, 16), (int)H, 128); }
@@ -308,6 +409,194 @@ Tensor kda_token_step(const Tensor& x_, const std::vector<Tensor>& w, const OptT
   return y;
 }
 
+
+// ------------------------------------------------------------------ KDA
+Tensor f32c(const Tensor& t, const char* name) {
+  TORCH_CHECK_VALUE(t.is_cuda() && t.scalar_type() == at::kFloat && t.is_contiguous(), name, " must be a contiguous float32 CUDA tensor");
+  return t;
+}
+
+// Tables of a packed batch on the device (see kda_varlen_tables); tok only if asked for.
+struct Packed { Tensor chunks, ptr, tok; int64_t n_chunks = 0, n_seq = 0, total = 0; };
+Packed pack_tables(const py::object& cu_seqlens, c10::Device dev, int64_t chunk, bool want_tok) {
+  std::vector<int64_t> cu;
+  if (THPVariable_Check(cu_seqlens.ptr())) {
+    Tensor c = THPVariable_Unpack(cu_seqlens.ptr()).to(at::kCPU, at::kLong).contiguous();
+    cu.assign(c.data_ptr<int64_t>(), c.data_ptr<int64_t>() + c.numel());
+  } else {
+    for (auto item : cu_seqlens) cu.push_back(py::cast<int64_t>(py::int_(py::reinterpret_borrow<py::object>(item))));
+  }
+  bool ok = cu.size() >= 2 && cu[0] == 0;
+  for (size_t i = 1; ok && i < cu.size(); ++i) ok = cu[i] >= cu[i - 1];
+  TORCH_CHECK_VALUE(ok, "cu_seqlens must start at 0 and not decrease");
+  Packed p;
+  p.n_seq = (int64_t)cu.size() - 1;
+  p.total = cu.back();
+  for (int64_t n = 0; n < p.n_seq; ++n) p.n_chunks += (cu[n + 1] - cu[n] + chunk - 1) / chunk;
+  // one staging buffer, one copy: [n_chunks][2], [n_seq + 1] (padded to 8 bytes), [total][2]
+  const int64_t at_ptr = 2 * p.n_chunks, at_tok = at_ptr + (p.n_seq + 2) / 2 * 2, size = at_tok + (want_tok ? 2 * p.total : 0);
+  Tensor host = at::empty({std::max<int64_t>(size, 1)}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
+  int32_t* h = host.data_ptr<int32_t>();
+  int64_t c = 0;
+  for (int64_t n = 0; n < p.n_seq; ++n) {
+    h[at_ptr + n] = (int32_t)c;
+    for (int64_t t = cu[n]; t < cu[n + 1]; t += chunk, ++c) { h[2 * c] = (int32_t)t; h[2 * c + 1] = (int32_t)std::min(chunk, cu[n + 1] - t); }
+    if (want_tok)
+      for (int64_t t = cu[n]; t < cu[n + 1]; ++t) { h[at_tok + 2 * t] = (int32_t)cu[n]; h[at_tok + 2 * t + 1] = (int32_t)n; }
+  }
+  h[at_ptr + p.n_seq] = (int32_t)c;
+  for (int64_t i = at_ptr + p.n_seq + 1; i < at_tok; ++i) h[i] = 0;
+  Tensor d = host.to(dev, /*non_blocking=*/true);
+  p.chunks = d.narrow(0, 0, 2 * p.n_chunks).view({p.n_chunks, 2});
+  p.ptr = d.narrow(0, at_ptr, p.n_seq + 1);
+  if (want_tok) p.tok = d.narrow(0, at_tok, 2 * p.total).view({p.total, 2});
+  return p;
+}
+
+// chunked forward, dense ([B,T,H,K], packed == nullptr) or packed ([1,T_total,H,K])
+std::pair<Tensor, OptTensor> kda_chunk(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g_, const Tensor& beta_, std::optional<double> scale,
+                                       const OptTensor& h0_, bool want_state, bool l2norm, bool out_fp32, const Packed* pk) {
+  const Tensor* in[] = {&q, &k, &v};
+  const char* names[] = {"q", "k", "v"};
+  for (int i = 0; i < 3; ++i) { req(*in[i], names[i]); TORCH_CHECK_VALUE(in[i]->is_contiguous(), names[i], " must be contiguous"); }
+  TORCH_CHECK_VALUE(!pk || q.size(0) == 1, "packed sequences come as one row: q must be [1, T_total, H, K]");
+  Tensor g = f32c(g_, "g"), beta = f32c(beta_, "beta");
+  const int64_t B = q.size(0), T = q.size(1), H = q.size(2), K = q.size(3), V = v.size(3), n = pk ? pk->n_seq : B;
+  TORCH_CHECK_VALUE(!pk || pk->total == T, "cu_seqlens covers ", pk ? pk->total : 0, " tokens, the inputs hold ", T);
+  Tensor h0;
+  if (h0_.has_value()) {
+    h0 = f32c(*h0_, "initial_state");
+    TORCH_CHECK_VALUE(!pk || (h0.dim() == 4 && h0.size(0) == n && h0.size(1) == H && h0.size(2) == K && h0.size(3) == V), "initial_state must be [", n, ", ", H, ", ",
+                      K, ", ", V, "]");
+  }
+  Tensor o = at::empty({B, T, H, V}, q.options().dtype(out_fp32 ? at::kFloat : at::kBFloat16));
+  OptTensor hT;
+  if (want_state) hT = at::empty({n, H, K, V}, q.options().dtype(at::kFloat));
+  if (pk && (T == 0 || pk->n_chunks == 0)) {
+    if (want_state) { if (h0.defined()) hT->copy_(h0); else hT->zero_(); }
+    return {o, hT};
+  }
+  const int64_t need = pk ? (int64_t)daisy_b200_kda_varlen_workspace_bytes((int)pk->n_chunks, (int)H, (int)K, (int)V)
+                          : (int64_t)daisy_b200_kda_workspace_bytes((int)B, (int)T, (int)H, (int)K, (int)V);
+  Tensor ws = at::empty({std::max<int64_t>(need, 16)}, q.options().dtype(at::kByte));
+  const unsigned flags = (l2norm ? DAISY_KDA_L2NORM_QK : 0) | (out_fp32 ? DAISY_KDA_OUT_FP32 : 0);
+  const float sc = scale.has_value() ? (float)*scale : 0.f;
+  const float* h0p = h0.defined() ? h0.data_ptr<float>() : nullptr;
+  float* hTp = want_state ? hT->data_ptr<float>() : nullptr;
+  if (pk)
+    check(daisy_b200_kda_chunk_fwd_varlen(q.data_ptr(), k.data_ptr(), v.data_ptr(), g.data_ptr<float>(), beta.data_ptr<float>(), h0p, o.data_ptr(), hTp, (int)T, (int)H,
+                                          (int)K, (int)V, 64, sc, flags, pk->chunks.data_ptr<int32_t>(), (int)pk->n_chunks, pk->ptr.data_ptr<int32_t>(), (int)n,
+                                          ws.data_ptr(), (size_t)ws.numel(), status_ptr(q), stream_of(q)),
+          "daisy_b200_kda_chunk_fwd_varlen");
+  else
+    check(daisy_b200_kda_chunk_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), g.data_ptr<float>(), beta.data_ptr<float>(), h0p, o.data_ptr(), hTp, (int)B, (int)T, (int)H,
+                                   (int)K, (int)V, 64, sc, flags, ws.data_ptr(), (size_t)ws.numel(), status_ptr(q), stream_of(q)),
+          "daisy_b200_kda_chunk_fwd");
+  return {o, hT};
+}
+
+// token by token; with in_place the state handed in is updated and returned
+std::pair<Tensor, OptTensor> kda_recurrent(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g_, const Tensor& beta_, std::optional<double> scale,
+                                           const OptTensor& h0_, bool want_state, bool l2norm, bool out_fp32, bool in_place) {
+  const Tensor* in[] = {&q, &k, &v};
+  const char* names[] = {"q", "k", "v"};
+  for (int i = 0; i < 3; ++i) { req(*in[i], names[i]); TORCH_CHECK_VALUE(in[i]->is_contiguous(), names[i], " must be contiguous"); }
+  Tensor g = f32c(g_, "g"), beta = f32c(beta_, "beta");
+  const int64_t B = q.size(0), T = q.size(1), H = q.size(2), K = q.size(3), V = v.size(3);
+  Tensor h0;
+  if (h0_.has_value()) h0 = f32c(*h0_, in_place ? "an in-place state" : "initial_state");
+  TORCH_CHECK_VALUE(!in_place || h0.defined(), "state_in_place needs an initial_state");
+  Tensor o = at::empty({B, T, H, V}, q.options().dtype(out_fp32 ? at::kFloat : at::kBFloat16));
+  OptTensor hT;
+  if (in_place) hT = h0;
+  else if (want_state) hT = at::empty({B, H, K, V}, q.options().dtype(at::kFloat));
+  const unsigned flags = (l2norm ? DAISY_KDA_L2NORM_QK : 0) | (out_fp32 ? DAISY_KDA_OUT_FP32 : 0);
+  check(daisy_b200_kda_recurrent_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), g.data_ptr<float>(), beta.data_ptr<float>(), h0.defined() ? h0.data_ptr<float>() : nullptr,
+                                     o.data_ptr(), hT.has_value() ? hT->data_ptr<float>() : nullptr, (int)B, (int)T, (int)H, (int)K, (int)V,
+                                     scale.has_value() ? (float)*scale : 0.f, flags, stream_of(q)),
+        "daisy_b200_kda_recurrent_fwd");
+  return {o, hT};
+}
+
+constexpr int64_t RECURRENT_MAX_T = 4;           // up to this many tokens the state is carried token by token in registers
+
+// the layer's chunk_kda call: any float types, dense or packed
+std::pair<Tensor, OptTensor> chunk_kda(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& g_, const Tensor& beta_, std::optional<double> scale,
+                                       const OptTensor& h0_, bool want_state, bool l2norm, const py::object& cu_seqlens, bool out_fp32) {
+  Tensor q = q_.to(at::kBFloat16).contiguous(), k = k_.to(at::kBFloat16).contiguous(), v = v_.to(at::kBFloat16).contiguous();
+  Tensor g = g_.to(at::kFloat).contiguous(), beta = beta_.to(at::kFloat).contiguous();
+  OptTensor h0;
+  if (h0_.has_value()) h0 = h0_->to(at::kFloat).contiguous();
+  if (!cu_seqlens.is_none()) {
+    Packed p = pack_tables(cu_seqlens, q.device(), 64, false);
+    return kda_chunk(q, k, v, g, beta, scale, h0, want_state, l2norm, out_fp32, &p);
+  }
+  return q.size(1) <= RECURRENT_MAX_T ? kda_recurrent(q, k, v, g, beta, scale, h0, want_state, l2norm, out_fp32, false)
+                                      : kda_chunk(q, k, v, g, beta, scale, h0, want_state, l2norm, out_fp32, nullptr);
+}
+
+// ------------------------------------------------------------------ Kimi layer, whole sequences
+// F.linear on this library's GEMM where its tiles apply; the narrow ones (the per-head beta projection, few rows) go to torch's
+Tensor kimi_linear(const Tensor& x, const Tensor& w) {
+  const int64_t N = w.size(0), K = w.size(1);
+  if (x.numel() / K >= 64 && N % 128 == 0 && K % 64 == 0 && w.scalar_type() == at::kBFloat16 && x.scalar_type() == at::kBFloat16) return gemm_nt(x, w);
+  return at::linear(x, w);
+}
+
+// weights: q, k, v, f0, f1, g0, g1, b, o.  conv_s, rec: carried states or nothing.  -> y, final state, convolution states
+std::tuple<Tensor, OptTensor, std::vector<Tensor>> kimi_layer(const Tensor& x, const std::vector<Tensor>& w, const OptTensor& g1_bias, const OptTensor& norm_w,
+                                                              const std::vector<Tensor>& conv_w, const std::vector<OptTensor>& conv_b, const Tensor& a_log,
+                                                              const Tensor& dt_bias, const std::vector<OptTensor>& conv_s, const OptTensor& rec, bool use_cache,
+                                                              bool silu, double eps, int64_t H, const py::object& cu_seqlens) {
+  TORCH_CHECK_VALUE(x.is_cuda(), "x must be a CUDA tensor (daisy_b200 has no CPU path)");
+  c10::cuda::CUDAGuard guard(x.device());
+  const int64_t B = x.size(0), T = x.size(1), C = w[0].size(0), M = B * T;
+  Packed p;
+  const bool packed = !cu_seqlens.is_none();
+  if (packed) p = pack_tables(cu_seqlens, x.device(), 64, true);
+  const int64_t n = packed ? p.n_seq : B;
+  Tensor qkv[3];
+  std::vector<Tensor> out_s;
+  for (int i = 0; i < 3; ++i) {
+    Tensor xi = kimi_linear(x, w[i]), y = at::empty_like(xi);
+    const bool have = conv_s[i].has_value(), in_place = have && !packed && T <= 32;
+    const int64_t W = conv_w[i].numel() / C;
+    if (have)
+      TORCH_CHECK_VALUE(conv_s[i]->scalar_type() == at::kBFloat16 && conv_s[i]->is_contiguous() && conv_s[i]->numel() == n * C * W,
+                        "state must be a contiguous bf16 [", n, ", ", C, ", ", W, "] tensor");
+    Tensor so;
+    if (in_place) so = *conv_s[i];
+    else if (use_cache && packed) so = have ? conv_s[i]->clone() : at::zeros({n, C, W}, x.options());     // sequences without tokens keep their state
+    else if (use_cache) so = at::empty({n, C, W}, x.options());
+    const void *wp = conv_w[i].data_ptr(), *bp = conv_b[i].has_value() ? conv_b[i]->data_ptr() : nullptr, *sp = have ? conv_s[i]->data_ptr() : nullptr;
+    void* op = so.defined() ? so.data_ptr() : nullptr;
+    if (packed)
+      check(daisy_b200_kda_short_conv_varlen(xi.data_ptr(), C, wp, bp, sp, op, y.data_ptr(), C, (int)T, (int)C, (int)W, p.tok.data_ptr<int32_t>(),
+                                             silu ? DAISY_KDA_CONV_SILU : 0, stream_of(x)),
+            "daisy_b200_kda_short_conv_varlen");
+    else
+      check(daisy_b200_kda_short_conv(xi.data_ptr(), T * C, C, wp, bp, sp, op, y.data_ptr(), T * C, C, (int)B, (int)T, (int)C, (int)W, silu ? DAISY_KDA_CONV_SILU : 0,
+                                      stream_of(x)),
+            "daisy_b200_kda_short_conv");
+    qkv[i] = y.view({B, T, H, 128});
+    if (so.defined()) out_s.push_back(so);
+  }
+  Tensor f = kimi_linear(kimi_linear(x, w[3]), w[4]);
+  Tensor g = at::empty({B, T, H, 128}, x.options().dtype(at::kFloat));
+  check(daisy_b200_kda_gate(f.data_ptr(), 1, a_log.data_ptr<float>(), dt_bias.data_ptr<float>(), g.data_ptr<float>(), M, (int)H, 128, 1.f, 20.f,
+                            DAISY_KDA_GATE_ROUND_BF16, stream_of(x)),
+        "daisy_b200_kda_gate");
+  Tensor beta = at::linear(x, w[7]).sigmoid_().to(at::kFloat);
+  std::pair<Tensor, OptTensor> r = packed ? kda_chunk(qkv[0], qkv[1], qkv[2], g, beta, std::nullopt, rec, use_cache, true, false, &p)
+                                   : T <= RECURRENT_MAX_T ? kda_recurrent(qkv[0], qkv[1], qkv[2], g, beta, std::nullopt, rec, use_cache, true, false, rec.has_value())
+                                                          : kda_chunk(qkv[0], qkv[1], qkv[2], g, beta, std::nullopt, rec, use_cache, true, false, nullptr);
+  Tensor gp = kimi_linear(kimi_linear(x, w[5]), w[6]), o = r.first, yn = at::empty({B, T, C}, x.options());
+  check(daisy_b200_kda_out_norm(o.data_ptr(), 0, gp.data_ptr(), g1_bias.has_value() ? g1_bias->data_ptr() : nullptr, g1_bias.has_value() ? (int)H : 1,
+                                norm_w.has_value() ? norm_w->data_ptr() : nullptr, yn.data_ptr(), M * H, 128, (float)eps, 2, stream_of(x)),
+        "daisy_b200_kda_out_norm");
+  return {kimi_linear(yn, w[8]), r.second, out_s};
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -335,6 +624,24 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     return swa_attend(q, k, v, window, scale, out, bounded, doc_start, in_blocks, true);
   });
   m.def("attn_layer", &attn_layer);
+  m.def("attn_train", &attn_train);
+  m.def("kda_tables", [](const py::object& cu, const py::object& device, int64_t chunk) {
+    Packed p = pack_tables(cu, py::cast<c10::Device>(device), chunk, true);
+    return std::make_tuple(p.chunks, p.ptr, p.tok, p.n_chunks);
+  });
+  m.def("kda_chunk_fwd", [](const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& beta, std::optional<double> scale, const OptTensor& h0,
+                            bool want_state, bool l2norm, bool out_fp32) {
+    return kda_chunk(q, k, v, g, beta, scale, h0, want_state, l2norm, out_fp32, nullptr);
+  });
+  m.def("kda_chunk_fwd_varlen", [](const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& beta, const Tensor& chunks, const Tensor& ptr,
+                                   int64_t total, int64_t n_chunks, std::optional<double> scale, const OptTensor& h0, bool want_state, bool l2norm, bool out_fp32) {
+    Packed p;
+    p.chunks = chunks; p.ptr = ptr; p.n_chunks = n_chunks; p.n_seq = ptr.numel() - 1; p.total = total;
+    return kda_chunk(q, k, v, g, beta, scale, h0, want_state, l2norm, out_fp32, &p);
+  });
+  m.def("kda_recurrent_fwd", &kda_recurrent);
+  m.def("chunk_kda", &chunk_kda);
+  m.def("kimi_layer", &kimi_layer);
   m.def("kda_token_supported", &kda_token_supported);
   m.def("kda_token_workspace_bytes", &kda_token_workspace_bytes);
   m.def("kda_token_step", &kda_token_step);

@@ -32,19 +32,13 @@ RECURRENT_MAX_T = 4      # up to this many tokens the state is carried token by 
 def chunk_kda(q, k, v, g, beta, scale: Optional[float] = None, initial_state: Optional[torch.Tensor] = None,
               output_final_state: bool = False, use_qk_l2norm_in_kernel: bool = False, cu_seqlens=None,
               out_fp32: bool = False, varlen_tables=None):
-    q, k, v = (x.contiguous() if x.dtype == torch.bfloat16 else x.to(torch.bfloat16).contiguous() for x in (q, k, v))
-    g = g.float().contiguous()
-    beta = beta.float().contiguous()
-    if initial_state is not None:
-        initial_state = initial_state.float().contiguous()
-    if cu_seqlens is not None or varlen_tables is not None:
-        # packed sequences [1, T_total, ...]: states are per sequence, no chunk spans two of them
-        return ops.kda_chunk_fwd_varlen(q, k, v, g, beta, cu_seqlens, scale, initial_state, output_final_state,
-                                        l2norm_qk=use_qk_l2norm_in_kernel, out_fp32=out_fp32, tables=varlen_tables)
-    fwd = ops.kda_recurrent_fwd if q.shape[1] <= RECURRENT_MAX_T else ops.kda_chunk_fwd
-    o, hT = fwd(q, k, v, g, beta, scale, initial_state, output_final_state,
-                l2norm_qk=use_qk_l2norm_in_kernel, out_fp32=out_fp32)
-    return o, hT
+    if varlen_tables is None:
+        return ext().chunk_kda(q, k, v, g, beta, scale, initial_state, output_final_state, use_qk_l2norm_in_kernel, cu_seqlens, out_fp32)
+    # packed sequences [1, T_total, ...] with their tables at hand: states are per sequence, no chunk spans two of them
+    q, k, v = (x.to(torch.bfloat16).contiguous() for x in (q, k, v))
+    initial_state = None if initial_state is None else initial_state.float().contiguous()
+    return ops.kda_chunk_fwd_varlen(q, k, v, g.float().contiguous(), beta.float().contiguous(), cu_seqlens, scale, initial_state, output_final_state,
+                                    l2norm_qk=use_qk_l2norm_in_kernel, out_fp32=out_fp32, tables=varlen_tables)
 
 
 def get_unpad_data(attention_mask: torch.Tensor):
@@ -189,25 +183,31 @@ class B200KimiLinearSelfAttention(torch.nn.Module):
         """The decode step as one launch (``csrc/kda_token.cu``; 16 batch rows at a time), states updated in place; None
         where the layer or its states are not of the form that kernel takes."""
         rec, conv = self._recurrent_state, self._conv_state
-        if (rec is None or conv is None or x.shape[1] != 1 or not x.is_cuda or self.conv_size != 4 or self.head_dim != 128
-                or self.head_v_dim != 128 or self.hidden_size != self.key_dim or not ext().kda_token_supported(self.num_heads)
+        if (rec is None or conv is None or x.shape[1] != 1 or not x.is_cuda or self.hidden_size != self.key_dim
+                or self.head_dim != 128 or not ext().kda_token_supported(self.num_heads)
                 or rec.dtype != torch.float32 or rec.shape[0] != x.shape[0] or not rec.is_contiguous() or not rec.is_cuda
                 or any(c.dtype != torch.bfloat16 or not c.is_contiguous() for c in conv)):
             return None
+        a = self._native_args()
+        return None if a is None else ext().kda_token_step(x, *a, rec, list(conv), self.q_conv1d.activation is not None, 1e-6, out, workspace)
+
+    def _native_args(self):
+        """Parameters in the order the native calls take them, or None where the layer is not of their form (four-tap
+        convolutions of one activation, 128-wide heads, bf16 weights, fp32 gate parameters)."""
         m, p = self._modules, self._parameters
+        if not self.use_short_conv or self.conv_size != 4 or self.head_dim != 128 or self.head_v_dim != 128:
+            return None
         lin = lambda name: m[name]._parameters["weight"]
         seq = lambda name, i: m[name]._modules[i]._parameters["weight"]
         w = [lin("q_proj"), lin("k_proj"), lin("v_proj"), seq("f_proj", "0"), seq("f_proj", "1"), seq("g_proj", "0"), seq("g_proj", "1"),
              lin("b_proj"), lin("o_proj")]
         cv = [m["q_conv1d"], m["k_conv1d"], m["v_conv1d"]]
-        act = cv[0].activation
-        fp32 = (p["A_log"], p["dt_bias"])
-        if (any(t.dtype != torch.bfloat16 for t in w) or any(t.dtype != torch.float32 for t in fp32)
-                or any(c.activation != act or c._parameters["weight"].dtype != torch.bfloat16 for c in cv)):
+        act, gb, nw = cv[0].activation, m["g_proj"]._modules["1"]._parameters["bias"], m["o_norm"]._parameters["weight"]
+        bf = w + [c._parameters["weight"] for c in cv] + [gb, nw]
+        if (any(t.dtype != torch.bfloat16 or not t.is_contiguous() for t in bf) or p["A_log"].dtype != torch.float32 or p["dt_bias"].dtype != torch.float32
+                or any(c.activation != act for c in cv)):
             return None
-        return ext().kda_token_step(x, w, m["g_proj"]._modules["1"]._parameters["bias"], m["o_norm"]._parameters["weight"],
-                                    [c._parameters["weight"] for c in cv], [c._parameters["bias"] for c in cv], p["A_log"], p["dt_bias"],
-                                    rec, list(conv), act is not None, 1e-6, out, workspace)
+        return w, gb, nw, [c._parameters["weight"] for c in cv], [c._parameters["bias"] for c in cv], p["A_log"], p["dt_bias"]
 
     def _forward_core(self, x, ve, sa_lambdas, attn_mask, use_cache: bool):
         if torch.is_grad_enabled() and (x.requires_grad or any(p.requires_grad for p in self.parameters())):
@@ -226,11 +226,24 @@ class B200KimiLinearSelfAttention(torch.nn.Module):
             x = index_first_axis(x.reshape(B0 * T0, -1), indices).unsqueeze(0)
             if ve is not None:
                 ve = index_first_axis(ve.reshape(B0 * T0, -1), indices).unsqueeze(0)
-            tabs = ops.kda_varlen_tables(cu_seqlens, x.device)
             if x.shape[1] == 0:
                 return x.new_zeros(B0, T0, self.hidden_size)
         B, T, _ = x.shape
         H = self.num_heads
+        args = self._native_args() if x.dtype == torch.bfloat16 and (ve is None or sa_lambdas is None) else None
+        if args is not None:
+            cs = self._conv_state if (use_cache and self._conv_state is not None) else (None, None, None)
+            rec = self._recurrent_state if use_cache else None
+            if rec is not None:
+                rec = rec.float().contiguous()
+            y, rec, cs = ext().kimi_layer(x if x.is_contiguous() else x.contiguous(), *args, [None if c is None else c.to(torch.bfloat16) for c in cs], rec,
+                                          use_cache, self.q_conv1d.activation is not None, 1e-6, H, cu_seqlens if indices is not None else None)
+            if use_cache:
+                self._recurrent_state, self._conv_state = rec, tuple(cs)
+                self._seen += T0
+            return y if indices is None else pad_input(y.squeeze(0), indices, B0, T0)
+        if indices is not None:
+            tabs = ops.kda_varlen_tables(cu_seqlens, x.device)
         q, k, v = _linear(x, self.q_proj.weight), _linear(x, self.k_proj.weight), _linear(x, self.v_proj.weight)
         if self.use_short_conv:
             cs = self._conv_state if (use_cache and self._conv_state is not None) else (None, None, None)

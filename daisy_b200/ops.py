@@ -10,8 +10,7 @@ import torch
 
 from . import _lib
 from ._native import ext
-from ._lib import (NORM_Q, NORM_K, NORM_V, ROPE, QKV_DEFAULT, WRITE_RING, OUT_BTHD, KV_BHTD, Q_IN_KERNEL, KDA_L2NORM_QK,
-                   KDA_OUT_FP32)
+from ._lib import (NORM_Q, NORM_K, NORM_V, ROPE, QKV_DEFAULT, WRITE_RING, OUT_BTHD, KV_BHTD, Q_IN_KERNEL)
 
 ATTN_SCALE = 0.12            # reference models/daisy/attention.py:88
 
@@ -418,29 +417,7 @@ def kda_chunk_fwd(q, k, v, g, beta, scale: Optional[float] = None, initial_state
                   output_final_state: bool = False, l2norm_qk: bool = True, out_fp32: bool = False):
     """KDA chunked forward.  ``q,k [B,T,H,K]`` ``v [B,T,H,V]`` bf16; ``g [B,T,H,K]`` fp32 log-decay; ``beta
     [B,T,H]`` fp32; state ``[B,H,K,V]`` fp32.  Returns ``(o [B,T,H,V], final_state or None)``."""
-    for n, t in (("q", q), ("k", k), ("v", v)):
-        _req(t, n)
-        if not t.is_contiguous():
-            raise ValueError(f"{n} must be contiguous")
-    g, beta = _f32c(g, "g"), _f32c(beta, "beta")
-    B, T, H, K = q.shape
-    V = v.shape[-1]
-    L = _lib.lib()
-    o = torch.empty(B, T, H, V, dtype=torch.float32 if out_fp32 else torch.bfloat16, device=q.device)
-    hT = torch.empty(B, H, K, V, dtype=torch.float32, device=q.device) if output_final_state else None
-    if initial_state is not None:
-        initial_state = _f32c(initial_state, "initial_state")
-    need = L.daisy_b200_kda_workspace_bytes(B, T, H, K, V)
-    ws = torch.empty(max(need, 16), dtype=torch.uint8, device=q.device)
-    flags = (KDA_L2NORM_QK if l2norm_qk else 0) | (KDA_OUT_FP32 if out_fp32 else 0)
-    rc = L.daisy_b200_kda_chunk_fwd(
-        q.data_ptr(), k.data_ptr(), v.data_ptr(), g.data_ptr(), beta.data_ptr(),
-        initial_state.data_ptr() if initial_state is not None else None, o.data_ptr(),
-        hT.data_ptr() if hT is not None else None, B, T, H, K, V, 64,
-        float(scale) if scale is not None else 0.0, flags, ws.data_ptr(), ws.numel(),
-        status_word(q.device).data_ptr(), _stream(q))
-    _lib.check(rc, "daisy_b200_kda_chunk_fwd")
-    return o, hT
+    return ext().kda_chunk_fwd(q, k, v, g, beta, scale, initial_state, output_final_state, l2norm_qk, out_fp32)
 
 
 def kda_varlen_tables(cu_seqlens, device, chunk: int = 64):
@@ -449,16 +426,7 @@ def kda_varlen_tables(cu_seqlens, device, chunk: int = 64):
     ``(chunk_tab [n_chunks, 2], seq_ptr [N + 1], tok_tab [T_total, 2], n_chunks)`` as int32 device tensors: first token
     and length of every chunk, the first chunk of every sequence, and for every token its sequence's first token and
     number."""
-    cu = [int(c) for c in (cu_seqlens.tolist() if torch.is_tensor(cu_seqlens) else cu_seqlens)]
-    if len(cu) < 2 or cu[0] != 0 or any(b < a for a, b in zip(cu, cu[1:])):
-        raise ValueError("cu_seqlens must start at 0 and not decrease")
-    chunks, ptr, tok = [], [0], []
-    for n, (a, b) in enumerate(zip(cu, cu[1:])):
-        chunks.extend((t, min(chunk, b - t)) for t in range(a, b, chunk))
-        ptr.append(len(chunks))
-        tok.extend((a, n) for _ in range(b - a))
-    mk = lambda rows, w: torch.tensor(rows, dtype=torch.int32).reshape(-1, w).to(device)
-    return mk(chunks, 2), torch.tensor(ptr, dtype=torch.int32, device=device), mk(tok, 2), len(chunks)
+    return ext().kda_tables(cu_seqlens, torch.device(device), int(chunk))
 
 
 def kda_chunk_fwd_varlen(q, k, v, g, beta, cu_seqlens, scale: Optional[float] = None, initial_state=None,
@@ -466,41 +434,11 @@ def kda_chunk_fwd_varlen(q, k, v, g, beta, cu_seqlens, scale: Optional[float] = 
     """KDA chunked forward over packed sequences: ``q,k [1,T,H,K]``, ``v [1,T,H,V]`` bf16, ``g`` fp32, ``beta [1,T,H]``,
     ``cu_seqlens`` the N + 1 sequence offsets; state ``[N,H,K,V]`` fp32.  ``tables``: the result of
     :func:`kda_varlen_tables` when the caller already has it."""
-    for n, t in (("q", q), ("k", k), ("v", v)):
-        _req(t, n)
-        if not t.is_contiguous():
-            raise ValueError(f"{n} must be contiguous")
-    if q.shape[0] != 1:
-        raise ValueError("packed sequences come as one row: q must be [1, T_total, H, K]")
-    g, beta = _f32c(g, "g"), _f32c(beta, "beta")
-    _, T, H, K = q.shape
-    V = v.shape[-1]
-    chunk_tab, seq_ptr, _tok, n_chunks = tables if tables is not None else kda_varlen_tables(cu_seqlens, q.device)
-    N = seq_ptr.numel() - 1
-    if int(_tok.shape[0]) != T:
-        raise ValueError(f"cu_seqlens covers {int(_tok.shape[0])} tokens, the inputs hold {T}")
-    L = _lib.lib()
-    o = torch.empty(1, T, H, V, dtype=torch.float32 if out_fp32 else torch.bfloat16, device=q.device)
-    if initial_state is not None:
-        initial_state = _f32c(initial_state, "initial_state")
-        if tuple(initial_state.shape) != (N, H, K, V):
-            raise ValueError(f"initial_state must be [{N}, {H}, {K}, {V}]")
-    hT = torch.empty(N, H, K, V, dtype=torch.float32, device=q.device) if output_final_state else None
-    if T == 0 or n_chunks == 0:
-        if hT is not None:
-            hT.copy_(initial_state) if initial_state is not None else hT.zero_()
-        return o, hT
-    need = L.daisy_b200_kda_varlen_workspace_bytes(n_chunks, H, K, V)
-    ws = torch.empty(max(need, 16), dtype=torch.uint8, device=q.device)
-    flags = (KDA_L2NORM_QK if l2norm_qk else 0) | (KDA_OUT_FP32 if out_fp32 else 0)
-    rc = L.daisy_b200_kda_chunk_fwd_varlen(
-        q.data_ptr(), k.data_ptr(), v.data_ptr(), g.data_ptr(), beta.data_ptr(),
-        initial_state.data_ptr() if initial_state is not None else None, o.data_ptr(),
-        hT.data_ptr() if hT is not None else None, T, H, K, V, 64,
-        float(scale) if scale is not None else 0.0, flags, chunk_tab.data_ptr(), n_chunks, seq_ptr.data_ptr(), N,
-        ws.data_ptr(), ws.numel(), status_word(q.device).data_ptr(), _stream(q))
-    _lib.check(rc, "daisy_b200_kda_chunk_fwd_varlen")
-    return o, hT
+    if tables is None:
+        tables = kda_varlen_tables(cu_seqlens, q.device)
+    chunk_tab, seq_ptr, tok, n_chunks = tables
+    return ext().kda_chunk_fwd_varlen(q, k, v, g, beta, chunk_tab, seq_ptr, int(tok.shape[0]), n_chunks, scale, initial_state, output_final_state,
+                                      l2norm_qk, out_fp32)
 
 
 def kda_recurrent_fwd(q, k, v, g, beta, scale: Optional[float] = None, initial_state=None,
@@ -508,32 +446,7 @@ def kda_recurrent_fwd(q, k, v, g, beta, scale: Optional[float] = None, initial_s
                       state_in_place: bool = False):
     """KDA token-by-token recurrence (short inputs, decode steps); same arguments and layouts as
     :func:`kda_chunk_fwd`.  ``state_in_place=True`` updates ``initial_state`` itself and returns it."""
-    for n, t in (("q", q), ("k", k), ("v", v)):
-        _req(t, n)
-        if not t.is_contiguous():
-            raise ValueError(f"{n} must be contiguous")
-    g, beta = _f32c(g, "g"), _f32c(beta, "beta")
-    B, T, H, K = q.shape
-    V = v.shape[-1]
-    o = torch.empty(B, T, H, V, dtype=torch.float32 if out_fp32 else torch.bfloat16, device=q.device)
-    if initial_state is not None:
-        if state_in_place and not (initial_state.dtype == torch.float32 and initial_state.is_contiguous()):
-            raise ValueError("an in-place state must be a contiguous float32 tensor")
-        initial_state = _f32c(initial_state, "initial_state")
-    if state_in_place:
-        if initial_state is None:
-            raise ValueError("state_in_place needs an initial_state")
-        hT = initial_state
-    else:
-        hT = torch.empty(B, H, K, V, dtype=torch.float32, device=q.device) if output_final_state else None
-    flags = (KDA_L2NORM_QK if l2norm_qk else 0) | (KDA_OUT_FP32 if out_fp32 else 0)
-    rc = _lib.lib().daisy_b200_kda_recurrent_fwd(
-        q.data_ptr(), k.data_ptr(), v.data_ptr(), g.data_ptr(), beta.data_ptr(),
-        initial_state.data_ptr() if initial_state is not None else None, o.data_ptr(),
-        hT.data_ptr() if hT is not None else None, B, T, H, K, V,
-        float(scale) if scale is not None else 0.0, flags, _stream(q))
-    _lib.check(rc, "daisy_b200_kda_recurrent_fwd")
-    return o, hT
+    return ext().kda_recurrent_fwd(q, k, v, g, beta, scale, initial_state, output_final_state, l2norm_qk, out_fp32, state_in_place)
 
 
 def kda_gate(g: torch.Tensor, a_log: torch.Tensor, head_k_dim: int, g_bias: Optional[torch.Tensor] = None,

@@ -131,6 +131,15 @@ int daisy_b200_qkv_gemm_ring(const void* x, int64_t ldx, const void* w_qkv, int6
                              int B, int T, int H, int D, int dim, float eps, unsigned flags,
                              int* status_word, void* stream);
 
+/* The same projection for a training step: every norm and RoPE applied, and also rstd [B T, 3 H] (1 / rms of each head row,
+ * what the norms' backward needs) and, with a value embedding, vn_out [B,T,H,D], v as normalised before the gate. */
+int daisy_b200_qkv_gemm_train(const void* x, int64_t ldx, const void* w_qkv, int64_t ldw,
+                              const float* cos, const float* sin,
+                              void* q_out, void* k_out, void* v_out, float* rstd, void* vn_out,
+                              const void* ve, int64_t ve_ld, const float* ve_gate_logit,
+                              int B, int T, int H, int D, int dim, float eps, unsigned flags,
+                              int* status_word, void* stream);
+
 /* C[M,N] = X[M,K] W[N,K]^T, bf16 in and out, fp32 accumulation: F.linear(y, qkvo_w[3]), the output projection
  * (models/daisy/attention.py:149).  K a multiple of 64, N a multiple of 128; ld* are row strides in elements. */
 int daisy_b200_gemm_nt(const void* x, int64_t ldx, const void* w, int64_t ldw, void* c, int64_t ldc,
@@ -457,6 +466,17 @@ int daisy_b200_kda_out_norm(const void* o, int o_is_fp32, const void* gate, cons
  */
 int daisy_b200_selftest_umma(const void* a, const void* b, float* c, int K, int mode,
                              int* status_word, void* stream);
+
+/* Gradients of the projections from those of the prepared rows (backward of the norms, RoPE and the value-embedding gate of
+ * models/daisy/attention.py:120-135), from what daisy_b200_qkv_gemm_train left: q_p, k_p and v_n (v', or vn where v is
+ * gated) [M,H,128], their gradients (dv_p: of v'), rstd -> dqkv [M, 3 H 128], rows q, k, v as the merged projection orders
+ * them.  With ve: d_ve [M,H,128] and *d_logit, the gate parameter's gradient; partial holds
+ * daisy_b200_qkv_prep_grad_blocks(M, H) floats.  No atomics: the same bits every run. */
+int64_t daisy_b200_qkv_prep_grad_blocks(int M, int H);
+int daisy_b200_qkv_prep_grad(const void* q_p, const void* k_p, const void* v_n, const void* dq_p, const void* dk_p, const void* dv_p,
+                             const float* rstd, const float* cos, const float* sin, void* dqkv,
+                             const void* ve, const float* ve_gate_logit, void* d_ve, float* d_logit, float* partial,
+                             int M, int T, int H, int D, void* stream);
 
 /* One decoded token through a Kimi-delta-attention layer in one launch (KimiLinearSelfAttention.step,
  * models/daisy/attention_kimi.py:128-211): projections, short convolutions (four taps, SiLU with DAISY_KDA_CONV_SILU), decay

@@ -28,31 +28,36 @@ namespace daisy {
 
 constexpr int KC = 64;                 // chunk length
 constexpr int KD = 128;                // K = V
-constexpr int LDT = 72;                // padded row (halves) of a [. x 64] image
-constexpr int IMG_T = KD * LDT * 2;    // one [128][72] fp16 image: 18432 bytes
-// per-chunk record in the workspace (bytes)
-constexpr int OFF_WT = 0;                              // W^T      [128][72] fp16
-constexpr int OFF_QT = OFF_WT + IMG_T;                 // q~^T     [128][72] fp16   (scale q e^G)^T
-constexpr int OFF_KT = OFF_QT + IMG_T;                 // k~^T     [128][72] fp16   (k e^{G_C-G})^T
-constexpr int OFF_AQK = OFF_KT + IMG_T;                // A_qk     [64][72]  fp16
-constexpr int OFF_D = OFF_AQK + KC * LDT * 2;          // e^{G_C}  [128]     fp32
-constexpr int SHARED_BYTES = OFF_D + KD * 4;           // 65024: identical for every V-slice
-constexpr int OFF_UT = SHARED_BYTES;                   // U0^T     [128][72] fp16
-constexpr int REC_BYTES = OFF_UT + IMG_T;              // 83456
+// per-chunk record in the workspace (bytes); every image is laid out so that ldmatrix reads it without bank conflicts after
+// a plain bulk copy (rec_off, ki_off)
+constexpr int OFF_WT = 0;                              // W^T      [128 channels][64 tokens] fp16
+constexpr int OFF_QT = OFF_WT + KD * KC * 2;           // q~       [64 tokens][128 channels] fp16   scale q e^G
+constexpr int OFF_KT = OFF_QT + KD * KC * 2;           // k~       [64 tokens][128 channels] fp16   k e^{G_C-G}
+constexpr int OFF_AQK = OFF_KT + KD * KC * 2;          // A_qk     [64][64]  fp16
+constexpr int OFF_D = OFF_AQK + KC * KC * 2;           // e^{G_C}  [128]     fp32
+constexpr int SHARED_BYTES = OFF_D + KD * 4;           // 57856: identical for every V-slice
+constexpr int OFF_UT = SHARED_BYTES;                   // U0^T     [128 value columns][64 tokens] fp16
+constexpr int REC_BYTES = OFF_UT + KD * KC * 2;        // 74240
 static_assert(SHARED_BYTES % 16 == 0 && REC_BYTES % 16 == 0, "bulk copies move 16-byte units");
+
+// byte offset of (row, token column) in an image of 64-token rows (128 bytes, 16-byte pieces exchanged by row)
+__device__ __forceinline__ uint32_t rec_off(int row, int col) { return (uint32_t)(row * 128 + (((col >> 3) ^ (row & 7)) << 4) + (col & 7) * 2); }
+// byte offset of 16-byte piece c (0..15) of a row in an image of 128-channel rows: the eight lanes that store two half rows,
+// and the eight rows of a (transposing) ldmatrix, all hit different banks
+__device__ __forceinline__ uint32_t ki_off(int row, int c) { return (uint32_t)(row * 256 + ((c ^ (((row & 1) << 2) | ((row >> 1) & 3))) << 4)); }
 
 // Four 8x8 fp16 matrices from shared memory: lanes 8m..8m+7 give the row addresses of matrix m (16 bytes per
 // row); register m of lane l then holds elements (row l/4, columns 2(l%4), 2(l%4)+1) of matrix m -- the B
 // fragment layout of mma.m16n8k16 when the rows are the n index and the columns the k index.
-__device__ __forceinline__ void ldmatrix_x4(uint32_t* r, const void* row_ptr) {
+__device__ __forceinline__ void ldmatrix_x4(uint32_t* r, uint32_t row_addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(row_ptr)));
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(row_addr));
 }
 // The transposing form: register m of lane l holds elements (rows 2(l%4), 2(l%4)+1, column l/4) of matrix m --
 // the same B fragment when the stored rows are the k index and the columns the n index.
-__device__ __forceinline__ void ldmatrix_x4_t(uint32_t* r, const void* row_ptr) {
+__device__ __forceinline__ void ldmatrix_x4_t(uint32_t* r, uint32_t row_addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(row_ptr)));
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(row_addr));
 }
 
 __device__ __forceinline__ void mma_f16(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
@@ -82,532 +87,399 @@ __device__ __forceinline__ void st_global16(void* p, uint32_t a, uint32_t b, uin
 //
 // Gated Gram matrices without a single positive exponent.  e^{G_i - G_j} (i > j) is needed per channel inside the
 // contraction over channels, so it must factor into a row term times a column term, and neither term may overflow
-// whatever the gates are.  Pairs are split by the highest bit in which i and j differ ("level" s = 1, 2, .., 32):
-// tokens fall into aligned groups of 2s, i lies in the upper half of its group, j in the lower half.  With r the
-// last row of the lower half,  e^{G_i - G_j} = e^{G_i - G_r} * e^{G_r - G_j}:  the row factor is the product of the
-// per-token decays d_t = e^{g_t} <= 1 from the start of the upper half up to i, the column factor their product from
-// j + 1 to the end of the lower half.  Every factor is a running product of numbers <= 1 -- ONE exponential per
-// input element, no cumulative sum, and underflow is the correct limit.  A level is then one plain product
-//      [ k * f ; q * f ]  (128 x 128 channels)   x   (k * f)^T  (128 channels x 64)      f = the level's factor per token
-// whose entries at (i upper, j lower, same group) are that level's Gram entries (everything else is ignored): six
-// 128 x 64 x 128 tcgen05 products per chunk with fp16 operand images staged in shared memory and fp32
-// accumulators in TMEM.  The prefix / suffix products are carried from one level to the next with one multiply per
-// element; after the last level they are e^{G} and e^{G_C - G}, the decay factors of the state-pass operands.
+// whatever the gates are.
+//   * Between different 16-token blocks I > J:  e^{G_i - G_j} = e^{G_i - G_{end J}} e^{G_{end J} - G_j}: the column term is
+//     the product of the decays d_t = e^{g_t} <= 1 behind j inside its block (`suf`), the row term the product up to i
+//     inside its block (`pre`) times the totals of the blocks between.
+//   * Inside a block, pairs are split by the highest bit in which i and j differ ("level" s = 1, 2, 4, 8): i lies in the
+//     upper, j in the lower half of an aligned group of 2s tokens, and the same identity holds with the group's middle.
+// Every factor is a running product of numbers <= 1 -- ONE exponential per input element, no cumulative sum, and underflow
+// is the correct limit.
+//
+// A CTA of four warps owns one (batch, head, chunk), warp w the tokens 16 w .. 16 w + 15, three CTAs to an SM.  A lane
+// holds rows g8 and g8 + 8 of its block and 32 of the 128 channels (four runs of eight: 16-byte loads) -- as m16n8k16
+// fragments with the channels in an order of our own, which a contraction over channels does not notice.  In that form the
+// A and the B operand of a Gram product are the same registers, so the in-block levels need no shared memory at all: k and
+// q rows of an octet are stacked into one A operand, and a level costs two products per 16 channels.  Blocks meet only
+// through their `suf` images (stored and read back register by register) and their totals.
+// Then the four diagonal blocks of I + A_kk are inverted (fp32, one per warp) and W, U0 come from a blocked forward
+// substitution on the transposed systems, a warp owning 64 of the 256 rows (see below).
+// Why not tcgen05: the version of this kernel that built six image sets in shared memory for 128 x 64 x 128 tcgen05 products
+// was a chain of hand-offs between warp groups (image -> fence -> product -> TMEM load), 20k cycles a chunk with the tensor
+// pipe at 10 %; here everything between two barriers stays in one warp's registers and three CTAs hide each other's latency.
 struct KdaIntraParams {
-  const float* beta;
+  const __nv_bfloat16 *q, *k, *v;
+  const float *g, *beta;
   uint8_t* ws;
   int T, H, NC;            // NC = chunks per sequence
-  int total;               // work items: B * H * NC
   float scale;
   int l2norm;
-  int* status;
   // packed variable-length sequences (B = 1): chunk c of the packed row covers tokens chunk_tab[2c] .. + chunk_tab[2c+1]
   // (1..64 of them; chunks never straddle a sequence boundary); null: chunk c covers tokens 64 c ..
   const int* chunk_tab;
 };
 
-constexpr int KI_ELEM_WARPS = 16, KI_SOLVER_WARPS = 8;
-constexpr int KI_ELEM_THREADS = 32 * KI_ELEM_WARPS;                         // 512
-constexpr int KI_SOLVER_THREADS = 32 * KI_SOLVER_WARPS;                     // 256
-// 24 warps = 6 per scheduler: 80 registers per thread
-constexpr int KI_THREADS = KI_ELEM_THREADS + KI_SOLVER_THREADS;             // 768
-constexpr int KI_IMG_BYTES = KD * KC * 2;                                   // one [128 channels][64 tokens] fp16 image: 16384
-constexpr int KI_IN_BYTES = KC * KD * 4 + 2 * KC * KD * 2;                  // g + q + k tiles: 65536
-constexpr int LDAKH = 72;
-constexpr int KI_SETS = 2;              // operand image sets in flight; divides the six levels of a chunk
-
-struct __align__(1024) KdaIntraSmem {
-  uint8_t img[KI_SETS][2 * KI_IMG_BYTES];   // level operand images, a ring of sets of (k image, q image); 128-byte swizzle
-  float g[KC][KD];                       // TMA destinations, plain rows
-  __nv_bfloat16 q[KC][KD];
-  __nv_bfloat16 k[KC][KD];
-  __nv_bfloat16 v[KC][KD];
-  __half xt[KD][LDT];                    // (k e^G)^T, fp16: right-hand side of the W solve
-  float akk_t[4][16][16];                // beta * A_kk, the four diagonal 16 x 16 blocks in fp32, column-major ([j][i])
-  __half akh[KC][LDAKH];                 //              the whole lower triangle as fp16 operands
-  __half th[KC][LDT];                    // the inverses of the diagonal blocks of I + A_kk, row-major, fp16
-  float tot[4][KD];                      // product of the decays of each 16-token segment
-  float rq[2][KC], rk[2][KC], beta[2][KC], qkd[2][KC];   // per-token scalars, double-buffered by chunk parity
-  float sbeta[KC];                       // the solver's own copy
-  uint64_t in_full, v_full, x_full, x_empty;
-  uint64_t img_full[KI_SETS], img_empty[KI_SETS], d_full[6], d_empty[6];
-  uint32_t tmem_base;
-  int abort_flag;
+constexpr int KI_THREADS = 128;
+constexpr int LDAK = 72;                                // halves per row of the A_kk image
+struct KdaIntraSmem {
+  // each block's images, register by register: [block][half run, octet][lane].  pk and pq (k pre, q pre) are read by their own
+  // warp only, which then lays k e^G and its v rows over them: token-major, swizzled rows of 256 bytes, block w in [w]
+  uint2 suf[4][16][32];
+  uint2 pk[4][16][32];
+  uint2 pq[4][16][32];
+  __half akh[KC][LDAK];                                 // beta A_kk below the diagonal blocks
+  float dg[4][16][20];                                  // beta A_kk, the diagonal blocks, column-major ([j][i])
+  __half th[4][16][24];                                 // their inverses (of I + A_kk), row-major
+  float tot[4][KD];                                     // product of the decays of each block, in the lanes' channel order
+  float beta[KC];
 };
-static_assert(sizeof(KdaIntraSmem) + 1024 <= 232448, "over the 227 KB a CTA may use");
 
-// byte offset of (row, 16-byte chunk) inside a 128-byte-swizzled image whose rows are 128 bytes
-__device__ __forceinline__ uint32_t sw128(int row, int chunk) {
-  return (uint32_t)((row >> 3) * 1024 + (row & 7) * 128 + (((chunk ^ row) & 7) << 4));
-}
-
-__device__ __forceinline__ void ki_coords(int w, int NC, int H, int& b, int& h, int& chunk) {
-  chunk = w % NC;
-  const int bh = w / NC;
-  h = bh % H;
-  b = bh / H;
-}
-// first token and number of tokens of a chunk
 __device__ __forceinline__ void ki_chunk_span(const int* chunk_tab, int chunk, int T, int& t0, int& rows) {
   if (chunk_tab) { t0 = chunk_tab[2 * chunk]; rows = chunk_tab[2 * chunk + 1]; }
   else { t0 = chunk * KC; rows = min(KC, T - t0); }
 }
-
 __device__ __forceinline__ uint32_t hmul2_u32(uint32_t a, uint32_t b) {
   uint32_t d;
   asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
   return d;
 }
+__device__ __forceinline__ uint4 ld_nc16(const void* p) {
+  uint4 r;
+  asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
+  return r;
+}
 
-// One level's operand images (this thread's 16 tokens of channel c; kn / qn hold them as fp16 pairs) into the image
-// set of the level's turn, then -- one warp per level, so that no warp falls far behind the others -- the level's
-// Gram product once every element thread has delivered its share.
-__device__ __forceinline__ void ki_emit_level(KdaIntraSmem& sm, const float (&f)[16], const uint32_t (&kn)[8], const uint32_t (&qn)[8],
-                                              const bool write_q, const int c, const int seg, const int warp, const uint32_t leader,
-                                              const uint32_t ci, uint32_t& n_img, bool& ok, const uint32_t tmem_base,
-                                              const uint32_t g_lo0, const uint32_t g_hi, volatile int* abort_flag, int* status) {
-  constexpr uint32_t idesc_g = umma_idesc_f16(128, KC, 1, 1);                   // A and B both token-contiguous (MN-major)
-  const uint32_t set = n_img % KI_SETS, use = n_img / KI_SETS;
-  uint32_t fh[8];
+__device__ __forceinline__ uint2 ld_nc8(const void* p) {
+  uint2 r;
+  asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(r.x), "=r"(r.y) : "l"(p));
+  return r;
+}
+__device__ __forceinline__ float4 ki_mul4(const float4 a, const float* b) {
+  const float4 c = *reinterpret_cast<const float4*>(b);
+  return make_float4(a.x * c.x, a.y * c.y, a.z * c.z, a.w * c.w);
+}
+// four fp16 values times fp32 factors, one rounding
+__device__ __forceinline__ uint2 ki_scale(const uint2 a, const float4 f) {
+  const float2 lo = unpack_h2(a.x), hi = unpack_h2(a.y);
+  return make_uint2(pack_h2(lo.x * f.x, lo.y * f.y), pack_h2(hi.x * f.z, hi.y * f.w));
+}
+
+__global__ void __launch_bounds__(KI_THREADS, 3) kda_intra_kernel(const KdaIntraParams p) {
+  extern __shared__ __align__(128) uint8_t kda_smem_raw[];
+  KdaIntraSmem& sm = *reinterpret_cast<KdaIntraSmem*>(kda_smem_raw);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g8 = lane >> 2, t4 = lane & 3;
+  const int chunk = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  int t0, rows;
+  ki_chunk_span(p.chunk_tab, chunk, p.T, t0, rows);
+  uint8_t* rec = p.ws + ((size_t)(b * p.H + h) * p.NC + chunk) * REC_BYTES;
+  const size_t tok = ((size_t)b * p.T + t0) * p.H + h, ts = (size_t)p.H * KD;      // row of token i: tok * KD + i * ts
+
+  if (tid < KC) sm.beta[tid] = tid < rows ? p.beta[tok + (size_t)tid * p.H] : 0.f;
+  for (int i = tid; i < 2 * rows; i += KI_THREADS)                                 // v is needed last: ask L2 for it now
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(p.v + tok * KD + (size_t)(i >> 1) * ts + 64 * (i & 1)));
+  const int r0 = 16 * warp + g8, r1 = r0 + 8;                                      // this lane's two tokens
+  const bool ok0 = r0 < rows, ok1 = r1 < rows;
+  const size_t o0 = tok * KD + (size_t)(ok0 ? r0 : 0) * ts + 8 * t4, o1 = tok * KD + (size_t)(ok1 ? r1 : 0) * ts + 8 * t4;
+
+  // A lane's channels: runs 32 m + 8 t4 .. + 7 (m = 0 .. 3) of rows r0, r1, taken in halves of four.  q and k are read twice,
+  // the second time from L2: first for the norms, then with g, run by run (kept, they and the level sums do not fit the
+  // 168 registers that three CTAs leave a thread).
+  float gv[2][4];                                                                  // the next half run: log-decays,
+  uint2 kv[2], qv[2];                                                              // k and q
+  auto load = [&](int x) {
+    const int c = 32 * (x >> 1) + 4 * (x & 1);
+    *reinterpret_cast<uint4*>(gv[0]) = ok0 ? ld_nc16(p.g + o0 + c) : make_uint4(0, 0, 0, 0);
+    *reinterpret_cast<uint4*>(gv[1]) = ok1 ? ld_nc16(p.g + o1 + c) : make_uint4(0, 0, 0, 0);
+    kv[0] = ok0 ? ld_nc8(p.k + o0 + c) : make_uint2(0, 0); kv[1] = ok1 ? ld_nc8(p.k + o1 + c) : make_uint2(0, 0);
+    qv[0] = ok0 ? ld_nc8(p.q + o0 + c) : make_uint2(0, 0); qv[1] = ok1 ? ld_nc8(p.q + o1 + c) : make_uint2(0, 0);
+  };
+  float qkd[2], rq[2], rk[2];                                                      // normalised q . k, and 1 / |q|, 1 / |k|, of the two tokens
+  {
+    float sq[2] = {0.f, 0.f}, sk[2] = {0.f, 0.f}, dd[2] = {0.f, 0.f};
+    uint32_t kr[4][2][4], qr[4][2][4];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) fh[i] = pack_h2(f[2 * i], f[2 * i + 1]);
-  if (use >= 1) ok = mbar_wait_long(&sm.img_empty[set], (use - 1) & 1, abort_flag, status, 2) && ok;
-  uint8_t* kimg = sm.img[set];
-#pragma unroll
-  for (int e = 0; e < 2; ++e) {
-    const uint32_t off = sw128(c, 2 * seg + e);
-    *reinterpret_cast<uint4*>(kimg + off) = make_uint4(hmul2_u32(kn[4 * e], fh[4 * e]), hmul2_u32(kn[4 * e + 1], fh[4 * e + 1]),
-                                                       hmul2_u32(kn[4 * e + 2], fh[4 * e + 2]), hmul2_u32(kn[4 * e + 3], fh[4 * e + 3]));
-    if (write_q)
-      *reinterpret_cast<uint4*>(kimg + KI_IMG_BYTES + off) = make_uint4(hmul2_u32(qn[4 * e], fh[4 * e]), hmul2_u32(qn[4 * e + 1], fh[4 * e + 1]),
-                                                                        hmul2_u32(qn[4 * e + 2], fh[4 * e + 2]), hmul2_u32(qn[4 * e + 3], fh[4 * e + 3]));
-  }
-  fence_proxy_async();
-  mbar_arrive(&sm.img_full[set]);
-  const int li = (int)(n_img % 6u);
-  if (warp == li) {                                                             // level li's product is issued by element warp li
-    ok = mbar_wait_long(&sm.img_full[set], use & 1, abort_flag, status, 4) && ok;
-    if (ci >= 1) ok = mbar_wait_long(&sm.d_empty[li], (ci - 1) & 1, abort_flag, status, 5) && ok;
-    ok = __all_sync(0xffffffffu, ok);
-    if (ok) {
-      tc_fence_after();
-      const uint32_t lo = g_lo0 + set * ((2 * KI_IMG_BYTES) >> 4);
-#pragma unroll
-      for (int ks = 0; ks < KD / 16; ++ks)                                      // 16 channels = 16 rows of 128 bytes per step
-        umma_ss_lh_p(leader, tmem_base + 64 * li, lo + ks * (2048 >> 4), g_hi, lo + ks * (2048 >> 4), g_hi, idesc_g, ks > 0 ? 1u : 0u);
+    for (int m = 0; m < 4; ++m) {
+      *reinterpret_cast<uint4*>(kr[m][0]) = ok0 ? ld_nc16(p.k + o0 + 32 * m) : make_uint4(0, 0, 0, 0);
+      *reinterpret_cast<uint4*>(kr[m][1]) = ok1 ? ld_nc16(p.k + o1 + 32 * m) : make_uint4(0, 0, 0, 0);
+      *reinterpret_cast<uint4*>(qr[m][0]) = ok0 ? ld_nc16(p.q + o0 + 32 * m) : make_uint4(0, 0, 0, 0);
+      *reinterpret_cast<uint4*>(qr[m][1]) = ok1 ? ld_nc16(p.q + o1 + 32 * m) : make_uint4(0, 0, 0, 0);
     }
-    tc_commit_p(leader, &sm.img_empty[set]);                                    // arrives at once when nothing was issued
-    tc_commit_p(leader, &sm.d_full[li]);
-  }
-  ++n_img;
-}
-
-// Level S < 16: the factor of token i is pre[i] if bit S of i is set, else suf[i]; afterwards both products are carried
-// from aligned blocks of S to blocks of 2 S (upper block: prefix times the lower block's total; lower block: suffix
-// times the upper block's total).
-template <int S, typename Emit>
-__device__ __forceinline__ void ki_level_inreg(float (&pre)[16], float (&suf)[16], Emit& emit) {
-  float f[16];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) f[i] = (i & S) ? pre[i] : suf[i];
-  emit(f, true);
+    for (int m = 0; m < 4; ++m)
 #pragma unroll
-  for (int a = 0; a < 16; a += 2 * S) {
-    const float tot_l = pre[a + S - 1], tot_u = pre[a + 2 * S - 1];
+      for (int u = 0; u < 2; ++u)
 #pragma unroll
-    for (int i = 0; i < S; ++i) { pre[a + S + i] *= tot_l; suf[a + i] *= tot_u; }
+        for (int j = 0; j < 4; ++j) {
+          const float k0 = bf16_lo(kr[m][u][j]), k1 = bf16_hi(kr[m][u][j]), q0 = bf16_lo(qr[m][u][j]), q1 = bf16_hi(qr[m][u][j]);
+          sk[u] = fmaf(k0, k0, sk[u]); sk[u] = fmaf(k1, k1, sk[u]);
+          sq[u] = fmaf(q0, q0, sq[u]); sq[u] = fmaf(q1, q1, sq[u]);
+          dd[u] = fmaf(q0, k0, dd[u]); dd[u] = fmaf(q1, k1, dd[u]);
+        }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+#pragma unroll
+      for (int o = 1; o <= 2; o <<= 1) {
+        sq[u] += __shfl_xor_sync(0xffffffffu, sq[u], o);
+        sk[u] += __shfl_xor_sync(0xffffffffu, sk[u], o);
+        dd[u] += __shfl_xor_sync(0xffffffffu, dd[u], o);
+      }
+      rq[u] = p.l2norm ? rsqrtf(sq[u] + 1e-6f) : 1.f;
+      rk[u] = p.l2norm ? rsqrtf(sk[u] + 1e-6f) : 1.f;
+      qkd[u] = rq[u] * rk[u] * dd[u];
+    }
   }
-}
 
-__global__ void __launch_bounds__(KI_THREADS, 1)
-kda_intra_kernel(const __grid_constant__ CUtensorMap tm_g, const __grid_constant__ CUtensorMap tm_q,
-                 const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
-                 const KdaIntraParams p) {
-  extern __shared__ uint8_t kda_smem_raw[];
-  KdaIntraSmem& sm = *reinterpret_cast<KdaIntraSmem*>((reinterpret_cast<uintptr_t>(kda_smem_raw) + 1023) & ~uintptr_t(1023));
-  volatile int* abort_flag = &sm.abort_flag;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-
-  if (tid == 0) {
-    mbar_init(&sm.in_full, 1); mbar_init(&sm.v_full, 1);
-    mbar_init(&sm.x_full, KI_ELEM_THREADS); mbar_init(&sm.x_empty, 1);
-    for (int i = 0; i < KI_SETS; ++i) { mbar_init(&sm.img_full[i], KI_ELEM_THREADS); mbar_init(&sm.img_empty[i], 1); }
-    for (int i = 0; i < 6; ++i) { mbar_init(&sm.d_full[i], 1); mbar_init(&sm.d_empty[i], KI_SOLVER_THREADS); }
-    sm.abort_flag = 0;
-    mbar_init_fence();
+  load(0);
+  // ---- in-block levels, 16 channels (a half run of every lane) at a time.  lv[s][octet]: {kk(g8, 2 t4), kk(g8, 2 t4 + 1), qk.., qk..} of levels 1, 2, 4;
+  //      l8: rows 8 + g8 against columns 2 t4, 2 t4 + 1
+  float lv[3][2][4], l8[4];
+#pragma unroll
+  for (int s = 0; s < 3; ++s)
+#pragma unroll
+    for (int u = 0; u < 2; ++u) { lv[s][u][0] = lv[s][u][1] = lv[s][u][2] = lv[s][u][3] = 0.f; }
+  l8[0] = l8[1] = l8[2] = l8[3] = 0.f;
+#pragma unroll 1
+  for (int x = 0; x < 8; ++x) {
+    float pre[2][4], suf[2][4], tt[2][4];
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float d = fast_exp2(gv[u][e] * 1.4426950408889634f);
+        pre[u][e] = d; tt[u][e] = d; suf[u][e] = 1.f;
+      }
+    uint32_t kh[2][2], qh[2][2];                                                   // normalised, fp16
+    float kf[2][4], qf[2][4];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      kf[u][0] = bf16_lo(kv[u].x) * rk[u]; kf[u][1] = bf16_hi(kv[u].x) * rk[u]; kf[u][2] = bf16_lo(kv[u].y) * rk[u]; kf[u][3] = bf16_hi(kv[u].y) * rk[u];
+      qf[u][0] = bf16_lo(qv[u].x) * rq[u]; qf[u][1] = bf16_hi(qv[u].x) * rq[u]; qf[u][2] = bf16_lo(qv[u].y) * rq[u]; qf[u][3] = bf16_hi(qv[u].y) * rq[u];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) { kh[u][j] = pack_h2(kf[u][2 * j], kf[u][2 * j + 1]); qh[u][j] = pack_h2(qf[u][2 * j], qf[u][2 * j + 1]); }
+    }
+    if (x < 7) load(x + 1);
+#pragma unroll
+    for (int s = 0; s < 3; ++s) {                                                  // levels 1, 2, 4: the partner is lane ^ (4 << s)
+      const bool up = (g8 >> s) & 1;
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const uint32_t f0 = pack_h2(up ? pre[u][0] : suf[u][0], up ? pre[u][1] : suf[u][1]), f1 = pack_h2(up ? pre[u][2] : suf[u][2], up ? pre[u][3] : suf[u][3]);
+        const uint32_t k0 = hmul2_u32(kh[u][0], f0), k1 = hmul2_u32(kh[u][1], f1);
+        const uint32_t a[4] = {k0, hmul2_u32(qh[u][0], f0), k1, hmul2_u32(qh[u][1], f1)};
+        mma_f16(lv[s][u], a, k0, k1);
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float o = __shfl_xor_sync(0xffffffffu, tt[u][e], 4 << s);
+          if (up) pre[u][e] *= o; else suf[u][e] *= o;
+          tt[u][e] *= o;
+        }
+    }
+    {                                                                              // level 8: the two octets
+      const uint32_t fu0 = pack_h2(pre[1][0], pre[1][1]), fu1 = pack_h2(pre[1][2], pre[1][3]);
+      const uint32_t a[4] = {hmul2_u32(kh[1][0], fu0), hmul2_u32(qh[1][0], fu0), hmul2_u32(kh[1][1], fu1), hmul2_u32(qh[1][1], fu1)};
+      mma_f16(l8, a, hmul2_u32(kh[0][0], pack_h2(suf[0][0], suf[0][1])), hmul2_u32(kh[0][1], pack_h2(suf[0][2], suf[0][3])));
+#pragma unroll
+      for (int e = 0; e < 4; ++e) { pre[1][e] *= tt[0][e]; suf[0][e] *= tt[1][e]; }
+    }
+    // the block's images
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      sm.suf[warp][2 * x + u][lane] = make_uint2(pack_h2(kf[u][0] * suf[u][0], kf[u][1] * suf[u][1]), pack_h2(kf[u][2] * suf[u][2], kf[u][3] * suf[u][3]));
+      sm.pk[warp][2 * x + u][lane] = make_uint2(pack_h2(kf[u][0] * pre[u][0], kf[u][1] * pre[u][1]), pack_h2(kf[u][2] * pre[u][2], kf[u][3] * pre[u][3]));
+      sm.pq[warp][2 * x + u][lane] = make_uint2(pack_h2(qf[u][0] * pre[u][0], qf[u][1] * pre[u][1]), pack_h2(qf[u][2] * pre[u][2], qf[u][3] * pre[u][3]));
+    }
+    if (g8 == 0)
+      *reinterpret_cast<float4*>(&sm.tot[warp][32 * (x >> 1) + 8 * t4 + 4 * (x & 1)]) = make_float4(tt[0][0] * tt[1][0], tt[0][1] * tt[1][1], tt[0][2] * tt[1][2], tt[0][3] * tt[1][3]);
   }
-  if (warp == 0) { tmem_alloc(&sm.tmem_base, 512); tmem_relinquish(); }
-  tc_fence_before();
   __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = sm.tmem_base;
 
-  if (warp < KI_ELEM_WARPS) {
-    // ================================================================== element warps
-    const int c = tid & (KD - 1), seg = tid >> 7;          // this thread's channel and 16-token segment (warp-uniform)
-    if (tid == 0 && (int)blockIdx.x < p.total) {
-      int b, h, chunk, ft0, frows;
-      ki_coords(blockIdx.x, p.NC, p.H, b, h, chunk);
-      ki_chunk_span(p.chunk_tab, chunk, p.T, ft0, frows);
-      prefetch_tmap(&tm_g); prefetch_tmap(&tm_q); prefetch_tmap(&tm_k);
-      mbar_expect_tx(&sm.in_full, KI_IN_BYTES);
-      tma_load_4d(&sm.g[0][0], &tm_g, &sm.in_full, 0, ft0, h, b);
-      tma_load_4d(&sm.q[0][0], &tm_q, &sm.in_full, 0, ft0, h, b);
-      tma_load_4d(&sm.k[0][0], &tm_k, &sm.in_full, 0, ft0, h, b);
+  // ---- products with the earlier blocks
+  const float b0 = sm.beta[r0], b1 = sm.beta[r1];
+#pragma unroll 1
+  for (int J = warp - 1; J >= 0; --J) {
+    float kk[2][4], qk[2][4];
+#pragma unroll
+    for (int n = 0; n < 2; ++n) { kk[n][0] = kk[n][1] = kk[n][2] = kk[n][3] = 0.f; qk[n][0] = qk[n][1] = qk[n][2] = qk[n][3] = 0.f; }
+#pragma unroll 2
+    for (int x = 0; x < 8; ++x) {
+      uint2 c[2], kr[2], qr[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) { c[u] = sm.suf[J][2 * x + u][lane]; kr[u] = sm.pk[warp][2 * x + u][lane]; qr[u] = sm.pq[warp][2 * x + u][lane]; }
+      if (J < warp - 1) {                                                          // blocks lie between: their totals
+        const int ch = 32 * (x >> 1) + 8 * t4 + 4 * (x & 1);
+        float4 f = *reinterpret_cast<const float4*>(&sm.tot[J + 1][ch]);
+        if (J < warp - 2) f = ki_mul4(f, &sm.tot[J + 2][ch]);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) { kr[u] = ki_scale(kr[u], f); qr[u] = ki_scale(qr[u], f); }
+      }
+      const uint32_t ak[4] = {kr[0].x, kr[1].x, kr[0].y, kr[1].y}, aq[4] = {qr[0].x, qr[1].x, qr[0].y, qr[1].y};
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        mma_f16(kk[n], ak, c[n].x, c[n].y);
+        mma_f16(qk[n], aq, c[n].x, c[n].y);
+      }
     }
-    // warps 0..5 double as the issuers of the six Gram products (warp li issues level li): after its own share of
-    // the level's images the warp waits for everybody else's (all element warps do the same work in step, so the
-    // wait is short) and issues the product
-    const uint32_t leader = (warp < 6 && elect_one()) ? 1u : 0u;
-    const uint64_t gd0 = umma_desc_sw128(smem_u32(sm.img[0]), KI_IMG_BYTES, 1024);
-    const uint32_t g_lo0 = (uint32_t)gd0, g_hi = (uint32_t)(gd0 >> 32);
-    uint32_t ci = 0, n_img = 0;
-    bool ok = true;
-    for (int w = blockIdx.x; w < p.total; w += gridDim.x, ++ci) {
-      int b, h, chunk;
-      ki_coords(w, p.NC, p.H, b, h, chunk);
-      const int par = ci & 1;
-      int t0, rows;
-      ki_chunk_span(p.chunk_tab, chunk, p.T, t0, rows);
-      uint8_t* rec = p.ws + (size_t)w * REC_BYTES;
-      ok = mbar_wait_long(&sm.in_full, ci & 1, abort_flag, p.status, 1) && ok;
-      if (p.chunk_tab && rows < KC) {
-        // a sequence's last chunk: the rows after it belong to the next sequence (the tile load only zero-fills past
-        // the end of the tensor) -- blank them, so that they behave like padding: g = 0, k = q = 0 (beta = 0 below)
-        for (int i = tid; i < (KC - rows) * (KD / 4); i += KI_ELEM_THREADS) {
-          const int r = rows + i / (KD / 4), c4 = (i % (KD / 4)) * 4;
-          *reinterpret_cast<float4*>(&sm.g[r][c4]) = make_float4(0.f, 0.f, 0.f, 0.f);
-          *reinterpret_cast<uint2*>(&sm.q[r][c4]) = make_uint2(0u, 0u);
-          *reinterpret_cast<uint2*>(&sm.k[r][c4]) = make_uint2(0u, 0u);
-        }
-        named_bar(1, KI_ELEM_THREADS);
-      }
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+      const int col = 16 * J + 8 * n + 2 * t4;
+      *reinterpret_cast<uint32_t*>(&sm.akh[r0][col]) = pack_h2(b0 * kk[n][0], b0 * kk[n][1]);
+      *reinterpret_cast<uint32_t*>(&sm.akh[r1][col]) = pack_h2(b1 * kk[n][2], b1 * kk[n][3]);
+      *reinterpret_cast<uint32_t*>(rec + OFF_AQK + rec_off(r0, col)) = pack_h2(p.scale * qk[n][0], p.scale * qk[n][1]);
+      *reinterpret_cast<uint32_t*>(rec + OFF_AQK + rec_off(r1, col)) = pack_h2(p.scale * qk[n][2], p.scale * qk[n][3]);
+    }
+  }
 
-      // ---- per-token scalars: 8 threads per row, 16 channels each
-      {
-        const int r = tid >> 3, part = tid & 7;
-        float qf[16], kf[16];
-        unpack8(*reinterpret_cast<const uint4*>(&sm.q[r][16 * part]), qf);
-        unpack8(*reinterpret_cast<const uint4*>(&sm.q[r][16 * part + 8]), qf + 8);
-        unpack8(*reinterpret_cast<const uint4*>(&sm.k[r][16 * part]), kf);
-        unpack8(*reinterpret_cast<const uint4*>(&sm.k[r][16 * part + 8]), kf + 8);
-        float sq = 0.f, sk = 0.f, dqk = 0.f;
+  // ---- the diagonal block: each entry from its level
+  {
+    const int jc = 2 * t4;
 #pragma unroll
-        for (int e = 0; e < 16; ++e) { sq = fmaf(qf[e], qf[e], sq); sk = fmaf(kf[e], kf[e], sk); dqk = fmaf(qf[e], kf[e], dqk); }
-#pragma unroll
-        for (int o = 1; o <= 4; o <<= 1) {
-          sq += __shfl_xor_sync(0xffffffffu, sq, o);
-          sk += __shfl_xor_sync(0xffffffffu, sk, o);
-          dqk += __shfl_xor_sync(0xffffffffu, dqk, o);
-        }
-        if (part == 0) {
-          const float a = p.l2norm ? rsqrtf(sq + 1e-6f) : 1.f, cc = p.l2norm ? rsqrtf(sk + 1e-6f) : 1.f;
-          sm.rq[par][r] = a; sm.rk[par][r] = cc; sm.qkd[par][r] = a * cc * dqk;
-        }
-        if (tid < KC) sm.beta[par][tid] = (tid < rows) ? p.beta[((size_t)b * p.T + t0 + tid) * p.H + h] : 0.f;
-      }
-      if (named_bar_or(1, KI_ELEM_THREADS, !ok)) break;
-
-      // ---- this thread's column of the chunk: 16 tokens of channel c
-      float pre[16], suf[16];
-      uint32_t kn[8], qn[8];                                                     // normalised k, q as fp16 pairs (tokens 2i, 2i + 1)
-      {
-        const int r0 = 16 * seg;
-        float rkv[16], rqv[16];
-#pragma unroll
-        for (int i = 0; i < 16; i += 4) {
-          *reinterpret_cast<float4*>(&rkv[i]) = *reinterpret_cast<const float4*>(&sm.rk[par][r0 + i]);
-          *reinterpret_cast<float4*>(&rqv[i]) = *reinterpret_cast<const float4*>(&sm.rq[par][r0 + i]);
-        }
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          pre[i] = fast_exp2(sm.g[r0 + i][c] * 1.4426950408889634f);           // d_t = e^{g_t}
-          suf[i] = 1.f;
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          kn[i] = pack_h2(__bfloat162float(sm.k[r0 + 2 * i][c]) * rkv[2 * i], __bfloat162float(sm.k[r0 + 2 * i + 1][c]) * rkv[2 * i + 1]);
-          qn[i] = pack_h2(__bfloat162float(sm.q[r0 + 2 * i][c]) * rqv[2 * i], __bfloat162float(sm.q[r0 + 2 * i + 1][c]) * rqv[2 * i + 1]);
-        }
-      }
-      named_bar(1, KI_ELEM_THREADS);                                            // every read of the input tiles is done
-      if (tid == 0 && w + (int)gridDim.x < p.total) {                           // next item's inputs land under this item's work
-        int nb, nh, nchunk, nt0, nrows;
-        ki_coords(w + gridDim.x, p.NC, p.H, nb, nh, nchunk);
-        ki_chunk_span(p.chunk_tab, nchunk, p.T, nt0, nrows);
-        mbar_expect_tx(&sm.in_full, KI_IN_BYTES);
-        tma_load_4d(&sm.g[0][0], &tm_g, &sm.in_full, 0, nt0, nh, nb);
-        tma_load_4d(&sm.q[0][0], &tm_q, &sm.in_full, 0, nt0, nh, nb);
-        tma_load_4d(&sm.k[0][0], &tm_k, &sm.in_full, 0, nt0, nh, nb);
-      }
-
-      // ---- six levels.  At level s token t is "upper" iff bit s of t is set; its factor is pre (upper) or suf (lower):
-      //      the inclusive prefix / exclusive suffix product of d inside the aligned s-block of t.
-      auto emit = [&](const float (&f)[16], const bool write_q) {
-        ki_emit_level(sm, f, kn, qn, write_q, c, seg, warp, leader, ci, n_img, ok, tmem_base, g_lo0, g_hi, abort_flag, p.status);
-      };
-      // s = 1, 2, 4, 8: inside the segment (rows of lower tokens in the q image are never read back)
-      ki_level_inreg<1>(pre, suf, emit);
-      ki_level_inreg<2>(pre, suf, emit);
-      ki_level_inreg<4>(pre, suf, emit);
-      ki_level_inreg<8>(pre, suf, emit);
-      sm.tot[seg][c] = pre[15];
-      if (named_bar_or(1, KI_ELEM_THREADS, !ok)) break;
-      {                                                                         // s = 16: segments pair up
-        const bool up = (seg & 1) != 0;
-        float f[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) f[i] = up ? pre[i] : suf[i];
-        emit(f, up);
-        const float m = sm.tot[seg ^ 1][c];
-        if (seg & 1) {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) pre[i] *= m;
-        } else {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) suf[i] *= m;
-        }
-      }
-      {                                                                         // s = 32: halves of the chunk
-        const bool up = (seg & 2) != 0;
-        float f[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) f[i] = up ? pre[i] : suf[i];
-        emit(f, up);
-        const float m = (seg & 2) ? sm.tot[0][c] * sm.tot[1][c] : sm.tot[2][c] * sm.tot[3][c];
-        if (seg & 2) {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) pre[i] *= m;
-        } else {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) suf[i] *= m;
-        }
-      }
-      // ---- pre = e^{G}, suf = e^{G_C - G}: the state-pass operands
-      if (ci >= 1) ok = mbar_wait_long(&sm.x_empty, (ci - 1) & 1, abort_flag, p.status, 3) && ok;
+    for (int u = 0; u < 2; ++u) {
+      float kk[2], qk[2];
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        float x[8], qt[8], kt[8];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float2 kf = unpack_h2(kn[4 * e + i]), qf = unpack_h2(qn[4 * e + i]);
-          const int t = 8 * e + 2 * i;
-          x[2 * i] = kf.x * pre[t]; x[2 * i + 1] = kf.y * pre[t + 1];
-          qt[2 * i] = qf.x * pre[t] * p.scale; qt[2 * i + 1] = qf.y * pre[t + 1] * p.scale;
-          kt[2 * i] = kf.x * suf[t]; kt[2 * i + 1] = kf.y * suf[t + 1];
-        }
-        *reinterpret_cast<uint4*>(&sm.xt[c][16 * seg + 8 * e]) =
-            make_uint4(pack_h2(x[0], x[1]), pack_h2(x[2], x[3]), pack_h2(x[4], x[5]), pack_h2(x[6], x[7]));
-        const size_t goff = ((size_t)c * LDT + 16 * seg + 8 * e) * 2;
-        st_global16(rec + OFF_QT + goff, pack_h2(qt[0], qt[1]), pack_h2(qt[2], qt[3]), pack_h2(qt[4], qt[5]), pack_h2(qt[6], qt[7]));
-        st_global16(rec + OFF_KT + goff, pack_h2(kt[0], kt[1]), pack_h2(kt[2], kt[3]), pack_h2(kt[4], kt[5]), pack_h2(kt[6], kt[7]));
+        const int x = g8 ^ (jc + e);                                               // highest differing bit of the two token numbers
+        const float a = x >= 4 ? lv[2][u][e] : x >= 2 ? lv[1][u][e] : lv[0][u][e];
+        const float c = x >= 4 ? lv[2][u][2 + e] : x >= 2 ? lv[1][u][2 + e] : lv[0][u][2 + e];
+        const bool low = jc + e < g8;
+        kk[e] = low ? (u ? b1 : b0) * a : 0.f;
+        qk[e] = p.scale * (low ? c : jc + e == g8 ? qkd[u] : 0.f);                 // the diagonal: q_i . k_i, no decay
+        sm.dg[warp][8 * u + jc + e][8 * u + g8] = kk[e];
       }
-      if (seg == 3) reinterpret_cast<float*>(rec + OFF_D)[c] = pre[15];         // e^{G_C}
-      mbar_arrive(&sm.x_full);
+      *reinterpret_cast<uint32_t*>(rec + OFF_AQK + rec_off(16 * warp + 8 * u + g8, 16 * warp + 8 * u + jc)) = pack_h2(qk[0], qk[1]);
     }
-  } else {
-    // ================================================================== solver warps
-    // Two warps share each quarter of the TMEM lanes (warp % 4): rows 32 hb .. 32 hb + 31 of the k (quarters 0, 1) or
-    // q (quarters 2, 3) products; `ch` splits a row's 32-column window into two halves of 16.
-    const int ws = warp - KI_ELEM_WARPS, st = tid - KI_ELEM_THREADS;            // 0..7, 0..255
-    const int g8 = lane >> 2, t4 = lane & 3;
-    const int qt4 = ws & 3, ch = ws >> 2;
-    const bool is_qk = qt4 >= 2;
-    const int hb = qt4 & 1;
-    const int row = 32 * hb + lane;
-    const uint32_t lane_base = tmem_base + ((uint32_t)(32 * qt4) << 16);
-    if (st == 0 && (int)blockIdx.x < p.total) {
-      int b, h, chunk, ft0, frows;
-      ki_coords(blockIdx.x, p.NC, p.H, b, h, chunk);
-      ki_chunk_span(p.chunk_tab, chunk, p.T, ft0, frows);
-      prefetch_tmap(&tm_v);
-      mbar_expect_tx(&sm.v_full, KI_IMG_BYTES);
-      tma_load_4d(&sm.v[0][0], &tm_v, &sm.v_full, 0, ft0, h, b);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) { sm.dg[warp][jc + e][8 + g8] = b1 * l8[e]; sm.dg[warp][8 + jc + e][g8] = 0.f; }
+    *reinterpret_cast<uint32_t*>(rec + OFF_AQK + rec_off(r1, 16 * warp + jc)) = pack_h2(p.scale * l8[2], p.scale * l8[3]);
+    *reinterpret_cast<uint32_t*>(rec + OFF_AQK + rec_off(r0, 16 * warp + 8 + jc)) = 0u;
+  }
+  __syncwarp();
+  // ---- its inverse in fp32, lane = column: a column sweep (once t_j is final every later row takes its update at once)
+  if (lane < 16) {
+    float t[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) t[i] = (i == lane) ? 1.f : 0.f;
+#pragma unroll
+    for (int j = 0; j < 15; ++j) {
+      float a[16];
+#pragma unroll
+      for (int i4 = (j + 1) & ~3; i4 < 16; i4 += 4) *reinterpret_cast<float4*>(&a[i4]) = *reinterpret_cast<const float4*>(&sm.dg[warp][j][i4]);
+#pragma unroll
+      for (int i = j + 1; i < 16; ++i) t[i] = fmaf(-a[i], t[j], t[i]);
     }
-    uint32_t ci = 0;
-    bool ok = true;
-    for (int w = blockIdx.x; w < p.total; w += gridDim.x, ++ci) {
-      const int par = ci & 1;
-      uint8_t* rec = p.ws + (size_t)w * REC_BYTES;
-      // ---- Gram entries out of TMEM.  acc[j] collects row `row`, column 32 hb + 16 ch + j, level by level: the
-      //      entry of (row, column) lives in the level of the highest bit in which the two token indices differ.
-      float acc[16];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) acc[j] = 0.f;
-      float my_beta = 0.f, my_qkd = 0.f;
-#pragma unroll
-      for (int li = 0; li < 6; ++li) {
-        ok = __all_sync(0xffffffffu, mbar_wait_long(&sm.d_full[li], ci & 1, abort_flag, p.status, 6)) && ok;
-        if (li == 0) {                                                          // the item's scalars are final once its first image exists
-          if (st < KC) sm.sbeta[st] = sm.beta[par][st];
-          my_beta = sm.beta[par][row]; my_qkd = sm.qkd[par][row];
-        }
-        tc_fence_after();
-        uint32_t r[16];
-        if (li < 5) {
-          tmem_ld16(lane_base + 64 * li + 32 * hb + 16 * ch, r);
-          tc_wait_ld();
-          const uint32_t lx = (uint32_t)lane >> li;
-#pragma unroll
-          for (int j = 0; j < 16; ++j)
-            if (lx == (uint32_t)((((16 * ch + j) >> li)) ^ 1)) acc[j] = __uint_as_float(r[j]);
-        } else if (hb == 1) {                                                   // s = 32: rows 32..63 against columns 0..31, all of them
-          tmem_ld16(lane_base + 64 * 5 + 16 * ch, r);
-          tc_wait_ld();
-          const float sc = is_qk ? p.scale : my_beta;
-          uint32_t pk[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) pk[j] = pack_h2(sc * __uint_as_float(r[2 * j]), sc * __uint_as_float(r[2 * j + 1]));
-          if (is_qk) {
-            uint8_t* dst = rec + OFF_AQK + ((size_t)row * LDT + 16 * ch) * 2;
-            st_global16(dst, pk[0], pk[1], pk[2], pk[3]);
-            st_global16(dst + 16, pk[4], pk[5], pk[6], pk[7]);
-          } else {
-            *reinterpret_cast<uint4*>(&sm.akh[row][16 * ch]) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-            *reinterpret_cast<uint4*>(&sm.akh[row][16 * ch + 8]) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-          }
-        }
-        tc_fence_before();
-        mbar_arrive(&sm.d_empty[li]);
-      }
-      {
-        const float sc = is_qk ? p.scale : my_beta;
-        const int lj = lane - 16 * ch;                                          // this row's own column inside the 16 (if 0 <= lj < 16)
-        float v[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] = (j < lj) ? sc * acc[j] : 0.f;
-        uint32_t pk[8];
-        if (is_qk) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) if (j == lj) v[j] = p.scale * my_qkd;    // the diagonal: q_i . k_i, no decay
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) pk[j] = pack_h2(v[2 * j], v[2 * j + 1]);
-        if (is_qk) {
-          uint8_t* dst = rec + OFF_AQK + ((size_t)row * LDT + 32 * hb + 16 * ch) * 2;
-          st_global16(dst, pk[0], pk[1], pk[2], pk[3]);
-          st_global16(dst + 16, pk[4], pk[5], pk[6], pk[7]);
-        } else {
-          *reinterpret_cast<uint4*>(&sm.akh[row][32 * hb + 16 * ch]) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-          *reinterpret_cast<uint4*>(&sm.akh[row][32 * hb + 16 * ch + 8]) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-          if ((lane >> 4) == ch) {                                              // the row's diagonal 16 x 16 block, in fp32
-            const int blk = row >> 4;
-#pragma unroll
-            for (int j = 0; j < 16; ++j) sm.akk_t[blk][j][row & 15] = v[j];
-          }
-        }
-      }
-      if (named_bar_or(2, KI_SOLVER_THREADS, !ok)) break;
+    for (int i = 0; i < 16; ++i) sm.th[warp][i][lane] = __float2half_rn(t[i]);
+  }
 
-      // ---- the four 16 x 16 diagonal blocks of I + A_kk inverted in fp32, one block per warp, lane = column: a column
-      //      sweep (once t_j is final every later row takes its update at once), so the chain is 16 steps deep
-      if (ws < 4 && lane < 16) {
-        float t[16];
+  // ---- state-pass operands: k e^G (shared memory), q e^G scale and k e^{G_C - G} (record)
+  uint8_t *xt = reinterpret_cast<uint8_t*>(sm.pk), *vt = reinterpret_cast<uint8_t*>(sm.pq);
+  {
+    uint2 qr[16];                                                                  // all of this warp's q pre, then v may take its place
 #pragma unroll
-        for (int i = 0; i < 16; ++i) t[i] = (i == lane) ? 1.f : 0.f;
+    for (int i = 0; i < 16; ++i) qr[i] = sm.pq[warp][i][lane];
+    __syncwarp();
+    const uint32_t vb = smem_u32(vt);
 #pragma unroll
-        for (int j = 0; j < 15; ++j) {
-          float a[16];
+    for (int i = 0; i < 8; ++i) {
+      const int r = 16 * warp + 2 * i + (lane >> 4), c = lane & 15;
+      const uint32_t n = r < rows ? 16u : 0u;                                      // rows past the end: zeros
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(vb + ki_off(r, c)), "l"(p.v + tok * KD + (size_t)(r < rows ? r : 0) * ts + 8 * c), "r"(n) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    uint2 kr[16];
 #pragma unroll
-          for (int i4 = (j + 1) & ~3; i4 < 16; i4 += 4)
-            *reinterpret_cast<float4*>(&a[i4]) = *reinterpret_cast<const float4*>(&sm.akk_t[ws][j][i4]);
+    for (int i = 0; i < 16; ++i) kr[i] = sm.pk[warp][i][lane];
+    __syncwarp();
 #pragma unroll
-          for (int i = j + 1; i < 16; ++i) t[i] = fmaf(-a[i], t[j], t[i]);
-        }
-        const int base = ws * 16;
+    for (int m = 0; m < 4; ++m) {
+      const int ch = 32 * m + 8 * t4;
+      float4 f0 = make_float4(1.f, 1.f, 1.f, 1.f), f1 = f0, s0 = f0, s1 = f0;
+      for (int K = 0; K < warp; ++K) { f0 = ki_mul4(f0, &sm.tot[K][ch]); f1 = ki_mul4(f1, &sm.tot[K][ch + 4]); }
+      for (int K = warp + 1; K < 4; ++K) { s0 = ki_mul4(s0, &sm.tot[K][ch]); s1 = ki_mul4(s1, &sm.tot[K][ch + 4]); }
+      const float4 g0 = make_float4(f0.x * p.scale, f0.y * p.scale, f0.z * p.scale, f0.w * p.scale);
+      const float4 g1 = make_float4(f1.x * p.scale, f1.y * p.scale, f1.z * p.scale, f1.w * p.scale);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) sm.th[base + i][base + lane] = __float2half_rn(t[i]);   // t[i] = T[base + i][base + lane]
-      }
-      ok = mbar_wait_long(&sm.x_full, ci & 1, abort_flag, p.status, 7) && ok;   // (k e^G)^T is in place
-      ok = mbar_wait_long(&sm.v_full, ci & 1, abort_flag, p.status, 8) && ok;   // and the v tile
-      if (named_bar_or(2, KI_SOLVER_THREADS, !ok)) break;
-
-      // ---- W and U0 by blocked forward substitution on the transposed systems
-      //          W^T (I + A)^T = (diag(beta) k e^G)^T,      U0^T (I + A)^T = (diag(beta) v)^T
-      //      A warp owns 32 of the 256 rows (channels of W^T: warps 0-3, value columns of U0^T: warps 4-7) for all
-      //      four 16-token block columns I, so there is nothing to exchange between warps:
-      //          Z_I = R_I - sum_{J<I} Z_J A_IJ^T,   then   Z_I <- Z_I T_II^T
-      //      with every product an m16n8k16 tile whose fp32 accumulators, rounded to fp16, are the A fragment of
-      //      the products that follow.  The two row tiles of a warp are independent chains issued side by side.
-      {
-        const bool is_w = ws < 4;
-        uint8_t* dst = rec + (is_w ? OFF_WT : OFF_UT);
-        uint32_t zf[2][3][4];                                                   // Z_J as fp16 A fragments: [row tile][J][4]
-#pragma unroll
-        for (int I = 0; I < 4; ++I) {
-          float acc1[2][2][4];
-#pragma unroll
-          for (int m = 0; m < 2; ++m)
-#pragma unroll
-            for (int nn = 0; nn < 2; ++nn) { acc1[m][nn][0] = acc1[m][nn][1] = acc1[m][nn][2] = acc1[m][nn][3] = 0.f; }
-#pragma unroll
-          for (int J = 0; J < I; ++J) {
-#pragma unroll
-            for (int nn = 0; nn < 2; ++nn) {
-              const __half* arow = &sm.akh[I * 16 + nn * 8 + g8][J * 16 + 2 * t4];
-              const uint32_t b0 = *reinterpret_cast<const uint32_t*>(arow), b1 = *reinterpret_cast<const uint32_t*>(arow + 8);
-#pragma unroll
-              for (int m = 0; m < 2; ++m) mma_f16(acc1[m][nn], zf[m][J], b0, b1);
-            }
-          }
-          uint32_t a2[2][4];
-#pragma unroll
-          for (int nn = 0; nn < 2; ++nn) {
-            const int tk = I * 16 + nn * 8 + 2 * t4;                            // this thread's two tokens of the tile
-            const float2 bt = *reinterpret_cast<const float2*>(&sm.sbeta[tk]);
-#pragma unroll
-            for (int m = 0; m < 2; ++m) {
-              const int r0 = 16 * (2 * (ws & 3) + m) + g8;                      // row inside this matrix: channel or value column
-              float2 lo, hi;                                                    // right-hand side at rows r0 and r0 + 8
-              if (is_w) {
-                lo = unpack_h2(*reinterpret_cast<const uint32_t*>(&sm.xt[r0][tk]));
-                hi = unpack_h2(*reinterpret_cast<const uint32_t*>(&sm.xt[r0 + 8][tk]));
-              } else {
-                lo = make_float2(__bfloat162float(sm.v[tk][r0]), __bfloat162float(sm.v[tk + 1][r0]));
-                hi = make_float2(__bfloat162float(sm.v[tk][r0 + 8]), __bfloat162float(sm.v[tk + 1][r0 + 8]));
-              }
-              a2[m][2 * nn] = pack_h2(lo.x * bt.x - acc1[m][nn][0], lo.y * bt.y - acc1[m][nn][1]);
-              a2[m][2 * nn + 1] = pack_h2(hi.x * bt.x - acc1[m][nn][2], hi.y * bt.y - acc1[m][nn][3]);
-            }
-          }
-#pragma unroll
-          for (int nn = 0; nn < 2; ++nn) {
-            const __half* trow = &sm.th[I * 16 + nn * 8 + g8][I * 16 + 2 * t4];
-            const uint32_t b0 = *reinterpret_cast<const uint32_t*>(trow), b1 = *reinterpret_cast<const uint32_t*>(trow + 8);
-            const int tk = I * 16 + nn * 8 + 2 * t4;
-#pragma unroll
-            for (int m = 0; m < 2; ++m) {
-              float acc2[4] = {0.f, 0.f, 0.f, 0.f};
-              mma_f16(acc2, a2[m], b0, b1);
-              const uint32_t z_lo = pack_h2(acc2[0], acc2[1]), z_hi = pack_h2(acc2[2], acc2[3]);
-              if (I < 3) { zf[m][I][2 * nn] = z_lo; zf[m][I][2 * nn + 1] = z_hi; }
-              const int r0 = 16 * (2 * (ws & 3) + m) + g8;
-              *reinterpret_cast<uint32_t*>(dst + ((size_t)r0 * LDT + tk) * 2) = z_lo;
-              *reinterpret_cast<uint32_t*>(dst + ((size_t)(r0 + 8) * LDT + tk) * 2) = z_hi;
-            }
-          }
-        }
-      }
-      if (named_bar_or(2, KI_SOLVER_THREADS, !ok)) break;                      // every warp is done with the X image and the v tile
-      if (st == 0) {
-        mbar_arrive(&sm.x_empty);
-        if (w + (int)gridDim.x < p.total) {
-          int nb, nh, nchunk, nt0, nrows;
-          ki_coords(w + gridDim.x, p.NC, p.H, nb, nh, nchunk);
-          ki_chunk_span(p.chunk_tab, nchunk, p.T, nt0, nrows);
-          mbar_expect_tx(&sm.v_full, KI_IMG_BYTES);
-          tma_load_4d(&sm.v[0][0], &tm_v, &sm.v_full, 0, nt0, nh, nb);
-        }
+      for (int u = 0; u < 2; ++u) {
+        const uint32_t off = ki_off(u ? r1 : r0, 4 * m + t4);
+        const uint2 x0 = ki_scale(kr[4 * m + u], f0), x1 = ki_scale(kr[4 * m + 2 + u], f1);
+        const uint2 q0 = ki_scale(qr[4 * m + u], g0), q1 = ki_scale(qr[4 * m + 2 + u], g1);
+        const uint2 k0 = ki_scale(sm.suf[warp][4 * m + u][lane], s0), k1 = ki_scale(sm.suf[warp][4 * m + 2 + u][lane], s1);
+        *reinterpret_cast<uint4*>(xt + off) = make_uint4(x0.x, x0.y, x1.x, x1.y);
+        st_global16(rec + OFF_QT + off, q0.x, q0.y, q1.x, q1.y);
+        st_global16(rec + OFF_KT + off, k0.x, k0.y, k1.x, k1.y);
       }
     }
   }
-
-  // ------------------------------------------------------------------ teardown
-  tc_fence_before();
+  reinterpret_cast<float*>(rec + OFF_D)[tid] = (sm.tot[0][tid] * sm.tot[1][tid]) * (sm.tot[2][tid] * sm.tot[3][tid]);   // e^{G_C}
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
-  if (warp == 0) {
-    tc_fence_after();
-    tmem_dealloc(tmem_base, 512);
+
+  // ---- W and U0 by blocked forward substitution on the transposed systems
+  //          W^T (I + A)^T = (diag(beta) k e^G)^T,      U0^T (I + A)^T = (diag(beta) v)^T
+  //      A warp owns 64 of the 256 rows (channels of W^T: warps 0, 1, value columns of U0^T: warps 2, 3) for all four
+  //      16-token block columns I, so there is nothing to exchange between warps:
+  //          Z_I = R_I - sum_{J<I} Z_J A_IJ^T,   then   Z_I <- Z_I T_II^T
+  //      with every product an m16n8k16 tile whose fp32 accumulators, rounded to fp16, are the A fragment of the products
+  //      that follow.  The four row tiles of a warp are independent chains issued side by side.
+  {
+    const bool is_w = warp < 2;
+    const uint32_t src = smem_u32(is_w ? xt : vt);
+    uint8_t* dst = rec + (is_w ? OFF_WT : OFF_UT);
+    const int c0 = 64 * (warp & 1);                                                // first row (channel or value column)
+    uint32_t zf[4][3][4];                                                          // Z_J as fp16 A fragments: [row tile][J][4]
+#pragma unroll
+    for (int I = 0; I < 4; ++I) {
+      float acc[4][2][4];
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+#pragma unroll
+        for (int n = 0; n < 2; ++n) { acc[m][n][0] = acc[m][n][1] = acc[m][n][2] = acc[m][n][3] = 0.f; }
+#pragma unroll
+      for (int J = 0; J < I; ++J) {
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+          const __half* arow = &sm.akh[I * 16 + n * 8 + g8][J * 16 + 2 * t4];
+          const uint32_t w0 = *reinterpret_cast<const uint32_t*>(arow), w1 = *reinterpret_cast<const uint32_t*>(arow + 8);
+#pragma unroll
+          for (int m = 0; m < 4; ++m) mma_f16(acc[m][n], zf[m][J], w0, w1);
+        }
+      }
+      uint32_t tw[2][2];
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        const __half* trow = &sm.th[I][n * 8 + g8][2 * t4];
+        tw[n][0] = *reinterpret_cast<const uint32_t*>(trow); tw[n][1] = *reinterpret_cast<const uint32_t*>(trow + 8);
+      }
+      const float2 bt0 = *reinterpret_cast<const float2*>(&sm.beta[I * 16 + 2 * t4]), bt1 = *reinterpret_cast<const float2*>(&sm.beta[I * 16 + 8 + 2 * t4]);
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        // right-hand side: tokens 16 I .. + 15 x rows c0 + 16 m .. + 15, transposed: register i = (tokens 8 (i >> 1) + 2 t4 (+1),
+        // row 8 (i & 1) + g8)
+        uint32_t rr[4];
+        const int row = I * 16 + (lane & 7) + 8 * (lane >> 4), pc = (c0 >> 3) + 2 * m + ((lane >> 3) & 1);
+        ldmatrix_x4_t(rr, src + ki_off(row, pc));
+        uint32_t a[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int n = i >> 1, hi = i & 1;
+          const float2 r = is_w ? unpack_h2(rr[i]) : make_float2(bf16_lo(rr[i]), bf16_hi(rr[i]));
+          const float2 bt = n ? bt1 : bt0;
+          a[2 * n + hi] = pack_h2(r.x * bt.x - acc[m][n][2 * hi], r.y * bt.y - acc[m][n][2 * hi + 1]);
+        }
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+          float z[4] = {0.f, 0.f, 0.f, 0.f};
+          mma_f16(z, a, tw[n][0], tw[n][1]);
+          const uint32_t zl = pack_h2(z[0], z[1]), zh = pack_h2(z[2], z[3]);
+          if (I < 3) { zf[m][I][2 * n] = zl; zf[m][I][2 * n + 1] = zh; }
+          const int cr = c0 + 16 * m + g8;
+          *reinterpret_cast<uint32_t*>(dst + rec_off(cr, I * 16 + n * 8 + 2 * t4)) = zl;
+          *reinterpret_cast<uint32_t*>(dst + rec_off(cr + 8, I * 16 + n * 8 + 2 * t4)) = zh;
+        }
+      }
+    }
   }
 }
 
@@ -639,7 +511,7 @@ template <int NW, int KS, int NST>
 struct KdaStateSmem {
   static constexpr int VS = 16 * NW;
   static constexpr int CW = NW * KS;                     // compute warps
-  static constexpr int U_BYTES = VS * LDT * 2;
+  static constexpr int U_BYTES = VS * KC * 2;
   static constexpr int STAGE = SHARED_BYTES + U_BYTES;
   static constexpr int O_LD = VS + 4;                    // floats; staging of one chunk of output
   static constexpr int XCH_WARP = 2 * 8 * 32 * 16;       // one warp's two partial accumulators: 8 tiles x 32 lanes x float4
@@ -688,7 +560,7 @@ __global__ void __launch_bounds__(32 * (NW * KS + 1), 1) kda_state_kernel(const 
         const uint8_t* rec = recs + (size_t)c * REC_BYTES;
         mbar_expect_tx(&full[s], L::STAGE);
         bulk_g2s(stages + s * L::STAGE, rec, SHARED_BYTES, &full[s]);
-        bulk_g2s(stages + s * L::STAGE + SHARED_BYTES, rec + OFF_UT + (size_t)v_base * LDT * 2, L::U_BYTES, &full[s]);
+        bulk_g2s(stages + s * L::STAGE + SHARED_BYTES, rec + OFF_UT + (size_t)v_base * KC * 2, L::U_BYTES, &full[s]);
       }
     }
     return;
@@ -715,12 +587,9 @@ __global__ void __launch_bounds__(32 * (NW * KS + 1), 1) kda_state_kernel(const 
     const bool ok = __all_sync(0xffffffffu, mbar_wait(&full[s], (c / KDA_NST) & 1, abort_flag, p.status, 2));
     if (!ok) break;
     const uint8_t* sb = stages + s * L::STAGE;
-    const __half* Wt = reinterpret_cast<const __half*>(sb + OFF_WT);
-    const __half* Qt = reinterpret_cast<const __half*>(sb + OFF_QT);
-    const __half* Kt = reinterpret_cast<const __half*>(sb + OFF_KT);
-    const __half* Aq = reinterpret_cast<const __half*>(sb + OFF_AQK);
+    const uint32_t Wt = smem_u32(sb + OFF_WT), Qt = smem_u32(sb + OFF_QT), Kt = smem_u32(sb + OFF_KT), Aq = smem_u32(sb + OFF_AQK);
     const float* dv = reinterpret_cast<const float*>(sb + OFF_D);
-    const __half* Ut = reinterpret_cast<const __half*>(sb + SHARED_BYTES);
+    const uint8_t* Ut = sb + SHARED_BYTES;
 
     // (1) accU = S^T W^T   and   (2a) accO = S^T q~^T      [16 x 64 tokens each], over this warp's K columns
     float au[8][4], ao[8][4];
@@ -732,14 +601,14 @@ __global__ void __launch_bounds__(32 * (NW * KS + 1), 1) kda_state_kernel(const 
       uint32_t a[4];
       a[0] = pack_h2(st[2 * ksl][0], st[2 * ksl][1]); a[1] = pack_h2(st[2 * ksl][2], st[2 * ksl][3]);
       a[2] = pack_h2(st[2 * ksl + 1][0], st[2 * ksl + 1][1]); a[3] = pack_h2(st[2 * ksl + 1][2], st[2 * ksl + 1][3]);
-      // B fragments of two token tiles per transposing ldmatrix.x4 from the channel-major images: matrix m =
-      // (k half m & 1, token tile nt + (m >> 1)); its stored rows are channels, its columns tokens
-      const int lrow = ks * 16 + ((lane >> 3) & 1) * 8 + (lane & 7), lcol = (lane >> 4) * 8;
+      // B fragments of two token tiles per ldmatrix.x4, matrix m = (channel octet m & 1, token tile nt + (m >> 1)): W^T rows
+      // are channels (transposing form), q~ rows are tokens
+      const int wrow = ks * 16 + ((lane >> 3) & 1) * 8 + (lane & 7), qrow = (lane & 7) + 8 * (lane >> 4), qpc = 2 * ks + ((lane >> 3) & 1);
 #pragma unroll
       for (int nt = 0; nt < 8; nt += 2) {
         uint32_t bw[4], bq[4];
-        ldmatrix_x4_t(bw, &Wt[lrow * LDT + nt * 8 + lcol]);
-        ldmatrix_x4_t(bq, &Qt[lrow * LDT + nt * 8 + lcol]);
+        ldmatrix_x4_t(bw, Wt + rec_off(wrow, (nt + (lane >> 4)) * 8));
+        ldmatrix_x4(bq, Qt + ki_off(nt * 8 + qrow, qpc));
         mma_f16(au[nt], a, bw[0], bw[1]);
         mma_f16(ao[nt], a, bq[0], bq[1]);
         mma_f16(au[nt + 1], a, bw[2], bw[3]);
@@ -785,8 +654,8 @@ __global__ void __launch_bounds__(32 * (NW * KS + 1), 1) kda_state_kernel(const 
 #pragma unroll
     for (int nt = 0; nt < 8; ++nt) {
       const int tok = nt * 8 + 2 * t4;
-      const float2 u0 = unpack_h2(*reinterpret_cast<const uint32_t*>(&Ut[vr0 * LDT + tok]));
-      const float2 u1 = unpack_h2(*reinterpret_cast<const uint32_t*>(&Ut[vr1 * LDT + tok]));
+      const float2 u0 = unpack_h2(*reinterpret_cast<const uint32_t*>(Ut + rec_off(vr0, tok)));
+      const float2 u1 = unpack_h2(*reinterpret_cast<const uint32_t*>(Ut + rec_off(vr1, tok)));
       const uint32_t lo = pack_h2(u0.x - au[nt][0], u0.y - au[nt][1]);
       const uint32_t hi = pack_h2(u1.x - au[nt][2], u1.y - au[nt][3]);
       ua[nt >> 1][(nt & 1) * 2 + 0] = lo;
@@ -800,7 +669,7 @@ __global__ void __launch_bounds__(32 * (NW * KS + 1), 1) kda_state_kernel(const 
       for (int nt = 2 * ks; nt < 8; nt += 2) {                     // A_qk[i][j] = 0 for j > i: tiles below 2 ks are empty
         if (KS > 1 && nt / TPW != kq) continue;
         uint32_t ba[4];
-        ldmatrix_x4(ba, &Aq[(nt * 8 + lrow) * LDT + lcol]);
+        ldmatrix_x4(ba, Aq + rec_off(nt * 8 + lrow, lcol));
         mma_f16(ao[nt], ua[ks], ba[0], ba[1]);
         mma_f16(ao[nt + 1], ua[ks], ba[2], ba[3]);
       }
@@ -813,11 +682,11 @@ __global__ void __launch_bounds__(32 * (NW * KS + 1), 1) kda_state_kernel(const 
     }
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks) {
-      const int lrow = (lane >> 4) * 8 + (lane & 7), lcol = ks * 16 + ((lane >> 3) & 1) * 8;
+      const int krow = ks * 16 + ((lane >> 3) & 1) * 8 + (lane & 7);            // k~ rows are tokens: transposing form
 #pragma unroll
       for (int j = 0; j < NKT; j += 2) {
         uint32_t bk[4];
-        ldmatrix_x4(bk, &Kt[((kq * NKT + j) * 8 + lrow) * LDT + lcol]);
+        ldmatrix_x4_t(bk, Kt + ki_off(krow, kq * NKT + j + (lane >> 4)));
         mma_f16(st[j], ua[ks], bk[0], bk[1]);
         mma_f16(st[j + 1], ua[ks], bk[2], bk[3]);
       }
@@ -905,7 +774,7 @@ static int kda_launch(const void* q, const void* k, const void* v, const float* 
   static bool attr[daisy_host::MAX_DEVICES] = {};             // the attribute is per device
   const int dev = daisy_host::device_slot();
   if (dev < 0) return DAISY_ENODEV;
-  constexpr int intra_smem = (int)sizeof(KdaIntraSmem) + 1024;   // the kernel aligns its image buffers to 1 KB itself
+  constexpr int intra_smem = (int)sizeof(KdaIntraSmem);
   if (!attr[dev]) {
     if (cudaFuncSetAttribute(kda_intra_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, intra_smem) != cudaSuccess) {
       (void)cudaGetLastError();
@@ -914,22 +783,14 @@ static int kda_launch(const void* q, const void* k, const void* v, const float* 
     attr[dev] = true;
   }
   if ((int64_t)B * H * NC >= ((int64_t)1 << 31)) return DAISY_EUNSUPPORTED;
-  CUtensorMap tg, tq, tk, tv;
-  int trc;
-  if ((trc = daisy_host::make_tmap_rows_bthd(&tg, g, 4, KD, T, H, B, KC)) != DAISY_OK) return trc;
-  if ((trc = daisy_host::make_tmap_rows_bthd(&tq, q, 2, KD, T, H, B, KC)) != DAISY_OK) return trc;
-  if ((trc = daisy_host::make_tmap_rows_bthd(&tk, k, 2, KD, T, H, B, KC)) != DAISY_OK) return trc;
-  if ((trc = daisy_host::make_tmap_rows_bthd(&tv, v, 2, KD, T, H, B, KC)) != DAISY_OK) return trc;
   KdaIntraParams ip;
+  ip.q = (const __nv_bfloat16*)q; ip.k = (const __nv_bfloat16*)k; ip.v = (const __nv_bfloat16*)v; ip.g = g;
   ip.beta = beta; ip.ws = (uint8_t*)workspace;
-  ip.T = T; ip.H = H; ip.NC = NC; ip.total = B * H * NC;
+  ip.T = T; ip.H = H; ip.NC = NC;
   ip.scale = scale > 0.f ? scale : 1.0f / sqrtf((float)K);
   ip.l2norm = (flags & DAISY_KDA_L2NORM_QK) ? 1 : 0;
-  ip.status = status_word;
   ip.chunk_tab = chunk_tab;
-  const int sms = daisy_host::sm_count_cached();
-  if (sms <= 0) return DAISY_ENODEV;
-  kda_intra_kernel<<<ip.total < sms ? ip.total : sms, KI_THREADS, intra_smem, st>>>(tg, tq, tk, tv, ip);
+  kda_intra_kernel<<<dim3(NC, H, B), KI_THREADS, intra_smem, st>>>(ip);
   DAISY_CHECK_LAUNCH();
 
   KdaStateParams sp;

@@ -7,12 +7,10 @@
 //     T = (I + A_kk)^-1          W = T (beta k e^G)          U0 = T (beta v)
 //     U = U0 - W S_0             O = (scale q e^G) S_0 + A_qk U          S_C = e^{G_C} S_0 + (k e^{G_C-G})^T U
 // Two kernels:
-//  * kda_intra_kernel  -- everything that does not depend on the state, all chunks in parallel, on tcgen05 tensor
-//    cores: a persistent CTA per SM walks (batch, head, chunk) work items; 16 "element" warps turn the TMA-staged
-//    inputs into fp16 operand images and issue the Gram products on them, 8 "solver" warps pull the Gram entries
-//    out of TMEM and solve (I + A_kk) W = beta k e^G, (I + A_kk) U0 = beta v block by block with register-chained
-//    mma.sync tiles -- two pipelines that overlap across consecutive chunks.  Per chunk it writes a record of fp16 operand images (rows padded so that fragment loads
-//    are bank-conflict free): W^T, (scale q e^G)^T, (k e^{G_C-G})^T, U0^T as [128][72], A_qk as [64][72], e^{G_C}.
+//  * kda_intra_kernel  -- everything that does not depend on the state, a small CTA per (batch, head, chunk), three to an SM:
+//    Gram products in mma.sync fragments, the blocked solve of (I + A_kk) W = beta k e^G, (I + A_kk) U0 = beta v in register
+//    chains.  Per chunk it writes a record of fp16 operand images (16-byte pieces exchanged so that fragment loads are
+//    bank-conflict free): W^T, scale q e^G, k e^{G_C-G}, A_qk, U0^T, and e^{G_C}.
 //  * kda_state_kernel  -- one CTA per (batch, head, V-slice), sequential over chunks: a producer warp
 //    bulk-copies the images of chunk c+1.. into a shared-memory ring while the compute warps hold their
 //    slice of S^T (16 V-rows x 128 K-columns per warp) in fp32 accumulator registers and chain the
@@ -22,6 +20,7 @@
 // Tensor-core operands are fp16 (10-bit mantissa, every decay factor and operand here is <= O(1)):
 // measured relative error of o against the fp32 token recurrence is ~4e-4, bf16 operands give ~3e-3.
 #include <cuda_fp16.h>
+#include <type_traits>
 #include "common.cuh"
 
 namespace daisy {
@@ -70,6 +69,17 @@ __device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
   __half2 h = __floats2half2_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&h);
 }
+__device__ __forceinline__ uint32_t pack_h2(uint64_t v) {
+  float lo, hi;
+  unpack2f(v, lo, hi);
+  return pack_h2(lo, hi);
+}
+__device__ __forceinline__ void mma_bf16(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
+  asm(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
 __device__ __forceinline__ float2 unpack_h2(uint32_t u) {
   return __half22float2(*reinterpret_cast<__half2*>(&u));
 }
@@ -96,17 +106,20 @@ __device__ __forceinline__ void st_global16(void* p, uint32_t a, uint32_t b, uin
 // Every factor is a running product of numbers <= 1 -- ONE exponential per input element, no cumulative sum, and underflow
 // is the correct limit.
 //
-// A CTA of four warps owns one (batch, head, chunk), warp w the tokens 16 w .. 16 w + 15, three CTAs to an SM.  A lane
-// holds rows g8 and g8 + 8 of its block and 32 of the 128 channels (four runs of eight: 16-byte loads) -- as m16n8k16
-// fragments with the channels in an order of our own, which a contraction over channels does not notice.  In that form the
-// A and the B operand of a Gram product are the same registers, so the in-block levels need no shared memory at all: k and
-// q rows of an octet are stacked into one A operand, and a level costs two products per 16 channels.  Blocks meet only
-// through their `suf` images (stored and read back register by register) and their totals.
-// Then the four diagonal blocks of I + A_kk are inverted (fp32, one per warp) and W, U0 come from a blocked forward
-// substitution on the transposed systems, a warp owning 64 of the 256 rows (see below).
+// A CTA of four warps owns one (batch, head, chunk), warp w the tokens 16 w .. 16 w + 15, three CTAs to an SM.  The running
+// products are taken with lane = two channels, all 16 tokens in registers (which half of a group a token is in is then
+// known at compile time, and no product crosses a lane), 64 channels at a time.  A level's images k f, q f go through 4 KB of
+// the warp's own shared memory into m16n8k16 fragments: k and q rows of an octet are stacked into one A operand, two of
+// whose four registers are also the B operand, so a level costs one ldmatrix and one product per octet and 16 channels.
+// The norms are diagonals of the raw bf16 products, formed the same way.  Blocks meet only through their `suf` images and
+// their totals.  Then the four diagonal blocks of I + A_kk are inverted (fp32, one per warp) and W, U0 come from a blocked
+// forward substitution on the transposed systems, a warp owning 64 of the 256 rows (see below).
+// What bounds it: 22k warp instructions a chunk at 35 % issue, the rest waits for the rows of g and v with 12 warps on an SM
+// (asking L2 for them at the start: 433 -> 425 us at 4 x 8192 x 16).  Lane = (2 tokens, 8 channels), as the fragments want
+// it, costs three shuffles and twice the selects per product: 27k instructions, 937 us at 4 x 16384 x 16 where this takes 840.
 // Why not tcgen05: the version of this kernel that built six image sets in shared memory for 128 x 64 x 128 tcgen05 products
 // was a chain of hand-offs between warp groups (image -> fence -> product -> TMEM load), 20k cycles a chunk with the tensor
-// pipe at 10 %; here everything between two barriers stays in one warp's registers and three CTAs hide each other's latency.
+// pipe at 10 %; here everything between two barriers stays inside one warp and three CTAs hide each other's latency.
 struct KdaIntraParams {
   const __nv_bfloat16 *q, *k, *v;
   const float *g, *beta;
@@ -121,16 +134,17 @@ struct KdaIntraParams {
 
 constexpr int KI_THREADS = 128;
 constexpr int LDAK = 72;                                // halves per row of the A_kk image
+constexpr int KI_LD = 256 + 16, KI_LV = 128 + 16;       // bytes between rows of a block's image, and of a level's (64 channels)
 struct KdaIntraSmem {
-  // each block's images, register by register: [block][half run, octet][lane].  pk and pq (k pre, q pre) are read by their own
-  // warp only, which then lays k e^G and its v rows over them: token-major, swizzled rows of 256 bytes, block w in [w]
-  uint2 suf[4][16][32];
-  uint2 pk[4][16][32];
-  uint2 pq[4][16][32];
+  // each block's k suf, k pre, q pre: [block], 16 token rows of 256 bytes, 16 bytes apart (conflict-free for whole rows and for
+  // ldmatrix, with addresses that are constants plus one register).  pk and pq hold the raw rows before and are read by their
+  // own warp only, which lays k e^G and its v rows over them afterwards; suf is the level images' room before
+  uint8_t suf[4][2 * 16 * KI_LV], pk[4][16 * KI_LD], pq[4][16 * KI_LD];
   __half akh[KC][LDAK];                                 // beta A_kk below the diagonal blocks
   float dg[4][16][20];                                  // beta A_kk, the diagonal blocks, column-major ([j][i])
   __half th[4][16][24];                                 // their inverses (of I + A_kk), row-major
-  float tot[4][KD];                                     // product of the decays of each block, in the lanes' channel order
+  float tot[4][KD];                                     // product of the decays of each block
+  float nrm[4][3][16];                                  // 1 / |k|, 1 / |q|, normalised q . k of each token
   float beta[KC];
 };
 
@@ -154,16 +168,11 @@ __device__ __forceinline__ uint2 ld_nc8(const void* p) {
   asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(r.x), "=r"(r.y) : "l"(p));
   return r;
 }
-__device__ __forceinline__ float4 ki_mul4(const float4 a, const float* b) {
-  const float4 c = *reinterpret_cast<const float4*>(b);
-  return make_float4(a.x * c.x, a.y * c.y, a.z * c.z, a.w * c.w);
+// two fp16 values times fp32 factors, one rounding
+__device__ __forceinline__ uint32_t ki_scale(uint32_t a, const float2 f) {
+  const float2 x = unpack_h2(a);
+  return pack_h2(fmul2(pack2f(x.x, x.y), pack2f(f.x, f.y)));
 }
-// four fp16 values times fp32 factors, one rounding
-__device__ __forceinline__ uint2 ki_scale(const uint2 a, const float4 f) {
-  const float2 lo = unpack_h2(a.x), hi = unpack_h2(a.y);
-  return make_uint2(pack_h2(lo.x * f.x, lo.y * f.y), pack_h2(hi.x * f.z, hi.y * f.w));
-}
-
 __global__ void __launch_bounds__(KI_THREADS, 3) kda_intra_kernel(const KdaIntraParams p) {
   extern __shared__ __align__(128) uint8_t kda_smem_raw[];
   KdaIntraSmem& sm = *reinterpret_cast<KdaIntraSmem*>(kda_smem_raw);
@@ -175,62 +184,50 @@ __global__ void __launch_bounds__(KI_THREADS, 3) kda_intra_kernel(const KdaIntra
   const size_t tok = ((size_t)b * p.T + t0) * p.H + h, ts = (size_t)p.H * KD;      // row of token i: tok * KD + i * ts
 
   if (tid < KC) sm.beta[tid] = tid < rows ? p.beta[tok + (size_t)tid * p.H] : 0.f;
-  for (int i = tid; i < 2 * rows; i += KI_THREADS)                                 // v is needed last: ask L2 for it now
+  for (int i = tid; i < 4 * rows; i += KI_THREADS)                                 // g and v are needed later: ask L2 for them now
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(p.g + tok * KD + (size_t)(i >> 2) * ts + 32 * (i & 3)));
+  for (int i = tid; i < 2 * rows; i += KI_THREADS)
     asm volatile("prefetch.global.L2 [%0];" ::"l"(p.v + tok * KD + (size_t)(i >> 1) * ts + 64 * (i & 1)));
-  const int r0 = 16 * warp + g8, r1 = r0 + 8;                                      // this lane's two tokens
-  const bool ok0 = r0 < rows, ok1 = r1 < rows;
-  const size_t o0 = tok * KD + (size_t)(ok0 ? r0 : 0) * ts + 8 * t4, o1 = tok * KD + (size_t)(ok1 ? r1 : 0) * ts + 8 * t4;
+  const int r0 = 16 * warp + g8, r1 = r0 + 8;                                      // this lane's two rows in the products
+  const int nrow = rows - 16 * warp;                                               // rows of this block that exist (<= 0: none)
+  const uint32_t s_suf = smem_u32(sm.suf[warp]), s_pk = smem_u32(sm.pk[warp]), s_pq = smem_u32(sm.pq[warp]);
+  // fragment addresses: A = {k octet, q octet} x 16 channels from images at s_pk, s_pq; lane l gives row (l & 7) of matrix l >> 3
+  const uint32_t s_kq = (lane & 8) ? s_pq : s_pk;
 
-  // A lane's channels: runs 32 m + 8 t4 .. + 7 (m = 0 .. 3) of rows r0, r1, taken in halves of four.  q and k are read twice,
-  // the second time from L2: first for the norms, then with g, run by run (kept, they and the level sums do not fit the
-  // 168 registers that three CTAs leave a thread).
-  float gv[2][4];                                                                  // the next half run: log-decays,
-  uint2 kv[2], qv[2];                                                              // k and q
-  auto load = [&](int x) {
-    const int c = 32 * (x >> 1) + 4 * (x & 1);
-    *reinterpret_cast<uint4*>(gv[0]) = ok0 ? ld_nc16(p.g + o0 + c) : make_uint4(0, 0, 0, 0);
-    *reinterpret_cast<uint4*>(gv[1]) = ok1 ? ld_nc16(p.g + o1 + c) : make_uint4(0, 0, 0, 0);
-    kv[0] = ok0 ? ld_nc8(p.k + o0 + c) : make_uint2(0, 0); kv[1] = ok1 ? ld_nc8(p.k + o1 + c) : make_uint2(0, 0);
-    qv[0] = ok0 ? ld_nc8(p.q + o0 + c) : make_uint2(0, 0); qv[1] = ok1 ? ld_nc8(p.q + o1 + c) : make_uint2(0, 0);
-  };
-  float qkd[2], rq[2], rk[2];                                                      // normalised q . k, and 1 / |q|, 1 / |k|, of the two tokens
+  // ---- raw rows (bf16) through shared memory: 1 / |k|, 1 / |q| and q . k are diagonals of products
   {
-    float sq[2] = {0.f, 0.f}, sk[2] = {0.f, 0.f}, dd[2] = {0.f, 0.f};
-    uint32_t kr[4][2][4], qr[4][2][4];
+    const size_t base = tok * KD + (size_t)(16 * warp) * ts;
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
-      *reinterpret_cast<uint4*>(kr[m][0]) = ok0 ? ld_nc16(p.k + o0 + 32 * m) : make_uint4(0, 0, 0, 0);
-      *reinterpret_cast<uint4*>(kr[m][1]) = ok1 ? ld_nc16(p.k + o1 + 32 * m) : make_uint4(0, 0, 0, 0);
-      *reinterpret_cast<uint4*>(qr[m][0]) = ok0 ? ld_nc16(p.q + o0 + 32 * m) : make_uint4(0, 0, 0, 0);
-      *reinterpret_cast<uint4*>(qr[m][1]) = ok1 ? ld_nc16(p.q + o1 + 32 * m) : make_uint4(0, 0, 0, 0);
-    }
-#pragma unroll
-    for (int m = 0; m < 4; ++m)
-#pragma unroll
-      for (int u = 0; u < 2; ++u)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float k0 = bf16_lo(kr[m][u][j]), k1 = bf16_hi(kr[m][u][j]), q0 = bf16_lo(qr[m][u][j]), q1 = bf16_hi(qr[m][u][j]);
-          sk[u] = fmaf(k0, k0, sk[u]); sk[u] = fmaf(k1, k1, sk[u]);
-          sq[u] = fmaf(q0, q0, sq[u]); sq[u] = fmaf(q1, q1, sq[u]);
-          dd[u] = fmaf(q0, k0, dd[u]); dd[u] = fmaf(q1, k1, dd[u]);
-        }
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-#pragma unroll
-      for (int o = 1; o <= 2; o <<= 1) {
-        sq[u] += __shfl_xor_sync(0xffffffffu, sq[u], o);
-        sk[u] += __shfl_xor_sync(0xffffffffu, sk[u], o);
-        dd[u] += __shfl_xor_sync(0xffffffffu, dd[u], o);
-      }
-      rq[u] = p.l2norm ? rsqrtf(sq[u] + 1e-6f) : 1.f;
-      rk[u] = p.l2norm ? rsqrtf(sk[u] + 1e-6f) : 1.f;
-      qkd[u] = rq[u] * rk[u] * dd[u];
+    for (int i = 0; i < 8; ++i) {
+      const int r = 2 * i + (lane >> 4), c = lane & 15;
+      const bool ok = r < nrow;
+      const uint4 kv = ok ? ld_nc16(p.k + base + r * ts + 8 * c) : make_uint4(0, 0, 0, 0), qv = ok ? ld_nc16(p.q + base + r * ts + 8 * c) : make_uint4(0, 0, 0, 0);
+      *reinterpret_cast<uint4*>(sm.pk[warp] + r * KI_LD + 16 * c) = kv;
+      *reinterpret_cast<uint4*>(sm.pq[warp] + r * KI_LD + 16 * c) = qv;
     }
   }
+  __syncwarp();
+  {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      float ck[4] = {0.f, 0.f, 0.f, 0.f}, cq[4] = {0.f, 0.f, 0.f, 0.f};            // {k; q} k^T, {k; q} q^T
+#pragma unroll
+      for (int ks = 0; ks < 8; ++ks) {
+        uint32_t a[4];
+        ldmatrix_x4(a, s_kq + (8 * u + (lane & 7)) * KI_LD + 32 * ks + 16 * (lane >> 4));
+        mma_bf16(ck, a, a[0], a[2]);
+        mma_bf16(cq, a, a[1], a[3]);
+      }
+      if ((g8 >> 1) == t4) {                                                       // the lane with column g8
+        const float kk = (g8 & 1) ? ck[1] : ck[0], qk = (g8 & 1) ? ck[3] : ck[2], qq = (g8 & 1) ? cq[3] : cq[2];
+        const float rk = p.l2norm ? rsqrtf(kk + 1e-6f) : 1.f, rq = p.l2norm ? rsqrtf(qq + 1e-6f) : 1.f;
+        sm.nrm[warp][0][8 * u + g8] = rk; sm.nrm[warp][1][8 * u + g8] = rq; sm.nrm[warp][2][8 * u + g8] = rk * rq * qk;
+      }
+    }
+  }
+  __syncwarp();
 
-  load(0);
-  // ---- in-block levels, 16 channels (a half run of every lane) at a time.  lv[s][octet]: {kk(g8, 2 t4), kk(g8, 2 t4 + 1), qk.., qk..} of levels 1, 2, 4;
+  // ---- in-block levels, 64 channels at a time.  lv[s][octet]: {kk(g8, 2 t4), kk(g8, 2 t4 + 1), qk.., qk..} of levels 1, 2, 4;
   //      l8: rows 8 + g8 against columns 2 t4, 2 t4 + 1
   float lv[3][2][4], l8[4];
 #pragma unroll
@@ -238,62 +235,100 @@ __global__ void __launch_bounds__(KI_THREADS, 3) kda_intra_kernel(const KdaIntra
 #pragma unroll
     for (int u = 0; u < 2; ++u) { lv[s][u][0] = lv[s][u][1] = lv[s][u][2] = lv[s][u][3] = 0.f; }
   l8[0] = l8[1] = l8[2] = l8[3] = 0.f;
-#pragma unroll 1
-  for (int x = 0; x < 8; ++x) {
-    float pre[2][4], suf[2][4], tt[2][4];
+  uint32_t sh[16];                                                                 // k suf of the first 64 channels
+  const uint32_t s_lv = s_suf + ((lane & 8) ? 16 * KI_LV : 0) + (lane & 7) * KI_LV + 16 * (lane >> 4);   // level images: k rows, then q rows
 #pragma unroll
-    for (int u = 0; u < 2; ++u)
+  for (int hf = 0; hf < 2; ++hf) {
+    uint64_t pre[16], suf[16];                                                     // fp32 pairs: the lane's two channels
+    uint32_t kh[16], qh[16];                                                       // normalised, fp16 pairs
+    {
+      const float* gp = p.g + tok * KD + (size_t)(16 * warp) * ts + 64 * hf + 2 * lane;
+      uint2 gv[16];
+#pragma unroll
+      for (int t = 0; t < 16; ++t) gv[t] = t < nrow ? ld_nc8(gp + t * ts) : make_uint2(0, 0);
+#pragma unroll
+      for (int t = 0; t < 16; ++t) {
+        pre[t] = pack2f(fast_exp2(__uint_as_float(gv[t].x) * 1.4426950408889634f), fast_exp2(__uint_as_float(gv[t].y) * 1.4426950408889634f));
+        suf[t] = pack2f(1.f, 1.f);
+      }
+    }
+#pragma unroll
+    for (int t4_ = 0; t4_ < 16; t4_ += 4) {
+      float rk[4], rq[4];
+      *reinterpret_cast<float4*>(rk) = *reinterpret_cast<const float4*>(&sm.nrm[warp][0][t4_]);
+      *reinterpret_cast<float4*>(rq) = *reinterpret_cast<const float4*>(&sm.nrm[warp][1][t4_]);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const float d = fast_exp2(gv[u][e] * 1.4426950408889634f);
-        pre[u][e] = d; tt[u][e] = d; suf[u][e] = 1.f;
+        const int t = t4_ + e;
+        const uint32_t off = t * KI_LD + 128 * hf + 4 * lane;
+        const uint32_t kr = *reinterpret_cast<const uint32_t*>(sm.pk[warp] + off), qr = *reinterpret_cast<const uint32_t*>(sm.pq[warp] + off);
+        kh[t] = pack_h2(bf16_lo(kr) * rk[e], bf16_hi(kr) * rk[e]);
+        qh[t] = pack_h2(bf16_lo(qr) * rq[e], bf16_hi(qr) * rq[e]);
       }
-    uint32_t kh[2][2], qh[2][2];                                                   // normalised, fp16
-    float kf[2][4], qf[2][4];
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      kf[u][0] = bf16_lo(kv[u].x) * rk[u]; kf[u][1] = bf16_hi(kv[u].x) * rk[u]; kf[u][2] = bf16_lo(kv[u].y) * rk[u]; kf[u][3] = bf16_hi(kv[u].y) * rk[u];
-      qf[u][0] = bf16_lo(qv[u].x) * rq[u]; qf[u][1] = bf16_hi(qv[u].x) * rq[u]; qf[u][2] = bf16_lo(qv[u].y) * rq[u]; qf[u][3] = bf16_hi(qv[u].y) * rq[u];
-#pragma unroll
-      for (int j = 0; j < 2; ++j) { kh[u][j] = pack_h2(kf[u][2 * j], kf[u][2 * j + 1]); qh[u][j] = pack_h2(qf[u][2 * j], qf[u][2 * j + 1]); }
     }
-    if (x < 7) load(x + 1);
+    auto level = [&](auto S) {                                                     // S = 1, 2, 4, 8
+      constexpr int s = decltype(S)::value;
+      __syncwarp();                                                                // the previous level's fragments are loaded
 #pragma unroll
-    for (int s = 0; s < 3; ++s) {                                                  // levels 1, 2, 4: the partner is lane ^ (4 << s)
-      const bool up = (g8 >> s) & 1;
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const uint32_t f0 = pack_h2(up ? pre[u][0] : suf[u][0], up ? pre[u][1] : suf[u][1]), f1 = pack_h2(up ? pre[u][2] : suf[u][2], up ? pre[u][3] : suf[u][3]);
-        const uint32_t k0 = hmul2_u32(kh[u][0], f0), k1 = hmul2_u32(kh[u][1], f1);
-        const uint32_t a[4] = {k0, hmul2_u32(qh[u][0], f0), k1, hmul2_u32(qh[u][1], f1)};
-        mma_f16(lv[s][u], a, k0, k1);
+      for (int t = 0; t < 16; ++t) {
+        float f0, f1;
+        unpack2f((t & s) ? pre[t] : suf[t], f0, f1);
+        const uint32_t f = pack_h2(f0, f1), off = t * KI_LV + 4 * lane;
+        *reinterpret_cast<uint32_t*>(sm.suf[warp] + off) = hmul2_u32(kh[t], f);
+        if (t & s) *reinterpret_cast<uint32_t*>(sm.suf[warp] + 16 * KI_LV + off) = hmul2_u32(qh[t], f);   // (lower tokens' results are not used)
       }
+      __syncwarp();
 #pragma unroll
-      for (int u = 0; u < 2; ++u)
+      for (int ks = 0; ks < 4; ++ks) {
+        if (s < 8) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float o = __shfl_xor_sync(0xffffffffu, tt[u][e], 4 << s);
-          if (up) pre[u][e] *= o; else suf[u][e] *= o;
-          tt[u][e] *= o;
+          for (int u = 0; u < 2; ++u) {
+            uint32_t a[4];
+            ldmatrix_x4(a, s_lv + 8 * u * KI_LV + 32 * ks);
+            mma_f16(lv[s == 1 ? 0 : s == 2 ? 1 : 2][u], a, a[0], a[2]);
+          }
+        } else {
+          uint32_t a[4], c[4];
+          ldmatrix_x4(a, s_lv + 8 * KI_LV + 32 * ks);
+          ldmatrix_x4(c, s_lv + 32 * ks);
+          mma_f16(l8, a, c[0], c[2]);
         }
-    }
-    {                                                                              // level 8: the two octets
-      const uint32_t fu0 = pack_h2(pre[1][0], pre[1][1]), fu1 = pack_h2(pre[1][2], pre[1][3]);
-      const uint32_t a[4] = {hmul2_u32(kh[1][0], fu0), hmul2_u32(qh[1][0], fu0), hmul2_u32(kh[1][1], fu1), hmul2_u32(qh[1][1], fu1)};
-      mma_f16(l8, a, hmul2_u32(kh[0][0], pack_h2(suf[0][0], suf[0][1])), hmul2_u32(kh[0][1], pack_h2(suf[0][2], suf[0][3])));
+      }
+      // both products from aligned blocks of s to blocks of 2 s: upper block: prefix times the lower block's total; lower block:
+      // suffix times the upper block's total
 #pragma unroll
-      for (int e = 0; e < 4; ++e) { pre[1][e] *= tt[0][e]; suf[0][e] *= tt[1][e]; }
-    }
-    // the block's images
+      for (int a = 0; a < 16; a += 2 * s) {
+        const uint64_t tl = pre[a + s - 1], tu = pre[a + 2 * s - 1];
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      sm.suf[warp][2 * x + u][lane] = make_uint2(pack_h2(kf[u][0] * suf[u][0], kf[u][1] * suf[u][1]), pack_h2(kf[u][2] * suf[u][2], kf[u][3] * suf[u][3]));
-      sm.pk[warp][2 * x + u][lane] = make_uint2(pack_h2(kf[u][0] * pre[u][0], kf[u][1] * pre[u][1]), pack_h2(kf[u][2] * pre[u][2], kf[u][3] * pre[u][3]));
-      sm.pq[warp][2 * x + u][lane] = make_uint2(pack_h2(qf[u][0] * pre[u][0], qf[u][1] * pre[u][1]), pack_h2(qf[u][2] * pre[u][2], qf[u][3] * pre[u][3]));
+        for (int i = 0; i < s; ++i) { pre[a + s + i] = fmul2(pre[a + s + i], tl); suf[a + i] = fmul2(suf[a + i], tu); }
+      }
+    };
+    level(std::integral_constant<int, 1>{});
+    level(std::integral_constant<int, 2>{});
+    level(std::integral_constant<int, 4>{});
+    level(std::integral_constant<int, 8>{});
+    __syncwarp();
+    // the block's images, from the unrounded rows
+#pragma unroll
+    for (int t = 0; t < 16; ++t) {
+      const float rk = sm.nrm[warp][0][t], rq = sm.nrm[warp][1][t];
+      const uint32_t off = t * KI_LD + 128 * hf + 4 * lane;
+      const uint32_t kr = *reinterpret_cast<const uint32_t*>(sm.pk[warp] + off), qr = *reinterpret_cast<const uint32_t*>(sm.pq[warp] + off);
+      const uint64_t kf = pack2f(bf16_lo(kr) * rk, bf16_hi(kr) * rk), qf = pack2f(bf16_lo(qr) * rq, bf16_hi(qr) * rq);
+      *reinterpret_cast<uint32_t*>(sm.pk[warp] + off) = pack_h2(fmul2(kf, pre[t]));
+      *reinterpret_cast<uint32_t*>(sm.pq[warp] + off) = pack_h2(fmul2(qf, pre[t]));
+      const uint32_t ks = pack_h2(fmul2(kf, suf[t]));
+      if (hf == 0) sh[t] = ks;
+      else {
+        *reinterpret_cast<uint32_t*>(sm.suf[warp] + off - 128) = sh[t];
+        *reinterpret_cast<uint32_t*>(sm.suf[warp] + off) = ks;
+      }
     }
-    if (g8 == 0)
-      *reinterpret_cast<float4*>(&sm.tot[warp][32 * (x >> 1) + 8 * t4 + 4 * (x & 1)]) = make_float4(tt[0][0] * tt[1][0], tt[0][1] * tt[1][1], tt[0][2] * tt[1][2], tt[0][3] * tt[1][3]);
+    float d0, d1;
+    unpack2f(pre[15], d0, d1);
+    *reinterpret_cast<float2*>(&sm.tot[warp][64 * hf + 2 * lane]) = make_float2(d0, d1);
   }
+  __syncwarp();
   __syncthreads();
 
   // ---- products with the earlier blocks
@@ -303,23 +338,27 @@ __global__ void __launch_bounds__(KI_THREADS, 3) kda_intra_kernel(const KdaIntra
     float kk[2][4], qk[2][4];
 #pragma unroll
     for (int n = 0; n < 2; ++n) { kk[n][0] = kk[n][1] = kk[n][2] = kk[n][3] = 0.f; qk[n][0] = qk[n][1] = qk[n][2] = qk[n][3] = 0.f; }
+    const uint32_t s_c = smem_u32(sm.suf[J]) + ((lane & 7) + 8 * (lane >> 4)) * KI_LD + 16 * ((lane >> 3) & 1);
+    const uint32_t ao = ((lane & 7) + 8 * ((lane >> 3) & 1)) * KI_LD + 16 * (lane >> 4);
 #pragma unroll 2
-    for (int x = 0; x < 8; ++x) {
-      uint2 c[2], kr[2], qr[2];
-#pragma unroll
-      for (int u = 0; u < 2; ++u) { c[u] = sm.suf[J][2 * x + u][lane]; kr[u] = sm.pk[warp][2 * x + u][lane]; qr[u] = sm.pq[warp][2 * x + u][lane]; }
+    for (int ks = 0; ks < 8; ++ks) {
+      uint32_t c[4], kr[4], qr[4];
+      ldmatrix_x4(c, s_c + 32 * ks);
+      ldmatrix_x4(kr, s_pk + ao + 32 * ks);
+      ldmatrix_x4(qr, s_pq + ao + 32 * ks);
       if (J < warp - 1) {                                                          // blocks lie between: their totals
-        const int ch = 32 * (x >> 1) + 8 * t4 + 4 * (x & 1);
-        float4 f = *reinterpret_cast<const float4*>(&sm.tot[J + 1][ch]);
-        if (J < warp - 2) f = ki_mul4(f, &sm.tot[J + 2][ch]);
+        float2 f0 = *reinterpret_cast<const float2*>(&sm.tot[J + 1][16 * ks + 2 * t4]), f1 = *reinterpret_cast<const float2*>(&sm.tot[J + 1][16 * ks + 8 + 2 * t4]);
+        if (J < warp - 2) {
+          const float2 e0 = *reinterpret_cast<const float2*>(&sm.tot[J + 2][16 * ks + 2 * t4]), e1 = *reinterpret_cast<const float2*>(&sm.tot[J + 2][16 * ks + 8 + 2 * t4]);
+          f0.x *= e0.x; f0.y *= e0.y; f1.x *= e1.x; f1.y *= e1.y;
+        }
 #pragma unroll
-        for (int u = 0; u < 2; ++u) { kr[u] = ki_scale(kr[u], f); qr[u] = ki_scale(qr[u], f); }
+        for (int i = 0; i < 4; ++i) { kr[i] = ki_scale(kr[i], i < 2 ? f0 : f1); qr[i] = ki_scale(qr[i], i < 2 ? f0 : f1); }
       }
-      const uint32_t ak[4] = {kr[0].x, kr[1].x, kr[0].y, kr[1].y}, aq[4] = {qr[0].x, qr[1].x, qr[0].y, qr[1].y};
 #pragma unroll
       for (int n = 0; n < 2; ++n) {
-        mma_f16(kk[n], ak, c[n].x, c[n].y);
-        mma_f16(qk[n], aq, c[n].x, c[n].y);
+        mma_f16(kk[n], kr, c[2 * n], c[2 * n + 1]);
+        mma_f16(qk[n], qr, c[2 * n], c[2 * n + 1]);
       }
     }
 #pragma unroll
@@ -345,7 +384,7 @@ __global__ void __launch_bounds__(KI_THREADS, 3) kda_intra_kernel(const KdaIntra
         const float c = x >= 4 ? lv[2][u][2 + e] : x >= 2 ? lv[1][u][2 + e] : lv[0][u][2 + e];
         const bool low = jc + e < g8;
         kk[e] = low ? (u ? b1 : b0) * a : 0.f;
-        qk[e] = p.scale * (low ? c : jc + e == g8 ? qkd[u] : 0.f);                 // the diagonal: q_i . k_i, no decay
+        qk[e] = p.scale * (low ? c : jc + e == g8 ? sm.nrm[warp][2][8 * u + g8] : 0.f);                 // the diagonal: q_i . k_i, no decay
         sm.dg[warp][8 * u + jc + e][8 * u + g8] = kk[e];
       }
       *reinterpret_cast<uint32_t*>(rec + OFF_AQK + rec_off(16 * warp + 8 * u + g8, 16 * warp + 8 * u + jc)) = pack_h2(qk[0], qk[1]);
@@ -374,43 +413,47 @@ __global__ void __launch_bounds__(KI_THREADS, 3) kda_intra_kernel(const KdaIntra
   }
 
   // ---- state-pass operands: k e^G (shared memory), q e^G scale and k e^{G_C - G} (record)
-  uint8_t *xt = reinterpret_cast<uint8_t*>(sm.pk), *vt = reinterpret_cast<uint8_t*>(sm.pq);
   {
-    uint2 qr[16];                                                                  // all of this warp's q pre, then v may take its place
+    const int c = lane & 15;                                                       // this lane's eight channels, in every other row
+    float f[8], s[8];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) qr[i] = sm.pq[warp][i][lane];
-    __syncwarp();
-    const uint32_t vb = smem_u32(vt);
+    for (int e = 0; e < 8; ++e) { f[e] = 1.f; s[e] = 1.f; }
+    for (int K = 0; K < 4; ++K) {
+      if (K == warp) continue;
+      const float4 lo = *reinterpret_cast<const float4*>(&sm.tot[K][8 * c]), hi = *reinterpret_cast<const float4*>(&sm.tot[K][8 * c + 4]);
+      const float t[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+      for (int e = 0; e < 8; ++e) { f[e] *= K < warp ? t[e] : 1.f; s[e] *= K < warp ? 1.f : t[e]; }
+    }
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const int r = 16 * warp + 2 * i + (lane >> 4), c = lane & 15;
-      const uint32_t n = r < rows ? 16u : 0u;                                      // rows past the end: zeros
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(vb + ki_off(r, c)), "l"(p.v + tok * KD + (size_t)(r < rows ? r : 0) * ts + 8 * c), "r"(n) : "memory");
+      const int r = 2 * i + (lane >> 4);
+      const uint32_t off = r * KI_LD + 16 * c, roff = 4096 * warp + ki_off(r, c);
+      uint32_t q[4], k[4], z[4];
+      *reinterpret_cast<uint4*>(q) = *reinterpret_cast<const uint4*>(sm.pq[warp] + off);
+      *reinterpret_cast<uint4*>(k) = *reinterpret_cast<const uint4*>(sm.pk[warp] + off);
+      *reinterpret_cast<uint4*>(z) = *reinterpret_cast<const uint4*>(sm.suf[warp] + off);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 fj = make_float2(f[2 * j], f[2 * j + 1]);
+        k[j] = ki_scale(k[j], fj);
+        q[j] = ki_scale(q[j], make_float2(fj.x * p.scale, fj.y * p.scale));
+        z[j] = ki_scale(z[j], make_float2(s[2 * j], s[2 * j + 1]));
+      }
+      *reinterpret_cast<uint4*>(sm.pk[warp] + off) = *reinterpret_cast<const uint4*>(k);
+      st_global16(rec + OFF_QT + roff, q[0], q[1], q[2], q[3]);
+      st_global16(rec + OFF_KT + roff, z[0], z[1], z[2], z[3]);
+    }
+    __syncwarp();
+    const uint32_t vb = s_pq;                                                      // v takes the place of q pre
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int r = 2 * i + (lane >> 4);
+      const uint32_t n = r < nrow ? 16u : 0u;                                      // rows past the end: zeros
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                   ::"r"(vb + r * KI_LD + 16 * c), "l"(p.v + tok * KD + (size_t)(r < nrow ? 16 * warp + r : 0) * ts + 8 * c), "r"(n) : "memory");
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
-    uint2 kr[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) kr[i] = sm.pk[warp][i][lane];
-    __syncwarp();
-#pragma unroll
-    for (int m = 0; m < 4; ++m) {
-      const int ch = 32 * m + 8 * t4;
-      float4 f0 = make_float4(1.f, 1.f, 1.f, 1.f), f1 = f0, s0 = f0, s1 = f0;
-      for (int K = 0; K < warp; ++K) { f0 = ki_mul4(f0, &sm.tot[K][ch]); f1 = ki_mul4(f1, &sm.tot[K][ch + 4]); }
-      for (int K = warp + 1; K < 4; ++K) { s0 = ki_mul4(s0, &sm.tot[K][ch]); s1 = ki_mul4(s1, &sm.tot[K][ch + 4]); }
-      const float4 g0 = make_float4(f0.x * p.scale, f0.y * p.scale, f0.z * p.scale, f0.w * p.scale);
-      const float4 g1 = make_float4(f1.x * p.scale, f1.y * p.scale, f1.z * p.scale, f1.w * p.scale);
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const uint32_t off = ki_off(u ? r1 : r0, 4 * m + t4);
-        const uint2 x0 = ki_scale(kr[4 * m + u], f0), x1 = ki_scale(kr[4 * m + 2 + u], f1);
-        const uint2 q0 = ki_scale(qr[4 * m + u], g0), q1 = ki_scale(qr[4 * m + 2 + u], g1);
-        const uint2 k0 = ki_scale(sm.suf[warp][4 * m + u][lane], s0), k1 = ki_scale(sm.suf[warp][4 * m + 2 + u][lane], s1);
-        *reinterpret_cast<uint4*>(xt + off) = make_uint4(x0.x, x0.y, x1.x, x1.y);
-        st_global16(rec + OFF_QT + off, q0.x, q0.y, q1.x, q1.y);
-        st_global16(rec + OFF_KT + off, k0.x, k0.y, k1.x, k1.y);
-      }
-    }
   }
   reinterpret_cast<float*>(rec + OFF_D)[tid] = (sm.tot[0][tid] * sm.tot[1][tid]) * (sm.tot[2][tid] * sm.tot[3][tid]);   // e^{G_C}
   asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -425,9 +468,9 @@ __global__ void __launch_bounds__(KI_THREADS, 3) kda_intra_kernel(const KdaIntra
   //      that follow.  The four row tiles of a warp are independent chains issued side by side.
   {
     const bool is_w = warp < 2;
-    const uint32_t src = smem_u32(is_w ? xt : vt);
     uint8_t* dst = rec + (is_w ? OFF_WT : OFF_UT);
     const int c0 = 64 * (warp & 1);                                                // first row (channel or value column)
+    const uint32_t src = smem_u32(is_w ? sm.pk : sm.pq) + ((lane & 7) + 8 * (lane >> 4)) * KI_LD + 2 * c0 + 16 * ((lane >> 3) & 1);
     uint32_t zf[4][3][4];                                                          // Z_J as fp16 A fragments: [row tile][J][4]
 #pragma unroll
     for (int I = 0; I < 4; ++I) {
@@ -458,8 +501,7 @@ __global__ void __launch_bounds__(KI_THREADS, 3) kda_intra_kernel(const KdaIntra
         // right-hand side: tokens 16 I .. + 15 x rows c0 + 16 m .. + 15, transposed: register i = (tokens 8 (i >> 1) + 2 t4 (+1),
         // row 8 (i & 1) + g8)
         uint32_t rr[4];
-        const int row = I * 16 + (lane & 7) + 8 * (lane >> 4), pc = (c0 >> 3) + 2 * m + ((lane >> 3) & 1);
-        ldmatrix_x4_t(rr, src + ki_off(row, pc));
+        ldmatrix_x4_t(rr, src + I * (16 * KI_LD) + 32 * m);
         uint32_t a[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {

@@ -188,10 +188,10 @@ class B200CausalSelfAttention(nn.Module):
 
     # ------------------------------------------------------------------ helpers
     def _linear(self, x: Tensor, w: Tensor) -> Tensor:
-        """``F.linear(x, w)`` on this library's kernels: the weight-streaming one for the few rows of a decode step,
-        the tcgen05 GEMM otherwise."""
+        """``F.linear(x, w)`` on this library's kernels: the weight-streaming one for up to 8 rows (one pass of its
+        register tile), the tcgen05 GEMM otherwise (64 rows, 2048 to 6144 columns: 8.6 us against 110)."""
         rows = x.numel() // x.size(-1)
-        return ops.gemm_skinny(x, w) if rows <= 64 else ops.gemm_nt(x, w)
+        return ops.gemm_skinny(x, w) if rows <= 8 else ops.gemm_nt(x, w)
 
     def _project(self, x: Tensor):
         self._no_autograd(x)
@@ -354,7 +354,7 @@ class B200CausalSelfAttention(nn.Module):
             return self._token_call(x, kr, vr, 0, cache.t_dev, self.rotary.cos, self.rotary.sin, ve, window, write_ring,
                                     None, None, self._token_ws)
         w = self.qkvo_w.detach()
-        qkv = ops.gemm_skinny(x.detach().to(w.dtype).view(B, self.m_dim), w[:3].flatten(end_dim=1)).view(B, 1, 3 * H, D)
+        qkv = self._linear(x.detach().to(w.dtype).view(B, self.m_dim), w[:3].flatten(end_dim=1)).view(B, 1, 3 * H, D)
         q, k, v = qkv[:, :, :H], qkv[:, :, H:2 * H], qkv[:, :, 2 * H:]
         kr, vr = cache.ring(layer)
         ve_kw = {}
@@ -370,7 +370,7 @@ class B200CausalSelfAttention(nn.Module):
         y = ops.swa_decode_step_fused(q, k, v, kr, vr, cache.t_dev, cache.W, window, self.rotary.cos, self.rotary.sin,
                                       self.attn_scale, self.norm_eps, QKV_DEFAULT, write_ring=write_ring,
                                       splits=self._fused_splits, workspace=self._fused_ws, **ve_kw)
-        return ops.gemm_skinny(y.view(B, self.m_dim), w[3]).view(B, 1, self.m_dim)
+        return self._linear(y.view(B, self.m_dim), w[3]).view(B, 1, self.m_dim)
 
     def _token_call(self, x, kc, vc, t, t_dev, cos, sin, ve, window, write_ring, k_new, v_new, workspace):
         gate = None

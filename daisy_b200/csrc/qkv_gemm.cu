@@ -26,6 +26,7 @@ namespace daisy {
 
 constexpr int GM = 128, GK = 64;
 constexpr int G_THREADS = 192;
+constexpr int G_SMALL_THREADS = 192;                   // 4 epilogue warps, TMA warp, MMA warp
 constexpr int G_A_BYTES = GM * GK * 2;                 // 16 KB
 constexpr int G_STAGE_ROW = 256 + 16;                  // one staged output row (128 bf16) + pad: conflict-free 16-byte accesses
 constexpr int G_STAGING = 4 * 16 * G_STAGE_ROW;        // per warp 16 rows at a time
@@ -303,6 +304,222 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
   }
 }
 
+
+// ---------------------------------------------------------------------- few rows, or few columns
+// One tile of at most 128 rows x BN columns per CTA, up to two CTAs to an SM: what these sizes need is the whole chip
+// pulling operands, not products per byte.  In the QKV form (BN = 64) a cluster of two CTAs shares a head: CTA r holds the
+// head's channels c0 .. c0 + 31 and their rotation partners 64 + c0 .., c0 = 32 r, so RoPE stays inside a thread and only
+// each row's sum of squares travels (one float per row and CTA, through the cluster's shared memory).
+// Launched as a dependent grid: barriers, TMEM and the hint that brings the weights into L2 come before the wait.
+// Bound by latency: launch, first operands, epilogue.  131 x 2304 x 768 with norm and RoPE 17.0 us as one 256 x 256 tile per
+// CTA pair, 11.1 as 128 x 128 tiles, 5.9 here; 64 x 6144 x 2048 (25 MB of weights) 110 us in the row-by-row kernel, 8.6 here.
+// (A head cut in four, BN = 32, costs more in the exchange than it gains: 9.8 us.)
+template <int BN>
+struct SmallCfg {
+  static constexpr int STAGE = G_A_BYTES + BN * GK * 2;
+  static constexpr int MAX_NST = 220 * 1024 / STAGE < 12 ? 220 * 1024 / STAGE : 12;      // alone on its SM
+  static constexpr int HALF_NST = 106 * 1024 / STAGE;                                    // two CTAs to an SM
+  static constexpr int RANKS = 128 / BN;                                                 // QKV: CTAs to a head
+  static constexpr int SMEM0 = 1024 + 1024 + 256;
+};
+struct SmallBars {
+  uint64_t full[12], empty[12], acc_full;
+  uint32_t tmem_base;
+  int abort_flag;
+};
+
+template <int BN, bool QKV>
+__global__ void __launch_bounds__(G_SMALL_THREADS, 2)
+small_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w, const GemmParams p, const int nst,
+                  const int tm, const __nv_bfloat16* w, const int64_t ldw, const int prefetch) {
+  using Cfg = SmallCfg<BN>;
+  static_assert(!QKV || BN == 64, "two CTAs to a head");
+  constexpr int HB = BN / 2;
+  extern __shared__ uint8_t gemm_smem_raw[];
+  uint8_t* stages = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(gemm_smem_raw) + 1023) & ~uintptr_t(1023));
+  float* part = reinterpret_cast<float*>(stages + nst * Cfg::STAGE);                     // [rank][row]: sums of squares
+  SmallBars* bars = reinterpret_cast<SmallBars*>(part + 2 * 128);
+  volatile int* abort_flag = &bars->abort_flag;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, kb_n = p.K / GK;
+  const int nx = p.N / BN, bn = (int)blockIdx.x % nx, bm = (int)blockIdx.x / nx;
+  const int rank = QKV ? bn % Cfg::RANKS : 0;
+  const int nh = bn / Cfg::RANKS;                                                        // QKV: head slot among 3 H
+  const int c0 = rank * HB;                                                              // and this CTA's channels of it
+  const int m0 = bm * tm;                                                                // tm <= 128 rows of X a tile, a multiple of 8
+  const int w_lo = QKV ? nh * 128 + c0 : bn * BN, w_hi = QKV ? w_lo + 64 : w_lo + HB;    // its weight rows: HB and HB
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < nst; ++i) { mbar_init(&bars->full[i], 1); mbar_init(&bars->empty[i], 1); }
+    mbar_init(&bars->acc_full, 1);
+    bars->abort_flag = 0;
+    mbar_init_fence();
+  }
+  if (warp == 5) {
+    tmem_alloc(&bars->tmem_base, BN);
+    tmem_relinquish();
+  } else if (prefetch && bm == 0 && threadIdx.x < BN) {
+    l2_prefetch_bulk(w + (int64_t)(threadIdx.x < HB ? w_lo + threadIdx.x : w_hi + (int)threadIdx.x - HB) * ldw, (uint32_t)p.K * 2u);
+  }
+  if (warp == 4 && lane == 0) { prefetch_tmap(&tm_x); prefetch_tmap(&tm_w); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (QKV) asm volatile("barrier.cluster.arrive.release;" ::: "memory");                 // (1) this CTA runs
+  const uint32_t tmem_base = bars->tmem_base;
+  grid_dep_launch();
+  grid_dep_wait();
+
+  if (warp < 5) {
+    // ------------------------------------------------------------------ TMA producers: a turn of the loop takes one thread some
+    // 450 cycles, so the epilogue's warps share it before the accumulator is theirs to read.  Never more producers than stages:
+    // a producer enters block kb after block kb - np's stage was free, so product kb - np - nst is done; with np <= nst that is
+    // no earlier than product kb - 2 nst, and the parity it waits for cannot be that of the round before the last.
+    const int np = min(5, nst);
+    if (lane == 0 && warp < np) {
+      for (int kb = warp; kb < kb_n; kb += np) {
+        const int st = kb % nst;
+        if (!mbar_wait(&bars->empty[st], ((kb / nst) & 1) ^ 1, abort_flag, p.status, 1)) break;
+        uint8_t* dst = stages + st * Cfg::STAGE;
+        mbar_expect_tx(&bars->full[st], tm * GK * 2 + BN * GK * 2);
+        tma_load_3d(dst + G_A_BYTES, &tm_w, &bars->full[st], kb * GK, w_lo, 0);
+        tma_load_3d(dst + G_A_BYTES + HB * GK * 2, &tm_w, &bars->full[st], kb * GK, w_hi, 0);
+        tma_load_3d(dst, &tm_x, &bars->full[st], kb * GK, m0, 0);
+      }
+    }
+    __syncwarp();
+  } else {
+    // ------------------------------------------------------------------ MMA issuer
+    const uint32_t leader = elect_one() ? 1u : 0u;
+    constexpr uint32_t idesc = umma_idesc_bf16(GM, BN, 0, 0);
+    const uint64_t ad = umma_desc_sw128(smem_u32(stages), 16, 1024);
+    const uint64_t bd = umma_desc_sw128(smem_u32(stages + G_A_BYTES), 16, 1024);
+    const uint32_t a_lo0 = (uint32_t)ad, b_lo0 = (uint32_t)bd, hi = (uint32_t)(ad >> 32);
+    bool ok = true;
+    for (int kb = 0, st = 0, ph = 0; kb < kb_n; ++kb) {
+      if (!mbar_wait(&bars->full[st], ph, abort_flag, p.status, 3)) { ok = false; break; }
+      tc_fence_after();
+      const uint32_t a_lo = a_lo0 + st * (Cfg::STAGE >> 4), b_lo = b_lo0 + st * (Cfg::STAGE >> 4);
+#pragma unroll
+      for (int k = 0; k < GK / 16; ++k) umma_ss_lh_p(leader, tmem_base, a_lo + k * 2, hi, b_lo + k * 2, hi, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+      tc_commit_p(leader, &bars->empty[st]);
+      if (++st == nst) { st = 0; ph ^= 1; }
+    }
+    if (ok) tc_commit_p(leader, &bars->acc_full);
+    __syncwarp();
+  }
+
+  if (warp < 4) {
+    // ------------------------------------------------------------------ epilogue: thread = output row, r[0 .. HB) low, r[HB ..) high columns
+    const int row = warp * 32 + lane, m = m0 + row;
+    const int which = nh / p.H, h = nh - which * p.H;                                    // QKV only
+    const bool rope = QKV && which < 2 && (p.flags & DAISY_ROPE);
+    float4 cs[HB / 4], sn[HB / 4];
+    if (rope) {                                                                          // rotations arrive under the products
+      const int pos = min(m, p.M - 1) % p.T;
+      const float4* cr = reinterpret_cast<const float4*>(p.cos + (size_t)pos * 64 + c0);
+      const float4* sr = reinterpret_cast<const float4*>(p.sin + (size_t)pos * 64 + c0);
+#pragma unroll
+      for (int i = 0; i < HB / 4; ++i) { cs[i] = cr[i]; sn[i] = sr[i]; }
+    }
+    const bool ok = __all_sync(0xffffffffu, mbar_wait(&bars->acc_full, 0, abort_flag, p.status, 4)), mine = ok && row < tm && m < p.M;
+    tc_fence_after();
+    uint32_t r[BN];
+    const uint32_t t0 = tmem_base + ((uint32_t)(warp * 32) << 16);
+#pragma unroll
+    for (int i = 0; i < BN / 32; ++i) tmem_ld32(t0 + 32 * i, r + 32 * i);
+    tc_wait_ld();
+    if (QKV) {
+      const bool do_norm = (p.flags & (which == 0 ? DAISY_NORM_Q : which == 1 ? DAISY_NORM_K : DAISY_NORM_V)) != 0;
+      float ss = 0.f;
+#pragma unroll
+      for (int i = 0; i < BN; ++i) { const float x = __uint_as_float(r[i]); ss = fmaf(x, x, ss); }
+      asm volatile("barrier.cluster.wait.acquire;" ::: "memory");                        // (1) both of the head's CTAs run
+#pragma unroll
+      for (int j = 0; j < Cfg::RANKS; ++j)
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(mapa_shared(smem_u32(part + rank * 128 + row), j)), "f"(ss) : "memory");
+      asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");   // (2)
+      ss = 0.f;
+#pragma unroll
+      for (int j = 0; j < Cfg::RANKS; ++j) ss += part[j * 128 + row];
+      if (do_norm) {
+        const float rs = rsqrtf(ss * (1.0f / 128.0f) + p.eps);
+        if (p.rstd && rank == 0 && mine) p.rstd[(size_t)m * (3 * p.H) + nh] = rs;
+#pragma unroll
+        for (int i = 0; i < BN; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * rs);
+      }
+      if (rope) {
+#pragma unroll
+        for (int i4 = 0; i4 < HB / 4; ++i4) {
+          const float cc[4] = {cs[i4].x, cs[i4].y, cs[i4].z, cs[i4].w}, sc[4] = {sn[i4].x, sn[i4].y, sn[i4].z, sn[i4].w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int i = 4 * i4 + e;
+            const float a = __uint_as_float(r[i]), b2 = __uint_as_float(r[i + HB]);
+            r[i] = __float_as_uint(a * cc[e] + b2 * sc[e]);
+            r[i + HB] = __float_as_uint(b2 * cc[e] - a * sc[e]);
+          }
+        }
+      }
+    }
+    if (mine) {
+      uint32_t hv[HB];                                                                   // bf16 pairs: HB / 2 low, HB / 2 high
+      const bool gated = QKV && which == 2 && p.ve;
+      // where the high columns follow the low ones, in 16-byte units
+      constexpr int HI = QKV ? 8 : HB / 8;
+      auto store = [&](void* at) {
+        uint4* d = reinterpret_cast<uint4*>(at);
+#pragma unroll
+        for (int i = 0; i < HB / 8; ++i) {
+          d[i] = make_uint4(hv[4 * i], hv[4 * i + 1], hv[4 * i + 2], hv[4 * i + 3]);
+          d[HI + i] = make_uint4(hv[HB / 2 + 4 * i], hv[HB / 2 + 4 * i + 1], hv[HB / 2 + 4 * i + 2], hv[HB / 2 + 4 * i + 3]);
+        }
+      };
+      if (gated) {                                                                       // value-embedding gate on the normalised v
+        if (p.vn) {
+#pragma unroll
+          for (int i = 0; i < HB; ++i) hv[i] = pack_bf16(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+          store(p.vn + ((size_t)m * p.H + h) * 128 + c0);
+        }
+        const float gte = 1.0f / (1.0f + __expf(-*p.ve_gate_logit));
+        const uint4* vr = reinterpret_cast<const uint4*>(p.ve + (size_t)m * p.ve_ld + h * 128 + c0);
+#pragma unroll
+        for (int c = 0; c < HB / 4; ++c) {
+          float f[8];
+          unpack8(c < HB / 8 ? vr[c] : vr[8 + c - HB / 8], f);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) r[8 * c + e] = __float_as_uint(gte * __uint_as_float(r[8 * c + e]) + (1.0f - gte) * f[e]);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < HB; ++i) hv[i] = pack_bf16(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+      store(QKV ? p.out[which] + ((size_t)m * p.H + h) * 128 + c0 : p.c + (size_t)m * p.ldc + w_lo);
+      if (QKV && which >= 1 && p.ring[which - 1]) {                                      // this row's slot in the ring cache, if it is kept
+        const int b = m / p.T, t = m - b * p.T;
+        if (t >= p.ring_first) {
+          if (p.ring_f16) {                                                              // the bf16 value as float16
+#pragma unroll
+            for (int i = 0; i < HB; ++i) {
+              const __half2 x = __floats2half2_rn(bf16_lo(hv[i]), bf16_hi(hv[i]));
+              hv[i] = *reinterpret_cast<const uint32_t*>(&x);
+            }
+          }
+          store(reinterpret_cast<__nv_bfloat16*>(p.ring[which - 1]) + (int64_t)b * p.r_sb + (int64_t)h * p.r_sh + (int64_t)(t % p.cap) * p.r_sr + c0);
+        }
+      }
+    }
+  } else if (QKV) {
+    asm volatile("barrier.cluster.wait.acquire;\n\tbarrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");   // (1), (2)
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 5) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, BN);
+  }
+}
+
 }  // namespace daisy
 
 using namespace daisy;
@@ -354,16 +571,75 @@ static int launch_gemm(const CUtensorMap& tx, const CUtensorMap& tw, const GemmP
   return DAISY_OK;
 }
 
+constexpr size_t G_PREFETCH_LIMIT = 48u << 20;          // weights up to this size are hinted into L2 ahead of the wait
+
+template <int BN, bool QKV>
+static int launch_small(const void* x, int64_t ldx, const void* w, int64_t ldw, const GemmParams& p, cudaStream_t st) {
+  using Cfg = SmallCfg<BN>;
+  auto kernel = small_gemm_kernel<BN, QKV>;
+  static bool attr[daisy_host::MAX_DEVICES] = {};
+  const int dev = daisy_host::device_slot();
+  if (dev < 0) return DAISY_ENODEV;
+  const int sms = daisy_host::sm_count_cached();
+  if (sms <= 0) return DAISY_ENODEV;
+  if (!attr[dev]) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM0 + Cfg::MAX_NST * Cfg::STAGE) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return DAISY_ECUDA;
+    }
+    attr[dev] = true;
+  }
+  // tiles of equal height: 131 rows are two tiles of 72, not one of 128 and one of 3
+  const int mt = (p.M - 1) / GM + 1, tm = ((p.M - 1) / mt + 8) & ~7;
+  CUtensorMap tx, tw;
+  int rc;
+  if ((rc = daisy_host::make_tmap_bf16_3d(&tx, x, p.K, p.M, 1, (uint64_t)ldx * 2, (uint64_t)ldx * 2 * p.M, GK, tm)) != DAISY_OK) return rc;
+  if ((rc = daisy_host::make_tmap_bf16_3d(&tw, w, p.K, p.N, 1, (uint64_t)ldw * 2, (uint64_t)ldw * 2 * p.N, GK, BN / 2)) != DAISY_OK) return rc;
+  const int tiles = mt * (p.N / BN);
+  int nst = tiles <= sms ? Cfg::MAX_NST : Cfg::HALF_NST;
+  if (nst > p.K / GK) nst = p.K / GK;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)tiles); cfg.blockDim = dim3(G_SMALL_THREADS); cfg.dynamicSmemBytes = Cfg::SMEM0 + nst * Cfg::STAGE; cfg.stream = st;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = Cfg::RANKS; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+  cfg.attrs = at; cfg.numAttrs = QKV ? 2 : 1;
+  if (cudaLaunchKernelEx(&cfg, kernel, tx, tw, p, nst, tm, (const __nv_bfloat16*)w, ldw, (size_t)p.N * p.K * 2 <= G_PREFETCH_LIMIT ? 1 : 0) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return DAISY_ECUDA;
+  }
+  DAISY_CHECK_LAUNCH();
+  return DAISY_OK;
+}
+
+// Which tile.  One wave of narrow tiles as long as they fit the chip (a second wave costs more than wider tiles do:
+// 2048 x 768 x 768 7.5 us in 128-column tiles, 8.4 in 64); from there 128 x 128 tiles against pairs on 256 x 256, whose
+// larger tiles want a large product.
+enum { TILE_32 = 32, TILE_64 = 64, TILE_128 = 128, TILE_PAIR = 256 };
+static int gemm_tile(const GemmParams& p, int sms) {
+  const int64_t mt = ((int64_t)p.M + GM - 1) / GM;
+  if (p.epi == 0 && mt * (p.N / 32) <= sms) return TILE_32;
+  if (mt * (p.N / 64) <= sms) return TILE_64;
+  return p.N % 256 == 0 && p.M > GM ? TILE_PAIR : TILE_128;
+}
+
 static int gemm_common(const void* x, int64_t ldx, const void* w, int64_t ldw, GemmParams& p, void* stream) {
   if (!x || !w || p.M <= 0 || p.N <= 0 || p.K <= 0) return DAISY_EINVAL;
   if (p.K % GK != 0 || p.N % 128 != 0) return DAISY_EUNSUPPORTED;
   if (!daisy_aligned16(x) || !daisy_aligned16(w) || (ldx & 7) || (ldw & 7) || ldx < p.K || ldw < p.K) return DAISY_EALIGN;
-  const bool pair = p.N % 256 == 0 && p.M > GM;        // CTA pairs on 256 x 256 tiles; else one CTA per 128 x 128 tile
+  const int sms = daisy_host::sm_count_cached();
+  if (sms <= 0) return DAISY_ENODEV;
+  cudaStream_t st = (cudaStream_t)stream;
+  const int tile = gemm_tile(p, sms);
+  if (tile == TILE_32) return launch_small<32, false>(x, ldx, w, ldw, p, st);
+  if (tile == TILE_64) return p.epi ? launch_small<64, true>(x, ldx, w, ldw, p, st) : launch_small<64, false>(x, ldx, w, ldw, p, st);
   CUtensorMap tx, tw;
   int rc;
   if ((rc = daisy_host::make_tmap_bf16_3d(&tx, x, p.K, p.M, 1, (uint64_t)ldx * 2, (uint64_t)ldx * 2 * p.M, GK, GM)) != DAISY_OK) return rc;
   if ((rc = daisy_host::make_tmap_bf16_3d(&tw, w, p.K, p.N, 1, (uint64_t)ldw * 2, (uint64_t)ldw * 2 * p.N, GK, 128)) != DAISY_OK) return rc;
-  return pair ? launch_gemm<256, true>(tx, tw, p, (cudaStream_t)stream) : launch_gemm<128, false>(tx, tw, p, (cudaStream_t)stream);
+  return tile == TILE_PAIR ? launch_gemm<256, true>(tx, tw, p, st) : launch_gemm<128, false>(tx, tw, p, st);
 }
 
 extern "C" int daisy_b200_gemm_nt(const void* x, int64_t ldx, const void* w, int64_t ldw, void* c, int64_t ldc,

@@ -95,6 +95,45 @@ def test_qkv_gemm_value_embedding_gate():
     assert_close_bf16(vp, ref, "ve gate in the epilogue")
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 128, 64), (8, 128, 128), (127, 256, 320), (129, 128, 832), (136, 640, 64), (640, 1024, 384), (592, 1024, 1600),
+                                   (1184, 1024, 384)])
+def test_gemm_small_tiles(M, N, K):
+    """One narrow tile per CTA: row counts around the 128-row tile and its equal division, one to many k-blocks (fewer than
+    producers, more than stages), the last sizes of 32 columns, of 64, and beyond."""
+    from daisy_b200 import ops
+    x = bf16_randn(M, K, seed=M)
+    w = bf16_randn(N, K, seed=N + K) * (K ** -0.5)
+    c = ops.gemm_nt(x, w)
+    ops.check_device_status(x.device)
+    assert_close_bf16(c, x.float().cpu() @ w.float().cpu().t(), f"gemm {M}x{N}x{K}")
+
+
+@pytest.mark.parametrize("B,T,H,dim", [(1, 1, 1, 64), (3, 43, 2, 320), (1, 128, 3, 832), (2, 200, 6, 768)])
+@pytest.mark.parametrize("f16", [False, True])
+def test_qkv_gemm_small_tiles_ring(B, T, H, dim, f16):
+    """A head shared by the two CTAs of a cluster: norm, RoPE, value gate and the rows kept in the ring."""
+    from daisy_b200 import ops
+    D, cap = 128, 50
+    x = bf16_randn(B, T, dim, seed=T)
+    w = bf16_randn(3 * H * D, dim, seed=dim) * (dim ** -0.5)
+    ve = bf16_randn(B, T, H * D, seed=5)
+    logit = torch.tensor([0.4], device="cuda")
+    cos, sin = swa.rope_tables(D, T)
+    ring = [torch.zeros(B, H, cap, D, dtype=torch.float16 if f16 else torch.bfloat16, device="cuda") for _ in range(2)]
+    first = max(0, T - cap + 1)
+    qp, kp, vp = ops.qkv_gemm(x, w, cos.cuda(), sin.cuda(), H, swa.FP32_EPS, ve=ve, ve_gate_logit=logit, ring=ring, ring_first=first)
+    ops.check_device_status(x.device)
+    qkv = (x.float().cpu() @ w.float().cpu().t()).view(B, T, 3 * H, D)
+    q, k, v = qkv.chunk(3, dim=-2)
+    qn, kn, vn = swa.qkv_transform(q, k, v, cos, sin, swa.FP32_EPS)
+    g = torch.sigmoid(torch.tensor(0.4))
+    assert_close_bf16(qp, qn, "q'")
+    assert_close_bf16(kp, kn, "k'")
+    assert_close_bf16(vp, g * vn + (1 - g) * ve.float().cpu().view(B, T, H, D), "v'")
+    for t in range(first, T):
+        assert torch.equal(ring[0][:, :, t % cap], kp[:, t].to(ring[0].dtype)) and torch.equal(ring[1][:, :, t % cap], vp[:, t].to(ring[1].dtype))
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 6144, 2048), (2, 2048, 2048), (5, 392, 256), (8, 777, 1024), (17, 2048, 512), (64, 256, 2048),
                                    (3, 512, 12288), (8, 130, 16384)])
 def test_skinny_gemm_matches_fp32_reference(M, N, K):

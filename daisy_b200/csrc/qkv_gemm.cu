@@ -9,11 +9,11 @@
 //   EPI_PLAIN  bf16 store of C (the output projection).
 //
 // Persistent CTAs walk 128 x BN output tiles (n fastest, so concurrently running CTAs share X tiles and the
-// whole W in L2).  Roles (192 threads): warps 0-3 epilogue, warp 4 TMA producer, warp 5 MMA issuer.  Both
+// whole W in L2).  Roles (352 threads): warps 0-7 epilogue, warp 8 MMA issuer, warps 9, 10 TMA producers.  Both
 // operands are K-major with 128-byte swizzle (64-element boxes), exactly the Q K^T operand form of the
-// attention kernel; BN = 256 halves the shared-memory bytes read per flop against BN = 128 (the SS form of a
-// 128 x 128 x 16 MMA reads 8 KB per 64 cycles, all the shared-memory pipe has).  Two accumulators in TMEM
-// (2 x BN columns) let the epilogue of tile i run under the main loop of tile i + 1.
+// attention kernel.  Two accumulators in TMEM (2 x BN columns) let the epilogue of tile i run under the main loop of
+// tile i + 1.  At K = 768 the epilogue bounds the QKV form, not the products: with four epilogue warps reading their
+// rotations row by row 65536 x 2304 x 768 took 270 us, with eight and rotations through shared memory 219.
 // PAIR form (N a multiple of 256): clusters of two CTAs on 256 x 256 tiles with cta_group::2 MMAs.  Each CTA loads its
 // own 128 rows of X and its own 128 of the tile's 256 weight rows (plain per-CTA TMA loads), the pair's tensor cores
 // read both weight halves, so the shared-memory fill and operand reads per flop drop by a third against the single-CTA
@@ -25,18 +25,18 @@
 namespace daisy {
 
 constexpr int GM = 128, GK = 64;
-constexpr int G_THREADS = 192;
+constexpr int G_THREADS = 352;                         // 8 epilogue warps, MMA warp, 2 TMA warps
 constexpr int G_SMALL_THREADS = 192;                   // 4 epilogue warps, TMA warp, MMA warp
 constexpr int G_A_BYTES = GM * GK * 2;                 // 16 KB
-constexpr int G_STAGE_ROW = 256 + 16;                  // one staged output row (128 bf16) + pad: conflict-free 16-byte accesses
-constexpr int G_STAGING = 4 * 16 * G_STAGE_ROW;        // per warp 16 rows at a time
 
-template <int BN, bool PAIR> struct GemmCfg {
+template <int BN, bool PAIR, bool QKV> struct GemmCfg {
   static constexpr int B_ROWS = PAIR ? BN / 2 : BN;    // weight rows this CTA keeps per stage
   static constexpr int B_BYTES = B_ROWS * GK * 2;
   static constexpr int STAGE = G_A_BYTES + B_BYTES;
-  static constexpr int NST = (BN == 256 && !PAIR) ? 4 : 6;
-  static constexpr int SMEM = 1024 + NST * STAGE + G_STAGING + 256;
+  // per epilogue warp: 16 output rows at a time; QKV: before that, two slices of rotations
+  static constexpr int WARP_STAGING = QKV ? 2 * 4096 : 4096;
+  static constexpr int NST = QKV ? 5 : 6;
+  static constexpr int SMEM = 1024 + NST * STAGE + 8 * WARP_STAGING + 256;
   static constexpr int TILE_M = PAIR ? 2 * GM : GM;
 };
 
@@ -65,6 +65,17 @@ struct GemmParams {
   __nv_bfloat16* vn;
 };
 
+__device__ __forceinline__ void cp_async16(uint32_t smem_dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ float4 ld_shared_f4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+
 struct GemmBars {
   uint64_t full[6], empty[6];
   uint64_t acc_full[2], acc_empty[2];
@@ -72,15 +83,15 @@ struct GemmBars {
   int abort_flag;
 };
 
-template <int BN, bool PAIR>
+template <int BN, bool PAIR, bool QKV>
 __global__ void __launch_bounds__(G_THREADS, 1)
 qkv_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w, const GemmParams p) {
-  using Cfg = GemmCfg<BN, PAIR>;
+  using Cfg = GemmCfg<BN, PAIR, QKV>;
   extern __shared__ uint8_t gemm_smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(gemm_smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* stages = smem;
   uint8_t* staging = smem + Cfg::NST * Cfg::STAGE;
-  GemmBars* bars = reinterpret_cast<GemmBars*>(staging + G_STAGING);
+  GemmBars* bars = reinterpret_cast<GemmBars*>(staging + 8 * Cfg::WARP_STAGING);
   volatile int* abort_flag = &bars->abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -92,11 +103,11 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < Cfg::NST; ++i) { mbar_init(&bars->full[i], 1); mbar_init(&bars->empty[i], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&bars->acc_full[i], 1); mbar_init(&bars->acc_empty[i], PAIR ? 256 : 128); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&bars->acc_full[i], 1); mbar_init(&bars->acc_empty[i], PAIR ? 512 : 128); }
     bars->abort_flag = 0;
     mbar_init_fence();
   }
-  if (warp == 5) {
+  if (warp == 8) {
     if (PAIR) { tmem_alloc_pair(&bars->tmem_base, 2 * BN); tmem_relinquish_pair(); }
     else { tmem_alloc(&bars->tmem_base, 2 * BN); tmem_relinquish(); }
   }
@@ -106,15 +117,17 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
 
-  if (warp == 4) {
-    // ------------------------------------------------------------------ TMA producer
+  if (warp >= 9) {
+    // ------------------------------------------------------------------ TMA producers: every other k-block each (a turn of the
+    // loop takes one thread some 450 cycles, the products of a k-block 256, PAIR 512)
     if (lane == 0) {
       prefetch_tmap(&tm_x); prefetch_tmap(&tm_w);
-      uint32_t n = 0;
+      uint32_t n = warp - 9, first = 0;                  // my next k-block, and the tile's first, counted over all tiles
       bool ok = true;
-      for (int tile = worker; tile < tiles && ok; tile += workers) {
+      for (int tile = worker; tile < tiles && ok; tile += workers, first += kb_n) {
         const int m0 = (tile / n_tiles) * Cfg::TILE_M + (int)rank * GM, n0 = (tile % n_tiles) * BN + (int)rank * Cfg::B_ROWS;
-        for (int kb = 0; kb < kb_n; ++kb, ++n) {
+        for (; n < first + kb_n; n += 2) {
+          const int kb = n - first;
           const int st = n % Cfg::NST;
           if (!mbar_wait(&bars->empty[st], ((n / Cfg::NST) & 1) ^ 1, abort_flag, p.status, 1)) { ok = false; break; }
           uint8_t* dst = stages + st * Cfg::STAGE;
@@ -132,7 +145,7 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
         }
       }
     }
-  } else if (warp == 5 && rank == 0) {
+  } else if (warp == 8 && rank == 0) {
     // ------------------------------------------------------------------ MMA issuer
     const uint32_t leader = elect_one() ? 1u : 0u;
     constexpr uint32_t idesc = umma_idesc_bf16(Cfg::TILE_M, BN, 0, 0);
@@ -164,35 +177,50 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
         else tc_commit_p(leader, &bars->acc_full[buf]);
       }
     }
-  } else if (warp < 4) {
-    // ------------------------------------------------------------------ epilogue: thread = output row
-    const int row = warp * 32 + lane;
-    const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
-    uint8_t* stg = staging + warp * 16 * G_STAGE_ROW;
+  } else if (warp < 8) {
+    // ------------------------------------------------------------------ epilogue: thread = output row.  Two groups of four warps:
+    // PAIR: one takes the tile's columns 0 .. 127, the other 128 .. 255; single: one takes the even tiles, the other the odd ones
+    const int grp = warp >> 2, row = (warp & 3) * 32 + lane;
+    const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
+    uint8_t* stg = staging + warp * Cfg::WARP_STAGING;
+    const uint32_t s_stg = smem_u32(stg), s_own = s_stg + lane * 128;
     uint32_t it = 0;
     bool ok = true;
     for (int tile = worker; tile < tiles && ok; tile += workers, ++it) {
       const uint32_t buf = it & 1;
-      const int m0 = (tile / n_tiles) * Cfg::TILE_M + (int)rank * GM, n0 = (tile % n_tiles) * BN;
+      if (!PAIR && (int)buf != grp) continue;
+      const int m0 = (tile / n_tiles) * Cfg::TILE_M + (int)rank * GM, n0 = (tile % n_tiles) * BN + (PAIR ? grp * 128 : 0);
       const int m = m0 + row;
+      // RoPE: slice i of the rotations (cos, sin of channels 16 i .. 16 i + 15 of the warp's 32 rows) goes through shared memory,
+      // two slices ahead: a lane's own row read straight from the tables is 32 lines an instruction, 4096 cycles a 128 x 128 tile
+      const bool rope = QKV && (n0 >> 7) < 2 * p.H && (p.flags & DAISY_ROPE);
+      const int pos = rope ? min(m, p.M - 1) % p.T : 0;
+      auto fetch = [&](int i) {
+        const float* tab = ((lane & 4) ? p.sin : p.cos) + 16 * i + 4 * (lane & 3);
+        const uint32_t dst = s_stg + (i & 1) * 4096;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int rr = 4 * j + (lane >> 3);
+          cp_async16(dst + rr * 128 + (((lane & 7) ^ (rr & 7)) << 4), tab + (size_t)__shfl_sync(0xffffffffu, pos, rr) * 64);
+        }
+        cp_async_commit();
+      };
+      if (rope) { fetch(0); fetch(1); }
       ok = __all_sync(0xffffffffu, mbar_wait(&bars->acc_full[buf], (it >> 1) & 1, abort_flag, p.status, 4));
-      if (!ok) break;
+      if (!ok) { if (QKV) cp_async_wait<0>(); break; }
       tc_fence_after();
-#pragma unroll 1
-      for (int half = 0; half < BN / 128; ++half) {
+      {
         uint32_t r[128];
-        const uint32_t t0 = tmem_base + lane_off + buf * BN + half * 128;
+        const uint32_t t0 = tmem_base + lane_off + buf * BN + (PAIR ? grp * 128 : 0);
         tmem_ld32(t0, r); tmem_ld32(t0 + 32, r + 32); tmem_ld32(t0 + 64, r + 64); tmem_ld32(t0 + 96, r + 96);
         tc_wait_ld();
-        if (half == BN / 128 - 1) {                                // accumulator read out: the MMA warp may refill it
-          tc_fence_before();
-          if (PAIR) mbar_arrive_cluster(mapa_shared(smem_u32(&bars->acc_empty[buf]), 0));   // the issuer waits for both CTAs
-          else mbar_arrive(&bars->acc_empty[buf]);
-        }
+        tc_fence_before();                                         // accumulator read out: the MMA warp may refill it
+        if (PAIR) mbar_arrive_cluster(mapa_shared(smem_u32(&bars->acc_empty[buf]), 0));   // the issuer waits for both CTAs
+        else mbar_arrive(&bars->acc_empty[buf]);
         __nv_bfloat16* dst_row;                                    // this thread's output row (128 bf16)
         uint8_t* ring_row = nullptr;
-        if (p.epi == 1) {
-          const int nh = (n0 + half * 128) >> 7;                   // head slot among 3 H
+        if (QKV) {
+          const int nh = n0 >> 7;                   // head slot among 3 H
           const int which = nh / p.H, h = nh - which * p.H;
           const bool do_norm = (p.flags & (which == 0 ? DAISY_NORM_Q : which == 1 ? DAISY_NORM_K : DAISY_NORM_V)) != 0;
           if (do_norm) {
@@ -204,21 +232,26 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
 #pragma unroll
             for (int i = 0; i < 128; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * rs);
           }
-          if (which < 2 && (p.flags & DAISY_ROPE)) {
-            const int pos = min(m, p.M - 1) % p.T;
-            const float4* cr = reinterpret_cast<const float4*>(p.cos + (size_t)pos * 64);
-            const float4* sr = reinterpret_cast<const float4*>(p.sin + (size_t)pos * 64);
+          if (rope) {
 #pragma unroll
-            for (int i4 = 0; i4 < 16; ++i4) {
-              const float4 c = cr[i4], s = sr[i4];
-              const float cc[4] = {c.x, c.y, c.z, c.w}, sn[4] = {s.x, s.y, s.z, s.w};
+            for (int i = 0; i < 4; ++i) {
+              if (i < 3) cp_async_wait<1>(); else cp_async_wait<0>();
+              __syncwarp();
 #pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const int i = 4 * i4 + e;
-                const float a = __uint_as_float(r[i]), b2 = __uint_as_float(r[i + 64]);
-                r[i] = __float_as_uint(a * cc[e] + b2 * sn[e]);
-                r[i + 64] = __float_as_uint(b2 * cc[e] - a * sn[e]);
+              for (int i4 = 0; i4 < 4; ++i4) {
+                const uint32_t a0 = s_own + (i & 1) * 4096;
+                const float4 c = ld_shared_f4(a0 + ((i4 ^ (lane & 7)) << 4)), s = ld_shared_f4(a0 + (((4 + i4) ^ (lane & 7)) << 4));
+                const float cc[4] = {c.x, c.y, c.z, c.w}, sn[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  const int j = 16 * i + 4 * i4 + e;
+                  const float a = __uint_as_float(r[j]), b2 = __uint_as_float(r[j + 64]);
+                  r[j] = __float_as_uint(a * cc[e] + b2 * sn[e]);
+                  r[j + 64] = __float_as_uint(b2 * cc[e] - a * sn[e]);
+                }
               }
+              __syncwarp();
+              if (i < 2) fetch(i + 2);
             }
           }
           if (which == 2 && p.vn && m < p.M) {                      // (thread = row: the gated layers of a model are few)
@@ -246,7 +279,7 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
               ring_row = reinterpret_cast<uint8_t*>(p.ring[which - 1]) + ((int64_t)b * p.r_sb + (int64_t)h * p.r_sh + (int64_t)(t % p.cap) * p.r_sr) * 2;
           }
         } else {
-          dst_row = p.c + (size_t)m * p.ldc + n0 + half * 128;
+          dst_row = p.c + (size_t)m * p.ldc + n0;
         }
         // bf16 pack, then through the warp's staging rows so that each store instruction writes two whole rows
         uint4 ch[16];
@@ -260,19 +293,19 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
         for (int pass = 0; pass < 2; ++pass) {
           if ((lane >> 4) == pass) {
 #pragma unroll
-            for (int c = 0; c < 16; ++c) *reinterpret_cast<uint4*>(stg + (lane & 15) * G_STAGE_ROW + c * 16) = ch[c];
+            for (int c = 0; c < 16; ++c) *reinterpret_cast<uint4*>(stg + (lane & 15) * 256 + ((c ^ (lane & 15)) << 4)) = ch[c];
           }
           __syncwarp();
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
             const int rr = 2 * i + (lane >> 4);                    // staged row, = warp row 16 pass + rr
-            const uint4 val = *reinterpret_cast<const uint4*>(stg + rr * G_STAGE_ROW + (lane & 15) * 16);
+            const uint4 val = *reinterpret_cast<const uint4*>(stg + rr * 256 + (((lane & 15) ^ rr) << 4));
             const int src_lane = 16 * pass + rr;
             // the row's global address lives in the lane that owns the row
             const unsigned long long base = __shfl_sync(0xffffffffu, (unsigned long long)reinterpret_cast<uintptr_t>(dst_row), src_lane);
             const int mm = __shfl_sync(0xffffffffu, m, src_lane);
             if (mm < p.M) *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(base) + (lane & 15) * 16) = val;
-            if (p.epi == 1 && p.ring[0]) {                         // warp-uniform: a ring is attached to this call
+            if (QKV && p.ring[0]) {                         // warp-uniform: a ring is attached to this call
               const unsigned long long rb = __shfl_sync(0xffffffffu, (unsigned long long)reinterpret_cast<uintptr_t>(ring_row), src_lane);
               if (rb) {
                 uint4 rv = val;
@@ -297,7 +330,7 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
   tc_fence_before();
   if (PAIR) cluster_sync_all();                        // neither CTA leaves while the other may still read its operands
   else __syncthreads();
-  if (warp == 5) {
+  if (warp == 8) {
     tc_fence_after();
     if (PAIR) tmem_dealloc_pair(tmem_base, 2 * BN);
     else tmem_dealloc(tmem_base, 2 * BN);
@@ -524,9 +557,9 @@ small_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
 
 using namespace daisy;
 
-template <int BN, bool PAIR>
+template <int BN, bool PAIR, bool QKV>
 static int launch_gemm(const CUtensorMap& tx, const CUtensorMap& tw, const GemmParams& p, cudaStream_t st) {
-  using Cfg = GemmCfg<BN, PAIR>;
+  using Cfg = GemmCfg<BN, PAIR, QKV>;
   static_assert(Cfg::SMEM <= 232448, "over the 227 KB a CTA may use");
   static bool attr[daisy_host::MAX_DEVICES] = {};
   static int max_clusters[daisy_host::MAX_DEVICES] = {};
@@ -541,14 +574,14 @@ static int launch_gemm(const CUtensorMap& tx, const CUtensorMap& tw, const GemmP
   at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
   if (PAIR) { cfg.attrs = at; cfg.numAttrs = 1; }
   if (!attr[dev]) {
-    if (cudaFuncSetAttribute(qkv_gemm_kernel<BN, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM) != cudaSuccess) {
+    if (cudaFuncSetAttribute(qkv_gemm_kernel<BN, PAIR, QKV>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM) != cudaSuccess) {
       (void)cudaGetLastError();
       return DAISY_ECUDA;
     }
     if (PAIR) {                                          // how many CTA pairs the device can hold at once
       cfg.gridDim = dim3((unsigned)(sms & ~1));
       int n = 0;
-      if (cudaOccupancyMaxActiveClusters(&n, qkv_gemm_kernel<BN, PAIR>, &cfg) != cudaSuccess || n <= 0) {
+      if (cudaOccupancyMaxActiveClusters(&n, qkv_gemm_kernel<BN, PAIR, QKV>, &cfg) != cudaSuccess || n <= 0) {
         (void)cudaGetLastError();
         return DAISY_ECUDA;
       }
@@ -563,7 +596,7 @@ static int launch_gemm(const CUtensorMap& tx, const CUtensorMap& tw, const GemmP
   } else {
     cfg.gridDim = dim3((unsigned)(tiles < sms ? tiles : sms));
   }
-  if (cudaLaunchKernelEx(&cfg, qkv_gemm_kernel<BN, PAIR>, tx, tw, p) != cudaSuccess) {
+  if (cudaLaunchKernelEx(&cfg, qkv_gemm_kernel<BN, PAIR, QKV>, tx, tw, p) != cudaSuccess) {
     (void)cudaGetLastError();
     return DAISY_ECUDA;
   }
@@ -615,14 +648,17 @@ static int launch_small(const void* x, int64_t ldx, const void* w, int64_t ldw, 
 }
 
 // Which tile.  One wave of narrow tiles as long as they fit the chip (a second wave costs more than wider tiles do:
-// 2048 x 768 x 768 7.5 us in 128-column tiles, 8.4 in 64); from there 128 x 128 tiles against pairs on 256 x 256, whose
-// larger tiles want a large product.
+// 2048 x 768 x 768 7.5 us in 128-column tiles, 8.4 in 64).  From there 128 x 128 tiles against pairs on 256 x 256, by what a
+// wave of either was measured to take: a pair's wave is twice the work at 0.7 of the time per product, with a longer start
+// and end (ns; 1024 x 2048 x 2048 12.4 against 16.9 us, 2048 x 6144 x 2048 51 against 42, 65536 x 768 x 768 80 against 67).
 enum { TILE_32 = 32, TILE_64 = 64, TILE_128 = 128, TILE_PAIR = 256 };
 static int gemm_tile(const GemmParams& p, int sms) {
   const int64_t mt = ((int64_t)p.M + GM - 1) / GM;
   if (p.epi == 0 && mt * (p.N / 32) <= sms) return TILE_32;
   if (mt * (p.N / 64) <= sms) return TILE_64;
-  return p.N % 256 == 0 && p.M > GM ? TILE_PAIR : TILE_128;
+  if (p.N % 256 != 0) return TILE_128;
+  const int64_t w1 = (mt * (p.N / 128) + sms - 1) / sms, w2 = ((mt + 1) / 2 * (p.N / 256) + sms / 2 - 1) / (sms / 2);
+  return 4000 + w1 * (37ll * p.K / 10 + 1000) < 7000 + w2 * (53ll * p.K / 10 + 2000) ? TILE_128 : TILE_PAIR;
 }
 
 static int gemm_common(const void* x, int64_t ldx, const void* w, int64_t ldw, GemmParams& p, void* stream) {
@@ -639,7 +675,8 @@ static int gemm_common(const void* x, int64_t ldx, const void* w, int64_t ldw, G
   int rc;
   if ((rc = daisy_host::make_tmap_bf16_3d(&tx, x, p.K, p.M, 1, (uint64_t)ldx * 2, (uint64_t)ldx * 2 * p.M, GK, GM)) != DAISY_OK) return rc;
   if ((rc = daisy_host::make_tmap_bf16_3d(&tw, w, p.K, p.N, 1, (uint64_t)ldw * 2, (uint64_t)ldw * 2 * p.N, GK, 128)) != DAISY_OK) return rc;
-  return tile == TILE_PAIR ? launch_gemm<256, true>(tx, tw, p, st) : launch_gemm<128, false>(tx, tw, p, st);
+  if (tile == TILE_PAIR) return p.epi ? launch_gemm<256, true, true>(tx, tw, p, st) : launch_gemm<256, true, false>(tx, tw, p, st);
+  return p.epi ? launch_gemm<128, false, true>(tx, tw, p, st) : launch_gemm<128, false, false>(tx, tw, p, st);
 }
 
 extern "C" int daisy_b200_gemm_nt(const void* x, int64_t ldx, const void* w, int64_t ldw, void* c, int64_t ldc,

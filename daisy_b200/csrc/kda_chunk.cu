@@ -11,12 +11,8 @@
 //    Gram products in mma.sync fragments, the blocked solve of (I + A_kk) W = beta k e^G, (I + A_kk) U0 = beta v in register
 //    chains.  Per chunk it writes a record of fp16 operand images (16-byte pieces exchanged so that fragment loads are
 //    bank-conflict free): W^T, scale q e^G, k e^{G_C-G}, A_qk, U0^T, and e^{G_C}.
-//  * kda_state_kernel  -- one CTA per (batch, head, V-slice), sequential over chunks: a producer warp
-//    bulk-copies the images of chunk c+1.. into a shared-memory ring while the compute warps hold their
-//    slice of S^T (16 V-rows x 128 K-columns per warp) in fp32 accumulator registers and chain the
-//    three products through register-resident fragments (an accumulator tile pair is exactly the next
-//    product's A fragment), so the state never leaves the register file between chunks.  With few (batch, head)
-//    pairs per GPU two warps share a slice, each holding half of the K-columns.
+//  * kda_state_kernel  -- one CTA per (batch, head), sequential over chunks, on tcgen05: S^T in TMEM, the records through a
+//    three-stage ring.
 // Tensor-core operands are fp16 (10-bit mantissa, every decay factor and operand here is <= O(1)):
 // measured relative error of o against the fp32 token recurrence is ~4e-4, bf16 operands give ~3e-3.
 #include <cuda_fp16.h>
@@ -27,11 +23,11 @@ namespace daisy {
 
 constexpr int KC = 64;                 // chunk length
 constexpr int KD = 128;                // K = V
-// per-chunk record in the workspace (bytes); every image is laid out so that ldmatrix reads it without bank conflicts after
-// a plain bulk copy (rec_off, ki_off)
+// per-chunk record in the workspace (bytes); after a plain bulk copy every image is a 128-byte-swizzled tcgen05 operand: rows of
+// 64 fp16 whose 16-byte pieces are exchanged by row (rec_off, panel_off)
 constexpr int OFF_WT = 0;                              // W^T      [128 channels][64 tokens] fp16
-constexpr int OFF_QT = OFF_WT + KD * KC * 2;           // q~       [64 tokens][128 channels] fp16   scale q e^G
-constexpr int OFF_KT = OFF_QT + KD * KC * 2;           // k~       [64 tokens][128 channels] fp16   k e^{G_C-G}
+constexpr int OFF_QT = OFF_WT + KD * KC * 2;           // q~       [2][64 tokens][64 channels] fp16   scale q e^G
+constexpr int OFF_KT = OFF_QT + KD * KC * 2;           // k~       [2][64 tokens][64 channels] fp16   k e^{G_C-G}
 constexpr int OFF_AQK = OFF_KT + KD * KC * 2;          // A_qk     [64][64]  fp16
 constexpr int OFF_D = OFF_AQK + KC * KC * 2;           // e^{G_C}  [128]     fp32
 constexpr int SHARED_BYTES = OFF_D + KD * 4;           // 57856: identical for every V-slice
@@ -41,9 +37,8 @@ static_assert(SHARED_BYTES % 16 == 0 && REC_BYTES % 16 == 0, "bulk copies move 1
 
 // byte offset of (row, token column) in an image of 64-token rows (128 bytes, 16-byte pieces exchanged by row)
 __device__ __forceinline__ uint32_t rec_off(int row, int col) { return (uint32_t)(row * 128 + (((col >> 3) ^ (row & 7)) << 4) + (col & 7) * 2); }
-// byte offset of 16-byte piece c (0..15) of a row in an image of 128-channel rows: the eight lanes that store two half rows,
-// and the eight rows of a (transposing) ldmatrix, all hit different banks
-__device__ __forceinline__ uint32_t ki_off(int row, int c) { return (uint32_t)(row * 256 + ((c ^ (((row & 1) << 2) | ((row >> 1) & 3))) << 4)); }
+// byte offset of 16-byte piece c (0..15) of a 128-channel row kept as two panels of 64 channels
+__device__ __forceinline__ uint32_t panel_off(int row, int c) { return (uint32_t)((c >> 3) * (KC * 128) + row * 128 + (((c ^ row) & 7) << 4)); }
 
 // Four 8x8 fp16 matrices from shared memory: lanes 8m..8m+7 give the row addresses of matrix m (16 bytes per
 // row); register m of lane l then holds elements (row l/4, columns 2(l%4), 2(l%4)+1) of matrix m -- the B
@@ -394,6 +389,7 @@ __global__ void __launch_bounds__(KI_THREADS, 3) kda_intra_kernel(const KdaIntra
     *reinterpret_cast<uint32_t*>(rec + OFF_AQK + rec_off(r1, 16 * warp + jc)) = pack_h2(p.scale * l8[2], p.scale * l8[3]);
     *reinterpret_cast<uint32_t*>(rec + OFF_AQK + rec_off(r0, 16 * warp + 8 + jc)) = 0u;
   }
+  for (int J = warp + 1; J < 4; ++J) st_global16(rec + OFF_AQK + rec_off(16 * warp + (lane >> 1), 16 * J + 8 * (lane & 1)), 0u, 0u, 0u, 0u);   // j > i
   __syncwarp();
   // ---- its inverse in fp32, lane = column: a column sweep (once t_j is final every later row takes its update at once)
   if (lane < 16) {
@@ -428,7 +424,7 @@ __global__ void __launch_bounds__(KI_THREADS, 3) kda_intra_kernel(const KdaIntra
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int r = 2 * i + (lane >> 4);
-      const uint32_t off = r * KI_LD + 16 * c, roff = 4096 * warp + ki_off(r, c);
+      const uint32_t off = r * KI_LD + 16 * c, roff = panel_off(16 * warp + r, c);
       uint32_t q[4], k[4], z[4];
       *reinterpret_cast<uint4*>(q) = *reinterpret_cast<const uint4*>(sm.pq[warp] + off);
       *reinterpret_cast<uint4*>(k) = *reinterpret_cast<const uint4*>(sm.pk[warp] + off);
@@ -535,241 +531,223 @@ struct KdaStateParams {
   void* o;
   int T, H, NC, out_fp32;
   int* status;
-  // packed variable-length sequences (B = 1): blockIdx.y = sequence * H + head, the sequence's chunks are
+  // packed variable-length sequences (B = 1): blockIdx.x = sequence * H + head, the sequence's chunks are
   // seq_ptr[s] .. seq_ptr[s + 1] - 1 of the packed row's NC chunks, chunk_tab as in the intra kernel; null: dense
   const int* chunk_tab;
   const int* seq_ptr;
 };
 
 
-// NW V-slices of 16 rows per CTA, each owned by KS warps that split the K dimension of the state between them.
-// KS = 1: a warp keeps its 16 V-rows x 128 K-columns of S^T in accumulator registers and chains everything through
-// register fragments.  KS > 1 (few (batch, head) pairs per GPU, where the serial chain over the chunks -- 212
-// dependent mma.sync per chunk and warp -- is all that is left): warp kq holds K-columns [128 kq / KS, 128 (kq+1) / KS);
-// the two products that contract over K (S^T W^T and S^T q~^T) become partial sums that the slice's warps exchange
-// through shared memory once per chunk (fragment order, double-buffered, one named barrier), after which every warp
-// has the whole U^T, finishes the output for its own token tiles and updates its own K-columns of the state.
-template <int NW, int KS, int NST>
-struct KdaStateSmem {
-  static constexpr int VS = 16 * NW;
-  static constexpr int CW = NW * KS;                     // compute warps
-  static constexpr int U_BYTES = VS * KC * 2;
-  static constexpr int STAGE = SHARED_BYTES + U_BYTES;
-  static constexpr int O_LD = VS + 4;                    // floats; staging of one chunk of output
-  static constexpr int XCH_WARP = 2 * 8 * 32 * 16;       // one warp's two partial accumulators: 8 tiles x 32 lanes x float4
-  static constexpr int XCH = KS > 1 ? CW * XCH_WARP : 0;
-  static constexpr int BYTES = NST * STAGE + KC * O_LD * 4 + XCH + 64;
+// One CTA per (batch, head); TMEM lane = value column, so all products have M = 128 and
+//     U^T [V x 64]   = U0^T - S^T W^T            S^T as fp16 from TMEM, W^T as the record has it (channels = depth)
+//     O^T [V x 64]   = S^T q~^T + U^T A_qk^T
+//     S^T [V x 128] <- S^T diag(e^{G_C}) + U^T k~  accumulated in TMEM on the scaled state
+// The chain from chunk to chunk is all that matters (a (batch, head) is serial, and there are rarely more of them than SMs):
+// read S -> fp16 -> 8 products of N = 64 -> subtract -> fp16 -> 4 products of N = 128.  Warps 0-3 (thread = value column) run
+// that chain; everything else is beside it: they scale the state while the U products run, q~'s products fill the tensor pipe
+// while U is converted, warps 4-7 write O out of two accumulators, warp 8 issues, warp 9 keeps the ring full.
+// The same chain in mma.sync fragments, 64 value columns to a CTA, took 3700 cycles a chunk (212 products of a warp on one
+// tensor pipe and as many cycles of ldmatrix): 500 us at 4 x 16384 x 16 against 418 here.
+constexpr int KS_NST = 3;
+constexpr int KS_STAGE = (REC_BYTES + 1023) / 1024 * 1024;     // operands start on 1024-byte boundaries
+constexpr int KS_THREADS = 320;
+constexpr int TM_S = 0, TM_S16 = 128, TM_U = 192, TM_U16 = 256, TM_O = 288;      // TMEM columns; O: two accumulators of 64
+static_assert(OFF_QT % 1024 == 0 && OFF_KT % 1024 == 0 && OFF_AQK % 1024 == 0, "swizzled operands");
+struct KdaStateBars {
+  uint64_t full[KS_NST], empty[KS_NST];
+  uint64_t s16, u, u16, s, o_full[2], o_free[2];
+  uint32_t tmem_base;
+  int abort_flag;
 };
+constexpr int KS_SMEM = 1024 + KS_NST * KS_STAGE + (int)sizeof(KdaStateBars);
+static_assert(KS_SMEM <= 232448, "over the 227 KB a CTA may use");
 
-template <int NW, int KS, int NST>
-__global__ void __launch_bounds__(32 * (NW * KS + 1), 1) kda_state_kernel(const KdaStateParams p) {
-  using L = KdaStateSmem<NW, KS, NST>;
-  constexpr int KDA_NST = NST;                             // ring stages of chunk records
-  constexpr int VS = L::VS, CW = L::CW;
-  constexpr int NKT = 16 / KS;                             // this warp's 8-column tiles of the state
-  constexpr int NKS = 8 / KS;                              // and its 16-deep steps of the contractions over K
-  constexpr int TPW = 8 / KS;                              // token tiles whose output this warp finishes
-  extern __shared__ __align__(128) uint8_t kda_smem_raw[];
-  uint8_t* stages = kda_smem_raw;
-  float* o_stage = reinterpret_cast<float*>(kda_smem_raw + KDA_NST * L::STAGE);
-  float4* xch = reinterpret_cast<float4*>(kda_smem_raw + KDA_NST * L::STAGE + KC * L::O_LD * 4);
-  uint64_t* full = reinterpret_cast<uint64_t*>(kda_smem_raw + KDA_NST * L::STAGE + KC * L::O_LD * 4 + L::XCH);
-  uint64_t* empty = full + KDA_NST;
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(empty + KDA_NST);
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g8 = lane >> 2, t4 = lane & 3;
-  const int vsl = blockIdx.x, bh = blockIdx.y;              // bh also indexes h0 / hT
-  const int h = bh % p.H;
-  const int b = p.seq_ptr ? 0 : bh / p.H;
-  const int c_begin = p.seq_ptr ? p.seq_ptr[bh / p.H] : 0, c_end = p.seq_ptr ? p.seq_ptr[bh / p.H + 1] : p.NC;
-  const int v_base = vsl * VS;
-  const uint8_t* recs = p.ws + ((size_t)(b * p.H + h) * p.NC + c_begin) * REC_BYTES;    // this sequence's first record
-  const int n_chunks = c_end - c_begin;
+__global__ void __launch_bounds__(KS_THREADS, 1) kda_state_kernel(const KdaStateParams p) {
+  extern __shared__ uint8_t kda_smem_raw[];
+  uint8_t* stages = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(kda_smem_raw) + 1023) & ~uintptr_t(1023));
+  KdaStateBars* bars = reinterpret_cast<KdaStateBars*>(stages + KS_NST * KS_STAGE);
+  volatile int* abort_flag = &bars->abort_flag;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < KDA_NST; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], CW); }
-    *abort_flag = 0;
+    for (int i = 0; i < KS_NST; ++i) { mbar_init(&bars->full[i], 1); mbar_init(&bars->empty[i], 5); }       // 4 state warps, 1 commit
+    mbar_init(&bars->s16, 128); mbar_init(&bars->u, 1); mbar_init(&bars->u16, 128); mbar_init(&bars->s, 1);
+    for (int i = 0; i < 2; ++i) { mbar_init(&bars->o_full[i], 1); mbar_init(&bars->o_free[i], 128); }
+    bars->abort_flag = 0;
     mbar_init_fence();
   }
+  if (warp == 8) { tmem_alloc(&bars->tmem_base, 512); tmem_relinquish(); }
+  tc_fence_before();
   __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = bars->tmem_base;
+  grid_dep_wait();
 
-  if (warp == CW) {
-    // ------------------------------------------------------------ producer: bulk copies into the ring
+  const int bh = blockIdx.x, h = bh % p.H, b = p.seq_ptr ? 0 : bh / p.H;           // bh also indexes h0 / hT
+  const int c_begin = p.seq_ptr ? p.seq_ptr[bh / p.H] : 0, c_end = p.seq_ptr ? p.seq_ptr[bh / p.H + 1] : p.NC;
+  const int n_chunks = c_end - c_begin;
+
+  if (warp == 9) {
+    // ------------------------------------------------------------ producer: one record a stage
     if (lane == 0) {
+      const uint8_t* recs = p.ws + ((size_t)(b * p.H + h) * p.NC + c_begin) * REC_BYTES;
       for (int c = 0; c < n_chunks; ++c) {
-        const int s = c % KDA_NST;
-        if (!mbar_wait(&empty[s], ((c / KDA_NST) & 1) ^ 1, abort_flag, p.status, 1)) break;
-        const uint8_t* rec = recs + (size_t)c * REC_BYTES;
-        mbar_expect_tx(&full[s], L::STAGE);
-        bulk_g2s(stages + s * L::STAGE, rec, SHARED_BYTES, &full[s]);
-        bulk_g2s(stages + s * L::STAGE + SHARED_BYTES, rec + OFF_UT + (size_t)v_base * KC * 2, L::U_BYTES, &full[s]);
-      }
-    }
-    return;
-  }
-
-  // ------------------------------------------------------------ compute warps: 16 V rows, 128 / KS K columns each
-  const int vs = warp / KS, kq = warp % KS;
-  const int vr0 = vs * 16 + g8, vr1 = vr0 + 8;                     // rows inside the CTA's V range
-  float st[NKT][4];                                                // S^T[v][k]: tile j -> k = 8 (kq NKT + j) + 2 t4 (+1)
-#pragma unroll
-  for (int j = 0; j < NKT; ++j) {
-    if (p.h0) {
-      const float* hp = p.h0 + (size_t)bh * KD * KD;
-      const int k0 = (kq * NKT + j) * 8 + 2 * t4;
-      st[j][0] = hp[(size_t)k0 * KD + v_base + vr0]; st[j][1] = hp[(size_t)(k0 + 1) * KD + v_base + vr0];
-      st[j][2] = hp[(size_t)k0 * KD + v_base + vr1]; st[j][3] = hp[(size_t)(k0 + 1) * KD + v_base + vr1];
-    } else {
-      st[j][0] = st[j][1] = st[j][2] = st[j][3] = 0.f;
-    }
-  }
-
-  for (int c = 0; c < n_chunks; ++c) {
-    const int s = c % KDA_NST;
-    const bool ok = __all_sync(0xffffffffu, mbar_wait(&full[s], (c / KDA_NST) & 1, abort_flag, p.status, 2));
-    if (!ok) break;
-    const uint8_t* sb = stages + s * L::STAGE;
-    const uint32_t Wt = smem_u32(sb + OFF_WT), Qt = smem_u32(sb + OFF_QT), Kt = smem_u32(sb + OFF_KT), Aq = smem_u32(sb + OFF_AQK);
-    const float* dv = reinterpret_cast<const float*>(sb + OFF_D);
-    const uint8_t* Ut = sb + SHARED_BYTES;
-
-    // (1) accU = S^T W^T   and   (2a) accO = S^T q~^T      [16 x 64 tokens each], over this warp's K columns
-    float au[8][4], ao[8][4];
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt) { au[nt][0] = au[nt][1] = au[nt][2] = au[nt][3] = 0.f; ao[nt][0] = ao[nt][1] = ao[nt][2] = ao[nt][3] = 0.f; }
-#pragma unroll
-    for (int ksl = 0; ksl < NKS; ++ksl) {
-      const int ks = kq * NKS + ksl;
-      uint32_t a[4];
-      a[0] = pack_h2(st[2 * ksl][0], st[2 * ksl][1]); a[1] = pack_h2(st[2 * ksl][2], st[2 * ksl][3]);
-      a[2] = pack_h2(st[2 * ksl + 1][0], st[2 * ksl + 1][1]); a[3] = pack_h2(st[2 * ksl + 1][2], st[2 * ksl + 1][3]);
-      // B fragments of two token tiles per ldmatrix.x4, matrix m = (channel octet m & 1, token tile nt + (m >> 1)): W^T rows
-      // are channels (transposing form), q~ rows are tokens
-      const int wrow = ks * 16 + ((lane >> 3) & 1) * 8 + (lane & 7), qrow = (lane & 7) + 8 * (lane >> 4), qpc = 2 * ks + ((lane >> 3) & 1);
-#pragma unroll
-      for (int nt = 0; nt < 8; nt += 2) {
-        uint32_t bw[4], bq[4];
-        ldmatrix_x4_t(bw, Wt + rec_off(wrow, (nt + (lane >> 4)) * 8));
-        ldmatrix_x4(bq, Qt + ki_off(nt * 8 + qrow, qpc));
-        mma_f16(au[nt], a, bw[0], bw[1]);
-        mma_f16(ao[nt], a, bq[0], bq[1]);
-        mma_f16(au[nt + 1], a, bw[2], bw[3]);
-        mma_f16(ao[nt + 1], a, bq[2], bq[3]);
-      }
-    }
-    if (KS > 1) {
-      // exchange: every warp of the slice needs the whole accU; accO only for the token tiles it finishes.  The sums
-      // run over the warps in a fixed order, so all of them hold the same bits.
-      float4* mine = xch + (size_t)warp * (L::XCH_WARP / 16);
-#pragma unroll
-      for (int nt = 0; nt < 8; ++nt) {
-        mine[nt * 32 + lane] = make_float4(au[nt][0], au[nt][1], au[nt][2], au[nt][3]);
-        mine[256 + nt * 32 + lane] = make_float4(ao[nt][0], ao[nt][1], ao[nt][2], ao[nt][3]);
-      }
-      named_bar(2 + vs, 32 * KS);
-      const float4* slice = xch + (size_t)(vs * KS) * (L::XCH_WARP / 16);
-#pragma unroll
-      for (int nt = 0; nt < 8; ++nt) {
-        float4 t = slice[nt * 32 + lane];
-#pragma unroll
-        for (int q = 1; q < KS; ++q) {
-          const float4 u = slice[q * (L::XCH_WARP / 16) + nt * 32 + lane];
-          t.x += u.x; t.y += u.y; t.z += u.z; t.w += u.w;
-        }
-        au[nt][0] = t.x; au[nt][1] = t.y; au[nt][2] = t.z; au[nt][3] = t.w;
-      }
-#pragma unroll
-      for (int nt = 0; nt < 8; ++nt) {
-        if (nt / TPW != kq) continue;                                // compile-time tile index, warp-uniform test
-        float4 t = slice[256 + nt * 32 + lane];
-#pragma unroll
-        for (int q = 1; q < KS; ++q) {
-          const float4 u = slice[q * (L::XCH_WARP / 16) + 256 + nt * 32 + lane];
-          t.x += u.x; t.y += u.y; t.z += u.z; t.w += u.w;
-        }
-        ao[nt][0] = t.x; ao[nt][1] = t.y; ao[nt][2] = t.z; ao[nt][3] = t.w;
-      }
-      named_bar(2 + vs, 32 * KS);                                    // everybody has read: the next chunk may overwrite
-    }
-    // U^T = U0^T - accU, as fp16 A fragments over the token axis
-    uint32_t ua[4][4];
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
-      const int tok = nt * 8 + 2 * t4;
-      const float2 u0 = unpack_h2(*reinterpret_cast<const uint32_t*>(Ut + rec_off(vr0, tok)));
-      const float2 u1 = unpack_h2(*reinterpret_cast<const uint32_t*>(Ut + rec_off(vr1, tok)));
-      const uint32_t lo = pack_h2(u0.x - au[nt][0], u0.y - au[nt][1]);
-      const uint32_t hi = pack_h2(u1.x - au[nt][2], u1.y - au[nt][3]);
-      ua[nt >> 1][(nt & 1) * 2 + 0] = lo;
-      ua[nt >> 1][(nt & 1) * 2 + 1] = hi;
-    }
-    // (2b) accO += U^T A_qk^T, for the token tiles this warp finishes
-#pragma unroll
-    for (int ks = 0; ks < 4; ++ks) {
-      const int lrow = (lane >> 4) * 8 + (lane & 7), lcol = ks * 16 + ((lane >> 3) & 1) * 8;
-#pragma unroll
-      for (int nt = 2 * ks; nt < 8; nt += 2) {                     // A_qk[i][j] = 0 for j > i: tiles below 2 ks are empty
-        if (KS > 1 && nt / TPW != kq) continue;
-        uint32_t ba[4];
-        ldmatrix_x4(ba, Aq + rec_off(nt * 8 + lrow, lcol));
-        mma_f16(ao[nt], ua[ks], ba[0], ba[1]);
-        mma_f16(ao[nt + 1], ua[ks], ba[2], ba[3]);
-      }
-    }
-    // (3) S^T = S^T diag(e^{G_C}) + U^T k~, this warp's K columns
-#pragma unroll
-    for (int j = 0; j < NKT; ++j) {
-      const float2 d2 = *reinterpret_cast<const float2*>(&dv[(kq * NKT + j) * 8 + 2 * t4]);
-      st[j][0] *= d2.x; st[j][1] *= d2.y; st[j][2] *= d2.x; st[j][3] *= d2.y;
-    }
-#pragma unroll
-    for (int ks = 0; ks < 4; ++ks) {
-      const int krow = ks * 16 + ((lane >> 3) & 1) * 8 + (lane & 7);            // k~ rows are tokens: transposing form
-#pragma unroll
-      for (int j = 0; j < NKT; j += 2) {
-        uint32_t bk[4];
-        ldmatrix_x4_t(bk, Kt + ki_off(krow, kq * NKT + j + (lane >> 4)));
-        mma_f16(st[j], ua[ks], bk[0], bk[1]);
-        mma_f16(st[j + 1], ua[ks], bk[2], bk[3]);
+        const int s = c % KS_NST;
+        if (!mbar_wait(&bars->empty[s], ((c / KS_NST) & 1) ^ 1, abort_flag, p.status, 1)) break;
+        mbar_expect_tx(&bars->full[s], REC_BYTES);
+        bulk_g2s(stages + s * KS_STAGE, recs + (size_t)c * REC_BYTES, REC_BYTES, &bars->full[s]);
       }
     }
     __syncwarp();
-    if (lane == 0) mbar_arrive(&empty[s]);                         // this warp is done with the stage
-
-    // output: stage [token][v] in shared memory, then coalesced rows
-    asm volatile("bar.sync 1, %0;" ::"n"(32 * CW) : "memory");    // previous chunk's copy-out finished
+  } else if (warp == 8) {
+    // ------------------------------------------------------------ MMA issuer
+    const uint32_t leader = elect_one() ? 1u : 0u;
+    constexpr uint32_t id_u = umma_idesc_f16(128, KC, 0, 1), id_o = umma_idesc_f16(128, KC, 0, 0), id_s = umma_idesc_f16(128, KD, 0, 1);
+    const uint32_t base = smem_u32(stages);
+    const uint64_t wd = umma_desc_sw128(base + OFF_WT, KC * 128, 1024), kd = umma_desc_sw128(base + OFF_KT, KC * 128, 1024);   // depth = rows
+    const uint64_t qd = umma_desc_sw128(base + OFF_QT, 16, 1024), ad = umma_desc_sw128(base + OFF_AQK, 16, 1024);             // depth along the row
+    const uint32_t w_hi = (uint32_t)(wd >> 32), k_hi = (uint32_t)(kd >> 32), q_hi = (uint32_t)(qd >> 32), a_hi = (uint32_t)(ad >> 32);
+    for (int c = 0; c < n_chunks; ++c) {
+      const uint32_t s = c % KS_NST, so = s * (KS_STAGE >> 4), o = tmem + TM_O + KC * (c & 1);
+      if (!mbar_wait(&bars->full[s], (c / KS_NST) & 1, abort_flag, p.status, 2)) break;
+      if (!mbar_wait(&bars->s16, c & 1, abort_flag, p.status, 3)) break;
+      tc_fence_after();
 #pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
-      if (KS > 1 && nt / TPW != kq) continue;
-      const int tok = nt * 8 + 2 * t4;
-      o_stage[tok * L::O_LD + vr0] = ao[nt][0]; o_stage[(tok + 1) * L::O_LD + vr0] = ao[nt][1];
-      o_stage[tok * L::O_LD + vr1] = ao[nt][2]; o_stage[(tok + 1) * L::O_LD + vr1] = ao[nt][3];
+      for (int k = 0; k < 8; ++k) umma_ts_lh_p(leader, tmem + TM_U, tmem + TM_S16 + 8 * k, (uint32_t)wd + so + k * (2048 >> 4), w_hi, id_u, k ? 1u : 0u);
+      tc_commit_p(leader, &bars->u);
+      if (!mbar_wait(&bars->o_free[c & 1], ((c >> 1) & 1) ^ 1, abort_flag, p.status, 4)) break;
+      tc_fence_after();
+#pragma unroll
+      for (int k = 0; k < 8; ++k) umma_ts_lh_p(leader, o, tmem + TM_S16 + 8 * k, (uint32_t)qd + so + ((k >> 2) * (KC * 128) + (k & 3) * 32) / 16, q_hi, id_o, k ? 1u : 0u);
+      if (!mbar_wait(&bars->u16, c & 1, abort_flag, p.status, 5)) break;
+      tc_fence_after();
+#pragma unroll
+      for (int k = 0; k < 4; ++k) umma_ts_lh_p(leader, tmem + TM_S, tmem + TM_U16 + 8 * k, (uint32_t)kd + so + k * (2048 >> 4), k_hi, id_s, 1u);
+      tc_commit_p(leader, &bars->s);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) umma_ts_lh_p(leader, o, tmem + TM_U16 + 8 * k, (uint32_t)ad + so + k * 2, a_hi, id_o, 1u);
+      tc_commit_p(leader, &bars->o_full[c & 1]);
+      tc_commit_p(leader, &bars->empty[s]);
     }
-    asm volatile("bar.sync 1, %0;" ::"n"(32 * CW) : "memory");
-    int t0, rows;
-    ki_chunk_span(p.chunk_tab, c_begin + c, p.T, t0, rows);
-    for (int idx = threadIdx.x; idx < KC * (VS / 4); idx += 32 * CW) {
-      const int tok = idx / (VS / 4), v4 = (idx % (VS / 4)) * 4;
-      if (tok >= rows) continue;
-      const float4 x = *reinterpret_cast<const float4*>(&o_stage[tok * L::O_LD + v4]);
-      const size_t off = (((size_t)b * p.T + (size_t)t0 + tok) * p.H + h) * KD + v_base + v4;
+    __syncwarp();
+  } else if (warp < 4) {
+    // ------------------------------------------------------------ the chain: thread = value column
+    const int v = 32 * warp + lane;
+    const uint32_t t = tmem + ((uint32_t)(32 * warp) << 16);
+    {
+      const float* hp = p.h0 ? p.h0 + (size_t)bh * KD * KD + v : nullptr;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        uint32_t x[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) x[i] = hp ? __float_as_uint(hp[(size_t)(32 * j + i) * KD]) : 0u;
+        tmem_st32(t + TM_S + 32 * j, x);
+      }
+      tc_wait_st();
+    }
+    bool ok = true;
+    for (int c = 0; c < n_chunks; ++c) {
+      const int s = c % KS_NST;
+      const uint8_t* rec = stages + s * KS_STAGE;
+      ok = __all_sync(0xffffffffu, c == 0 || mbar_wait(&bars->s, (c - 1) & 1, abort_flag, p.status, 6));
+      if (!ok) break;
+      tc_fence_after();
+      uint32_t x[128];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) tmem_ld32(t + TM_S + 32 * j, x + 32 * j);
+      tc_wait_ld();
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        uint32_t y[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) y[i] = pack_h2(__uint_as_float(x[32 * j + 2 * i]), __uint_as_float(x[32 * j + 2 * i + 1]));
+        tmem_st16(t + TM_S16 + 16 * j, y);
+      }
+      tc_wait_st();
+      tc_fence_before();
+      mbar_arrive(&bars->s16);
+      // beside the U products: scale the state, fetch this column of U0
+      ok = __all_sync(0xffffffffu, mbar_wait(&bars->full[s], (c / KS_NST) & 1, abort_flag, p.status, 7));
+      if (!ok) break;
+      const float4* dv = reinterpret_cast<const float4*>(rec + OFF_D);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float4 d = dv[8 * j + i];
+          uint32_t* xx = x + 32 * j + 4 * i;
+          unpack2f(fmul2(pack2f(__uint_as_float(xx[0]), __uint_as_float(xx[1])), pack2f(d.x, d.y)), reinterpret_cast<float&>(xx[0]), reinterpret_cast<float&>(xx[1]));
+          unpack2f(fmul2(pack2f(__uint_as_float(xx[2]), __uint_as_float(xx[3])), pack2f(d.z, d.w)), reinterpret_cast<float&>(xx[2]), reinterpret_cast<float&>(xx[3]));
+        }
+        tmem_st32(t + TM_S + 32 * j, x + 32 * j);
+      }
+      uint32_t u0[32];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) *reinterpret_cast<uint4*>(u0 + 4 * j) = *reinterpret_cast<const uint4*>(rec + OFF_UT + rec_off(v, 8 * j));
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars->empty[s]);
+      ok = __all_sync(0xffffffffu, mbar_wait(&bars->u, c & 1, abort_flag, p.status, 8));
+      if (!ok) break;
+      tc_fence_after();
+      tmem_ld32(t + TM_U, x);
+      tmem_ld32(t + TM_U + 32, x + 32);
+      tc_wait_ld();
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        const float2 u = unpack_h2(u0[i]);
+        u0[i] = pack_h2(u.x - __uint_as_float(x[2 * i]), u.y - __uint_as_float(x[2 * i + 1]));
+      }
+      tmem_st32(t + TM_U16, u0);
+      tc_wait_st();
+      tc_fence_before();
+      mbar_arrive(&bars->u16);
+    }
+    if (ok && n_chunks > 0) ok = __all_sync(0xffffffffu, mbar_wait(&bars->s, (n_chunks - 1) & 1, abort_flag, p.status, 9));
+    if (ok && p.hT) {
+      tc_fence_after();
+      float* hp = p.hT + (size_t)bh * KD * KD + v;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        uint32_t x[32];
+        tmem_ld32(t + TM_S + 32 * j, x);
+        tc_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 32; ++i) hp[(size_t)(32 * j + i) * KD] = __uint_as_float(x[i]);
+      }
+    }
+  } else {
+    // ------------------------------------------------------------ output: thread = value column, a warp stores 32 of a token's row
+    const int v = 32 * (warp - 4) + lane;
+    const uint32_t t = tmem + ((uint32_t)(32 * (warp - 4)) << 16) + TM_O;
+    for (int c = 0; c < n_chunks; ++c) {
+      if (!__all_sync(0xffffffffu, mbar_wait(&bars->o_full[c & 1], (c >> 1) & 1, abort_flag, p.status, 10))) break;
+      tc_fence_after();
+      uint32_t x[64];
+      tmem_ld32(t + KC * (c & 1), x);
+      tmem_ld32(t + KC * (c & 1) + 32, x + 32);
+      tc_wait_ld();
+      tc_fence_before();
+      mbar_arrive(&bars->o_free[c & 1]);
+      int t0, rows;
+      ki_chunk_span(p.chunk_tab, c_begin + c, p.T, t0, rows);
+      const size_t off = (((size_t)b * p.T + t0) * p.H + h) * KD + v, ts = (size_t)p.H * KD;
       if (p.out_fp32) {
-        *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.o) + off) = x;
+        float* o = reinterpret_cast<float*>(p.o) + off;
+#pragma unroll
+        for (int i = 0; i < KC; ++i) if (i < rows) o[i * ts] = __uint_as_float(x[i]);
       } else {
-        uint2 pk = make_uint2(pack_bf16(x.x, x.y), pack_bf16(x.z, x.w));
-        *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.o) + off) = pk;
+        __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.o) + off;
+#pragma unroll
+        for (int i = 0; i < KC; ++i) if (i < rows) o[i * ts] = __float2bfloat16_rn(__uint_as_float(x[i]));
       }
     }
   }
 
-  if (p.hT) {
-    float* hp = p.hT + (size_t)bh * KD * KD;
-#pragma unroll
-    for (int j = 0; j < NKT; ++j) {
-      const int k0 = (kq * NKT + j) * 8 + 2 * t4;
-      hp[(size_t)k0 * KD + v_base + vr0] = st[j][0]; hp[(size_t)(k0 + 1) * KD + v_base + vr0] = st[j][1];
-      hp[(size_t)k0 * KD + v_base + vr1] = st[j][2]; hp[(size_t)(k0 + 1) * KD + v_base + vr1] = st[j][3];
-    }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 8) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 512);
   }
 }
 
@@ -781,21 +759,6 @@ extern "C" size_t daisy_b200_kda_workspace_bytes(int B, int T, int H, int K, int
   if (B <= 0 || T <= 0 || H <= 0 || K != KD || V != KD) return 0;
   const size_t nc = (size_t)(T + KC - 1) / KC;
   return (size_t)B * H * nc * REC_BYTES;
-}
-
-template <int NW, int KS, int NST>
-static int launch_state(const KdaStateParams& sp, int BH, cudaStream_t st) {
-  using L = KdaStateSmem<NW, KS, NST>;
-  static_assert(L::BYTES <= 232448, "over the 227 KB a CTA may use");
-  static bool attr[daisy_host::MAX_DEVICES] = {};             // the attribute is per device
-  const int dev = daisy_host::device_slot();
-  if (dev < 0) return DAISY_ENODEV;
-  if (!attr[dev]) {
-    if (cudaFuncSetAttribute(kda_state_kernel<NW, KS, NST>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::BYTES) != cudaSuccess) return DAISY_ECUDA;
-    attr[dev] = true;
-  }
-  kda_state_kernel<NW, KS, NST><<<dim3(KD / L::VS, BH), 32 * (L::CW + 1), L::BYTES, st>>>(sp);
-  return cudaGetLastError() == cudaSuccess ? DAISY_OK : DAISY_ECUDA;
 }
 
 // Shared launcher.  Dense: NC = ceil(T / 64) chunks per (batch, head) row, n_seq = B.  Packed variable-length (B = 1):
@@ -818,7 +781,8 @@ static int kda_launch(const void* q, const void* k, const void* v, const float* 
   if (dev < 0) return DAISY_ENODEV;
   constexpr int intra_smem = (int)sizeof(KdaIntraSmem);
   if (!attr[dev]) {
-    if (cudaFuncSetAttribute(kda_intra_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, intra_smem) != cudaSuccess) {
+    if (cudaFuncSetAttribute(kda_intra_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, intra_smem) != cudaSuccess ||
+        cudaFuncSetAttribute(kda_state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, KS_SMEM) != cudaSuccess) {
       (void)cudaGetLastError();
       return DAISY_ECUDA;
     }
@@ -840,13 +804,11 @@ static int kda_launch(const void* q, const void* k, const void* v, const float* 
   sp.T = T; sp.H = H; sp.NC = NC; sp.out_fp32 = (flags & DAISY_KDA_OUT_FP32) ? 1 : 0;
   sp.status = status_word;
   sp.chunk_tab = chunk_tab; sp.seq_ptr = seq_ptr;
-  const int BH = n_seq * H;
-  // V-slices: 64 rows (4 warps) fill the machine when there are >= 48 (sequence, head) pairs; fewer take narrower slices
-  int rc;
-  if (BH * 2 >= 96) rc = launch_state<4, 1, 2>(sp, BH, st);
-  else if (BH * 4 >= 96) rc = launch_state<2, 2, 2>(sp, BH, st);
-  else rc = launch_state<1, 2, 3>(sp, BH, st);
-  if (rc != DAISY_OK) { (void)cudaGetLastError(); return rc; }
+  if (daisy_host::launch_dependent(kda_state_kernel, dim3(n_seq * H), dim3(KS_THREADS), KS_SMEM, st, sp) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return DAISY_ECUDA;
+  }
+  DAISY_CHECK_LAUNCH();
   return DAISY_OK;
 }
 

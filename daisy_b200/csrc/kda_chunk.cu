@@ -543,24 +543,31 @@ struct KdaStateParams {
 //     O^T [V x 64]   = S^T q~^T + U^T A_qk^T
 //     S^T [V x 128] <- S^T diag(e^{G_C}) + U^T k~  accumulated in TMEM on the scaled state
 // The chain from chunk to chunk is all that matters (a (batch, head) is serial, and there are rarely more of them than SMs):
-// read S -> fp16 -> 8 products of N = 64 -> subtract -> fp16 -> 4 products of N = 128.  Warps 0-3 (thread = value column) run
-// that chain; everything else is beside it: they scale the state while the U products run, q~'s products fill the tensor pipe
-// while U is converted, warps 4-7 write O out of two accumulators, warp 8 issues, warp 9 keeps the ring full.
-// The same chain in mma.sync fragments, 64 value columns to a CTA, took 3700 cycles a chunk (212 products of a warp on one
-// tensor pipe and as many cycles of ldmatrix): 500 us at 4 x 16384 x 16 against 418 here.
+// S to fp16, 8 products of N = 64, U to fp16, 4 products of N = 128.  Warps 0-7 (thread = half a value column) run it with the
+// state in fp32 registers, scaled while the U products run; TMEM carries only fp16 operands and fresh sums.  Two warps to a
+// scheduler: one warp's conversions alone are twice as long as the products.  q~'s products fill the tensor pipe while U is
+// converted, warps 8-11 write O out of two accumulators, transposed through the record's spent W^T, warp 12 issues, warp 13
+// keeps the ring full.
+// The same recurrence in mma.sync fragments, 64 value columns to a CTA, took 3700 cycles a chunk (212 products of a warp on
+// one tensor pipe and as many cycles of ldmatrix): 500 us at 4 x 16384 x 16.  With the state in TMEM, scaled there, 2850
+// cycles, 418 us; this form 2560 cycles, 365 us.
 constexpr int KS_NST = 3;
 constexpr int KS_STAGE = (REC_BYTES + 1023) / 1024 * 1024;     // operands start on 1024-byte boundaries
-constexpr int KS_THREADS = 320;
-constexpr int TM_S = 0, TM_S16 = 128, TM_U = 192, TM_U16 = 256, TM_O = 288;      // TMEM columns; O: two accumulators of 64
+constexpr int KS_THREADS = 448;
+constexpr int TM_D = 0, TM_S16 = 128, TM_U = 192, TM_U16 = 256, TM_O = 288;      // TMEM columns; D: the state's increment; O: two accumulators of 64
 static_assert(OFF_QT % 1024 == 0 && OFF_KT % 1024 == 0 && OFF_AQK % 1024 == 0, "swizzled operands");
 struct KdaStateBars {
   uint64_t full[KS_NST], empty[KS_NST];
-  uint64_t s16, u, u16, s, o_full[2], o_free[2];
+  uint64_t s16[2], u, u16, s, o_full[2], o_free[2];
   uint32_t tmem_base;
   int abort_flag;
 };
 constexpr int KS_SMEM = 1024 + KS_NST * KS_STAGE + (int)sizeof(KdaStateBars);
 static_assert(KS_SMEM <= 232448, "over the 227 KB a CTA may use");
+
+__device__ __forceinline__ void ld_shared16(uint32_t* r, uint32_t addr) {
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
 
 __global__ void __launch_bounds__(KS_THREADS, 1) kda_state_kernel(const KdaStateParams p) {
   extern __shared__ uint8_t kda_smem_raw[];
@@ -570,13 +577,13 @@ __global__ void __launch_bounds__(KS_THREADS, 1) kda_state_kernel(const KdaState
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < KS_NST; ++i) { mbar_init(&bars->full[i], 1); mbar_init(&bars->empty[i], 5); }       // 4 state warps, 1 commit
-    mbar_init(&bars->s16, 128); mbar_init(&bars->u, 1); mbar_init(&bars->u16, 128); mbar_init(&bars->s, 1);
+    for (int i = 0; i < KS_NST; ++i) { mbar_init(&bars->full[i], 1); mbar_init(&bars->empty[i], 12); }      // warps 0-11
+    mbar_init(&bars->s16[0], 128); mbar_init(&bars->s16[1], 128); mbar_init(&bars->u, 1); mbar_init(&bars->u16, 256); mbar_init(&bars->s, 1);
     for (int i = 0; i < 2; ++i) { mbar_init(&bars->o_full[i], 1); mbar_init(&bars->o_free[i], 128); }
     bars->abort_flag = 0;
     mbar_init_fence();
   }
-  if (warp == 8) { tmem_alloc(&bars->tmem_base, 512); tmem_relinquish(); }
+  if (warp == 12) { tmem_alloc(&bars->tmem_base, 512); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -587,7 +594,7 @@ __global__ void __launch_bounds__(KS_THREADS, 1) kda_state_kernel(const KdaState
   const int c_begin = p.seq_ptr ? p.seq_ptr[bh / p.H] : 0, c_end = p.seq_ptr ? p.seq_ptr[bh / p.H + 1] : p.NC;
   const int n_chunks = c_end - c_begin;
 
-  if (warp == 9) {
+  if (warp == 13) {
     // ------------------------------------------------------------ producer: one record a stage
     if (lane == 0) {
       const uint8_t* recs = p.ws + ((size_t)(b * p.H + h) * p.NC + c_begin) * REC_BYTES;
@@ -599,7 +606,7 @@ __global__ void __launch_bounds__(KS_THREADS, 1) kda_state_kernel(const KdaState
       }
     }
     __syncwarp();
-  } else if (warp == 8) {
+  } else if (warp == 12) {
     // ------------------------------------------------------------ MMA issuer
     const uint32_t leader = elect_one() ? 1u : 0u;
     constexpr uint32_t id_u = umma_idesc_f16(128, KC, 0, 1), id_o = umma_idesc_f16(128, KC, 0, 0), id_s = umma_idesc_f16(128, KD, 0, 1);
@@ -610,10 +617,14 @@ __global__ void __launch_bounds__(KS_THREADS, 1) kda_state_kernel(const KdaState
     for (int c = 0; c < n_chunks; ++c) {
       const uint32_t s = c % KS_NST, so = s * (KS_STAGE >> 4), o = tmem + TM_O + KC * (c & 1);
       if (!mbar_wait(&bars->full[s], (c / KS_NST) & 1, abort_flag, p.status, 2)) break;
-      if (!mbar_wait(&bars->s16, c & 1, abort_flag, p.status, 3)) break;
+      if (!mbar_wait(&bars->s16[0], c & 1, abort_flag, p.status, 3)) break;
       tc_fence_after();
 #pragma unroll
-      for (int k = 0; k < 8; ++k) umma_ts_lh_p(leader, tmem + TM_U, tmem + TM_S16 + 8 * k, (uint32_t)wd + so + k * (2048 >> 4), w_hi, id_u, k ? 1u : 0u);
+      for (int k = 0; k < 4; ++k) umma_ts_lh_p(leader, tmem + TM_U, tmem + TM_S16 + 8 * k, (uint32_t)wd + so + k * (2048 >> 4), w_hi, id_u, k ? 1u : 0u);
+      if (!mbar_wait(&bars->s16[1], c & 1, abort_flag, p.status, 3)) break;
+      tc_fence_after();
+#pragma unroll
+      for (int k = 4; k < 8; ++k) umma_ts_lh_p(leader, tmem + TM_U, tmem + TM_S16 + 8 * k, (uint32_t)wd + so + k * (2048 >> 4), w_hi, id_u, 1u);
       tc_commit_p(leader, &bars->u);
       if (!mbar_wait(&bars->o_free[c & 1], ((c >> 1) & 1) ^ 1, abort_flag, p.status, 4)) break;
       tc_fence_after();
@@ -622,104 +633,94 @@ __global__ void __launch_bounds__(KS_THREADS, 1) kda_state_kernel(const KdaState
       if (!mbar_wait(&bars->u16, c & 1, abort_flag, p.status, 5)) break;
       tc_fence_after();
 #pragma unroll
-      for (int k = 0; k < 4; ++k) umma_ts_lh_p(leader, tmem + TM_S, tmem + TM_U16 + 8 * k, (uint32_t)kd + so + k * (2048 >> 4), k_hi, id_s, 1u);
+      for (int k = 0; k < 4; ++k) umma_ts_lh_p(leader, tmem + TM_D, tmem + TM_U16 + 8 * k, (uint32_t)kd + so + k * (2048 >> 4), k_hi, id_s, k ? 1u : 0u);
       tc_commit_p(leader, &bars->s);
 #pragma unroll
       for (int k = 0; k < 4; ++k) umma_ts_lh_p(leader, o, tmem + TM_U16 + 8 * k, (uint32_t)ad + so + k * 2, a_hi, id_o, 1u);
       tc_commit_p(leader, &bars->o_full[c & 1]);
-      tc_commit_p(leader, &bars->empty[s]);
     }
     __syncwarp();
-  } else if (warp < 4) {
-    // ------------------------------------------------------------ the chain: thread = value column
-    const int v = 32 * warp + lane;
-    const uint32_t t = tmem + ((uint32_t)(32 * warp) << 16);
+  } else if (warp < 8) {
+    // ------------------------------------------------------------ the chain: thread = half of a value column
+    const int half = warp >> 2, v = 32 * (warp & 3) + lane;
+    const uint32_t t = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+    float S[64];                                                                   // row v of S^T, channels 64 half ..
     {
-      const float* hp = p.h0 ? p.h0 + (size_t)bh * KD * KD + v : nullptr;
+      const float* hp = p.h0 ? p.h0 + (size_t)bh * KD * KD + 64 * half * KD + v : nullptr;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        uint32_t x[32];
-#pragma unroll
-        for (int i = 0; i < 32; ++i) x[i] = hp ? __float_as_uint(hp[(size_t)(32 * j + i) * KD]) : 0u;
-        tmem_st32(t + TM_S + 32 * j, x);
-      }
-      tc_wait_st();
+      for (int i = 0; i < 64; ++i) S[i] = hp ? hp[(size_t)i * KD] : 0.f;
     }
     bool ok = true;
-    for (int c = 0; c < n_chunks; ++c) {
-      const int s = c % KS_NST;
-      const uint8_t* rec = stages + s * KS_STAGE;
-      ok = __all_sync(0xffffffffu, c == 0 || mbar_wait(&bars->s, (c - 1) & 1, abort_flag, p.status, 6));
-      if (!ok) break;
-      tc_fence_after();
-      uint32_t x[128];
+    for (int c = 0; c <= n_chunks; ++c) {
+      if (c > 0) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&bars->s, (c - 1) & 1, abort_flag, p.status, 6));
+        if (!ok) break;
+        tc_fence_after();
 #pragma unroll
-      for (int j = 0; j < 4; ++j) tmem_ld32(t + TM_S + 32 * j, x + 32 * j);
-      tc_wait_ld();
+        for (int j = 0; j < 2; ++j) {
+          uint32_t x[32];
+          tmem_ld32(t + TM_D + 64 * half + 32 * j, x);
+          tc_wait_ld();
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        uint32_t y[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) y[i] = pack_h2(__uint_as_float(x[32 * j + 2 * i]), __uint_as_float(x[32 * j + 2 * i + 1]));
-        tmem_st16(t + TM_S16 + 16 * j, y);
+          for (int i = 0; i < 32; ++i) S[32 * j + i] += __uint_as_float(x[i]);
+        }
       }
+      if (c == n_chunks) break;
+      uint32_t y[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) y[i] = pack_h2(S[2 * i], S[2 * i + 1]);
+      tmem_st32(t + TM_S16 + 32 * half, y);
       tc_wait_st();
       tc_fence_before();
-      mbar_arrive(&bars->s16);
-      // beside the U products: scale the state, fetch this column of U0
+      mbar_arrive(&bars->s16[half]);
+      // beside the U products: scale the state, fetch this column's 32 tokens of U0
+      const int s = c % KS_NST;
       ok = __all_sync(0xffffffffu, mbar_wait(&bars->full[s], (c / KS_NST) & 1, abort_flag, p.status, 7));
       if (!ok) break;
-      const float4* dv = reinterpret_cast<const float4*>(rec + OFF_D);
+      const uint32_t rec = smem_u32(stages) + s * KS_STAGE;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
+      for (int j = 0; j < 2; ++j) {
+        uint32_t d[32];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const float4 d = dv[8 * j + i];
-          uint32_t* xx = x + 32 * j + 4 * i;
-          unpack2f(fmul2(pack2f(__uint_as_float(xx[0]), __uint_as_float(xx[1])), pack2f(d.x, d.y)), reinterpret_cast<float&>(xx[0]), reinterpret_cast<float&>(xx[1]));
-          unpack2f(fmul2(pack2f(__uint_as_float(xx[2]), __uint_as_float(xx[3])), pack2f(d.z, d.w)), reinterpret_cast<float&>(xx[2]), reinterpret_cast<float&>(xx[3]));
-        }
-        tmem_st32(t + TM_S + 32 * j, x + 32 * j);
+        for (int i = 0; i < 8; ++i) ld_shared16(d + 4 * i, rec + OFF_D + 256 * half + 128 * j + 16 * i);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) S[32 * j + i] *= __uint_as_float(d[i]);
       }
-      uint32_t u0[32];
+      uint32_t u0[16];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) *reinterpret_cast<uint4*>(u0 + 4 * j) = *reinterpret_cast<const uint4*>(rec + OFF_UT + rec_off(v, 8 * j));
+      for (int j = 0; j < 4; ++j) ld_shared16(u0 + 4 * j, rec + OFF_UT + rec_off(v, 32 * half + 8 * j));
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars->empty[s]);
       ok = __all_sync(0xffffffffu, mbar_wait(&bars->u, c & 1, abort_flag, p.status, 8));
       if (!ok) break;
       tc_fence_after();
-      tmem_ld32(t + TM_U, x);
-      tmem_ld32(t + TM_U + 32, x + 32);
+      tmem_ld32(t + TM_U + 32 * half, y);
       tc_wait_ld();
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
+      for (int i = 0; i < 16; ++i) {
         const float2 u = unpack_h2(u0[i]);
-        u0[i] = pack_h2(u.x - __uint_as_float(x[2 * i]), u.y - __uint_as_float(x[2 * i + 1]));
+        u0[i] = pack_h2(u.x - __uint_as_float(y[2 * i]), u.y - __uint_as_float(y[2 * i + 1]));
       }
-      tmem_st32(t + TM_U16, u0);
+      tmem_st16(t + TM_U16 + 16 * half, u0);
       tc_wait_st();
       tc_fence_before();
       mbar_arrive(&bars->u16);
     }
-    if (ok && n_chunks > 0) ok = __all_sync(0xffffffffu, mbar_wait(&bars->s, (n_chunks - 1) & 1, abort_flag, p.status, 9));
     if (ok && p.hT) {
-      tc_fence_after();
-      float* hp = p.hT + (size_t)bh * KD * KD + v;
+      float* hp = p.hT + (size_t)bh * KD * KD + 64 * half * KD + v;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        uint32_t x[32];
-        tmem_ld32(t + TM_S + 32 * j, x);
-        tc_wait_ld();
-#pragma unroll
-        for (int i = 0; i < 32; ++i) hp[(size_t)(32 * j + i) * KD] = __uint_as_float(x[i]);
-      }
+      for (int i = 0; i < 64; ++i) hp[(size_t)i * KD] = S[i];
     }
   } else {
-    // ------------------------------------------------------------ output: thread = value column, a warp stores 32 of a token's row
-    const int v = 32 * (warp - 4) + lane;
-    const uint32_t t = tmem + ((uint32_t)(32 * (warp - 4)) << 16) + TM_O;
+    // ------------------------------------------------------------ output: a warp's 64 tokens x 32 columns, bf16 in 64-byte stores.
+    // Its columns lie as rows of 64 tokens in shared memory, from where a transposing ldmatrix gives a lane eight columns of a token:
+    // rows 2 j, 2 j + 1 of matrix m are columns 8 j + 2 m, + 1.  Pieces are exchanged by (v & 7) ^ 2 (v >> 3): both the eight
+    // lanes of a store and the eight rows of a matrix hit different banks
+    const int w = warp - 8;
+    const uint32_t t = tmem + ((uint32_t)(32 * w) << 16) + TM_O;
+    const int vr = 8 * ((lane & 7) >> 1) + 2 * (lane >> 3) + (lane & 1);           // the row this lane addresses
     for (int c = 0; c < n_chunks; ++c) {
+      const int s = c % KS_NST;
       if (!__all_sync(0xffffffffu, mbar_wait(&bars->o_full[c & 1], (c >> 1) & 1, abort_flag, p.status, 10))) break;
       tc_fence_after();
       uint32_t x[64];
@@ -730,22 +731,40 @@ __global__ void __launch_bounds__(KS_THREADS, 1) kda_state_kernel(const KdaState
       mbar_arrive(&bars->o_free[c & 1]);
       int t0, rows;
       ki_chunk_span(p.chunk_tab, c_begin + c, p.T, t0, rows);
-      const size_t off = (((size_t)b * p.T + t0) * p.H + h) * KD + v, ts = (size_t)p.H * KD;
+      const size_t off = (((size_t)b * p.T + t0) * p.H + h) * KD + 32 * w, ts = (size_t)p.H * KD;
       if (p.out_fp32) {
-        float* o = reinterpret_cast<float*>(p.o) + off;
+        float* o = reinterpret_cast<float*>(p.o) + off + lane;
 #pragma unroll
         for (int i = 0; i < KC; ++i) if (i < rows) o[i * ts] = __uint_as_float(x[i]);
       } else {
-        __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.o) + off;
+        const uint32_t stg = smem_u32(stages) + s * KS_STAGE + OFF_WT + w * 4096;  // the products that read it are done
 #pragma unroll
-        for (int i = 0; i < KC; ++i) if (i < rows) o[i * ts] = __float2bfloat16_rn(__uint_as_float(x[i]));
+        for (int j = 0; j < 8; ++j) {
+          const uint32_t* xx = x + 8 * j;
+          asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};"
+                       ::"r"(stg + lane * 128 + ((j ^ ((lane & 7) ^ (2 * (lane >> 3)))) << 4)),
+                       "r"(pack_bf16(__uint_as_float(xx[0]), __uint_as_float(xx[1]))), "r"(pack_bf16(__uint_as_float(xx[2]), __uint_as_float(xx[3]))),
+                       "r"(pack_bf16(__uint_as_float(xx[4]), __uint_as_float(xx[5]))), "r"(pack_bf16(__uint_as_float(xx[6]), __uint_as_float(xx[7]))) : "memory");
+        }
+        __syncwarp();
+        __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.o) + off + 8 * (lane & 3);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) ldmatrix_x4_t(x + 4 * j, stg + vr * 128 + ((j ^ ((vr & 7) ^ (2 * (vr >> 3)))) << 4));
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int tok = 8 * j + (lane >> 2);
+          if (tok < rows) st_global16(o + tok * ts, x[4 * j], x[4 * j + 1], x[4 * j + 2], x[4 * j + 3]);
+        }
+        fence_proxy_async();                                                       // the next record lands where this was staged
       }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars->empty[s]);
     }
   }
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 8) {
+  if (warp == 12) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);
   }

@@ -34,6 +34,9 @@ constexpr int SHARED_BYTES = OFF_D + KD * 4;           // 57856: identical for e
 constexpr int OFF_UT = SHARED_BYTES;                   // U0^T     [128 value columns][64 tokens] fp16
 constexpr int REC_BYTES = OFF_UT + KD * KC * 2;        // 74240
 static_assert(SHARED_BYTES % 16 == 0 && REC_BYTES % 16 == 0, "bulk copies move 16-byte units");
+// what a caller provides per record: part of the ABI, from when records had padded rows; the record uses the front of the buffer
+constexpr size_t WS_REC_BYTES = 83456;
+static_assert(REC_BYTES <= WS_REC_BYTES, "a record fits what callers provide");
 
 // byte offset of (row, token column) in an image of 64-token rows (128 bytes, 16-byte pieces exchanged by row)
 __device__ __forceinline__ uint32_t rec_off(int row, int col) { return (uint32_t)(row * 128 + (((col >> 3) ^ (row & 7)) << 4) + (col & 7) * 2); }
@@ -777,7 +780,7 @@ using namespace daisy;
 extern "C" size_t daisy_b200_kda_workspace_bytes(int B, int T, int H, int K, int V) {
   if (B <= 0 || T <= 0 || H <= 0 || K != KD || V != KD) return 0;
   const size_t nc = (size_t)(T + KC - 1) / KC;
-  return (size_t)B * H * nc * REC_BYTES;
+  return (size_t)B * H * nc * WS_REC_BYTES;
 }
 
 // Shared launcher.  Dense: NC = ceil(T / 64) chunks per (batch, head) row, n_seq = B.  Packed variable-length (B = 1):
@@ -790,7 +793,7 @@ static int kda_launch(const void* q, const void* k, const void* v, const float* 
   if (!q || !k || !v || !g || !beta || !o || !workspace || B <= 0 || T <= 0 || H <= 0 || NC <= 0 || n_seq <= 0) return DAISY_EINVAL;
   if (K != KD || V != KD || chunk != KC) return DAISY_EUNSUPPORTED;
   if (B > 65535 || H > 65535 || (size_t)n_seq * H > 65535) return DAISY_EUNSUPPORTED;
-  if (workspace_bytes < (size_t)B * H * NC * REC_BYTES) return DAISY_EWORKSPACE;
+  if (workspace_bytes < (size_t)B * H * NC * WS_REC_BYTES) return DAISY_EWORKSPACE;
   if (!daisy_aligned16(q) || !daisy_aligned16(k) || !daisy_aligned16(v) || !daisy_aligned16(g) || !daisy_aligned16(o) ||
       !daisy_aligned16(workspace) || (h0 && !daisy_aligned16(h0)) || (hT && !daisy_aligned16(hT)))
     return DAISY_EALIGN;
@@ -843,7 +846,7 @@ extern "C" int daisy_b200_kda_chunk_fwd(const void* q, const void* k, const void
 
 extern "C" size_t daisy_b200_kda_varlen_workspace_bytes(int n_chunks, int H, int K, int V) {
   if (n_chunks <= 0 || H <= 0 || K != KD || V != KD) return 0;
-  return (size_t)H * n_chunks * REC_BYTES;
+  return (size_t)H * n_chunks * WS_REC_BYTES;
 }
 
 extern "C" int daisy_b200_kda_chunk_fwd_varlen(const void* q, const void* k, const void* v, const float* g,

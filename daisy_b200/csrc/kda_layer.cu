@@ -30,6 +30,10 @@ struct ShortConvParams {
                                  // s_in / s_out are then [n_seq, C, W]
 };
 
+// up to three convolutions of one shape (q, k and v) in one launch
+constexpr int SC_GROUP = 3;
+struct ShortConvGroup { ShortConvParams p[SC_GROUP]; int n; };
+
 __device__ __forceinline__ void unpack4(const uint2 u, float* f) {
   f[0] = bf16_lo(u.x); f[1] = bf16_hi(u.x); f[2] = bf16_lo(u.y); f[3] = bf16_hi(u.y);
 }
@@ -60,10 +64,11 @@ __device__ __forceinline__ uint4 conv_state_row(const ShortConvParams& p, int b,
 // carried state (or zeros), patched into the sliding registers at the first three rows of each sequence -- and the row
 // that ends a sequence leaves that sequence's state.
 template <bool SILU, bool VARLEN>
-__global__ void __launch_bounds__(SC_THREADS) kda_short_conv_kernel(const ShortConvParams p) {
+__global__ void __launch_bounds__(SC_THREADS) kda_short_conv_kernel(const __grid_constant__ ShortConvGroup grp) {
+  const ShortConvParams& p = grp.p[blockIdx.z % grp.n];
   __shared__ uint4 tile[SC_TILE_ROWS][SC_COLS / 8];
   const int cblk = blockIdx.x * SC_COLS;                           // channel blocks vary fastest, then time blocks:
-  const int b = blockIdx.z;                                        // CTAs launched together walk the tensor front to back
+  const int b = blockIdx.z / grp.n;                                // CTAs launched together walk the tensor front to back
   const int tblk = blockIdx.y * SC_ROWS;
   const int t_end = min(tblk + SC_ROWS, p.T);
 
@@ -281,6 +286,11 @@ __global__ void __launch_bounds__(256) kda_out_norm_kernel(const OutNormParams p
   }
 }
 
+__global__ void __launch_bounds__(256) kda_beta_kernel(const __nv_bfloat16* x, float* out, long long n) {
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (i < n) out[i] = __bfloat162float(__float2bfloat16_rn(1.f / (1.f + expf(-__bfloat162float(x[i])))));
+}
+
 template <int MODE>
 static void launch_out_norm(const OutNormParams& p, unsigned grid, cudaStream_t st) {
   if (p.o_fp32) kda_out_norm_kernel<MODE, true><<<grid, 256, 0, st>>>(p);
@@ -291,49 +301,70 @@ static void launch_out_norm(const OutNormParams& p, unsigned grid, cudaStream_t 
 
 using namespace daisy;
 
+static int short_conv_launch(int n, const void* const* x, int64_t x_sb, int64_t x_st, const void* const* w, const void* const* bias,
+                             const void* const* state_in, void* const* state_out, void* const* y, int64_t y_sb, int64_t y_st,
+                             int B, int T, int C, int W, const int32_t* tok_tab, unsigned flags, void* stream) {
+  if (n < 1 || n > SC_GROUP || B <= 0 || T <= 0 || C <= 0) return DAISY_EINVAL;
+  for (int i = 0; i < n; ++i) if (!x[i] || !w[i] || !y[i]) return DAISY_EINVAL;
+  if (W < 1 || W > SC_MAX_W || C % 8 != 0 || (int64_t)B * n > 65535 || (T + SC_ROWS - 1) / SC_ROWS > 65535) return DAISY_EUNSUPPORTED;
+  if (flags & ~DAISY_KDA_CONV_SILU) return DAISY_EINVAL;
+  if (x_sb % 8 || x_st % 8 || y_sb % 8 || y_st % 8 || (reinterpret_cast<uintptr_t>(tok_tab) & 7)) return DAISY_EALIGN;
+  ShortConvGroup g{};
+  g.n = n;
+  for (int i = 0; i < n; ++i) {
+    const void* b = bias ? bias[i] : nullptr;
+    const void* si = state_in ? state_in[i] : nullptr;
+    void* so = state_out ? state_out[i] : nullptr;
+    if (!daisy_aligned16(x[i]) || !daisy_aligned16(y[i]) || !daisy_aligned16(w[i]) || (b && !daisy_aligned16(b))) return DAISY_EALIGN;
+    // a state updated in place is read by the threads of the first rows and written by the CTA of the last: one CTA only;
+    // packed sequences end in different CTAs
+    if (si && si == so && (tok_tab || T > SC_ROWS)) return DAISY_EINVAL;
+    ShortConvParams& p = g.p[i];
+    p.x = (const __nv_bfloat16*)x[i]; p.w = (const __nv_bfloat16*)w[i]; p.bias = (const __nv_bfloat16*)b;
+    p.s_in = (const __nv_bfloat16*)si; p.s_out = (__nv_bfloat16*)so; p.y = (__nv_bfloat16*)y[i];
+    p.x_sb = x_sb; p.x_st = x_st; p.y_sb = y_sb; p.y_st = y_st;
+    p.T = T; p.C = C; p.W = W; p.silu = (flags & DAISY_KDA_CONV_SILU) ? 1 : 0;
+    p.tok = reinterpret_cast<const int2*>(tok_tab);
+  }
+  const dim3 grid((C + SC_COLS - 1) / SC_COLS, (T + SC_ROWS - 1) / SC_ROWS, B * n);
+  cudaStream_t st = (cudaStream_t)stream;
+  const bool silu = flags & DAISY_KDA_CONV_SILU;
+  if (tok_tab) {
+    if (silu) kda_short_conv_kernel<true, true><<<grid, SC_THREADS, 0, st>>>(g);
+    else      kda_short_conv_kernel<false, true><<<grid, SC_THREADS, 0, st>>>(g);
+  } else {
+    if (silu) kda_short_conv_kernel<true, false><<<grid, SC_THREADS, 0, st>>>(g);
+    else      kda_short_conv_kernel<false, false><<<grid, SC_THREADS, 0, st>>>(g);
+  }
+  DAISY_CHECK_LAUNCH();
+  return DAISY_OK;
+}
+
 extern "C" int daisy_b200_kda_short_conv(const void* x, int64_t x_sb, int64_t x_st, const void* w, const void* bias,
                                          const void* state_in, void* state_out, void* y, int64_t y_sb, int64_t y_st,
                                          int B, int T, int C, int W, unsigned flags, void* stream) {
-  if (!x || !w || !y || B <= 0 || T <= 0 || C <= 0) return DAISY_EINVAL;
-  if (W < 1 || W > SC_MAX_W || C % 8 != 0 || B > 65535 || (T + SC_ROWS - 1) / SC_ROWS > 65535) return DAISY_EUNSUPPORTED;
-  if (flags & ~DAISY_KDA_CONV_SILU) return DAISY_EINVAL;
-  if (!daisy_aligned16(x) || !daisy_aligned16(y) || !daisy_aligned16(w) || (bias && !daisy_aligned16(bias)) ||
-      x_sb % 8 || x_st % 8 || y_sb % 8 || y_st % 8)
-    return DAISY_EALIGN;
-  // a state updated in place is read by the threads of the first rows and written by the CTA of the last: one CTA only
-  if (state_in && state_in == state_out && T > SC_ROWS) return DAISY_EINVAL;
-  ShortConvParams p;
-  p.x = (const __nv_bfloat16*)x; p.w = (const __nv_bfloat16*)w; p.bias = (const __nv_bfloat16*)bias;
-  p.s_in = (const __nv_bfloat16*)state_in; p.s_out = (__nv_bfloat16*)state_out; p.y = (__nv_bfloat16*)y;
-  p.x_sb = x_sb; p.x_st = x_st; p.y_sb = y_sb; p.y_st = y_st;
-  p.T = T; p.C = C; p.W = W; p.silu = (flags & DAISY_KDA_CONV_SILU) ? 1 : 0;
-  p.tok = nullptr;
-  const dim3 grid((C + SC_COLS - 1) / SC_COLS, (T + SC_ROWS - 1) / SC_ROWS, B);
-  if (p.silu) kda_short_conv_kernel<true, false><<<grid, SC_THREADS, 0, (cudaStream_t)stream>>>(p);
-  else        kda_short_conv_kernel<false, false><<<grid, SC_THREADS, 0, (cudaStream_t)stream>>>(p);
-  DAISY_CHECK_LAUNCH();
-  return DAISY_OK;
+  return short_conv_launch(1, &x, x_sb, x_st, &w, &bias, &state_in, &state_out, &y, y_sb, y_st, B, T, C, W, nullptr, flags, stream);
 }
 
 extern "C" int daisy_b200_kda_short_conv_varlen(const void* x, int64_t x_st, const void* w, const void* bias,
                                                 const void* state_in, void* state_out, void* y, int64_t y_st,
                                                 int T, int C, int W, const int32_t* tok_tab, unsigned flags, void* stream) {
-  if (!x || !w || !y || !tok_tab || T <= 0 || C <= 0) return DAISY_EINVAL;
-  if (W < 1 || W > SC_MAX_W || C % 8 != 0 || (T + SC_ROWS - 1) / SC_ROWS > 65535) return DAISY_EUNSUPPORTED;
-  if (flags & ~DAISY_KDA_CONV_SILU) return DAISY_EINVAL;
-  if (!daisy_aligned16(x) || !daisy_aligned16(y) || !daisy_aligned16(w) || (bias && !daisy_aligned16(bias)) ||
-      x_st % 8 || y_st % 8 || (reinterpret_cast<uintptr_t>(tok_tab) & 7))
-    return DAISY_EALIGN;
-  if (state_in && state_in == state_out) return DAISY_EINVAL;     // sequences end in different CTAs
-  ShortConvParams p;
-  p.x = (const __nv_bfloat16*)x; p.w = (const __nv_bfloat16*)w; p.bias = (const __nv_bfloat16*)bias;
-  p.s_in = (const __nv_bfloat16*)state_in; p.s_out = (__nv_bfloat16*)state_out; p.y = (__nv_bfloat16*)y;
-  p.x_sb = 0; p.x_st = x_st; p.y_sb = 0; p.y_st = y_st;
-  p.T = T; p.C = C; p.W = W; p.silu = (flags & DAISY_KDA_CONV_SILU) ? 1 : 0;
-  p.tok = reinterpret_cast<const int2*>(tok_tab);
-  const dim3 grid((C + SC_COLS - 1) / SC_COLS, (T + SC_ROWS - 1) / SC_ROWS, 1);
-  if (p.silu) kda_short_conv_kernel<true, true><<<grid, SC_THREADS, 0, (cudaStream_t)stream>>>(p);
-  else        kda_short_conv_kernel<false, true><<<grid, SC_THREADS, 0, (cudaStream_t)stream>>>(p);
+  if (!tok_tab) return DAISY_EINVAL;
+  return short_conv_launch(1, &x, 0, x_st, &w, &bias, &state_in, &state_out, &y, 0, y_st, 1, T, C, W, tok_tab, flags, stream);
+}
+
+extern "C" int daisy_b200_kda_short_conv_group(int n, const void* const* x, int64_t x_sb, int64_t x_st, const void* const* w, const void* const* bias,
+                                               const void* const* state_in, void* const* state_out, void* const* y, int64_t y_sb, int64_t y_st,
+                                               int B, int T, int C, int W, const int32_t* tok_tab, unsigned flags, void* stream) {
+  if (!x || !w || !y || (tok_tab && B != 1)) return DAISY_EINVAL;
+  return short_conv_launch(n, x, x_sb, x_st, w, bias, state_in, state_out, y, y_sb, y_st, B, T, C, W, tok_tab, flags, stream);
+}
+
+// beta = sigmoid(x), rounded to bf16 as the reference's bf16 sigmoid leaves it, kept as fp32: one launch for two passes
+extern "C" int daisy_b200_kda_beta(const void* x, float* out, int64_t n, void* stream) {
+  if (!x || !out || n <= 0) return DAISY_EINVAL;
+  if ((n + 255) / 256 > 0x7fffffffLL) return DAISY_EUNSUPPORTED;
+  kda_beta_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)x, out, n);
   DAISY_CHECK_LAUNCH();
   return DAISY_OK;
 }

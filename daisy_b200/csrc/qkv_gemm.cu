@@ -6,7 +6,8 @@
 //              tokens, so the weightless RMS norm over D and the half-rotation RoPE are per-thread work on the
 //              accumulator row (thread = token = TMEM lane); q', k', v' leave as [B,T,H,D] bf16 and the separate
 //              norm/RoPE pass over q, k, v (1.6 GB at B=8, T=8192, 16 heads) disappears.
-//   EPI_PLAIN  bf16 store of C (the output projection).
+//   EPI_PLAIN  bf16 store of C (the output projection); up to three products of one shape in one launch (the Kimi layer's
+//              q, k and v projections: 3 x 192 tiles in 8 waves instead of 3 x 3).
 //
 // Persistent CTAs walk 128 x BN output tiles (n fastest, so concurrently running CTAs share X tiles and the
 // whole W in L2).  Roles (352 threads): warps 0-7 epilogue, warp 8 MMA issuer, warps 9, 10 TMA producers.  Both
@@ -40,11 +41,15 @@ template <int BN, bool PAIR, bool QKV> struct GemmCfg {
   static constexpr int TILE_M = PAIR ? 2 * GM : GM;
 };
 
+constexpr int GROUP = 3;
+struct GemmMaps { CUtensorMap x[GROUP], w[GROUP]; };
+
 struct GemmParams {
   int M, N, K;
   int epi;                       // 0 plain, 1 qkv
-  // plain
-  __nv_bfloat16* c; int64_t ldc;
+  // plain: up to GROUP products of one shape, columns [i per, (i + 1) per) of N are product i's
+  __nv_bfloat16* c[GROUP]; int64_t ldc;
+  int per;
   // qkv
   __nv_bfloat16* out[3];         // q', k', v'  [M, H, 128]
   const float *cos, *sin;        // [T, 64]
@@ -85,7 +90,7 @@ struct GemmBars {
 
 template <int BN, bool PAIR, bool QKV>
 __global__ void __launch_bounds__(G_THREADS, 1)
-qkv_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w, const GemmParams p) {
+qkv_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p) {
   using Cfg = GemmCfg<BN, PAIR, QKV>;
   extern __shared__ uint8_t gemm_smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(gemm_smem_raw) + 1023) & ~uintptr_t(1023));
@@ -121,11 +126,13 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
     // ------------------------------------------------------------------ TMA producers: every other k-block each (a turn of the
     // loop takes one thread some 450 cycles, the products of a k-block 256, PAIR 512)
     if (lane == 0) {
-      prefetch_tmap(&tm_x); prefetch_tmap(&tm_w);
+      prefetch_tmap(&maps.x[0]); prefetch_tmap(&maps.w[0]);
       uint32_t n = warp - 9, first = 0;                  // my next k-block, and the tile's first, counted over all tiles
       bool ok = true;
       for (int tile = worker; tile < tiles && ok; tile += workers, first += kb_n) {
-        const int m0 = (tile / n_tiles) * Cfg::TILE_M + (int)rank * GM, n0 = (tile % n_tiles) * BN + (int)rank * Cfg::B_ROWS;
+        const int m0 = (tile / n_tiles) * Cfg::TILE_M + (int)rank * GM, n0 = (tile % n_tiles) * BN;
+        const int prod = QKV ? 0 : n0 / p.per, w0 = n0 - prod * p.per + (int)rank * Cfg::B_ROWS;
+        const CUtensorMap *tm_x = &maps.x[prod], *tm_w = &maps.w[prod];
         for (; n < first + kb_n; n += 2) {
           const int kb = n - first;
           const int st = n % Cfg::NST;
@@ -135,12 +142,12 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
             // both CTAs' bytes are counted on rank 0's barrier, which the MMA issuer waits on
             const uint32_t full0 = mapa_shared(smem_u32(&bars->full[st]), 0);
             if (rank == 0) mbar_expect_tx(&bars->full[st], 2 * Cfg::STAGE);
-            tma_load_3d_pair(dst, &tm_x, full0, kb * GK, m0, 0);
-            tma_load_3d_pair(dst + G_A_BYTES, &tm_w, full0, kb * GK, n0, 0);
+            tma_load_3d_pair(dst, tm_x, full0, kb * GK, m0, 0);
+            tma_load_3d_pair(dst + G_A_BYTES, tm_w, full0, kb * GK, w0, 0);
           } else {
             mbar_expect_tx(&bars->full[st], Cfg::STAGE);
-            tma_load_3d(dst, &tm_x, &bars->full[st], kb * GK, m0, 0);
-            tma_load_3d(dst + G_A_BYTES, &tm_w, &bars->full[st], kb * GK, n0, 0);
+            tma_load_3d(dst, tm_x, &bars->full[st], kb * GK, m0, 0);
+            tma_load_3d(dst + G_A_BYTES, tm_w, &bars->full[st], kb * GK, w0, 0);
           }
         }
       }
@@ -279,7 +286,8 @@ qkv_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
               ring_row = reinterpret_cast<uint8_t*>(p.ring[which - 1]) + ((int64_t)b * p.r_sb + (int64_t)h * p.r_sh + (int64_t)(t % p.cap) * p.r_sr) * 2;
           }
         } else {
-          dst_row = p.c + (size_t)m * p.ldc + n0;
+          const int prod = n0 / p.per;
+          dst_row = p.c[prod] + (size_t)m * p.ldc + (n0 - prod * p.per);
         }
         // bf16 pack, then through the warp's staging rows so that each store instruction writes two whole rows
         uint4 ch[16];
@@ -355,6 +363,7 @@ struct SmallCfg {
   static constexpr int RANKS = 128 / BN;                                                 // QKV: CTAs to a head
   static constexpr int SMEM0 = 1024 + 1024 + 256;
 };
+struct GemmWeights { const __nv_bfloat16* p[GROUP]; };
 struct SmallBars {
   uint64_t full[12], empty[12], acc_full;
   uint32_t tmem_base;
@@ -363,8 +372,8 @@ struct SmallBars {
 
 template <int BN, bool QKV>
 __global__ void __launch_bounds__(G_SMALL_THREADS, 2)
-small_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w, const GemmParams p, const int nst,
-                  const int tm, const __nv_bfloat16* w, const int64_t ldw, const int prefetch) {
+small_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p, const int nst,
+                  const int tm, const GemmWeights w, const int64_t ldw, const int prefetch) {
   using Cfg = SmallCfg<BN>;
   static_assert(!QKV || BN == 64, "two CTAs to a head");
   constexpr int HB = BN / 2;
@@ -380,7 +389,8 @@ small_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
   const int nh = bn / Cfg::RANKS;                                                        // QKV: head slot among 3 H
   const int c0 = rank * HB;                                                              // and this CTA's channels of it
   const int m0 = bm * tm;                                                                // tm <= 128 rows of X a tile, a multiple of 8
-  const int w_lo = QKV ? nh * 128 + c0 : bn * BN, w_hi = QKV ? w_lo + 64 : w_lo + HB;    // its weight rows: HB and HB
+  const int prod = QKV ? 0 : bn * BN / p.per;                                            // plain: which product
+  const int w_lo = QKV ? nh * 128 + c0 : bn * BN - prod * p.per, w_hi = QKV ? w_lo + 64 : w_lo + HB;    // its weight rows: HB and HB
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < nst; ++i) { mbar_init(&bars->full[i], 1); mbar_init(&bars->empty[i], 1); }
@@ -392,9 +402,9 @@ small_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
     tmem_alloc(&bars->tmem_base, BN);
     tmem_relinquish();
   } else if (prefetch && bm == 0 && threadIdx.x < BN) {
-    l2_prefetch_bulk(w + (int64_t)(threadIdx.x < HB ? w_lo + threadIdx.x : w_hi + (int)threadIdx.x - HB) * ldw, (uint32_t)p.K * 2u);
+    l2_prefetch_bulk(w.p[prod] + (int64_t)(threadIdx.x < HB ? w_lo + threadIdx.x : w_hi + (int)threadIdx.x - HB) * ldw, (uint32_t)p.K * 2u);
   }
-  if (warp == 4 && lane == 0) { prefetch_tmap(&tm_x); prefetch_tmap(&tm_w); }
+  if (warp == 4 && lane == 0) { prefetch_tmap(&maps.x[prod]); prefetch_tmap(&maps.w[prod]); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -415,9 +425,9 @@ small_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
         if (!mbar_wait(&bars->empty[st], ((kb / nst) & 1) ^ 1, abort_flag, p.status, 1)) break;
         uint8_t* dst = stages + st * Cfg::STAGE;
         mbar_expect_tx(&bars->full[st], tm * GK * 2 + BN * GK * 2);
-        tma_load_3d(dst + G_A_BYTES, &tm_w, &bars->full[st], kb * GK, w_lo, 0);
-        tma_load_3d(dst + G_A_BYTES + HB * GK * 2, &tm_w, &bars->full[st], kb * GK, w_hi, 0);
-        tma_load_3d(dst, &tm_x, &bars->full[st], kb * GK, m0, 0);
+        tma_load_3d(dst + G_A_BYTES, &maps.w[prod], &bars->full[st], kb * GK, w_lo, 0);
+        tma_load_3d(dst + G_A_BYTES + HB * GK * 2, &maps.w[prod], &bars->full[st], kb * GK, w_hi, 0);
+        tma_load_3d(dst, &maps.x[prod], &bars->full[st], kb * GK, m0, 0);
       }
     }
     __syncwarp();
@@ -526,7 +536,7 @@ small_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
       }
 #pragma unroll
       for (int i = 0; i < HB; ++i) hv[i] = pack_bf16(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
-      store(QKV ? p.out[which] + ((size_t)m * p.H + h) * 128 + c0 : p.c + (size_t)m * p.ldc + w_lo);
+      store(QKV ? p.out[which] + ((size_t)m * p.H + h) * 128 + c0 : p.c[prod] + (size_t)m * p.ldc + w_lo);
       if (QKV && which >= 1 && p.ring[which - 1]) {                                      // this row's slot in the ring cache, if it is kept
         const int b = m / p.T, t = m - b * p.T;
         if (t >= p.ring_first) {
@@ -558,7 +568,7 @@ small_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
 using namespace daisy;
 
 template <int BN, bool PAIR, bool QKV>
-static int launch_gemm(const CUtensorMap& tx, const CUtensorMap& tw, const GemmParams& p, cudaStream_t st) {
+static int launch_gemm(const GemmMaps& maps, const GemmParams& p, cudaStream_t st) {
   using Cfg = GemmCfg<BN, PAIR, QKV>;
   static_assert(Cfg::SMEM <= 232448, "over the 227 KB a CTA may use");
   static bool attr[daisy_host::MAX_DEVICES] = {};
@@ -596,7 +606,7 @@ static int launch_gemm(const CUtensorMap& tx, const CUtensorMap& tw, const GemmP
   } else {
     cfg.gridDim = dim3((unsigned)(tiles < sms ? tiles : sms));
   }
-  if (cudaLaunchKernelEx(&cfg, qkv_gemm_kernel<BN, PAIR, QKV>, tx, tw, p) != cudaSuccess) {
+  if (cudaLaunchKernelEx(&cfg, qkv_gemm_kernel<BN, PAIR, QKV>, maps, p) != cudaSuccess) {
     (void)cudaGetLastError();
     return DAISY_ECUDA;
   }
@@ -604,10 +614,21 @@ static int launch_gemm(const CUtensorMap& tx, const CUtensorMap& tw, const GemmP
   return DAISY_OK;
 }
 
+static int make_maps(GemmMaps& maps, const void* const* x, int64_t ldx, int x_rows, const void* const* w, int64_t ldw, int w_rows, int n, const GemmParams& p) {
+  for (int i = 0; i < n; ++i) {
+    int rc = daisy_host::make_tmap_bf16_3d(&maps.x[i], x[i], p.K, p.M, 1, (uint64_t)ldx * 2, (uint64_t)ldx * 2 * p.M, GK, x_rows);
+    if (rc != DAISY_OK) return rc;
+    rc = daisy_host::make_tmap_bf16_3d(&maps.w[i], w[i], p.K, p.per, 1, (uint64_t)ldw * 2, (uint64_t)ldw * 2 * p.per, GK, w_rows);
+    if (rc != DAISY_OK) return rc;
+  }
+  for (int i = n; i < GROUP; ++i) { maps.x[i] = maps.x[0]; maps.w[i] = maps.w[0]; }
+  return DAISY_OK;
+}
+
 constexpr size_t G_PREFETCH_LIMIT = 48u << 20;          // weights up to this size are hinted into L2 ahead of the wait
 
 template <int BN, bool QKV>
-static int launch_small(const void* x, int64_t ldx, const void* w, int64_t ldw, const GemmParams& p, cudaStream_t st) {
+static int launch_small(const void* const* x, int64_t ldx, const void* const* w, int64_t ldw, int n, const GemmParams& p, cudaStream_t st) {
   using Cfg = SmallCfg<BN>;
   auto kernel = small_gemm_kernel<BN, QKV>;
   static bool attr[daisy_host::MAX_DEVICES] = {};
@@ -624,10 +645,11 @@ static int launch_small(const void* x, int64_t ldx, const void* w, int64_t ldw, 
   }
   // tiles of equal height: 131 rows are two tiles of 72, not one of 128 and one of 3
   const int mt = (p.M - 1) / GM + 1, tm = ((p.M - 1) / mt + 8) & ~7;
-  CUtensorMap tx, tw;
-  int rc;
-  if ((rc = daisy_host::make_tmap_bf16_3d(&tx, x, p.K, p.M, 1, (uint64_t)ldx * 2, (uint64_t)ldx * 2 * p.M, GK, tm)) != DAISY_OK) return rc;
-  if ((rc = daisy_host::make_tmap_bf16_3d(&tw, w, p.K, p.N, 1, (uint64_t)ldw * 2, (uint64_t)ldw * 2 * p.N, GK, BN / 2)) != DAISY_OK) return rc;
+  GemmMaps maps;
+  GemmWeights wp{};
+  const int rc = make_maps(maps, x, ldx, tm, w, ldw, BN / 2, n, p);
+  if (rc != DAISY_OK) return rc;
+  for (int i = 0; i < n; ++i) wp.p[i] = (const __nv_bfloat16*)w[i];
   const int tiles = mt * (p.N / BN);
   int nst = tiles <= sms ? Cfg::MAX_NST : Cfg::HALF_NST;
   if (nst > p.K / GK) nst = p.K / GK;
@@ -639,7 +661,7 @@ static int launch_small(const void* x, int64_t ldx, const void* w, int64_t ldw, 
   at[1].id = cudaLaunchAttributeClusterDimension;
   at[1].val.clusterDim.x = Cfg::RANKS; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
   cfg.attrs = at; cfg.numAttrs = QKV ? 2 : 1;
-  if (cudaLaunchKernelEx(&cfg, kernel, tx, tw, p, nst, tm, (const __nv_bfloat16*)w, ldw, (size_t)p.N * p.K * 2 <= G_PREFETCH_LIMIT ? 1 : 0) != cudaSuccess) {
+  if (cudaLaunchKernelEx(&cfg, kernel, maps, p, nst, tm, wp, ldw, (size_t)p.N * p.K * 2 <= G_PREFETCH_LIMIT ? 1 : 0) != cudaSuccess) {
     (void)cudaGetLastError();
     return DAISY_ECUDA;
   }
@@ -656,37 +678,49 @@ static int gemm_tile(const GemmParams& p, int sms) {
   const int64_t mt = ((int64_t)p.M + GM - 1) / GM;
   if (p.epi == 0 && mt * (p.N / 32) <= sms) return TILE_32;
   if (mt * (p.N / 64) <= sms) return TILE_64;
-  if (p.N % 256 != 0) return TILE_128;
+  if (p.per % 256 != 0) return TILE_128;
   const int64_t w1 = (mt * (p.N / 128) + sms - 1) / sms, w2 = ((mt + 1) / 2 * (p.N / 256) + sms / 2 - 1) / (sms / 2);
   return 4000 + w1 * (37ll * p.K / 10 + 1000) < 7000 + w2 * (53ll * p.K / 10 + 2000) ? TILE_128 : TILE_PAIR;
 }
 
-static int gemm_common(const void* x, int64_t ldx, const void* w, int64_t ldw, GemmParams& p, void* stream) {
-  if (!x || !w || p.M <= 0 || p.N <= 0 || p.K <= 0) return DAISY_EINVAL;
-  if (p.K % GK != 0 || p.N % 128 != 0) return DAISY_EUNSUPPORTED;
-  if (!daisy_aligned16(x) || !daisy_aligned16(w) || (ldx & 7) || (ldw & 7) || ldx < p.K || ldw < p.K) return DAISY_EALIGN;
+// n products of one shape; p.N counts all their columns, p.per one's
+static int gemm_common(const void* const* x, int64_t ldx, const void* const* w, int64_t ldw, int n, GemmParams& p, void* stream) {
+  if (p.M <= 0 || p.per <= 0 || p.K <= 0) return DAISY_EINVAL;
+  for (int i = 0; i < n; ++i) if (!x[i] || !w[i]) return DAISY_EINVAL;
+  if (p.K % GK != 0 || p.per % 128 != 0) return DAISY_EUNSUPPORTED;
+  for (int i = 0; i < n; ++i) if (!daisy_aligned16(x[i]) || !daisy_aligned16(w[i])) return DAISY_EALIGN;
+  if ((ldx & 7) || (ldw & 7) || ldx < p.K || ldw < p.K) return DAISY_EALIGN;
+  p.N = n * p.per;
   const int sms = daisy_host::sm_count_cached();
   if (sms <= 0) return DAISY_ENODEV;
   cudaStream_t st = (cudaStream_t)stream;
   const int tile = gemm_tile(p, sms);
-  if (tile == TILE_32) return launch_small<32, false>(x, ldx, w, ldw, p, st);
-  if (tile == TILE_64) return p.epi ? launch_small<64, true>(x, ldx, w, ldw, p, st) : launch_small<64, false>(x, ldx, w, ldw, p, st);
-  CUtensorMap tx, tw;
-  int rc;
-  if ((rc = daisy_host::make_tmap_bf16_3d(&tx, x, p.K, p.M, 1, (uint64_t)ldx * 2, (uint64_t)ldx * 2 * p.M, GK, GM)) != DAISY_OK) return rc;
-  if ((rc = daisy_host::make_tmap_bf16_3d(&tw, w, p.K, p.N, 1, (uint64_t)ldw * 2, (uint64_t)ldw * 2 * p.N, GK, 128)) != DAISY_OK) return rc;
-  if (tile == TILE_PAIR) return p.epi ? launch_gemm<256, true, true>(tx, tw, p, st) : launch_gemm<256, true, false>(tx, tw, p, st);
-  return p.epi ? launch_gemm<128, false, true>(tx, tw, p, st) : launch_gemm<128, false, false>(tx, tw, p, st);
+  if (tile == TILE_32) return launch_small<32, false>(x, ldx, w, ldw, n, p, st);
+  if (tile == TILE_64) return p.epi ? launch_small<64, true>(x, ldx, w, ldw, n, p, st) : launch_small<64, false>(x, ldx, w, ldw, n, p, st);
+  GemmMaps maps;
+  const int rc = make_maps(maps, x, ldx, GM, w, ldw, 128, n, p);
+  if (rc != DAISY_OK) return rc;
+  if (tile == TILE_PAIR) return p.epi ? launch_gemm<256, true, true>(maps, p, st) : launch_gemm<256, true, false>(maps, p, st);
+  return p.epi ? launch_gemm<128, false, true>(maps, p, st) : launch_gemm<128, false, false>(maps, p, st);
+}
+
+extern "C" int daisy_b200_gemm_nt_group(const void* const* x, int64_t ldx, const void* const* w, int64_t ldw, void* const* c, int64_t ldc,
+                                        int n, int M, int N, int K, int* status_word, void* stream) {
+  if (!x || !w || !c || n < 1 || n > GROUP) return DAISY_EINVAL;
+  GemmParams p{};
+  p.M = M; p.per = N; p.K = K; p.epi = 0; p.ldc = ldc; p.status = status_word;
+  for (int i = 0; i < n; ++i) {
+    if (!c[i]) return DAISY_EINVAL;
+    if (!daisy_aligned16(c[i])) return DAISY_EALIGN;
+    p.c[i] = (__nv_bfloat16*)c[i];
+  }
+  if ((ldc & 7) || ldc < N) return DAISY_EALIGN;
+  return gemm_common(x, ldx, w, ldw, n, p, stream);
 }
 
 extern "C" int daisy_b200_gemm_nt(const void* x, int64_t ldx, const void* w, int64_t ldw, void* c, int64_t ldc,
                                   int M, int N, int K, int* status_word, void* stream) {
-  if (!c) return DAISY_EINVAL;
-  if (!daisy_aligned16(c) || (ldc & 7) || ldc < N) return DAISY_EALIGN;
-  GemmParams p{};
-  p.M = M; p.N = N; p.K = K; p.epi = 0;
-  p.c = (__nv_bfloat16*)c; p.ldc = ldc; p.status = status_word;
-  return gemm_common(x, ldx, w, ldw, p, stream);
+  return daisy_b200_gemm_nt_group(&x, ldx, &w, ldw, &c, ldc, 1, M, N, K, status_word, stream);
 }
 
 static int qkv_gemm_launch(const void* x, int64_t ldx, const void* w_qkv, int64_t ldw, const float* cos, const float* sin,
@@ -709,13 +743,13 @@ static int qkv_gemm_launch(const void* x, int64_t ldx, const void* w_qkv, int64_
   if (ve && (!ve_gate_logit || !daisy_aligned16(ve) || (ve_ld & 7) || ve_ld < (int64_t)H * D)) return ve_gate_logit ? DAISY_EALIGN : DAISY_EINVAL;
   GemmParams p{};
   p.ve = (const __nv_bfloat16*)ve; p.ve_ld = ve_ld; p.ve_gate_logit = ve_gate_logit;
-  p.M = B * T; p.N = 3 * H * D; p.K = dim; p.epi = 1;
+  p.M = B * T; p.per = 3 * H * D; p.K = dim; p.epi = 1;
   p.out[0] = (__nv_bfloat16*)q_out; p.out[1] = (__nv_bfloat16*)k_out; p.out[2] = (__nv_bfloat16*)v_out;
   p.cos = cos; p.sin = sin; p.T = T; p.H = H; p.eps = eps; p.flags = flags & DAISY_QKV_DEFAULT; p.status = status_word;
   p.ring[0] = ring_k; p.ring[1] = ring_v; p.r_sb = r_sb; p.r_sh = r_sh; p.r_sr = r_sr;
   p.rstd = rstd; p.vn = (__nv_bfloat16*)vn;
   p.cap = cap; p.ring_first = ring_first; p.ring_f16 = (flags & DAISY_CACHE_FP16) ? 1 : 0;
-  return gemm_common(x, ldx, w_qkv, ldw, p, stream);
+  return gemm_common(&x, ldx, &w_qkv, ldw, 1, p, stream);
 }
 
 extern "C" int daisy_b200_qkv_gemm(const void* x, int64_t ldx, const void* w_qkv, int64_t ldw,

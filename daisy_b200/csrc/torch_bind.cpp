@@ -435,7 +435,7 @@ Packed pack_tables(const py::object& cu_seqlens, c10::Device dev, int64_t chunk,
   for (int64_t n = 0; n < p.n_seq; ++n) p.n_chunks += (cu[n + 1] - cu[n] + chunk - 1) / chunk;
   // one staging buffer, one copy: [n_chunks][2], [n_seq + 1] (padded to 8 bytes), [total][2]
   const int64_t at_ptr = 2 * p.n_chunks, at_tok = at_ptr + (p.n_seq + 2) / 2 * 2, size = at_tok + (want_tok ? 2 * p.total : 0);
-  Tensor host = at::empty({std::max<int64_t>(size, 1)}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
+  Tensor host = at::empty({std::max<int64_t>(size, 1)}, at::TensorOptions().dtype(at::kInt).pinned_memory(dev.is_cuda()));
   int32_t* h = host.data_ptr<int32_t>();
   int64_t c = 0;
   for (int64_t n = 0; n < p.n_seq; ++n) {
@@ -543,6 +543,29 @@ Tensor kimi_linear(const Tensor& x, const Tensor& w) {
   return at::linear(x, w);
 }
 
+// y[i] = x[i] w[i]^T; products of one shape go out in one launch
+void kimi_linears(std::vector<Tensor> x, std::vector<Tensor> w, Tensor* y) {
+  const size_t n = x.size();
+  const int64_t N = w[0].size(0), K = w[0].size(1);
+  bool group = x[0].numel() / K >= 64 && N % 128 == 0 && K % 64 == 0;
+  for (size_t i = 0; i < n; ++i)
+    group = group && x[i].scalar_type() == at::kBFloat16 && w[i].scalar_type() == at::kBFloat16 && x[i].sizes() == x[0].sizes() && w[i].sizes() == w[0].sizes() &&
+            x[i].is_contiguous() && w[i].is_contiguous();
+  if (!group) {
+    for (size_t i = 0; i < n; ++i) y[i] = kimi_linear(x[i], w[i]);
+    return;
+  }
+  const void *xp[3], *wp[3];
+  void* cp[3];
+  auto shape = x[0].sizes().vec();
+  shape.back() = N;
+  for (size_t i = 0; i < n; ++i) {
+    y[i] = at::empty(shape, x[0].options());
+    xp[i] = x[i].data_ptr(); wp[i] = w[i].data_ptr(); cp[i] = y[i].data_ptr();
+  }
+  check(daisy_b200_gemm_nt_group(xp, K, wp, K, cp, N, (int)n, (int)(x[0].numel() / K), (int)N, (int)K, status_ptr(x[0]), stream_of(x[0])), "daisy_b200_gemm_nt_group");
+}
+
 // weights: q, k, v, f0, f1, g0, g1, b, o.  conv_s, rec: carried states or nothing.  -> y, final state, convolution states
 std::tuple<Tensor, OptTensor, std::vector<Tensor>> kimi_layer(const Tensor& x, const std::vector<Tensor>& w, const OptTensor& g1_bias, const OptTensor& norm_w,
                                                               const std::vector<Tensor>& conv_w, const std::vector<OptTensor>& conv_b, const Tensor& a_log,
@@ -555,42 +578,52 @@ std::tuple<Tensor, OptTensor, std::vector<Tensor>> kimi_layer(const Tensor& x, c
   const bool packed = !cu_seqlens.is_none();
   if (packed) p = pack_tables(cu_seqlens, x.device(), 64, true);
   const int64_t n = packed ? p.n_seq : B;
-  Tensor qkv[3];
+  Tensor qkv[3], pr[3];
   std::vector<Tensor> out_s;
+  kimi_linears({x, x, x}, {w[0], w[1], w[2]}, pr);
+  const void *xp[3], *wp[3], *bp[3], *sp[3];
+  void *op[3], *yp[3];
+  int64_t W[3];
   for (int i = 0; i < 3; ++i) {
-    Tensor xi = kimi_linear(x, w[i]), y = at::empty_like(xi);
+    qkv[i] = at::empty_like(pr[i]);
     const bool have = conv_s[i].has_value(), in_place = have && !packed && T <= 32;
-    const int64_t W = conv_w[i].numel() / C;
+    W[i] = conv_w[i].numel() / C;
     if (have)
-      TORCH_CHECK_VALUE(conv_s[i]->scalar_type() == at::kBFloat16 && conv_s[i]->is_contiguous() && conv_s[i]->numel() == n * C * W,
-                        "state must be a contiguous bf16 [", n, ", ", C, ", ", W, "] tensor");
+      TORCH_CHECK_VALUE(conv_s[i]->scalar_type() == at::kBFloat16 && conv_s[i]->is_contiguous() && conv_s[i]->numel() == n * C * W[i],
+                        "state must be a contiguous bf16 [", n, ", ", C, ", ", W[i], "] tensor");
     Tensor so;
     if (in_place) so = *conv_s[i];
-    else if (use_cache && packed) so = have ? conv_s[i]->clone() : at::zeros({n, C, W}, x.options());     // sequences without tokens keep their state
-    else if (use_cache) so = at::empty({n, C, W}, x.options());
-    const void *wp = conv_w[i].data_ptr(), *bp = conv_b[i].has_value() ? conv_b[i]->data_ptr() : nullptr, *sp = have ? conv_s[i]->data_ptr() : nullptr;
-    void* op = so.defined() ? so.data_ptr() : nullptr;
-    if (packed)
-      check(daisy_b200_kda_short_conv_varlen(xi.data_ptr(), C, wp, bp, sp, op, y.data_ptr(), C, (int)T, (int)C, (int)W, p.tok.data_ptr<int32_t>(),
-                                             silu ? DAISY_KDA_CONV_SILU : 0, stream_of(x)),
-            "daisy_b200_kda_short_conv_varlen");
-    else
-      check(daisy_b200_kda_short_conv(xi.data_ptr(), T * C, C, wp, bp, sp, op, y.data_ptr(), T * C, C, (int)B, (int)T, (int)C, (int)W, silu ? DAISY_KDA_CONV_SILU : 0,
-                                      stream_of(x)),
-            "daisy_b200_kda_short_conv");
-    qkv[i] = y.view({B, T, H, 128});
+    else if (use_cache && packed) so = have ? conv_s[i]->clone() : at::zeros({n, C, W[i]}, x.options());     // sequences without tokens keep their state
+    else if (use_cache) so = at::empty({n, C, W[i]}, x.options());
+    xp[i] = pr[i].data_ptr(); wp[i] = conv_w[i].data_ptr(); bp[i] = conv_b[i].has_value() ? conv_b[i]->data_ptr() : nullptr;
+    sp[i] = have ? conv_s[i]->data_ptr() : nullptr; op[i] = so.defined() ? so.data_ptr() : nullptr; yp[i] = qkv[i].data_ptr();
+    qkv[i] = qkv[i].view({B, T, H, 128});
     if (so.defined()) out_s.push_back(so);
   }
-  Tensor f = kimi_linear(kimi_linear(x, w[3]), w[4]);
+  const int step = W[0] == W[1] && W[1] == W[2] && B * 3 <= 65535 ? 3 : 1;                 // one launch for the three
+  for (int i = 0; i < 3; i += step)
+    check(daisy_b200_kda_short_conv_group(step, xp + i, T * C, C, wp + i, bp + i, sp + i, op + i, yp + i, T * C, C, (int)B, (int)T, (int)C, (int)W[i],
+                                          packed ? p.tok.data_ptr<int32_t>() : nullptr, silu ? DAISY_KDA_CONV_SILU : 0, stream_of(x)),
+          "daisy_b200_kda_short_conv_group");
+  Tensor low[2], up[2];                                                                    // the two low-rank projections: decay gate, output gate
+  kimi_linears({x, x}, {w[3], w[5]}, low);
+  kimi_linears({low[0], low[1]}, {w[4], w[6]}, up);
+  const Tensor &f = up[0], &gp = up[1];
   Tensor g = at::empty({B, T, H, 128}, x.options().dtype(at::kFloat));
   check(daisy_b200_kda_gate(f.data_ptr(), 1, a_log.data_ptr<float>(), dt_bias.data_ptr<float>(), g.data_ptr<float>(), M, (int)H, 128, 1.f, 20.f,
                             DAISY_KDA_GATE_ROUND_BF16, stream_of(x)),
         "daisy_b200_kda_gate");
-  Tensor beta = at::linear(x, w[7]).sigmoid_().to(at::kFloat);
+  Tensor bx = at::linear(x, w[7]), beta;
+  if (bx.scalar_type() == at::kBFloat16) {
+    beta = at::empty(bx.sizes(), bx.options().dtype(at::kFloat));
+    check(daisy_b200_kda_beta(bx.data_ptr(), beta.data_ptr<float>(), beta.numel(), stream_of(x)), "daisy_b200_kda_beta");
+  } else {
+    beta = bx.sigmoid_().to(at::kFloat);
+  }
   std::pair<Tensor, OptTensor> r = packed ? kda_chunk(qkv[0], qkv[1], qkv[2], g, beta, std::nullopt, rec, use_cache, true, false, &p)
                                    : T <= RECURRENT_MAX_T ? kda_recurrent(qkv[0], qkv[1], qkv[2], g, beta, std::nullopt, rec, use_cache, true, false, rec.has_value())
                                                           : kda_chunk(qkv[0], qkv[1], qkv[2], g, beta, std::nullopt, rec, use_cache, true, false, nullptr);
-  Tensor gp = kimi_linear(kimi_linear(x, w[5]), w[6]), o = r.first, yn = at::empty({B, T, C}, x.options());
+  Tensor o = r.first, yn = at::empty({B, T, C}, x.options());
   check(daisy_b200_kda_out_norm(o.data_ptr(), 0, gp.data_ptr(), g1_bias.has_value() ? g1_bias->data_ptr() : nullptr, g1_bias.has_value() ? (int)H : 1,
                                 norm_w.has_value() ? norm_w->data_ptr() : nullptr, yn.data_ptr(), M * H, 128, (float)eps, 2, stream_of(x)),
         "daisy_b200_kda_out_norm");

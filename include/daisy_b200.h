@@ -144,6 +144,9 @@ int daisy_b200_qkv_gemm_train(const void* x, int64_t ldx, const void* w_qkv, int
  * (models/daisy/attention.py:149).  K a multiple of 64, N a multiple of 128; ld* are row strides in elements. */
 int daisy_b200_gemm_nt(const void* x, int64_t ldx, const void* w, int64_t ldw, void* c, int64_t ldc,
                        int M, int N, int K, int* status_word, void* stream);
+/* The same for n <= 3 products of one shape in one launch: c[i] = x[i] w[i]^T. */
+int daisy_b200_gemm_nt_group(const void* const* x, int64_t ldx, const void* const* w, int64_t ldw, void* const* c, int64_t ldc,
+                             int n, int M, int N, int K, int* status_word, void* stream);
 
 /* y[M,N] = x[M,K] W[N,K]^T for M <= 64 rows: the projections of a single decode token, F.linear(x, qkvo_w[:3]
  * flattened) and F.linear(y, qkvo_w[3]) with x [B,1,dim] (models/daisy/attention.py:119,201).  bf16 in and out, fp32
@@ -443,6 +446,13 @@ int daisy_b200_kda_short_conv(const void* x, int64_t x_sb, int64_t x_st, const v
 int daisy_b200_kda_short_conv_varlen(const void* x, int64_t x_st, const void* w, const void* bias,
                                      const void* state_in, void* state_out, void* y, int64_t y_st,
                                      int T, int C, int W, const int32_t* tok_tab, unsigned flags, void* stream);
+/* n <= 3 convolutions of one shape (a layer's q, k, v) in one launch: dense, or packed (B = 1) with tok_tab.  bias, state_in,
+ * state_out: arrays of pointers that may be null, or null. */
+int daisy_b200_kda_short_conv_group(int n, const void* const* x, int64_t x_sb, int64_t x_st, const void* const* w, const void* const* bias,
+                                    const void* const* state_in, void* const* state_out, void* const* y, int64_t y_sb, int64_t y_st,
+                                    int B, int T, int C, int W, const int32_t* tok_tab, unsigned flags, void* stream);
+/* beta = sigmoid(x) of a KDA layer (models/daisy/attention_kimi.py:124): x bf16, out the bf16-rounded value as fp32, n elements. */
+int daisy_b200_kda_beta(const void* x, float* out, int64_t n, void* stream);
 
 /* Gated RMS norm of the KDA output over the head dimension.  Replaces self.o_norm(o, gp) at
  * models/daisy/attention_kimi.py:137 (CompilableFusedRMSNormGated, :41-62; third-party fla rms_norm_gated):

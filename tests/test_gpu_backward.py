@@ -177,3 +177,28 @@ def test_value_embedding_layer_under_autograd():
     with torch.inference_mode():
         y_inf = m(x.detach(), ve.detach(), attn_mask=WindowMask(W))
     assert_close_bf16(y_inf, y.detach().float().cpu(), "inference vs training forward", max_tol=3e-2, mean_tol=3e-3)
+
+
+@pytest.mark.parametrize("B,T,H", [(1, 40, 1), (2, 33, 1), (1, 63, 3), (3, 129, 6)])
+def test_gated_layer_backward_ragged_rows(B, T, H):
+    """The row-wise gradient pass takes 64 (token, head) rows a block, two to a thread group: fewer rows than a block, remainders
+    of either kind, against ``torch.autograd`` over the fp32 oracle."""
+    from daisy_b200 import B200CausalSelfAttention, WindowMask
+    os.environ["DISABLE_O_ZERO_INIT"] = "1"
+    torch.manual_seed(T)
+    m = B200CausalSelfAttention(H * D, H, D, receives_ve=True, layer_idx=2).cuda()
+    m.norm_eps = swa.FP32_EPS
+    x = torch.randn(B, T, H * D, device="cuda").bfloat16().requires_grad_(True)
+    ve = torch.randn(B, T, H * D, device="cuda").bfloat16().requires_grad_(True)
+    cot = torch.randn(B, T, H * D, device="cuda")
+    (m(x, ve, attn_mask=WindowMask(50)).float() * cot).sum().backward()
+    xo, vo, wo = (t.detach().float().cpu().requires_grad_(True) for t in (x, ve, m.qkvo_w))
+    q, k, v = swa.project_qkv(xo, wo, H, D)
+    cos, sin = swa.rope_tables(D, T)
+    qn, kn, vn = swa.qkv_transform(q, k, v, cos, sin, swa.FP32_EPS)
+    gate = torch.sigmoid(m.g_ve.detach().float().cpu())
+    vn = gate * vn + (1 - gate) * vo.view_as(vn)
+    yo = swa.attend_windowed(qn, kn, vn, 50).reshape(B, T, H * D) @ wo[3].t()
+    (yo * cot.cpu()).sum().backward()
+    for got, ref, n in ((x.grad, xo.grad, "dx"), (ve.grad, vo.grad, "d ve"), (m.qkvo_w.grad, wo.grad, "dw")):
+        assert_close_bf16(got, ref, n, max_tol=4e-2, mean_tol=4e-3)

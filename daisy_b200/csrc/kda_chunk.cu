@@ -176,6 +176,7 @@ __global__ void __launch_bounds__(KI_THREADS, 3) kda_intra_kernel(const KdaIntra
   KdaIntraSmem& sm = *reinterpret_cast<KdaIntraSmem*>(kda_smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g8 = lane >> 2, t4 = lane & 3;
   const int chunk = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  grid_dep_wait();
   int t0, rows;
   ki_chunk_span(p.chunk_tab, chunk, p.T, t0, rows);
   uint8_t* rec = p.ws + ((size_t)(b * p.H + h) * p.NC + chunk) * REC_BYTES;
@@ -818,7 +819,10 @@ static int kda_launch(const void* q, const void* k, const void* v, const float* 
   ip.scale = scale > 0.f ? scale : 1.0f / sqrtf((float)K);
   ip.l2norm = (flags & DAISY_KDA_L2NORM_QK) ? 1 : 0;
   ip.chunk_tab = chunk_tab;
-  kda_intra_kernel<<<dim3(NC, H, B), KI_THREADS, intra_smem, st>>>(ip);
+  if (daisy_host::launch_dependent(kda_intra_kernel, dim3(NC, H, B), dim3(KI_THREADS), intra_smem, st, ip) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return DAISY_ECUDA;
+  }
   DAISY_CHECK_LAUNCH();
 
   KdaStateParams sp;

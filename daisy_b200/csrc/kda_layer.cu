@@ -70,6 +70,8 @@ __global__ void __launch_bounds__(SC_THREADS) kda_short_conv_kernel(const __grid
   const int cblk = blockIdx.x * SC_COLS;                           // channel blocks vary fastest, then time blocks:
   const int b = blockIdx.z / grp.n;                                // CTAs launched together walk the tensor front to back
   const int tblk = blockIdx.y * SC_ROWS;
+  grid_dep_launch();
+  grid_dep_wait();
   const int t_end = min(tblk + SC_ROWS, p.T);
 
   uint4 v[SC_LOADS];
@@ -235,6 +237,8 @@ __global__ void __launch_bounds__(256) kda_out_norm_kernel(const OutNormParams p
   const int sub = threadIdx.x & (ON_LPR - 1);
   const long long row_raw = ((long long)blockIdx.x * 256 + threadIdx.x) / ON_LPR;
   const bool live = row_raw < p.rows;
+  grid_dep_launch();
+  grid_dep_wait();
   const long long row = live ? row_raw : p.rows - 1;               // past the end the last row is repeated: the
   float x1[8], x2[8], g1[8], g2[8];                                // shuffles below need whole warps
   if (O32) {
@@ -288,13 +292,15 @@ __global__ void __launch_bounds__(256) kda_out_norm_kernel(const OutNormParams p
 
 __global__ void __launch_bounds__(256) kda_beta_kernel(const __nv_bfloat16* x, float* out, long long n) {
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  grid_dep_launch();
+  grid_dep_wait();
   if (i < n) out[i] = __bfloat162float(__float2bfloat16_rn(1.f / (1.f + expf(-__bfloat162float(x[i])))));
 }
 
 template <int MODE>
 static void launch_out_norm(const OutNormParams& p, unsigned grid, cudaStream_t st) {
-  if (p.o_fp32) kda_out_norm_kernel<MODE, true><<<grid, 256, 0, st>>>(p);
-  else          kda_out_norm_kernel<MODE, false><<<grid, 256, 0, st>>>(p);
+  if (p.o_fp32) (void)daisy_host::launch_dependent(kda_out_norm_kernel<MODE, true>, dim3(grid), dim3(256), 0, st, p);
+  else          (void)daisy_host::launch_dependent(kda_out_norm_kernel<MODE, false>, dim3(grid), dim3(256), 0, st, p);
 }
 
 }  // namespace daisy
@@ -330,11 +336,11 @@ static int short_conv_launch(int n, const void* const* x, int64_t x_sb, int64_t 
   cudaStream_t st = (cudaStream_t)stream;
   const bool silu = flags & DAISY_KDA_CONV_SILU;
   if (tok_tab) {
-    if (silu) kda_short_conv_kernel<true, true><<<grid, SC_THREADS, 0, st>>>(g);
-    else      kda_short_conv_kernel<false, true><<<grid, SC_THREADS, 0, st>>>(g);
+    if (silu) (void)daisy_host::launch_dependent(kda_short_conv_kernel<true, true>, grid, dim3(SC_THREADS), 0, st, g);
+    else      (void)daisy_host::launch_dependent(kda_short_conv_kernel<false, true>, grid, dim3(SC_THREADS), 0, st, g);
   } else {
-    if (silu) kda_short_conv_kernel<true, false><<<grid, SC_THREADS, 0, st>>>(g);
-    else      kda_short_conv_kernel<false, false><<<grid, SC_THREADS, 0, st>>>(g);
+    if (silu) (void)daisy_host::launch_dependent(kda_short_conv_kernel<true, false>, grid, dim3(SC_THREADS), 0, st, g);
+    else      (void)daisy_host::launch_dependent(kda_short_conv_kernel<false, false>, grid, dim3(SC_THREADS), 0, st, g);
   }
   DAISY_CHECK_LAUNCH();
   return DAISY_OK;
@@ -364,7 +370,7 @@ extern "C" int daisy_b200_kda_short_conv_group(int n, const void* const* x, int6
 extern "C" int daisy_b200_kda_beta(const void* x, float* out, int64_t n, void* stream) {
   if (!x || !out || n <= 0) return DAISY_EINVAL;
   if ((n + 255) / 256 > 0x7fffffffLL) return DAISY_EUNSUPPORTED;
-  kda_beta_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)x, out, n);
+  (void)daisy_host::launch_dependent(kda_beta_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, (cudaStream_t)stream, (const __nv_bfloat16*)x, out, (long long)n);
   DAISY_CHECK_LAUNCH();
   return DAISY_OK;
 }

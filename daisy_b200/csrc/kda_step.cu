@@ -72,6 +72,8 @@ __device__ __forceinline__ float log1p_unit(float u) {
 template <bool IN_BF16, bool ROUND>
 __global__ void __launch_bounds__(256) kda_gate8_kernel(const KdaGateParams p) {
   const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;         // group of eight elements
+  grid_dep_launch();
+  grid_dep_wait();
   if (i >= p.n4 / 2) return;
   const int col = (int)((i * 8) % (size_t)p.HD);                   // D % 8 == 0: one head per group
   float x[8];
@@ -191,10 +193,10 @@ extern "C" int daisy_b200_kda_gate(const void* g, int g_is_bf16, const float* a_
   if (D % 8 == 0 && (p.n4 / 2 + 255) / 256 <= 0x7fffffffULL) {
     const unsigned grid8 = (unsigned)((p.n4 / 2 + 255) / 256);
     cudaStream_t st = (cudaStream_t)stream;
-    if (p.in_bf16) { if (p.round_bf16) kda_gate8_kernel<true, true><<<grid8, 256, 0, st>>>(p);
-                     else              kda_gate8_kernel<true, false><<<grid8, 256, 0, st>>>(p); }
-    else           { if (p.round_bf16) kda_gate8_kernel<false, true><<<grid8, 256, 0, st>>>(p);
-                     else              kda_gate8_kernel<false, false><<<grid8, 256, 0, st>>>(p); }
+    if (p.in_bf16) { if (p.round_bf16) (void)daisy_host::launch_dependent(kda_gate8_kernel<true, true>, dim3(grid8), dim3(256), 0, st, p);
+                     else              (void)daisy_host::launch_dependent(kda_gate8_kernel<true, false>, dim3(grid8), dim3(256), 0, st, p); }
+    else           { if (p.round_bf16) (void)daisy_host::launch_dependent(kda_gate8_kernel<false, true>, dim3(grid8), dim3(256), 0, st, p);
+                     else              (void)daisy_host::launch_dependent(kda_gate8_kernel<false, false>, dim3(grid8), dim3(256), 0, st, p); }
     DAISY_CHECK_LAUNCH();
     return DAISY_OK;
   }

@@ -121,6 +121,8 @@ qkv_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p) {
   else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
+  grid_dep_launch();
+  grid_dep_wait();
 
   if (warp >= 9) {
     // ------------------------------------------------------------------ TMA producers: every other k-block each (a turn of the
@@ -579,10 +581,12 @@ static int launch_gemm(const GemmMaps& maps, const GemmParams& p, cudaStream_t s
   if (sms <= 0) return DAISY_ENODEV;
   cudaLaunchConfig_t cfg = {};
   cfg.blockDim = dim3(G_THREADS); cfg.dynamicSmemBytes = Cfg::SMEM; cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-  if (PAIR) { cfg.attrs = at; cfg.numAttrs = 1; }
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = 2; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+  cfg.attrs = at; cfg.numAttrs = PAIR ? 2 : 1;
   if (!attr[dev]) {
     if (cudaFuncSetAttribute(qkv_gemm_kernel<BN, PAIR, QKV>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM) != cudaSuccess) {
       (void)cudaGetLastError();

@@ -218,6 +218,8 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
+  grid_dep_launch();
+  grid_dep_wait();
 
   if (warp == TMA_WARP) {
     // ------------------------------------------------------------------ TMA producer
@@ -843,11 +845,12 @@ static int launch_attend(const void* q, const void* k, const void* v,
   // with RMS-normalised q and k every logit is bounded by scale * D: 2^(logit - reference) cannot overflow
   const bool bounded = bounded_qk && scale * 1.4426950408889634f * (float)D <= 60.f;
   cudaStream_t st = (cudaStream_t)stream;
-  // bounded logits take the form with two softmax warpgroups per stream, everything else the general form
-  if (raw && bounded)  swa_prefill_kernel<true, true, 2><<<grid, PREFILL_THREADS_SPLIT, PREFILL_SMEM, st>>>(tq, tk, tv, p);
-  else if (raw)        swa_prefill_kernel<true, false, 1><<<grid, PREFILL_THREADS, PREFILL_SMEM, st>>>(tq, tk, tv, p);
-  else if (bounded)    swa_prefill_kernel<false, true, 2><<<grid, PREFILL_THREADS_SPLIT, PREFILL_SMEM, st>>>(tq, tk, tv, p);
-  else                 swa_prefill_kernel<false, false, 1><<<grid, PREFILL_THREADS, PREFILL_SMEM, st>>>(tq, tk, tv, p);
+  // bounded logits take the form with two softmax warpgroups per stream, everything else the general form (a failed launch
+  // is what the check below reads)
+  if (raw && bounded)  (void)daisy_host::launch_dependent(swa_prefill_kernel<true, true, 2>, dim3(grid), dim3(PREFILL_THREADS_SPLIT), PREFILL_SMEM, st, tq, tk, tv, p);
+  else if (raw)        (void)daisy_host::launch_dependent(swa_prefill_kernel<true, false, 1>, dim3(grid), dim3(PREFILL_THREADS), PREFILL_SMEM, st, tq, tk, tv, p);
+  else if (bounded)    (void)daisy_host::launch_dependent(swa_prefill_kernel<false, true, 2>, dim3(grid), dim3(PREFILL_THREADS_SPLIT), PREFILL_SMEM, st, tq, tk, tv, p);
+  else                 (void)daisy_host::launch_dependent(swa_prefill_kernel<false, false, 1>, dim3(grid), dim3(PREFILL_THREADS), PREFILL_SMEM, st, tq, tk, tv, p);
   DAISY_CHECK_LAUNCH();
   return DAISY_OK;
 }

@@ -266,6 +266,44 @@ std::vector<Tensor> attn_layer(const Tensor& x_, const Tensor& qkvo_w, const Ten
   return {y, p[1], p[2], p[0]};
 }
 
+// A stack of plain layers over a prompt: layer l fills ring k[l], v[l] with rows t >= ring_first (none if negative).  The layers
+// share their scratch (they run one after another on the stream), so a prompt costs seven allocations, not seven a layer.
+Tensor attn_stack(const Tensor& x_, const std::vector<Tensor>& weights, const std::vector<Tensor>& cos, const std::vector<Tensor>& sin, int64_t H, double eps, double scale,
+                  int64_t window, const Tensor& k, const Tensor& v, int64_t ring_first) {
+  const size_t L = weights.size();
+  TORCH_CHECK_VALUE(L >= 1 && cos.size() == L && sin.size() == L && k.dim() == 5 && (size_t)k.size(0) == L && v.sizes() == k.sizes() && v.strides() == k.strides(),
+                    "one weight, one RoPE table pair and one ring per layer");
+  TORCH_CHECK_VALUE(x_.is_cuda(), "x must be a CUDA tensor (daisy_b200 has no CPU path)");
+  TORCH_CHECK_VALUE(x_.dim() == 3, "x must be [B, T, dim]");
+  c10::cuda::CUDAGuard guard(x_.device());
+  Tensor x = x_.detach().to(weights[0].scalar_type());
+  const int64_t B = x.size(0), T = x.size(1), dim = x.size(2), M = B * T;
+  const bool f16 = k.scalar_type() == at::kHalf, ring = ring_first >= 0;
+  req(x, "x"); req(k, "ring k", f16 ? at::kHalf : at::kBFloat16); req(v, "ring v", k.scalar_type());
+  TORCH_CHECK_VALUE(dim == H * 128 && k.size(1) == B && k.size(2) == H && k.size(4) == 128, "rings must be [layers, ", B, ", ", H, ", cap, 128], x [B, T, ", H * 128, "]");
+  Tensor q = at::empty({B, T, H, 128}, x.options()), kp = at::empty_like(q), vp = at::empty_like(q), o = at::empty_like(q), ya = at::empty({B, T, dim}, x.options());
+  Tensor yb = L > 1 ? at::empty_like(ya) : Tensor(), in = rows_of(x, dim);
+  int* status = status_ptr(x);
+  void* st = stream_of(x);
+  for (size_t l = 0; l < L; ++l) {
+    const Tensor& w = weights[l];
+    req(w, "qkvo_w");
+    TORCH_CHECK_VALUE(w.dim() == 3 && w.size(0) == 4 && w.size(1) == dim && w.size(2) == dim && w.is_contiguous(), "qkvo_w must be a contiguous [4, ", dim, ", ", dim, "]");
+    rope_table(cos[l], "cos"); rope_table(sin[l], "sin");
+    TORCH_CHECK_VALUE(cos[l].size(0) >= T && sin[l].size(0) >= T, "cos, sin must be contiguous float32 CUDA tensors of at least T rows");
+    char *rk = ring ? (char*)k.data_ptr() + l * k.stride(0) * 2 : nullptr, *rv = ring ? (char*)v.data_ptr() + l * v.stride(0) * 2 : nullptr;
+    check(daisy_b200_qkv_gemm_ring(in.data_ptr(), in.stride(0), w.data_ptr(), dim, cos[l].data_ptr<float>(), sin[l].data_ptr<float>(), q.data_ptr(), kp.data_ptr(),
+                                   vp.data_ptr(), nullptr, 0, nullptr, rk, rv, k.stride(1), k.stride(2), k.stride(3), (int)k.size(3), ring ? (int)ring_first : 0, (int)B,
+                                   (int)T, (int)H, 128, (int)dim, (float)eps, DAISY_QKV_DEFAULT | (f16 ? DAISY_CACHE_FP16 : 0), status, st),
+          "daisy_b200_qkv_gemm_ring");
+    swa_attend(q, kp, vp, window, scale, o, true, std::nullopt, false, false);             // q, k are RMS-normalised
+    Tensor& y = (L - 1 - l) % 2 ? yb : ya;
+    check(daisy_b200_gemm_nt(o.data_ptr(), dim, (char*)w.data_ptr() + 3 * dim * dim * 2, dim, y.data_ptr(), dim, (int)M, (int)dim, (int)dim, status, st), "daisy_b200_gemm_nt");
+    in = y.view({M, dim});
+  }
+  return ya;
+}
+
 // ------------------------------------------------------------------ attention layer under autograd
 // Forward: the fused projection (which also leaves 1 / rms of every head row), attention with its log-sum-exp, output
 // projection.  Backward: two library products for each projection, the attention backward, and one row-wise pass that undoes
@@ -656,6 +694,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                              const OptTensor& doc_start, bool in_blocks) {
     return swa_attend(q, k, v, window, scale, out, bounded, doc_start, in_blocks, true);
   });
+  m.def("attn_stack", &attn_stack);
   m.def("attn_layer", &attn_layer);
   m.def("attn_train", &attn_train);
   m.def("kda_tables", [](const py::object& cu, const py::object& device, int64_t chunk) {

@@ -37,7 +37,15 @@ class StepRunner:
     def _prefill(self, x: torch.Tensor) -> torch.Tensor:
         """``x [B,T,dim]`` through every layer's ``prefill`` (each layer sees the previous layer's output),
         the cache receives the rows ``Generator._prefill`` stores through ``bulk_write_packed``."""
-        T = x.size(1)
+        T, c, a = x.size(1), self.cache, self.layers[0]
+        if x.is_cuda and x.size(0) == c.B and self._plain():               # the same launches, issued by one native call
+            rot = [m._modules["rotary"]._buffers for m in self.layers]
+            if T >= 1 and all(r["cos"].size(0) >= T for r in rot):
+                r = min(T, max(c.W - 1, 0))
+                x = ext().attn_stack(x, [m._parameters["qkvo_w"] for m in self.layers], [r_["cos"] for r_ in rot], [r_["sin"] for r_ in rot],
+                                     a.num_heads, a.norm_eps, a.attn_scale, self.window, c.k, c.v, T - r if r > 0 else -1)
+                c.set_position(T)
+                return x
         for i, a in enumerate(self.layers):
             # the projection's epilogue stores the rows bulk_write_packed keeps straight into their ring slots
             x, _, _ = a.prefill_ring(x, None, self.cache, i, attn_mask=WindowMask(self.window))
@@ -45,12 +53,16 @@ class StepRunner:
         return x
 
     # ------------------------------------------------------------------ all layers in one launch
+    def _plain(self) -> bool:
+        """Plain layers of one shape with the same constants."""
+        a = self.layers[0]
+        return all(type(m) is B200CausalSelfAttention and not m.receives_ve and m.num_heads == a.num_heads
+                   and m.attn_scale == a.attn_scale and m.norm_eps == a.norm_eps for m in self.layers)
+
     def _one_launch(self, x: torch.Tensor) -> bool:
-        """Whether the whole stack fits the single-launch step: plain layers of one shape with the same constants."""
-        c, a = self.cache, self.layers[0]
-        return (x.size(0) == c.B and all(type(m) is B200CausalSelfAttention and not m.receives_ve and m.num_heads == a.num_heads
-                                         and m.attn_scale == a.attn_scale and m.norm_eps == a.norm_eps for m in self.layers)
-                and ext().token_step_supported(c.B, c.H, len(self.layers)))
+        """Whether the whole stack fits the single-launch step."""
+        c = self.cache
+        return x.size(0) == c.B and self._plain() and ext().token_step_supported(c.B, c.H, len(self.layers))
 
     def _token(self, x, t, t_dev, out=None, workspace=None):
         c, a = self.cache, self.layers[0]

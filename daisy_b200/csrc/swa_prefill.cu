@@ -50,6 +50,7 @@ struct PrefillParams {
   __nv_bfloat16* out;
   int64_t o_sb, o_st, o_sh;
   int T, H, B, window;
+  int streams;             // query tiles of 128 rows in an item: 2, or 1 (few items)
   int window_blocks;       // > 0: block-granular window (key tile >= query tile - window_blocks + 1), window = 0
   float scale_log2;
   int* status;
@@ -91,15 +92,15 @@ struct ItemGeom {
   bool valid[2];
   int jlo, jhi;
 };
-__device__ __forceinline__ ItemGeom item_geom(int item, int nq, int H, int T, int window,
+__device__ __forceinline__ ItemGeom item_geom(int item, int nq, int H, int T, int window, int streams,
                                               const int* doc_start = nullptr, int64_t doc_sb = 0, int window_blocks = 0) {
   ItemGeom g;
   const int qp = item % nq, bh = item / nq;
   g.h = bh % H; g.b = bh / H;
 #pragma unroll
   for (int s = 0; s < 2; ++s) {
-    g.q0[s] = (qp * 2 + s) * BM;
-    g.valid[s] = g.q0[s] < T;
+    g.q0[s] = (qp * streams + s) * BM;
+    g.valid[s] = s < streams && g.q0[s] < T;
     int klo = window > 0 ? max(0, g.q0[s] - window + 1) : 0;
     // block-granular window of the training form: whole key tiles, the nearest window_blocks of them
     if (window_blocks > 0) klo = max(0, g.q0[s] / BM - window_blocks + 1) * BN;
@@ -166,9 +167,9 @@ __device__ __forceinline__ bool prepare_q_tile(PrefillBarriers* bars, uint8_t* q
 
 // Persistent schedule: item = (batch*H + head) * nq + q-pair, walked in the balanced order of BalancedWalk (all
 // q-pairs that see a full window first, (batch, head)-major; then the causal-ramp q-pairs, longest first).
-__device__ __forceinline__ BalancedWalk prefill_walk(int nq, int BH, int window, int window_blocks) {
+__device__ __forceinline__ BalancedWalk prefill_walk(int nq, int BH, int window, int window_blocks, int streams) {
   const int span = window > 0 ? window : (window_blocks > 0 ? window_blocks * BN : 0);       // keys a full row sees
-  return BalancedWalk(nq, BH, span > 0 ? (span + 2 * BM - 1) / (2 * BM) : nq, false);
+  return BalancedWalk(nq, BH, span > 0 ? (span + streams * BM - 1) / (streams * BM) : nq, false);
 }
 
 // Barrier phases are kept as
@@ -196,8 +197,8 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   constexpr int TMA_WARP = 8 * NSPLIT, MMA_WARP = 8 * NSPLIT + 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int T = p.T, window = p.window;
-  const int nq = (T + 2 * BM - 1) / (2 * BM);
-  const BalancedWalk walk = prefill_walk(nq, p.H * p.B, window, p.window_blocks);
+  const int nq = (T + p.streams * BM - 1) / (p.streams * BM);
+  const BalancedWalk walk = prefill_walk(nq, p.H * p.B, window, p.window_blocks, p.streams);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < 2; ++s) {
@@ -231,7 +232,7 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       // Q tiles run one item ahead of the K/V stream (double buffer), so the softmax warps can prepare the
       // next item's Q while the current item is still computing.
       auto load_q = [&](int it_item) {
-        const ItemGeom gq = item_geom(it_item, nq, p.H, T, window, p.doc_start, p.doc_sb, p.window_blocks);
+        const ItemGeom gq = item_geom(it_item, nq, p.H, T, window, p.streams, p.doc_start, p.doc_sb, p.window_blocks);
         for (int s = 0; s < 2 && ok; ++s) {
           if (!gq.valid[s]) continue;
           const int qb = qn[s] % NQBUF;
@@ -245,7 +246,7 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       };
       if (walk.at(0) >= 0) load_q(walk.at(0));
       for (int rd = 0, item; (item = walk.at(rd)) >= 0 && ok; ++rd) {
-        const ItemGeom g = item_geom(item, nq, p.H, T, window, p.doc_start, p.doc_sb, p.window_blocks);
+        const ItemGeom g = item_geom(item, nq, p.H, T, window, p.streams, p.doc_start, p.doc_sb, p.window_blocks);
         for (int j = g.jlo; j <= g.jhi && ok; ++j) {
           for (int kv = 0; kv < 2; ++kv, ++n) {
             const int stage = n % NSTAGE;
@@ -285,7 +286,7 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       uint32_t n_q[2] = {0, 0};          // Q tiles consumed so far per stream (phase of q_full)
       bool ok = true;
       for (int rd = 0, item; (item = walk.at(rd)) >= 0 && ok; ++rd) {
-        const ItemGeom g = item_geom(item, nq, p.H, T, window, p.doc_start, p.doc_sb, p.window_blocks);
+        const ItemGeom g = item_geom(item, nq, p.H, T, window, p.streams, p.doc_start, p.doc_sb, p.window_blocks);
         for (int j = g.jlo; j <= g.jhi + 1 && ok; ++j) {
 #pragma unroll
           for (int s = 0; s < 2; ++s) {
@@ -355,7 +356,7 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     bool ok = true;
     bool q_prepared = false;                                       // raw-Q mode: the lower half prepares the stream's Q rows
     for (int rd = 0, item; (item = walk.at(rd)) >= 0 && ok; ++rd) {
-      const ItemGeom g = item_geom(item, nq, p.H, T, window, p.doc_start, p.doc_sb, p.window_blocks);
+      const ItemGeom g = item_geom(item, nq, p.H, T, window, p.streams, p.doc_start, p.doc_sb, p.window_blocks);
       if (!g.valid[s]) continue;
       const int q0 = g.q0[s];
       const int q_row = q0 + row;
@@ -368,7 +369,7 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         q_prepared = false;
         const int item_next = walk.at(rd + 1);
         if (item_next >= 0) {
-          const ItemGeom gn = item_geom(item_next, nq, p.H, T, window, p.doc_start, p.doc_sb, p.window_blocks);
+          const ItemGeom gn = item_geom(item_next, nq, p.H, T, window, p.streams, p.doc_start, p.doc_sb, p.window_blocks);
           next_valid = gn.valid[s];
           q_row_next = gn.q0[s] + row;
         }
@@ -511,7 +512,7 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     bool q_prepared = false;
     auto prepare_q = [&](int qrow) -> bool { return prepare_q_tile(bars, q_tiles, s, row, n_qs, qrow, p, abort_flag); };
     for (int rd = 0, item; (item = walk.at(rd)) >= 0 && ok; ++rd) {
-      const ItemGeom g = item_geom(item, nq, p.H, T, window, p.doc_start, p.doc_sb, p.window_blocks);
+      const ItemGeom g = item_geom(item, nq, p.H, T, window, p.streams, p.doc_start, p.doc_sb, p.window_blocks);
       if (!g.valid[s]) continue;
       const int q0 = g.q0[s];
       const int q_row = q0 + row;
@@ -526,7 +527,7 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       bool next_valid = false;
       int q_row_next = 0;
       if (QRAW && item_next >= 0) {
-        const ItemGeom gn = item_geom(item_next, nq, p.H, T, window, p.doc_start, p.doc_sb, p.window_blocks);
+        const ItemGeom gn = item_geom(item_next, nq, p.H, T, window, p.streams, p.doc_start, p.doc_sb, p.window_blocks);
         next_valid = gn.valid[s];
         q_row_next = gn.q0[s] + row;
       }
@@ -836,10 +837,14 @@ static int launch_attend(const void* q, const void* k, const void* v,
   p.cos = qt ? qt->cos : nullptr; p.sin = qt ? qt->sin : nullptr;
   p.eps = qt ? qt->eps : 0.f; p.q_norm = qt ? qt->norm : 0; p.q_rope = qt ? qt->rope : 0;
   p.lse2 = lse2;
-  const int64_t items = (int64_t)((T + 2 * BM - 1) / (2 * BM)) * H * B;
-  if (items >= (int64_t)1 << 31) return DAISY_EUNSUPPORTED;
   const int sms = daisy_host::sm_count_cached();
   if (sms <= 0) return DAISY_ENODEV;
+  // where one wave holds all 128-row tiles each gets an SM: the second stream pays by sharing K and V, not for latency
+  // (1 x 1024 tokens, 6 heads, window 512: 16.7 -> 13.6 us)
+  const int64_t tiles = (int64_t)((T + BM - 1) / BM) * H * B;
+  p.streams = tiles <= sms ? 1 : 2;
+  const int64_t items = (int64_t)((T + p.streams * BM - 1) / (p.streams * BM)) * H * B;
+  if (items >= (int64_t)1 << 31) return DAISY_EUNSUPPORTED;
   dim3 grid((unsigned)(items < sms ? items : sms), 1, 1);
   const bool raw = qt && (qt->norm || qt->rope);
   // with RMS-normalised q and k every logit is bounded by scale * D: 2^(logit - reference) cannot overflow

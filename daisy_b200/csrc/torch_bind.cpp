@@ -310,6 +310,18 @@ Tensor attn_stack(const Tensor& x_, const std::vector<Tensor>& weights, const st
 // norms, RoPE and gate into the merged gradient matrix.  As F.linear calls around the attention core this took a copy of the
 // merged gradient (concatenation of three), zero fills and an addition for the two slices of the weight's gradient, a separate
 // norm / RoPE pass and its raw inputs.
+// What the forward leaves for the backward, in one allocation (a small step costs more in allocator calls than in kernels):
+// byte offsets of q', k', v', vn (gated layers), o, 1 / rms and the log-sum-exp.
+struct Saved {
+  int64_t q, k, v, vn, o, rstd, lse, elems;
+  static int64_t up(int64_t n) { return (n + 255) / 256 * 256; }
+  Saved(int64_t M, int64_t H, bool gated) {
+    const int64_t rows = up(M * H * 256);
+    q = 0; k = rows; v = 2 * rows; vn = 3 * rows;
+    o = (gated ? 4 : 3) * rows; rstd = o + rows; lse = rstd + up(M * 3 * H * 4);
+    elems = (lse + up(M * H * 4)) / 2;                                                      // of bf16
+  }
+};
 struct AttnFunction : public torch::autograd::Function<AttnFunction> {
   static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& x, const Tensor& w, const OptTensor& ve, const OptTensor& logit, const Tensor& cos,
                         const Tensor& sin, int64_t H, double eps, double scale, int64_t window, const OptTensor& doc_start, bool in_blocks) {
@@ -319,23 +331,30 @@ struct AttnFunction : public torch::autograd::Function<AttnFunction> {
     TORCH_CHECK_VALUE(w.dim() == 3 && w.size(0) == 4 && w.is_contiguous() && dim == H * 128 && x.size(2) == dim, "qkvo_w must be a contiguous [4, dim, dim]");
     rope_table(cos, "cos"); rope_table(sin, "sin");
     Tensor x2 = rows_of(x, dim);
-    auto q = at::empty({B, T, H, 128}, x.options()), k = at::empty_like(q), v = at::empty_like(q);
-    Tensor rstd = at::empty({M, 3 * H}, x.options().dtype(at::kFloat)), vn = v, ve2, g32;
+    Tensor ve2, g32;
     if (ve.has_value()) {
       req(*ve, "ve");
       ve2 = ve->reshape({M, dim});
       if (!ve2.is_contiguous()) ve2 = ve2.contiguous();
       g32 = logit->to(at::kFloat).reshape({1});
-      vn = at::empty_like(q);
     }
-    check(daisy_b200_qkv_gemm_train(x2.data_ptr(), x2.stride(0), w.data_ptr(), dim, cos.data_ptr<float>(), sin.data_ptr<float>(), q.data_ptr(), k.data_ptr(),
-                                    v.data_ptr(), rstd.data_ptr<float>(), ve2.defined() ? vn.data_ptr() : nullptr, ve2.defined() ? ve2.data_ptr() : nullptr,
-                                    ve2.defined() ? dim : 0, ve2.defined() ? g32.data_ptr<float>() : nullptr, (int)B, (int)T, (int)H, 128, (int)dim, (float)eps,
-                                    DAISY_QKV_DEFAULT, status_ptr(x), stream_of(x)),
+    const Saved at_(M, H, ve2.defined());
+    Tensor buf = at::empty({at_.elems}, x.options());
+    char* p = (char*)buf.data_ptr();
+    Doc dc = doc_arg(doc_start, B, T, x);
+    int* status = status_ptr(x);
+    void* st = stream_of(x);
+    check(daisy_b200_qkv_gemm_train(x2.data_ptr(), x2.stride(0), w.data_ptr(), dim, cos.data_ptr<float>(), sin.data_ptr<float>(), p + at_.q, p + at_.k, p + at_.v,
+                                    (float*)(p + at_.rstd), ve2.defined() ? p + at_.vn : nullptr, ve2.defined() ? ve2.data_ptr() : nullptr, ve2.defined() ? dim : 0,
+                                    ve2.defined() ? g32.data_ptr<float>() : nullptr, (int)B, (int)T, (int)H, 128, (int)dim, (float)eps, DAISY_QKV_DEFAULT, status, st),
           "daisy_b200_qkv_gemm_train");
-    auto [o, lse] = swa_attend(q, k, v, window, scale, std::nullopt, true, doc_start, in_blocks, true);
-    Tensor y = gemm_nt(o.view({B, T, dim}), w.select(0, 3));
-    ctx->save_for_backward({x2, w, q, k, v, o, lse, rstd, cos, sin, ve2, g32, vn, doc_start.has_value() ? *doc_start : Tensor()});
+    const int64_t sb = T * dim, sh = 128;
+    check(daisy_b200_swa_attend_lse(p + at_.q, p + at_.k, p + at_.v, sb, dim, sh, sb, dim, sh, sb, dim, sh, p + at_.o, sb, dim, sh, (float*)(p + at_.lse), (int)B, (int)T,
+                                    (int)H, 128, (int)window, (float)scale, dc.ptr, dc.sb, DAISY_BOUNDED_QK | (in_blocks ? DAISY_WINDOW_BLOCKS : 0), status, st),
+          "daisy_b200_swa_attend_lse");                                                    // q, k are RMS-normalised
+    Tensor y = at::empty({B, T, dim}, x.options());
+    check(daisy_b200_gemm_nt(p + at_.o, dim, (char*)w.data_ptr() + 3 * dim * dim * 2, dim, y.data_ptr(), dim, (int)M, (int)dim, (int)dim, status, st), "daisy_b200_gemm_nt");
+    ctx->save_for_backward({x2, w, buf, cos, sin, ve2, g32, doc_start.has_value() ? *doc_start : Tensor()});
     ctx->saved_data["dims"] = std::vector<int64_t>{B, T, H, window, in_blocks ? 1 : 0};
     ctx->saved_data["scale"] = scale;
     if (ve.has_value()) {
@@ -348,39 +367,43 @@ struct AttnFunction : public torch::autograd::Function<AttnFunction> {
   static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
     at::AutoDispatchBelowADInplaceOrView guard;
     auto s = ctx->get_saved_variables();
-    const Tensor &x2 = s[0], &w = s[1], &q = s[2], &k = s[3], &v = s[4], &o = s[5], &lse = s[6], &rstd = s[7], &cos = s[8], &sin = s[9], &ve2 = s[10], &g32 = s[11],
-                 &vn = s[12], &doc = s[13];
+    const Tensor &x2 = s[0], &w = s[1], &buf = s[2], &cos = s[3], &sin = s[4], &ve2 = s[5], &g32 = s[6], &doc = s[7];
     auto d = ctx->saved_data["dims"].toIntVector();
     const int64_t B = d[0], T = d[1], H = d[2], window = d[3], dim = H * 128, M = B * T;
     const float scale = (float)ctx->saved_data["scale"].toDouble();
     const bool need_x = ctx->needs_input_grad(0), need_w = ctx->needs_input_grad(1);
     Tensor dy = grads[0].to(at::kBFloat16).reshape({M, dim});
     if (dy.stride(1) != 1) dy = dy.contiguous();
+    const Saved at_(M, H, ve2.defined());
+    char* p = (char*)buf.data_ptr();
     Tensor dw, dx;
     if (need_w) {
       dw = at::empty_like(w);
       Tensor dwo = dw.select(0, 3);
-      at::mm_out(dwo, dy.t(), o.view({M, dim}));
+      at::mm_out(dwo, dy.t(), buf.narrow(0, at_.o / 2, M * dim).view({M, dim}));
     }
-    Tensor d_o = at::mm(dy, w.select(0, 3)).view({B, T, H, 128});
-    auto dq = at::empty_like(q), dk = at::empty_like(q), dv = at::empty_like(q);
-    Tensor ws = at::empty({(int64_t)daisy_b200_swa_attend_bwd_workspace_bytes((int)B, (int)T, (int)H)}, q.options().dtype(at::kByte));
-    Doc dc = doc_arg(doc.defined() ? OptTensor(doc) : std::nullopt, B, T, q);
+    Tensor d_o = at::mm(dy, w.select(0, 3));
+    const size_t ws_bytes = daisy_b200_swa_attend_bwd_workspace_bytes((int)B, (int)T, (int)H);
+    const int64_t row = Saved::up(M * dim * 2), ws_at = 6 * row, part_at = ws_at + Saved::up((int64_t)ws_bytes);
+    const int64_t n_part = ve2.defined() ? daisy_b200_qkv_prep_grad_blocks((int)M, (int)H) : 0;
+    Tensor tmp = at::empty({(part_at + Saved::up(4 * n_part)) / 2}, buf.options());          // dqkv, dq, dk, dv, workspace, partial sums
+    char *g = (char*)tmp.data_ptr(), *dq = g + 3 * row, *dk = g + 4 * row, *dv = g + 5 * row;
+    Tensor dqkv = tmp.narrow(0, 0, M * 3 * dim).view({M, 3 * dim}), d_ve, d_logit;
+    Doc dc = doc_arg(doc.defined() ? OptTensor(doc) : std::nullopt, B, T, buf);
     const int64_t sb = T * H * 128, st = H * 128, sh = 128;
-    check(daisy_b200_swa_attend_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), d_o.data_ptr(), sb, st, sh, sb, st, sh, sb, st, sh, sb, st, sh, sb, st, sh,
-                                    lse.data_ptr<float>(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), (int)B, (int)T, (int)H, 128, (int)window, scale, dc.ptr, dc.sb,
-                                    d[4] ? DAISY_WINDOW_BLOCKS : 0, ws.data_ptr(), (size_t)ws.numel(), status_ptr(q), stream_of(q)),
+    void* stream = stream_of(buf);
+    check(daisy_b200_swa_attend_bwd(p + at_.q, p + at_.k, p + at_.v, p + at_.o, d_o.data_ptr(), sb, st, sh, sb, st, sh, sb, st, sh, sb, st, sh, sb, st, sh,
+                                    (const float*)(p + at_.lse), dq, dk, dv, (int)B, (int)T, (int)H, 128, (int)window, scale, dc.ptr, dc.sb,
+                                    d[4] ? DAISY_WINDOW_BLOCKS : 0, g + ws_at, ws_bytes, status_ptr(buf), stream),
           "daisy_b200_swa_attend_bwd");
-    Tensor dqkv = at::empty({M, 3 * dim}, q.options()), d_ve, d_logit, part;
     if (ve2.defined()) {
-      d_ve = at::empty({M, dim}, q.options());
-      d_logit = at::empty({1}, q.options().dtype(at::kFloat));
-      part = at::empty({daisy_b200_qkv_prep_grad_blocks((int)M, (int)H)}, q.options().dtype(at::kFloat));
+      d_ve = at::empty({M, dim}, buf.options());
+      d_logit = at::empty({1}, buf.options().dtype(at::kFloat));
     }
     auto ptr = [](const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; };
-    check(daisy_b200_qkv_prep_grad(q.data_ptr(), k.data_ptr(), vn.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), rstd.data_ptr<float>(), cos.data_ptr<float>(),
-                                   sin.data_ptr<float>(), dqkv.data_ptr(), ptr(ve2), (const float*)ptr(g32), ptr(d_ve), (float*)ptr(d_logit), (float*)ptr(part), (int)M,
-                                   (int)T, (int)H, 128, stream_of(q)),
+    check(daisy_b200_qkv_prep_grad(p + at_.q, p + at_.k, p + (ve2.defined() ? at_.vn : at_.v), dq, dk, dv, (const float*)(p + at_.rstd), cos.data_ptr<float>(),
+                                   sin.data_ptr<float>(), dqkv.data_ptr(), ptr(ve2), (const float*)ptr(g32), ptr(d_ve), (float*)ptr(d_logit),
+                                   n_part ? (float*)(g + part_at) : nullptr, (int)M, (int)T, (int)H, 128, stream),
           "daisy_b200_qkv_prep_grad");
     const Tensor wqkv = w.narrow(0, 0, 3).view({3 * dim, dim});
     if (need_w) {

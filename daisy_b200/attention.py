@@ -278,8 +278,13 @@ class B200CausalSelfAttention(nn.Module):
         mask = self._window_of(attn_mask)
         if self._needs_grad(x) or (ve is not None and torch.is_grad_enabled() and ve.requires_grad):
             return self._attend_autograd(x, ve, mask)
-        y, _, _, _ = self._attend(x, ve, mask)
-        return y
+        cos, sin = self.rotary.tables(x.size(1))
+        gate = None
+        if self.receives_ve:
+            torch._assert(ve is not None, "ve must be provided when receives_ve=True")
+            ve, gate = ve.to(torch.bfloat16), self.g_ve.detach().float().reshape(1)
+        return ext().attn_forward(x, self.qkvo_w, cos, sin, self.num_heads, self.norm_eps, self.attn_scale, int(mask[0] or 0), mask[1],
+                                  len(mask) > 2 and mask[2], ve if self.receives_ve else None, gate)
 
     def prefill(self, x: Tensor, ve: Optional[Tensor], attn_mask=None, debug: bool = False):
         """Returns ``(y [B,T,dim], k [B,H,T,D], v [B,H,T,D])`` (models/daisy/attention.py:173-179)."""

@@ -252,6 +252,43 @@ std::pair<Tensor, Tensor> swa_attend(const Tensor& q, const Tensor& k, const Ten
   return {out, lse};
 }
 
+// The layer's output alone: q', k', v' and the attention output are scratch, one allocation.
+Tensor attn_forward(const Tensor& x_, const Tensor& qkvo_w, const Tensor& cos, const Tensor& sin, int64_t H, double eps, double scale, int64_t window,
+                    const OptTensor& doc_start, bool in_blocks, const OptTensor& ve, const OptTensor& ve_gate) {
+  TORCH_CHECK_VALUE(x_.is_cuda(), "x must be a CUDA tensor (daisy_b200 has no CPU path)");
+  const Tensor x = x_.detach().to(qkvo_w.scalar_type());
+  req(x, "x"); req(qkvo_w, "qkvo_w");
+  c10::cuda::CUDAGuard guard(x.device());
+  TORCH_CHECK_VALUE(x.dim() == 3, "x must be [B, T, dim]");
+  const int64_t B = x.size(0), T = x.size(1), dim = x.size(2), M = B * T;
+  TORCH_CHECK_VALUE(qkvo_w.dim() == 3 && qkvo_w.size(0) == 4 && qkvo_w.size(1) == dim && qkvo_w.size(2) == dim && dim == H * 128 && qkvo_w.is_contiguous(),
+                    "qkvo_w must be a contiguous [4, ", dim, ", ", dim, "]");
+  rope_table(cos, "cos"); rope_table(sin, "sin");
+  TORCH_CHECK_VALUE(cos.size(0) >= T && sin.size(0) >= T, "cos, sin must be contiguous float32 CUDA tensors of at least T rows");
+  Tensor x2 = rows_of(x, dim), ve2;
+  if (ve.has_value()) {
+    TORCH_CHECK_VALUE(ve_gate.has_value() && ve_gate->is_cuda() && ve_gate->scalar_type() == at::kFloat && ve_gate->numel() == 1,
+                      "ve needs ve_gate_logit, a float32 scalar CUDA tensor");
+    ve2 = ve->reshape({M, dim});
+    req(ve2, "ve");
+  }
+  const int64_t n = M * dim, sb = T * dim;
+  Tensor buf = at::empty({4 * n}, x.options()), y = at::empty({B, T, dim}, x.options());
+  char *q = (char*)buf.data_ptr(), *k = q + 2 * n, *v = k + 2 * n, *o = v + 2 * n;
+  Doc dc = doc_arg(doc_start, B, T, x);
+  int* status = status_ptr(x);
+  void* st = stream_of(x);
+  check(daisy_b200_qkv_gemm(x2.data_ptr(), x2.stride(0), qkvo_w.data_ptr(), dim, cos.data_ptr<float>(), sin.data_ptr<float>(), q, k, v,
+                            ve2.defined() ? ve2.data_ptr() : nullptr, ve2.defined() ? ve2.stride(0) : 0, ve2.defined() ? ve_gate->data_ptr<float>() : nullptr, (int)B,
+                            (int)T, (int)H, 128, (int)dim, (float)eps, DAISY_QKV_DEFAULT, status, st),
+        "daisy_b200_qkv_gemm");
+  check(daisy_b200_swa_attend(q, k, v, sb, dim, 128, sb, dim, 128, sb, dim, 128, o, sb, dim, 128, (int)B, (int)T, (int)H, 128, (int)window, (float)scale, dc.ptr, dc.sb,
+                              DAISY_BOUNDED_QK | (in_blocks ? DAISY_WINDOW_BLOCKS : 0), status, st),
+        "daisy_b200_swa_attend");                                                          // q, k are RMS-normalised
+  check(daisy_b200_gemm_nt(o, dim, (char*)qkvo_w.data_ptr() + 3 * dim * dim * 2, dim, y.data_ptr(), dim, (int)M, (int)dim, (int)dim, status, st), "daisy_b200_gemm_nt");
+  return y;
+}
+
 // One attention layer: projection, attention, output projection -> (y, k', v', q')
 std::vector<Tensor> attn_layer(const Tensor& x_, const Tensor& qkvo_w, const Tensor& cos, const Tensor& sin, int64_t H, double eps, double scale, int64_t window,
                                const OptTensor& doc_start, bool in_blocks, const OptTensor& ve, const OptTensor& ve_gate, const OptTensor& ring_k,
@@ -718,6 +755,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     return swa_attend(q, k, v, window, scale, out, bounded, doc_start, in_blocks, true);
   });
   m.def("attn_stack", &attn_stack);
+  m.def("attn_forward", &attn_forward);
   m.def("attn_layer", &attn_layer);
   m.def("attn_train", &attn_train);
   m.def("kda_tables", [](const py::object& cu, const py::object& device, int64_t chunk) {

@@ -155,17 +155,6 @@ __device__ __forceinline__ uint32_t hmul2_u32(uint32_t a, uint32_t b) {
   asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
   return d;
 }
-__device__ __forceinline__ uint4 ld_nc16(const void* p) {
-  uint4 r;
-  asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
-  return r;
-}
-
-__device__ __forceinline__ uint2 ld_nc8(const void* p) {
-  uint2 r;
-  asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(r.x), "=r"(r.y) : "l"(p));
-  return r;
-}
 // two fp16 values times fp32 factors, one rounding
 __device__ __forceinline__ uint32_t ki_scale(uint32_t a, const float2 f) {
   const float2 x = unpack_h2(a);
@@ -183,8 +172,7 @@ __global__ void __launch_bounds__(KI_THREADS, 3) kda_intra_kernel(const KdaIntra
   const size_t tok = ((size_t)b * p.T + t0) * p.H + h, ts = (size_t)p.H * KD;      // row of token i: tok * KD + i * ts
 
   if (tid < KC) sm.beta[tid] = tid < rows ? p.beta[tok + (size_t)tid * p.H] : 0.f;
-  for (int i = tid; i < 4 * rows; i += KI_THREADS)                                 // g and v are needed later: ask L2 for them now
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(p.g + tok * KD + (size_t)(i >> 2) * ts + 32 * (i & 3)));
+  // v is needed last: ask L2 for it now
   for (int i = tid; i < 2 * rows; i += KI_THREADS)
     asm volatile("prefetch.global.L2 [%0];" ::"l"(p.v + tok * KD + (size_t)(i >> 1) * ts + 64 * (i & 1)));
   const int r0 = 16 * warp + g8, r1 = r0 + 8;                                      // this lane's two rows in the products
@@ -193,18 +181,39 @@ __global__ void __launch_bounds__(KI_THREADS, 3) kda_intra_kernel(const KdaIntra
   // fragment addresses: A = {k octet, q octet} x 16 channels from images at s_pk, s_pq; lane l gives row (l & 7) of matrix l >> 3
   const uint32_t s_kq = (lane & 8) ? s_pq : s_pk;
 
-  // ---- raw rows (bf16) through shared memory: 1 / |k|, 1 / |q| and q . k are diagonals of products
+  // ---- everything the levels read is on its way before the first wait: the raw rows of k and q (bf16), then g, 64 channels at a
+  //      time (fp32): the first half where the level images come later, the second where this warp's rows of the solve's operands do
+  const uint32_t s_akh = smem_u32(&sm.akh[16 * warp][0]), s_dg = smem_u32(sm.dg[warp]), s_th = smem_u32(sm.th[warp]);
+  auto g1_row = [&](int r) { return r < 9 ? s_akh + 256 * r : r < 14 ? s_dg + 256 * (r - 9) : s_th + 256 * (r - 14); };
+  static_assert(sizeof(sm.akh) / 4 >= 9 * 256 && sizeof(sm.dg[0]) >= 5 * 256 && sizeof(sm.th[0]) >= 2 * 256, "room for 16 rows of g");
   {
     const size_t base = tok * KD + (size_t)(16 * warp) * ts;
+    const int c = lane & 15;
+    auto copy = [&](uint32_t dst, const void* src, bool ok) {                      // rows past the end: zeros
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16u : 0u) : "memory");
+    };
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const int r = 2 * i + (lane >> 4), c = lane & 15;
+      const int r = 2 * i + (lane >> 4);
       const bool ok = r < nrow;
-      const uint4 kv = ok ? ld_nc16(p.k + base + r * ts + 8 * c) : make_uint4(0, 0, 0, 0), qv = ok ? ld_nc16(p.q + base + r * ts + 8 * c) : make_uint4(0, 0, 0, 0);
-      *reinterpret_cast<uint4*>(sm.pk[warp] + r * KI_LD + 16 * c) = kv;
-      *reinterpret_cast<uint4*>(sm.pq[warp] + r * KI_LD + 16 * c) = qv;
+      const size_t at = ok ? base + r * ts + 8 * c : tok * KD;
+      copy(s_pk + r * KI_LD + 16 * c, p.k + at, ok);
+      copy(s_pq + r * KI_LD + 16 * c, p.q + at, ok);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+#pragma unroll
+    for (int hf = 0; hf < 2; ++hf) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int r = 2 * i + (lane >> 4);
+        const bool ok = r < nrow;
+        copy((hf ? g1_row(r) : s_suf + 256 * r) + 16 * c, p.g + (ok ? base + r * ts + 64 * hf + 4 * c : tok * KD), ok);
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
     }
   }
+  // 1 / |k|, 1 / |q| and q . k are diagonals of products
+  asm volatile("cp.async.wait_group 2;" ::: "memory");
   __syncwarp();
   {
 #pragma unroll
@@ -241,10 +250,13 @@ __global__ void __launch_bounds__(KI_THREADS, 3) kda_intra_kernel(const KdaIntra
     uint64_t pre[16], suf[16];                                                     // fp32 pairs: the lane's two channels
     uint32_t kh[16], qh[16];                                                       // normalised, fp16 pairs
     {
-      const float* gp = p.g + tok * KD + (size_t)(16 * warp) * ts + 64 * hf + 2 * lane;
+      if (hf == 0) asm volatile("cp.async.wait_group 1;" ::: "memory");
+      else asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncwarp();
       uint2 gv[16];
 #pragma unroll
-      for (int t = 0; t < 16; ++t) gv[t] = t < nrow ? ld_nc8(gp + t * ts) : make_uint2(0, 0);
+      for (int t = 0; t < 16; ++t)
+        asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(gv[t].x), "=r"(gv[t].y) : "r"((hf ? g1_row(t) : s_suf + 256 * t) + 8 * lane) : "memory");
 #pragma unroll
       for (int t = 0; t < 16; ++t) {
         pre[t] = pack2f(fast_exp2(__uint_as_float(gv[t].x) * 1.4426950408889634f), fast_exp2(__uint_as_float(gv[t].y) * 1.4426950408889634f));

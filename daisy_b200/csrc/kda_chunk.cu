@@ -171,10 +171,6 @@ __global__ void __launch_bounds__(KI_THREADS, 3) kda_intra_kernel(const KdaIntra
   uint8_t* rec = p.ws + ((size_t)(b * p.H + h) * p.NC + chunk) * REC_BYTES;
   const size_t tok = ((size_t)b * p.T + t0) * p.H + h, ts = (size_t)p.H * KD;      // row of token i: tok * KD + i * ts
 
-  if (tid < KC) sm.beta[tid] = tid < rows ? p.beta[tok + (size_t)tid * p.H] : 0.f;
-  // v is needed last: ask L2 for it now
-  for (int i = tid; i < 2 * rows; i += KI_THREADS)
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(p.v + tok * KD + (size_t)(i >> 1) * ts + 64 * (i & 1)));
   const int r0 = 16 * warp + g8, r1 = r0 + 8;                                      // this lane's two rows in the products
   const int nrow = rows - 16 * warp;                                               // rows of this block that exist (<= 0: none)
   const uint32_t s_suf = smem_u32(sm.suf[warp]), s_pk = smem_u32(sm.pk[warp]), s_pq = smem_u32(sm.pq[warp]);
@@ -200,6 +196,9 @@ __global__ void __launch_bounds__(KI_THREADS, 3) kda_intra_kernel(const KdaIntra
       copy(s_pk + r * KI_LD + 16 * c, p.k + at, ok);
       copy(s_pq + r * KI_LD + 16 * c, p.q + at, ok);
     }
+    if (lane < 16)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;"
+                   ::"r"(smem_u32(&sm.beta[16 * warp + lane])), "l"(p.beta + tok + (size_t)(lane < nrow ? 16 * warp + lane : 0) * p.H), "r"(lane < nrow ? 4u : 0u) : "memory");
     asm volatile("cp.async.commit_group;" ::: "memory");
 #pragma unroll
     for (int hf = 0; hf < 2; ++hf) {
@@ -212,6 +211,9 @@ __global__ void __launch_bounds__(KI_THREADS, 3) kda_intra_kernel(const KdaIntra
       asm volatile("cp.async.commit_group;" ::: "memory");
     }
   }
+  // v is needed last: ask L2 for it now
+  for (int i = tid; i < 2 * rows; i += KI_THREADS)
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(p.v + tok * KD + (size_t)(i >> 1) * ts + 64 * (i & 1)));
   // 1 / |k|, 1 / |q| and q . k are diagonals of products
   asm volatile("cp.async.wait_group 2;" ::: "memory");
   __syncwarp();
@@ -342,10 +344,14 @@ __global__ void __launch_bounds__(KI_THREADS, 3) kda_intra_kernel(const KdaIntra
   __syncwarp();
   __syncthreads();
 
-  // ---- products with the earlier blocks
+  // ---- products with the earlier blocks: (1, 0); (2, 1), (2, 0); (3, 2), (3, 1) and, by warp 0, which has none of its own, (3, 0)
   const float b0 = sm.beta[r0], b1 = sm.beta[r1];
+  const int I = warp ? warp : 3;
 #pragma unroll 1
-  for (int J = warp - 1; J >= 0; --J) {
+  for (int J = warp ? warp - 1 : 0; J >= (warp == 3 ? 1 : 0); --J) {
+    const int i0 = 16 * I + g8, i1 = i0 + 8;
+    const float e0_ = sm.beta[i0], e1_ = sm.beta[i1];
+    const uint32_t s_ki = smem_u32(sm.pk[I]), s_qi = smem_u32(sm.pq[I]);
     float kk[2][4], qk[2][4];
 #pragma unroll
     for (int n = 0; n < 2; ++n) { kk[n][0] = kk[n][1] = kk[n][2] = kk[n][3] = 0.f; qk[n][0] = qk[n][1] = qk[n][2] = qk[n][3] = 0.f; }
@@ -355,11 +361,11 @@ __global__ void __launch_bounds__(KI_THREADS, 3) kda_intra_kernel(const KdaIntra
     for (int ks = 0; ks < 8; ++ks) {
       uint32_t c[4], kr[4], qr[4];
       ldmatrix_x4(c, s_c + 32 * ks);
-      ldmatrix_x4(kr, s_pk + ao + 32 * ks);
-      ldmatrix_x4(qr, s_pq + ao + 32 * ks);
-      if (J < warp - 1) {                                                          // blocks lie between: their totals
+      ldmatrix_x4(kr, s_ki + ao + 32 * ks);
+      ldmatrix_x4(qr, s_qi + ao + 32 * ks);
+      if (J < I - 1) {                                                          // blocks lie between: their totals
         float2 f0 = *reinterpret_cast<const float2*>(&sm.tot[J + 1][16 * ks + 2 * t4]), f1 = *reinterpret_cast<const float2*>(&sm.tot[J + 1][16 * ks + 8 + 2 * t4]);
-        if (J < warp - 2) {
+        if (J < I - 2) {
           const float2 e0 = *reinterpret_cast<const float2*>(&sm.tot[J + 2][16 * ks + 2 * t4]), e1 = *reinterpret_cast<const float2*>(&sm.tot[J + 2][16 * ks + 8 + 2 * t4]);
           f0.x *= e0.x; f0.y *= e0.y; f1.x *= e1.x; f1.y *= e1.y;
         }
@@ -375,12 +381,13 @@ __global__ void __launch_bounds__(KI_THREADS, 3) kda_intra_kernel(const KdaIntra
 #pragma unroll
     for (int n = 0; n < 2; ++n) {
       const int col = 16 * J + 8 * n + 2 * t4;
-      *reinterpret_cast<uint32_t*>(&sm.akh[r0][col]) = pack_h2(b0 * kk[n][0], b0 * kk[n][1]);
-      *reinterpret_cast<uint32_t*>(&sm.akh[r1][col]) = pack_h2(b1 * kk[n][2], b1 * kk[n][3]);
-      *reinterpret_cast<uint32_t*>(rec + OFF_AQK + rec_off(r0, col)) = pack_h2(p.scale * qk[n][0], p.scale * qk[n][1]);
-      *reinterpret_cast<uint32_t*>(rec + OFF_AQK + rec_off(r1, col)) = pack_h2(p.scale * qk[n][2], p.scale * qk[n][3]);
+      *reinterpret_cast<uint32_t*>(&sm.akh[i0][col]) = pack_h2(e0_ * kk[n][0], b0 * kk[n][1]);
+      *reinterpret_cast<uint32_t*>(&sm.akh[i1][col]) = pack_h2(e1_ * kk[n][2], b1 * kk[n][3]);
+      *reinterpret_cast<uint32_t*>(rec + OFF_AQK + rec_off(i0, col)) = pack_h2(p.scale * qk[n][0], p.scale * qk[n][1]);
+      *reinterpret_cast<uint32_t*>(rec + OFF_AQK + rec_off(i1, col)) = pack_h2(p.scale * qk[n][2], p.scale * qk[n][3]);
     }
   }
+  if (warp == 0) { __syncwarp(); asm volatile("bar.arrive 1, 64;" ::: "memory"); }  // block 3's images may change
 
   // ---- the diagonal block: each entry from its level
   {
@@ -424,6 +431,7 @@ __global__ void __launch_bounds__(KI_THREADS, 3) kda_intra_kernel(const KdaIntra
     for (int i = 0; i < 16; ++i) sm.th[warp][i][lane] = __float2half_rn(t[i]);
   }
 
+  if (warp == 3) asm volatile("bar.sync 1, 64;" ::: "memory");
   // ---- state-pass operands: k e^G (shared memory), q e^G scale and k e^{G_C - G} (record)
   {
     const int c = lane & 15;                                                       // this lane's eight channels, in every other row

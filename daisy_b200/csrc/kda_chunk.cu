@@ -112,9 +112,10 @@ __device__ __forceinline__ void st_global16(void* p, uint32_t a, uint32_t b, uin
 // The norms are diagonals of the raw bf16 products, formed the same way.  Blocks meet only through their `suf` images and
 // their totals.  Then the four diagonal blocks of I + A_kk are inverted (fp32, one per warp) and W, U0 come from a blocked
 // forward substitution on the transposed systems, a warp owning 64 of the 256 rows (see below).
-// What bounds it: 22k warp instructions a chunk at 35 % issue, the rest waits for the rows of g and v with 12 warps on an SM
-// (asking L2 for them at the start: 433 -> 425 us at 4 x 8192 x 16).  Lane = (2 tokens, 8 channels), as the fragments want
-// it, costs three shuffles and twice the selects per product: 27k instructions, 937 us at 4 x 16384 x 16 where this takes 840.
+// What bounds it: 22k warp instructions a chunk at some 45 % issue with 12 warps on an SM, latency between.  Rows of k, q and g
+// by asynchronous copies before the first wait instead of register loads where they are used: 447 -> 374 us at 4 x 8192 x 16;
+// the six products between blocks two to a warp instead of three for the last and none for the first: 357.  Lane =
+// (2 tokens, 8 channels), as the fragments want it, costs three shuffles and twice the selects per product: 27k instructions.
 // Why not tcgen05: the version of this kernel that built six image sets in shared memory for 128 x 64 x 128 tcgen05 products
 // was a chain of hand-offs between warp groups (image -> fence -> product -> TMEM load), 20k cycles a chunk with the tensor
 // pipe at 10 %; here everything between two barriers stays inside one warp and three CTAs hide each other's latency.
@@ -350,7 +351,7 @@ __global__ void __launch_bounds__(KI_THREADS, 3) kda_intra_kernel(const KdaIntra
 #pragma unroll 1
   for (int J = warp ? warp - 1 : 0; J >= (warp == 3 ? 1 : 0); --J) {
     const int i0 = 16 * I + g8, i1 = i0 + 8;
-    const float e0_ = sm.beta[i0], e1_ = sm.beta[i1];
+    const float bi0 = sm.beta[i0], bi1 = sm.beta[i1];
     const uint32_t s_ki = smem_u32(sm.pk[I]), s_qi = smem_u32(sm.pq[I]);
     float kk[2][4], qk[2][4];
 #pragma unroll
@@ -381,8 +382,8 @@ __global__ void __launch_bounds__(KI_THREADS, 3) kda_intra_kernel(const KdaIntra
 #pragma unroll
     for (int n = 0; n < 2; ++n) {
       const int col = 16 * J + 8 * n + 2 * t4;
-      *reinterpret_cast<uint32_t*>(&sm.akh[i0][col]) = pack_h2(e0_ * kk[n][0], b0 * kk[n][1]);
-      *reinterpret_cast<uint32_t*>(&sm.akh[i1][col]) = pack_h2(e1_ * kk[n][2], b1 * kk[n][3]);
+      *reinterpret_cast<uint32_t*>(&sm.akh[i0][col]) = pack_h2(bi0 * kk[n][0], bi0 * kk[n][1]);
+      *reinterpret_cast<uint32_t*>(&sm.akh[i1][col]) = pack_h2(bi1 * kk[n][2], bi1 * kk[n][3]);
       *reinterpret_cast<uint32_t*>(rec + OFF_AQK + rec_off(i0, col)) = pack_h2(p.scale * qk[n][0], p.scale * qk[n][1]);
       *reinterpret_cast<uint32_t*>(rec + OFF_AQK + rec_off(i1, col)) = pack_h2(p.scale * qk[n][2], p.scale * qk[n][3]);
     }

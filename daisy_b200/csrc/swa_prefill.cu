@@ -50,7 +50,6 @@ struct PrefillParams {
   __nv_bfloat16* out;
   int64_t o_sb, o_st, o_sh;
   int T, H, B, window;
-  int streams;             // query tiles of 128 rows in an item: 2, or 1 (few items)
   int window_blocks;       // > 0: block-granular window (key tile >= query tile - window_blocks + 1), window = 0
   float scale_log2;
   int* status;
@@ -182,7 +181,7 @@ __device__ __forceinline__ BalancedWalk prefill_walk(int nq, int BH, int window,
 // |logit * log2 e| <= 60 no reference maximum is needed at all (2^x stays far inside fp32 and bf16 range), so the
 // two halves of a row never talk to each other until the epilogue adds their partial row sums.  Each half writes
 // its P over the first 32 columns of its OWN 64 S columns (P_s = two 32-column pieces at S_s + 0 and S_s + 64).
-template <bool QRAW, bool BOUNDED, int NSPLIT>
+template <bool QRAW, bool BOUNDED, int NSPLIT, int STREAMS>
 __global__ void __launch_bounds__(32 * (8 * NSPLIT + 2), 1)
 swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                    const __grid_constant__ CUtensorMap tm_v, const PrefillParams p) {
@@ -197,8 +196,8 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   constexpr int TMA_WARP = 8 * NSPLIT, MMA_WARP = 8 * NSPLIT + 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int T = p.T, window = p.window;
-  const int nq = (T + p.streams * BM - 1) / (p.streams * BM);
-  const BalancedWalk walk = prefill_walk(nq, p.H * p.B, window, p.window_blocks, p.streams);
+  const int nq = (T + STREAMS * BM - 1) / (STREAMS * BM);                  // items of 256 query rows, or of 128 (few items)
+  const BalancedWalk walk = prefill_walk(nq, p.H * p.B, window, p.window_blocks, STREAMS);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < 2; ++s) {
@@ -232,7 +231,7 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       // Q tiles run one item ahead of the K/V stream (double buffer), so the softmax warps can prepare the
       // next item's Q while the current item is still computing.
       auto load_q = [&](int it_item) {
-        const ItemGeom gq = item_geom(it_item, nq, p.H, T, window, p.streams, p.doc_start, p.doc_sb, p.window_blocks);
+        const ItemGeom gq = item_geom(it_item, nq, p.H, T, window, STREAMS, p.doc_start, p.doc_sb, p.window_blocks);
         for (int s = 0; s < 2 && ok; ++s) {
           if (!gq.valid[s]) continue;
           const int qb = qn[s] % NQBUF;
@@ -246,7 +245,7 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       };
       if (walk.at(0) >= 0) load_q(walk.at(0));
       for (int rd = 0, item; (item = walk.at(rd)) >= 0 && ok; ++rd) {
-        const ItemGeom g = item_geom(item, nq, p.H, T, window, p.streams, p.doc_start, p.doc_sb, p.window_blocks);
+        const ItemGeom g = item_geom(item, nq, p.H, T, window, STREAMS, p.doc_start, p.doc_sb, p.window_blocks);
         for (int j = g.jlo; j <= g.jhi && ok; ++j) {
           for (int kv = 0; kv < 2; ++kv, ++n) {
             const int stage = n % NSTAGE;
@@ -286,7 +285,7 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       uint32_t n_q[2] = {0, 0};          // Q tiles consumed so far per stream (phase of q_full)
       bool ok = true;
       for (int rd = 0, item; (item = walk.at(rd)) >= 0 && ok; ++rd) {
-        const ItemGeom g = item_geom(item, nq, p.H, T, window, p.streams, p.doc_start, p.doc_sb, p.window_blocks);
+        const ItemGeom g = item_geom(item, nq, p.H, T, window, STREAMS, p.doc_start, p.doc_sb, p.window_blocks);
         for (int j = g.jlo; j <= g.jhi + 1 && ok; ++j) {
 #pragma unroll
           for (int s = 0; s < 2; ++s) {
@@ -356,7 +355,7 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     bool ok = true;
     bool q_prepared = false;                                       // raw-Q mode: the lower half prepares the stream's Q rows
     for (int rd = 0, item; (item = walk.at(rd)) >= 0 && ok; ++rd) {
-      const ItemGeom g = item_geom(item, nq, p.H, T, window, p.streams, p.doc_start, p.doc_sb, p.window_blocks);
+      const ItemGeom g = item_geom(item, nq, p.H, T, window, STREAMS, p.doc_start, p.doc_sb, p.window_blocks);
       if (!g.valid[s]) continue;
       const int q0 = g.q0[s];
       const int q_row = q0 + row;
@@ -369,7 +368,7 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         q_prepared = false;
         const int item_next = walk.at(rd + 1);
         if (item_next >= 0) {
-          const ItemGeom gn = item_geom(item_next, nq, p.H, T, window, p.streams, p.doc_start, p.doc_sb, p.window_blocks);
+          const ItemGeom gn = item_geom(item_next, nq, p.H, T, window, STREAMS, p.doc_start, p.doc_sb, p.window_blocks);
           next_valid = gn.valid[s];
           q_row_next = gn.q0[s] + row;
         }
@@ -512,7 +511,7 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     bool q_prepared = false;
     auto prepare_q = [&](int qrow) -> bool { return prepare_q_tile(bars, q_tiles, s, row, n_qs, qrow, p, abort_flag); };
     for (int rd = 0, item; (item = walk.at(rd)) >= 0 && ok; ++rd) {
-      const ItemGeom g = item_geom(item, nq, p.H, T, window, p.streams, p.doc_start, p.doc_sb, p.window_blocks);
+      const ItemGeom g = item_geom(item, nq, p.H, T, window, STREAMS, p.doc_start, p.doc_sb, p.window_blocks);
       if (!g.valid[s]) continue;
       const int q0 = g.q0[s];
       const int q_row = q0 + row;
@@ -527,7 +526,7 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       bool next_valid = false;
       int q_row_next = 0;
       if (QRAW && item_next >= 0) {
-        const ItemGeom gn = item_geom(item_next, nq, p.H, T, window, p.streams, p.doc_start, p.doc_sb, p.window_blocks);
+        const ItemGeom gn = item_geom(item_next, nq, p.H, T, window, STREAMS, p.doc_start, p.doc_sb, p.window_blocks);
         next_valid = gn.valid[s];
         q_row_next = gn.q0[s] + row;
       }
@@ -788,10 +787,10 @@ static int ensure_smem_attr() {
   const int dev = daisy_host::device_slot();
   if (dev < 0) return DAISY_ENODEV;
   if (done[dev]) return DAISY_OK;
-  if (cudaFuncSetAttribute(swa_prefill_kernel<false, false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, PREFILL_SMEM) != cudaSuccess) return DAISY_ECUDA;
-  if (cudaFuncSetAttribute(swa_prefill_kernel<false, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, PREFILL_SMEM) != cudaSuccess) return DAISY_ECUDA;
-  if (cudaFuncSetAttribute(swa_prefill_kernel<true, false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, PREFILL_SMEM) != cudaSuccess) return DAISY_ECUDA;
-  if (cudaFuncSetAttribute(swa_prefill_kernel<true, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, PREFILL_SMEM) != cudaSuccess) return DAISY_ECUDA;
+  const auto allow = [](auto kernel) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PREFILL_SMEM) == cudaSuccess; };
+  if (!allow(swa_prefill_kernel<false, false, 1, 2>) || !allow(swa_prefill_kernel<false, true, 2, 2>) || !allow(swa_prefill_kernel<false, true, 2, 1>) ||
+      !allow(swa_prefill_kernel<true, false, 1, 2>) || !allow(swa_prefill_kernel<true, true, 2, 2>) || !allow(swa_prefill_kernel<true, true, 2, 1>))
+    return DAISY_ECUDA;
   if (cudaFuncSetAttribute(umma_selftest_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 1024 + 2 * TILE_BYTES + 64) != cudaSuccess) return DAISY_ECUDA;
   done[dev] = true;
   return DAISY_OK;
@@ -837,25 +836,27 @@ static int launch_attend(const void* q, const void* k, const void* v,
   p.cos = qt ? qt->cos : nullptr; p.sin = qt ? qt->sin : nullptr;
   p.eps = qt ? qt->eps : 0.f; p.q_norm = qt ? qt->norm : 0; p.q_rope = qt ? qt->rope : 0;
   p.lse2 = lse2;
+  const bool raw = qt && (qt->norm || qt->rope);
+  // with RMS-normalised q and k every logit is bounded by scale * D: 2^(logit - reference) cannot overflow
+  const bool bounded = bounded_qk && scale * 1.4426950408889634f * (float)D <= 60.f;
   const int sms = daisy_host::sm_count_cached();
   if (sms <= 0) return DAISY_ENODEV;
   // where one wave holds all 128-row tiles each gets an SM: the second stream pays by sharing K and V, not for latency
   // (1 x 1024 tokens, 6 heads, window 512: 16.7 -> 13.6 us)
   const int64_t tiles = (int64_t)((T + BM - 1) / BM) * H * B;
-  p.streams = tiles <= sms ? 1 : 2;
-  const int64_t items = (int64_t)((T + p.streams * BM - 1) / (p.streams * BM)) * H * B;
+  const bool solo = bounded && tiles <= sms;
+  const int64_t items = solo ? tiles : (int64_t)((T + 2 * BM - 1) / (2 * BM)) * H * B;
   if (items >= (int64_t)1 << 31) return DAISY_EUNSUPPORTED;
   dim3 grid((unsigned)(items < sms ? items : sms), 1, 1);
-  const bool raw = qt && (qt->norm || qt->rope);
-  // with RMS-normalised q and k every logit is bounded by scale * D: 2^(logit - reference) cannot overflow
-  const bool bounded = bounded_qk && scale * 1.4426950408889634f * (float)D <= 60.f;
   cudaStream_t st = (cudaStream_t)stream;
   // bounded logits take the form with two softmax warpgroups per stream, everything else the general form (a failed launch
   // is what the check below reads)
-  if (raw && bounded)  (void)daisy_host::launch_dependent(swa_prefill_kernel<true, true, 2>, dim3(grid), dim3(PREFILL_THREADS_SPLIT), PREFILL_SMEM, st, tq, tk, tv, p);
-  else if (raw)        (void)daisy_host::launch_dependent(swa_prefill_kernel<true, false, 1>, dim3(grid), dim3(PREFILL_THREADS), PREFILL_SMEM, st, tq, tk, tv, p);
-  else if (bounded)    (void)daisy_host::launch_dependent(swa_prefill_kernel<false, true, 2>, dim3(grid), dim3(PREFILL_THREADS_SPLIT), PREFILL_SMEM, st, tq, tk, tv, p);
-  else                 (void)daisy_host::launch_dependent(swa_prefill_kernel<false, false, 1>, dim3(grid), dim3(PREFILL_THREADS), PREFILL_SMEM, st, tq, tk, tv, p);
+  if (raw && solo)          (void)daisy_host::launch_dependent(swa_prefill_kernel<true, true, 2, 1>, dim3(grid), dim3(PREFILL_THREADS_SPLIT), PREFILL_SMEM, st, tq, tk, tv, p);
+  else if (raw && bounded)  (void)daisy_host::launch_dependent(swa_prefill_kernel<true, true, 2, 2>, dim3(grid), dim3(PREFILL_THREADS_SPLIT), PREFILL_SMEM, st, tq, tk, tv, p);
+  else if (raw)             (void)daisy_host::launch_dependent(swa_prefill_kernel<true, false, 1, 2>, dim3(grid), dim3(PREFILL_THREADS), PREFILL_SMEM, st, tq, tk, tv, p);
+  else if (solo)            (void)daisy_host::launch_dependent(swa_prefill_kernel<false, true, 2, 1>, dim3(grid), dim3(PREFILL_THREADS_SPLIT), PREFILL_SMEM, st, tq, tk, tv, p);
+  else if (bounded)         (void)daisy_host::launch_dependent(swa_prefill_kernel<false, true, 2, 2>, dim3(grid), dim3(PREFILL_THREADS_SPLIT), PREFILL_SMEM, st, tq, tk, tv, p);
+  else                      (void)daisy_host::launch_dependent(swa_prefill_kernel<false, false, 1, 2>, dim3(grid), dim3(PREFILL_THREADS), PREFILL_SMEM, st, tq, tk, tv, p);
   DAISY_CHECK_LAUNCH();
   return DAISY_OK;
 }

@@ -11,8 +11,8 @@
 //    Gram products in mma.sync fragments, the blocked solve of (I + A_kk) W = beta k e^G, (I + A_kk) U0 = beta v in register
 //    chains.  Per chunk it writes a record of fp16 operand images (16-byte pieces exchanged so that fragment loads are
 //    bank-conflict free): W^T, scale q e^G, k e^{G_C-G}, A_qk, U0^T, and e^{G_C}.
-//  * kda_state_kernel  -- one CTA per (batch, head), sequential over chunks, on tcgen05: S^T in TMEM, the records through a
-//    three-stage ring.
+//  * kda_state_kernel  -- one CTA per (batch, head), sequential over chunks, on tcgen05: the state in registers, fp16 operands
+//    and sums in TMEM, the records through rings in shared memory.
 // Tensor-core operands are fp16 (10-bit mantissa, every decay factor and operand here is <= O(1)):
 // measured relative error of o against the fp32 token recurrence is ~4e-4, bf16 operands give ~3e-3.
 #include <cuda_fp16.h>
@@ -571,23 +571,26 @@ struct KdaStateParams {
 // S to fp16, 8 products of N = 64, U to fp16, 4 products of N = 128.  Warps 0-7 (thread = half a value column) run it with the
 // state in fp32 registers, scaled while the U products run; TMEM carries only fp16 operands and fresh sums.  Two warps to a
 // scheduler: one warp's conversions alone are twice as long as the products.  q~'s products fill the tensor pipe while U is
-// converted, warps 8-11 write O out of two accumulators, transposed through the record's spent W^T, warp 12 issues, warp 13
-// keeps the ring full.
+// converted, warps 8-11 write O out of two accumulators, transposed through shared memory, warp 12 issues, warps 13 and 14
+// keep the rings full.
 // The same recurrence in mma.sync fragments, 64 value columns to a CTA, took 3700 cycles a chunk (212 products of a warp on
 // one tensor pipe and as many cycles of ldmatrix): 500 us at 4 x 16384 x 16.  With the state in TMEM, scaled there, 2850
-// cycles, 418 us; this form 2560 cycles, 365 us.
-constexpr int KS_NST = 3;
-constexpr int KS_STAGE = (REC_BYTES + 1023) / 1024 * 1024;     // operands start on 1024-byte boundaries
-constexpr int KS_THREADS = 448;
+// cycles, 418 us; with one three-stage ring of whole records, which the output held back, 2560 cycles, 370 us; this form 344.
+// The record comes in two parts with rings of their own: W^T, D and U0^T are spent when U is there, the rest a product later
+constexpr int KS_A = 3, KS_B = 2;
+constexpr int KS_A_BYTES = 33 * 1024, KS_B_BYTES = 40 * 1024;  // operands start on 1024-byte boundaries
+constexpr int KS_AD = KD * KC * 2, KS_AU = KS_AD + KD * 4;     // in part A: W^T, then D and U0^T
+constexpr int KS_OUT = 16 * 1024;                              // output of one chunk, bf16
+constexpr int KS_THREADS = 480;
+static_assert(OFF_KT - OFF_QT == 16384 && OFF_AQK - OFF_QT == 32768 && OFF_D - OFF_QT == KS_B_BYTES && OFF_UT - OFF_D == KD * 4, "q~, k~, A_qk in one copy; D, U0^T in another");
 constexpr int TM_D = 0, TM_S16 = 128, TM_U = 192, TM_U16 = 256, TM_O = 288;      // TMEM columns; D: the state's increment; O: two accumulators of 64
-static_assert(OFF_QT % 1024 == 0 && OFF_KT % 1024 == 0 && OFF_AQK % 1024 == 0, "swizzled operands");
 struct KdaStateBars {
-  uint64_t full[KS_NST], empty[KS_NST];
+  uint64_t a_full[KS_A], a_empty[KS_A], b_full[KS_B], b_empty[KS_B];
   uint64_t s16[2], u, u16, s, o_full[2], o_free[2];
   uint32_t tmem_base;
   int abort_flag;
 };
-constexpr int KS_SMEM = 1024 + KS_NST * KS_STAGE + (int)sizeof(KdaStateBars);
+constexpr int KS_SMEM = 1024 + KS_A * KS_A_BYTES + KS_B * KS_B_BYTES + KS_OUT + (int)sizeof(KdaStateBars);
 static_assert(KS_SMEM <= 232448, "over the 227 KB a CTA may use");
 
 __device__ __forceinline__ void ld_shared16(uint32_t* r, uint32_t addr) {
@@ -596,13 +599,15 @@ __device__ __forceinline__ void ld_shared16(uint32_t* r, uint32_t addr) {
 
 __global__ void __launch_bounds__(KS_THREADS, 1) kda_state_kernel(const KdaStateParams p) {
   extern __shared__ uint8_t kda_smem_raw[];
-  uint8_t* stages = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(kda_smem_raw) + 1023) & ~uintptr_t(1023));
-  KdaStateBars* bars = reinterpret_cast<KdaStateBars*>(stages + KS_NST * KS_STAGE);
+  uint8_t* part_a = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(kda_smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t *part_b = part_a + KS_A * KS_A_BYTES, *out = part_b + KS_B * KS_B_BYTES;
+  KdaStateBars* bars = reinterpret_cast<KdaStateBars*>(out + KS_OUT);
   volatile int* abort_flag = &bars->abort_flag;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < KS_NST; ++i) { mbar_init(&bars->full[i], 1); mbar_init(&bars->empty[i], 12); }      // warps 0-11
+    for (int i = 0; i < KS_A; ++i) { mbar_init(&bars->a_full[i], 1); mbar_init(&bars->a_empty[i], 9); }     // warps 0-7, one commit
+    for (int i = 0; i < KS_B; ++i) { mbar_init(&bars->b_full[i], 1); mbar_init(&bars->b_empty[i], 1); }
     mbar_init(&bars->s16[0], 128); mbar_init(&bars->s16[1], 128); mbar_init(&bars->u, 1); mbar_init(&bars->u16, 256); mbar_init(&bars->s, 1);
     for (int i = 0; i < 2; ++i) { mbar_init(&bars->o_full[i], 1); mbar_init(&bars->o_free[i], 128); }
     bars->abort_flag = 0;
@@ -619,15 +624,27 @@ __global__ void __launch_bounds__(KS_THREADS, 1) kda_state_kernel(const KdaState
   const int c_begin = p.seq_ptr ? p.seq_ptr[bh / p.H] : 0, c_end = p.seq_ptr ? p.seq_ptr[bh / p.H + 1] : p.NC;
   const int n_chunks = c_end - c_begin;
 
+  const uint8_t* recs = p.ws + ((size_t)(b * p.H + h) * p.NC + c_begin) * REC_BYTES;
   if (warp == 13) {
-    // ------------------------------------------------------------ producer: one record a stage
+    // ------------------------------------------------------------ producers: part A, part B
     if (lane == 0) {
-      const uint8_t* recs = p.ws + ((size_t)(b * p.H + h) * p.NC + c_begin) * REC_BYTES;
       for (int c = 0; c < n_chunks; ++c) {
-        const int s = c % KS_NST;
-        if (!mbar_wait(&bars->empty[s], ((c / KS_NST) & 1) ^ 1, abort_flag, p.status, 1)) break;
-        mbar_expect_tx(&bars->full[s], REC_BYTES);
-        bulk_g2s(stages + s * KS_STAGE, recs + (size_t)c * REC_BYTES, REC_BYTES, &bars->full[s]);
+        const int s = c % KS_A;
+        const uint8_t* rec = recs + (size_t)c * REC_BYTES;
+        if (!mbar_wait(&bars->a_empty[s], ((c / KS_A) & 1) ^ 1, abort_flag, p.status, 1)) break;
+        mbar_expect_tx(&bars->a_full[s], KS_AU + KD * KC * 2);
+        bulk_g2s(part_a + s * KS_A_BYTES, rec + OFF_WT, KD * KC * 2, &bars->a_full[s]);
+        bulk_g2s(part_a + s * KS_A_BYTES + KS_AD, rec + OFF_D, KD * 4 + KD * KC * 2, &bars->a_full[s]);
+      }
+    }
+    __syncwarp();
+  } else if (warp == 14) {
+    if (lane == 0) {
+      for (int c = 0; c < n_chunks; ++c) {
+        const int s = c % KS_B;
+        if (!mbar_wait(&bars->b_empty[s], ((c / KS_B) & 1) ^ 1, abort_flag, p.status, 1)) break;
+        mbar_expect_tx(&bars->b_full[s], KS_B_BYTES);
+        bulk_g2s(part_b + s * KS_B_BYTES, recs + (size_t)c * REC_BYTES + OFF_QT, KS_B_BYTES, &bars->b_full[s]);
       }
     }
     __syncwarp();
@@ -635,34 +652,37 @@ __global__ void __launch_bounds__(KS_THREADS, 1) kda_state_kernel(const KdaState
     // ------------------------------------------------------------ MMA issuer
     const uint32_t leader = elect_one() ? 1u : 0u;
     constexpr uint32_t id_u = umma_idesc_f16(128, KC, 0, 1), id_o = umma_idesc_f16(128, KC, 0, 0), id_s = umma_idesc_f16(128, KD, 0, 1);
-    const uint32_t base = smem_u32(stages);
-    const uint64_t wd = umma_desc_sw128(base + OFF_WT, KC * 128, 1024), kd = umma_desc_sw128(base + OFF_KT, KC * 128, 1024);   // depth = rows
-    const uint64_t qd = umma_desc_sw128(base + OFF_QT, 16, 1024), ad = umma_desc_sw128(base + OFF_AQK, 16, 1024);             // depth along the row
+    const uint32_t base = smem_u32(part_b);
+    const uint64_t wd = umma_desc_sw128(smem_u32(part_a), KC * 128, 1024), kd = umma_desc_sw128(base + OFF_KT - OFF_QT, KC * 128, 1024);   // depth = rows
+    const uint64_t qd = umma_desc_sw128(base, 16, 1024), ad = umma_desc_sw128(base + OFF_AQK - OFF_QT, 16, 1024);              // depth along the row
     const uint32_t w_hi = (uint32_t)(wd >> 32), k_hi = (uint32_t)(kd >> 32), q_hi = (uint32_t)(qd >> 32), a_hi = (uint32_t)(ad >> 32);
     for (int c = 0; c < n_chunks; ++c) {
-      const uint32_t s = c % KS_NST, so = s * (KS_STAGE >> 4), o = tmem + TM_O + KC * (c & 1);
-      if (!mbar_wait(&bars->full[s], (c / KS_NST) & 1, abort_flag, p.status, 2)) break;
+      const uint32_t sa = c % KS_A, sb = c % KS_B, ao = sa * (KS_A_BYTES >> 4), bo = sb * (KS_B_BYTES >> 4), o = tmem + TM_O + KC * (c & 1);
+      if (!mbar_wait(&bars->a_full[sa], (c / KS_A) & 1, abort_flag, p.status, 2)) break;
       if (!mbar_wait(&bars->s16[0], c & 1, abort_flag, p.status, 3)) break;
       tc_fence_after();
 #pragma unroll
-      for (int k = 0; k < 4; ++k) umma_ts_lh_p(leader, tmem + TM_U, tmem + TM_S16 + 8 * k, (uint32_t)wd + so + k * (2048 >> 4), w_hi, id_u, k ? 1u : 0u);
+      for (int k = 0; k < 4; ++k) umma_ts_lh_p(leader, tmem + TM_U, tmem + TM_S16 + 8 * k, (uint32_t)wd + ao + k * (2048 >> 4), w_hi, id_u, k ? 1u : 0u);
       if (!mbar_wait(&bars->s16[1], c & 1, abort_flag, p.status, 3)) break;
       tc_fence_after();
 #pragma unroll
-      for (int k = 4; k < 8; ++k) umma_ts_lh_p(leader, tmem + TM_U, tmem + TM_S16 + 8 * k, (uint32_t)wd + so + k * (2048 >> 4), w_hi, id_u, 1u);
+      for (int k = 4; k < 8; ++k) umma_ts_lh_p(leader, tmem + TM_U, tmem + TM_S16 + 8 * k, (uint32_t)wd + ao + k * (2048 >> 4), w_hi, id_u, 1u);
       tc_commit_p(leader, &bars->u);
+      tc_commit_p(leader, &bars->a_empty[sa]);
+      if (!mbar_wait(&bars->b_full[sb], (c / KS_B) & 1, abort_flag, p.status, 2)) break;
       if (!mbar_wait(&bars->o_free[c & 1], ((c >> 1) & 1) ^ 1, abort_flag, p.status, 4)) break;
       tc_fence_after();
 #pragma unroll
-      for (int k = 0; k < 8; ++k) umma_ts_lh_p(leader, o, tmem + TM_S16 + 8 * k, (uint32_t)qd + so + ((k >> 2) * (KC * 128) + (k & 3) * 32) / 16, q_hi, id_o, k ? 1u : 0u);
+      for (int k = 0; k < 8; ++k) umma_ts_lh_p(leader, o, tmem + TM_S16 + 8 * k, (uint32_t)qd + bo + ((k >> 2) * (KC * 128) + (k & 3) * 32) / 16, q_hi, id_o, k ? 1u : 0u);
       if (!mbar_wait(&bars->u16, c & 1, abort_flag, p.status, 5)) break;
       tc_fence_after();
 #pragma unroll
-      for (int k = 0; k < 4; ++k) umma_ts_lh_p(leader, tmem + TM_D, tmem + TM_U16 + 8 * k, (uint32_t)kd + so + k * (2048 >> 4), k_hi, id_s, k ? 1u : 0u);
+      for (int k = 0; k < 4; ++k) umma_ts_lh_p(leader, tmem + TM_D, tmem + TM_U16 + 8 * k, (uint32_t)kd + bo + k * (2048 >> 4), k_hi, id_s, k ? 1u : 0u);
       tc_commit_p(leader, &bars->s);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) umma_ts_lh_p(leader, o, tmem + TM_U16 + 8 * k, (uint32_t)ad + so + k * 2, a_hi, id_o, 1u);
+      for (int k = 0; k < 4; ++k) umma_ts_lh_p(leader, o, tmem + TM_U16 + 8 * k, (uint32_t)ad + bo + k * 2, a_hi, id_o, 1u);
       tc_commit_p(leader, &bars->o_full[c & 1]);
+      tc_commit_p(leader, &bars->b_empty[sb]);
     }
     __syncwarp();
   } else if (warp < 8) {
@@ -699,23 +719,23 @@ __global__ void __launch_bounds__(KS_THREADS, 1) kda_state_kernel(const KdaState
       tc_fence_before();
       mbar_arrive(&bars->s16[half]);
       // beside the U products: scale the state, fetch this column's 32 tokens of U0
-      const int s = c % KS_NST;
-      ok = __all_sync(0xffffffffu, mbar_wait(&bars->full[s], (c / KS_NST) & 1, abort_flag, p.status, 7));
+      const int s = c % KS_A;
+      ok = __all_sync(0xffffffffu, mbar_wait(&bars->a_full[s], (c / KS_A) & 1, abort_flag, p.status, 7));
       if (!ok) break;
-      const uint32_t rec = smem_u32(stages) + s * KS_STAGE;
+      const uint32_t rec = smem_u32(part_a) + s * KS_A_BYTES;
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         uint32_t d[32];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) ld_shared16(d + 4 * i, rec + OFF_D + 256 * half + 128 * j + 16 * i);
+        for (int i = 0; i < 8; ++i) ld_shared16(d + 4 * i, rec + KS_AD + 256 * half + 128 * j + 16 * i);
 #pragma unroll
         for (int i = 0; i < 32; ++i) S[32 * j + i] *= __uint_as_float(d[i]);
       }
       uint32_t u0[16];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) ld_shared16(u0 + 4 * j, rec + OFF_UT + rec_off(v, 32 * half + 8 * j));
+      for (int j = 0; j < 4; ++j) ld_shared16(u0 + 4 * j, rec + KS_AU + rec_off(v, 32 * half + 8 * j));
       __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->empty[s]);
+      if (lane == 0) mbar_arrive(&bars->a_empty[s]);
       ok = __all_sync(0xffffffffu, mbar_wait(&bars->u, c & 1, abort_flag, p.status, 8));
       if (!ok) break;
       tc_fence_after();
@@ -745,7 +765,6 @@ __global__ void __launch_bounds__(KS_THREADS, 1) kda_state_kernel(const KdaState
     const uint32_t t = tmem + ((uint32_t)(32 * w) << 16) + TM_O;
     const int vr = 8 * ((lane & 7) >> 1) + 2 * (lane >> 3) + (lane & 1);           // the row this lane addresses
     for (int c = 0; c < n_chunks; ++c) {
-      const int s = c % KS_NST;
       if (!__all_sync(0xffffffffu, mbar_wait(&bars->o_full[c & 1], (c >> 1) & 1, abort_flag, p.status, 10))) break;
       tc_fence_after();
       uint32_t x[64];
@@ -762,7 +781,7 @@ __global__ void __launch_bounds__(KS_THREADS, 1) kda_state_kernel(const KdaState
 #pragma unroll
         for (int i = 0; i < KC; ++i) if (i < rows) o[i * ts] = __uint_as_float(x[i]);
       } else {
-        const uint32_t stg = smem_u32(stages) + s * KS_STAGE + OFF_WT + w * 4096;  // the products that read it are done
+        const uint32_t stg = smem_u32(out) + w * 4096;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const uint32_t* xx = x + 8 * j;
@@ -780,10 +799,7 @@ __global__ void __launch_bounds__(KS_THREADS, 1) kda_state_kernel(const KdaState
           const int tok = 8 * j + (lane >> 2);
           if (tok < rows) st_global16(o + tok * ts, x[4 * j], x[4 * j + 1], x[4 * j + 2], x[4 * j + 3]);
         }
-        fence_proxy_async();                                                       // the next record lands where this was staged
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->empty[s]);
     }
   }
 

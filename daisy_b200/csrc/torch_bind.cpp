@@ -9,6 +9,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
+#include <functional>
 #include <list>
 #include <mutex>
 
@@ -516,11 +517,23 @@ Tensor f32c(const Tensor& t, const char* name) {
 
 // Tables of a packed batch on the device (see kda_varlen_tables); tok only if asked for.
 struct Packed { Tensor chunks, ptr, tok; int64_t n_chunks = 0, n_seq = 0, total = 0; };
-Packed pack_tables(const py::object& cu_seqlens, c10::Device dev, int64_t chunk, bool want_tok) {
+// `meanwhile(n_seq)` runs while lengths that lie on the device are on their way.
+Packed pack_tables(const py::object& cu_seqlens, c10::Device dev, int64_t chunk, bool want_tok, const std::function<void(int64_t)>& meanwhile = {}) {
   std::vector<int64_t> cu;
   if (THPVariable_Check(cu_seqlens.ptr())) {
-    Tensor c = THPVariable_Unpack(cu_seqlens.ptr()).to(at::kCPU, at::kLong).contiguous();
-    cu.assign(c.data_ptr<int64_t>(), c.data_ptr<int64_t>() + c.numel());
+    Tensor t = THPVariable_Unpack(cu_seqlens.ptr());
+    if (t.is_cuda() && t.dim() == 1 && t.numel() > 1 && (t.scalar_type() == at::kInt || t.scalar_type() == at::kLong)) {
+      c10::cuda::CUDAGuard guard(t.device());
+      Tensor c = at::empty(t.sizes(), at::TensorOptions().dtype(t.scalar_type()).pinned_memory(true));
+      c.copy_(t, /*non_blocking=*/true);
+      if (meanwhile) meanwhile(t.numel() - 1);
+      at::cuda::getCurrentCUDAStream(t.get_device()).synchronize();
+      if (t.scalar_type() == at::kInt) cu.assign(c.data_ptr<int32_t>(), c.data_ptr<int32_t>() + c.numel());
+      else cu.assign(c.data_ptr<int64_t>(), c.data_ptr<int64_t>() + c.numel());
+    } else {
+      Tensor c = t.to(at::kCPU, at::kLong).contiguous();
+      cu.assign(c.data_ptr<int64_t>(), c.data_ptr<int64_t>() + c.numel());
+    }
   } else {
     for (auto item : cu_seqlens) cu.push_back(py::cast<int64_t>(py::int_(py::reinterpret_borrow<py::object>(item))));
   }
@@ -551,9 +564,20 @@ Packed pack_tables(const py::object& cu_seqlens, c10::Device dev, int64_t chunk,
   return p;
 }
 
+// What a chunked call writes; made ahead of the call where there is a wait to fill.
+struct KdaOut { Tensor o, ws; OptTensor hT; };
+KdaOut kda_out(const Tensor& q, const Tensor& v, int64_t n, int64_t ws_bytes, bool want_state, bool out_fp32) {
+  const int64_t B = q.size(0), T = q.size(1), H = q.size(2), K = q.size(3), V = v.size(3);
+  KdaOut r;
+  r.o = at::empty({B, T, H, V}, q.options().dtype(out_fp32 ? at::kFloat : at::kBFloat16));
+  if (want_state) r.hT = at::empty({n, H, K, V}, q.options().dtype(at::kFloat));
+  r.ws = at::empty({std::max<int64_t>(ws_bytes, 16)}, q.options().dtype(at::kByte));
+  return r;
+}
+
 // chunked forward, dense ([B,T,H,K], packed == nullptr) or packed ([1,T_total,H,K])
 std::pair<Tensor, OptTensor> kda_chunk(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g_, const Tensor& beta_, std::optional<double> scale,
-                                       const OptTensor& h0_, bool want_state, bool l2norm, bool out_fp32, const Packed* pk) {
+                                       const OptTensor& h0_, bool want_state, bool l2norm, bool out_fp32, const Packed* pk, const KdaOut* made = nullptr) {
   const Tensor* in[] = {&q, &k, &v};
   const char* names[] = {"q", "k", "v"};
   for (int i = 0; i < 3; ++i) { req(*in[i], names[i]); TORCH_CHECK_VALUE(in[i]->is_contiguous(), names[i], " must be contiguous"); }
@@ -567,16 +591,15 @@ std::pair<Tensor, OptTensor> kda_chunk(const Tensor& q, const Tensor& k, const T
     TORCH_CHECK_VALUE(!pk || (h0.dim() == 4 && h0.size(0) == n && h0.size(1) == H && h0.size(2) == K && h0.size(3) == V), "initial_state must be [", n, ", ", H, ", ",
                       K, ", ", V, "]");
   }
-  Tensor o = at::empty({B, T, H, V}, q.options().dtype(out_fp32 ? at::kFloat : at::kBFloat16));
-  OptTensor hT;
-  if (want_state) hT = at::empty({n, H, K, V}, q.options().dtype(at::kFloat));
+  const int64_t need = pk ? (int64_t)daisy_b200_kda_varlen_workspace_bytes((int)pk->n_chunks, (int)H, (int)K, (int)V)
+                          : (int64_t)daisy_b200_kda_workspace_bytes((int)B, (int)T, (int)H, (int)K, (int)V);
+  const KdaOut r = made && made->ws.defined() && made->ws.numel() >= need ? *made : kda_out(q, v, n, need, want_state, out_fp32);
+  const Tensor &o = r.o, &ws = r.ws;
+  const OptTensor& hT = r.hT;
   if (pk && (T == 0 || pk->n_chunks == 0)) {
     if (want_state) { if (h0.defined()) hT->copy_(h0); else hT->zero_(); }
     return {o, hT};
   }
-  const int64_t need = pk ? (int64_t)daisy_b200_kda_varlen_workspace_bytes((int)pk->n_chunks, (int)H, (int)K, (int)V)
-                          : (int64_t)daisy_b200_kda_workspace_bytes((int)B, (int)T, (int)H, (int)K, (int)V);
-  Tensor ws = at::empty({std::max<int64_t>(need, 16)}, q.options().dtype(at::kByte));
   const unsigned flags = (l2norm ? DAISY_KDA_L2NORM_QK : 0) | (out_fp32 ? DAISY_KDA_OUT_FP32 : 0);
   const float sc = scale.has_value() ? (float)*scale : 0.f;
   const float* h0p = h0.defined() ? h0.data_ptr<float>() : nullptr;
@@ -626,8 +649,13 @@ std::pair<Tensor, OptTensor> chunk_kda(const Tensor& q_, const Tensor& k_, const
   OptTensor h0;
   if (h0_.has_value()) h0 = h0_->to(at::kFloat).contiguous();
   if (!cu_seqlens.is_none()) {
-    Packed p = pack_tables(cu_seqlens, q.device(), 64, false);
-    return kda_chunk(q, k, v, g, beta, scale, h0, want_state, l2norm, out_fp32, &p);
+    KdaOut made;
+    Packed p = pack_tables(cu_seqlens, q.device(), 64, false, [&](int64_t n) {
+      if (q.dim() != 4 || v.dim() != 4 || q.size(0) != 1) return;                          // the call itself reports what is wrong
+      const int64_t most = q.size(1) / 64 + n;                                             // every sequence may end in a short chunk
+      made = kda_out(q, v, n, (int64_t)daisy_b200_kda_varlen_workspace_bytes((int)most, (int)q.size(2), (int)q.size(3), (int)v.size(3)), want_state, out_fp32);
+    });
+    return kda_chunk(q, k, v, g, beta, scale, h0, want_state, l2norm, out_fp32, &p, &made);
   }
   return q.size(1) <= RECURRENT_MAX_T ? kda_recurrent(q, k, v, g, beta, scale, h0, want_state, l2norm, out_fp32, false)
                                       : kda_chunk(q, k, v, g, beta, scale, h0, want_state, l2norm, out_fp32, nullptr);

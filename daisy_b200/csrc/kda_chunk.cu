@@ -114,7 +114,8 @@ __device__ __forceinline__ void st_global16(void* p, uint32_t a, uint32_t b, uin
 // forward substitution on the transposed systems, a warp owning 64 of the 256 rows (see below).
 // What bounds it: 22k warp instructions a chunk at some 45 % issue with 12 warps on an SM, latency between.  Rows of k, q and g
 // by asynchronous copies before the first wait instead of register loads where they are used: 447 -> 374 us at 4 x 8192 x 16;
-// the six products between blocks two to a warp instead of three for the last and none for the first: 357.  Lane =
+// the six products between blocks two to a warp instead of three for the last and none for the first: 357; the halves and the
+// solve's tiles rolled, which ended the spills and most waits for instructions: 326.  Lane =
 // (2 tokens, 8 channels), as the fragments want it, costs three shuffles and twice the selects per product: 27k instructions.
 // Why not tcgen05: the version of this kernel that built six image sets in shared memory for 128 x 64 x 128 tcgen05 products
 // was a chain of hand-offs between warp groups (image -> fence -> product -> TMEM load), 20k cycles a chunk with the tensor
@@ -248,8 +249,8 @@ __global__ void __launch_bounds__(KI_THREADS, 3) kda_intra_kernel(const KdaIntra
   l8[0] = l8[1] = l8[2] = l8[3] = 0.f;
   uint32_t sh[16];                                                                 // k suf of the first 64 channels
   const uint32_t s_lv = s_suf + ((lane & 8) ? 16 * KI_LV : 0) + (lane & 7) * KI_LV + 16 * (lane >> 4);   // level images: k rows, then q rows
-#pragma unroll
-  for (int hf = 0; hf < 2; ++hf) {
+#pragma unroll 1
+  for (int hf = 0; hf < 2; ++hf) {                                                 // (rolled: the instruction cache bounds three CTAs too)
     uint64_t pre[16], suf[16];                                                     // fp32 pairs: the lane's two channels
     uint32_t kh[16], qh[16];                                                       // normalised, fp16 pairs
     {
@@ -486,60 +487,63 @@ __global__ void __launch_bounds__(KI_THREADS, 3) kda_intra_kernel(const KdaIntra
   //      16-token block columns I, so there is nothing to exchange between warps:
   //          Z_I = R_I - sum_{J<I} Z_J A_IJ^T,   then   Z_I <- Z_I T_II^T
   //      with every product an m16n8k16 tile whose fp32 accumulators, rounded to fp16, are the A fragment of the products
-  //      that follow.  The four row tiles of a warp are independent chains issued side by side.
+  //      that follow.  Two row tiles of a warp are independent chains issued side by side, twice (all four unrolled were more
+  //      registers and more code than they hid: 336 -> 326 us).
   {
     const bool is_w = warp < 2;
     uint8_t* dst = rec + (is_w ? OFF_WT : OFF_UT);
-    const int c0 = 64 * (warp & 1);                                                // first row (channel or value column)
-    const uint32_t src = smem_u32(is_w ? sm.pk : sm.pq) + ((lane & 7) + 8 * (lane >> 4)) * KI_LD + 2 * c0 + 16 * ((lane >> 3) & 1);
-    uint32_t zf[4][3][4];                                                          // Z_J as fp16 A fragments: [row tile][J][4]
+#pragma unroll 1
+    for (int c0 = 64 * (warp & 1), end = c0 + 64; c0 < end; c0 += 32) {               // first row (channel or value column) of two tiles
+      const uint32_t src = smem_u32(is_w ? sm.pk : sm.pq) + ((lane & 7) + 8 * (lane >> 4)) * KI_LD + 2 * c0 + 16 * ((lane >> 3) & 1);
+      uint32_t zf[2][3][4];                                                          // Z_J as fp16 A fragments: [row tile][J][4]
 #pragma unroll
-    for (int I = 0; I < 4; ++I) {
-      float acc[4][2][4];
+      for (int I = 0; I < 4; ++I) {
+        float acc[2][2][4];
 #pragma unroll
-      for (int m = 0; m < 4; ++m)
+        for (int m = 0; m < 2; ++m)
 #pragma unroll
-        for (int n = 0; n < 2; ++n) { acc[m][n][0] = acc[m][n][1] = acc[m][n][2] = acc[m][n][3] = 0.f; }
+          for (int n = 0; n < 2; ++n) { acc[m][n][0] = acc[m][n][1] = acc[m][n][2] = acc[m][n][3] = 0.f; }
 #pragma unroll
-      for (int J = 0; J < I; ++J) {
+        for (int J = 0; J < I; ++J) {
+#pragma unroll
+          for (int n = 0; n < 2; ++n) {
+            const __half* arow = &sm.akh[I * 16 + n * 8 + g8][J * 16 + 2 * t4];
+            const uint32_t w0 = *reinterpret_cast<const uint32_t*>(arow), w1 = *reinterpret_cast<const uint32_t*>(arow + 8);
+#pragma unroll
+            for (int m = 0; m < 2; ++m) mma_f16(acc[m][n], zf[m][J], w0, w1);
+          }
+        }
+        uint32_t tw[2][2];
 #pragma unroll
         for (int n = 0; n < 2; ++n) {
-          const __half* arow = &sm.akh[I * 16 + n * 8 + g8][J * 16 + 2 * t4];
-          const uint32_t w0 = *reinterpret_cast<const uint32_t*>(arow), w1 = *reinterpret_cast<const uint32_t*>(arow + 8);
-#pragma unroll
-          for (int m = 0; m < 4; ++m) mma_f16(acc[m][n], zf[m][J], w0, w1);
+          const __half* trow = &sm.th[I][n * 8 + g8][2 * t4];
+          tw[n][0] = *reinterpret_cast<const uint32_t*>(trow); tw[n][1] = *reinterpret_cast<const uint32_t*>(trow + 8);
         }
-      }
-      uint32_t tw[2][2];
+        const float2 bt0 = *reinterpret_cast<const float2*>(&sm.beta[I * 16 + 2 * t4]), bt1 = *reinterpret_cast<const float2*>(&sm.beta[I * 16 + 8 + 2 * t4]);
 #pragma unroll
-      for (int n = 0; n < 2; ++n) {
-        const __half* trow = &sm.th[I][n * 8 + g8][2 * t4];
-        tw[n][0] = *reinterpret_cast<const uint32_t*>(trow); tw[n][1] = *reinterpret_cast<const uint32_t*>(trow + 8);
-      }
-      const float2 bt0 = *reinterpret_cast<const float2*>(&sm.beta[I * 16 + 2 * t4]), bt1 = *reinterpret_cast<const float2*>(&sm.beta[I * 16 + 8 + 2 * t4]);
+        for (int m = 0; m < 2; ++m) {
+          // right-hand side: tokens 16 I .. + 15 x rows c0 + 16 m .. + 15, transposed: register i = (tokens 8 (i >> 1) + 2 t4 (+1),
+          // row 8 (i & 1) + g8)
+          uint32_t rr[4];
+          ldmatrix_x4_t(rr, src + I * (16 * KI_LD) + 32 * m);
+          uint32_t a[4];
 #pragma unroll
-      for (int m = 0; m < 4; ++m) {
-        // right-hand side: tokens 16 I .. + 15 x rows c0 + 16 m .. + 15, transposed: register i = (tokens 8 (i >> 1) + 2 t4 (+1),
-        // row 8 (i & 1) + g8)
-        uint32_t rr[4];
-        ldmatrix_x4_t(rr, src + I * (16 * KI_LD) + 32 * m);
-        uint32_t a[4];
+          for (int i = 0; i < 4; ++i) {
+            const int n = i >> 1, hi = i & 1;
+            const float2 r = is_w ? unpack_h2(rr[i]) : make_float2(bf16_lo(rr[i]), bf16_hi(rr[i]));
+            const float2 bt = n ? bt1 : bt0;
+            a[2 * n + hi] = pack_h2(r.x * bt.x - acc[m][n][2 * hi], r.y * bt.y - acc[m][n][2 * hi + 1]);
+          }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int n = i >> 1, hi = i & 1;
-          const float2 r = is_w ? unpack_h2(rr[i]) : make_float2(bf16_lo(rr[i]), bf16_hi(rr[i]));
-          const float2 bt = n ? bt1 : bt0;
-          a[2 * n + hi] = pack_h2(r.x * bt.x - acc[m][n][2 * hi], r.y * bt.y - acc[m][n][2 * hi + 1]);
-        }
-#pragma unroll
-        for (int n = 0; n < 2; ++n) {
-          float z[4] = {0.f, 0.f, 0.f, 0.f};
-          mma_f16(z, a, tw[n][0], tw[n][1]);
-          const uint32_t zl = pack_h2(z[0], z[1]), zh = pack_h2(z[2], z[3]);
-          if (I < 3) { zf[m][I][2 * n] = zl; zf[m][I][2 * n + 1] = zh; }
-          const int cr = c0 + 16 * m + g8;
-          *reinterpret_cast<uint32_t*>(dst + rec_off(cr, I * 16 + n * 8 + 2 * t4)) = zl;
-          *reinterpret_cast<uint32_t*>(dst + rec_off(cr + 8, I * 16 + n * 8 + 2 * t4)) = zh;
+          for (int n = 0; n < 2; ++n) {
+            float z[4] = {0.f, 0.f, 0.f, 0.f};
+            mma_f16(z, a, tw[n][0], tw[n][1]);
+            const uint32_t zl = pack_h2(z[0], z[1]), zh = pack_h2(z[2], z[3]);
+            if (I < 3) { zf[m][I][2 * n] = zl; zf[m][I][2 * n + 1] = zh; }
+            const int cr = c0 + 16 * m + g8;
+            *reinterpret_cast<uint32_t*>(dst + rec_off(cr, I * 16 + n * 8 + 2 * t4)) = zl;
+            *reinterpret_cast<uint32_t*>(dst + rec_off(cr + 8, I * 16 + n * 8 + 2 * t4)) = zh;
+          }
         }
       }
     }

@@ -108,6 +108,23 @@ def test_gemm_small_tiles(M, N, K):
     assert_close_bf16(c, x.float().cpu() @ w.float().cpu().t(), f"gemm {M}x{N}x{K}")
 
 
+@pytest.mark.parametrize("n,M,N,K", [(2, 70, 128, 64), (3, 300, 256, 128), (3, 1100, 384, 192), (2, 2500, 640, 256), (3, 5000, 768, 1024)])
+def test_gemm_group_matches_single_products(n, M, N, K):
+    """Products of one shape in one launch: narrow tiles, 128 x 128 tiles, pairs; tiles of different products side by side."""
+    import ctypes
+    from daisy_b200 import _lib, ops
+    x = [bf16_randn(M, K, seed=M + i) for i in range(n)]
+    w = [bf16_randn(N, K, seed=N + i) * (K ** -0.5) for i in range(n)]
+    c = [torch.full((M, N), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(n)]
+    ptrs = lambda ts: (ctypes.c_void_p * n)(*[t.data_ptr() for t in ts])
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    rc = _lib.lib().daisy_b200_gemm_nt_group(ptrs(x), K, ptrs(w), K, ptrs(c), N, n, M, N, K, status.data_ptr(),
+                                             torch.cuda.current_stream().cuda_stream)
+    assert rc == 0 and status.item() == 0
+    for i in range(n):
+        assert_close_bf16(c[i], x[i].float().cpu() @ w[i].float().cpu().t(), f"product {i} of {n}")
+
+
 @pytest.mark.parametrize("B,T,H,dim", [(1, 1, 1, 64), (3, 43, 2, 320), (1, 128, 3, 832), (2, 200, 6, 768)])
 @pytest.mark.parametrize("f16", [False, True])
 def test_qkv_gemm_small_tiles_ring(B, T, H, dim, f16):

@@ -38,6 +38,16 @@ void req(const Tensor& t, const char* name, at::ScalarType dt = at::kBFloat16) {
   TORCH_CHECK_VALUE(t.dim() > 0 && t.stride(-1) == 1, name, " must be contiguous in its last dimension");
 }
 
+// A decode step's vectors: x beside the state or ring it goes with, and the caller's buffer for the result.
+void req_step(const Tensor& x, const OptTensor& out, const Tensor& state, int64_t B, int64_t dim) {
+  TORCH_CHECK_VALUE(x.is_cuda(), "x must be a CUDA tensor (daisy_b200 has no CPU path)");
+  TORCH_CHECK_VALUE(x.device() == state.device(), "x is on ", x.device(), ", the states are on ", state.device());
+  TORCH_CHECK_VALUE(x.dim() > 0 && x.numel() == B * dim && x.size(-1) == dim, "x must be [", B, ", 1, ", dim, "]");
+  if (!out.has_value()) return;
+  TORCH_CHECK_VALUE(out->device() == state.device() && out->scalar_type() == at::kBFloat16 && out->is_contiguous() && out->numel() == B * dim,
+                    "out must be a contiguous bf16 [", B, ", 1, ", dim, "] on ", state.device());
+}
+
 // ------------------------------------------------------------------ per-device status word, per-stream workspaces
 constexpr int MAX_DEV = 64;
 std::mutex g_mutex;
@@ -112,8 +122,7 @@ Tensor token_step(const Tensor& x_, const std::vector<Tensor>& weights, const st
   const bool f16 = k.scalar_type() == at::kHalf;
   req(k, "kcache", f16 ? at::kHalf : at::kBFloat16);
   req(v, "vcache", k.scalar_type());
-  TORCH_CHECK_VALUE(x_.is_cuda(), "x must be a CUDA tensor (daisy_b200 has no CPU path)");
-  TORCH_CHECK_VALUE(x_.numel() == B * dim && x_.size(-1) == dim, "x must be [", B, ", 1, ", dim, "]");
+  req_step(x_, out, k, B, dim);
   c10::cuda::CUDAGuard guard(k.device());
   Tensor x = x_.scalar_type() == at::kBFloat16 ? x_ : x_.to(at::kBFloat16);
   int64_t x_sb = dim;
@@ -476,7 +485,7 @@ Tensor kda_token_step(const Tensor& x_, const std::vector<Tensor>& w, const OptT
                       bool silu, double eps, const OptTensor& out, const OptTensor& workspace) {
   TORCH_CHECK_VALUE(w.size() == 9 && conv_w.size() == 3 && conv_b.size() == 3 && conv_s.size() == 3, "nine weights, three convolutions");
   const int64_t B = state.size(0), H = state.size(1), dim = H * 128;
-  TORCH_CHECK_VALUE(x_.is_cuda() && x_.numel() == B * dim && x_.size(-1) == dim, "x must be a CUDA tensor [", B, ", 1, ", dim, "]");
+  req_step(x_, out, state, B, dim);
   c10::cuda::CUDAGuard guard(x_.device());
   Tensor x = x_.to(at::kBFloat16).reshape({B, dim}).contiguous();
   for (const Tensor& t : w) { req(t, "weight"); TORCH_CHECK_VALUE(t.is_contiguous(), "weights must be contiguous"); }

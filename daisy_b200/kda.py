@@ -310,16 +310,25 @@ class B200KimiLinearSelfAttention(torch.nn.Module):
         if one_launch:
             return
         self._graph = torch.cuda.CUDAGraph()
+        self._gstates = (self._recurrent_state, *(self._conv_state or ()))     # what the graph updates: kept as long as it is
         with torch.cuda.graph(self._graph):
             self._gy = self._forward_core(self._gx, None, None, None, use_cache=True)
         restore()
 
     @torch.inference_mode()
     def step_graph(self, x):
-        """``step`` into the fixed buffer: ``x [batch, 1, dim]`` -> ``y`` (overwritten by the next call)."""
+        """``step`` into the fixed buffer: ``x [batch, 1, dim]`` -> ``y`` (overwritten by the next call).  ``x`` may lie on the
+        host or broadcast to that shape.  The states of the layer must be there: one launch takes them where they are (another
+        ``prefill`` of the same batch may have made them), a graph only those ``capture_step`` saw."""
         if self._graph is None:
-            self._token_step(x, self._gy, self._gws)
+            if x.shape != self._gx.shape or x.device != self._gx.device:
+                x = self._gx.copy_(x)
+            if self._token_step(x, self._gy, self._gws) is None:
+                raise RuntimeError("step_graph: the cached states are gone or of another batch size (prefill, then capture_step)")
         else:
+            now = (self._recurrent_state, *(self._conv_state or ()))
+            if len(now) != len(self._gstates) or any(a is None or a.data_ptr() != b.data_ptr() for a, b in zip(now, self._gstates)):
+                raise RuntimeError("step_graph: the cached states are not the ones capture_step recorded; call it again")
             self._gx.copy_(x)
             self._graph.replay()
         self._seen += 1

@@ -248,6 +248,48 @@ def test_layer_step_graph_matches_eager():
     assert m._seen == T0 + n
 
 
+@pytest.mark.parametrize("H", [2, 17])
+def test_layer_step_graph_inputs_and_states(H):
+    """``step_graph`` in both its forms (one launch; a captured graph above 2048 channels): inputs on the host and inputs that
+    broadcast are taken as ``copy_`` takes them, others raise, and so do states that are gone or not the ones it steps; the
+    one-launch form goes on from the states of another prefill."""
+    m, dim = _layer(128 * H, H, seed=4), 128 * H
+    B, T0 = 2, 40
+    x = torch.randn(B, T0 + 1, dim, device="cuda").bfloat16()
+    x[:, T0:] = x[:1, T0:]                                                 # the same token in each row
+    forms = (x[:, T0:], x[:, T0:].cpu(), x[:1, T0:], x[0, T0:], x[:, T0:].float())
+    with torch.inference_mode():
+        m.prefill(x[:, :T0])
+        ref = m.step(x[:, T0:])[0].clone()
+        m.reset_history()
+        m.prefill(x[:, :T0])
+        m.capture_step(batch=B)
+        assert (m._graph is not None) == (H == 17)
+        first = [m._recurrent_state.clone()] + [c.clone() for c in m._conv_state]
+        for form in forms:
+            for a, b in zip((m._recurrent_state, *m._conv_state), first):
+                a.copy_(b)
+            assert torch.equal(m.step_graph(form), ref), form.shape
+        seen = m._seen
+        for bad in (x[:, :2], x[:, T0:, :-1], torch.cat([x, x])[:, T0:]):
+            with pytest.raises((RuntimeError, ValueError)):
+                m.step_graph(bad)
+        assert m._seen == seen
+        m.reset_history()
+        with pytest.raises(RuntimeError, match="states"):
+            m.step_graph(x[:, T0:])
+        m.prefill(x[:1, :T0])                                              # one row, captured for two
+        with pytest.raises(RuntimeError, match="states"):
+            m.step_graph(x[:, T0:])
+        m.reset_history()
+        m.prefill(x[:, :T0])
+        if H == 17:
+            with pytest.raises(RuntimeError, match="states"):
+                m.step_graph(x[:, T0:])
+        else:
+            assert torch.equal(m.step_graph(x[:, T0:]), ref)
+
+
 # ------------------------------------------------------------------------------------ packed variable-length batches
 @pytest.mark.parametrize("W", [4, 2])
 @pytest.mark.parametrize("cu", [[0, 40], [0, 1, 2, 3, 4, 40], [0, 2, 2, 35, 67, 200], [0, 31, 32, 33, 96, 97]])

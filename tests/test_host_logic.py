@@ -190,3 +190,17 @@ def test_accounting_matches_the_oracle_formulas():
     assert a.kda_bytes_per_token_head() == kda.kda_bytes_per_token_head() == 1540
     assert a.kda_flops_per_token_head() == kda.kda_flops_per_token_head()
     assert a.FP32_EPS == swa.FP32_EPS
+
+
+def test_kda_step_graph_without_states_raises():
+    """``step_graph`` never hands out the last token's output: it raises where there are no states to step, and where ``x``
+    does not fill the buffer that ``capture_step`` made."""
+    from daisy_b200 import B200KimiLinearSelfAttention
+    m = B200KimiLinearSelfAttention(256, 2, 64, 128)
+    m._graph, m._gws = None, None                                   # as capture_step leaves a layer of the single-launch form
+    m._gx, m._gy = torch.zeros(2, 1, 256, dtype=torch.bfloat16), torch.zeros(2, 1, 256, dtype=torch.bfloat16)
+    m.reset_history()
+    for x in (torch.zeros(2, 1, 256), torch.zeros(1, 1, 256), torch.zeros(3, 1, 256), torch.zeros(2, 2, 256)):
+        with pytest.raises(RuntimeError):
+            m.step_graph(x)
+    assert m._seen == 0

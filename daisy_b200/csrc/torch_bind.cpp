@@ -381,8 +381,7 @@ struct AttnFunction : public torch::autograd::Function<AttnFunction> {
     Tensor ve2, g32;
     if (ve.has_value()) {
       req(*ve, "ve");
-      ve2 = ve->reshape({M, dim});
-      if (!ve2.is_contiguous()) ve2 = ve2.contiguous();
+      ve2 = ve->reshape({M, dim}).contiguous();
       g32 = logit->to(at::kFloat).reshape({1});
     }
     const Saved at_(M, H, ve2.defined());
@@ -401,7 +400,9 @@ struct AttnFunction : public torch::autograd::Function<AttnFunction> {
           "daisy_b200_swa_attend_lse");                                                    // q, k are RMS-normalised
     Tensor y = at::empty({B, T, dim}, x.options());
     check(daisy_b200_gemm_nt(p + at_.o, dim, (char*)w.data_ptr() + 3 * dim * dim * 2, dim, y.data_ptr(), dim, (int)M, (int)dim, (int)dim, status, st), "daisy_b200_gemm_nt");
-    ctx->save_for_backward({x2, w, buf, cos, sin, ve2, g32, doc_start.has_value() ? *doc_start : Tensor()});
+    // the inputs themselves, not views of them made here: below the autograd keys a view has a version counter of its own, and
+    // a change in place between forward and backward would go unnoticed
+    ctx->save_for_backward({x, w, buf, cos, sin, ve.value_or(Tensor()), ve.has_value() ? *logit : Tensor(), doc_start.value_or(Tensor())});
     ctx->saved_data["dims"] = std::vector<int64_t>{B, T, H, window, in_blocks ? 1 : 0};
     ctx->saved_data["scale"] = scale;
     if (ve.has_value()) {
@@ -414,9 +415,12 @@ struct AttnFunction : public torch::autograd::Function<AttnFunction> {
   static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
     at::AutoDispatchBelowADInplaceOrView guard;
     auto s = ctx->get_saved_variables();
-    const Tensor &x2 = s[0], &w = s[1], &buf = s[2], &cos = s[3], &sin = s[4], &ve2 = s[5], &g32 = s[6], &doc = s[7];
+    const Tensor &w = s[1], &buf = s[2], &cos = s[3], &sin = s[4], &doc = s[7];
     auto d = ctx->saved_data["dims"].toIntVector();
     const int64_t B = d[0], T = d[1], H = d[2], window = d[3], dim = H * 128, M = B * T;
+    const Tensor x2 = rows_of(s[0], dim);
+    Tensor ve2, g32;
+    if (s[5].defined()) { ve2 = s[5].reshape({M, dim}).contiguous(); g32 = s[6].to(at::kFloat).reshape({1}); }
     const float scale = (float)ctx->saved_data["scale"].toDouble();
     const bool need_x = ctx->needs_input_grad(0), need_w = ctx->needs_input_grad(1);
     Tensor dy = grads[0].to(at::kBFloat16).reshape({M, dim});

@@ -202,3 +202,35 @@ def test_gated_layer_backward_ragged_rows(B, T, H):
     (yo * cot.cpu()).sum().backward()
     for got, ref, n in ((x.grad, xo.grad, "dx"), (ve.grad, vo.grad, "d ve"), (m.qkvo_w.grad, wo.grad, "dw")):
         assert_close_bf16(got, ref, n, max_tol=4e-2, mean_tol=4e-3)
+
+
+@pytest.mark.parametrize("changed", ["x", "ve", "g_ve", "qkvo_w", "doc_start", None])
+def test_in_place_change_before_backward_raises(changed):
+    """What the backward reads again is saved as it was handed in: an in-place change between forward and backward is
+    refused, and without one the gradients do not depend on saved-tensor hooks that move what was saved."""
+    from daisy_b200 import B200CausalSelfAttention, WindowMask
+    os.environ["DISABLE_O_ZERO_INIT"] = "1"
+    torch.manual_seed(1)
+    H, T = 2, 96
+    m = B200CausalSelfAttention(H * D, H, D, receives_ve=True, layer_idx=2).cuda()
+    leaf = torch.randn(1, T, H * D, device="cuda").bfloat16().requires_grad_(True)
+    ve = torch.randn(1, T, H * D, device="cuda").bfloat16()
+    doc = torch.zeros(T, dtype=torch.int32, device="cuda")
+
+    def forward():
+        x = leaf * 1                                                       # not a leaf: it may be changed in place
+        return x, m(x, ve, attn_mask=WindowMask(40, doc))
+
+    if changed is None:
+        wrt = [leaf, m.qkvo_w, m.g_ve]
+        _, y = forward()
+        ref = torch.autograd.grad(y.sum(), wrt)
+        with torch.autograd.graph.save_on_cpu():
+            _, y = forward()
+        assert all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(y.sum(), wrt), ref))
+        return
+    x, y = forward()
+    with torch.no_grad():
+        dict(x=x, ve=ve, g_ve=m.g_ve, qkvo_w=m.qkvo_w, doc_start=doc)[changed].add_(1)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        y.sum().backward()

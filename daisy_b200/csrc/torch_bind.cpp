@@ -476,7 +476,9 @@ Tensor attn_train(const Tensor& x, const Tensor& w, const OptTensor& ve, const O
                   double scale, int64_t window, const OptTensor& doc_start, bool in_blocks) {
   TORCH_CHECK_VALUE(x.is_cuda(), "x must be a CUDA tensor (daisy_b200 has no CPU path)");
   c10::cuda::CUDAGuard guard(x.device());
-  return AttnFunction::apply(x.scalar_type() == w.scalar_type() ? x : x.to(w.scalar_type()), w, ve, logit, cos, sin, H, eps, scale, window, doc_start, in_blocks);
+  // an embedding made in inference mode cannot be saved for the backward: a copy can
+  const OptTensor e = ve.has_value() && ve->is_inference() ? OptTensor(ve->clone()) : ve;
+  return AttnFunction::apply(x.scalar_type() == w.scalar_type() ? x : x.to(w.scalar_type()), w, e, logit, cos, sin, H, eps, scale, window, doc_start, in_blocks);
 }
 
 // ------------------------------------------------------------------ Kimi layer, one token

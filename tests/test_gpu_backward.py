@@ -228,6 +228,10 @@ def test_in_place_change_before_backward_raises(changed):
         with torch.autograd.graph.save_on_cpu():
             _, y = forward()
         assert all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(y.sum(), wrt), ref))
+        with torch.inference_mode():
+            ve = ve.clone()                                                # an embedding made in inference mode
+        _, y = forward()
+        assert all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(y.sum(), wrt), ref))
         return
     x, y = forward()
     with torch.no_grad():

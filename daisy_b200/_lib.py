@@ -56,6 +56,7 @@ SIGNATURES = {
     "daisy_b200_swa_token_workspace_bytes": (_sz, [_i] * 3),
     "daisy_b200_swa_token_step": (_i, [_vp, _i, _vp, _i64, _vp] + [_i64] * 3 + [_i64, _vp, _vp, _i, _i] + [_i, _i64] +
                                   [_i] * 3 + [_f, _f, _u, _vp, _sz, _vp, _vp]),
+    "daisy_b200_swa_token_rows": (_i, [_i] * 4 + [_vp] * 2),
     "daisy_b200_qkv_gemm_train": (_i, [_vp, _i64, _vp, _i64] + [_vp] * 7 + [_vp, _i64, _vp] + [_i] * 5 + [_f, _u, _vp, _vp]),
     "daisy_b200_qkv_prep_grad_blocks": (_i64, [_i] * 2),
     "daisy_b200_qkv_prep_grad": (_i, [_vp] * 15 + [_i] * 4 + [_vp]),

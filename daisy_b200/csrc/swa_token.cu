@@ -19,7 +19,10 @@
 // Exchanges carry their own flags: every 8-byte word is {4 bytes of data, the launch's and layer's tag}, written with one
 // store, and the reader polls the words it needs until the tags match.  That is one trip to L2 and back (~1.2k cycles)
 // where a counter barrier followed by the load was three (barrier alone: 2.4k), needs no fence, no atomic and nothing reset
-// between launches.  A buffer is rewritten one layer later, which needs the whole next x, hence every CTA's reads done.
+// between launches.  A buffer is rewritten one layer later, which needs the whole next x, hence the reads done of every CTA
+// that contributes to it.  With 256 channels 20 of 148 CTAs have no row of the output projection: nobody waits for those, and
+// one head's next o could be stored while such a CTA, owner of q, k or v rows of the other head only, still reads the old one.
+// So a CTA without rows does not read the vector (tk_gathers); in the last phase, after which nothing is rewritten, all do.
 // Both contractions run as m16n8k16 tensor-core products (16 weight rows or cache rows x batch rows or q) -- not for their
 // rate (HBM is the bound) but because a piece then costs a quarter of the instructions.  q and the softmax weights stay at
 // fp32 precision: each is split into a high and a low 16-bit part that occupy two of the product's empty columns / rows.
@@ -79,6 +82,11 @@ struct TokenGeom {
   int lo, hi;                                         // this CTA's pieces
   long long pos;
 };
+// First row of a CTA's share of a projection, in pairs of rows; whether a CTA of `rows` rows reads the vector it multiplies.
+__host__ __device__ __forceinline__ int tk_row(int cta, int ctas, int rows) { return 2 * (cta * (rows / 2) / ctas); }
+__host__ __device__ __forceinline__ bool tk_gathers(int rows, bool last) { return rows > 0 || last; }
+// every CTA has rows of q, k or v, so that whoever has seen all of them knows every CTA's reads of x, position and tag done
+static_assert(daisy_host::MAX_SMS <= 3 * DAISY_HEAD_DIM / 2, "row pairs of the smallest QKV projection");
 // (the launcher keeps pieces x CTAs below 2^31)
 __device__ __forceinline__ int tk_lo(int c, int tot, int parts) { return (int)tk_div((unsigned)c * (unsigned)tot, (unsigned)parts); }
 __device__ __forceinline__ int tk_owner(int tile, int tot, int parts) { return (int)tk_div(((unsigned)tile + 1u) * (unsigned)parts - 1u, (unsigned)tot); }
@@ -270,8 +278,8 @@ __global__ void __launch_bounds__(TK_CT, 1) swa_token_kernel(const __grid_consta
   const TokenGeom g = tk_geom(p);
   const uint32_t tag0 = *p.epoch + 1;                                           // stepped by the last act of CTA 0
   // rows of the projections, in pairs
-  const int a0 = 2 * (cta * (3 * p.dim / 2) / G), a1 = 2 * ((cta + 1) * (3 * p.dim / 2) / G);
-  const int c0 = 2 * (cta * (p.dim / 2) / G), c1 = 2 * ((cta + 1) * (p.dim / 2) / G);
+  const int a0 = tk_row(cta, G, 3 * p.dim), a1 = tk_row(cta + 1, G, 3 * p.dim);
+  const int c0 = tk_row(cta, G, p.dim), c1 = tk_row(cta + 1, G, p.dim);
   __syncthreads();
 
   const int ks_n = (p.dim + TK_KW - 1) / TK_KW, na = (a1 - a0 + 15) / 16 * ks_n, nb = g.hi - g.lo, nc = (c1 - c0 + 15) / 16 * ks_n;
@@ -304,8 +312,9 @@ __global__ void __launch_bounds__(TK_CT, 1) swa_token_kernel(const __grid_consta
     const TokenLayer& ly = p.layer[l];
     const uint32_t tag = tag0 + l;
     // ---- phases A and C: the vector, then the projection
+    const bool gathers = tk_gathers(is_c ? c1 - c0 : a1 - a0, ph == 2 * p.L - 1);
 #pragma unroll 1
-    for (int b = 0; b < p.B; ++b) {
+    for (int b = 0; gathers && b < p.B; ++b) {
       if (ph == 0) {
         for (int k = threadIdx.x; k < p.dim / 8; k += TK_CT) *reinterpret_cast<uint4*>(xs + b * xs_ld + k * 16) = ld_cg16(p.x + b * p.x_sb + k * 8);
       } else {
@@ -443,7 +452,7 @@ __global__ void __launch_bounds__(TK_CT, 1) swa_token_kernel(const __grid_consta
       tk_finish<F16>(p, g, ly, bars, kv, own, psum, any, others > 0 && sg == 0, bh_lo + sg * seg_step, sg, tag, lane);
   }
   in.drain();
-  // CTA 0 is done only when every CTA has contributed, hence read the position and the tag
+  // CTA 0 has read the last o: every CTA has contributed, hence read the position and the tag
   if (threadIdx.x == 0 && cta == 0) {
     *p.epoch = tag0 + p.L - 1;
     if (p.t_advance) *p.t_advance += 1;
@@ -461,6 +470,13 @@ extern "C" size_t daisy_b200_swa_token_workspace_bytes(int B, int H, int D) {
   const size_t dim = (size_t)H * D;
   const size_t parts = (size_t)daisy_host::MAX_SMS * TK_MAX_SEG;
   return 256 + tk_align(B * 3 * dim * 4) + 2 * TK_COPIES * tk_align(B * dim * 4) + parts * TK_PART * 16;
+}
+
+extern "C" int daisy_b200_swa_token_rows(int cta, int ctas, int dim, int phase, int* first, int* end) {
+  if (ctas <= 0 || cta < 0 || cta >= ctas || dim <= 0 || dim % DAISY_HEAD_DIM || dim > TK_MAX_DIM || phase < 0 || phase > 2 || !first || !end) return DAISY_EINVAL;
+  const int rows = phase ? dim : 3 * dim;
+  *first = tk_row(cta, ctas, rows); *end = tk_row(cta + 1, ctas, rows);
+  return tk_gathers(*end - *first, phase == 2) ? 1 : 0;
 }
 
 template <bool F16, int NB>

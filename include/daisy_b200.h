@@ -176,6 +176,10 @@ int daisy_b200_swa_token_step(const daisy_b200_token_layer* layers, int n_layers
                               int cap, int window, int table_rows, int64_t ve_sb,
                               int B, int H, int D, float scale, float eps, unsigned flags,
                               void* workspace, size_t workspace_bytes, int* status_word, void* stream);
+/* How that launch of `ctas` CTAs splits the projections of a layer: rows [*first, *end) that CTA `cta` computes in `phase` (0: QKV
+ * projection, 1: output projection, 2: that of the last layer); returns 1 if the CTA reads the projection's input vector, 0
+ * if not, or a negative status.  Used by the tests only. */
+int daisy_b200_swa_token_rows(int cta, int ctas, int dim, int phase, int* first, int* end);
 
 /* ---------------------------------------------------------------------------------------------
  * Sliding-window causal softmax attention, prefill form.

@@ -106,3 +106,33 @@ def test_decode_split_heuristic(lib):
     assert s(1, 1, 100, 148) == 1                             # short contexts are not split
     assert s(1, 1, 100000, 148) == 64                         # capped
     assert s(0, 16, 10, 148) == 1
+
+
+def test_token_step_rewrites_no_vector_that_may_still_be_read(lib):
+    """The single-launch step stores a layer's attention output o over the one of the layer before.  Head h's part is stored
+    once that head's q, k and v rows of the new layer are there, and those once the whole x is: so everybody who reads the old o
+    must own output rows (part of that x) or some of those q, k, v rows.  CTA 0, which steps the launch's tag and the position at
+    the end, must have read the last o, which needs QKV rows of every CTA."""
+    first, end = C.c_int(), C.c_int()
+
+    def rows(cta, ctas, dim, phase):
+        reads = lib.daisy_b200_swa_token_rows(cta, ctas, dim, phase, C.byref(first), C.byref(end))
+        assert reads in (0, 1)
+        return first.value, end.value, bool(reads)
+
+    for ctas in (1, 74, 132, 148, 160, 192):
+        for H in range(1, 17):
+            dim = 128 * H
+            qkv, out, last = ([rows(c, ctas, dim, ph) for c in range(ctas)] for ph in (0, 1, 2))
+            for part, n in ((qkv, 3 * dim), (out, dim), (last, dim)):
+                assert part[0][0] == 0 and part[-1][1] == n and all(a[1] == b[0] for a, b in zip(part, part[1:]))
+            assert all(b > a and reads for a, b, reads in qkv)
+            assert all(reads for a, b, reads in out if b > a) and last[0][2]
+            owners = {c for c, (a, b, _) in enumerate(out) if b > a}
+            readers = {c for c, (_, _, reads) in enumerate(out) if reads}
+            for h in range(H):
+                spans = [(part * dim + 128 * h, part * dim + 128 * h + 128) for part in range(3)]
+                seen = {c for c, (a, b, _) in enumerate(qkv) if any(a < hi and b > lo for lo, hi in spans)}
+                assert readers <= owners | seen, (ctas, H, h, sorted(readers - owners - seen))
+    assert lib.daisy_b200_swa_token_rows(148, 148, 256, 0, C.byref(first), C.byref(end)) < 0
+    assert lib.daisy_b200_swa_token_rows(0, 148, 200, 0, C.byref(first), C.byref(end)) < 0

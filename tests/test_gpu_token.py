@@ -66,6 +66,22 @@ def test_token_step_matches_oracle(B, H, L, t, cap, window, f16):
     assert torch.equal(k1[:, :, :, mask].cpu(), rk[:, :, :, mask]) and torch.equal(v1[:, :, :, mask].cpu(), rv[:, :, :, mask])
 
 
+@pytest.mark.parametrize("B,H", [(1, 2), (3, 2), (1, 1)])
+def test_token_step_of_narrow_layers_repeats(B, H):
+    """Layers of which some CTAs own no output row (128 and 256 channels), sixteen of them: the same bits in a hundred launches."""
+    from daisy_b200 import ops
+    from daisy_b200._lib import QKV_DEFAULT
+    from daisy_b200._native import ext
+    L, cap, t = 16, 64, 500
+    w, (rk, rv), x = _setup(B, H, L, cap, False, seed=7)
+    cos, sin = (a.cuda() for a in swa.rope_tables(D, t + 1))
+    w, rk, rv, x = [a.cuda() for a in w], rk.cuda(), rv.cuda(), x.cuda()
+    ys = [ext().token_step(x, w, [cos] * L, [sin] * L, rk, rv, t, None, None, 48, 0.12, 1e-6, QKV_DEFAULT, None, None, None, None, None, None)
+          for _ in range(100)]
+    ops.check_device_status("cuda")
+    assert all(torch.equal(y, ys[0]) for y in ys[1:])
+
+
 @pytest.mark.parametrize("B,H,bias", [(1, 1, False), (3, 6, True), (8, 16, False), (9, 5, True), (17, 2, False)])
 def test_kimi_token_step_continues_a_prefill(B, H, bias):
     """The single-launch Kimi step (csrc/kda_token.cu) after a prefill of T tokens against a prefill of T + 1: the output,

@@ -105,10 +105,12 @@ class StepRunner:
 
     @torch.inference_mode()
     def _step_graph(self, x: torch.Tensor) -> torch.Tensor:
-        """``_step`` into the fixed buffer.  Neither the warm-up run (made without the ring store) nor the
+        """``_step`` into the fixed buffer; ``x`` may lie on the host or broadcast to ``[batch, 1, dim]``.  Neither the warm-up run (made without the ring store) nor the
         capture itself (which executes nothing) has touched the ring, so a capture is safe at any position, also
         with a window larger than the ring, where the slot of the next token is the oldest row still attended."""
         if self._graph is None:
+            if x.shape != self._gx.shape or x.device != self._gx.device:
+                x = self._gx.copy_(x)
             self._token(x, 0, self.cache.t_dev, self._gy, self._gws)
         else:
             self._gx.copy_(x)

@@ -437,3 +437,30 @@ def test_step_runner_with_float16_cache():
     for m in layers:
         h, _, _ = swa.csa_prefill(h.bfloat16().float(), m.qkvo_w.detach().float().cpu(), H, D, W, cos, sin)
     assert_close_bf16(torch.cat(ys, 1), h[:, P:], "stepped part, fp16 cache", max_tol=6e-2, mean_tol=6e-3)
+
+
+@pytest.mark.parametrize("B", [2, 17])
+def test_graph_step_takes_what_copy_takes(B):
+    """``_step_graph`` in both its forms (one launch; a captured graph above 16 rows): ``x`` on the host, broadcast over the
+    batch or in another dtype gives the bits of the plain call; other shapes raise and step nothing."""
+    from daisy_b200 import B200CausalSelfAttention, StepRunner
+    os.environ["DISABLE_O_ZERO_INIT"] = "1"
+    torch.manual_seed(5)
+    H, D, T0 = 3, 128, 10
+    layers = [B200CausalSelfAttention(H * D, H, D, max_seq_len=64).cuda().eval() for _ in range(2)]
+    x = torch.randn(1, T0 + 1, H * D, device="cuda", dtype=torch.bfloat16).expand(B, -1, -1)     # the same rows
+    x, xt = x[:, :T0].contiguous(), x[:, T0:].contiguous()
+    run = StepRunner(layers, window=8, cache_capacity=8, batch=B)
+    run._prefill(x)
+    ref = run._step(xt)
+    run._prefill(x)
+    run.capture_step(B, H * D)
+    assert (run._graph is not None) == (B == 17)
+    for form in (xt, xt.cpu(), xt[:1], xt[0], xt[0, 0], xt.float()):
+        run._prefill(x)
+        assert torch.equal(run._step_graph(form), ref), form.shape
+    t = run.cache.t
+    for bad in (torch.cat([xt, xt], 1), xt[..., :-1], torch.cat([xt, xt])):
+        with pytest.raises((RuntimeError, ValueError)):
+            run._step_graph(bad)
+    assert run.cache.t == t == int(run.cache.t_dev)

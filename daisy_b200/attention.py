@@ -318,7 +318,10 @@ class B200CausalSelfAttention(nn.Module):
             kc, vc = kc.to(torch.bfloat16), vc.to(torch.bfloat16)
         if kc is None:                                        # no context yet: an empty one
             kc = vc = x.new_empty((B, self.num_heads, 0, self.head_dim), dtype=torch.bfloat16)
-        res = self._step_one_launch(x, kc, vc, n, pos, ve, window, write_ring=False)
+        # a broadcast context (a dimension of stride 0) has no tile form: the split kernel reads it row by row
+        res = None
+        if all(s > 0 or m == 1 for c in (kc, vc) for s, m in zip(c.stride(), c.shape)):
+            res = self._step_one_launch(x, kc, vc, n, pos, ve, window, write_ring=False)
         if res is not None:
             return res
         q, k, v = self._project(x)

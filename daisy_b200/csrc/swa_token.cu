@@ -522,22 +522,26 @@ extern "C" int daisy_b200_swa_token_step(const daisy_b200_token_layer* layers, i
   if ((flags & DAISY_WRITE_RING) && cap == 0) return DAISY_EINVAL;
   if (!t_dev && t >= table_rows) return DAISY_EINVAL;
   if ((reinterpret_cast<uintptr_t>(t_dev) & 7) || (reinterpret_cast<uintptr_t>(t_advance) & 7)) return DAISY_EINVAL;
+  const bool need_cache = (flags & DAISY_WRITE_RING) || (cap > 0 && window != 1 && (t_dev || t > 0));
+  if (!daisy_aligned16(x) || !daisy_aligned16(y) || (reinterpret_cast<uintptr_t>(workspace) & 255) || (x_sb & 7) ||
+      (need_cache && ((c_sb | c_sh | c_sr) & 7)))
+    return DAISY_EALIGN;
+  // a zero stride on a dimension longer than 1 is a broadcast (expanded) view, which the tile loads cannot express
+  if (need_cache && (c_sb < 0 || c_sh < 0 || c_sr < 0 || (B > 1 && c_sb == 0) || (H > 1 && c_sh == 0) || (cap > 1 && c_sr == 0))) return DAISY_EINVAL;
   const int sms = daisy_host::sm_count_cached();
   if (sms <= 0) return DAISY_ENODEV;
   // segments of a CTA's range: at most BH / G + 2 of them (see TK_MAX_SEG)
   if ((int64_t)B * H * ((int64_t)cap / 16 + 2) * sms >= ((int64_t)1 << 31)) return DAISY_EUNSUPPORTED;
   if (sms > daisy_host::MAX_SMS || (int64_t)B * H > (int64_t)sms * (TK_MAX_SEG - 2)) return DAISY_EUNSUPPORTED;
-  const bool need_cache = (flags & DAISY_WRITE_RING) || (cap > 0 && window != 1 && (t_dev || t > 0));
-  if (!daisy_aligned16(x) || !daisy_aligned16(y) ||
-      (reinterpret_cast<uintptr_t>(workspace) & 255) || (x_sb & 7) || ((c_sb | c_sh | c_sr) & 7))
-    return DAISY_EALIGN;
+  // a dimension of length 1 may come with any stride; the encoder wants a non-zero multiple of 16 bytes
+  auto stride = [](int64_t s, int n) { return (cuuint64_t)(n == 1 ? 16 : s * 2); };
   static_assert(sizeof(TokenParams) <= 32764, "kernel parameters");
   TokenParams p;
   const int dim = H * D;
   for (int l = 0; l < n_layers; ++l) {
     const daisy_b200_token_layer& s = layers[l];
     if (!s.qkvo_w || !s.cos || !s.sin || (need_cache && (!s.kcache || !s.vcache)) || (s.ve && !s.ve_gate_logit)) return DAISY_EINVAL;
-    if (!daisy_aligned16(s.qkvo_w) || !daisy_aligned16(s.kcache) || !daisy_aligned16(s.vcache) || !daisy_aligned16(s.ve) ||
+    if (!daisy_aligned16(s.qkvo_w) || (need_cache && (!daisy_aligned16(s.kcache) || !daisy_aligned16(s.vcache))) || !daisy_aligned16(s.ve) ||
         !daisy_aligned16(s.k_new_out) || !daisy_aligned16(s.v_new_out) || !daisy_aligned16(s.cos) || !daisy_aligned16(s.sin) || (s.ve && (ve_sb & 7)))
       return DAISY_EALIGN;
     TokenLayer& ly = p.layer[l];
@@ -545,7 +549,7 @@ extern "C" int daisy_b200_swa_token_step(const daisy_b200_token_layer* layers, i
     if ((rc = tk_make_weight_map(&ly.tw, s.qkvo_w, 4 * dim, dim)) != DAISY_OK) return rc;
     if (need_cache) {                                 // a ring as (64 elements, slots, halves of a row, h, b)
       const cuuint64_t dims[5] = {64, (cuuint64_t)cap, 2, (cuuint64_t)H, (cuuint64_t)B};
-      const cuuint64_t st[4] = {(cuuint64_t)c_sr * 2, 128, (cuuint64_t)c_sh * 2, (cuuint64_t)c_sb * 2};
+      const cuuint64_t st[4] = {stride(c_sr, cap), 128, stride(c_sh, H), stride(c_sb, B)};
       const cuuint32_t box[5] = {64, 16, 2, 1, 1};
       if ((rc = tk_make_map(&ly.tk, s.kcache, 5, dims, st, box)) != DAISY_OK) return rc;
       if ((rc = tk_make_map(&ly.tv, s.vcache, 5, dims, st, box)) != DAISY_OK) return rc;

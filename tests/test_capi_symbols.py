@@ -74,6 +74,12 @@ def test_argument_validation_without_gpu(lib):
     assert lib.daisy_b200_swa_decode_step(*bad, a, w, 4, None, None) == _lib.EUNSUPPORTED
     bad = list(args); bad[14] = -1
     assert lib.daisy_b200_swa_decode_step(*bad, a, w, 4, None, None) == _lib.EINVAL
+    # single-launch step: broadcast rings (a zero stride on a dimension longer than 1) and misaligned strides are refused
+    layer = (C.c_void_p * 9)(*[a] * 9)
+    tw = lib.daisy_b200_swa_token_workspace_bytes(2, 3, 128)
+    for strides, rc in (((0, 128, 384), _lib.EINVAL), ((6144, 0, 384), _lib.EINVAL), ((6144, 128, 0), _lib.EINVAL), ((6144, 132, 384), _lib.EALIGN)):
+        assert lib.daisy_b200_swa_token_step(C.addressof(layer), 1, a, 384, a, *strides, 16, None, None, 16, 8, 64, 0, 2, 3, 128, 0.12, 1e-6,
+                                             _lib.QKV_DEFAULT, a, tw, None, None) == rc
     # KDA: K != 128, chunk != 64, workspace
     kw = lib.daisy_b200_kda_workspace_bytes(1, 100, 2, 128, 128)
     assert kw == 1 * 2 * 2 * 83456

@@ -464,3 +464,30 @@ def test_graph_step_takes_what_copy_takes(B):
         with pytest.raises((RuntimeError, ValueError)):
             run._step_graph(bad)
     assert run.cache.t == t == int(run.cache.t_dev)
+
+
+@pytest.mark.parametrize("window", [None, 5, 1])
+def test_step_over_contexts_of_any_strides(window):
+    """``step`` over contexts that are not plain: one context broadcast over the batch, over the heads or over the rows, token-major
+    memory, a slice, a context of one row.  The same numbers as over a contiguous copy: bit for bit where the same kernel takes
+    both, else to the rounding of two kernels."""
+    H, D, B, n = 2, 128, 3, 21
+    m = _module(H * D, H, D)
+    g = torch.Generator(device="cuda").manual_seed(2)
+    x = torch.randn(B, 1, H * D, device="cuda", generator=g).bfloat16()
+    base = [torch.randn(B, n, H, D, device="cuda", generator=g).bfloat16() for _ in range(2)]
+    forms = dict(batch=lambda c: c[:1].expand(B, -1, -1, -1), heads=lambda c: c[:, :, :1].expand(-1, -1, H, -1), rows=lambda c: c[:, :1].expand(-1, n, -1, -1),
+                 token_major=lambda c: c.transpose(0, 1).contiguous().transpose(0, 1), head_major=lambda c: c.transpose(1, 2).contiguous().transpose(1, 2),
+                 a_slice=lambda c: c[:, 3:17], one_row=lambda c: c[:, 4:5])
+    with torch.inference_mode():
+        for name, form in forms.items():
+            k, v = (form(c) for c in base)
+            got = m.step(x, k, v, k.size(1), None, window)
+            ref = m.step(x, k.contiguous(), v.contiguous(), k.size(1), None, window)
+            for a, b, what in zip(got, ref, ("y", "k", "v")):
+                if name in ("batch", "heads", "rows"):
+                    assert_close_bf16(a, b.float().cpu(), f"{name} {what}")
+                else:
+                    assert torch.equal(a, b), (name, what)
+    from daisy_b200 import ops
+    ops.check_device_status("cuda")

@@ -4,6 +4,10 @@
 // call from Python and converting them one by one costs more than that.  Here the checks, the allocations and the launches
 // of a whole layer are native, the Python classes above only hold parameters and state.  Nothing is computed by torch on
 // these paths: it supplies device memory, the stream and the tensor type.
+//
+// Python objects are read first; the calls then run without the interpreter lock, as torch's own do.  A launch waits when the
+// queue is full and packed lengths on the device wait for the stream: other Python threads go on, also the one whose launch
+// that stream may be waiting for.
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAGraphsUtils.cuh>
 #include <c10/cuda/CUDAGuard.h>
@@ -530,13 +534,23 @@ Tensor f32c(const Tensor& t, const char* name) {
   return t;
 }
 
+// `cu_seqlens` as the caller gave it: nothing, a tensor, or any sequence of integers.
+struct Lengths { bool given = false; Tensor t; std::vector<int64_t> list; };
+Lengths lengths_of(const py::object& cu_seqlens) {
+  Lengths r;
+  r.given = !cu_seqlens.is_none();
+  if (THPVariable_Check(cu_seqlens.ptr())) r.t = THPVariable_Unpack(cu_seqlens.ptr());
+  else if (r.given)
+    for (auto item : cu_seqlens) r.list.push_back(py::cast<int64_t>(py::int_(py::reinterpret_borrow<py::object>(item))));
+  return r;
+}
+
 // Tables of a packed batch on the device (see kda_varlen_tables); tok only if asked for.
 struct Packed { Tensor chunks, ptr, tok; int64_t n_chunks = 0, n_seq = 0, total = 0; };
 // `meanwhile(n_seq)` runs while lengths that lie on the device are on their way.
-Packed pack_tables(const py::object& cu_seqlens, c10::Device dev, int64_t chunk, bool want_tok, const std::function<void(int64_t)>& meanwhile = {}) {
-  std::vector<int64_t> cu;
-  if (THPVariable_Check(cu_seqlens.ptr())) {
-    Tensor t = THPVariable_Unpack(cu_seqlens.ptr());
+Packed pack_tables(const Lengths& lengths, c10::Device dev, int64_t chunk, bool want_tok, const std::function<void(int64_t)>& meanwhile = {}) {
+  std::vector<int64_t> cu = lengths.list;
+  if (const Tensor& t = lengths.t; t.defined()) {
     if (t.is_cuda() && t.dim() == 1 && t.numel() > 1 && (t.scalar_type() == at::kInt || t.scalar_type() == at::kLong)) {
       c10::cuda::CUDAGuard guard(t.device());
       Tensor c = at::empty(t.sizes(), at::TensorOptions().dtype(t.scalar_type()).pinned_memory(true));
@@ -549,8 +563,6 @@ Packed pack_tables(const py::object& cu_seqlens, c10::Device dev, int64_t chunk,
       Tensor c = t.to(at::kCPU, at::kLong).contiguous();
       cu.assign(c.data_ptr<int64_t>(), c.data_ptr<int64_t>() + c.numel());
     }
-  } else {
-    for (auto item : cu_seqlens) cu.push_back(py::cast<int64_t>(py::int_(py::reinterpret_borrow<py::object>(item))));
   }
   bool ok = cu.size() >= 2 && cu[0] == 0;
   for (size_t i = 1; ok && i < cu.size(); ++i) ok = cu[i] >= cu[i - 1];
@@ -658,12 +670,12 @@ constexpr int64_t RECURRENT_MAX_T = 4;           // up to this many tokens the s
 
 // the layer's chunk_kda call: any float types, dense or packed
 std::pair<Tensor, OptTensor> chunk_kda(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& g_, const Tensor& beta_, std::optional<double> scale,
-                                       const OptTensor& h0_, bool want_state, bool l2norm, const py::object& cu_seqlens, bool out_fp32) {
+                                       const OptTensor& h0_, bool want_state, bool l2norm, const Lengths& cu_seqlens, bool out_fp32) {
   Tensor q = q_.to(at::kBFloat16).contiguous(), k = k_.to(at::kBFloat16).contiguous(), v = v_.to(at::kBFloat16).contiguous();
   Tensor g = g_.to(at::kFloat).contiguous(), beta = beta_.to(at::kFloat).contiguous();
   OptTensor h0;
   if (h0_.has_value()) h0 = h0_->to(at::kFloat).contiguous();
-  if (!cu_seqlens.is_none()) {
+  if (cu_seqlens.given) {
     KdaOut made;
     Packed p = pack_tables(cu_seqlens, q.device(), 64, false, [&](int64_t n) {
       if (q.dim() != 4 || v.dim() != 4 || q.size(0) != 1) return;                          // the call itself reports what is wrong
@@ -711,12 +723,12 @@ void kimi_linears(std::vector<Tensor> x, std::vector<Tensor> w, Tensor* y) {
 std::tuple<Tensor, OptTensor, std::vector<Tensor>> kimi_layer(const Tensor& x, const std::vector<Tensor>& w, const OptTensor& g1_bias, const OptTensor& norm_w,
                                                               const std::vector<Tensor>& conv_w, const std::vector<OptTensor>& conv_b, const Tensor& a_log,
                                                               const Tensor& dt_bias, const std::vector<OptTensor>& conv_s, const OptTensor& rec, bool use_cache,
-                                                              bool silu, double eps, int64_t H, const py::object& cu_seqlens) {
+                                                              bool silu, double eps, int64_t H, const Lengths& cu_seqlens) {
   TORCH_CHECK_VALUE(x.is_cuda(), "x must be a CUDA tensor (daisy_b200 has no CPU path)");
   c10::cuda::CUDAGuard guard(x.device());
   const int64_t B = x.size(0), T = x.size(1), C = w[0].size(0), M = B * T;
   Packed p;
-  const bool packed = !cu_seqlens.is_none();
+  const bool packed = cu_seqlens.given;
   if (packed) p = pack_tables(cu_seqlens, x.device(), 64, true);
   const int64_t n = packed ? p.n_seq : B;
   Tensor qkv[3], pr[3];
@@ -782,43 +794,58 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       PyErr_SetObject(cls.ptr(), cls(e.code, e.what()).ptr());
     }
   });
-  m.def("status_word", &status_word);
-  m.def("release_workspaces", &release_workspaces);
+  using nogil = py::call_guard<py::gil_scoped_release>;
+  m.def("status_word", &status_word, nogil());
+  m.def("release_workspaces", &release_workspaces, nogil());
   m.def("token_workspace_bytes", [](int64_t B, int64_t H) { return (int64_t)daisy_b200_swa_token_workspace_bytes((int)B, (int)H, 128); });
   m.def("token_step_supported", &token_step_supported);
-  m.def("token_step", &token_step);
-  m.def("gemm_nt", &gemm_nt);
-  m.def("qkv_gemm", &qkv_gemm);
+  m.def("token_step", &token_step, nogil());
+  m.def("gemm_nt", &gemm_nt, nogil());
+  m.def("qkv_gemm", &qkv_gemm, nogil());
   m.def("swa_attend", [](const Tensor& q, const Tensor& k, const Tensor& v, int64_t window, double scale, const OptTensor& out, bool bounded,
                          const OptTensor& doc_start, bool in_blocks) {
     return swa_attend(q, k, v, window, scale, out, bounded, doc_start, in_blocks, false).first;
-  });
+  }, nogil());
   m.def("swa_attend_lse", [](const Tensor& q, const Tensor& k, const Tensor& v, int64_t window, double scale, const OptTensor& out, bool bounded,
                              const OptTensor& doc_start, bool in_blocks) {
     return swa_attend(q, k, v, window, scale, out, bounded, doc_start, in_blocks, true);
-  });
-  m.def("attn_stack", &attn_stack);
-  m.def("attn_forward", &attn_forward);
-  m.def("attn_layer", &attn_layer);
-  m.def("attn_train", &attn_train);
+  }, nogil());
+  m.def("attn_stack", &attn_stack, nogil());
+  m.def("attn_forward", &attn_forward, nogil());
+  m.def("attn_layer", &attn_layer, nogil());
+  m.def("attn_train", &attn_train, nogil());
   m.def("kda_tables", [](const py::object& cu, const py::object& device, int64_t chunk) {
-    Packed p = pack_tables(cu, py::cast<c10::Device>(device), chunk, true);
+    const Lengths lengths = lengths_of(cu);
+    const c10::Device dev = py::cast<c10::Device>(device);
+    py::gil_scoped_release released;
+    Packed p = pack_tables(lengths, dev, chunk, true);
     return std::make_tuple(p.chunks, p.ptr, p.tok, p.n_chunks);
   });
   m.def("kda_chunk_fwd", [](const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& beta, std::optional<double> scale, const OptTensor& h0,
                             bool want_state, bool l2norm, bool out_fp32) {
     return kda_chunk(q, k, v, g, beta, scale, h0, want_state, l2norm, out_fp32, nullptr);
-  });
+  }, nogil());
   m.def("kda_chunk_fwd_varlen", [](const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& beta, const Tensor& chunks, const Tensor& ptr,
                                    int64_t total, int64_t n_chunks, std::optional<double> scale, const OptTensor& h0, bool want_state, bool l2norm, bool out_fp32) {
     Packed p;
     p.chunks = chunks; p.ptr = ptr; p.n_chunks = n_chunks; p.n_seq = ptr.numel() - 1; p.total = total;
     return kda_chunk(q, k, v, g, beta, scale, h0, want_state, l2norm, out_fp32, &p);
+  }, nogil());
+  m.def("kda_recurrent_fwd", &kda_recurrent, nogil());
+  m.def("chunk_kda", [](const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& beta, std::optional<double> scale, const OptTensor& h0,
+                        bool want_state, bool l2norm, const py::object& cu, bool out_fp32) {
+    const Lengths lengths = lengths_of(cu);
+    py::gil_scoped_release released;
+    return chunk_kda(q, k, v, g, beta, scale, h0, want_state, l2norm, lengths, out_fp32);
   });
-  m.def("kda_recurrent_fwd", &kda_recurrent);
-  m.def("chunk_kda", &chunk_kda);
-  m.def("kimi_layer", &kimi_layer);
+  m.def("kimi_layer", [](const Tensor& x, const std::vector<Tensor>& w, const OptTensor& g1_bias, const OptTensor& norm_w, const std::vector<Tensor>& conv_w,
+                         const std::vector<OptTensor>& conv_b, const Tensor& a_log, const Tensor& dt_bias, const std::vector<OptTensor>& conv_s, const OptTensor& rec,
+                         bool use_cache, bool silu, double eps, int64_t H, const py::object& cu) {
+    const Lengths lengths = lengths_of(cu);
+    py::gil_scoped_release released;
+    return kimi_layer(x, w, g1_bias, norm_w, conv_w, conv_b, a_log, dt_bias, conv_s, rec, use_cache, silu, eps, H, lengths);
+  });
   m.def("kda_token_supported", &kda_token_supported);
   m.def("kda_token_workspace_bytes", &kda_token_workspace_bytes);
-  m.def("kda_token_step", &kda_token_step);
+  m.def("kda_token_step", &kda_token_step, nogil());
 }

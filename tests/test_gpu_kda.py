@@ -277,3 +277,31 @@ def test_kda_varlen_against_fla_triton():
                      use_qk_l2norm_in_kernel=True, cu_seqlens=cu_t)
     assert ((o.float() - o_ref.float()).norm() / o_ref.float().norm()).item() <= 5e-3
     assert ((s.float() - s_ref.float()).norm() / s_ref.float().norm()).item() <= 5e-3
+
+
+def test_waiting_for_packed_lengths_leaves_other_threads_running():
+    """Lengths that lie on the device are read once the stream has come to them; the interpreter lock is free meanwhile."""
+    import threading
+    import time
+    from daisy_b200 import ops
+    a = torch.ones(16384, 16384, device="cuda", dtype=torch.bfloat16)
+    out = a @ a                                                            # the library's workspace, before the clock runs
+    q, k, v, g, beta = (t.cuda() for t in _inputs(1, 100, 2, seed=3))
+    cu = torch.tensor([0, 40, 100], dtype=torch.int32, device="cuda")
+    from daisy_b200.kda import chunk_kda
+    for call in (lambda: ops.kda_varlen_tables(cu, "cuda"), lambda: chunk_kda(q, k, v, g, beta, cu_seqlens=cu)):
+        call()
+        torch.cuda.synchronize()
+        for _ in range(60):                                                # some 0.3 s of work in front of them
+            torch.mm(a, a, out=out)
+        waiter = threading.Thread(target=call)
+        start = last = time.perf_counter()
+        waiter.start()
+        gap = 0.0
+        while waiter.is_alive():
+            now = time.perf_counter()
+            gap, last = max(gap, now - last), now
+        waited = time.perf_counter() - start
+        assert waited > 0.15, waited
+        assert max(gap, time.perf_counter() - last) < 0.5 * waited, (gap, waited)
+        torch.cuda.synchronize()

@@ -549,6 +549,7 @@ Lengths lengths_of(const py::object& cu_seqlens) {
 struct Packed { Tensor chunks, ptr, tok; int64_t n_chunks = 0, n_seq = 0, total = 0; };
 // `meanwhile(n_seq)` runs while lengths that lie on the device are on their way.
 Packed pack_tables(const Lengths& lengths, c10::Device dev, int64_t chunk, bool want_tok, const std::function<void(int64_t)>& meanwhile = {}) {
+  TORCH_CHECK_VALUE(chunk > 0, "chunk must be positive, got ", chunk);
   std::vector<int64_t> cu = lengths.list;
   if (const Tensor& t = lengths.t; t.defined()) {
     if (t.is_cuda() && t.dim() == 1 && t.numel() > 1 && (t.scalar_type() == at::kInt || t.scalar_type() == at::kLong)) {

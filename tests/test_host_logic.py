@@ -146,6 +146,9 @@ def test_varlen_tables_and_unpad_helpers():
     for bad in ([1, 5], [0, 5, 3], [0]):
         with pytest.raises(ValueError):
             ops.kda_varlen_tables(bad, "cpu")
+    for chunk in (0, -64):
+        with pytest.raises(ValueError):
+            ops.kda_varlen_tables([0, 5], "cpu", chunk)
     mask = torch.tensor([[0, 0, 1, 1, 1], [1, 1, 0, 1, 0], [0, 0, 0, 0, 0]])
     idx, cu, mx = get_unpad_data(mask)
     assert idx.tolist() == [2, 3, 4, 5, 6, 8] and cu.tolist() == [0, 3, 6, 6] and mx == 3 and cu.dtype == torch.int32

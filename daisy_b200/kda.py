@@ -193,18 +193,22 @@ class B200KimiLinearSelfAttention(torch.nn.Module):
 
     def _native_args(self):
         """Parameters in the order the native calls take them, or None where the layer is not of their form (four-tap
-        convolutions of one activation, 128-wide heads, bf16 weights, fp32 gate parameters)."""
+        convolutions of one activation, 128-wide heads, bf16 weights, fp32 gate parameters) or where its parts do more than
+        hold parameters: parametrized weights, other convolutions or norms in place of the layer's own, forward hooks on them."""
         m, p = self._modules, self._parameters
         if not self.use_short_conv or self.conv_size != 4 or self.head_dim != 128 or self.head_v_dim != 128:
             return None
-        lin = lambda name: m[name]._parameters["weight"]
-        seq = lambda name, i: m[name]._modules[i]._parameters["weight"]
+        lin = lambda name: m[name]._parameters.get("weight")               # absent where a parametrization makes the weight
+        seq = lambda name, i: m[name]._modules[i]._parameters.get("weight")
         w = [lin("q_proj"), lin("k_proj"), lin("v_proj"), seq("f_proj", "0"), seq("f_proj", "1"), seq("g_proj", "0"), seq("g_proj", "1"),
              lin("b_proj"), lin("o_proj")]
         cv = [m["q_conv1d"], m["k_conv1d"], m["v_conv1d"]]
-        act, gb, nw = cv[0].activation, m["g_proj"]._modules["1"]._parameters["bias"], m["o_norm"]._parameters["weight"]
-        bf = w + [c._parameters["weight"] for c in cv] + [gb, nw]
-        if (any(t.dtype != torch.bfloat16 or not t.is_contiguous() for t in bf) or p["A_log"].dtype != torch.float32 or p["dt_bias"].dtype != torch.float32
+        if (any(type(c) is not B200ShortConvolution or c._forward_hooks or c._forward_pre_hooks for c in cv)
+                or type(m["o_norm"]) is not B200FusedRMSNormGated or m["o_norm"]._forward_hooks or m["o_norm"]._forward_pre_hooks):
+            return None
+        act, gb, nw = cv[0].activation, m["g_proj"]._modules["1"]._parameters.get("bias"), m["o_norm"]._parameters.get("weight")
+        bf = w + [c._parameters.get("weight") for c in cv] + [gb, nw]
+        if (any(t is None or t.dtype != torch.bfloat16 or not t.is_contiguous() for t in bf) or p["A_log"].dtype != torch.float32 or p["dt_bias"].dtype != torch.float32
                 or any(c.activation != act for c in cv)):
             return None
         return w, gb, nw, [c._parameters["weight"] for c in cv], [c._parameters["bias"] for c in cv], p["A_log"], p["dt_bias"]
@@ -215,7 +219,7 @@ class B200KimiLinearSelfAttention(torch.nn.Module):
             raise NotImplementedError("daisy_b200 implements the forward pass only: call under torch.no_grad() / "
                                       "inference_mode(), or detach the input and freeze the parameters")
         B0, T0, _ = x.shape
-        if use_cache and T0 == 1 and attn_mask is None and (ve is None or sa_lambdas is None):
+        if use_cache and T0 == 1 and attn_mask is None and (ve is None or sa_lambdas is None) and x.dtype == torch.bfloat16:
             y = self._token_step(x)
             if y is not None:
                 self._seen += 1

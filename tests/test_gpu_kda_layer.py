@@ -290,6 +290,28 @@ def test_layer_step_graph_inputs_and_states(H):
             assert torch.equal(m.step_graph(x[:, T0:]), ref)
 
 
+@pytest.mark.parametrize("part", ["q_proj", "f_proj.1", "k_conv1d", "o_norm", "hook"])
+def test_layer_whose_parts_are_not_plain(part):
+    """A parametrized weight, or a hook on a convolution: the native calls take a layer's parameters past its modules, so such a
+    layer takes the composed route and gives the plain layer's numbers."""
+    from torch.nn.utils import parametrize
+    plain, m = _layer(seed=6), _layer(seed=6)
+    calls = []
+    if part == "hook":
+        m.q_conv1d.register_forward_hook(lambda *a: calls.append(1))
+    else:
+        parametrize.register_parametrization(m.get_submodule(part), "weight", torch.nn.Identity())
+    x = torch.randn(2, 70, 256, device="cuda").bfloat16()
+    with torch.inference_mode():
+        for layer in (plain, m):
+            layer.out = [layer.prefill(x[:, :69])[0], layer.step(x[:, 69:])[0]]
+    for a, b in zip(m.out, plain.out):
+        assert ((a.float() - b.float()).norm() / b.float().norm()).item() <= 1e-2
+    assert len(calls) == (2 if part == "hook" else 0)
+    with torch.inference_mode(), pytest.raises(RuntimeError):
+        plain.step(x[:, 69:].float())                                      # refused, as a prompt in float32 is
+
+
 # ------------------------------------------------------------------------------------ packed variable-length batches
 @pytest.mark.parametrize("W", [4, 2])
 @pytest.mark.parametrize("cu", [[0, 40], [0, 1, 2, 3, 4, 40], [0, 2, 2, 35, 67, 200], [0, 31, 32, 33, 96, 97]])

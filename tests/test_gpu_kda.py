@@ -53,12 +53,13 @@ def test_kda_matches_recurrence(B, T, H):
 @pytest.mark.parametrize("T", [49, 64, 200, 1000])
 def test_kda_weak_decay(T):
     """Gates near zero: every pair of 16-token blocks of a chunk, and the state over many chunks, weighs in (under ordinary
-    gates a block two away is already forgotten).  Keys shared by all tokens make the products between blocks large."""
+    gates a block two away is already forgotten).  Keys shared by all tokens make the products between blocks large.  fp16
+    operands give 7e-4 to 9e-4 here (21 draws over these and other lengths)."""
     q, k, v, g, beta = _inputs(2, T, 2, seed=T, gate_scale=0.002)
     k = (k + 1.5 * k[:, :1]).bfloat16()
     o_ref, s_ref = okda.kda_recurrent(q.float(), k.float(), v.float(), g, beta)
     o, s = _run(q, k, v, g, beta, output_final_state=True, out_fp32=True)
-    assert _rel(o, o_ref) <= 2 * REL_TOL and _rel(s, s_ref) <= 2 * REL_TOL
+    assert _rel(o, o_ref) <= REL_TOL and _rel(s, s_ref) <= REL_TOL
 
 
 def test_kda_third_party_fixture(golden_dir):

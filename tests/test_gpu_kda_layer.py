@@ -229,11 +229,13 @@ def test_layer_prefill_then_steps():
     assert m._recurrent_state is None and m._conv_state is None and m._seen == 0
 
 
-def test_layer_step_graph_matches_eager():
-    """The captured single-token step replays to the bits of the step launched kernel by kernel, states included."""
-    m = _layer(seed=9)
+@pytest.mark.parametrize("H", [2, 17])
+def test_layer_step_graph_matches_eager(H):
+    """``step_graph`` gives the bits of ``step``, states included: the single launch into a fixed buffer, and above 2048 channels
+    a captured graph against the step issued kernel by kernel, whose numbers the oracle's chained run confirms."""
+    m = _layer(128 * H, H, seed=9)
     B, T0, n = 2, 70, 6
-    x = torch.randn(B, T0 + n, 256, device="cuda").bfloat16()
+    x = torch.randn(B, T0 + n, 128 * H, device="cuda").bfloat16()
     with torch.inference_mode():
         m.prefill(x[:, :T0], None, None)
         eager = [m.step(x[:, t:t + 1], None, None, t, None, None, None)[0].clone() for t in range(T0, T0 + n)]
@@ -241,11 +243,20 @@ def test_layer_step_graph_matches_eager():
         m.reset_history()
         m.prefill(x[:, :T0], None, None)
         m.capture_step(batch=B)
+        assert (m._graph is not None) == (H == 17)
         graph = [m.step_graph(x[:, t:t + 1]).clone() for t in range(T0, T0 + n)]
     for a, b in zip(eager, graph):
         assert torch.equal(a, b)
     assert torch.equal(m._recurrent_state, rec_e) and all(torch.equal(a, b) for a, b in zip(m._conv_state, conv_e))
     assert m._seen == T0 + n
+    params = {k: p.detach().cpu() for k, p in m.named_parameters()}
+    _, st = okda.kimi_layer_forward(x[:, :T0].cpu(), params, H, 128)
+    refs = []
+    for t in range(T0, T0 + n):
+        y, st = okda.kimi_layer_forward(x[:, t:t + 1].cpu(), params, H, 128, state=st)
+        refs.append(y)
+    got, ref = torch.cat(graph, 1).float().cpu(), torch.cat(refs, 1)
+    assert ((got - ref).norm() / ref.norm()).item() <= 2e-2
 
 
 @pytest.mark.parametrize("H", [2, 17])

@@ -306,9 +306,10 @@ def test_forward_with_block_mask_training_form():
 
 
 def test_step_through_cuda_graph_equals_eager_steps():
-    """``StepRunner.capture_step`` / ``_step_graph``: one captured launch sequence with the position in device
-    memory, replayed per token, gives bit-identical outputs and ring contents to the eager ``_step`` -- through
-    the ramp-up (fewer context rows than the window), the steady state and the ring wrap."""
+    """``StepRunner.capture_step`` / ``_step_graph`` of a small stack, where both are the single launch: position from device
+    memory and fixed buffers against position from the host, bit-identical outputs and ring contents through the ramp-up (fewer
+    context rows than the window), the steady state and the ring wrap.  (A real capture:
+    ``test_captured_step_equals_eager_steps_and_the_oracle``.)"""
     from daisy_b200 import B200CausalSelfAttention, StepRunner
     os.environ["DISABLE_O_ZERO_INIT"] = "1"
     torch.manual_seed(4)
@@ -360,9 +361,9 @@ def test_prefill_fills_the_ring_like_bulk_write_packed(T, cap, dtype):
 
 
 def test_graph_capture_after_the_ring_wrapped_with_window_larger_than_capacity():
-    """Capturing the graph step must leave the ring alone: with a window larger than the ring capacity the slot of
-    the next token holds the oldest row the next step still attends to.  Eager steps first (so that slot holds a real
-    row), then the capture, then graph steps against eager ones."""
+    """``capture_step`` must leave the ring alone: with a window larger than the ring capacity the slot of the next token
+    holds the oldest row the next step still attends to.  Eager steps first (so that slot holds a real row), then
+    ``capture_step`` (nothing to record here: one launch is the step), then fixed-buffer steps against eager ones."""
     from daisy_b200 import B200CausalSelfAttention, StepRunner
     os.environ["DISABLE_O_ZERO_INIT"] = "1"
     torch.manual_seed(8)
@@ -389,8 +390,8 @@ def test_graph_capture_after_the_ring_wrapped_with_window_larger_than_capacity()
 
 
 def test_graph_step_with_value_embedding_layer():
-    """A layer that receives a value embedding through ``step_ring_dev`` (what the CUDA-graph step runs): same bits as
-    the eager ``step_ring``, and the step chain matches the windowed forward under the same embeddings."""
+    """A layer that receives a value embedding through ``step_ring_dev`` (position on the device): same bits as the
+    ``step_ring`` (position from the host), and the step chain matches the windowed forward under the same embeddings."""
     from daisy_b200 import B200CausalSelfAttention, B200KVCache, WindowMask
     os.environ["DISABLE_O_ZERO_INIT"] = "1"
     torch.manual_seed(3)
@@ -415,7 +416,7 @@ def test_graph_step_with_value_embedding_layer():
 
 def test_step_runner_with_float16_cache():
     """The runner with ``dtype=torch.float16`` for the cache, as ``Generator`` defaults to: prefill fills the fp16
-    ring, eager and CUDA-graph steps read and extend it; results stay within the bf16 bar of the oracle."""
+    ring, eager and fixed-buffer steps read and extend it; results stay within the bf16 bar of the oracle."""
     from daisy_b200 import B200CausalSelfAttention, StepRunner
     os.environ["DISABLE_O_ZERO_INIT"] = "1"
     torch.manual_seed(6)
@@ -491,3 +492,96 @@ def test_step_over_contexts_of_any_strides(window):
                     assert torch.equal(a, b), (name, what)
     from daisy_b200 import ops
     ops.check_device_status("cuda")
+
+
+def _rel(a, b):
+    a, b = a.float().cpu(), b.float().cpu()
+    return ((a - b).norm() / b.norm()).item()
+
+
+@pytest.mark.parametrize("B,H,ve,f16", [(17, 2, False, False), (64, 3, True, False), (1, 17, False, True), (9, 17, True, False)])
+def test_steps_above_the_single_launch_match_oracle(B, H, ve, f16):
+    """``step``, ``step_ring`` and ``step_ring_dev`` of batches above 16 rows and layers wider than 2048, which are three
+    launches (projection, ring decode, projection): a few tokens over a wrapped ring against the oracle.  Bars: bf16 results
+    of bf16 operands once for the rows and twice (attention, output projection) for y."""
+    from daisy_b200 import B200CausalSelfAttention, B200KVCache, ops
+    from daisy_b200._native import ext
+    assert not ext().token_step_supported(B, H, 1)
+    torch.manual_seed(B + H)
+    D, cap, W, t0, N = 128, 16, 12, 21, 3
+    dim = H * D
+    m = B200CausalSelfAttention(dim, H, D, receives_ve=ve, layer_idx=2, max_seq_len=64).cuda().eval()
+    with torch.no_grad():
+        m.qkvo_w.copy_(torch.randn(4, dim, dim) * dim ** -0.5)
+    w, cos, sin = m.qkvo_w.detach().float().cpu(), m.rotary.cos.cpu(), m.rotary.sin.cpu()
+    dtype = torch.float16 if f16 else torch.bfloat16
+    ring, dev, ctx = (B200KVCache(1, B, H, cap, D, "cuda", dtype) for _ in range(3))
+    ring.k.normal_(); ring.v.normal_()
+    for c in (dev, ctx):
+        c.k.copy_(ring.k); c.v.copy_(ring.v)
+    for c in (ring, dev, ctx):
+        c.set_position(t0)
+    with torch.inference_mode():
+        for t in range(t0, t0 + N):
+            x = torch.randn(B, 1, dim, device="cuda").bfloat16()
+            e = torch.randn(B, 1, dim, device="cuda").bfloat16() if ve else None
+            idx = torch.arange(t - cap, t) % cap
+            kc, vc = (r[0][:, :, idx].transpose(1, 2).float().cpu() for r in (ring.k, ring.v))
+            y, k, v = m.step_ring(x, ring, 0, t, e, W)
+            assert torch.equal(m.step_ring_dev(x, dev, 0, W, ve=e), y)
+            yc, k2, v2 = m.step(x, *ctx.view(0), t, e, W)
+            ctx.write(0, k2, v2)
+            assert torch.equal(k2, k) and torch.equal(v2, v) and _rel(yc, y) < 5e-3
+            for c in (ring, dev, ctx):
+                c.advance()
+            q, kr, vr = swa.project_qkv(x.float().cpu(), w, H, D)
+            qn, kn, vn = swa.qkv_transform(q, kr, vr, cos[t:t + 1], sin[t:t + 1], m.norm_eps)
+            if ve:
+                gate = torch.sigmoid(m.g_ve.detach().float().cpu())
+                vn = gate * vn + (1 - gate) * e.float().cpu().view_as(vn)
+            K, V = torch.cat([kc[:, cap - W + 1:], kn], 1), torch.cat([vc[:, cap - W + 1:], vn], 1)
+            p = torch.softmax(torch.einsum("bqhd,bkhd->bhqk", qn, K) * swa.ATTN_SCALE, -1)
+            yo = torch.einsum("bhqk,bkhd->bqhd", p, V).reshape(B, 1, dim) @ w[3].t()
+            assert _rel(k, kn) < 5e-3 and _rel(v, vn) < 5e-3 and _rel(y, yo) < 1e-2, (_rel(k, kn), _rel(v, vn), _rel(y, yo))
+    ops.check_device_status("cuda")
+    assert torch.equal(ring.k, dev.k) and torch.equal(ring.v, dev.v)
+    assert _rel(ctx.k, ring.k) < 5e-3 and _rel(ctx.v, ring.v) < 5e-3
+
+
+@pytest.mark.parametrize("B,H", [(17, 2), (2, 17)])
+def test_captured_step_equals_eager_steps_and_the_oracle(B, H):
+    """Stacks above the single launch: ``capture_step`` records a CUDA graph.  Replays against the steps issued layer by layer,
+    bit for bit, through ramp-up, steady state, ring wrap and a capture after the wrap with the window larger than the ring; and
+    against the oracle's prefill of all tokens through both layers."""
+    from daisy_b200 import B200CausalSelfAttention, StepRunner, ops
+    torch.manual_seed(B)
+    D, P, N = 128, 10, 30
+    dim = H * D
+    layers = [B200CausalSelfAttention(dim, H, D, max_seq_len=64).cuda().eval() for _ in range(2)]
+    for m in layers:
+        with torch.no_grad():
+            m.qkvo_w.copy_(torch.randn(4, dim, dim) * dim ** -0.5)
+    x = torch.randn(B, P + N, dim, device="cuda").bfloat16()
+    for W, cap, before in ((12, 16, 0), (40, 16, 9)):
+        eager, graph = (StepRunner(layers, window=W, cache_capacity=cap, batch=B) for _ in range(2))
+        ys = []
+        for run in (eager, graph):
+            run._prefill(x[:, :P])
+            for t in range(P, P + before):
+                run._step(x[:, t:t + 1])
+        rings = graph.cache.k.clone(), graph.cache.v.clone()
+        graph.capture_step(B, dim)
+        assert graph._graph is not None
+        assert torch.equal(graph.cache.k, rings[0]) and torch.equal(graph.cache.v, rings[1])
+        for t in range(P + before, P + N):
+            ys.append(graph._step_graph(x[:, t:t + 1]).clone())
+            assert torch.equal(eager._step(x[:, t:t + 1]), ys[-1]), f"token {t}"
+        ops.check_device_status("cuda")
+        assert torch.equal(graph.cache.k, eager.cache.k) and torch.equal(graph.cache.v, eager.cache.v)
+        assert graph.cache.t == eager.cache.t == int(graph.cache.t_dev) == P + N
+        if W > cap:
+            continue                                                       # the ring holds fewer rows than the window asks for
+        h = x.float().cpu()
+        for m in layers:
+            h, _, _ = swa.csa_prefill(h.bfloat16().float(), m.qkvo_w.detach().float().cpu(), H, D, W, m.rotary.cos.cpu(), m.rotary.sin.cpu(), m.norm_eps)
+        assert _rel(torch.cat(ys, 1), h[:, P:]) < 1.5e-2                   # 1e-2 a layer, two layers

@@ -66,6 +66,29 @@ def test_token_step_matches_oracle(B, H, L, t, cap, window, f16):
     assert torch.equal(k1[:, :, :, mask].cpu(), rk[:, :, :, mask]) and torch.equal(v1[:, :, :, mask].cpu(), rv[:, :, :, mask])
 
 
+@pytest.mark.parametrize("t,cap,window", [(5, 64, 40), (16, 64, 40), (47, 64, 48), (100, 64, 20), (130, 64, 50), (63, 64, 64), (0, 64, 40)])
+@pytest.mark.parametrize("f16", [False, True])
+def test_token_step_ignores_rows_outside_the_context(t, cap, window, f16):
+    """Ring slots outside the context hold infinities and NaN (a ring that another sequence has used): the same bits as over
+    zeros, with the context ending inside a piece of 16 rows, at one, at the ring's end, and wrapped."""
+    from daisy_b200 import ops
+    from daisy_b200._lib import QKV_DEFAULT
+    from daisy_b200._native import ext
+    B, H = 2, 3
+    w, ring, x = _setup(B, H, 1, cap, f16, seed=t)
+    cos, sin = (a.cuda() for a in swa.rope_tables(D, t + 1))
+    keep = torch.zeros(cap, dtype=torch.bool)
+    keep[torch.arange(t - min(t, cap, window - 1), t) % cap] = True
+    ys = []
+    for fill in ((0.0, 0.0), (float("nan"), float("inf")), (float("-inf"), float("nan"))):
+        rk, rv = (r.clone() for r in ring)
+        rk[:, :, :, ~keep], rv[:, :, :, ~keep] = fill
+        ys.append(ext().token_step(x.cuda(), [w[0].cuda()], [cos], [sin], rk.cuda(), rv.cuda(), t, None, None, window, 0.12, 1e-6, QKV_DEFAULT,
+                                   None, None, None, None, None, None))
+    ops.check_device_status("cuda")
+    assert torch.isfinite(ys[0].float()).all() and all(torch.equal(y, ys[0]) for y in ys[1:])
+
+
 @pytest.mark.parametrize("B,H", [(1, 2), (3, 2), (1, 1)])
 def test_token_step_of_narrow_layers_repeats(B, H):
     """Layers of which some CTAs own no output row (128 and 256 channels), sixteen of them: the same bits in a hundred launches."""

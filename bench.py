@@ -50,12 +50,12 @@ KDA_SMALL = dict(B=1, T=8192, H=16, K=128, V=128, chunk=64)
 # sequences).  NOT measured by this run: each entry names the summary and the source revision it was captured at,
 # and goes stale when that kernel changes.
 NCU_TRAFFIC = {
-    "prefill_per_batch_row": {"bytes": 1077.9e6 / 8, "profile": "profiles/swa_prefill_kernel__prefill_small.md",
-                              "captured_at": "813cf57"},
+    "prefill_per_batch_row": {"bytes": 1260.8e6 / 8, "profile": "profiles/swa_prefill_kernel__prefill_small.md",
+                              "captured_at": "09937ab"},
     "decode_per_batch_row": {"bytes": 137.3e6 / 4, "profile": "profiles/swa_decode_partial_kernel__decode_small.md",
                              "captured_at": "c27d954"},
-    "kda_per_token_head": {"bytes": 455.3e6 / 131072, "profile": "profiles/kda_intra_kernel__kda_small.md + profiles/kda_state_kernel__kda_small.md",
-                           "captured_at": "e346a2c"},
+    "kda_per_token_head": {"bytes": 445.9e6 / 131072, "profile": "profiles/kda_intra_kernel__kda_small.md + profiles/kda_state_kernel__kda_small.md",
+                           "captured_at": "a470085"},
 }
 ROPE_BASE = 10000.0     # the benchmark configs name base 10000 (the module default is 1024, half-truncated)
 
@@ -652,8 +652,10 @@ def run_decode(cfg, warmup, dist, rank, world, peaks, lean=False, extras=True):
 
 def generator_step_latency(H, D, W, layers=4, batch=1, steps=200):
     """The reference's Generator shape (batch 1, `inference/generate.py:76`): one token through `layers` attention
-    layers (projections + fused ring decode), issued launch by launch from Python and as one CUDA-graph replay
-    with the position in device memory.  Microseconds per token, steady state (full window, wrapped ring)."""
+    layers (projections + ring decode).  Both keys time the single launch that takes the token through the stack:
+    "eager" with the position from the host and a new output per call, "graph" with the position in device memory and
+    fixed buffers (`capture_step`; stacks above that launch record a CUDA graph there).  Microseconds per token, steady
+    state (full window, wrapped ring)."""
     from daisy_b200 import B200CausalSelfAttention, StepRunner
     os.environ["DISABLE_O_ZERO_INIT"] = "1"
     torch.manual_seed(0)

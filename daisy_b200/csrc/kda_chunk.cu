@@ -30,7 +30,7 @@ constexpr int OFF_QT = OFF_WT + KD * KC * 2;           // q~       [2][64 tokens
 constexpr int OFF_KT = OFF_QT + KD * KC * 2;           // k~       [2][64 tokens][64 channels] fp16   k e^{G_C-G}
 constexpr int OFF_AQK = OFF_KT + KD * KC * 2;          // A_qk     [64][64]  fp16
 constexpr int OFF_D = OFF_AQK + KC * KC * 2;           // e^{G_C}  [128]     fp32
-constexpr int SHARED_BYTES = OFF_D + KD * 4;           // 57856: identical for every V-slice
+constexpr int SHARED_BYTES = OFF_D + KD * 4;           // 57856: up to here what the state is multiplied with; then what is added
 constexpr int OFF_UT = SHARED_BYTES;                   // U0^T     [128 value columns][64 tokens] fp16
 constexpr int REC_BYTES = OFF_UT + KD * KC * 2;        // 74240
 static_assert(SHARED_BYTES % 16 == 0 && REC_BYTES % 16 == 0, "bulk copies move 16-byte units");
@@ -570,7 +570,7 @@ struct KdaStateParams {
 // One CTA per (batch, head); TMEM lane = value column, so all products have M = 128 and
 //     U^T [V x 64]   = U0^T - S^T W^T            S^T as fp16 from TMEM, W^T as the record has it (channels = depth)
 //     O^T [V x 64]   = S^T q~^T + U^T A_qk^T
-//     S^T [V x 128] <- S^T diag(e^{G_C}) + U^T k~  accumulated in TMEM on the scaled state
+//     S^T [V x 128] <- S^T diag(e^{G_C}) + U^T k~  the product summed in TMEM, added to the state in registers
 // The chain from chunk to chunk is all that matters (a (batch, head) is serial, and there are rarely more of them than SMs):
 // S to fp16, 8 products of N = 64, U to fp16, 4 products of N = 128.  Warps 0-7 (thread = half a value column) run it with the
 // state in fp32 registers, scaled while the U products run; TMEM carries only fp16 operands and fresh sums.  Two warps to a

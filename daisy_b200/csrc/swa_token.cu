@@ -389,14 +389,13 @@ __global__ void __launch_bounds__(TK_CT, 1) swa_token_kernel(const __grid_consta
 #pragma unroll
           for (int j = 0; j < 4; ++j) a[j] = g8 == 0 ? a[j] : 0u;
           // V rows past the context hold whatever an earlier sequence left in the ring: their weights are zero, but zero times
-          // an infinity is not.  (Masked for every piece: a branch for the last one costs the same 1 % of a token.)
-          const uint32_t keep0 = (2 * t4 < valid ? 0xffffu : 0u) | (2 * t4 + 1 < valid ? 0xffff0000u : 0u);
-          const uint32_t keep1 = (2 * t4 + 8 < valid ? 0xffffu : 0u) | (2 * t4 + 9 < valid ? 0xffff0000u : 0u);
+          // an infinity is not.  The lanes that address such rows read the last row of the context instead.
+          const int vr = min((lane & 7) + 8 * ((lane >> 3) & 1), valid - 1);
+          const uint32_t vrow = blk + 2 * TK_BLK + vr * 128 + (((lane >> 4) ^ (vr & 7)) << 4);
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             uint32_t bv[4];
-            tk_ldm4_t(bv, blk + (2 + (j >> 2)) * TK_BLK + swz[j & 3]);
-            bv[0] &= keep0; bv[1] &= keep1; bv[2] &= keep0; bv[3] &= keep1;
+            tk_ldm4_t(bv, (vrow ^ ((j & 3) << 5)) + (j >> 2) * TK_BLK);
             tk_mma<F16>(acc[2 * j], a, bv[0], bv[1]);
             tk_mma<F16>(acc[2 * j + 1], a, bv[2], bv[3]);
           }

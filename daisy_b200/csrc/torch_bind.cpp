@@ -42,6 +42,10 @@ void req(const Tensor& t, const char* name, at::ScalarType dt = at::kBFloat16) {
   TORCH_CHECK_VALUE(t.dim() > 0 && t.stride(-1) == 1, name, " must be contiguous in its last dimension");
 }
 
+bool on16(const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0; }
+// the same values where 16-byte loads can fetch them
+Tensor aligned(const Tensor& t) { return t.is_contiguous() && on16(t) ? t : t.clone(at::MemoryFormat::Contiguous); }
+
 // A decode step's vectors: x beside the state or ring it goes with, and the caller's buffer for the result.
 void req_step(const Tensor& x, const OptTensor& out, const Tensor& state, int64_t B, int64_t dim) {
   TORCH_CHECK_VALUE(x.is_cuda(), "x must be a CUDA tensor (daisy_b200 has no CPU path)");
@@ -374,18 +378,21 @@ struct Saved {
   }
 };
 struct AttnFunction : public torch::autograd::Function<AttnFunction> {
-  static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& x, const Tensor& w, const OptTensor& ve, const OptTensor& logit, const Tensor& cos,
+  static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& x, const Tensor& w_, const OptTensor& ve, const OptTensor& logit, const Tensor& cos,
                         const Tensor& sin, int64_t H, double eps, double scale, int64_t window, const OptTensor& doc_start, bool in_blocks) {
     at::AutoDispatchBelowADInplaceOrView guard;
-    req(x, "x"); req(w, "qkvo_w");
-    const int64_t B = x.size(0), T = x.size(1), dim = w.size(2), M = B * T;
-    TORCH_CHECK_VALUE(w.dim() == 3 && w.size(0) == 4 && w.is_contiguous() && dim == H * 128 && x.size(2) == dim, "qkvo_w must be a contiguous [4, dim, dim]");
+    req(x, "x"); req(w_, "qkvo_w");
+    TORCH_CHECK_VALUE(x.dim() == 3 && w_.dim() == 3, "x must be [B, T, dim], qkvo_w [4, dim, dim]");
+    const int64_t B = x.size(0), T = x.size(1), dim = H * 128, M = B * T;
+    TORCH_CHECK_VALUE(w_.size(0) == 4 && w_.size(1) == dim && w_.size(2) == dim && x.size(2) == dim, "qkvo_w must be [4, dim, dim]");
     rope_table(cos, "cos"); rope_table(sin, "sin");
+    const Tensor w = aligned(w_);
     Tensor x2 = rows_of(x, dim);
+    if (!on16(x2) || x2.stride(0) % 8) x2 = x2.clone(at::MemoryFormat::Contiguous);
     Tensor ve2, g32;
     if (ve.has_value()) {
       req(*ve, "ve");
-      ve2 = ve->reshape({M, dim}).contiguous();
+      ve2 = aligned(ve->reshape({M, dim}));
       g32 = logit->to(at::kFloat).reshape({1});
     }
     const Saved at_(M, H, ve2.defined());
@@ -406,7 +413,7 @@ struct AttnFunction : public torch::autograd::Function<AttnFunction> {
     check(daisy_b200_gemm_nt(p + at_.o, dim, (char*)w.data_ptr() + 3 * dim * dim * 2, dim, y.data_ptr(), dim, (int)M, (int)dim, (int)dim, status, st), "daisy_b200_gemm_nt");
     // the inputs themselves, not views of them made here: below the autograd keys a view has a version counter of its own, and
     // a change in place between forward and backward would go unnoticed
-    ctx->save_for_backward({x, w, buf, cos, sin, ve.value_or(Tensor()), ve.has_value() ? *logit : Tensor(), doc_start.value_or(Tensor())});
+    ctx->save_for_backward({x, w_, buf, cos, sin, ve.value_or(Tensor()), ve.has_value() ? *logit : Tensor(), doc_start.value_or(Tensor())});
     ctx->saved_data["dims"] = std::vector<int64_t>{B, T, H, window, in_blocks ? 1 : 0};
     ctx->saved_data["scale"] = scale;
     if (ve.has_value()) {
@@ -424,7 +431,7 @@ struct AttnFunction : public torch::autograd::Function<AttnFunction> {
     const int64_t B = d[0], T = d[1], H = d[2], window = d[3], dim = H * 128, M = B * T;
     const Tensor x2 = rows_of(s[0], dim);
     Tensor ve2, g32;
-    if (s[5].defined()) { ve2 = s[5].reshape({M, dim}).contiguous(); g32 = s[6].to(at::kFloat).reshape({1}); }
+    if (s[5].defined()) { ve2 = aligned(s[5].reshape({M, dim})); g32 = s[6].to(at::kFloat).reshape({1}); }
     const float scale = (float)ctx->saved_data["scale"].toDouble();
     const bool need_x = ctx->needs_input_grad(0), need_w = ctx->needs_input_grad(1);
     Tensor dy = grads[0].to(at::kBFloat16).reshape({M, dim});
@@ -433,7 +440,7 @@ struct AttnFunction : public torch::autograd::Function<AttnFunction> {
     char* p = (char*)buf.data_ptr();
     Tensor dw, dx;
     if (need_w) {
-      dw = at::empty_like(w);
+      dw = at::empty(w.sizes(), w.options());
       Tensor dwo = dw.select(0, 3);
       at::mm_out(dwo, dy.t(), buf.narrow(0, at_.o / 2, M * dim).view({M, dim}));
     }
@@ -460,7 +467,7 @@ struct AttnFunction : public torch::autograd::Function<AttnFunction> {
                                    sin.data_ptr<float>(), dqkv.data_ptr(), ptr(ve2), (const float*)ptr(g32), ptr(d_ve), (float*)ptr(d_logit),
                                    n_part ? (float*)(g + part_at) : nullptr, (int)M, (int)T, (int)H, 128, stream),
           "daisy_b200_qkv_prep_grad");
-    const Tensor wqkv = w.narrow(0, 0, 3).view({3 * dim, dim});
+    const Tensor wqkv = w.narrow(0, 0, 3).reshape({3 * dim, dim});
     if (need_w) {
       Tensor dwq = dw.narrow(0, 0, 3).view({3 * dim, dim});
       at::mm_out(dwq, dqkv.t(), x2);

@@ -238,3 +238,30 @@ def test_in_place_change_before_backward_raises(changed):
         dict(x=x, ve=ve, g_ve=m.g_ve, qkvo_w=m.qkvo_w, doc_start=doc)[changed].add_(1)
     with pytest.raises(RuntimeError, match="modified by an inplace operation"):
         y.sum().backward()
+
+
+def test_training_layer_takes_any_alignment():
+    """x, ve and the weights at addresses and strides that no 16-byte load can fetch against the call on aligned copies: the
+    same y; gradients from the library's products, whose fp32 sums may go in another order there, up to one bf16 rounding
+    (2^-8 of a value)."""
+    from daisy_b200 import B200CausalSelfAttention, WindowMask
+    os.environ["DISABLE_O_ZERO_INIT"] = "1"
+    torch.manual_seed(2)
+    H, T = 2, 96
+    dim = H * D
+    m = B200CausalSelfAttention(dim, H, D, receives_ve=True, layer_idx=2).cuda()
+    w, x, ve = m.qkvo_w.detach().clone(), *(torch.randn(2, T, dim, device="cuda").bfloat16() for _ in range(2))
+
+    def off(t):                                                            # the same values one element further on
+        return torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")[1:].view(t.shape).copy_(t)
+
+    wide = torch.empty(2, T, dim + 3, dtype=x.dtype, device="cuda")[..., :dim].copy_(x)      # rows 2 * 259 bytes apart
+    ref = None
+    for x_, ve_, w_ in ((x, ve, w), (off(x), ve, w), (wide, ve, w), (x, off(ve), w), (x, ve, off(w))):
+        x_, ve_ = x_.requires_grad_(True), ve_.requires_grad_(True)
+        m.qkvo_w = torch.nn.Parameter(w_)
+        y = m(x_, ve_, attn_mask=WindowMask(40))
+        got = [y.detach(), *torch.autograd.grad(y.float().square().sum(), [x_, ve_, m.qkvo_w, m.g_ve])]
+        ref = ref or got
+        assert torch.equal(got[0], ref[0])
+        assert all(((a.float() - b.float()).norm() / b.float().norm()).item() <= 2 ** -8 for a, b in zip(got[1:], ref[1:]))

@@ -46,6 +46,13 @@ bool on16(const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) &
 // the same values where 16-byte loads can fetch them
 Tensor aligned(const Tensor& t) { return t.is_contiguous() && on16(t) ? t : t.clone(at::MemoryFormat::Contiguous); }
 
+// An attention layer's weights; a layout with gaps between rows or matrices is packed.
+Tensor layer_weight(const Tensor& w, int64_t dim) {
+  req(w, "qkvo_w");
+  TORCH_CHECK_VALUE(w.dim() == 3 && w.size(0) == 4 && w.size(1) == dim && w.size(2) == dim, "qkvo_w must be [4, ", dim, ", ", dim, "]");
+  return w.contiguous();
+}
+
 // A decode step's vectors: x beside the state or ring it goes with, and the caller's buffer for the result.
 void req_step(const Tensor& x, const OptTensor& out, const Tensor& state, int64_t B, int64_t dim) {
   TORCH_CHECK_VALUE(x.is_cuda(), "x must be a CUDA tensor (daisy_b200 has no CPU path)");
@@ -137,11 +144,11 @@ Tensor token_step(const Tensor& x_, const std::vector<Tensor>& weights, const st
   if (x.dim() == 3 && x.size(1) == 1 && x.stride(2) == 1 && x.stride(0) % 8 == 0) x_sb = x.stride(0);
   else if (!x.is_contiguous()) x = x.contiguous();
   std::vector<daisy_b200_token_layer> ly(L);
+  std::vector<Tensor> packed;                                            // weights that had to be copied, until the launch
   int64_t rows = INT32_MAX;
   for (int64_t l = 0; l < L; ++l) {
-    const Tensor& w = weights[l];
-    req(w, "qkvo_w");
-    TORCH_CHECK_VALUE(w.dim() == 3 && w.size(0) == 4 && w.size(1) == dim && w.size(2) == dim && w.is_contiguous(), "qkvo_w must be a contiguous [4, ", dim, ", ", dim, "]");
+    const Tensor w = layer_weight(weights[l], dim);
+    if (!w.is_same(weights[l])) packed.push_back(w);
     rope_table(cos[l], "cos"); rope_table(sin[l], "sin");
     rows = std::min({rows, cos[l].size(0), sin[l].size(0)});
     ly[l].qkvo_w = w.data_ptr();
@@ -271,16 +278,16 @@ std::pair<Tensor, Tensor> swa_attend(const Tensor& q, const Tensor& k, const Ten
 }
 
 // The layer's output alone: q', k', v' and the attention output are scratch, one allocation.
-Tensor attn_forward(const Tensor& x_, const Tensor& qkvo_w, const Tensor& cos, const Tensor& sin, int64_t H, double eps, double scale, int64_t window,
+Tensor attn_forward(const Tensor& x_, const Tensor& w_, const Tensor& cos, const Tensor& sin, int64_t H, double eps, double scale, int64_t window,
                     const OptTensor& doc_start, bool in_blocks, const OptTensor& ve, const OptTensor& ve_gate) {
   TORCH_CHECK_VALUE(x_.is_cuda(), "x must be a CUDA tensor (daisy_b200 has no CPU path)");
-  const Tensor x = x_.detach().to(qkvo_w.scalar_type());
-  req(x, "x"); req(qkvo_w, "qkvo_w");
+  const Tensor x = x_.detach().to(w_.scalar_type());
+  req(x, "x");
   c10::cuda::CUDAGuard guard(x.device());
   TORCH_CHECK_VALUE(x.dim() == 3, "x must be [B, T, dim]");
   const int64_t B = x.size(0), T = x.size(1), dim = x.size(2), M = B * T;
-  TORCH_CHECK_VALUE(qkvo_w.dim() == 3 && qkvo_w.size(0) == 4 && qkvo_w.size(1) == dim && qkvo_w.size(2) == dim && dim == H * 128 && qkvo_w.is_contiguous(),
-                    "qkvo_w must be a contiguous [4, ", dim, ", ", dim, "]");
+  const Tensor qkvo_w = layer_weight(w_, H * 128);
+  TORCH_CHECK_VALUE(dim == H * 128, "x must be [B, T, ", H * 128, "]");
   rope_table(cos, "cos"); rope_table(sin, "sin");
   TORCH_CHECK_VALUE(cos.size(0) >= T && sin.size(0) >= T, "cos, sin must be contiguous float32 CUDA tensors of at least T rows");
   Tensor x2 = rows_of(x, dim), ve2;
@@ -311,7 +318,7 @@ Tensor attn_forward(const Tensor& x_, const Tensor& qkvo_w, const Tensor& cos, c
 std::vector<Tensor> attn_layer(const Tensor& x_, const Tensor& qkvo_w, const Tensor& cos, const Tensor& sin, int64_t H, double eps, double scale, int64_t window,
                                const OptTensor& doc_start, bool in_blocks, const OptTensor& ve, const OptTensor& ve_gate, const OptTensor& ring_k,
                                const OptTensor& ring_v, int64_t ring_first) {
-  Tensor w = qkvo_w.detach(), x = x_.detach().to(w.scalar_type());
+  Tensor w = layer_weight(qkvo_w.detach(), H * 128), x = x_.detach().to(w.scalar_type());
   TORCH_CHECK_VALUE(x.is_cuda(), "x must be a CUDA tensor (daisy_b200 has no CPU path)");
   c10::cuda::CUDAGuard guard(x.device());
   const int64_t B = x.size(0), T = x.size(1), dim = w.size(2);
@@ -341,9 +348,7 @@ Tensor attn_stack(const Tensor& x_, const std::vector<Tensor>& weights, const st
   int* status = status_ptr(x);
   void* st = stream_of(x);
   for (size_t l = 0; l < L; ++l) {
-    const Tensor& w = weights[l];
-    req(w, "qkvo_w");
-    TORCH_CHECK_VALUE(w.dim() == 3 && w.size(0) == 4 && w.size(1) == dim && w.size(2) == dim && w.is_contiguous(), "qkvo_w must be a contiguous [4, ", dim, ", ", dim, "]");
+    const Tensor w = layer_weight(weights[l], dim);
     rope_table(cos[l], "cos"); rope_table(sin[l], "sin");
     TORCH_CHECK_VALUE(cos[l].size(0) >= T && sin[l].size(0) >= T, "cos, sin must be contiguous float32 CUDA tensors of at least T rows");
     char *rk = ring ? (char*)k.data_ptr() + l * k.stride(0) * 2 : nullptr, *rv = ring ? (char*)v.data_ptr() + l * v.stride(0) * 2 : nullptr;

@@ -585,3 +585,26 @@ def test_captured_step_equals_eager_steps_and_the_oracle(B, H):
         for m in layers:
             h, _, _ = swa.csa_prefill(h.bfloat16().float(), m.qkvo_w.detach().float().cpu(), H, D, W, m.rotary.cos.cpu(), m.rotary.sin.cpu(), m.norm_eps)
         assert _rel(torch.cat(ys, 1), h[:, P:]) < 1.5e-2                   # 1e-2 a layer, two layers
+
+
+def test_weights_with_gaps_between_rows():
+    """A ``qkvo_w`` that is a view into larger storage (rows with gaps): every call gives the bits of the packed copy."""
+    from daisy_b200 import B200KVCache, StepRunner, WindowMask
+    H, D, T = 2, 128, 40
+    dim = H * D
+    plain, m = _module(dim, H, D), _module(dim, H, D)
+    store = torch.randn(4, dim, dim + 64, device="cuda").bfloat16() * dim ** -0.5
+    plain.qkvo_w = torch.nn.Parameter(store[:, :, :dim].contiguous())
+    m.qkvo_w = torch.nn.Parameter(store[:, :, :dim])
+    assert not m.qkvo_w.is_contiguous()
+    x = torch.randn(2, T, dim, device="cuda").bfloat16()
+    outs = []
+    for a in (plain, m):
+        with torch.inference_mode():
+            run = StepRunner([a, a], window=12, batch=2)
+            cache = B200KVCache(1, 2, H, 16, D, "cuda")
+            out = [a(x, None, attn_mask=WindowMask(12)), *a.prefill(x, None, attn_mask=WindowMask(12)), run._prefill(x[:, :-1]), run._step(x[:, -1:]),
+                   *a.step_ring(x[:, :1], cache, 0, 0, None, 12), run.cache.k, run.cache.v]
+        y = a(x, None, attn_mask=WindowMask(12))
+        outs.append(out + [y.detach(), *torch.autograd.grad(y.float().square().sum(), [a.qkvo_w])])
+    assert all(torch.equal(p, q) for p, q in zip(*outs))

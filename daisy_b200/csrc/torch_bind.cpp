@@ -502,15 +502,16 @@ bool kda_token_supported(int64_t H) { return H >= 1 && daisy_b200_kda_token_work
 int64_t kda_token_workspace_bytes(int64_t B, int64_t H) { return (int64_t)daisy_b200_kda_token_workspace_bytes((int)std::min<int64_t>(B, 16), (int)H, 128); }
 
 // weights: q, k, v, f0, f1, g0, g1, b, o; conv: q, k, v weights (and biases); the states are updated in place
-Tensor kda_token_step(const Tensor& x_, const std::vector<Tensor>& w, const OptTensor& g1_bias, const OptTensor& norm_w, const std::vector<Tensor>& conv_w,
+Tensor kda_token_step(const Tensor& x_, const std::vector<Tensor>& w_, const OptTensor& g1_bias, const OptTensor& norm_w, const std::vector<Tensor>& conv_w,
                       const std::vector<OptTensor>& conv_b, const Tensor& a_log, const Tensor& dt_bias, Tensor state, const std::vector<Tensor>& conv_s,
                       bool silu, double eps, const OptTensor& out, const OptTensor& workspace) {
-  TORCH_CHECK_VALUE(w.size() == 9 && conv_w.size() == 3 && conv_b.size() == 3 && conv_s.size() == 3, "nine weights, three convolutions");
+  TORCH_CHECK_VALUE(w_.size() == 9 && conv_w.size() == 3 && conv_b.size() == 3 && conv_s.size() == 3, "nine weights, three convolutions");
   const int64_t B = state.size(0), H = state.size(1), dim = H * 128;
   req_step(x_, out, state, B, dim);
   c10::cuda::CUDAGuard guard(x_.device());
-  Tensor x = x_.to(at::kBFloat16).reshape({B, dim}).contiguous();
-  for (const Tensor& t : w) { req(t, "weight"); TORCH_CHECK_VALUE(t.is_contiguous(), "weights must be contiguous"); }
+  Tensor x = aligned(x_.to(at::kBFloat16).reshape({B, dim}));
+  std::vector<Tensor> w(w_);
+  for (Tensor& t : w) { req(t, "weight"); TORCH_CHECK_VALUE(t.is_contiguous(), "weights must be contiguous"); t = aligned(t); }
   daisy_b200_kda_layer ly{};
   ly.q_w = w[0].data_ptr(); ly.k_w = w[1].data_ptr(); ly.v_w = w[2].data_ptr(); ly.f0_w = w[3].data_ptr(); ly.f1_w = w[4].data_ptr();
   ly.g0_w = w[5].data_ptr(); ly.g1_w = w[6].data_ptr(); ly.b_w = w[7].data_ptr(); ly.o_w = w[8].data_ptr();

@@ -323,6 +323,20 @@ def test_layer_whose_parts_are_not_plain(part):
         plain.step(x[:, 69:].float())                                      # refused, as a prompt in float32 is
 
 
+def test_layer_step_takes_any_alignment():
+    """A token and weights at odd addresses: the bits of the step on aligned ones."""
+    off = lambda t: torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")[1:].view(t.shape).copy_(t)
+    x, ys = torch.randn(2, 70, 256, device="cuda").bfloat16(), []
+    for change in (lambda m, x: x, lambda m, x: off(x), lambda m, x: setattr(m.q_proj, "weight", torch.nn.Parameter(off(m.q_proj.weight.detach()))) or x):
+        m = _layer(seed=8)
+        with torch.inference_mode():
+            m.prefill(x[:, :69])
+        xt = change(m, x[:, 69:])
+        with torch.inference_mode():
+            ys.append(m.step(xt)[0])
+    assert torch.equal(ys[1], ys[0]) and torch.equal(ys[2], ys[0])
+
+
 # ------------------------------------------------------------------------------------ packed variable-length batches
 @pytest.mark.parametrize("W", [4, 2])
 @pytest.mark.parametrize("cu", [[0, 40], [0, 1, 2, 3, 4, 40], [0, 2, 2, 35, 67, 200], [0, 31, 32, 33, 96, 97]])

@@ -88,8 +88,7 @@ _lib = None
 class DaisyB200Error(RuntimeError):
     def __init__(self, code: int, what: str):
         self.code = code
-        msg = lib().daisy_b200_strerror(code).decode() if _lib is not None else "?"
-        super().__init__(f"{what}: daisy_b200 status {code} ({msg})")
+        super().__init__(f"{what}: daisy_b200 status {code} ({lib().daisy_b200_strerror(code).decode()})")
 
 
 def lib() -> C.CDLL:

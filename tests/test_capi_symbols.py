@@ -35,6 +35,13 @@ def test_version_and_strerror(lib):
     assert b"unknown" in lib.daisy_b200_strerror(-99)
 
 
+def test_error_names_the_status_before_any_ctypes_call(monkeypatch):
+    """Errors of the native binding, which does not load the library through ctypes, say what the status means too."""
+    from daisy_b200 import _lib
+    monkeypatch.setattr(_lib, "_lib", None)
+    assert "aligned" in str(_lib.DaisyB200Error(_lib.EALIGN, "call"))
+
+
 def test_missing_library_fails_loudly(tmp_path, monkeypatch):
     from daisy_b200 import _lib
     monkeypatch.setattr(_lib, "_lib", None)

@@ -565,7 +565,8 @@ Packed pack_tables(const Lengths& lengths, c10::Device dev, int64_t chunk, bool 
   TORCH_CHECK_VALUE(chunk > 0, "chunk must be positive, got ", chunk);
   std::vector<int64_t> cu = lengths.list;
   if (const Tensor& t = lengths.t; t.defined()) {
-    if (t.is_cuda() && t.dim() == 1 && t.numel() > 1 && (t.scalar_type() == at::kInt || t.scalar_type() == at::kLong)) {
+    TORCH_CHECK_VALUE(t.dim() == 1, "cu_seqlens must have one dimension, got ", t.sizes());
+    if (t.is_cuda() && t.numel() > 1 && (t.scalar_type() == at::kInt || t.scalar_type() == at::kLong)) {
       c10::cuda::CUDAGuard guard(t.device());
       Tensor c = at::empty(t.sizes(), at::TensorOptions().dtype(t.scalar_type()).pinned_memory(true));
       c.copy_(t, /*non_blocking=*/true);

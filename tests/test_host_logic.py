@@ -143,7 +143,7 @@ def test_varlen_tables_and_unpad_helpers():
     assert tok_tab[198].tolist() == [135, 3] and chunk_tab.dtype == seq_ptr.dtype == tok_tab.dtype == torch.int32
     t2 = ops.kda_varlen_tables(torch.tensor([0, 64]), "cpu")
     assert t2[0].tolist() == [[0, 64]] and t2[3] == 1
-    for bad in ([1, 5], [0, 5, 3], [0]):
+    for bad in ([1, 5], [0, 5, 3], [0], torch.tensor([[0, 5]]), torch.tensor(0)):
         with pytest.raises(ValueError):
             ops.kda_varlen_tables(bad, "cpu")
     for chunk in (0, -64):

@@ -397,8 +397,9 @@ struct AttnFunction : public torch::autograd::Function<AttnFunction> {
     Tensor ve2, g32;
     if (ve.has_value()) {
       req(*ve, "ve");
-      ve2 = aligned(ve->reshape({M, dim}));
-      g32 = logit->to(at::kFloat).reshape({1});
+      TORCH_CHECK_VALUE(ve->numel() == M * dim && logit->numel() == 1, "ve must be [", B, ", ", T, ", ", dim, "], its gate one number");
+      ve2 = aligned(*ve);
+      g32 = logit->to(at::kFloat);
     }
     const Saved at_(M, H, ve2.defined());
     Tensor buf = at::empty({at_.elems}, x.options());
@@ -434,9 +435,8 @@ struct AttnFunction : public torch::autograd::Function<AttnFunction> {
     const Tensor &w = s[1], &buf = s[2], &cos = s[3], &sin = s[4], &doc = s[7];
     auto d = ctx->saved_data["dims"].toIntVector();
     const int64_t B = d[0], T = d[1], H = d[2], window = d[3], dim = H * 128, M = B * T;
-    const Tensor x2 = rows_of(s[0], dim);
     Tensor ve2, g32;
-    if (s[5].defined()) { ve2 = aligned(s[5].reshape({M, dim})); g32 = s[6].to(at::kFloat).reshape({1}); }
+    if (s[5].defined()) { ve2 = aligned(s[5]); g32 = s[6].to(at::kFloat); }
     const float scale = (float)ctx->saved_data["scale"].toDouble();
     const bool need_x = ctx->needs_input_grad(0), need_w = ctx->needs_input_grad(1);
     Tensor dy = grads[0].to(at::kBFloat16).reshape({M, dim});
@@ -475,7 +475,7 @@ struct AttnFunction : public torch::autograd::Function<AttnFunction> {
     const Tensor wqkv = w.narrow(0, 0, 3).reshape({3 * dim, dim});
     if (need_w) {
       Tensor dwq = dw.narrow(0, 0, 3).view({3 * dim, dim});
-      at::mm_out(dwq, dqkv.t(), x2);
+      at::mm_out(dwq, dqkv.t(), rows_of(s[0], dim));
     }
     if (need_x) dx = at::mm(dqkv, wqkv).view({B, T, dim});
     torch::autograd::variable_list out(12);
@@ -498,6 +498,12 @@ Tensor attn_train(const Tensor& x, const Tensor& w, const OptTensor& ve, const O
 }
 
 // ------------------------------------------------------------------ Kimi layer, one token
+// whether all of them are there, bf16 and contiguous
+bool plain_bf16(const std::vector<OptTensor>& ts) {
+  for (const OptTensor& t : ts)
+    if (!t.has_value() || t->scalar_type() != at::kBFloat16 || !t->is_contiguous()) return false;
+  return true;
+}
 bool kda_token_supported(int64_t H) { return H >= 1 && daisy_b200_kda_token_workspace_bytes(1, (int)H, 128) != 0; }
 int64_t kda_token_workspace_bytes(int64_t B, int64_t H) { return (int64_t)daisy_b200_kda_token_workspace_bytes((int)std::min<int64_t>(B, 16), (int)H, 128); }
 
@@ -510,8 +516,11 @@ Tensor kda_token_step(const Tensor& x_, const std::vector<Tensor>& w_, const Opt
   req_step(x_, out, state, B, dim);
   c10::cuda::CUDAGuard guard(x_.device());
   Tensor x = aligned(x_.to(at::kBFloat16).reshape({B, dim}));
-  std::vector<Tensor> w(w_);
-  for (Tensor& t : w) { req(t, "weight"); TORCH_CHECK_VALUE(t.is_contiguous(), "weights must be contiguous"); t = aligned(t); }
+  bool as_is = true;
+  for (const Tensor& t : w_) { req(t, "weight"); TORCH_CHECK_VALUE(t.is_contiguous(), "weights must be contiguous"); as_is = as_is && on16(t); }
+  std::vector<Tensor> copies;
+  if (!as_is) for (const Tensor& t : w_) copies.push_back(aligned(t));
+  const std::vector<Tensor>& w = as_is ? w_ : copies;
   daisy_b200_kda_layer ly{};
   ly.q_w = w[0].data_ptr(); ly.k_w = w[1].data_ptr(); ly.v_w = w[2].data_ptr(); ly.f0_w = w[3].data_ptr(); ly.f1_w = w[4].data_ptr();
   ly.g0_w = w[5].data_ptr(); ly.g1_w = w[6].data_ptr(); ly.b_w = w[7].data_ptr(); ly.o_w = w[8].data_ptr();
@@ -860,6 +869,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     py::gil_scoped_release released;
     return kimi_layer(x, w, g1_bias, norm_w, conv_w, conv_b, a_log, dt_bias, conv_s, rec, use_cache, silu, eps, H, lengths);
   });
+  m.def("plain_bf16", &plain_bf16);
   m.def("kda_token_supported", &kda_token_supported);
   m.def("kda_token_workspace_bytes", &kda_token_workspace_bytes);
   m.def("kda_token_step", &kda_token_step, nogil());

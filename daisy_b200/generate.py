@@ -109,7 +109,7 @@ class StepRunner:
         capture itself (which executes nothing) has touched the ring, so a capture is safe at any position, also
         with a window larger than the ring, where the slot of the next token is the oldest row still attended."""
         if self._graph is None:
-            if x.shape != self._gx.shape or x.device != self._gx.device:
+            if x.get_device() != self._gx.get_device() or x.shape != self._gx.shape:
                 x = self._gx.copy_(x)
             self._token(x, 0, self.cache.t_dev, self._gy, self._gws)
         else:

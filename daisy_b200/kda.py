@@ -202,16 +202,18 @@ class B200KimiLinearSelfAttention(torch.nn.Module):
         seq = lambda name, i: m[name]._modules[i]._parameters.get("weight")
         w = [lin("q_proj"), lin("k_proj"), lin("v_proj"), seq("f_proj", "0"), seq("f_proj", "1"), seq("g_proj", "0"), seq("g_proj", "1"),
              lin("b_proj"), lin("o_proj")]
-        cv = [m["q_conv1d"], m["k_conv1d"], m["v_conv1d"]]
-        if (any(type(c) is not B200ShortConvolution or c._forward_hooks or c._forward_pre_hooks for c in cv)
-                or type(m["o_norm"]) is not B200FusedRMSNormGated or m["o_norm"]._forward_hooks or m["o_norm"]._forward_pre_hooks):
+        cq, ck, cc, no = cv = m["q_conv1d"], m["k_conv1d"], m["v_conv1d"], m["o_norm"]
+        if (not (type(cq) is type(ck) is type(cc) is B200ShortConvolution and type(no) is B200FusedRMSNormGated)
+                or cq._forward_hooks or ck._forward_hooks or cc._forward_hooks or no._forward_hooks
+                or cq._forward_pre_hooks or ck._forward_pre_hooks or cc._forward_pre_hooks or no._forward_pre_hooks):
             return None
-        act, gb, nw = cv[0].activation, m["g_proj"]._modules["1"]._parameters.get("bias"), m["o_norm"]._parameters.get("weight")
+        cv, act, gb, nw = cv[:3], cq.activation, m["g_proj"]._modules["1"]._parameters.get("bias"), no._parameters.get("weight")
         bf = w + [c._parameters.get("weight") for c in cv] + [gb, nw]
-        if (any(t is None or t.dtype != torch.bfloat16 or not t.is_contiguous() for t in bf) or p["A_log"].dtype != torch.float32 or p["dt_bias"].dtype != torch.float32
+        a_log, dt = p.get("A_log"), p.get("dt_bias")
+        if (not ext().plain_bf16(bf) or a_log is None or dt is None or a_log.dtype != torch.float32 or dt.dtype != torch.float32
                 or any(c.activation != act for c in cv)):
             return None
-        return w, gb, nw, [c._parameters["weight"] for c in cv], [c._parameters["bias"] for c in cv], p["A_log"], p["dt_bias"]
+        return w, gb, nw, [c._parameters["weight"] for c in cv], [c._parameters["bias"] for c in cv], a_log, dt
 
     def _forward_core(self, x, ve, sa_lambdas, attn_mask, use_cache: bool):
         if torch.is_grad_enabled() and (x.requires_grad or any(p.requires_grad for p in self.parameters())):
@@ -325,7 +327,7 @@ class B200KimiLinearSelfAttention(torch.nn.Module):
         host or broadcast to that shape.  The states of the layer must be there: one launch takes them where they are (another
         ``prefill`` of the same batch may have made them), a graph only those ``capture_step`` saw."""
         if self._graph is None:
-            if x.shape != self._gx.shape or x.device != self._gx.device:
+            if x.get_device() != self._gx.get_device() or x.shape != self._gx.shape:
                 x = self._gx.copy_(x)
             if self._token_step(x, self._gy, self._gws) is None:
                 raise RuntimeError("step_graph: the cached states are gone or of another batch size (prefill, then capture_step)")

@@ -301,7 +301,7 @@ def test_layer_step_graph_inputs_and_states(H):
             assert torch.equal(m.step_graph(x[:, T0:]), ref)
 
 
-@pytest.mark.parametrize("part", ["q_proj", "f_proj.1", "k_conv1d", "o_norm", "hook"])
+@pytest.mark.parametrize("part", ["q_proj", "f_proj.1", "k_conv1d", "o_norm", "", "hook"])
 def test_layer_whose_parts_are_not_plain(part):
     """A parametrized weight, or a hook on a convolution: the native calls take a layer's parameters past its modules, so such a
     layer takes the composed route and gives the plain layer's numbers."""
@@ -311,7 +311,7 @@ def test_layer_whose_parts_are_not_plain(part):
     if part == "hook":
         m.q_conv1d.register_forward_hook(lambda *a: calls.append(1))
     else:
-        parametrize.register_parametrization(m.get_submodule(part), "weight", torch.nn.Identity())
+        parametrize.register_parametrization(m.get_submodule(part), "weight" if part else "A_log", torch.nn.Identity())
     x = torch.randn(2, 70, 256, device="cuda").bfloat16()
     with torch.inference_mode():
         for layer in (plain, m):

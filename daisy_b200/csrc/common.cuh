@@ -204,6 +204,11 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t saddr, uint32_t lbo
   d |= (uint64_t)2 << 61;
   return d;
 }
+// The same without a swizzle (layout type 0): core matrices of 8 rows x 16 bytes in 128 contiguous bytes.  MN-major: rows = depth,
+// lbo between groups of 8 depths, sbo between groups of 8 of the other index.
+__device__ __forceinline__ uint64_t umma_desc_plain(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
+  return umma_desc_sw128(saddr, lbo_bytes, sbo_bytes) & ~((uint64_t)7 << 61);
+}
 // Instruction descriptor for kind::f16 with bf16 inputs and fp32 accumulation.
 //   bits [4,6) D format (1 = f32)   [7,10) A format (1 = bf16)   [10,13) B format (1 = bf16)
 //   bit 15 A major (0 = K)          bit 16 B major (0 = K, 1 = MN)

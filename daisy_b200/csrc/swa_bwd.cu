@@ -6,18 +6,9 @@
 //     dV = P^T dO        dK = scale dZ^T Q        dQ = scale dZ K
 // P is rebuilt from the forward's per-row log2 denominators: P[q,k] = 2^(Z[q,k] log2 e - lse2[q]).
 //
-// One kernel template, two launches, no atomics (bitwise deterministic):
-//   MODE 0  key block stationary:  item = 128 keys of one (batch, head); K_j, V_j stay in shared memory, the query
-//           blocks that can see them stream through (Q_i, dO_i).  Scores are formed TRANSPOSED,
-//           S^T = K_j Q_i^T and dP^T = V_j dO_i^T (TMEM lane = key), so P^T and dZ^T, rounded to bf16 and written back
-//           over them, are exactly the TMEM A operands of  dV += P^T dO_i  and  dK += dZ^T Q_i.
-//   MODE 1  query block stationary:  item = 128 queries; Q_i, dO_i stay, the key blocks of the window stream
-//           (K_j, V_j);  S = Q_i K_j^T, dP = dO_i V_j^T (TMEM lane = query),  dQ += dZ K_j.
-// In both:  S = X0 Y0^T,  dP = X1 Y1^T  (X stationary, Y streamed),  acc1 += dZ Y0,  and MODE 0 also acc0 += P Y1.
-// Roles (576 threads): warps 0-15 rebuild P / dZ -- four warpgroups, thread = TMEM lane, 32 of a tile's 128 columns
-// each (every warpgroup writes its bf16 results over the first 16 columns of its OWN 32, so nobody overwrites
-// columns somebody else still has to read) -- and write the results; warp 16 TMA producer, warp 17 MMA issuer.
-// TMEM: S [0,128) dP [128,256) acc0 [256,384) acc1 [384,512).
+// No atomics: results are bitwise reproducible.  swa_bwd_kv_kernel is key block stationary and gives dK, dV, and dZ as operand
+// images where there is room for them, from which swa_bwd_dq_kernel gets dQ; without that room swa_bwd_q_kernel, query block
+// stationary, forms the scores again.
 // All mbarrier waits are bounded (abort flag, DAISY_ETIMEOUT through the status word).
 #include "common.cuh"
 
@@ -29,7 +20,8 @@ constexpr int W_HALF = W_TILE / 2;
 constexpr int W_NST = 2;                                  // stages of streamed (Y0, Y1) tile pairs
 constexpr int BWD_THREADS = 576;
 constexpr int BWD_WORKERS = 512;                          // threads of warps 0-15
-constexpr int BWD_SMEM = 1024 + 2 * W_TILE + W_NST * 2 * W_TILE + 2 * 3 * WB * 4 + 256;
+constexpr int BWD_SMEM = 1024 + 2 * W_TILE + W_NST * 2 * W_TILE + 256;
+constexpr uint32_t DZ_KBLOCK = 128, DZ_MBLOCK = 2048;     // dZ image: bytes between groups of 8 keys, of 8 queries
 static_assert(BWD_SMEM <= 232448, "over the 227 KB a CTA may use");
 
 struct BwdParams {
@@ -37,9 +29,12 @@ struct BwdParams {
   const float* delta;       // [B,H,T]
   const int* doc_start;     // null or [.,T], batch stride doc_sb
   int64_t doc_sb;
-  __nv_bfloat16 *d0, *d1;   // outputs: MODE 0: dV, dK; MODE 1: (unused), dQ -- [B,T,H,D] contiguous
+  __nv_bfloat16 *d0, *d1;   // outputs: dV, dK; or (unused), dQ -- [B,T,H,D] contiguous
   int T, H, B, window, window_blocks;
   float scale, scale_log2;
+  int bh0, n_bh;            // the launch's (batch, head) pairs: bh0 .. bh0 + n_bh - 1
+  uint8_t* tiles;           // dZ images, [n_bh][query block][tiles_row key blocks] of 32 KB
+  int tiles_row;
   int* status;
 };
 
@@ -49,7 +44,14 @@ struct BwdBars {
   int abort_flag;
 };
 
-// Streamed block range [lo, hi] of an item.
+// First key block that query block `blk` sees, documents aside.
+__device__ __forceinline__ int bwd_first_key_block(int blk, int window, int window_blocks) {
+  if (window_blocks > 0) return max(0, blk - window_blocks + 1);
+  return window > 0 ? max(0, blk * WB - window + 1) / WB : 0;
+}
+
+// Streamed block range [lo, hi] of an item: MODE 0, key block stationary; MODE 1, query block stationary.  Both say the same
+// about a pair of blocks.
 template <int MODE>
 __device__ __forceinline__ void bwd_range(int blk, int nblk, int T, int window, int window_blocks, const int* doc_row, int& lo, int& hi) {
   if (MODE == 0) {                                         // key block blk: query blocks that can see it
@@ -70,36 +72,551 @@ __device__ __forceinline__ void bwd_range(int blk, int nblk, int T, int window, 
     }
   } else {                                                 // query block blk: key blocks inside its window
     hi = blk;
-    int klo = 0;
-    if (window_blocks > 0) klo = max(0, blk - window_blocks + 1) * WB;
-    else if (window > 0) klo = max(0, blk * WB - window + 1);
-    if (doc_row) klo = max(klo, min(doc_row[blk * WB], blk * WB));    // keys before the first row's document: invisible to all
-    lo = klo / WB;
+    lo = bwd_first_key_block(blk, window, window_blocks);
+    if (doc_row) lo = max(lo, min(doc_row[blk * WB], blk * WB) / WB);  // keys before the first row's document: invisible to all
   }
 }
 
-template <int MODE>
+// ---------------------------------------------------------------------------------------------
+// dK, dV: key block stationary.  Item = 128 keys of one (batch, head); K_j, V_j stay in shared memory, the query blocks that can
+// see them stream through.  Scores are formed TRANSPOSED, S^T = K_j Q_i^T and dP^T = V_j dO_i^T (TMEM lane = key), so P^T and
+// dZ^T, rounded to bf16 and written back over them, are exactly the TMEM A operands of dV += P^T dO_i and dK += dZ^T Q_i.
+//
+// The four products of a tile are issued in the order
+//     dV(y)  S(y+1)  dK(y)  dP(y+1)
+// with dV waiting for P(y) and dK for dZ(y).  The tensor core executes one thread's products in order, so S(y+1) overwrites the
+// columns of P(y), and dP(y+1) those of dZ(y), after they have been read, and whichever of P and dZ the workers rebuild, two
+// products of 512 cycles run beside it.  Whole tiles of N = 128: in halves of 64 columns (the form this one replaces) a product
+// reads 6 KB of shared memory in the 32 cycles it should take, at 128 bytes a cycle.
+//
+// 2 x 8192 x 16, window 2048: 684 us in halves -> 486 (tensor pipe 36 -> 53 % of elapsed at 1.62 GHz).  What is left is the workers'
+// chain from S to P; a quarter or half of the exponentials by polynomial changed nothing.  Documents: an item's range takes five
+// dependent reads, which warp 18 does an item ahead (6 documents of 8192 tokens: 737 -> 705 us a round).
+//
+// With a place to put them (`tiles`) the workers also leave dZ_ij as 32 KB operand images, from which swa_bwd_dq_kernel gets
+// dQ_i = scale sum_j dZ_ij K_j with one product a tile instead of three and no exponentials.
+//
+// Roles (608 threads): warps 0-15 rebuild P / dZ -- four warpgroups, thread = TMEM lane (key), 32 of a tile's 128 columns each,
+// every warpgroup writing its bf16 results over the first 16 columns of its OWN 32 -- and write the results; warp 16 TMA
+// producer (Q through three stages, dO, which is spent earlier, through two); warp 17 MMA issuer; warp 18 hands out the items and
+// fetches the streamed rows' scalars and each key's last query.
+constexpr int KV_THREADS = 608, KV_NQ = 3, KV_NO = 2, KV_NI = 3;
+struct KvBars {
+  uint64_t k_full, k_empty, v_full, v_empty, q_full[KV_NQ], q_empty[KV_NQ], o_full[KV_NO], o_empty[KV_NO], c_full[2], c_empty[2], e_full, e_empty, i_full[KV_NI], i_empty[KV_NI];
+  uint64_t s_full, p_full, dp_full, z_full, acc_full, acc_empty;
+  int4 item[KV_NI];         // an item's block (-1: no more), (batch, head), first and last streamed block
+  uint32_t tmem_base;
+  int abort_flag;
+};
+constexpr int KV_TILES = (2 + KV_NQ + KV_NO) * W_TILE;
+constexpr int KV_SMEM = KV_TILES + 2 * 2 * WB * 4 + WB * 4 + (int)sizeof(KvBars);      // tiles, -lse2 and -delta (two stages), ends, barriers
+static_assert(KV_SMEM <= 232448, "over the 227 KB a CTA may use");
+
+// 8 x 8 transpose of 16-byte pieces, or 4 x 4, inside groups of N lanes: afterwards lane l of a group holds piece l of the
+// group's rows, so that a store writes whole row segments
+template <int N>
+__device__ __forceinline__ void exchange_pieces(uint4 (&ch)[N], int lane) {
+#pragma unroll
+  for (int m = N / 2; m >= 1; m >>= 1) {
+    const bool up = (lane & m) != 0;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      if (i & m) continue;
+      const uint4 send = up ? ch[i] : ch[i | m];
+      uint4 recv;
+      recv.x = __shfl_xor_sync(0xffffffffu, send.x, m);
+      recv.y = __shfl_xor_sync(0xffffffffu, send.y, m);
+      recv.z = __shfl_xor_sync(0xffffffffu, send.z, m);
+      recv.w = __shfl_xor_sync(0xffffffffu, send.w, m);
+      if (up) ch[i] = recv; else ch[i | m] = recv;
+    }
+  }
+}
+
+template <bool STORE>
+__global__ void __launch_bounds__(KV_THREADS, 1)
+swa_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                  const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do, const BwdParams p) {
+  extern __shared__ __align__(1024) uint8_t bwd_smem_raw[];          // (the tiles leave no room to align the start by hand)
+  uint8_t* x_tiles = bwd_smem_raw;                                   // K_j, V_j
+  uint8_t* q_tiles = x_tiles + 2 * W_TILE;
+  uint8_t* o_tiles = q_tiles + KV_NQ * W_TILE;
+  float* col_f = reinterpret_cast<float*>(x_tiles + KV_TILES);       // [2][-lse2 | -delta][128]
+  int* ends = reinterpret_cast<int*>(col_f + 2 * 2 * WB);            // each key's first query that no longer sees it
+  KvBars* bars = reinterpret_cast<KvBars*>(ends + WB);
+  volatile int* abort_flag = &bars->abort_flag;
+  if (smem_u32(x_tiles) & 1023) {                                    // never seen; swizzled tiles need it
+    if (threadIdx.x == 0 && p.status) *p.status = DAISY_EALIGN;
+    return;
+  }
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int T = p.T, nblk = (T + WB - 1) / WB;
+  // blocks whose range is cut short by the sequence's end (the last key blocks) go last, longest first
+  const int span = p.window_blocks > 0 ? p.window_blocks * WB : p.window;
+  const BalancedWalk walk(nblk, p.n_bh, span > 0 ? (span + WB - 1) / WB : nblk, true);
+
+  if (threadIdx.x == 0) {
+    mbar_init(&bars->k_full, 1); mbar_init(&bars->k_empty, 1); mbar_init(&bars->v_full, 1); mbar_init(&bars->v_empty, 1);
+    for (int i = 0; i < KV_NQ; ++i) { mbar_init(&bars->q_full[i], 1); mbar_init(&bars->q_empty[i], 1); }
+    for (int i = 0; i < KV_NO; ++i) { mbar_init(&bars->o_full[i], 1); mbar_init(&bars->o_empty[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&bars->c_full[i], 1); mbar_init(&bars->c_empty[i], 16); }
+    mbar_init(&bars->e_full, 1); mbar_init(&bars->e_empty, 16);
+    for (int i = 0; i < KV_NI; ++i) { mbar_init(&bars->i_full[i], 1); mbar_init(&bars->i_empty[i], 18); }   // producer, issuer, workers
+    mbar_init(&bars->s_full, 1); mbar_init(&bars->p_full, 16); mbar_init(&bars->dp_full, 1); mbar_init(&bars->z_full, 16);
+    mbar_init(&bars->acc_full, 1); mbar_init(&bars->acc_empty, 16);
+    bars->abort_flag = 0;
+    mbar_init_fence();
+  }
+  if (warp == 17) { tmem_alloc(&bars->tmem_base, 512); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = bars->tmem_base;
+  grid_dep_launch();
+  grid_dep_wait();
+
+  // the it-th item as warp 18 published it: false when there are no more, or a wait ran out
+  auto next_item = [&](uint32_t it, int4& item) -> bool {
+    const uint32_t s = it % KV_NI;
+    if (!__all_sync(0xffffffffu, mbar_wait(&bars->i_full[s], (it / KV_NI) & 1, abort_flag, p.status, 10))) return false;
+    item = bars->item[s];
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&bars->i_empty[s]);
+    return item.x >= 0;
+  };
+
+  if (warp == 16) {
+    // ------------------------------------------------------------------ TMA producer
+    if (lane == 0) { prefetch_tmap(&tm_q); prefetch_tmap(&tm_k); prefetch_tmap(&tm_v); prefetch_tmap(&tm_do); }
+    uint32_t n = 0;
+    bool ok = true;
+    int4 item;
+    for (uint32_t it = 0; ok && next_item(it, item); ++it) {
+      const int blk = item.x, h = item.y % p.H, b = item.y / p.H, lo = item.z, hi = item.w;
+      if (lane == 0) {
+        auto tile = [&](uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, int y) {
+          mbar_expect_tx(bar, W_TILE);
+          tma_load_4d(dst, tm, bar, 0, y * WB, h, b);
+          tma_load_4d(dst + W_HALF, tm, bar, 64, y * WB, h, b);
+        };
+        // K_j is free after the previous item's last S, V_j after its last dP: both come while that item ends
+        ok = mbar_wait(&bars->k_empty, (it & 1) ^ 1, abort_flag, p.status, 1);
+        if (ok) tile(x_tiles, &tm_k, &bars->k_full, blk);
+        for (int y = lo; ok && y <= hi; ++y, ++n) {
+          const int sq = n % KV_NQ, so = n % KV_NO;
+          if (!(ok = mbar_wait(&bars->q_empty[sq], ((n / KV_NQ) & 1) ^ 1, abort_flag, p.status, 2))) break;
+          tile(q_tiles + sq * W_TILE, &tm_q, &bars->q_full[sq], y);
+          if (y == lo) {
+            if (!(ok = mbar_wait(&bars->v_empty, (it & 1) ^ 1, abort_flag, p.status, 1))) break;
+            tile(x_tiles + W_TILE, &tm_v, &bars->v_full, blk);
+          }
+          if (!(ok = mbar_wait(&bars->o_empty[so], ((n / KV_NO) & 1) ^ 1, abort_flag, p.status, 2))) break;
+          tile(o_tiles + so * W_TILE, &tm_do, &bars->o_full[so], y);
+        }
+      }
+      ok = __all_sync(0xffffffffu, ok);
+    }
+  } else if (warp == 17) {
+    // ------------------------------------------------------------------ MMA issuer
+    const uint32_t leader = elect_one() ? 1u : 0u;
+    constexpr uint32_t idesc_s = umma_idesc_bf16(WB, WB, 0, 0);                   // X Y^T: both K-major
+    constexpr uint32_t idesc_a = umma_idesc_bf16(WB, DAISY_HEAD_DIM, 0, 1);       // (P | dZ from TMEM) x Y: Y as an MN-major operand
+    const uint64_t xd = umma_desc_sw128(smem_u32(x_tiles), 16, 1024), ymn = umma_desc_sw128(smem_u32(q_tiles), W_HALF, 1024);
+    const uint32_t x_lo = (uint32_t)xd, k_hi = (uint32_t)(xd >> 32), mn_hi = (uint32_t)(ymn >> 32);
+    const uint32_t q_lo = (uint32_t)umma_desc_sw128(smem_u32(q_tiles), 16, 1024), o_lo = (uint32_t)umma_desc_sw128(smem_u32(o_tiles), 16, 1024);
+    const uint32_t qmn_lo = (uint32_t)ymn, omn_lo = (uint32_t)umma_desc_sw128(smem_u32(o_tiles), W_HALF, 1024);
+    const uint32_t s_t = tmem_base, dp_t = tmem_base + 128, dv_t = tmem_base + 256, dk_t = tmem_base + 384;
+    auto score = [&](uint32_t d, uint32_t x, uint32_t y) {
+#pragma unroll
+      for (int k = 0; k < DAISY_HEAD_DIM / 16; ++k) {
+        const uint32_t off = ((k >> 2) * W_HALF + (k & 3) * 32) >> 4;
+        umma_ss_lh_p(leader, d, x + off, k_hi, y + off, k_hi, idesc_s, k > 0 ? 1u : 0u);
+      }
+    };
+    auto accumulate = [&](uint32_t d, uint32_t a, uint32_t y, uint32_t acc) {
+#pragma unroll
+      for (int k = 0; k < WB / 16; ++k)
+        umma_ts_lh_p(leader, d, a + (k & 1) * 8 + (k >> 1) * 32, y + k * (2048 >> 4), mn_hi, idesc_a, (acc || k > 0) ? 1u : 0u);
+    };
+    uint32_t n = 0;
+    bool ok = true;
+    int4 item;
+    for (uint32_t it = 0; ok && next_item(it, item); ++it) {
+      const int lo = item.z, hi = item.w;
+      if (!mbar_wait(&bars->k_full, it & 1, abort_flag, p.status, 3)) break;
+      if (!mbar_wait(&bars->q_full[n % KV_NQ], (n / KV_NQ) & 1, abort_flag, p.status, 4)) break;
+      tc_fence_after();
+      score(s_t, x_lo, q_lo + (n % KV_NQ) * (W_TILE >> 4));
+      tc_commit_p(leader, &bars->s_full);
+      if (lo == hi) tc_commit_p(leader, &bars->k_empty);
+      if (!mbar_wait(&bars->v_full, it & 1, abort_flag, p.status, 3)) break;
+      if (!mbar_wait(&bars->o_full[n % KV_NO], (n / KV_NO) & 1, abort_flag, p.status, 4)) break;
+      tc_fence_after();
+      score(dp_t, x_lo + (W_TILE >> 4), o_lo + (n % KV_NO) * (W_TILE >> 4));
+      tc_commit_p(leader, &bars->dp_full);
+      if (lo == hi) tc_commit_p(leader, &bars->v_empty);
+      // the first accumulating products overwrite the accumulators: the workers have read out the previous item's
+      if (!mbar_wait(&bars->acc_empty, (it & 1) ^ 1, abort_flag, p.status, 8)) break;
+      for (int y = lo; y <= hi; ++y, ++n) {
+        const uint32_t sq = n % KV_NQ, so = n % KV_NO, sq1 = (n + 1) % KV_NQ, so1 = (n + 1) % KV_NO;
+        const bool more = y < hi;
+        if (!mbar_wait(&bars->p_full, n & 1, abort_flag, p.status, 5)) { ok = false; break; }
+        tc_fence_after();
+        accumulate(dv_t, s_t, omn_lo + so * (W_TILE >> 4), y > lo);               // dV += P^T dO
+        tc_commit_p(leader, &bars->o_empty[so]);
+        if (more) {
+          if (!mbar_wait(&bars->q_full[sq1], ((n + 1) / KV_NQ) & 1, abort_flag, p.status, 4)) { ok = false; break; }
+          tc_fence_after();
+          score(s_t, x_lo, q_lo + sq1 * (W_TILE >> 4));
+          tc_commit_p(leader, &bars->s_full);
+          if (y + 1 == hi) tc_commit_p(leader, &bars->k_empty);
+        }
+        if (!mbar_wait(&bars->z_full, n & 1, abort_flag, p.status, 5)) { ok = false; break; }
+        tc_fence_after();
+        accumulate(dk_t, dp_t, qmn_lo + sq * (W_TILE >> 4), y > lo);              // dK += dZ^T Q
+        tc_commit_p(leader, &bars->q_empty[sq]);
+        if (more) {
+          if (!mbar_wait(&bars->o_full[so1], ((n + 1) / KV_NO) & 1, abort_flag, p.status, 4)) { ok = false; break; }
+          tc_fence_after();
+          score(dp_t, x_lo + (W_TILE >> 4), o_lo + so1 * (W_TILE >> 4));
+          tc_commit_p(leader, &bars->dp_full);
+          if (y + 1 == hi) tc_commit_p(leader, &bars->v_empty);
+        } else {
+          tc_commit_p(leader, &bars->acc_full);
+        }
+      }
+    }
+  } else if (warp == 18) {
+    // ------------------------------------------------------------------ items, one ahead; scalars: four keys and four streamed queries a lane
+    uint32_t n = 0;
+    bool ok = true;
+    int4 item;
+    int end[4];
+    auto publish = [&](uint32_t it) -> bool {                         // item `it` and its keys' ends
+      const int at = walk.at((int)it);
+      item = make_int4(at < 0 ? -1 : at % nblk, at < 0 ? 0 : p.bh0 + at / nblk, 0, 0);
+      const int* doc_row = p.doc_start ? p.doc_start + item.y / p.H * p.doc_sb : nullptr;
+      if (at >= 0) bwd_range<0>(item.x, nblk, T, p.window, p.window_blocks, doc_row, item.z, item.w);
+      const uint32_t s = it % KV_NI;
+      if (!__all_sync(0xffffffffu, mbar_wait(&bars->i_empty[s], ((it / KV_NI) & 1) ^ 1, abort_flag, p.status, 9))) return false;
+      if (lane == 0) { bars->item[s] = item; mbar_arrive(&bars->i_full[s]); }
+      if (at < 0) return true;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int k = item.x * WB + lane + 32 * e;
+        int c = min(T, (item.w + 1) * WB);
+        if (p.window_blocks <= 0 && p.window > 0) c = min(c, k + min(p.window, T));
+        if (doc_row) {                                                // doc_start does not decrease: bisect for the first query of a later document
+          int a = k + 1;
+          while (a < c) {
+            const int m = (a + c) >> 1;
+            if (__ldg(doc_row + m) > k) c = m; else a = m + 1;
+          }
+        }
+        end[e] = k < T ? c : 0;
+      }
+      return true;
+    };
+    ok = publish(0);
+    for (uint32_t it = 0; ok && item.x >= 0; ++it) {
+      ok = __all_sync(0xffffffffu, mbar_wait(&bars->e_empty, (it & 1) ^ 1, abort_flag, p.status, 9));
+      if (!ok) break;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) ends[lane + 32 * e] = end[e];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars->e_full);
+      const float *lse = p.lse2 + (int64_t)item.y * T, *delta = p.delta + (int64_t)item.y * T;
+      const int lo = item.z, hi = item.w;
+      for (int y = lo; y <= hi; ++y, ++n) {
+        float l[4], d[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int q = y * WB + lane + 32 * e;
+          l[e] = q < T ? -__ldg(lse + q) : 0.f; d[e] = q < T ? -__ldg(delta + q) : 0.f;
+        }
+        ok = __all_sync(0xffffffffu, mbar_wait(&bars->c_empty[n & 1], ((n >> 1) & 1) ^ 1, abort_flag, p.status, 9));
+        if (!ok) break;
+        float* cf = col_f + (n & 1) * 2 * WB;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { cf[lane + 32 * e] = l[e]; cf[WB + lane + 32 * e] = d[e]; }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->c_full[n & 1]);
+        if (y == lo && !(ok = publish(it + 1))) break;                // in the shadow of this item
+      }
+    }
+  } else {
+    // ------------------------------------------------------------------ P / dZ rebuild and epilogue: thread = TMEM lane = key
+    const int grp = warp >> 2, quarter = warp & 3;                    // which 32 columns; which 32 TMEM lanes
+    const int row = quarter * 32 + lane;
+    const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
+    const uint32_t s_t = tmem_base + lane_off + 32 * grp, dp_t = s_t + 128;        // this thread's 32 S and 32 dP columns
+    const uint32_t a0_t = tmem_base + lane_off + 256 + 32 * grp, a1_t = a0_t + 128;    // and its 32 output columns of each accumulator
+    const uint64_t c2 = pack2f(p.scale_log2, p.scale_log2);
+    uint32_t n = 0;
+    bool ok = true;
+    int4 item;
+    for (uint32_t it = 0; ok && next_item(it, item); ++it) {
+      const int blk = item.x, h = item.y % p.H, b = item.y / p.H, lo = item.z, hi = item.w;
+      const int k = blk * WB + row;
+      ok = __all_sync(0xffffffffu, mbar_wait(&bars->e_full, it & 1, abort_flag, p.status, 6));
+      if (!ok) break;
+      const int end = ends[row], first_end = ends[0];                 // ends do not decrease with the key
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars->e_empty);
+      for (int y = lo; y <= hi; ++y, ++n) {
+        const float* cf = col_f + (n & 1) * 2 * WB + 32 * grp;
+        const int y0 = y * WB;
+        // is every (key, query) pair of this tile visible?
+        const bool full = blk * WB + WB - 1 <= y0 && y0 + WB <= first_end;
+        // and which of this thread's 32: queries k .. end - 1
+        const int v_lo = min(max(k - y0 - 32 * grp, 0), 32), v_hi = min(max(end - y0 - 32 * grp, 0), 32);
+        const uint32_t visible = (uint32_t)(((uint64_t)1 << v_hi) - 1) & ~(uint32_t)(((uint64_t)1 << v_lo) - 1);
+        ok = __all_sync(0xffffffffu, mbar_wait(&bars->c_full[n & 1], (n >> 1) & 1, abort_flag, p.status, 6) &&
+                                     mbar_wait(&bars->s_full, n & 1, abort_flag, p.status, 6));
+        if (!ok) break;
+        tc_fence_after();
+        uint64_t pv[16];                                              // P, fp32 pairs
+        {
+          uint32_t r[32], pp[16];
+          tmem_ld32(s_t, r);
+          tc_wait_ld();
+#pragma unroll
+          for (int i = 0; i < 32; i += 4) {
+            float l[4];
+            *reinterpret_cast<float4*>(l) = *reinterpret_cast<const float4*>(cf + i);
+            float x[4];
+            unpack2f(ffma2(pack2f(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), c2, pack2f(l[0], l[1])), x[0], x[1]);
+            unpack2f(ffma2(pack2f(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 3])), c2, pack2f(l[2], l[3])), x[2], x[3]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) x[e] = fast_exp2(x[e]);
+            if (!full) {
+#pragma unroll
+              for (int e = 0; e < 4; ++e)
+                if (!((visible >> (i + e)) & 1u)) x[e] = 0.f;
+            }
+            pp[i >> 1] = pack_bf16(x[0], x[1]); pp[(i >> 1) + 1] = pack_bf16(x[2], x[3]);
+            pv[i >> 1] = pack2f(x[0], x[1]); pv[(i >> 1) + 1] = pack2f(x[2], x[3]);
+          }
+          tmem_st16(s_t, pp);
+        }
+        tc_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->p_full);
+        ok = __all_sync(0xffffffffu, mbar_wait(&bars->dp_full, n & 1, abort_flag, p.status, 6));
+        if (!ok) break;
+        tc_fence_after();
+        uint32_t pz[16];
+        {
+          uint32_t r[32];
+          tmem_ld32(dp_t, r);
+          tc_wait_ld();
+#pragma unroll
+          for (int i = 0; i < 32; i += 4) {
+            float d[4], z[4];
+            *reinterpret_cast<float4*>(d) = *reinterpret_cast<const float4*>(cf + WB + i);
+            unpack2f(fmul2(pv[i >> 1], fadd2(pack2f(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), pack2f(d[0], d[1]))), z[0], z[1]);
+            unpack2f(fmul2(pv[(i >> 1) + 1], fadd2(pack2f(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 3])), pack2f(d[2], d[3]))), z[2], z[3]);
+            pz[i >> 1] = pack_bf16(z[0], z[1]); pz[(i >> 1) + 1] = pack_bf16(z[2], z[3]);
+          }
+          tmem_st16(dp_t, pz);
+        }
+        tc_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) { mbar_arrive(&bars->z_full); mbar_arrive(&bars->c_empty[n & 1]); }
+        if (STORE) {
+          uint8_t* dst = p.tiles + ((int64_t)((item.y - p.bh0) * nblk + y) * p.tiles_row + blk - bwd_first_key_block(y, p.window, p.window_blocks)) * W_TILE +
+                         grp * 4 * DZ_MBLOCK + row * 16;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(dst + j * DZ_MBLOCK) = make_uint4(pz[4 * j], pz[4 * j + 1], pz[4 * j + 2], pz[4 * j + 3]);
+        }
+      }
+      // ---- epilogue: the item's accumulators -> global rows, 64 bytes of eight rows a store
+      if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&bars->acc_full, it & 1, abort_flag, p.status, 7));
+      if (!ok) break;
+      tc_fence_after();
+#pragma unroll 1
+      for (int which = 0; which < 2; ++which) {
+        const float sc = which == 0 ? 1.f : p.scale;
+        uint32_t r[32];
+        tmem_ld32(which == 0 ? a0_t : a1_t, r);
+        tc_wait_ld();
+        if (which == 1) {                                             // the next item's first accumulating products overwrite what was just read
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars->acc_empty);
+        }
+        uint4 ch[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          float f[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(r[8 * i + e]) * sc;
+          ch[i] = pack8(f);
+        }
+        exchange_pieces(ch, lane);
+        const int k0 = k & ~3;
+        __nv_bfloat16* dst = (which == 0 ? p.d0 : p.d1) + (((int64_t)b * T + k0) * p.H + h) * DAISY_HEAD_DIM + 32 * grp + 8 * (lane & 3);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (k0 + i < T) *reinterpret_cast<uint4*>(dst + (int64_t)i * p.H * DAISY_HEAD_DIM) = ch[i];
+      }
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 17) { tc_fence_after(); tmem_dealloc(tmem_base, 512); }
+}
+
+// ---------------------------------------------------------------------------------------------
+// dQ_i = scale sum_j dZ_ij K_j from the images swa_bwd_kv_kernel left: a banded product that reads each image once.  Item = 128
+// queries of one (batch, head).  Warps 0-3 write the results out of one of two accumulators, warp 4 keeps three stages of
+// (dZ_ij, K_j) full, warp 5 issues.  The images are read as MN-major operands without a swizzle: core matrices of 8 keys x 8
+// queries in 128 contiguous bytes, which is also how 32 lanes (keys) write 512 contiguous bytes at a time.
+// HBM-bound: 6.5 TB/s of the images.  2 x 8192 x 16, window 2048: 176 us, where forming the scores again takes 408.
+constexpr int DQ_THREADS = 192, DQ_NST = 3;
+struct DqBars {
+  uint64_t full[DQ_NST], empty[DQ_NST], acc_full[2], acc_empty[2];
+  uint32_t tmem_base;
+  int abort_flag;
+};
+constexpr int DQ_SMEM = 1024 + DQ_NST * 2 * W_TILE + (int)sizeof(DqBars);
+
+__global__ void __launch_bounds__(DQ_THREADS, 1) swa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_k, const BwdParams p) {
+  extern __shared__ __align__(1024) uint8_t bwd_smem_raw[];
+  uint8_t* stages = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(bwd_smem_raw) + 1023) & ~uintptr_t(1023));
+  DqBars* bars = reinterpret_cast<DqBars*>(stages + DQ_NST * 2 * W_TILE);
+  volatile int* abort_flag = &bars->abort_flag;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int T = p.T, nblk = (T + WB - 1) / WB;
+  const int span = p.window_blocks > 0 ? p.window_blocks * WB : p.window;
+  const BalancedWalk walk(nblk, p.n_bh, span > 0 ? (span + WB - 1) / WB : nblk, false);
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < DQ_NST; ++i) { mbar_init(&bars->full[i], 1); mbar_init(&bars->empty[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&bars->acc_full[i], 1); mbar_init(&bars->acc_empty[i], 4); }
+    bars->abort_flag = 0;
+    mbar_init_fence();
+  }
+  if (warp == 5) { tmem_alloc(&bars->tmem_base, 256); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = bars->tmem_base;
+  grid_dep_launch();
+  grid_dep_wait();
+
+  if (warp == 4) {
+    if (lane == 0) {
+      prefetch_tmap(&tm_k);
+      uint32_t n = 0, it = 0;
+      bool ok = true;
+      for (int item; (item = walk.at((int)it)) >= 0 && ok; ++it) {
+        const int blk = item % nblk, bh = p.bh0 + item / nblk, h = bh % p.H, b = bh / p.H;
+        int lo, hi;
+        bwd_range<1>(blk, nblk, T, p.window, p.window_blocks, p.doc_start ? p.doc_start + b * p.doc_sb : nullptr, lo, hi);
+        const uint8_t* row = p.tiles + ((int64_t)item * p.tiles_row - bwd_first_key_block(blk, p.window, p.window_blocks)) * W_TILE;
+        for (int y = lo; y <= hi; ++y, ++n) {
+          const int st = n % DQ_NST;
+          if (!mbar_wait(&bars->empty[st], ((n / DQ_NST) & 1) ^ 1, abort_flag, p.status, 2)) { ok = false; break; }
+          uint8_t* dst = stages + st * 2 * W_TILE;
+          mbar_expect_tx(&bars->full[st], 2 * W_TILE);
+          asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                       ::"r"(smem_u32(dst)), "l"(row + (int64_t)y * W_TILE), "r"(W_TILE), "r"(smem_u32(&bars->full[st])) : "memory");
+          tma_load_4d(dst + W_TILE, &tm_k, &bars->full[st], 0, y * WB, h, b);
+          tma_load_4d(dst + W_TILE + W_HALF, &tm_k, &bars->full[st], 64, y * WB, h, b);
+        }
+      }
+    }
+  } else if (warp == 5) {
+    const uint32_t leader = elect_one() ? 1u : 0u;
+    constexpr uint32_t idesc = umma_idesc_bf16(WB, DAISY_HEAD_DIM, 1, 1);         // both MN-major
+    const uint64_t zd = umma_desc_plain(smem_u32(stages), DZ_KBLOCK, DZ_MBLOCK), kd = umma_desc_sw128(smem_u32(stages) + W_TILE, W_HALF, 1024);
+    const uint32_t z_hi = (uint32_t)(zd >> 32), k_hi = (uint32_t)(kd >> 32);
+    uint32_t n = 0, it = 0;
+    bool ok = true;
+    for (int item; (item = walk.at((int)it)) >= 0 && ok; ++it) {
+      const int blk = item % nblk, b = (p.bh0 + item / nblk) / p.H;
+      int lo, hi;
+      bwd_range<1>(blk, nblk, T, p.window, p.window_blocks, p.doc_start ? p.doc_start + b * p.doc_sb : nullptr, lo, hi);
+      if (!mbar_wait(&bars->acc_empty[it & 1], ((it >> 1) & 1) ^ 1, abort_flag, p.status, 8)) break;
+      for (int y = lo; y <= hi; ++y, ++n) {
+        const uint32_t st = n % DQ_NST, off = st * ((2 * W_TILE) >> 4);
+        if (!mbar_wait(&bars->full[st], (n / DQ_NST) & 1, abort_flag, p.status, 4)) { ok = false; break; }
+        tc_fence_after();
+#pragma unroll
+        for (int k = 0; k < WB / 16; ++k)
+          umma_ss_lh_p(leader, tmem_base + 128 * (it & 1), (uint32_t)zd + off + k * ((2 * DZ_KBLOCK) >> 4), z_hi, (uint32_t)kd + off + k * (2048 >> 4), k_hi,
+                       idesc, (y > lo || k > 0) ? 1u : 0u);
+        tc_commit_p(leader, &bars->empty[st]);
+      }
+      if (ok) tc_commit_p(leader, &bars->acc_full[it & 1]);
+    }
+  } else {
+    const int row = 32 * warp + lane;
+    uint32_t it = 0;
+    for (int item; (item = walk.at((int)it)) >= 0; ++it) {
+      const int blk = item % nblk, bh = p.bh0 + item / nblk, h = bh % p.H, b = bh / p.H;
+      if (!__all_sync(0xffffffffu, mbar_wait(&bars->acc_full[it & 1], (it >> 1) & 1, abort_flag, p.status, 7))) break;
+      tc_fence_after();
+      const int q0 = blk * WB + (row & ~7);
+#pragma unroll 1
+      for (int half = 0; half < 2; ++half) {
+        uint32_t r[64];
+        tmem_ld32(tmem_base + ((uint32_t)(32 * warp) << 16) + 128 * (it & 1) + 64 * half, r);
+        tmem_ld32(tmem_base + ((uint32_t)(32 * warp) << 16) + 128 * (it & 1) + 64 * half + 32, r + 32);
+        tc_wait_ld();
+        if (half == 1) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars->acc_empty[it & 1]);
+        }
+        uint4 ch[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          float f[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(r[8 * i + e]) * p.scale;
+          ch[i] = pack8(f);
+        }
+        exchange_pieces(ch, lane);
+        __nv_bfloat16* dst = p.d1 + (((int64_t)b * T + q0) * p.H + h) * DAISY_HEAD_DIM + 64 * half + 8 * (lane & 7);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          if (q0 + i < T) *reinterpret_cast<uint4*>(dst + (int64_t)i * p.H * DAISY_HEAD_DIM) = ch[i];
+      }
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 5) { tc_fence_after(); tmem_dealloc(tmem_base, 256); }
+}
+
+// ---------------------------------------------------------------------------------------------
+// dQ without the images: query block stationary.  Item = 128 queries; Q_i, dO_i stay, the key blocks of the window stream (K_j,
+// V_j);  S = Q_i K_j^T, dP = dO_i V_j^T (TMEM lane = query),  dQ += dZ K_j.  576 threads: warps 0-15 rebuild dZ (four
+// warpgroups, thread = TMEM lane, 32 of a tile's 128 columns each) and write the results; warp 16 TMA producer, warp 17 MMA
+// issuer.  TMEM: S [0,128) dP [128,256) dQ [384,512).
 __global__ void __launch_bounds__(BWD_THREADS, 1)
-swa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+swa_bwd_q_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do, const BwdParams p) {
-  extern __shared__ uint8_t bwd_smem_raw[];
+  extern __shared__ __align__(1024) uint8_t bwd_smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(bwd_smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* x_tiles = smem;                                           // X0, X1
   uint8_t* y_tiles = smem + 2 * W_TILE;                              // per stage: Y0, Y1
-  float* col_f = reinterpret_cast<float*>(y_tiles + W_NST * 2 * W_TILE);   // MODE 0: [2][lse2 | delta | doc_start][128]
-  BwdBars* bars = reinterpret_cast<BwdBars*>(reinterpret_cast<uint8_t*>(col_f) + 2 * 3 * WB * 4);
+  BwdBars* bars = reinterpret_cast<BwdBars*>(y_tiles + W_NST * 2 * W_TILE);
   volatile int* abort_flag = &bars->abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int T = p.T, nblk = (T + WB - 1) / WB;
-  // blocks whose range is cut short by the sequence's end (MODE 0: the last key blocks) or start (MODE 1: the first
-  // query blocks) go last, longest first
+  // blocks whose range is cut short by the sequence's start (the first query blocks) go last, longest first
   const int span = p.window_blocks > 0 ? p.window_blocks * WB : p.window;
-  const BalancedWalk walk(nblk, p.H * p.B, span > 0 ? (span + WB - 1) / WB : nblk, MODE == 0);
-  const CUtensorMap* tx0 = MODE == 0 ? &tm_k : &tm_q;
-  const CUtensorMap* tx1 = MODE == 0 ? &tm_v : &tm_do;
-  const CUtensorMap* ty0 = MODE == 0 ? &tm_q : &tm_k;
-  const CUtensorMap* ty1 = MODE == 0 ? &tm_do : &tm_v;
+  const BalancedWalk walk(nblk, p.H * p.B, span > 0 ? (span + WB - 1) / WB : nblk, false);
+  const CUtensorMap *tx0 = &tm_q, *tx1 = &tm_do, *ty0 = &tm_k, *ty1 = &tm_v;
 
   if (threadIdx.x == 0) {
     mbar_init(&bars->x_full, 1); mbar_init(&bars->x_empty, 1);
@@ -114,6 +631,8 @@ swa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
+  grid_dep_launch();
+  grid_dep_wait();
 
   if (warp == 16) {
     // ------------------------------------------------------------------ TMA producer
@@ -124,7 +643,7 @@ swa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       for (int item; (item = walk.at((int)it)) >= 0 && ok; ++it) {
         const int blk = item % nblk, bh = item / nblk, h = bh % p.H, b = bh / p.H;
         int lo, hi;
-        bwd_range<MODE>(blk, nblk, T, p.window, p.window_blocks, p.doc_start ? p.doc_start + b * p.doc_sb : nullptr, lo, hi);
+        bwd_range<1>(blk, nblk, T, p.window, p.window_blocks, p.doc_start ? p.doc_start + b * p.doc_sb : nullptr, lo, hi);
         if (!mbar_wait(&bars->x_empty, (it & 1) ^ 1, abort_flag, p.status, 1)) { ok = false; break; }
         mbar_expect_tx(&bars->x_full, 2 * W_TILE);
         tma_load_4d(x_tiles, tx0, &bars->x_full, 0, blk * WB, h, b);
@@ -146,21 +665,21 @@ swa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   } else if (warp == 17) {
     // ------------------------------------------------------------------ MMA issuer
     // The score tiles are formed and consumed in two halves of 64 streamed rows (= 64 TMEM columns), two worker
-    // warpgroups each, and the halves are software-pipelined: while the warpgroups of a half rebuild its P / dZ, the tensor core
+    // warpgroups each, and the halves are software-pipelined: while the warpgroups of a half rebuild its dZ, the tensor core
     // forms the other half's scores, accumulates the previous half's products and already forms the NEXT tile's
     // scores of a half as soon as that half's columns have been consumed:
-    //   S0(y) S1(y) | wait P0(y): A0(y) S0(y+1) | wait P1(y): A1(y) S1(y+1) | wait P0(y+1): ...
-    // (S = both score products of a half, A = both accumulating products).  tcgen05 MMAs of one thread execute in
+    //   S0(y) S1(y) | wait dZ0(y): A0(y) S0(y+1) | wait dZ1(y): A1(y) S1(y+1) | wait dZ0(y+1): ...
+    // (S = both score products of a half, A = the accumulating product).  tcgen05 MMAs of one thread execute in
     // order, so S_h(y+1) overwrites columns that A_h(y) has finished reading.
     const uint32_t leader = elect_one() ? 1u : 0u;
     constexpr uint32_t idesc_s = umma_idesc_bf16(WB, WB / 2, 0, 0);               // X Y_half^T: both K-major, 64 streamed rows
-    constexpr uint32_t idesc_a = umma_idesc_bf16(WB, DAISY_HEAD_DIM, 0, 1);       // (P | dZ from TMEM) x Y: Y as an MN-major operand
+    constexpr uint32_t idesc_a = umma_idesc_bf16(WB, DAISY_HEAD_DIM, 0, 1);       // dZ (from TMEM) x Y: Y as an MN-major operand
     const uint64_t xd = umma_desc_sw128(smem_u32(x_tiles), 16, 1024);
     const uint64_t yd = umma_desc_sw128(smem_u32(y_tiles), 16, 1024);
     const uint64_t ymn = umma_desc_sw128(smem_u32(y_tiles), W_HALF, 1024);
     const uint32_t x_lo0 = (uint32_t)xd, y_lo0 = (uint32_t)yd, k_hi = (uint32_t)(xd >> 32);
     const uint32_t ymn_lo0 = (uint32_t)ymn, ymn_hi = (uint32_t)(ymn >> 32);
-    const uint32_t s_t = tmem_base, dp_t = tmem_base + 128, a0_t = tmem_base + 256, a1_t = tmem_base + 384;
+    const uint32_t s_t = tmem_base, dp_t = tmem_base + 128, a1_t = tmem_base + 384;
     uint32_t n = 0, it = 0;
     bool ok = true;
     // both score products of half hf of the tile in stage st
@@ -178,22 +697,17 @@ swa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       }
       tc_commit_p(leader, &bars->s_full[hf]);
     };
-    // both accumulating products over the 64 streamed rows of half hf
+    // the accumulating product over the 64 streamed rows of half hf
     auto accumulate = [&](int st, int hf, uint32_t acc) {
-      const uint32_t ymn0 = ymn_lo0 + st * ((2 * W_TILE) >> 4), ymn1 = ymn0 + (W_TILE >> 4);
-      if (MODE == 0) {
+      const uint32_t ymn0 = ymn_lo0 + st * ((2 * W_TILE) >> 4);
 #pragma unroll
-        for (int k = 4 * hf; k < 4 * hf + 4; ++k)                               // acc0 += P Y1   (dV += P^T dO)
-          umma_ts_lh_p(leader, a0_t, s_t + (k & 1) * 8 + (k >> 1) * 32, ymn1 + k * (2048 >> 4), ymn_hi, idesc_a, (acc || k > 4 * hf) ? 1u : 0u);
-      }
-#pragma unroll
-      for (int k = 4 * hf; k < 4 * hf + 4; ++k)                                 // acc1 += dZ Y0  (dK += dZ^T Q | dQ += dZ K)
+      for (int k = 4 * hf; k < 4 * hf + 4; ++k)                                 // dQ += dZ K
         umma_ts_lh_p(leader, a1_t, dp_t + (k & 1) * 8 + (k >> 1) * 32, ymn0 + k * (2048 >> 4), ymn_hi, idesc_a, (acc || k > 4 * hf) ? 1u : 0u);
     };
     for (int item; (item = walk.at((int)it)) >= 0 && ok; ++it) {
       const int blk = item % nblk, bh = item / nblk, b = bh / p.H;
       int lo, hi;
-      bwd_range<MODE>(blk, nblk, T, p.window, p.window_blocks, p.doc_start ? p.doc_start + b * p.doc_sb : nullptr, lo, hi);
+      bwd_range<1>(blk, nblk, T, p.window, p.window_blocks, p.doc_start ? p.doc_start + b * p.doc_sb : nullptr, lo, hi);
       if (!mbar_wait(&bars->x_full, it & 1, abort_flag, p.status, 3)) { ok = false; break; }
       // the item's first tile
       if (!mbar_wait(&bars->y_full[n % W_NST], (n / W_NST) & 1, abort_flag, p.status, 4)) { ok = false; break; }
@@ -223,13 +737,13 @@ swa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       }
     }
   } else {
-    // ------------------------------------------------------------------ P / dZ rebuild and epilogue: thread = TMEM lane
+    // ------------------------------------------------------------------ dZ rebuild and epilogue: thread = TMEM lane
     const int grp = warp >> 2, quarter = warp & 3;                    // which 32 columns; which 32 TMEM lanes
     const int half = grp >> 1;                                        // the 64-column half whose barriers this warpgroup uses
     const int row = quarter * 32 + lane;
     const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
     const uint32_t s_t = tmem_base + lane_off + 32 * grp, dp_t = s_t + 128;        // this thread's 32 S and 32 dP columns
-    const uint32_t a0_t = tmem_base + lane_off + 256 + 32 * grp, a1_t = a0_t + 128;    // and its 32 output columns of each accumulator
+    const uint32_t a1_t = tmem_base + lane_off + 384 + 32 * grp;                    // and its 32 output columns
     const float c2 = p.scale_log2;
     uint32_t n = 0, it = 0;
     bool ok = true;
@@ -237,88 +751,44 @@ swa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       const int blk = item % nblk, bh = item / nblk, h = bh % p.H, b = bh / p.H;
       const int* doc_row = p.doc_start ? p.doc_start + b * p.doc_sb : nullptr;
       int lo, hi;
-      bwd_range<MODE>(blk, nblk, T, p.window, p.window_blocks, doc_row, lo, hi);
+      bwd_range<1>(blk, nblk, T, p.window, p.window_blocks, doc_row, lo, hi);
       const int64_t rowbase = ((int64_t)b * p.H + h) * T;
-      const int xr = blk * WB + row;                                  // this lane's key (MODE 0) or query (MODE 1)
+      const int xr = blk * WB + row;                                  // this lane's query
       float my_lse = 0.f, my_delta = 0.f;
       int my_doc = 0;
-      if (MODE == 1 && xr < T) {
+      if (xr < T) {
         my_lse = p.lse2[rowbase + xr]; my_delta = p.delta[rowbase + xr];
         my_doc = doc_row ? min(doc_row[xr], xr) : 0;
       }
       for (int y = lo; y <= hi; ++y, ++n) {
-        float* cf = col_f + (n & 1) * 3 * WB;
-        if (MODE == 0) {                                              // the streamed queries' scalars, shared by all lanes
-          if (grp == 0) {
-            const int q = y * WB + row;
-            cf[row] = q < T ? p.lse2[rowbase + q] : 0.f;
-            cf[WB + row] = q < T ? p.delta[rowbase + q] : 0.f;
-            reinterpret_cast<int*>(cf)[2 * WB + row] = (doc_row && q < T) ? min(doc_row[q], q) : 0;
-          }
-          // the eight warps leave together: a warp that gave up still comes here, and everybody learns of it
-          if (named_bar_or(1, BWD_WORKERS, !ok)) { ok = false; break; }
-        }
         ok = __all_sync(0xffffffffu, mbar_wait(&bars->s_full[half], n & 1, abort_flag, p.status, 6));
-        if (!ok) { if (MODE == 0) continue; else break; }
+        if (!ok) break;
         tc_fence_after();
         const int y0 = y * WB;
         // is every (lane, column) pair of this tile pair visible?
-        bool full;
-        if (MODE == 0) {
-          full = (blk * WB + WB - 1 <= y0) && (y0 + WB - 1 < T) && (p.window_blocks > 0 || p.window <= 0 || y0 + WB - 1 - blk * WB < p.window) &&
-                 (!doc_row || doc_row[min(y0 + WB - 1, T - 1)] <= blk * WB);
-        } else {
-          full = (y0 + WB - 1 <= blk * WB) && (p.window_blocks > 0 || p.window <= 0 || blk * WB + WB - 1 - y0 < p.window) &&
-                 (!doc_row || doc_row[min(blk * WB + WB - 1, T - 1)] <= y0);
-        }
+        const bool full = (y0 + WB - 1 <= blk * WB) && (p.window_blocks > 0 || p.window <= 0 || blk * WB + WB - 1 - y0 < p.window) &&
+                          (!doc_row || doc_row[min(blk * WB + WB - 1, T - 1)] <= y0);
         {                                                             // the results go back over the first 16 of the 32 columns
           uint32_t rs[32], rd[32];
           tmem_ld32(s_t, rs);
           tmem_ld32(dp_t, rd);
           tc_wait_ld();
-          uint32_t pp[16], pz[16];
+          uint32_t pz[16];
+          const uint64_t nl = pack2f(-my_lse, -my_lse), nd = pack2f(-my_delta, -my_delta);
 #pragma unroll
-          for (int i = 0; i < 32; i += 4) {
-            const int col0 = 32 * grp + i;
-            float lse4[4], dl4[4];
-            int doc4[4] = {0, 0, 0, 0};
-            if (MODE == 0) {                                          // four columns' scalars per shared-memory load
-              *reinterpret_cast<float4*>(lse4) = *reinterpret_cast<const float4*>(cf + col0);
-              *reinterpret_cast<float4*>(dl4) = *reinterpret_cast<const float4*>(cf + WB + col0);
-              if (!full) *reinterpret_cast<int4*>(doc4) = *reinterpret_cast<const int4*>(reinterpret_cast<const int*>(cf) + 2 * WB + col0);
+          for (int i = 0; i < 32; i += 2) {                           // two columns per packed instruction: x = S c2 - lse, then dZ = P (dP - delta)
+            float x0, x1, z0, z1;
+            unpack2f(ffma2(pack2f(__uint_as_float(rs[i]), __uint_as_float(rs[i + 1])), pack2f(c2, c2), nl), x0, x1);
+            float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
+            if (!full) {
+              const int q = xr, k = y0 + 32 * grp + i;
+              const int klo = max(my_doc, p.window_blocks > 0 || p.window <= 0 ? 0 : q - p.window + 1);
+              if (k > q || k < klo) p0 = 0.f;
+              if (k + 1 > q || k + 1 < klo) p1 = 0.f;
             }
-            float pv[4], zv[4];
-            // two columns per packed instruction: x = S c2 - lse, then dZ = P (dP - delta)
-#pragma unroll
-            for (int e = 0; e < 4; e += 2) {
-              const float l0 = MODE == 0 ? lse4[e] : my_lse, l1 = MODE == 0 ? lse4[e + 1] : my_lse;
-              const float d0 = MODE == 0 ? dl4[e] : my_delta, d1 = MODE == 0 ? dl4[e + 1] : my_delta;
-              float x0, x1;
-              unpack2f(ffma2(pack2f(__uint_as_float(rs[i + e]), __uint_as_float(rs[i + e + 1])), pack2f(c2, c2), pack2f(-l0, -l1)), x0, x1);
-              float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
-              if (!full) {
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                  const int col = col0 + e + u;
-                  bool vis;
-                  if (MODE == 0) {
-                    const int q = y0 + col, k = xr;
-                    vis = (k <= q) && (q < T) && (p.window_blocks > 0 || p.window <= 0 || q - k < p.window) && (k >= doc4[e + u]);
-                  } else {
-                    const int q = xr, k = y0 + col;
-                    vis = (k <= q) && (p.window_blocks > 0 || p.window <= 0 || q - k < p.window) && (k >= my_doc);
-                  }
-                  if (!vis) { if (u == 0) p0 = 0.f; else p1 = 0.f; }
-                }
-              }
-              pv[e] = p0; pv[e + 1] = p1;
-              unpack2f(fmul2(pack2f(p0, p1), fadd2(pack2f(__uint_as_float(rd[i + e]), __uint_as_float(rd[i + e + 1])), pack2f(-d0, -d1))),
-                       zv[e], zv[e + 1]);
-            }
-            pp[i >> 1] = pack_bf16(pv[0], pv[1]); pp[(i >> 1) + 1] = pack_bf16(pv[2], pv[3]);
-            pz[i >> 1] = pack_bf16(zv[0], zv[1]); pz[(i >> 1) + 1] = pack_bf16(zv[2], zv[3]);
+            unpack2f(fmul2(pack2f(p0, p1), fadd2(pack2f(__uint_as_float(rd[i]), __uint_as_float(rd[i + 1])), nd)), z0, z1);
+            pz[i >> 1] = pack_bf16(z0, z1);
           }
-          if (MODE == 0) tmem_st16(s_t, pp);
           tmem_st16(dp_t, pz);
         }
         tc_wait_st();
@@ -331,25 +801,17 @@ swa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       }
       if (ok) {
         tc_fence_after();
-#pragma unroll 1
-        for (int which = (MODE == 0 ? 0 : 1); which < 2; ++which) {
-          __nv_bfloat16* dst = (which == 0 ? p.d0 : p.d1) + (((int64_t)b * T + xr) * p.H + h) * DAISY_HEAD_DIM + 32 * grp;
-          const float sc = which == 0 ? 1.f : p.scale;
-          {
-            uint32_t r[32];
-            tmem_ld32(which == 0 ? a0_t : a1_t, r);
-            tc_wait_ld();
-            if (xr < T) {
+        __nv_bfloat16* dst = p.d1 + (((int64_t)b * T + xr) * p.H + h) * DAISY_HEAD_DIM + 32 * grp;
+        uint32_t r[32];
+        tmem_ld32(a1_t, r);
+        tc_wait_ld();
+        if (xr < T) {
 #pragma unroll
-              for (int i = 0; i < 32; i += 8) {
-                uint4 o;
-                o.x = pack_bf16(__uint_as_float(r[i]) * sc, __uint_as_float(r[i + 1]) * sc);
-                o.y = pack_bf16(__uint_as_float(r[i + 2]) * sc, __uint_as_float(r[i + 3]) * sc);
-                o.z = pack_bf16(__uint_as_float(r[i + 4]) * sc, __uint_as_float(r[i + 5]) * sc);
-                o.w = pack_bf16(__uint_as_float(r[i + 6]) * sc, __uint_as_float(r[i + 7]) * sc);
-                *reinterpret_cast<uint4*>(dst + i) = o;
-              }
-            }
+          for (int i = 0; i < 32; i += 8) {
+            float f[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(r[i + e]) * p.scale;
+            *reinterpret_cast<uint4*>(dst + i) = pack8(f);
           }
         }
         // the next item's first accumulating products overwrite what was just read
@@ -374,6 +836,8 @@ struct DeltaParams {
 };
 
 __global__ void __launch_bounds__(256) swa_bwd_delta_kernel(const DeltaParams p) {
+  grid_dep_launch();
+  grid_dep_wait();
   const int64_t rows = (int64_t)p.B * p.T * p.H;
   const int64_t r = ((int64_t)blockIdx.x * 256 + threadIdx.x) >> 3;
   const int sub = threadIdx.x & 7;
@@ -592,13 +1056,20 @@ __global__ void __launch_bounds__(1024) gate_grad_kernel(const float* partial, i
 
 using namespace daisy;
 
+// Most bytes of dZ images that a call asks room for (above that the (batch, head) pairs go in several rounds).  8 x 8192 tokens,
+// 16 heads, window 2048 are 4.3 GB: two rounds.
+static constexpr size_t BWD_TILES_MAX = (size_t)2 << 30;
+
 static int bwd_smem_attr() {
   static bool done[daisy_host::MAX_DEVICES] = {};
   const int dev = daisy_host::device_slot();
   if (dev < 0) return DAISY_ENODEV;
   if (done[dev]) return DAISY_OK;
-  if (cudaFuncSetAttribute(swa_bwd_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_SMEM) != cudaSuccess) return DAISY_ECUDA;
-  if (cudaFuncSetAttribute(swa_bwd_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_SMEM) != cudaSuccess) return DAISY_ECUDA;
+  if (cudaFuncSetAttribute(swa_bwd_kv_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, KV_SMEM) != cudaSuccess ||
+      cudaFuncSetAttribute(swa_bwd_kv_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, KV_SMEM) != cudaSuccess ||
+      cudaFuncSetAttribute(swa_bwd_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DQ_SMEM) != cudaSuccess ||
+      cudaFuncSetAttribute(swa_bwd_q_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_SMEM) != cudaSuccess)
+    return DAISY_ECUDA;
   done[dev] = true;
   return DAISY_OK;
 }
@@ -606,6 +1077,23 @@ static int bwd_smem_attr() {
 extern "C" size_t daisy_b200_swa_attend_bwd_workspace_bytes(int B, int T, int H) {
   if (B <= 0 || T <= 0 || H <= 0) return 0;
   return (size_t)B * T * H * sizeof(float);                        // delta
+}
+
+// dZ images of one (batch, head): every query block's key blocks inside the window, 32 KB each
+static size_t bwd_tiles_row(int T, int window, bool in_blocks) {
+  const int64_t nblk = ((int64_t)T + WB - 1) / WB, seen = window <= 0 ? nblk : in_blocks ? window : ((int64_t)window + WB - 2) / WB + 1;
+  return (size_t)(seen < nblk ? seen : nblk);
+}
+static size_t bwd_tiles_bytes(int T, int window, bool in_blocks) {
+  return (size_t)((T + WB - 1) / WB) * bwd_tiles_row(T, window, in_blocks) * W_TILE;
+}
+static size_t bwd_delta_bytes(int B, int T, int H) { return (daisy_b200_swa_attend_bwd_workspace_bytes(B, T, H) + 1023) & ~(size_t)1023; }
+
+extern "C" size_t daisy_b200_swa_attend_bwd_workspace_bytes_full(int B, int T, int H, int window, unsigned flags) {
+  if (B <= 0 || T <= 0 || H <= 0 || (flags & ~DAISY_WINDOW_BLOCKS)) return 0;
+  const size_t one = bwd_tiles_bytes(T, window, (flags & DAISY_WINDOW_BLOCKS) != 0), pairs = (size_t)B * H;
+  const size_t n = BWD_TILES_MAX / one < pairs ? BWD_TILES_MAX / one : pairs;
+  return n ? bwd_delta_bytes(B, T, H) + n * one : daisy_b200_swa_attend_bwd_workspace_bytes(B, T, H);
 }
 
 extern "C" int daisy_b200_swa_attend_bwd(const void* q, const void* k, const void* v, const void* o, const void* d_o,
@@ -636,7 +1124,7 @@ extern "C" int daisy_b200_swa_attend_bwd(const void* q, const void* k, const voi
   {
     DeltaParams dp{(const __nv_bfloat16*)o, (const __nv_bfloat16*)d_o, o_sb, o_st, o_sh, g_sb, g_st, g_sh, delta, B, T, H};
     const int64_t rows = (int64_t)B * T * H;
-    swa_bwd_delta_kernel<<<(unsigned)((rows * 8 + 255) / 256), 256, 0, st>>>(dp);
+    (void)daisy_host::launch_dependent(swa_bwd_delta_kernel, dim3((unsigned)((rows * 8 + 255) / 256)), dim3(256), 0, st, dp);
     DAISY_CHECK_LAUNCH();
   }
   CUtensorMap tq, tk, tv, tg;
@@ -656,14 +1144,25 @@ extern "C" int daisy_b200_swa_attend_bwd(const void* q, const void* k, const voi
   p.status = status_word;
   const int sms = daisy_host::sm_count_cached();
   if (sms <= 0) return DAISY_ENODEV;
-  const int64_t items = (int64_t)((T + WB - 1) / WB) * H * B;
-  const unsigned grid = (unsigned)(items < sms ? items : sms);
-  p.d0 = (__nv_bfloat16*)dv; p.d1 = (__nv_bfloat16*)dk;
-  swa_bwd_kernel<0><<<grid, BWD_THREADS, BWD_SMEM, st>>>(tq, tk, tv, tg, p);
-  DAISY_CHECK_LAUNCH();
-  p.d0 = nullptr; p.d1 = (__nv_bfloat16*)dq;
-  swa_bwd_kernel<1><<<grid, BWD_THREADS, BWD_SMEM, st>>>(tq, tk, tv, tg, p);
-  DAISY_CHECK_LAUNCH();
+  const int nblk = (T + WB - 1) / WB;
+  const size_t one = bwd_tiles_bytes(T, window, in_blocks), delta_bytes = bwd_delta_bytes(B, T, H);
+  const size_t room = workspace_bytes > delta_bytes ? (workspace_bytes - delta_bytes) / one : 0;
+  const int pairs = B * H;
+  p.tiles = (uint8_t*)workspace + delta_bytes; p.tiles_row = (int)bwd_tiles_row(T, window, in_blocks);
+  // rounds of equal size, as many (batch, head) pairs at a time as there is room for images; without room for one pair's all in one
+  const int rounds = room ? (int)((pairs + room - 1) / room) : 1, per = (pairs + rounds - 1) / rounds;
+  for (p.bh0 = 0; p.bh0 < pairs; p.bh0 += per) {
+    p.n_bh = pairs - p.bh0 < per ? pairs - p.bh0 : per;
+    const int64_t items = (int64_t)nblk * p.n_bh;
+    const unsigned grid = (unsigned)(items < sms ? items : sms);
+    p.d0 = (__nv_bfloat16*)dv; p.d1 = (__nv_bfloat16*)dk;
+    (void)daisy_host::launch_dependent(room ? swa_bwd_kv_kernel<true> : swa_bwd_kv_kernel<false>, dim3(grid), dim3(KV_THREADS), KV_SMEM, st, tq, tk, tv, tg, p);
+    DAISY_CHECK_LAUNCH();
+    p.d0 = nullptr; p.d1 = (__nv_bfloat16*)dq;
+    if (room) (void)daisy_host::launch_dependent(swa_bwd_dq_kernel, dim3(grid), dim3(DQ_THREADS), DQ_SMEM, st, tk, p);
+    else      (void)daisy_host::launch_dependent(swa_bwd_q_kernel, dim3(grid), dim3(BWD_THREADS), BWD_SMEM, st, tq, tk, tv, tg, p);
+    DAISY_CHECK_LAUNCH();
+  }
   return DAISY_OK;
 }
 

@@ -169,13 +169,14 @@ def swa_attend_bwd(q, k, v, o, d_o, lse2, window: Optional[int], scale: float = 
     assert lse2.shape == (B, H, T)
     dq, dk, dv = (torch.empty(B, T, H, D, dtype=torch.bfloat16, device=q.device) for _ in range(3))
     L = _lib.lib()
-    ws = torch.empty(L.daisy_b200_swa_attend_bwd_workspace_bytes(B, T, H), dtype=torch.uint8, device=q.device)
+    flags = _lib.WINDOW_BLOCKS if window_in_blocks else 0
+    ws = torch.empty(L.daisy_b200_swa_attend_bwd_workspace_bytes_full(B, T, H, int(window or 0), flags), dtype=torch.uint8, device=q.device)
     _doc, doc_ptr, doc_sb = _doc_arg(doc_start, B, T, q.device)
     st = lambda t: (t.stride(0), t.stride(1), t.stride(2))
     rc = L.daisy_b200_swa_attend_bwd(
         q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), d_o.data_ptr(), *st(q), *st(k), *st(v), *st(o), *st(d_o),
         lse2.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), B, T, H, D, int(window or 0), scale, doc_ptr, doc_sb,
-        _lib.WINDOW_BLOCKS if window_in_blocks else 0, ws.data_ptr(), ws.numel(), status_word(q.device).data_ptr(), _stream(q))
+        flags, ws.data_ptr(), ws.numel(), status_word(q.device).data_ptr(), _stream(q))
     _lib.check(rc, "daisy_b200_swa_attend_bwd")
     return dq, dk, dv
 

@@ -242,10 +242,14 @@ int daisy_b200_swa_attend_lse(const void* q, const void* k, const void* v,
  *              bf16 with strides (s_b, s_t, s_h) each (o: o_s*, d_o: g_s*)
  *   lse2       [B,H,T] float32 from daisy_b200_swa_attend_lse
  *   dq,dk,dv   gradients w.r.t. the prepared q, k, v: [B,T,H,D] bf16 contiguous
- *   workspace  daisy_b200_swa_attend_bwd_workspace_bytes(B,T,H) bytes
- * Three launches (row-wise delta = sum_d dO O; a key-block-stationary kernel for dK, dV; a query-block-stationary
- * kernel for dQ); no atomics: results are bitwise reproducible. */
+ *   workspace  daisy_b200_swa_attend_bwd_workspace_bytes(B,T,H) bytes at least; with
+ *              daisy_b200_swa_attend_bwd_workspace_bytes_full(B,T,H,window,flags) bytes (2 GB and delta at most) dZ is kept between
+ *              the kernel for dK, dV and the one for dQ instead of being formed again.  Any size between is used as far as it goes
+ *              (the dQ of both ways agree to bf16 rounding).
+ * Launches: row-wise delta = sum_d dO O; a key-block-stationary kernel for dK, dV and a kernel for dQ, both once for as many
+ * (batch, head) pairs as the workspace holds; no atomics: results are bitwise reproducible. */
 size_t daisy_b200_swa_attend_bwd_workspace_bytes(int B, int T, int H);
+size_t daisy_b200_swa_attend_bwd_workspace_bytes_full(int B, int T, int H, int window, unsigned flags);
 int daisy_b200_swa_attend_bwd(const void* q, const void* k, const void* v, const void* o, const void* d_o,
                               int64_t q_sb, int64_t q_st, int64_t q_sh,
                               int64_t k_sb, int64_t k_st, int64_t k_sh,

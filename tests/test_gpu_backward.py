@@ -100,6 +100,48 @@ def test_attend_backward_block_window_training_form(T, wb, n_docs):
     _check_grads(got, ref, f"block window T={T} wb={wb}")
 
 
+@pytest.mark.parametrize("T,window,in_blocks,docs", [(128, None, False, False), (129, 1, False, False), (300, 130, False, True),
+                                                     (700, 127, False, False), (640, 2, True, True), (1000, None, False, True)])
+def test_attend_backward_workspaces(T, window, in_blocks, docs):
+    """dZ kept for dQ (workspace for all (batch, head) pairs, for two of six, i.e. several rounds, for one) or formed again
+    (delta alone): the same dK, dV and, of the first three, dQ bit for bit; both dQ at the bf16 bar of the oracle."""
+    from daisy_b200 import _lib, ops
+    B, H = 2, 3
+    q, k, v = _prepared(B, T, H, seed=T + 3)
+    d_o = bf16_randn(B, T, H, D, seed=T + 7, device="cpu")
+    ds = torch.zeros(T, dtype=torch.int32)
+    if docs:
+        for c in (T // 5, T // 3, T - 60):
+            ds[c:] = c
+    _, *ref = swa.attend_backward(q.float(), k.float(), v.float(), d_o.float(), None if in_blocks else window,
+                                  doc_start=ds if docs else None, window_blocks=window if in_blocks else None)
+    q, k, v, d_o = (t.cuda() for t in (q, k, v, d_o))
+    doc = ds.cuda() if docs else None
+    y, lse = ops.swa_attend(q, k, v, window, bounded_qk=True, doc_start=doc, window_in_blocks=in_blocks, return_lse=True)
+    L, flags = _lib.lib(), _lib.WINDOW_BLOCKS if in_blocks else 0
+    full = L.daisy_b200_swa_attend_bwd_workspace_bytes_full(B, T, H, window or 0, flags)
+    delta = -(-L.daisy_b200_swa_attend_bwd_workspace_bytes(B, T, H) // 1024) * 1024
+    one = (full - delta) // (B * H)
+    assert one % 32768 == 0 and one > 0
+    st = (T * H * D, H * D, D) * 5
+    got = []
+    for size in (full, delta + 2 * one, delta + one, delta):
+        out = [torch.full((B, T, H, D), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(3)]
+        ws = torch.full((size + 4096,), 0xff, dtype=torch.uint8, device="cuda")          # NaN images; guard behind the workspace
+        rc = L.daisy_b200_swa_attend_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), y.data_ptr(), d_o.data_ptr(), *st, lse.data_ptr(),
+                                         *(t.data_ptr() for t in out), B, T, H, D, window or 0, 0.12, doc.data_ptr() if docs else None, 0,
+                                         flags, ws.data_ptr(), size, ops.status_word(q.device).data_ptr(), torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
+        ops.check_device_status("cuda")
+        assert bool((ws[size:] == 0xff).all())
+        got.append(out)
+    for out in got[1:]:
+        assert torch.equal(out[1], got[0][1]) and torch.equal(out[2], got[0][2])
+    assert torch.equal(got[1][0], got[0][0]) and torch.equal(got[2][0], got[0][0])
+    for out in (got[0], got[3]):
+        _check_grads(out, ref, f"T={T} W={window}", cancelling=not in_blocks and window == 1)
+
+
 def test_prep_backward_matches_autograd():
     """Norm / RoPE backward on strided views of a merged projection."""
     from daisy_b200 import ops

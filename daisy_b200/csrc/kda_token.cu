@@ -63,6 +63,107 @@ struct KdaTokenStream : TokenRing {
 
 __device__ __forceinline__ float kt_sigmoid(float a) { return __fdividef(1.f, 1.f + fast_exp2(a * -1.4426950408889634f)); }
 
+// two channels of the short convolution: state s (the last four inputs of each, oldest first), taps w, new inputs v
+__device__ __forceinline__ void kt_conv(const uint4& s, const uint4& w, uint32_t v, const __nv_bfloat16* bias, int silu, float* out) {
+  float st[8], wt[8];
+  unpack8(s, st); unpack8(w, wt);
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const float cur = e ? bf16_hi(v) : bf16_lo(v);
+    float a = bias ? __bfloat162float(bias[e]) : 0.f;
+    a = fmaf(wt[4 * e], st[4 * e + 1], a);
+    a = fmaf(wt[4 * e + 1], st[4 * e + 2], a);
+    a = fmaf(wt[4 * e + 2], st[4 * e + 3], a);
+    a = fmaf(wt[4 * e + 3], cur, a);
+    out[e] = silu ? a * kt_sigmoid(a) : a;
+  }
+}
+__device__ __forceinline__ uint4 kt_shift(const uint4& s, uint32_t v) {
+  return make_uint4(s.x >> 16 | s.y << 16, s.y >> 16 | v << 16, s.z >> 16 | s.w << 16, s.w >> 16 | (v & 0xffff0000u));
+}
+
+// ---- one (batch, head), its vectors in shared memory: sv [9][128] = q, k, v, f0, g0, decay, output gate, two partial sums; sv[9 * 128]
+//      the write strength
+// decay gate (f1 row block x f0) and output gate (g1 row block x g0): half-warp hw takes rows hw, hw + HW, ..
+template <int HW>
+__device__ __forceinline__ void kt_gates(float* sv, const __nv_bfloat16* f1, const __nv_bfloat16* g1, const __nv_bfloat16* g1_bias, const float* a_log,
+                                         const float* dt_bias, int h, int tid) {
+  const int hw = tid >> 4, sub = tid & 15;
+  float f[8], g[8];
+  *reinterpret_cast<float4*>(f) = reinterpret_cast<const float4*>(sv + 3 * 128)[2 * sub]; *reinterpret_cast<float4*>(f + 4) = reinterpret_cast<const float4*>(sv + 3 * 128)[2 * sub + 1];
+  *reinterpret_cast<float4*>(g) = reinterpret_cast<const float4*>(sv + 4 * 128)[2 * sub]; *reinterpret_cast<float4*>(g + 4) = reinterpret_cast<const float4*>(sv + 4 * 128)[2 * sub + 1];
+  const float ea = -expf(__ldg(a_log + h));
+#pragma unroll
+  for (int k = 0; k < (256 + HW - 1) / HW; ++k) {
+    const int r = hw + HW * k;
+    float d = 0.f;
+    if (r < 256) {
+      float w[8];
+      unpack8(__ldg(reinterpret_cast<const uint4*>((r < 128 ? f1 : g1) + ((size_t)h * 128 + (r & 127)) * 128 + 8 * sub)), w);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) d = fmaf(w[e], r < 128 ? f[e] : g[e], d);
+    }
+    d += __shfl_xor_sync(0xffffffffu, d, 8); d += __shfl_xor_sync(0xffffffffu, d, 4);
+    d += __shfl_xor_sync(0xffffffffu, d, 2); d += __shfl_xor_sync(0xffffffffu, d, 1);
+    if (sub == 0 && r < 256) {
+      d = __bfloat162float(__float2bfloat16_rn(d));
+      if (r < 128) {                                  // decay e^g, g = -exp(A) softplus(f + dt_bias) at bf16
+        const float z = d + __ldg(dt_bias + h * 128 + r);
+        const float sp_ = z > 20.f ? z : log1pf(expf(z));
+        sv[5 * 128 + r] = __expf(__bfloat162float(__float2bfloat16_rn(ea * sp_)));
+      } else {
+        if (g1_bias) d = __bfloat162float(__float2bfloat16_rn(d + __bfloat162float(g1_bias[h * 128 + r - 128])));
+        sv[6 * 128 + r - 128] = d;
+      }
+    }
+  }
+}
+// state update and gated norm by 256 threads (value column tid & 127, keys 64 (tid >> 7) ..); store(columns 4 lane, + 1; + 2, + 3) by warp 0
+template <typename Store>
+__device__ __forceinline__ void kt_update(float (&S)[64], float* sv, const __nv_bfloat16* norm_w, float eps, int tid, Store&& store) {
+  const int vcol = tid & 127, kq = tid >> 7, lane = tid & 31;
+    const float* dk = sv + 5 * 128 + 64 * kq;
+    const float* kk = sv + 128 + 64 * kq;
+    float dot[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < 64; i += 4) {
+      const float4 d4 = *reinterpret_cast<const float4*>(dk + i), k4 = *reinterpret_cast<const float4*>(kk + i);
+      S[i] *= d4.x; S[i + 1] *= d4.y; S[i + 2] *= d4.z; S[i + 3] *= d4.w;
+      dot[0] = fmaf(S[i], k4.x, dot[0]); dot[1] = fmaf(S[i + 1], k4.y, dot[1]);
+      dot[2] = fmaf(S[i + 2], k4.z, dot[2]); dot[3] = fmaf(S[i + 3], k4.w, dot[3]);
+    }
+    sv[(7 + kq) * 128 + vcol] = (dot[0] + dot[1]) + (dot[2] + dot[3]);
+    named_bar(2, 256);
+    const float ut = sv[9 * 128] * (sv[2 * 128 + vcol] - (sv[7 * 128 + vcol] + sv[8 * 128 + vcol]));
+    named_bar(2, 256);
+    const float* qq = sv + 64 * kq;
+    float od[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < 64; i += 4) {
+      const float4 k4 = *reinterpret_cast<const float4*>(kk + i), q4 = *reinterpret_cast<const float4*>(qq + i);
+      S[i] = fmaf(k4.x, ut, S[i]); S[i + 1] = fmaf(k4.y, ut, S[i + 1]); S[i + 2] = fmaf(k4.z, ut, S[i + 2]); S[i + 3] = fmaf(k4.w, ut, S[i + 3]);
+      od[0] = fmaf(S[i], q4.x, od[0]); od[1] = fmaf(S[i + 1], q4.y, od[1]); od[2] = fmaf(S[i + 2], q4.z, od[2]); od[3] = fmaf(S[i + 3], q4.w, od[3]);
+    }
+    sv[(7 + kq) * 128 + vcol] = (od[0] + od[1]) + (od[2] + od[3]);
+    named_bar(2, 256);
+    if (tid < 32) {                                // gated norm: lane = 4 value columns
+      float4 a = reinterpret_cast<const float4*>(sv + 7 * 128)[lane], c = reinterpret_cast<const float4*>(sv + 8 * 128)[lane];
+      const float4 gt = reinterpret_cast<const float4*>(sv + 6 * 128)[lane];
+      const uint32_t o01 = pack_bf16(a.x + c.x, a.y + c.y), o23 = pack_bf16(a.z + c.z, a.w + c.w);
+      float x[4] = {bf16_lo(o01), bf16_hi(o01), bf16_lo(o23), bf16_hi(o23)};
+      const float gg[4] = {gt.x, gt.y, gt.z, gt.w};
+      const float rstd = rsqrtf(tk_warp_sum(x[0] * x[0] + x[1] * x[1] + x[2] * x[2] + x[3] * x[3]) * (1.0f / 128) + eps);
+      float r[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float n = x[e] * (rstd * (norm_w ? __bfloat162float(norm_w[4 * lane + e]) : 1.f)), s = kt_sigmoid(gg[e]);
+        r[e] = __bfloat162float(__float2bfloat16_rn(n * gg[e] * s)) * __bfloat162float(__float2bfloat16_rn(s));
+      }
+      const uint32_t r01 = pack_bf16(r[0], r[1]), r23 = pack_bf16(r[2], r[3]);
+      store(r01, r23);
+    }
+}
+
 template <int NB>
 __global__ void __launch_bounds__(TK_CT, 1) kda_token_kernel(const __grid_constant__ KdaTokenParams p) {
   extern __shared__ __align__(128) uint8_t kt_smem[];
@@ -128,19 +229,9 @@ __global__ void __launch_bounds__(TK_CT, 1) kda_token_kernel(const __grid_consta
       __nv_bfloat16* sp = p.conv_s[m] + ((size_t)b * p.dim + row) * 4;
       uint4 s = cs, w = cw;
       if (!first) { s = *reinterpret_cast<const uint4*>(sp); w = __ldg(reinterpret_cast<const uint4*>(p.conv_w[m] + (size_t)row * 4)); }
-      float st[8], wt[8], out[2];
-      unpack8(s, st); unpack8(w, wt);
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {                   // state: the last four inputs, oldest first
-        const float cur = e ? bf16_hi(v) : bf16_lo(v);
-        float a = p.conv_b[m] ? __bfloat162float(p.conv_b[m][row + e]) : 0.f;
-        a = fmaf(wt[4 * e], st[4 * e + 1], a);
-        a = fmaf(wt[4 * e + 1], st[4 * e + 2], a);
-        a = fmaf(wt[4 * e + 2], st[4 * e + 3], a);
-        a = fmaf(wt[4 * e + 3], cur, a);
-        out[e] = p.silu ? a * kt_sigmoid(a) : a;
-      }
-      *reinterpret_cast<uint4*>(sp) = make_uint4(s.x >> 16 | s.y << 16, s.y >> 16 | v << 16, s.z >> 16 | s.w << 16, s.w >> 16 | (v & 0xffff0000u));
+      float out[2];
+      kt_conv(s, w, v, p.conv_b[m] ? p.conv_b[m] + row : nullptr, p.silu, out);
+      *reinterpret_cast<uint4*>(sp) = kt_shift(s, v);
       tk_put2(p.qkv + (size_t)b * 3 * (p.dim / 2) + m * (p.dim / 2) + (row >> 1), pack_bf16(out[0], out[1]), tag);
     } else if (m < 5) {
       tk_put2(p.fg + (size_t)b * 128 + (m - 3) * 64 + (row >> 1), v, tag);
@@ -176,82 +267,14 @@ __global__ void __launch_bounds__(TK_CT, 1) kda_token_kernel(const __grid_consta
       sv[9 * 128] = __bfloat162float(__float2bfloat16_rn(kt_sigmoid(z)));
     }
     named_bar(1, TK_CT);
-    {                                                 // half-warp hw: rows hw, hw + 24, .. of [f1 block; g1 block]
-      const int hw = tid >> 4, sub = tid & 15;
-      float f[8], g[8];
-      *reinterpret_cast<float4*>(f) = reinterpret_cast<const float4*>(sv + 3 * 128)[2 * sub]; *reinterpret_cast<float4*>(f + 4) = reinterpret_cast<const float4*>(sv + 3 * 128)[2 * sub + 1];
-      *reinterpret_cast<float4*>(g) = reinterpret_cast<const float4*>(sv + 4 * 128)[2 * sub]; *reinterpret_cast<float4*>(g + 4) = reinterpret_cast<const float4*>(sv + 4 * 128)[2 * sub + 1];
-      const float ea = -expf(__ldg(p.a_log + h));
-#pragma unroll
-      for (int k = 0; k < 11; ++k) {
-        const int r = hw + 24 * k;
-        float d = 0.f;
-        if (r < 256) {
-          float w[8];
-          unpack8(__ldg(reinterpret_cast<const uint4*>((r < 128 ? p.f1 : p.g1) + ((size_t)h * 128 + (r & 127)) * 128 + 8 * sub)), w);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) d = fmaf(w[e], r < 128 ? f[e] : g[e], d);
-        }
-        d += __shfl_xor_sync(0xffffffffu, d, 8); d += __shfl_xor_sync(0xffffffffu, d, 4);
-        d += __shfl_xor_sync(0xffffffffu, d, 2); d += __shfl_xor_sync(0xffffffffu, d, 1);
-        if (sub == 0 && r < 256) {
-          d = __bfloat162float(__float2bfloat16_rn(d));
-          if (r < 128) {                              // decay e^g, g = -exp(A) softplus(f + dt_bias) at bf16
-            const float z = d + __ldg(p.dt_bias + h * 128 + r);
-            const float sp_ = z > 20.f ? z : log1pf(expf(z));
-            sv[5 * 128 + r] = __expf(__bfloat162float(__float2bfloat16_rn(ea * sp_)));
-          } else {
-            if (p.g1_bias) d = __bfloat162float(__float2bfloat16_rn(d + __bfloat162float(p.g1_bias[h * 128 + r - 128])));
-            sv[6 * 128 + r - 128] = d;
-          }
-        }
-      }
-    }
+    kt_gates<TK_CT / 16>(sv, p.f1, p.g1, p.g1_bias, p.a_log, p.dt_bias, h, tid);
     named_bar(1, TK_CT);
-    const int vcol = tid & 127, kq = tid >> 7;
     if (tid < 256) {
-      const float* dk = sv + 5 * 128 + 64 * kq;
-      const float* kk = sv + 128 + 64 * kq;
-      float dot[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-      for (int i = 0; i < 64; i += 4) {
-        const float4 d4 = *reinterpret_cast<const float4*>(dk + i), k4 = *reinterpret_cast<const float4*>(kk + i);
-        S[i] *= d4.x; S[i + 1] *= d4.y; S[i + 2] *= d4.z; S[i + 3] *= d4.w;
-        dot[0] = fmaf(S[i], k4.x, dot[0]); dot[1] = fmaf(S[i + 1], k4.y, dot[1]);
-        dot[2] = fmaf(S[i + 2], k4.z, dot[2]); dot[3] = fmaf(S[i + 3], k4.w, dot[3]);
-      }
-      sv[(7 + kq) * 128 + vcol] = (dot[0] + dot[1]) + (dot[2] + dot[3]);
-      named_bar(2, 256);
-      const float ut = sv[9 * 128] * (sv[2 * 128 + vcol] - (sv[7 * 128 + vcol] + sv[8 * 128 + vcol]));
-      named_bar(2, 256);
-      const float* qq = sv + 64 * kq;
-      float od[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-      for (int i = 0; i < 64; i += 4) {
-        const float4 k4 = *reinterpret_cast<const float4*>(kk + i), q4 = *reinterpret_cast<const float4*>(qq + i);
-        S[i] = fmaf(k4.x, ut, S[i]); S[i + 1] = fmaf(k4.y, ut, S[i + 1]); S[i + 2] = fmaf(k4.z, ut, S[i + 2]); S[i + 3] = fmaf(k4.w, ut, S[i + 3]);
-        od[0] = fmaf(S[i], q4.x, od[0]); od[1] = fmaf(S[i + 1], q4.y, od[1]); od[2] = fmaf(S[i + 2], q4.z, od[2]); od[3] = fmaf(S[i + 3], q4.w, od[3]);
-      }
-      sv[(7 + kq) * 128 + vcol] = (od[0] + od[1]) + (od[2] + od[3]);
-      named_bar(2, 256);
-      if (warp == 0) {                                // gated norm: lane = 4 value columns
-        float4 a = reinterpret_cast<const float4*>(sv + 7 * 128)[lane], c = reinterpret_cast<const float4*>(sv + 8 * 128)[lane];
-        const float4 gt = reinterpret_cast<const float4*>(sv + 6 * 128)[lane];
-        const uint32_t o01 = pack_bf16(a.x + c.x, a.y + c.y), o23 = pack_bf16(a.z + c.z, a.w + c.w);
-        float x[4] = {bf16_lo(o01), bf16_hi(o01), bf16_lo(o23), bf16_hi(o23)};
-        const float gg[4] = {gt.x, gt.y, gt.z, gt.w};
-        const float rstd = rsqrtf(tk_warp_sum(x[0] * x[0] + x[1] * x[1] + x[2] * x[2] + x[3] * x[3]) * (1.0f / 128) + p.eps);
-        float r[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float n = x[e] * (rstd * (p.norm_w ? __bfloat162float(p.norm_w[4 * lane + e]) : 1.f)), s = kt_sigmoid(gg[e]);
-          r[e] = __bfloat162float(__float2bfloat16_rn(n * gg[e] * s)) * __bfloat162float(__float2bfloat16_rn(s));
-        }
-        const uint32_t r01 = pack_bf16(r[0], r[1]), r23 = pack_bf16(r[2], r[3]);
+      kt_update(S, sv, p.norm_w, p.eps, tid, [&](uint32_t r01, uint32_t r23) {
 #pragma unroll
         for (int c4 = 0; c4 < TK_COPIES; ++c4)
           tk_put4(reinterpret_cast<uint4*>(p.o + (size_t)(c4 * p.B + b) * (p.dim / 2) + h * 64) + lane, r01, r23, tag);
-      }
+      });
 #pragma unroll
       for (int i = 0; i < 64; ++i) sp[i * 128] = S[i];
     }
@@ -267,6 +290,79 @@ __global__ void __launch_bounds__(TK_CT, 1) kda_token_kernel(const __grid_consta
   if (tid == 0 && cta == 0) *p.epoch = tag;           // every CTA has contributed by now, hence read the tag
 }
 
+// ---------------------------------------------------------------------------------------------
+// The same step for batches that the launch above would take in several: projections by the GEMM, everything between by this
+// kernel, one CTA per (batch, head).  It is bound by the state, 64 KB in and out (12 heads x 54 rows: 85 MB, 13 us at copy
+// bandwidth); the gates' second projections are formed here (64 KB of weights a CTA, from L2) rather than as two more products.
+struct KdaBatchParams {
+  const __nv_bfloat16 *x, *pr[3], *f0, *g0;           // [B, dim] (row stride x_sb); projections [B, dim] and [B, 128]
+  const __nv_bfloat16 *b_w, *f1, *g1, *g1_bias, *norm_w, *conv_w[3], *conv_b[3];
+  __nv_bfloat16 *conv_s[3], *o;                       // o [B, dim]
+  const float *a_log, *dt_bias;
+  float* state;
+  int64_t x_sb;
+  int H, dim, silu;
+  float eps, scale;
+};
+
+__global__ void __launch_bounds__(256, 2) kda_batch_kernel(const __grid_constant__ KdaBatchParams p) {
+  __shared__ __align__(16) float sv[9 * 128 + 4];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, u = blockIdx.x, h = u % p.H, b = u / p.H;
+  if (tid < 2) l2_prefetch_bulk(p.state + (size_t)u * 128 * 128 + tid * 8192, 32768);
+  else if (tid < 4) l2_prefetch_bulk((tid == 2 ? p.f1 : p.g1) + (size_t)h * 128 * 128, 32768);
+  grid_dep_launch();
+  grid_dep_wait();
+  float S[64];
+  float* sp = p.state + (size_t)u * 128 * 128 + (size_t)(tid >> 7) * 64 * 128 + (tid & 127);
+#pragma unroll
+  for (int i = 0; i < 64; ++i) S[i] = __ldcg(sp + i * 128);
+  if (warp < 3) {                                     // convolution of q, k, v: four channels a lane
+    const int ch = h * 128 + 4 * lane;
+    __nv_bfloat16* cs = p.conv_s[warp] + ((size_t)b * p.dim + ch) * 4;
+    const uint2 cur2 = *reinterpret_cast<const uint2*>(p.pr[warp] + (size_t)b * p.dim + ch);
+    float x[4];
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const uint32_t v = half ? cur2.y : cur2.x;
+      const uint4 s = *reinterpret_cast<const uint4*>(cs + 8 * half), w = __ldg(reinterpret_cast<const uint4*>(p.conv_w[warp] + (size_t)(ch + 2 * half) * 4));
+      float out[2];
+      kt_conv(s, w, v, p.conv_b[warp] ? p.conv_b[warp] + ch + 2 * half : nullptr, p.silu, out);
+      *reinterpret_cast<uint4*>(cs + 8 * half) = kt_shift(s, v);
+      const uint32_t r = pack_bf16(out[0], out[1]);
+      x[2 * half] = bf16_lo(r); x[2 * half + 1] = bf16_hi(r);
+    }
+    if (warp < 2) {                                   // q, k: L2 norm
+      const float n = rsqrtf(tk_warp_sum(x[0] * x[0] + x[1] * x[1] + x[2] * x[2] + x[3] * x[3]) + 1e-6f) * (warp == 0 ? p.scale : 1.f);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) x[e] *= n;
+    }
+    reinterpret_cast<float4*>(sv + warp * 128)[lane] = make_float4(x[0], x[1], x[2], x[3]);
+  } else if (warp < 5) {
+    const uint2 r = *reinterpret_cast<const uint2*>((warp == 3 ? p.f0 : p.g0) + (size_t)b * 128 + 4 * lane);
+    reinterpret_cast<float4*>(sv + warp * 128)[lane] = make_float4(bf16_lo(r.x), bf16_hi(r.x), bf16_lo(r.y), bf16_hi(r.y));
+  } else if (warp == 5) {                             // the write strength: sigmoid at bf16, as the layer computes it
+    float d = 0.f;
+#pragma unroll 4
+    for (int k = 8 * lane; k < p.dim; k += 256) {
+      float a[8], w[8];
+      unpack8(*reinterpret_cast<const uint4*>(p.x + b * p.x_sb + k), a);
+      unpack8(__ldg(reinterpret_cast<const uint4*>(p.b_w + (size_t)h * p.dim + k)), w);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) d = fmaf(a[e], w[e], d);
+    }
+    d = tk_warp_sum(d);
+    if (lane == 0) sv[9 * 128] = __bfloat162float(__float2bfloat16_rn(kt_sigmoid(__bfloat162float(__float2bfloat16_rn(d)))));
+  }
+  __syncthreads();
+  kt_gates<16>(sv, p.f1, p.g1, p.g1_bias, p.a_log, p.dt_bias, h, tid);
+  __syncthreads();
+  kt_update(S, sv, p.norm_w, p.eps, tid, [&](uint32_t r01, uint32_t r23) {
+    *reinterpret_cast<uint2*>(p.o + (size_t)b * p.dim + h * 128 + 4 * lane) = make_uint2(r01, r23);
+  });
+#pragma unroll
+  for (int i = 0; i < 64; ++i) sp[i * 128] = S[i];
+}
+
 }  // namespace daisy
 
 using namespace daisy;
@@ -274,8 +370,9 @@ using namespace daisy;
 static inline size_t kt_align(size_t n) { return (n + 255) / 256 * 256; }
 
 extern "C" size_t daisy_b200_kda_token_workspace_bytes(int B, int H, int D) {
-  if (B <= 0 || H <= 0 || D != 128 || B > TK_MAX_B || H * D > TK_MAX_DIM) return 0;
+  if (B <= 0 || H <= 0 || D != 128 || H * D > TK_MAX_DIM) return 0;
   const size_t dim = (size_t)H * D;
+  if (B > TK_MAX_B) return 4 * kt_align(B * dim * 2) + 2 * kt_align((size_t)B * 128 * 2);   // q, k, v, o; f0, g0
   return 256 + kt_align(B * 3 * dim * 4) + kt_align((size_t)B * 128 * 8) + kt_align((size_t)B * 64) + TK_COPIES * kt_align(B * dim * 4);
 }
 
@@ -306,6 +403,36 @@ static int launch_kda_token(KdaTokenParams& p, int sms, cudaStream_t st) {
   return DAISY_OK;
 }
 
+// More rows than a launch of kda_token_kernel takes: four launches for all of them.
+static int kda_batch_step(const daisy_b200_kda_layer* ly, const void* x, int64_t x_sb, void* y, float* state, void* conv_q, void* conv_k, void* conv_v,
+                          int B, int H, float eps, unsigned flags, void* workspace, int* status_word, void* stream) {
+  const int dim = H * 128;
+  if ((int64_t)B * H >= (int64_t)1 << 31) return DAISY_EUNSUPPORTED;
+  uint8_t* ws = (uint8_t*)workspace;
+  void *pr[3], *o, *low[2];
+  for (void*& c : pr) { c = ws; ws += kt_align((size_t)B * dim * 2); }
+  o = ws; ws += kt_align((size_t)B * dim * 2);
+  for (void*& c : low) { c = ws; ws += kt_align((size_t)B * 128 * 2); }
+  const void *xs[3] = {x, x, x}, *w1[3] = {ly->q_w, ly->k_w, ly->v_w}, *w2[2] = {ly->f0_w, ly->g0_w};
+  int rc;
+  if ((rc = daisy_b200_gemm_nt_group(xs, x_sb, w2, dim, low, 128, 2, B, 128, dim, status_word, stream)) != DAISY_OK) return rc;
+  if ((rc = daisy_b200_gemm_nt_group(xs, x_sb, w1, dim, pr, dim, 3, B, dim, dim, status_word, stream)) != DAISY_OK) return rc;
+  KdaBatchParams p;
+  p.x = (const __nv_bfloat16*)x; p.x_sb = x_sb; p.f0 = (const __nv_bfloat16*)low[0]; p.g0 = (const __nv_bfloat16*)low[1];
+  p.b_w = (const __nv_bfloat16*)ly->b_w; p.f1 = (const __nv_bfloat16*)ly->f1_w; p.g1 = (const __nv_bfloat16*)ly->g1_w;
+  p.g1_bias = (const __nv_bfloat16*)ly->g1_bias; p.norm_w = (const __nv_bfloat16*)ly->norm_w;
+  void* cs[3] = {conv_q, conv_k, conv_v};
+  for (int i = 0; i < 3; ++i) {
+    p.pr[i] = (const __nv_bfloat16*)pr[i];
+    p.conv_w[i] = (const __nv_bfloat16*)ly->conv_w[i]; p.conv_b[i] = (const __nv_bfloat16*)ly->conv_bias[i]; p.conv_s[i] = (__nv_bfloat16*)cs[i];
+  }
+  p.o = (__nv_bfloat16*)o; p.a_log = ly->a_log; p.dt_bias = ly->dt_bias; p.state = state;
+  p.H = H; p.dim = dim; p.silu = (flags & DAISY_KDA_CONV_SILU) ? 1 : 0; p.eps = eps; p.scale = 1.0f / sqrtf(128.f);
+  (void)daisy_host::launch_dependent(kda_batch_kernel, dim3((unsigned)(B * H)), dim3(256), 0, (cudaStream_t)stream, p);
+  DAISY_CHECK_LAUNCH();
+  return daisy_b200_gemm_nt(o, dim, ly->o_w, dim, y, dim, B, dim, dim, status_word, stream);
+}
+
 extern "C" int daisy_b200_kda_token_step(const daisy_b200_kda_layer* ly, const void* x, int64_t x_sb, void* y, float* state,
                                          void* conv_q, void* conv_k, void* conv_v, int B, int H, int D, float eps, unsigned flags,
                                          void* workspace, size_t workspace_bytes, int* status_word, void* stream) {
@@ -326,6 +453,7 @@ extern "C" int daisy_b200_kda_token_step(const daisy_b200_kda_layer* ly, const v
   const int sms = daisy_host::sm_count_cached();
   if (sms <= 0) return DAISY_ENODEV;
   const int dim = H * D;
+  if (B > TK_MAX_B) return kda_batch_step(ly, x, x_sb, y, state, conv_q, conv_k, conv_v, B, H, eps, flags, workspace, status_word, stream);
   KdaTokenParams p;
   const void* w[7] = {ly->q_w, ly->k_w, ly->v_w, ly->f0_w, ly->g0_w, ly->b_w, ly->o_w};
   const int rows[7] = {dim, dim, dim, 128, 128, H, dim};

@@ -506,7 +506,7 @@ bool plain_bf16(const std::vector<OptTensor>& ts) {
   return true;
 }
 bool kda_token_supported(int64_t H) { return H >= 1 && daisy_b200_kda_token_workspace_bytes(1, (int)H, 128) != 0; }
-int64_t kda_token_workspace_bytes(int64_t B, int64_t H) { return (int64_t)daisy_b200_kda_token_workspace_bytes((int)std::min<int64_t>(B, 16), (int)H, 128); }
+int64_t kda_token_workspace_bytes(int64_t B, int64_t H) { return (int64_t)daisy_b200_kda_token_workspace_bytes((int)B, (int)H, 128); }
 
 // weights: q, k, v, f0, f1, g0, g1, b, o; conv: q, k, v weights (and biases); the states are updated in place
 Tensor kda_token_step(const Tensor& x_, const std::vector<Tensor>& w_, const OptTensor& g1_bias, const OptTensor& norm_w, const std::vector<Tensor>& conv_w,
@@ -539,14 +539,11 @@ Tensor kda_token_step(const Tensor& x_, const std::vector<Tensor>& w_, const Opt
   }
   ly.a_log = a_log.data_ptr<float>(); ly.dt_bias = dt_bias.data_ptr<float>();
   Tensor y = out.has_value() ? *out : at::empty({B, 1, dim}, x.options());
-  Tensor ws = workspace.has_value() ? *workspace : stream_workspace(x, WS_KDA_TOKEN, kda_token_workspace_bytes(B, H));
-  for (int64_t b0 = 0; b0 < B; b0 += 16) {                               // larger batches: 16 rows a launch, the weights come from L2 again
-    const int64_t n = std::min<int64_t>(16, B - b0);
-    check(daisy_b200_kda_token_step(&ly, (char*)x.data_ptr() + b0 * dim * 2, dim, (char*)y.data_ptr() + b0 * dim * 2, state.data_ptr<float>() + b0 * H * 128 * 128,
-                                    (char*)conv_s[0].data_ptr() + b0 * dim * 8, (char*)conv_s[1].data_ptr() + b0 * dim * 8, (char*)conv_s[2].data_ptr() + b0 * dim * 8,
-                                    (int)n, (int)H, 128, (float)eps, silu ? DAISY_KDA_CONV_SILU : 0, ws.data_ptr(), (size_t)ws.numel(), status_ptr(x), stream_of(x)),
-          "daisy_b200_kda_token_step");
-  }
+  const int64_t need = kda_token_workspace_bytes(B, H);                  // above 16 rows plain scratch, below words that have to be zero at first
+  Tensor ws = workspace.has_value() ? *workspace : B > 16 ? at::empty({need}, x.options().dtype(at::kByte)) : stream_workspace(x, WS_KDA_TOKEN, need);
+  check(daisy_b200_kda_token_step(&ly, x.data_ptr(), dim, y.data_ptr(), state.data_ptr<float>(), conv_s[0].data_ptr(), conv_s[1].data_ptr(), conv_s[2].data_ptr(),
+                                  (int)B, (int)H, 128, (float)eps, silu ? DAISY_KDA_CONV_SILU : 0, ws.data_ptr(), (size_t)ws.numel(), status_ptr(x), stream_of(x)),
+        "daisy_b200_kda_token_step");
   return y;
 }
 

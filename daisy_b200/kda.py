@@ -180,8 +180,8 @@ class B200KimiLinearSelfAttention(torch.nn.Module):
         self._recurrent_state, self._conv_state, self._seen = None, None, 0
 
     def _token_step(self, x, out=None, workspace=None):
-        """The decode step as one launch (``csrc/kda_token.cu``; 16 batch rows at a time), states updated in place; None
-        where the layer or its states are not of the form that kernel takes."""
+        """The decode step as one native call (``csrc/kda_token.cu``; one launch up to 16 batch rows, four above), states updated
+        in place; None where the layer or its states are not of the form those kernels take."""
         rec, conv = self._recurrent_state, self._conv_state
         if (rec is None or conv is None or x.shape[1] != 1 or not x.is_cuda or self.hidden_size != self.key_dim
                 or self.head_dim != 128 or not ext().kda_token_supported(self.num_heads)

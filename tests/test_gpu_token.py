@@ -129,3 +129,29 @@ def test_kimi_token_step_continues_a_prefill(B, H, bias):
     for a, b in zip(layer._conv_state, conv):
         assert torch.equal(a[..., :3], b[..., :3]), "the carried inputs move up"
         assert_close_bf16(a, b, "the new input")
+
+
+@pytest.mark.parametrize("B,H,bias", [(17, 1, True), (33, 3, False), (64, 16, True)])
+def test_kimi_batch_step_matches_row_launches(B, H, bias):
+    """Above 16 rows (kda_batch_kernel between GEMMs) against the single launch on 16 rows at a time: the convolution states bit
+    for bit but for the new input, everything else to the order of fp32 sums under bf16 roundings."""
+    from daisy_b200 import B200KimiLinearSelfAttention, ops
+    torch.manual_seed(B)
+    layer = B200KimiLinearSelfAttention(H * D, H, 4096, D, conv_bias=bias).cuda()
+    x = torch.randn(B, 30, H * D, device="cuda", dtype=torch.bfloat16)
+    with torch.inference_mode():
+        layer.prefill(x[:, :29])
+        rec, conv = layer._recurrent_state.clone(), [c.clone() for c in layer._conv_state]
+        y, _, _ = layer.step(x[:, 29:])
+        got = (y, layer._recurrent_state, *layer._conv_state)
+        ys = []
+        for b in range(0, B, 16):
+            layer._recurrent_state, layer._conv_state = rec[b:b + 16].clone(), tuple(c[b:b + 16].clone() for c in conv)
+            ys.append((layer.step(x[b:b + 16, 29:])[0], layer._recurrent_state, *layer._conv_state))
+    ops.check_device_status("cuda")
+    ref = [torch.cat(t) for t in zip(*ys)]
+    assert_close_bf16(got[0], ref[0], "y", max_tol=3e-2, mean_tol=3e-3)
+    assert ((got[1] - ref[1]).norm() / ref[1].norm()).item() < 5e-3
+    for a, b in zip(got[2:], ref[2:]):
+        assert torch.equal(a[..., :3], b[..., :3])
+        assert_close_bf16(a, b, "the new input")

@@ -36,7 +36,8 @@ constexpr int HALF_BYTES = TILE_BYTES / 2;               // one [128 x 64] swizz
 constexpr int PREFILL_THREADS = 320;          // one softmax warpgroup per stream
 constexpr int PREFILL_THREADS_SPLIT = 576;    // two softmax warpgroups per stream (64 key columns each)
 constexpr int SMEM_TILES = (2 * NQBUF + NSTAGE) * TILE_BYTES;
-constexpr int PREFILL_SMEM = 1024 + SMEM_TILES + 256 + 2 * 128 * 4;   // alignment slack, tiles, barriers, row-sum exchange
+constexpr int PREFILL_BARS = 512;
+constexpr int PREFILL_SMEM = 1024 + SMEM_TILES + PREFILL_BARS + 2 * 128 * 4;   // alignment slack, tiles, barriers, row-sum exchange
 static_assert(PREFILL_SMEM <= 232448, "over the 227 KB a CTA may use");
 constexpr float NEG_BIG = -1.0e30f;
 #ifndef POLY_MASK
@@ -67,6 +68,15 @@ struct PrefillParams {
   float* lse2;
 };
 
+// Geometry of one work item: 256 query rows (two streams) of one (batch, head).
+struct ItemGeom {
+  int b, h;                        // b < 0: no more items
+  int q0[2], jlo_s[2], jhi_s[2];
+  bool valid[2];
+  int jlo, jhi;
+};
+constexpr int NITEM = 3;           // items handed out ahead
+
 struct PrefillBarriers {
   uint64_t q_full[2][NQBUF];
   uint64_t q_empty[2][NQBUF];
@@ -76,21 +86,17 @@ struct PrefillBarriers {
   uint64_t s_full[2];
   uint64_t p_full[2];
   uint64_t o_full[2];
+  uint64_t i_full[NITEM], i_empty[NITEM];
+  ItemGeom item[NITEM];            // as the producer hands them out
   uint32_t tmem_base;
   int abort_flag;
 };
+static_assert(sizeof(PrefillBarriers) <= PREFILL_BARS, "room for the barriers");
 
 __device__ __forceinline__ bool key_visible(int q, int k, int window) {
   return (k <= q) && (window <= 0 || k > q - window);
 }
 
-// Geometry of one work item: 256 query rows (two streams) of one (batch, head).
-struct ItemGeom {
-  int b, h;
-  int q0[2], jlo_s[2], jhi_s[2];
-  bool valid[2];
-  int jlo, jhi;
-};
 __device__ __forceinline__ ItemGeom item_geom(int item, int nq, int H, int T, int window, int streams,
                                               const int* doc_start = nullptr, int64_t doc_sb = 0, int window_blocks = 0) {
   ItemGeom g;
@@ -181,10 +187,16 @@ __device__ __forceinline__ BalancedWalk prefill_walk(int nq, int BH, int window,
 // |logit * log2 e| <= 60 no reference maximum is needed at all (2^x stays far inside fp32 and bf16 range), so the
 // two halves of a row never talk to each other until the epilogue adds their partial row sums.  Each half writes
 // its P over the first 32 columns of its OWN 64 S columns (P_s = two 32-column pieces at S_s + 0 and S_s + 64).
+// What an item costs beside its tiles, and what a partly visible tile costs, is what short windows and documents are bound by
+// (7 x 1009 x 16, window 249: 22500 cycles an item of four tiles).  So the producer works out the items ahead and hands them out,
+// the output leaves through the item's Q buffer as bulk copies, and a partial tile's 32-column pieces are masked, skipped or
+// taken whole as a warp's rows see them: 44.1 -> 32.1 us there, 8 x 8192 x 16 at window 2048 873 -> 833.  A thread's second 32
+// scores are fetched under its first 32: all 64 at once spilled in the tile loop (1 x 65536, window 8192: 3090 -> 3048; 3031 before
+// all this).
 template <bool QRAW, bool BOUNDED, int NSPLIT, int STREAMS>
 __global__ void __launch_bounds__(32 * (8 * NSPLIT + 2), 1)
 swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                   const __grid_constant__ CUtensorMap tm_v, const PrefillParams p) {
+                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const PrefillParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* q_tiles = smem;
@@ -201,12 +213,13 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < 2; ++s) {
-      for (int qb = 0; qb < NQBUF; ++qb) { mbar_init(&bars->q_full[s][qb], 1); mbar_init(&bars->q_empty[s][qb], 1); mbar_init(&bars->q_ready[s][qb], 128); }
+      for (int qb = 0; qb < NQBUF; ++qb) { mbar_init(&bars->q_full[s][qb], 1); mbar_init(&bars->q_empty[s][qb], NSPLIT); mbar_init(&bars->q_ready[s][qb], 128); }
       mbar_init(&bars->s_full[s], 1);
       mbar_init(&bars->p_full[s], 128 * NSPLIT);
       mbar_init(&bars->o_full[s], 1);
     }
     for (int i = 0; i < NSTAGE; ++i) { mbar_init(&bars->kv_full[i], 1); mbar_init(&bars->kv_empty[i], 1); }
+    for (int i = 0; i < NITEM; ++i) { mbar_init(&bars->i_full[i], 1); mbar_init(&bars->i_empty[i], 8 * NSPLIT + 1); }   // issuer, softmax warps
     bars->abort_flag = 0;
     mbar_init_fence();
   }
@@ -221,17 +234,29 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   grid_dep_launch();
   grid_dep_wait();
 
+  // the rd-th item as the producer hands it out (an item's place and ranges are a dozen dependent divisions and document reads,
+  // which the producer has the time for); null when there are no more, or a wait ran out
+  auto next_item = [&](int rd) -> const ItemGeom* {
+    const ItemGeom* g = &bars->item[rd % NITEM];
+    if (!__all_sync(0xffffffffu, mbar_wait(&bars->i_full[rd % NITEM], (rd / NITEM) & 1, abort_flag, p.status, 13))) return nullptr;
+    return g->b >= 0 ? g : nullptr;
+  };
+  auto item_done = [&](int rd) {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&bars->i_empty[rd % NITEM]);
+  };
+
   if (warp == TMA_WARP) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
       prefetch_tmap(&tm_q); prefetch_tmap(&tm_k); prefetch_tmap(&tm_v);
+      if (NSPLIT == 2) prefetch_tmap(&tm_o);
       int n = 0;                         // K/V tiles loaded so far (ring position)
       uint32_t qn[2] = {0, 0};           // Q tiles loaded so far per stream
       bool ok = true;
       // Q tiles run one item ahead of the K/V stream (double buffer), so the softmax warps can prepare the
       // next item's Q while the current item is still computing.
-      auto load_q = [&](int it_item) {
-        const ItemGeom gq = item_geom(it_item, nq, p.H, T, window, STREAMS, p.doc_start, p.doc_sb, p.window_blocks);
+      auto load_q = [&](const ItemGeom& gq) {
         for (int s = 0; s < 2 && ok; ++s) {
           if (!gq.valid[s]) continue;
           const int qb = qn[s] % NQBUF;
@@ -243,9 +268,18 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           tma_load_4d(qdst + HALF_BYTES, &tm_q, &bars->q_full[s][qb], 64, gq.q0[s], gq.h, gq.b);
         }
       };
-      if (walk.at(0) >= 0) load_q(walk.at(0));
-      for (int rd = 0, item; (item = walk.at(rd)) >= 0 && ok; ++rd) {
-        const ItemGeom g = item_geom(item, nq, p.H, T, window, STREAMS, p.doc_start, p.doc_sb, p.window_blocks);
+      auto publish = [&](int rd, ItemGeom& g) {
+        const int item = walk.at(rd), slot = rd % NITEM;
+        if (item >= 0) g = item_geom(item, nq, p.H, T, window, STREAMS, p.doc_start, p.doc_sb, p.window_blocks);
+        else g.b = -1;
+        if (!mbar_wait(&bars->i_empty[slot], ((rd / NITEM) & 1) ^ 1, abort_flag, p.status, 14)) { ok = false; return; }
+        bars->item[slot] = g;
+        mbar_arrive(&bars->i_full[slot]);
+      };
+      ItemGeom g, g_next;
+      publish(0, g);
+      if (ok && g.b >= 0) load_q(g);
+      for (int rd = 0; ok && g.b >= 0; ++rd, g = g_next) {
         for (int j = g.jlo; j <= g.jhi && ok; ++j) {
           for (int kv = 0; kv < 2; ++kv, ++n) {
             const int stage = n % NSTAGE;
@@ -257,9 +291,12 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             tma_load_4d(dst, tm, &bars->kv_full[stage], 0, j * BN, g.h, g.b);
             tma_load_4d(dst + HALF_BYTES, tm, &bars->kv_full[stage], 64, j * BN, g.h, g.b);
           }
-          // next item's Q: after this item's first K/V tiles are on their way (its buffer was released when the
-          // previous item issued its last Q K^T, which the ring has long passed by now)
-          if (j == (NQBUF > 1 ? g.jlo : g.jhi) && walk.at(rd + 1) >= 0) load_q(walk.at(rd + 1));
+          // next item's Q.  Its buffer is free when the output of the item before this one, which goes out through it, has been read:
+          // by the time this item's last tiles are asked for.  Raw Q is wanted earlier: it is prepared under this item's second tile
+          if (ok && j == (QRAW ? g.jlo : g.jhi)) {
+            publish(rd + 1, g_next);
+            if (ok && g_next.b >= 0) load_q(g_next);
+          }
         }
       }
     }
@@ -284,8 +321,10 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       uint32_t n_pv[2] = {0, 0};         // P tiles consumed so far per stream (phase of p_full)
       uint32_t n_q[2] = {0, 0};          // Q tiles consumed so far per stream (phase of q_full)
       bool ok = true;
-      for (int rd = 0, item; (item = walk.at(rd)) >= 0 && ok; ++rd) {
-        const ItemGeom g = item_geom(item, nq, p.H, T, window, STREAMS, p.doc_start, p.doc_sb, p.window_blocks);
+      const ItemGeom* item;
+      for (int rd = 0; ok && (item = next_item(rd)); ++rd) {
+        const ItemGeom g = *item;
+        item_done(rd);
         for (int j = g.jlo; j <= g.jhi + 1 && ok; ++j) {
 #pragma unroll
           for (int s = 0; s < 2; ++s) {
@@ -332,7 +371,7 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 umma_ss_lh_p(leader, s_tmem, q_lo + off, qk_hi, k_lo + off, qk_hi, idesc_qk, k > 0 ? 1u : 0u);
               }
               tc_commit_p(leader, &bars->s_full[s]);
-              if (j == g.jhi_s[s]) tc_commit_p(leader, &bars->q_empty[s][q_buf]);     // Q_s may be overwritten by the next item
+              if (NSPLIT == 1 && j == g.jhi_s[s]) tc_commit_p(leader, &bars->q_empty[s][q_buf]);   // Q_s may be overwritten (split form: after the output)
               const bool other_uses = (s == 0) && g.valid[1] && (j >= g.jlo_s[1]) && (j <= g.jhi_s[1]);
               if (!other_uses) tc_commit_p(leader, &bars->kv_empty[stage]);
             }
@@ -349,15 +388,20 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
     const uint32_t s_tmem = tmem_base + lane_off + s * 128 + half * 64;          // this thread's 64 S columns; P over the first 32
     const uint32_t o_tmem = tmem_base + lane_off + 256 + s * 128 + half * 64;    // and its 64 output columns in the epilogue
-    float* lsum = reinterpret_cast<float*>(smem + SMEM_TILES + 256) + s * 128 + row;   // one exchange slot per row
+    float* lsum = reinterpret_cast<float*>(smem + SMEM_TILES + PREFILL_BARS) + s * 128 + row;   // one exchange slot per row
     const uint64_t c2p = pack2f(p.scale_log2, p.scale_log2);
     uint32_t n_s = 0, n_o = 0, n_qs = 0;
     bool ok = true;
     bool q_prepared = false;                                       // raw-Q mode: the lower half prepares the stream's Q rows
-    for (int rd = 0, item; (item = walk.at(rd)) >= 0 && ok; ++rd) {
-      const ItemGeom g = item_geom(item, nq, p.H, T, window, STREAMS, p.doc_start, p.doc_sb, p.window_blocks);
-      if (!g.valid[s]) continue;
-      const int q0 = g.q0[s];
+    const bool out_thread = (warp & 3) == 0 && lane == 0;          // the one that sends this half's output
+    const ItemGeom* item;
+    for (int rd = 0; ok && (item = next_item(rd)); item_done(rd), ++rd) {
+      const int q0 = item->q0[s], jlo = item->jlo_s[s], jhi = item->jhi_s[s];
+      if (jhi < jlo) continue;                                     // no rows of this stream
+      if (out_thread && n_o > 0) {                                 // the previous item's output has left its Q buffer
+        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        mbar_arrive(&bars->q_empty[s][(n_o - 1) % NQBUF]);
+      }
       const int q_row = q0 + row;
       bool next_valid = false;
       int q_row_next = 0;
@@ -374,32 +418,24 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         }
       }
       uint64_t sum_a = pack2f(0.f, 0.f), sum_b = sum_a;
-      // first visible key of this row's document, and the latest such start among the stream's rows
-      const int ds_row = p.doc_start ? min(p.doc_start[g.b * p.doc_sb + min(q_row, T - 1)], q_row) : 0;   // a row always sees itself
-      const int ds_max = p.doc_start ? p.doc_start[g.b * p.doc_sb + min(q0 + BM - 1, T - 1)] : 0;
-      for (int j = g.jlo_s[s]; ok && j <= g.jhi_s[s]; ++j) {
+      // all rows of the stream see all keys of the tiles f_lo .. f_hi
+      int f_lo = window > 0 ? max(q0 + BM + BN - 1 - window, 0) / BN : 0;
+      const int f_hi = q0 / BN - 1;
+      if (p.doc_start) f_lo = max(f_lo, (p.doc_start[item->b * p.doc_sb + min(q0 + BM - 1, T - 1)] + BN - 1) / BN);
+      for (int j = jlo; ok && j <= jhi; ++j) {
         ok = __all_sync(0xffffffffu, mbar_wait(&bars->s_full[s], n_s & 1, abort_flag, p.status, 6));
         if (!ok) break;
         ++n_s;
         tc_fence_after();
-        const int k0 = j * BN + half * 64;                            // key index of this thread's first column
-        const bool full_tile = (j * BN + BN - 1 <= q0) && (window <= 0 || j * BN > q0 + BM - 1 - window) && ds_max <= j * BN;
         uint32_t r[64];
         tmem_ld32(s_tmem, r);
-        tmem_ld32(s_tmem + 32, r + 32);
         tc_wait_ld();
-        if (!full_tile) {
-          const int hi = q_row - k0;                                   // column i is visible iff lo < i <= hi
-          const int lo = max(window > 0 ? q_row - window - k0 : -1, ds_row - 1 - k0);
-#pragma unroll
-          for (int i = 0; i < 64; ++i)
-            if (!(i > lo && i <= hi)) r[i] = 0xff800000u;              // -inf -> weight 0
-        }
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
+        // P of 32 columns and its share of the row sums
+        auto rebuild = [&](int c) {
           uint32_t pk[16];
 #pragma unroll
           for (int i = 0; i < 32; i += 4) {
+            if (c == 0 && i == 16) tmem_ld32(s_tmem + 32, r + 32);       // the other half of the scores, under this one
             const uint64_t xa = fmul2(pack2f(__uint_as_float(r[32 * c + i]), __uint_as_float(r[32 * c + i + 1])), c2p);
             const uint64_t xb = fmul2(pack2f(__uint_as_float(r[32 * c + i + 2]), __uint_as_float(r[32 * c + i + 3])), c2p);
             float x0, x1, p2, p3;
@@ -421,11 +457,43 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             pk[(i >> 1) + 1] = pack_bf16(p2, p3);
           }
           tmem_st16(s_tmem + 16 * c, pk);
+          if (c == 0) tc_wait_ld();
+        };
+        if (j >= f_lo && j <= f_hi) {
+          rebuild(0);
+          rebuild(1);
+        } else {
+          // column i is visible iff lo < i <= hi.  Of a partly visible tile a warp's 32 x 32 piece is mostly all or nothing
+          // (element-wise over all 64 columns: 2000 - 2500 cycles a tile against 1250 for a full one)
+          const int hi = item->q0[s] + row - (j * BN + half * 64);
+          int lo = window > 0 ? hi - window : -1;
+          if (p.doc_start) {                                       // the first key of the row's document; a row always sees itself
+            const int q = item->q0[s] + row;
+            lo = max(lo, hi - q + min(p.doc_start[item->b * p.doc_sb + min(q, T - 1)], q) - 1);
+          }
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            if (!__any_sync(0xffffffffu, hi >= 32 * c && lo < 32 * c + 31)) {
+              const uint32_t zero[16] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+              if (c == 0) tmem_ld32(s_tmem + 32, r + 32);
+              tmem_st16(s_tmem + 16 * c, zero);
+              if (c == 0) tc_wait_ld();
+              continue;
+            }
+            if (!__all_sync(0xffffffffu, hi >= 32 * c + 31 && lo < 32 * c)) {
+              const int b_lo = min(max(lo + 1 - 32 * c, 0), 32), b_hi = min(max(hi + 1 - 32 * c, 0), 32);
+              const uint32_t visible = (uint32_t)(((uint64_t)1 << b_hi) - 1) & ~(uint32_t)(((uint64_t)1 << b_lo) - 1);
+#pragma unroll
+              for (int i = 0; i < 32; ++i)
+                if (!((visible >> i) & 1u)) r[32 * c + i] = 0xff800000u;      // -inf -> weight 0
+            }
+            rebuild(c);
+          }
         }
         tc_wait_st();
         tc_fence_before();
         mbar_arrive(&bars->p_full[s]);
-        if (QRAW && half == 0 && next_valid && !q_prepared && j == g.jlo_s[s] + 1) {   // next item's Q, inside this item
+        if (QRAW && half == 0 && next_valid && !q_prepared && j == jlo + 1) {   // next item's Q, inside this item
           ok = prepare_q_tile(bars, q_tiles, s, row, n_qs, q_row_next, p, abort_flag);
           if (!ok) break;
           q_prepared = true;
@@ -446,7 +514,7 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       if (s == 0) asm volatile("bar.sync 1, 256;" ::: "memory");
       else        asm volatile("bar.sync 2, 256;" ::: "memory");
       if (half == 1) l = *lsum;
-      if (p.lse2 && half == 0 && q_row < T) p.lse2[((int64_t)g.b * p.H + g.h) * T + q_row] = __log2f(l);   // no reference maximum in this form
+      if (p.lse2 && half == 0 && q_row < T) p.lse2[((int64_t)item->b * p.H + item->h) * T + q_row] = __log2f(l);   // no reference maximum in this form
       if (ok) {
         ok = __all_sync(0xffffffffu, mbar_wait(&bars->o_full[s], n_o & 1, abort_flag, p.status, 7));
         ++n_o;
@@ -467,36 +535,25 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           ch[c].z = pack_bf16(__uint_as_float(r[8 * c + 4]) * inv, __uint_as_float(r[8 * c + 5]) * inv);
           ch[c].w = pack_bf16(__uint_as_float(r[8 * c + 6]) * inv, __uint_as_float(r[8 * c + 7]) * inv);
         }
-        // 8 x 8 transpose of chunks inside each group of eight lanes (three butterfly stages): afterwards lane l of
-        // a group holds chunk l of the group's eight rows, so one store instruction writes four whole 128-byte
-        // row segments instead of 32 scattered 16-byte pieces (rows are H*D*2 bytes apart in memory).
+        // out through this item's Q buffer, whose last product was over before O_s was: this half's 64 columns are one swizzled box
+        // (stores from registers, transposed to whole row segments by shuffles, took 2200 cycles an item)
+        uint8_t* box = q_tiles + (((n_o - 1) % NQBUF) * 2 + s) * TILE_BYTES + half * HALF_BYTES;
+        const uint32_t dst = smem_u32(box) + row * 128;
 #pragma unroll
-        for (int m = 4; m >= 1; m >>= 1) {
-          const bool up = (lane & m) != 0;
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            if (i & m) continue;
-            const uint4 send = up ? ch[i] : ch[i | m];
-            uint4 recv;
-            recv.x = __shfl_xor_sync(0xffffffffu, send.x, m);
-            recv.y = __shfl_xor_sync(0xffffffffu, send.y, m);
-            recv.z = __shfl_xor_sync(0xffffffffu, send.z, m);
-            recv.w = __shfl_xor_sync(0xffffffffu, send.w, m);
-            if (up) ch[i] = recv; else ch[i | m] = recv;
-          }
-        }
-        {
-          const int l8 = lane & 7, row_g = q_row - l8;                   // first row of this lane's group
-          __nv_bfloat16* dst = p.out + g.b * p.o_sb + (int64_t)row_g * p.o_st + g.h * p.o_sh + half * 64 + l8 * 8;
-#pragma unroll
-          for (int jr = 0; jr < 8; ++jr)
-            if (row_g + jr < T) *reinterpret_cast<uint4*>(dst + (int64_t)jr * p.o_st) = ch[jr];
+        for (int c = 0; c < 8; ++c)
+          asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst + ((c ^ (row & 7)) << 4)), "r"(ch[c].x), "r"(ch[c].y), "r"(ch[c].z), "r"(ch[c].w) : "memory");
+        fence_proxy_async();
+        named_bar(3 + 2 * s + half, 128);
+        if (out_thread) {
+          tma_store_4d(&tm_o, box, 64 * half, q0, item->h, item->b);       // rows past T stay out of it
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
         // the next item's first PV overwrites O_s only after every thread's P of that item has been signalled,
         // i.e. after these loads: program order is the guard
         tc_fence_before();
       }
     }
+    if (out_thread) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   } else {
     // ------------------------------------------------------------------ softmax + epilogue
     const int s = warp >> 2, quarter = warp & 3;
@@ -510,10 +567,10 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     uint32_t r[128];
     bool q_prepared = false;
     auto prepare_q = [&](int qrow) -> bool { return prepare_q_tile(bars, q_tiles, s, row, n_qs, qrow, p, abort_flag); };
-    for (int rd = 0, item; (item = walk.at(rd)) >= 0 && ok; ++rd) {
-      const ItemGeom g = item_geom(item, nq, p.H, T, window, STREAMS, p.doc_start, p.doc_sb, p.window_blocks);
-      if (!g.valid[s]) continue;
-      const int q0 = g.q0[s];
+    const ItemGeom* item;
+    for (int rd = 0; ok && (item = next_item(rd)); item_done(rd), ++rd) {
+      const int q0 = item->q0[s], jlo = item->jlo_s[s], jhi = item->jhi_s[s];
+      if (jhi < jlo) continue;                                     // no rows of this stream
       const int q_row = q0 + row;
       if (QRAW && !q_prepared) {
         ok = prepare_q(q_row);
@@ -531,10 +588,10 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         q_row_next = gn.q0[s] + row;
       }
       float m_ref = NEG_BIG, l = 0.f, pend = 0.f;   // pend: how far the reference is known to lag (applied before the next P)
-      const int ds_row = p.doc_start ? min(p.doc_start[g.b * p.doc_sb + min(q_row, T - 1)], q_row) : 0;   // a row always sees itself
-      const int ds_max = p.doc_start ? p.doc_start[g.b * p.doc_sb + min(q0 + BM - 1, T - 1)] : 0;
-      for (int j = g.jlo_s[s]; j <= g.jhi_s[s]; ++j) {
-        const bool first = (j == g.jlo_s[s]);
+      const int ds_row = p.doc_start ? min(p.doc_start[item->b * p.doc_sb + min(q_row, T - 1)], q_row) : 0;   // a row always sees itself
+      const int ds_max = p.doc_start ? p.doc_start[item->b * p.doc_sb + min(q0 + BM - 1, T - 1)] : 0;
+      for (int j = jlo; j <= jhi; ++j) {
+        const bool first = (j == jlo);
         ok = __all_sync(0xffffffffu, mbar_wait(&bars->s_full[s], n_s & 1, abort_flag, p.status, 6));
         if (!ok) break;
         ++n_s;
@@ -641,7 +698,7 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         tc_wait_st();
         tc_fence_before();
         mbar_arrive(&bars->p_full[s]);
-        if (QRAW && next_valid && !q_prepared && j == g.jlo_s[s] + 1) {
+        if (QRAW && next_valid && !q_prepared && j == jlo + 1) {
           ok = prepare_q(q_row_next);
           if (!ok) break;
           q_prepared = true;
@@ -654,8 +711,8 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       if (ok) {
         tc_fence_after();
         const float inv = 1.0f / l;
-        if (p.lse2 && q_row < T) p.lse2[((int64_t)g.b * p.H + g.h) * T + q_row] = m_ref + __log2f(l);
-        __nv_bfloat16* dst = p.out + g.b * p.o_sb + (int64_t)q_row * p.o_st + g.h * p.o_sh;
+        if (p.lse2 && q_row < T) p.lse2[((int64_t)item->b * p.H + item->h) * T + q_row] = m_ref + __log2f(l);
+        __nv_bfloat16* dst = p.out + item->b * p.o_sb + (int64_t)q_row * p.o_st + item->h * p.o_sh;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           tmem_ld32(o_tmem + 32 * c, r);
@@ -825,6 +882,10 @@ static int launch_attend(const void* q, const void* k, const void* v,
   if ((rc = daisy_host::make_tmap_bf16_dthb(&tq, q, D, T, H, B, q_st * 2, sb(q_sh, H), sb(q_sb, B), 64, BM)) != DAISY_OK) return rc;
   if ((rc = daisy_host::make_tmap_bf16_dthb(&tk, k, D, T, H, B, k_st * 2, sb(k_sh, H), sb(k_sb, B), 64, BN)) != DAISY_OK) return rc;
   if ((rc = daisy_host::make_tmap_bf16_dthb(&tv, v, D, T, H, B, v_st * 2, sb(v_sh, H), sb(v_sb, B), 64, BN)) != DAISY_OK) return rc;
+  // the split form sends its output through a tensor map; strides that one cannot say (a dimension of stride zero) take the general form
+  CUtensorMap to = tq;
+  const bool out_map = o_st > 0 && (H == 1 || o_sh > 0) && (B == 1 || o_sb > 0) &&
+                       daisy_host::make_tmap_bf16_dthb(&to, out, D, T, H, B, o_st * 2, sb(o_sh, H), sb(o_sb, B), 64, BM) == DAISY_OK;
   PrefillParams p;
   p.out = (__nv_bfloat16*)out; p.o_sb = o_sb; p.o_st = o_st; p.o_sh = o_sh;
   p.T = T; p.H = H; p.B = B;
@@ -838,7 +899,7 @@ static int launch_attend(const void* q, const void* k, const void* v,
   p.lse2 = lse2;
   const bool raw = qt && (qt->norm || qt->rope);
   // with RMS-normalised q and k every logit is bounded by scale * D: 2^(logit - reference) cannot overflow
-  const bool bounded = bounded_qk && scale * 1.4426950408889634f * (float)D <= 60.f;
+  const bool bounded = out_map && bounded_qk && scale * 1.4426950408889634f * (float)D <= 60.f;
   const int sms = daisy_host::sm_count_cached();
   if (sms <= 0) return DAISY_ENODEV;
   // where one wave holds all 128-row tiles each gets an SM: the second stream pays by sharing K and V, not for latency
@@ -851,12 +912,12 @@ static int launch_attend(const void* q, const void* k, const void* v,
   cudaStream_t st = (cudaStream_t)stream;
   // bounded logits take the form with two softmax warpgroups per stream, everything else the general form (a failed launch
   // is what the check below reads)
-  if (raw && solo)          (void)daisy_host::launch_dependent(swa_prefill_kernel<true, true, 2, 1>, dim3(grid), dim3(PREFILL_THREADS_SPLIT), PREFILL_SMEM, st, tq, tk, tv, p);
-  else if (raw && bounded)  (void)daisy_host::launch_dependent(swa_prefill_kernel<true, true, 2, 2>, dim3(grid), dim3(PREFILL_THREADS_SPLIT), PREFILL_SMEM, st, tq, tk, tv, p);
-  else if (raw)             (void)daisy_host::launch_dependent(swa_prefill_kernel<true, false, 1, 2>, dim3(grid), dim3(PREFILL_THREADS), PREFILL_SMEM, st, tq, tk, tv, p);
-  else if (solo)            (void)daisy_host::launch_dependent(swa_prefill_kernel<false, true, 2, 1>, dim3(grid), dim3(PREFILL_THREADS_SPLIT), PREFILL_SMEM, st, tq, tk, tv, p);
-  else if (bounded)         (void)daisy_host::launch_dependent(swa_prefill_kernel<false, true, 2, 2>, dim3(grid), dim3(PREFILL_THREADS_SPLIT), PREFILL_SMEM, st, tq, tk, tv, p);
-  else                      (void)daisy_host::launch_dependent(swa_prefill_kernel<false, false, 1, 2>, dim3(grid), dim3(PREFILL_THREADS), PREFILL_SMEM, st, tq, tk, tv, p);
+  if (raw && solo)          (void)daisy_host::launch_dependent(swa_prefill_kernel<true, true, 2, 1>, dim3(grid), dim3(PREFILL_THREADS_SPLIT), PREFILL_SMEM, st, tq, tk, tv, to, p);
+  else if (raw && bounded)  (void)daisy_host::launch_dependent(swa_prefill_kernel<true, true, 2, 2>, dim3(grid), dim3(PREFILL_THREADS_SPLIT), PREFILL_SMEM, st, tq, tk, tv, to, p);
+  else if (raw)             (void)daisy_host::launch_dependent(swa_prefill_kernel<true, false, 1, 2>, dim3(grid), dim3(PREFILL_THREADS), PREFILL_SMEM, st, tq, tk, tv, to, p);
+  else if (solo)            (void)daisy_host::launch_dependent(swa_prefill_kernel<false, true, 2, 1>, dim3(grid), dim3(PREFILL_THREADS_SPLIT), PREFILL_SMEM, st, tq, tk, tv, to, p);
+  else if (bounded)         (void)daisy_host::launch_dependent(swa_prefill_kernel<false, true, 2, 2>, dim3(grid), dim3(PREFILL_THREADS_SPLIT), PREFILL_SMEM, st, tq, tk, tv, to, p);
+  else                      (void)daisy_host::launch_dependent(swa_prefill_kernel<false, false, 1, 2>, dim3(grid), dim3(PREFILL_THREADS), PREFILL_SMEM, st, tq, tk, tv, to, p);
   DAISY_CHECK_LAUNCH();
   return DAISY_OK;
 }

@@ -3,6 +3,7 @@
 //   * the token-by-token recurrence for short inputs (decode steps): the state S [K x V] of one (batch, head)
 //     lives in registers of one CTA per 32 value columns, is read once, updated T times and written once.
 #include "common.cuh"
+#include "kda_gate.cuh"
 
 namespace daisy {
 
@@ -52,23 +53,7 @@ __global__ void __launch_bounds__(256) kda_gate_kernel(const KdaGateParams p) {
 }
 
 // The same gate, eight elements per thread and one pass per thread (no loop), for D % 8 == 0.  The element-wise
-// arithmetic, not DRAM, bounds the version above (precise expf + log1pf: 0.4 of the copy bandwidth), so softplus is
-// evaluated as  max(z, 0) + log1p(u),  u = exp(-|z|) in (0, 1]  with one ex2.approx and a degree-9 polynomial for
-// log1p(u) / u  (Chebyshev interpolant on [0, 1]; 1.6e-7 relative in fp32 arithmetic).
-__device__ __forceinline__ float log1p_unit(float u) {
-  float r = -0.0031760570127516985f;
-  r = fmaf(r, u, 0.019542528316378593f);
-  r = fmaf(r, u, -0.05637361481785774f);
-  r = fmaf(r, u, 0.10543623566627502f);
-  r = fmaf(r, u, -0.1526966691017151f);
-  r = fmaf(r, u, 0.1966327428817749f);
-  r = fmaf(r, u, -0.24951615929603577f);
-  r = fmaf(r, u, 0.33329710364341736f);
-  r = fmaf(r, u, -0.49999892711639404f);
-  r = fmaf(r, u, 1.0f);
-  return r * u;
-}
-
+// arithmetic, not DRAM, bounds the version above (precise expf + log1pf: 0.4 of the copy bandwidth).
 template <bool IN_BF16, bool ROUND>
 __global__ void __launch_bounds__(256) kda_gate8_kernel(const KdaGateParams p) {
   const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;         // group of eight elements
@@ -94,11 +79,8 @@ __global__ void __launch_bounds__(256) kda_gate8_kernel(const KdaGateParams p) {
   float y[8];
 #pragma unroll
   for (int e = 0; e < 8; ++e) {
-    const float z = x[e] * p.beta;
-    const float u = fast_exp2(fabsf(z) * -1.4426950408889634f);
-    const float sp = z > p.threshold ? x[e] : (fmaxf(z, 0.f) + log1p_unit(u)) * inv_beta;
-    y[e] = a * sp;
-    if (ROUND) y[e] = __uint_as_float(pack_bf16(0.f, y[e]) & 0xffff0000u);
+    y[e] = a * kda_softplus(x[e], p.beta, inv_beta, p.threshold);
+    if (ROUND) y[e] = round_bf16(y[e]);
   }
   float4* dst = reinterpret_cast<float4*>(p.out + i * 8);
   dst[0] = make_float4(y[0], y[1], y[2], y[3]);

@@ -7,7 +7,11 @@
 //              accumulator row (thread = token = TMEM lane); q', k', v' leave as [B,T,H,D] bf16 and the separate
 //              norm/RoPE pass over q, k, v (1.6 GB at B=8, T=8192, 16 heads) disappears.
 //   EPI_PLAIN  bf16 store of C (the output projection); up to three products of one shape in one launch (the Kimi layer's
-//              q, k and v projections: 3 x 192 tiles in 8 waves instead of 3 x 3).
+//              q, k and v projections: 3 x 192 tiles in 8 waves instead of 3 x 3).  Two of the Kimi layer's groups end in its
+//              gates: beside the two low-rank products a third of H columns leaves as sigmoid(C) in float32 (the write
+//              strength), and the first of the two that follow as  -exp(A_log) softplus(C + dt_bias)  (the log-decay).
+//              2 x 3001 tokens, 16 heads: 12.5 + 8.6 + 2.7 us (low-rank products, library product, sigmoid) -> 18.3, 18 + 18.4
+//              (second products, gate) -> 33.9; 2 x 127, 12 heads: the layer 86 -> 65 us with three launches fewer.
 //
 // Persistent CTAs walk 128 x BN output tiles (n fastest, so concurrently running CTAs share X tiles and the
 // whole W in L2).  Roles (352 threads): warps 0-7 epilogue, warp 8 MMA issuer, warps 9, 10 TMA producers.  Both
@@ -21,6 +25,7 @@
 // 128 x 256 tile; rank 0 issues the MMAs, both CTAs run the epilogue on their own 128 accumulator rows.
 // All mbarrier waits are bounded (abort flag, DAISY_ETIMEOUT through the status word), as everywhere else.
 #include "common.cuh"
+#include "kda_gate.cuh"
 #include <cuda_fp16.h>
 
 namespace daisy {
@@ -50,6 +55,10 @@ struct GemmParams {
   // plain: up to GROUP products of one shape, columns [i per, (i + 1) per) of N are product i's
   __nv_bfloat16* c[GROUP]; int64_t ldc;
   int per;
+  // plain: product 0 as the log-decay gate [M, per] float32; product 2 as sigmoid [M, beta_n] float32, of beta_n weight rows; or null
+  float *gate, *beta;
+  const float *a_log, *dt_bias;
+  int beta_n;
   // qkv
   __nv_bfloat16* out[3];         // q', k', v'  [M, H, 128]
   const float *cos, *sin;        // [T, 64]
@@ -80,6 +89,43 @@ __device__ __forceinline__ float4 ld_shared_f4(uint32_t addr) {
   asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
   return v;
 }
+
+// Two products that end in a gate take what a bf16 store of the product would have left.
+// a softplus(bf16(c) + bias), rounded to bf16, of N pairs side by side, each step for all of them before the next (left to itself a
+// warp goes through one chain of twenty dependent instructions after the other: 61 us instead of 34 at 6002 x 2048).  softplus is that of
+// kda_gate.cuh; its threshold of 20 changes nothing here, where log1p(e^-20) is far below an ulp of 20.
+template <int N>
+__device__ __forceinline__ void gemm_decay2(uint64_t (&c)[N], const uint64_t (&bias)[2], float a) {
+  uint64_t u[N], r[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    float x0, x1;
+    unpack2f(c[i], x0, x1);
+    const uint32_t b = pack_bf16(x0, x1);
+    c[i] = fadd2(pack2f(bf16_lo(b), bf16_hi(b)), bias[i & 1]);
+  }
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    float x0, x1;
+    unpack2f(c[i], x0, x1);
+    u[i] = pack2f(fast_exp2(fabsf(x0) * -1.4426950408889634f), fast_exp2(fabsf(x1) * -1.4426950408889634f));
+    r[i] = pack2f(LOG1P_C[0], LOG1P_C[0]);
+  }
+#pragma unroll
+  for (int k = 1; k < 10; ++k)
+#pragma unroll
+    for (int i = 0; i < N; ++i) r[i] = ffma2(r[i], u[i], pack2f(LOG1P_C[k], LOG1P_C[k]));
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    float x0, x1, y0, y1;
+    unpack2f(c[i], x0, x1);
+    unpack2f(fmul2(fadd2(pack2f(fmaxf(x0, 0.f), fmaxf(x1, 0.f)), fmul2(r[i], u[i])), pack2f(a, a)), y0, y1);
+    const uint32_t b = pack_bf16(y0, y1);
+    c[i] = pack2f(bf16_lo(b), bf16_hi(b));
+  }
+}
+__device__ __forceinline__ float gemm_sigmoid(float c) { return round_bf16(1.f / (1.f + expf(-round_bf16(c)))); }
+constexpr int BETA_MAX = 32;
 
 struct GemmBars {
   uint64_t full[6], empty[6];
@@ -218,14 +264,56 @@ qkv_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p) {
       ok = __all_sync(0xffffffffu, mbar_wait(&bars->acc_full[buf], (it >> 1) & 1, abort_flag, p.status, 4));
       if (!ok) { if (QKV) cp_async_wait<0>(); break; }
       tc_fence_after();
-      {
+      const uint32_t t0 = tmem_base + lane_off + buf * BN + (PAIR ? grp * 128 : 0);
+      if (!QKV && p.gate && n0 < p.per) {
+        // 32 columns at a time, transposed through the staging rows: a lane then has four columns of eight rows, eight lanes 128
+        // bytes of a row
+        const float a = -expf(__ldg(p.a_log + (n0 >> 7)));
+#pragma unroll 1
+        for (int q = 0; q < 4; ++q) {
+          uint32_t r[32];
+          tmem_ld32(t0 + 32 * q, r);
+          const int c = 4 * (lane & 7);
+          const float4 bias = __ldg(reinterpret_cast<const float4*>(p.dt_bias + n0 + 32 * q + c));
+          tc_wait_ld();
+#pragma unroll
+          for (int i = 0; i < 8; ++i) *reinterpret_cast<uint4*>(stg + lane * 128 + ((i ^ (lane & 7)) << 4)) = make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
+          __syncwarp();
+          float* dst = p.gate + (size_t)(m0 + (warp & 3) * 32) * p.per + n0 + 32 * q + c;
+          const uint64_t bias2[2] = {pack2f(bias.x, bias.y), pack2f(bias.z, bias.w)};
+          uint64_t v[16];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int rr = 4 * i + (lane >> 3);
+            const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(stg + rr * 128 + (((lane ^ rr) & 7) << 4));
+            v[2 * i] = t.x; v[2 * i + 1] = t.y;
+          }
+          gemm_decay2(v, bias2, a);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int rr = 4 * i + (lane >> 3);
+            if (m0 + (warp & 3) * 32 + rr < p.M) *reinterpret_cast<ulonglong2*>(dst + (size_t)rr * p.per) = make_ulonglong2(v[2 * i], v[2 * i + 1]);
+          }
+          __syncwarp();
+        }
+        tc_fence_before();
+        if (PAIR) mbar_arrive_cluster(mapa_shared(smem_u32(&bars->acc_empty[buf]), 0));
+        else mbar_arrive(&bars->acc_empty[buf]);
+      } else {
         uint32_t r[128];
-        const uint32_t t0 = tmem_base + lane_off + buf * BN + (PAIR ? grp * 128 : 0);
         tmem_ld32(t0, r); tmem_ld32(t0 + 32, r + 32); tmem_ld32(t0 + 64, r + 64); tmem_ld32(t0 + 96, r + 96);
         tc_wait_ld();
         tc_fence_before();                                         // accumulator read out: the MMA warp may refill it
         if (PAIR) mbar_arrive_cluster(mapa_shared(smem_u32(&bars->acc_empty[buf]), 0));   // the issuer waits for both CTAs
         else mbar_arrive(&bars->acc_empty[buf]);
+        if (!QKV && p.beta && n0 >= 2 * p.per) {
+          if (m < p.M) {
+#pragma unroll
+            for (int i = 0; i < BETA_MAX; ++i)
+              if (i < p.beta_n) p.beta[(size_t)m * p.beta_n + i] = gemm_sigmoid(__uint_as_float(r[i]));
+          }
+          continue;
+        }
         __nv_bfloat16* dst_row;                                    // this thread's output row (128 bf16)
         uint8_t* ring_row = nullptr;
         if (QKV) {
@@ -404,7 +492,8 @@ small_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p, con
     tmem_alloc(&bars->tmem_base, BN);
     tmem_relinquish();
   } else if (prefetch && bm == 0 && threadIdx.x < BN) {
-    l2_prefetch_bulk(w.p[prod] + (int64_t)(threadIdx.x < HB ? w_lo + threadIdx.x : w_hi + (int)threadIdx.x - HB) * ldw, (uint32_t)p.K * 2u);
+    const int wr = (int)threadIdx.x < HB ? w_lo + (int)threadIdx.x : w_hi + (int)threadIdx.x - HB;
+    if (QKV || !p.beta || prod < 2 || wr < p.beta_n) l2_prefetch_bulk(w.p[prod] + (int64_t)wr * ldw, (uint32_t)p.K * 2u);
   }
   if (warp == 4 && lane == 0) { prefetch_tmap(&maps.x[prod]); prefetch_tmap(&maps.w[prod]); }
   tc_fence_before();
@@ -507,7 +596,27 @@ small_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p, con
         }
       }
     }
-    if (mine) {
+    if (!QKV && p.gate && prod == 0) {
+      if (mine) {
+        const float a = -expf(__ldg(p.a_log + (w_lo >> 7)));
+        float4* d = reinterpret_cast<float4*>(p.gate + (size_t)m * p.per + w_lo);
+        const float4* bp = reinterpret_cast<const float4*>(p.dt_bias + w_lo);
+#pragma unroll
+        for (int i = 0; i < BN / 4; ++i) {
+          const float4 bias = __ldg(bp + i);
+          const uint64_t bias2[2] = {pack2f(bias.x, bias.y), pack2f(bias.z, bias.w)};
+          uint64_t v[2] = {pack2f(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1])), pack2f(__uint_as_float(r[4 * i + 2]), __uint_as_float(r[4 * i + 3]))};
+          gemm_decay2(v, bias2, a);
+          *reinterpret_cast<ulonglong2*>(d + i) = make_ulonglong2(v[0], v[1]);
+        }
+      }
+    } else if (!QKV && p.beta && prod == 2) {
+      if (mine) {
+#pragma unroll
+        for (int i = 0; i < (BN < BETA_MAX ? BN : BETA_MAX); ++i)
+          if (w_lo + i < p.beta_n) p.beta[(size_t)m * p.beta_n + w_lo + i] = gemm_sigmoid(__uint_as_float(r[i]));
+      }
+    } else if (mine) {
       uint32_t hv[HB];                                                                   // bf16 pairs: HB / 2 low, HB / 2 high
       const bool gated = QKV && which == 2 && p.ve;
       // where the high columns follow the low ones, in 16-byte units
@@ -622,7 +731,8 @@ static int make_maps(GemmMaps& maps, const void* const* x, int64_t ldx, int x_ro
   for (int i = 0; i < n; ++i) {
     int rc = daisy_host::make_tmap_bf16_3d(&maps.x[i], x[i], p.K, p.M, 1, (uint64_t)ldx * 2, (uint64_t)ldx * 2 * p.M, GK, x_rows);
     if (rc != DAISY_OK) return rc;
-    rc = daisy_host::make_tmap_bf16_3d(&maps.w[i], w[i], p.K, p.per, 1, (uint64_t)ldw * 2, (uint64_t)ldw * 2 * p.per, GK, w_rows);
+    const int rows = p.beta && i == 2 ? p.beta_n : p.per;              // rows past the last read as zeros
+    rc = daisy_host::make_tmap_bf16_3d(&maps.w[i], w[i], p.K, rows, 1, (uint64_t)ldw * 2, (uint64_t)ldw * 2 * rows, GK, w_rows);
     if (rc != DAISY_OK) return rc;
   }
   for (int i = n; i < GROUP; ++i) { maps.x[i] = maps.x[0]; maps.w[i] = maps.w[0]; }
@@ -720,6 +830,29 @@ extern "C" int daisy_b200_gemm_nt_group(const void* const* x, int64_t ldx, const
   }
   if ((ldc & 7) || ldc < N) return DAISY_EALIGN;
   return gemm_common(x, ldx, w, ldw, n, p, stream);
+}
+
+extern "C" int daisy_b200_kda_low_rank(const void* x, int64_t ldx, const void* f0_w, const void* g0_w, const void* b_w, void* f0, void* g0, float* beta,
+                                       int M, int H, int dim, int* status_word, void* stream) {
+  if (!f0 || !g0 || !beta || H <= 0) return DAISY_EINVAL;
+  if (H > BETA_MAX) return DAISY_EUNSUPPORTED;
+  if (!daisy_aligned16(f0) || !daisy_aligned16(g0)) return DAISY_EALIGN;
+  const void *xs[3] = {x, x, x}, *w[3] = {f0_w, g0_w, b_w};
+  GemmParams p{};
+  p.M = M; p.per = 128; p.K = dim; p.ldc = 128; p.status = status_word;
+  p.c[0] = (__nv_bfloat16*)f0; p.c[1] = (__nv_bfloat16*)g0; p.beta = beta; p.beta_n = H;
+  return gemm_common(xs, ldx, w, dim, 3, p, stream);
+}
+
+extern "C" int daisy_b200_kda_gates(const void* f0, const void* g0, const void* f1_w, const void* g1_w, const float* a_log, const float* dt_bias,
+                                    float* g, void* gate, int M, int H, int* status_word, void* stream) {
+  if (!a_log || !dt_bias || !g || !gate || H <= 0) return DAISY_EINVAL;
+  if (!daisy_aligned16(dt_bias) || !daisy_aligned16(g) || !daisy_aligned16(gate)) return DAISY_EALIGN;
+  const void *xs[2] = {f0, g0}, *w[2] = {f1_w, g1_w};
+  GemmParams p{};
+  p.M = M; p.per = H * 128; p.K = 128; p.ldc = p.per; p.status = status_word;
+  p.c[1] = (__nv_bfloat16*)gate; p.gate = g; p.a_log = a_log; p.dt_bias = dt_bias;
+  return gemm_common(xs, 128, w, 128, 2, p, stream);
 }
 
 extern "C" int daisy_b200_gemm_nt(const void* x, int64_t ldx, const void* w, int64_t ldw, void* c, int64_t ldc,

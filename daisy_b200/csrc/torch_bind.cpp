@@ -780,20 +780,36 @@ std::tuple<Tensor, OptTensor, std::vector<Tensor>> kimi_layer(const Tensor& x, c
     check(daisy_b200_kda_short_conv_group(step, xp + i, T * C, C, wp + i, bp + i, sp + i, op + i, yp + i, T * C, C, (int)B, (int)T, (int)C, (int)W[i],
                                           packed ? p.tok.data_ptr<int32_t>() : nullptr, silu ? DAISY_KDA_CONV_SILU : 0, stream_of(x)),
           "daisy_b200_kda_short_conv_group");
-  Tensor low[2], up[2];                                                                    // the two low-rank projections: decay gate, output gate
-  kimi_linears({x, x}, {w[3], w[5]}, low);
-  kimi_linears({low[0], low[1]}, {w[4], w[6]}, up);
-  const Tensor &f = up[0], &gp = up[1];
-  Tensor g = at::empty({B, T, H, 128}, x.options().dtype(at::kFloat));
-  check(daisy_b200_kda_gate(f.data_ptr(), 1, a_log.data_ptr<float>(), dt_bias.data_ptr<float>(), g.data_ptr<float>(), M, (int)H, 128, 1.f, 20.f,
-                            DAISY_KDA_GATE_ROUND_BF16, stream_of(x)),
-        "daisy_b200_kda_gate");
-  Tensor bx = at::linear(x, w[7]), beta;
-  if (bx.scalar_type() == at::kBFloat16) {
-    beta = at::empty(bx.sizes(), bx.options().dtype(at::kFloat));
-    check(daisy_b200_kda_beta(bx.data_ptr(), beta.data_ptr<float>(), beta.numel(), stream_of(x)), "daisy_b200_kda_beta");
+  Tensor g = at::empty({B, T, H, 128}, x.options().dtype(at::kFloat)), gp, beta;
+  bool fused = M >= 64 && H <= 32 && x.scalar_type() == at::kBFloat16 && C == x.size(2) && x.is_contiguous() && on16(x) && on16(dt_bias);
+  for (int i = 3; i < 8; ++i) fused = fused && w[i].scalar_type() == at::kBFloat16 && w[i].is_contiguous() && on16(w[i]) && w[i].size(0) == (i == 7 ? H : i % 2 ? 128 : C);
+  if (fused) {                                                                             // low-rank products and write strength, then both gates
+    Tensor low = at::empty({2, M, 128}, x.options());
+    beta = at::empty({B, T, H}, g.options());
+    gp = at::empty({B, T, C}, x.options());
+    void *f0 = low.data_ptr(), *g0 = low.select(0, 1).data_ptr();
+    check(daisy_b200_kda_low_rank(x.data_ptr(), C, w[3].data_ptr(), w[5].data_ptr(), w[7].data_ptr(), f0, g0, beta.data_ptr<float>(), (int)M, (int)H, (int)C,
+                                  status_ptr(x), stream_of(x)),
+          "daisy_b200_kda_low_rank");
+    check(daisy_b200_kda_gates(f0, g0, w[4].data_ptr(), w[6].data_ptr(), a_log.data_ptr<float>(), dt_bias.data_ptr<float>(), g.data_ptr<float>(), gp.data_ptr(), (int)M,
+                               (int)H, status_ptr(x), stream_of(x)),
+          "daisy_b200_kda_gates");
   } else {
-    beta = bx.sigmoid_().to(at::kFloat);
+    Tensor low[2], up[2];                                                                    // the two low-rank projections: decay gate, output gate
+    kimi_linears({x, x}, {w[3], w[5]}, low);
+    kimi_linears({low[0], low[1]}, {w[4], w[6]}, up);
+    const Tensor& f = up[0];
+    gp = up[1];
+    check(daisy_b200_kda_gate(f.data_ptr(), 1, a_log.data_ptr<float>(), dt_bias.data_ptr<float>(), g.data_ptr<float>(), M, (int)H, 128, 1.f, 20.f,
+                              DAISY_KDA_GATE_ROUND_BF16, stream_of(x)),
+          "daisy_b200_kda_gate");
+    Tensor bx = at::linear(x, w[7]);
+    if (bx.scalar_type() == at::kBFloat16) {
+      beta = at::empty(bx.sizes(), bx.options().dtype(at::kFloat));
+      check(daisy_b200_kda_beta(bx.data_ptr(), beta.data_ptr<float>(), beta.numel(), stream_of(x)), "daisy_b200_kda_beta");
+    } else {
+      beta = bx.sigmoid_().to(at::kFloat);
+    }
   }
   std::pair<Tensor, OptTensor> r = packed ? kda_chunk(qkv[0], qkv[1], qkv[2], g, beta, std::nullopt, rec, use_cache, true, false, &p)
                                    : T <= RECURRENT_MAX_T ? kda_recurrent(qkv[0], qkv[1], qkv[2], g, beta, std::nullopt, rec, use_cache, true, false, rec.has_value())

@@ -398,6 +398,16 @@ int daisy_b200_kda_chunk_fwd(const void* q, const void* k, const void* v, const 
                              unsigned flags, void* workspace, size_t workspace_bytes,
                              int* status_word, void* stream);
 
+/* The Kimi layer's narrow projections with their element-wise ends (models/daisy/attention_kimi.py:128-134), bf16 in:
+ *   kda_low_rank   f0, g0 [M,128] bf16 = x f0_w^T, x g0_w^T;  beta [M,H] float32 = bf16(sigmoid(bf16(x b_w^T))).  x [M,dim] (row
+ *                  stride ldx), f0_w, g0_w [128,dim], b_w [H,dim], H <= 32.  One launch.
+ *   kda_gates      g [M,H*128] float32 = bf16(-exp(a_log[h]) softplus(bf16(f0 f1_w^T) + dt_bias)), threshold 20;  gate [M,H*128]
+ *                  bf16 = g0 g1_w^T.  f1_w, g1_w [H*128,128].  One launch. */
+int daisy_b200_kda_low_rank(const void* x, int64_t ldx, const void* f0_w, const void* g0_w, const void* b_w, void* f0, void* g0, float* beta,
+                            int M, int H, int dim, int* status_word, void* stream);
+int daisy_b200_kda_gates(const void* f0, const void* g0, const void* f1_w, const void* g1_w, const float* a_log, const float* dt_bias,
+                         float* g, void* gate, int M, int H, int* status_word, void* stream);
+
 /* Packed variable-length form of the same call: chunk_kda(..., cu_seqlens=cu_seqlens) at
  * models/daisy/attention_kimi.py:133-134, with cu_seqlens from get_unpad_data (:150-154; helpers :19-33).  The
  * sequences lie end to end in one row: q, k [1, T_total, H, K], v, o [1, T_total, H, V], g fp32, beta [1, T_total, H];

@@ -416,3 +416,36 @@ def test_short_conv_varlen_against_fla_triton():
         y, s = ours(x=x, cache=None, output_final_state=True, cu_seqlens=cu_t)
     assert_close_bf16(y, y_ref.float().cpu(), "varlen conv vs fla")
     assert s.shape == s_ref.shape and torch.equal(s.float().cpu(), s_ref.float().cpu())
+
+
+@pytest.mark.parametrize("M,H", [(1, 1), (64, 6), (131, 1), (131, 16), (700, 32), (3001, 6), (6002, 16)])
+def test_projections_that_end_in_gates(M, H):
+    """kda_low_rank and kda_gates (narrow tiles, 128-column tiles, CTA pairs; rows and heads off the tiles' edges) against the
+    products and the element-wise gate in launches of their own: the same bits but for the write strength, whose product is summed
+    in another order (one bf16 step before and one after the sigmoid, whose slope is at most 1/4)."""
+    from daisy_b200 import _lib, ops
+    L, dim = _lib.lib(), H * 128
+    torch.manual_seed(M + H)
+    rnd = lambda *s, std=1.0: torch.randn(*s, device="cuda").mul_(std).bfloat16()
+    x, f0_w, g0_w, b_w = rnd(M, dim), rnd(128, dim, std=dim ** -0.5), rnd(128, dim, std=dim ** -0.5), rnd(H, dim, std=2 * dim ** -0.5)
+    f1_w, g1_w = rnd(dim, 128, std=0.3), rnd(dim, 128, std=0.3)
+    a_log, dt_bias = torch.rand(H, device="cuda").mul_(2.7), torch.randn(dim, device="cuda").mul_(4)     # both sides of the threshold
+    f0, g0 = torch.full((2, M, 128), float("nan"), device="cuda", dtype=torch.bfloat16)
+    beta = torch.full((M + 1, H), -7.0, device="cuda")
+    g = torch.full((M + 1, dim), -7.0, device="cuda")
+    gate = torch.full((M + 1, dim), -7.0, device="cuda", dtype=torch.bfloat16)
+    st, status = torch.cuda.current_stream().cuda_stream, ops.status_word(x.device).data_ptr()
+    assert L.daisy_b200_kda_low_rank(x.data_ptr(), dim, f0_w.data_ptr(), g0_w.data_ptr(), b_w.data_ptr(), f0.data_ptr(), g0.data_ptr(), beta.data_ptr(),
+                                     M, H, dim, status, st) == 0
+    assert L.daisy_b200_kda_gates(f0.data_ptr(), g0.data_ptr(), f1_w.data_ptr(), g1_w.data_ptr(), a_log.data_ptr(), dt_bias.data_ptr(), g.data_ptr(),
+                                  gate.data_ptr(), M, H, status, st) == 0
+    ops.check_device_status("cuda")
+    assert bool((beta[M] == -7).all()) and bool((g[M] == -7).all()) and bool((gate[M] == -7).all())          # nothing past the last row
+    assert torch.equal(f0, ops.gemm_nt(x, f0_w)) and torch.equal(g0, ops.gemm_nt(x, g0_w))
+    assert torch.equal(gate[:M], ops.gemm_nt(g0, g1_w))
+    assert torch.equal(g[:M], ops.kda_gate(ops.gemm_nt(f0, f1_w), a_log, 128, dt_bias).reshape(M, dim))
+    z = x.double() @ b_w.double().t()
+    tol = 2 ** -8 * (0.25 * z.abs() + 1) + 1e-3
+    assert bool(((beta[:M].double() - z.sigmoid()).abs() <= tol).all())
+    assert L.daisy_b200_kda_low_rank(x.data_ptr(), dim, f0_w.data_ptr(), g0_w.data_ptr(), b_w.data_ptr(), f0.data_ptr(), g0.data_ptr(), beta.data_ptr(),
+                                     M, 33, dim, status, st) == _lib.EUNSUPPORTED

@@ -297,6 +297,56 @@ __global__ void __launch_bounds__(256) kda_beta_kernel(const __nv_bfloat16* x, f
   if (i < n) out[i] = __bfloat162float(__float2bfloat16_rn(1.f / (1.f + expf(-__bfloat162float(x[i])))));
 }
 
+// ---------------------------------------------------------------------------------------------
+// Rows of a padded batch [B, T] <-> the packed row of its kept tokens.  One block per batch row numbers the kept tokens: rank
+// [B, T] (-1: padding), idx [B, T] (token of each number), len [B].  (sum, nonzero, cumsum, pad, max, gather, fill, index_copy as
+// tensor operations are a dozen launches and three waits for the device.)
+template <typename E>
+__global__ void __launch_bounds__(1024) kda_mask_rows_kernel(const E* mask, int64_t ld, int T, int* rank, int* idx, int* len) {
+  __shared__ int sums[32];
+  const int b = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  grid_dep_launch();
+  grid_dep_wait();
+  int base = 0;
+  for (int t0 = 0; t0 < T; t0 += 1024) {
+    const int t = t0 + tid;
+    const bool keep = t < T && mask[(int64_t)b * ld + t] != 0;
+    const unsigned m = __ballot_sync(0xffffffffu, keep);
+    if (lane == 0) sums[warp] = __popc(m);
+    __syncthreads();
+    int before = base, all = 0;
+#pragma unroll 8
+    for (int w = 0; w < 32; ++w) { const int s = sums[w]; before += w < warp ? s : 0; all += s; }
+    if (t < T) {
+      const int r = before + __popc(m & ((1u << lane) - 1));
+      rank[(int64_t)b * T + t] = keep ? r : -1;
+      if (keep) idx[(int64_t)b * T + r] = t;
+    }
+    base += all;
+    __syncthreads();
+  }
+  if (tid == 0) len[b] = base;
+}
+// a thread moves 16 bytes; n8 = dim / 8 of them to a row
+__global__ void __launch_bounds__(256) kda_pack_rows_kernel(const uint4* x, const int* idx, const int2* tok, uint4* y, int64_t n, int n8, int T) {
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  grid_dep_launch();
+  grid_dep_wait();
+  if (i >= n) return;
+  const int64_t r = i / n8;
+  const int2 s = __ldg(tok + r);                       // its sequence's first token, its sequence
+  y[i] = __ldg(x + ((int64_t)s.y * T + idx[(int64_t)s.y * T + (r - s.x)]) * n8 + (i - r * n8));
+}
+__global__ void __launch_bounds__(256) kda_unpack_rows_kernel(const uint4* y, const int* rank, const int* cu, uint4* out, int64_t n, int n8, int T) {
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  grid_dep_launch();
+  grid_dep_wait();
+  if (i >= n) return;
+  const int64_t r = i / n8;
+  const int k = rank[r];
+  out[i] = k < 0 ? make_uint4(0, 0, 0, 0) : y[((int64_t)cu[r / T] + k) * n8 + (i - r * n8)];
+}
+
 template <int MODE>
 static void launch_out_norm(const OutNormParams& p, unsigned grid, cudaStream_t st) {
   if (p.o_fp32) (void)daisy_host::launch_dependent(kda_out_norm_kernel<MODE, true>, dim3(grid), dim3(256), 0, st, p);
@@ -371,6 +421,51 @@ extern "C" int daisy_b200_kda_beta(const void* x, float* out, int64_t n, void* s
   if (!x || !out || n <= 0) return DAISY_EINVAL;
   if ((n + 255) / 256 > 0x7fffffffLL) return DAISY_EUNSUPPORTED;
   (void)daisy_host::launch_dependent(kda_beta_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, (cudaStream_t)stream, (const __nv_bfloat16*)x, out, (long long)n);
+  DAISY_CHECK_LAUNCH();
+  return DAISY_OK;
+}
+
+extern "C" int daisy_b200_kda_mask_rows(const void* mask, int elem_bytes, int64_t ld, int B, int T, int32_t* rank, int32_t* idx, int32_t* len, void* stream) {
+  if (!mask || !rank || !idx || !len || B <= 0 || T <= 0 || ld < 0) return DAISY_EINVAL;
+  const auto go = [&](auto e) {
+    typedef decltype(e) E;
+    return daisy_host::launch_dependent(kda_mask_rows_kernel<E>, dim3((unsigned)B), dim3(1024), 0, (cudaStream_t)stream, (const E*)mask, ld, T, rank, idx, len);
+  };
+  if (elem_bytes == 1) (void)go((int8_t)0);
+  else if (elem_bytes == 4) (void)go((int32_t)0);
+  else if (elem_bytes == 8) (void)go((int64_t)0);
+  else return DAISY_EUNSUPPORTED;
+  DAISY_CHECK_LAUNCH();
+  return DAISY_OK;
+}
+
+static int kda_rows_grid(const void* a, const void* b, int64_t rows, int dim, unsigned& grid) {
+  if (rows <= 0 || dim <= 0) return DAISY_EINVAL;
+  if (dim % 8) return DAISY_EUNSUPPORTED;
+  if (!daisy_aligned16(a) || !daisy_aligned16(b)) return DAISY_EALIGN;
+  const int64_t blocks = (rows * (dim / 8) + 255) / 256;
+  if (blocks > 0x7fffffff) return DAISY_EUNSUPPORTED;
+  grid = (unsigned)blocks;
+  return DAISY_OK;
+}
+
+extern "C" int daisy_b200_kda_pack_rows(const void* x, const int32_t* idx, const int32_t* token_tab, void* y, int total, int T, int dim, void* stream) {
+  unsigned grid;
+  if (!x || !idx || !token_tab || !y || T <= 0) return DAISY_EINVAL;
+  if (reinterpret_cast<uintptr_t>(token_tab) & 7) return DAISY_EALIGN;
+  if (const int rc = kda_rows_grid(x, y, total, dim, grid); rc != DAISY_OK) return rc;
+  (void)daisy_host::launch_dependent(kda_pack_rows_kernel, dim3(grid), dim3(256), 0, (cudaStream_t)stream, (const uint4*)x, idx, (const int2*)token_tab, (uint4*)y,
+                                     (int64_t)total * (dim / 8), dim / 8, T);
+  DAISY_CHECK_LAUNCH();
+  return DAISY_OK;
+}
+
+extern "C" int daisy_b200_kda_unpack_rows(const void* y, const int32_t* rank, const int32_t* cu, void* out, int B, int T, int dim, void* stream) {
+  unsigned grid;
+  if (!y || !rank || !cu || !out || B <= 0 || T <= 0) return DAISY_EINVAL;
+  if (const int rc = kda_rows_grid(y, out, (int64_t)B * T, dim, grid); rc != DAISY_OK) return rc;
+  (void)daisy_host::launch_dependent(kda_unpack_rows_kernel, dim3(grid), dim3(256), 0, (cudaStream_t)stream, (const uint4*)y, rank, cu, (uint4*)out,
+                                     (int64_t)B * T * (dim / 8), dim / 8, T);
   DAISY_CHECK_LAUNCH();
   return DAISY_OK;
 }

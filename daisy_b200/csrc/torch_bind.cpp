@@ -566,7 +566,7 @@ Lengths lengths_of(const py::object& cu_seqlens) {
 }
 
 // Tables of a packed batch on the device (see kda_varlen_tables); tok only if asked for.
-struct Packed { Tensor chunks, ptr, tok; int64_t n_chunks = 0, n_seq = 0, total = 0; };
+struct Packed { Tensor chunks, ptr, tok, cu; int64_t n_chunks = 0, n_seq = 0, total = 0; };
 // `meanwhile(n_seq)` runs while lengths that lie on the device are on their way.
 Packed pack_tables(const Lengths& lengths, c10::Device dev, int64_t chunk, bool want_tok, const std::function<void(int64_t)>& meanwhile = {}) {
   TORCH_CHECK_VALUE(chunk > 0, "chunk must be positive, got ", chunk);
@@ -593,8 +593,9 @@ Packed pack_tables(const Lengths& lengths, c10::Device dev, int64_t chunk, bool 
   p.n_seq = (int64_t)cu.size() - 1;
   p.total = cu.back();
   for (int64_t n = 0; n < p.n_seq; ++n) p.n_chunks += (cu[n + 1] - cu[n] + chunk - 1) / chunk;
-  // one staging buffer, one copy: [n_chunks][2], [n_seq + 1] (padded to 8 bytes), [total][2]
-  const int64_t at_ptr = 2 * p.n_chunks, at_tok = at_ptr + (p.n_seq + 2) / 2 * 2, size = at_tok + (want_tok ? 2 * p.total : 0);
+  // one staging buffer, one copy: [n_chunks][2], [n_seq + 1] (padded to 8 bytes), [total][2], [n_seq + 1]
+  const int64_t at_ptr = 2 * p.n_chunks, at_tok = at_ptr + (p.n_seq + 2) / 2 * 2, at_cu = at_tok + (want_tok ? 2 * p.total : 0);
+  const int64_t size = at_cu + (want_tok ? p.n_seq + 1 : 0);
   Tensor host = at::empty({std::max<int64_t>(size, 1)}, at::TensorOptions().dtype(at::kInt).pinned_memory(dev.is_cuda()));
   int32_t* h = host.data_ptr<int32_t>();
   int64_t c = 0;
@@ -606,10 +607,11 @@ Packed pack_tables(const Lengths& lengths, c10::Device dev, int64_t chunk, bool 
   }
   h[at_ptr + p.n_seq] = (int32_t)c;
   for (int64_t i = at_ptr + p.n_seq + 1; i < at_tok; ++i) h[i] = 0;
+  for (int64_t n = 0; want_tok && n <= p.n_seq; ++n) h[at_cu + n] = (int32_t)cu[n];
   Tensor d = host.to(dev, /*non_blocking=*/true);
   p.chunks = d.narrow(0, 0, 2 * p.n_chunks).view({p.n_chunks, 2});
   p.ptr = d.narrow(0, at_ptr, p.n_seq + 1);
-  if (want_tok) p.tok = d.narrow(0, at_tok, 2 * p.total).view({p.total, 2});
+  if (want_tok) { p.tok = d.narrow(0, at_tok, 2 * p.total).view({p.total, 2}); p.cu = d.narrow(0, at_cu, p.n_seq + 1); }
   return p;
 }
 
@@ -742,16 +744,44 @@ void kimi_linears(std::vector<Tensor> x, std::vector<Tensor> w, Tensor* y) {
 }
 
 // weights: q, k, v, f0, f1, g0, g1, b, o.  conv_s, rec: carried states or nothing.  -> y, final state, convolution states
-std::tuple<Tensor, OptTensor, std::vector<Tensor>> kimi_layer(const Tensor& x, const std::vector<Tensor>& w, const OptTensor& g1_bias, const OptTensor& norm_w,
+// With a mask [B, T] the kept tokens of all rows are one packed row, one sequence per batch row, and y is zero elsewhere; without
+// any kept token there is nothing but y.
+std::tuple<Tensor, OptTensor, std::vector<Tensor>> kimi_layer(const Tensor& x_, const std::vector<Tensor>& w, const OptTensor& g1_bias, const OptTensor& norm_w,
                                                               const std::vector<Tensor>& conv_w, const std::vector<OptTensor>& conv_b, const Tensor& a_log,
                                                               const Tensor& dt_bias, const std::vector<OptTensor>& conv_s, const OptTensor& rec, bool use_cache,
-                                                              bool silu, double eps, int64_t H, const Lengths& cu_seqlens) {
-  TORCH_CHECK_VALUE(x.is_cuda(), "x must be a CUDA tensor (daisy_b200 has no CPU path)");
-  c10::cuda::CUDAGuard guard(x.device());
-  const int64_t B = x.size(0), T = x.size(1), C = w[0].size(0), M = B * T;
+                                                              bool silu, double eps, int64_t H, const Lengths& cu_seqlens, const OptTensor& mask_) {
+  TORCH_CHECK_VALUE(x_.is_cuda(), "x must be a CUDA tensor (daisy_b200 has no CPU path)");
+  c10::cuda::CUDAGuard guard(x_.device());
   Packed p;
-  const bool packed = cu_seqlens.given;
-  if (packed) p = pack_tables(cu_seqlens, x.device(), 64, true);
+  const bool packed = cu_seqlens.given || mask_.has_value();
+  Tensor x = x_, rank;
+  if (mask_.has_value()) {
+    const int64_t B0 = x.size(0), T0 = x.size(1), dim = x.size(2);
+    Tensor mask = *mask_;
+    TORCH_CHECK_VALUE(mask.dim() == 2 && mask.size(0) == B0 && mask.size(1) == T0 && mask.device() == x.device(), "mask must be [", B0, ", ", T0, "] beside x");
+    const auto type = mask.scalar_type();
+    if (type != at::kBool && type != at::kByte && type != at::kChar && type != at::kInt && type != at::kLong) mask = mask.to(at::kBool);
+    if (mask.stride(1) != 1 || mask.stride(0) < 0) mask = mask.contiguous();
+    const auto ints = x.options().dtype(at::kInt);
+    rank = at::empty({2 * B0 * T0 + B0}, ints);                                            // rank, idx, len
+    int32_t *r = rank.data_ptr<int32_t>(), *idx = r + B0 * T0, *len = idx + B0 * T0;
+    check(daisy_b200_kda_mask_rows(mask.data_ptr(), (int)mask.element_size(), mask.stride(0), (int)B0, (int)T0, r, idx, len, stream_of(x)), "daisy_b200_kda_mask_rows");
+    Tensor host = at::empty({B0}, ints.device(at::kCPU).pinned_memory(true));
+    host.copy_(rank.narrow(0, 2 * B0 * T0, B0), /*non_blocking=*/true);
+    Tensor rows = aligned(x.contiguous());                                                 // while the lengths are on their way
+    at::cuda::getCurrentCUDAStream(x.get_device()).synchronize();
+    Lengths lengths;
+    lengths.given = true;
+    lengths.list.push_back(0);
+    for (int64_t b = 0; b < B0; ++b) lengths.list.push_back(lengths.list.back() + host.data_ptr<int32_t>()[b]);
+    p = pack_tables(lengths, x.device(), 64, true);
+    if (p.total == 0) return {at::zeros_like(x), OptTensor(), {}};
+    x = at::empty({1, p.total, dim}, x.options());
+    check(daisy_b200_kda_pack_rows(rows.data_ptr(), idx, p.tok.data_ptr<int32_t>(), x.data_ptr(), (int)p.total, (int)T0, (int)dim, stream_of(x)), "daisy_b200_kda_pack_rows");
+  } else if (packed) {
+    p = pack_tables(cu_seqlens, x.device(), 64, true);
+  }
+  const int64_t B = x.size(0), T = x.size(1), C = w[0].size(0), M = B * T;
   const int64_t n = packed ? p.n_seq : B;
   Tensor qkv[3], pr[3];
   std::vector<Tensor> out_s;
@@ -759,6 +789,9 @@ std::tuple<Tensor, OptTensor, std::vector<Tensor>> kimi_layer(const Tensor& x, c
   const void *xp[3], *wp[3], *bp[3], *sp[3];
   void *op[3], *yp[3];
   int64_t W[3];
+  Tensor fresh;                                                                            // states of packed sequences that begin here
+  if (use_cache && packed && !conv_s[0].has_value() && conv_w[0].numel() == conv_w[1].numel() && conv_w[0].numel() == conv_w[2].numel())
+    fresh = at::zeros({3, n, C, conv_w[0].numel() / C}, x.options());
   for (int i = 0; i < 3; ++i) {
     qkv[i] = at::empty_like(pr[i]);
     const bool have = conv_s[i].has_value(), in_place = have && !packed && T <= 32;
@@ -768,7 +801,7 @@ std::tuple<Tensor, OptTensor, std::vector<Tensor>> kimi_layer(const Tensor& x, c
                         "state must be a contiguous bf16 [", n, ", ", C, ", ", W[i], "] tensor");
     Tensor so;
     if (in_place) so = *conv_s[i];
-    else if (use_cache && packed) so = have ? conv_s[i]->clone() : at::zeros({n, C, W[i]}, x.options());     // sequences without tokens keep their state
+    else if (use_cache && packed) so = have ? conv_s[i]->clone() : fresh.defined() ? fresh.select(0, i) : at::zeros({n, C, W[i]}, x.options());   // sequences without tokens keep their state
     else if (use_cache) so = at::empty({n, C, W[i]}, x.options());
     xp[i] = pr[i].data_ptr(); wp[i] = conv_w[i].data_ptr(); bp[i] = conv_b[i].has_value() ? conv_b[i]->data_ptr() : nullptr;
     sp[i] = have ? conv_s[i]->data_ptr() : nullptr; op[i] = so.defined() ? so.data_ptr() : nullptr; yp[i] = qkv[i].data_ptr();
@@ -818,7 +851,15 @@ std::tuple<Tensor, OptTensor, std::vector<Tensor>> kimi_layer(const Tensor& x, c
   check(daisy_b200_kda_out_norm(o.data_ptr(), 0, gp.data_ptr(), g1_bias.has_value() ? g1_bias->data_ptr() : nullptr, g1_bias.has_value() ? (int)H : 1,
                                 norm_w.has_value() ? norm_w->data_ptr() : nullptr, yn.data_ptr(), M * H, 128, (float)eps, 2, stream_of(x)),
         "daisy_b200_kda_out_norm");
-  return {kimi_linear(yn, w[8]), r.second, out_s};
+  Tensor y = kimi_linear(yn, w[8]);
+  if (mask_.has_value()) {
+    Tensor out = at::empty(x_.sizes(), y.options());
+    check(daisy_b200_kda_unpack_rows(y.data_ptr(), rank.data_ptr<int32_t>(), p.cu.data_ptr<int32_t>(), out.data_ptr(), (int)x_.size(0), (int)x_.size(1), (int)x_.size(2),
+                                     stream_of(y)),
+          "daisy_b200_kda_unpack_rows");
+    y = out;
+  }
+  return {y, r.second, out_s};
 }
 
 }  // namespace
@@ -878,10 +919,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   });
   m.def("kimi_layer", [](const Tensor& x, const std::vector<Tensor>& w, const OptTensor& g1_bias, const OptTensor& norm_w, const std::vector<Tensor>& conv_w,
                          const std::vector<OptTensor>& conv_b, const Tensor& a_log, const Tensor& dt_bias, const std::vector<OptTensor>& conv_s, const OptTensor& rec,
-                         bool use_cache, bool silu, double eps, int64_t H, const py::object& cu) {
+                         bool use_cache, bool silu, double eps, int64_t H, const py::object& cu, const OptTensor& mask) {
     const Lengths lengths = lengths_of(cu);
     py::gil_scoped_release released;
-    return kimi_layer(x, w, g1_bias, norm_w, conv_w, conv_b, a_log, dt_bias, conv_s, rec, use_cache, silu, eps, H, lengths);
+    return kimi_layer(x, w, g1_bias, norm_w, conv_w, conv_b, a_log, dt_bias, conv_s, rec, use_cache, silu, eps, H, lengths, mask);
   });
   m.def("plain_bf16", &plain_bf16);
   m.def("kda_token_supported", &kda_token_supported);

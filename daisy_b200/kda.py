@@ -227,7 +227,11 @@ class B200KimiLinearSelfAttention(torch.nn.Module):
                 self._seen += 1
                 return y
         indices = tabs = None
-        if attn_mask is not None:                                          # attention_kimi.py:150-154
+        args = self._native_args() if x.dtype == torch.bfloat16 and (ve is None or sa_lambdas is None) else None
+        # a mask beside x on the device: packed, unpacked and everything between in the native call
+        masked = (args is not None and isinstance(attn_mask, torch.Tensor) and attn_mask.dim() == 2 and attn_mask.shape[0] == B0
+                  and B0 > 0 and attn_mask.shape[1] >= T0 > 0 and x.is_cuda and attn_mask.device == x.device and x.shape[-1] == self.hidden_size == self.key_dim)
+        if attn_mask is not None and not masked:                           # attention_kimi.py:150-154
             indices, cu_seqlens, _ = get_unpad_data(attn_mask[:, -T0:])
             x = index_first_axis(x.reshape(B0 * T0, -1), indices).unsqueeze(0)
             if ve is not None:
@@ -236,14 +240,16 @@ class B200KimiLinearSelfAttention(torch.nn.Module):
                 return x.new_zeros(B0, T0, self.hidden_size)
         B, T, _ = x.shape
         H = self.num_heads
-        args = self._native_args() if x.dtype == torch.bfloat16 and (ve is None or sa_lambdas is None) else None
         if args is not None:
             cs = self._conv_state if (use_cache and self._conv_state is not None) else (None, None, None)
             rec = self._recurrent_state if use_cache else None
             if rec is not None:
                 rec = rec.float().contiguous()
             y, rec, cs = ext().kimi_layer(x if x.is_contiguous() else x.contiguous(), *args, [None if c is None else c.to(torch.bfloat16) for c in cs], rec,
-                                          use_cache, self.q_conv1d.activation is not None, 1e-6, H, cu_seqlens if indices is not None else None)
+                                          use_cache, self.q_conv1d.activation is not None, 1e-6, H, cu_seqlens if indices is not None else None,
+                                          attn_mask[:, -T0:] if masked else None)
+            if masked and not cs and use_cache:                            # no token is kept: the states stay as they are
+                return y
             if use_cache:
                 self._recurrent_state, self._conv_state = rec, tuple(cs)
                 self._seen += T0

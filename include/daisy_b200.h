@@ -408,6 +408,15 @@ int daisy_b200_kda_low_rank(const void* x, int64_t ldx, const void* f0_w, const 
 int daisy_b200_kda_gates(const void* f0, const void* g0, const void* f1_w, const void* g1_w, const float* a_log, const float* dt_bias,
                          float* g, void* gate, int M, int H, int* status_word, void* stream);
 
+/* A padded batch [B,T] and the packed row of its kept tokens (get_unpad_data, index_first_axis, pad_input,
+ * models/daisy/attention_kimi.py:150-154,193).  mask: integers of 1, 4 or 8 bytes, row stride ld, kept where not zero.
+ *   kda_mask_rows     rank [B,T] (number among the row's kept tokens, -1: padding), idx [B,T] (token of each number), len [B]
+ *   kda_pack_rows     y [total,dim] from x [B,T,dim] (bf16), token_tab [total][2] as for the packed convolution
+ *   kda_unpack_rows   out [B,T,dim] from y [total,dim], zeros at the padding; cu [B + 1]: first packed token of each row */
+int daisy_b200_kda_mask_rows(const void* mask, int elem_bytes, int64_t ld, int B, int T, int32_t* rank, int32_t* idx, int32_t* len, void* stream);
+int daisy_b200_kda_pack_rows(const void* x, const int32_t* idx, const int32_t* token_tab, void* y, int total, int T, int dim, void* stream);
+int daisy_b200_kda_unpack_rows(const void* y, const int32_t* rank, const int32_t* cu, void* out, int B, int T, int dim, void* stream);
+
 /* Packed variable-length form of the same call: chunk_kda(..., cu_seqlens=cu_seqlens) at
  * models/daisy/attention_kimi.py:133-134, with cu_seqlens from get_unpad_data (:150-154; helpers :19-33).  The
  * sequences lie end to end in one row: q, k [1, T_total, H, K], v, o [1, T_total, H, V], g fp32, beta [1, T_total, H];

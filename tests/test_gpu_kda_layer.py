@@ -449,3 +449,32 @@ def test_projections_that_end_in_gates(M, H):
     assert bool(((beta[:M].double() - z.sigmoid()).abs() <= tol).all())
     assert L.daisy_b200_kda_low_rank(x.data_ptr(), dim, f0_w.data_ptr(), g0_w.data_ptr(), b_w.data_ptr(), f0.data_ptr(), g0.data_ptr(), beta.data_ptr(),
                                      M, 33, dim, status, st) == _lib.EUNSUPPORTED
+
+
+@pytest.mark.parametrize("T,kind", [(1, "int64"), (37, "bool"), (300, "scattered"), (1025, "float"), (1024, "uint8"), (2100, "int32")])
+def test_layer_mask_equals_packing_by_hand(T, kind):
+    """The mask handled inside the native call (numbering, packing, unpacking; rows beyond one block pass of 1024 tokens, a row
+    without tokens, kept tokens anywhere, a mask wider than the input, every mask type) against the tensor operations around the
+    packed call: the same bits, and states that continue."""
+    from daisy_b200 import B200KimiLinearSelfAttention
+    from daisy_b200.kda import get_unpad_data, index_first_axis, pad_input
+    H, B = 2, 4
+    torch.manual_seed(T)
+    m = B200KimiLinearSelfAttention(H * 128, H, 4096, 128).cuda()
+    x = torch.randn(B, T, H * 128, device="cuda", dtype=torch.bfloat16)
+    keep = torch.rand(B, T + 5, device="cuda") < 0.6 if kind == "scattered" else torch.arange(T + 5, device="cuda")[None] >= torch.tensor([[5], [T + 5], [T // 2 + 5], [T + 4]], device="cuda")
+    mask = keep if kind in ("bool", "scattered") else keep.to(getattr(torch, {"float": "float32"}.get(kind, kind)))
+    if kind == "int32":
+        mask = mask.t().contiguous().t()
+    with torch.inference_mode():
+        indices, cu, _ = get_unpad_data(mask[:, -T:])
+        from daisy_b200._native import ext
+        y_ref, rec, cs = ext().kimi_layer(index_first_axis(x.reshape(B * T, -1), indices).unsqueeze(0), *m._native_args(), [None] * 3, None, True, True, 1e-6, H, cu, None)
+        y, _, _ = m.prefill(x, attn_mask=mask)
+        assert torch.equal(y, pad_input(y_ref.squeeze(0), indices, B, T))
+        assert torch.equal(m._recurrent_state, rec) and all(torch.equal(a, b) for a, b in zip(m._conv_state, cs))
+        assert torch.equal(m.forward(x, attn_mask=mask), y)
+        before = [t.clone() for t in (m._recurrent_state, *m._conv_state)]
+        none, _, _ = m.prefill(x, attn_mask=torch.zeros_like(mask))
+        assert not none.any() and none.shape == x.shape
+        assert all(torch.equal(a, b) for a, b in zip((m._recurrent_state, *m._conv_state), before))

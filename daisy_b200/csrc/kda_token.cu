@@ -84,7 +84,8 @@ __device__ __forceinline__ uint4 kt_shift(const uint4& s, uint32_t v) {
 
 // ---- one (batch, head), its vectors in shared memory: sv [9][128] = q, k, v, f0, g0, decay, output gate, two partial sums; sv[9 * 128]
 //      the write strength
-// decay gate (f1 row block x f0) and output gate (g1 row block x g0): half-warp hw takes rows hw, hw + HW, ..
+// decay gate (f1 row block x f0) and output gate (g1 row block x g0): half-warp hw takes rows hw, hw + HW, ..  (A sum at a time, its gate by
+// one lane of sixteen: the exponentials eleven or sixteen times one after the other.)
 template <int HW>
 __device__ __forceinline__ void kt_gates(float* sv, const __nv_bfloat16* f1, const __nv_bfloat16* g1, const __nv_bfloat16* g1_bias, const float* a_log,
                                          const float* dt_bias, int h, int tid) {
@@ -92,29 +93,37 @@ __device__ __forceinline__ void kt_gates(float* sv, const __nv_bfloat16* f1, con
   float f[8], g[8];
   *reinterpret_cast<float4*>(f) = reinterpret_cast<const float4*>(sv + 3 * 128)[2 * sub]; *reinterpret_cast<float4*>(f + 4) = reinterpret_cast<const float4*>(sv + 3 * 128)[2 * sub + 1];
   *reinterpret_cast<float4*>(g) = reinterpret_cast<const float4*>(sv + 4 * 128)[2 * sub]; *reinterpret_cast<float4*>(g + 4) = reinterpret_cast<const float4*>(sv + 4 * 128)[2 * sub + 1];
-  const float ea = -expf(__ldg(a_log + h));
+  constexpr int N = (256 + HW - 1) / HW;
+  static_assert(N <= 16, "a row for each lane of a half-warp");
+  float d[16];
 #pragma unroll
-  for (int k = 0; k < (256 + HW - 1) / HW; ++k) {
+  for (int k = 0; k < 16; ++k) {
+    d[k] = 0.f;
     const int r = hw + HW * k;
-    float d = 0.f;
-    if (r < 256) {
+    if (k < N && r < 256) {
       float w[8];
       unpack8(__ldg(reinterpret_cast<const uint4*>((r < 128 ? f1 : g1) + ((size_t)h * 128 + (r & 127)) * 128 + 8 * sub)), w);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) d = fmaf(w[e], r < 128 ? f[e] : g[e], d);
+      for (int e = 0; e < 8; ++e) d[k] = fmaf(w[e], r < 128 ? f[e] : g[e], d[k]);
     }
-    d += __shfl_xor_sync(0xffffffffu, d, 8); d += __shfl_xor_sync(0xffffffffu, d, 4);
-    d += __shfl_xor_sync(0xffffffffu, d, 2); d += __shfl_xor_sync(0xffffffffu, d, 1);
-    if (sub == 0 && r < 256) {
-      d = __bfloat162float(__float2bfloat16_rn(d));
-      if (r < 128) {                                  // decay e^g, g = -exp(A) softplus(f + dt_bias) at bf16
-        const float z = d + __ldg(dt_bias + h * 128 + r);
-        const float sp_ = z > 20.f ? z : log1pf(expf(z));
-        sv[5 * 128 + r] = __expf(__bfloat162float(__float2bfloat16_rn(ea * sp_)));
-      } else {
-        if (g1_bias) d = __bfloat162float(__float2bfloat16_rn(d + __bfloat162float(g1_bias[h * 128 + r - 128])));
-        sv[6 * 128 + r - 128] = d;
-      }
+  }
+  // sixteen sums over sixteen lanes, half of them handed on at each step: lane `sub` ends with row hw + HW sub
+#pragma unroll
+  for (int m = 8; m >= 1; m >>= 1) {
+    const bool up = (sub & m) != 0;
+#pragma unroll
+    for (int i = 0; i < m; ++i) d[i] = (up ? d[i + m] : d[i]) + __shfl_xor_sync(0xffffffffu, up ? d[i] : d[i + m], m);
+  }
+  const int r = hw + HW * sub;
+  if (r < 256) {
+    float x = __bfloat162float(__float2bfloat16_rn(d[0]));
+    if (r < 128) {                                    // decay e^g, g = -exp(A) softplus(f + dt_bias) at bf16
+      const float z = x + __ldg(dt_bias + h * 128 + r);
+      const float sp_ = z > 20.f ? z : log1pf(expf(z));
+      sv[5 * 128 + r] = __expf(__bfloat162float(__float2bfloat16_rn(-expf(__ldg(a_log + h)) * sp_)));
+    } else {
+      if (g1_bias) x = __bfloat162float(__float2bfloat16_rn(x + __bfloat162float(g1_bias[h * 128 + r - 128])));
+      sv[6 * 128 + r - 128] = x;
     }
   }
 }

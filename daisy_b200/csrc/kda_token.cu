@@ -86,14 +86,23 @@ __device__ __forceinline__ uint4 kt_shift(const uint4& s, uint32_t v) {
 //      the write strength
 // decay gate (f1 row block x f0) and output gate (g1 row block x g0): half-warp hw takes rows hw, hw + HW, ..  (A sum at a time, its gate by
 // one lane of sixteen: the exponentials eleven or sixteen times one after the other.)
+template <int HW> struct KtGateRows { static constexpr int N = (256 + HW - 1) / HW; uint4 w[N]; };
 template <int HW>
-__device__ __forceinline__ void kt_gates(float* sv, const __nv_bfloat16* f1, const __nv_bfloat16* g1, const __nv_bfloat16* g1_bias, const float* a_log,
-                                         const float* dt_bias, int h, int tid) {
+__device__ __forceinline__ void kt_gate_rows(KtGateRows<HW>& rows, const __nv_bfloat16* f1, const __nv_bfloat16* g1, int h, int tid) {
+  const int hw = tid >> 4, sub = tid & 15;
+#pragma unroll
+  for (int k = 0; k < KtGateRows<HW>::N; ++k) {
+    const int r = hw + HW * k;
+    if (r < 256) rows.w[k] = __ldg(reinterpret_cast<const uint4*>((r < 128 ? f1 : g1) + ((size_t)h * 128 + (r & 127)) * 128 + 8 * sub));
+  }
+}
+template <int HW>
+__device__ __forceinline__ void kt_gates(float* sv, const KtGateRows<HW>& rows, const __nv_bfloat16* g1_bias, const float* a_log, const float* dt_bias, int h, int tid) {
   const int hw = tid >> 4, sub = tid & 15;
   float f[8], g[8];
   *reinterpret_cast<float4*>(f) = reinterpret_cast<const float4*>(sv + 3 * 128)[2 * sub]; *reinterpret_cast<float4*>(f + 4) = reinterpret_cast<const float4*>(sv + 3 * 128)[2 * sub + 1];
   *reinterpret_cast<float4*>(g) = reinterpret_cast<const float4*>(sv + 4 * 128)[2 * sub]; *reinterpret_cast<float4*>(g + 4) = reinterpret_cast<const float4*>(sv + 4 * 128)[2 * sub + 1];
-  constexpr int N = (256 + HW - 1) / HW;
+  constexpr int N = KtGateRows<HW>::N;
   static_assert(N <= 16, "a row for each lane of a half-warp");
   float d[16];
 #pragma unroll
@@ -102,7 +111,7 @@ __device__ __forceinline__ void kt_gates(float* sv, const __nv_bfloat16* f1, con
     const int r = hw + HW * k;
     if (k < N && r < 256) {
       float w[8];
-      unpack8(__ldg(reinterpret_cast<const uint4*>((r < 128 ? f1 : g1) + ((size_t)h * 128 + (r & 127)) * 128 + 8 * sub)), w);
+      unpack8(rows.w[k < N ? k : 0], w);
 #pragma unroll
       for (int e = 0; e < 8; ++e) d[k] = fmaf(w[e], r < 128 ? f[e] : g[e], d[k]);
     }
@@ -257,6 +266,8 @@ __global__ void __launch_bounds__(TK_CT, 1) kda_token_kernel(const __grid_consta
 #pragma unroll
       for (int i = 0; i < 64; ++i) S[i] = __ldcg(sp + i * 128);
     }
+    KtGateRows<TK_CT / 16> gate_rows;                 // on their way while the vectors are waited for
+    kt_gate_rows(gate_rows, p.f1, p.g1, h, tid);
     if (warp < 5) {                                   // q, k, v, f0, g0
       const uint2* src = warp < 3 ? p.qkv + (size_t)b * 3 * (p.dim / 2) + warp * (p.dim / 2) + h * 64 : p.fg + (size_t)b * 128 + (warp - 3) * 64;
       uint4 r[1];
@@ -276,7 +287,7 @@ __global__ void __launch_bounds__(TK_CT, 1) kda_token_kernel(const __grid_consta
       sv[9 * 128] = __bfloat162float(__float2bfloat16_rn(kt_sigmoid(z)));
     }
     named_bar(1, TK_CT);
-    kt_gates<TK_CT / 16>(sv, p.f1, p.g1, p.g1_bias, p.a_log, p.dt_bias, h, tid);
+    kt_gates(sv, gate_rows, p.g1_bias, p.a_log, p.dt_bias, h, tid);
     named_bar(1, TK_CT);
     if (tid < 256) {
       kt_update(S, sv, p.norm_w, p.eps, tid, [&](uint32_t r01, uint32_t r23) {
@@ -363,7 +374,9 @@ __global__ void __launch_bounds__(256, 2) kda_batch_kernel(const __grid_constant
     if (lane == 0) sv[9 * 128] = __bfloat162float(__float2bfloat16_rn(kt_sigmoid(__bfloat162float(__float2bfloat16_rn(d)))));
   }
   __syncthreads();
-  kt_gates<16>(sv, p.f1, p.g1, p.g1_bias, p.a_log, p.dt_bias, h, tid);
+  KtGateRows<16> gate_rows;
+  kt_gate_rows(gate_rows, p.f1, p.g1, h, tid);
+  kt_gates(sv, gate_rows, p.g1_bias, p.a_log, p.dt_bias, h, tid);
   __syncthreads();
   kt_update(S, sv, p.norm_w, p.eps, tid, [&](uint32_t r01, uint32_t r23) {
     *reinterpret_cast<uint2*>(p.o + (size_t)b * p.dim + h * 128 + 4 * lane) = make_uint2(r01, r23);

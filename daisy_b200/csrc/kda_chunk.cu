@@ -6,7 +6,7 @@
 //     A_kk[i,j] = beta_i sum_c k_ic k_jc e^{G_ic-G_jc} (j < i)     A_qk[i,j] = scale sum_c q_ic k_jc e^{G_ic-G_jc} (j <= i)
 //     T = (I + A_kk)^-1          W = T (beta k e^G)          U0 = T (beta v)
 //     U = U0 - W S_0             O = (scale q e^G) S_0 + A_qk U          S_C = e^{G_C} S_0 + (k e^{G_C-G})^T U
-// Two kernels:
+// Two kernels, on long rows in several parts that run beside one another (kda_split):
 //  * kda_intra_kernel  -- everything that does not depend on the state, a small CTA per (batch, head, chunk), three to an SM:
 //    Gram products in mma.sync fragments, the blocked solve of (I + A_kk) W = beta k e^G, (I + A_kk) U0 = beta v in register
 //    chains.  Per chunk it writes a record of fp16 operand images (16-byte pieces exchanged so that fragment loads are
@@ -125,6 +125,7 @@ struct KdaIntraParams {
   const float *g, *beta;
   uint8_t* ws;
   int T, H, NC;            // NC = chunks per sequence
+  int c0, behind;          // first chunk of this launch; behind: it runs beside the state's pass over the chunks before (kda_split)
   float scale;
   int l2norm;
   // packed variable-length sequences (B = 1): chunk c of the packed row covers tokens chunk_tab[2c] .. + chunk_tab[2c+1]
@@ -166,8 +167,9 @@ __global__ void __launch_bounds__(KI_THREADS, 3) kda_intra_kernel(const KdaIntra
   extern __shared__ __align__(128) uint8_t kda_smem_raw[];
   KdaIntraSmem& sm = *reinterpret_cast<KdaIntraSmem*>(kda_smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g8 = lane >> 2, t4 = lane & 3;
-  const int chunk = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
-  grid_dep_wait();
+  const int chunk = p.c0 + blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  if (!p.behind) grid_dep_wait();
+  grid_dep_launch();
   int t0, rows;
   ki_chunk_span(p.chunk_tab, chunk, p.T, t0, rows);
   uint8_t* rec = p.ws + ((size_t)(b * p.H + h) * p.NC + chunk) * REC_BYTES;
@@ -548,6 +550,7 @@ __global__ void __launch_bounds__(KI_THREADS, 3) kda_intra_kernel(const KdaIntra
       }
     }
   }
+  if (p.behind && blockIdx.x == gridDim.x - 1 && blockIdx.y == gridDim.y - 1 && blockIdx.z == gridDim.z - 1) grid_dep_wait();
 }
 
 // =============================================================================================
@@ -555,10 +558,12 @@ __global__ void __launch_bounds__(KI_THREADS, 3) kda_intra_kernel(const KdaIntra
 // =============================================================================================
 struct KdaStateParams {
   const uint8_t* ws;
-  const float* h0;
+  const float* h0;         // state before the first chunk (null: zero) and after the last (null: not kept)
   float* hT;
   void* o;
+  int64_t ld_in, ld_out;   // floats between the states of two CTAs
   int T, H, NC, out_fp32;
+  int c0, c1, more;        // dense: chunks of this launch; more: another one follows it (kda_split)
   int* status;
   // packed variable-length sequences (B = 1): blockIdx.x = sequence * H + head, the sequence's chunks are
   // seq_ptr[s] .. seq_ptr[s + 1] - 1 of the packed row's NC chunks, chunk_tab as in the intra kernel; null: dense
@@ -622,10 +627,11 @@ __global__ void __launch_bounds__(KS_THREADS, 1) kda_state_kernel(const KdaState
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = bars->tmem_base;
+  if (p.more) grid_dep_launch();
   grid_dep_wait();
 
   const int bh = blockIdx.x, h = bh % p.H, b = p.seq_ptr ? 0 : bh / p.H;           // bh also indexes h0 / hT
-  const int c_begin = p.seq_ptr ? p.seq_ptr[bh / p.H] : 0, c_end = p.seq_ptr ? p.seq_ptr[bh / p.H + 1] : p.NC;
+  const int c_begin = p.seq_ptr ? p.seq_ptr[bh / p.H] : p.c0, c_end = p.seq_ptr ? p.seq_ptr[bh / p.H + 1] : p.c1;
   const int n_chunks = c_end - c_begin;
 
   const uint8_t* recs = p.ws + ((size_t)(b * p.H + h) * p.NC + c_begin) * REC_BYTES;
@@ -695,9 +701,9 @@ __global__ void __launch_bounds__(KS_THREADS, 1) kda_state_kernel(const KdaState
     const uint32_t t = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
     float S[64];                                                                   // row v of S^T, channels 64 half ..
     {
-      const float* hp = p.h0 ? p.h0 + (size_t)bh * KD * KD + 64 * half * KD + v : nullptr;
+      const float* hp = p.h0 ? p.h0 + bh * p.ld_in + 64 * half * KD + v : nullptr;
 #pragma unroll
-      for (int i = 0; i < 64; ++i) S[i] = hp ? hp[(size_t)i * KD] : 0.f;
+      for (int i = 0; i < 64; ++i) S[i] = hp ? __ldcg(hp + (size_t)i * KD) : 0.f;      // (L2: the part before may have written it)
     }
     bool ok = true;
     for (int c = 0; c <= n_chunks; ++c) {
@@ -756,7 +762,7 @@ __global__ void __launch_bounds__(KS_THREADS, 1) kda_state_kernel(const KdaState
       mbar_arrive(&bars->u16);
     }
     if (ok && p.hT) {
-      float* hp = p.hT + (size_t)bh * KD * KD + 64 * half * KD + v;
+      float* hp = p.hT + bh * p.ld_out + 64 * half * KD + v;
 #pragma unroll
       for (int i = 0; i < 64; ++i) hp[(size_t)i * KD] = S[i];
     }
@@ -825,6 +831,45 @@ extern "C" size_t daisy_b200_kda_workspace_bytes(int B, int T, int H, int K, int
   return (size_t)B * H * nc * WS_REC_BYTES;
 }
 
+// Where to cut a row of chunks, so that the state's pass over one part runs beside the intra-chunk pass over the next: the state
+// takes a CTA per (batch, head), the other SMs are the next part's.  Launches: intra, state, intra, state, ..  A launch may start
+// when every CTA of the one before has started; the state's waits for the intra-chunk launch before it, which ends only after the
+// state's launch before that has (its last CTA waits for it).  An intra-chunk launch after the first waits for nothing at its
+// start: all CTAs of the first have waited for what the stream held before.  The state goes from part to part in fp32 through the
+// room of a record that is spent, so the results have the same bits.
+// Each part takes as long beside the state's pass as that pass: by the measured 5.7 us of an SM per record, 1.35 us of the chain per
+// chunk alone and 1.8 beside the other pass, and 5 us that a cut costs (SMs run empty, the state is stored and read).
+// One pass each -> in parts: 4 x 16384 x 16 977 -> 874 us, 2 x 8192 x 16 343 -> 287, 1 x 16384 x 16 512 -> 427, 3 x 7000 x 12
+// 312 -> 262, 2 x 3001 x 16 136 -> 119, 2 x 1000 x 16 54 -> 49; rows of fewer chunks do not gain what a cut costs (2 x 700 x 16 level).
+constexpr int KDA_PARTS = 4;
+static_assert(KD * KD * 4 <= REC_BYTES, "a state fits a record");
+static int kda_split(int rows, int NC, int sms, int* end) {
+  if (rows >= sms * 7 / 8) return 1;
+  const double intra = 5.7 * rows / sms, beside = 5.7 * rows / (sms - rows), chain = 1.35, slow = 1.8, cost = 5;
+  int best = 1;
+  double best_us = NC * (intra + chain);
+  for (int n = 2; n <= KDA_PARTS; ++n) {
+    double sum = 0, part = 1;
+    for (int i = 0; i < n; ++i, part *= slow / beside) sum += part;
+    int cut[KDA_PARTS], at = 0;
+    double us = 0, size = NC / sum;
+    bool ok = true;
+    for (int i = 0, before = 0; i < n; ++i, size *= slow / beside) {
+      const int len = i + 1 == n ? NC - at : (int)(size + 0.5);
+      ok = ok && len >= 4;
+      const double state = before * slow, own = len * beside;
+      us += i == 0 ? len * intra : cost + (state > own ? state : own);
+      cut[i] = at += len;
+      before = len;
+      if (i + 1 == n) us += len * chain;
+    }
+    if (!ok || us >= best_us) continue;
+    best = n; best_us = us;
+    for (int i = 0; i < n; ++i) end[i] = cut[i];
+  }
+  return best;
+}
+
 // Shared launcher.  Dense: NC = ceil(T / 64) chunks per (batch, head) row, n_seq = B.  Packed variable-length (B = 1):
 // chunk_tab [NC][2] and seq_ptr [n_seq + 1] (both in device memory) say which tokens each chunk covers and which
 // chunks each sequence owns; h0 / hT are [n_seq, H, K, V].
@@ -860,22 +905,35 @@ static int kda_launch(const void* q, const void* k, const void* v, const float* 
   ip.scale = scale > 0.f ? scale : 1.0f / sqrtf((float)K);
   ip.l2norm = (flags & DAISY_KDA_L2NORM_QK) ? 1 : 0;
   ip.chunk_tab = chunk_tab;
-  if (daisy_host::launch_dependent(kda_intra_kernel, dim3(NC, H, B), dim3(KI_THREADS), intra_smem, st, ip) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return DAISY_ECUDA;
-  }
-  DAISY_CHECK_LAUNCH();
-
   KdaStateParams sp;
-  sp.ws = (const uint8_t*)workspace; sp.h0 = h0; sp.hT = hT; sp.o = o;
+  sp.ws = (const uint8_t*)workspace; sp.o = o;
   sp.T = T; sp.H = H; sp.NC = NC; sp.out_fp32 = (flags & DAISY_KDA_OUT_FP32) ? 1 : 0;
   sp.status = status_word;
   sp.chunk_tab = chunk_tab; sp.seq_ptr = seq_ptr;
-  if (daisy_host::launch_dependent(kda_state_kernel, dim3(n_seq * H), dim3(KS_THREADS), KS_SMEM, st, sp) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return DAISY_ECUDA;
+
+  int end[KDA_PARTS];
+  const int parts = seq_ptr ? 1 : kda_split(n_seq * H, NC, daisy_host::sm_count_cached(), end);
+  if (parts == 1) end[0] = NC;
+  float* kept = nullptr;                                      // the state between two parts
+  for (int i = 0, c0 = 0; i < parts; c0 = end[i++]) {
+    const bool last = i + 1 == parts;
+    ip.c0 = c0; ip.behind = i > 0;
+    if (daisy_host::launch_dependent(kda_intra_kernel, dim3(end[i] - c0, H, B), dim3(KI_THREADS), intra_smem, st, ip) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return DAISY_ECUDA;
+    }
+    DAISY_CHECK_LAUNCH();
+    const int64_t ld_rec = (int64_t)NC * (REC_BYTES / 4);
+    sp.h0 = i ? kept : h0; sp.ld_in = i ? ld_rec : KD * KD;
+    kept = reinterpret_cast<float*>((uint8_t*)workspace + (size_t)c0 * REC_BYTES);      // over a record this part has read
+    sp.hT = last ? hT : kept; sp.ld_out = last ? KD * KD : ld_rec;
+    sp.c0 = c0; sp.c1 = end[i]; sp.more = !last;
+    if (daisy_host::launch_dependent(kda_state_kernel, dim3(n_seq * H), dim3(KS_THREADS), KS_SMEM, st, sp) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return DAISY_ECUDA;
+    }
+    DAISY_CHECK_LAUNCH();
   }
-  DAISY_CHECK_LAUNCH();
   return DAISY_OK;
 }
 

@@ -306,3 +306,17 @@ def test_waiting_for_packed_lengths_leaves_other_threads_running():
         assert waited > 0.15, waited
         assert max(gap, time.perf_counter() - last) < 0.5 * waited, (gap, waited)
         torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("B,T,H", [(1, 64 * 30 + 1, 4), (2, 64 * 47 - 7, 16), (1, 64 * 150, 12), (4, 64 * 60 + 33, 16), (1, 64 * 20, 112)])
+def test_kda_in_parts_has_the_bits_of_one_pass(B, T, H):
+    """Long rows are cut into parts, the state's pass over one beside the intra-chunk pass over the next.  Packed sequences are
+    not cut, so a packed call on each row says what one pass gives."""
+    q, k, v, g, beta = _inputs(B, T, H, seed=B * T + H)
+    h0 = torch.randn(B, H, 128, 128, device="cuda", generator=torch.Generator("cuda").manual_seed(1)) * 0.1
+    for _ in range(3):                                        # back to back: a call's first launch reuses the room of the last
+        o, s = _run(q, k, v, g, beta, initial_state=h0, output_final_state=True)
+    for b in range(B):
+        o1, s1 = _run(*(a[b:b + 1] for a in (q, k, v, g, beta)), initial_state=h0[b:b + 1], output_final_state=True,
+                      cu_seqlens=torch.tensor([0, T], dtype=torch.int32))
+        assert torch.equal(o[b:b + 1], o1) and torch.equal(s[b:b + 1], s1)

@@ -72,6 +72,7 @@ SIGNATURES = {
     "daisy_b200_kda_chunk_fwd": (_i, [_vp] * 8 + [_i] * 6 + [_f, _u, _vp, _sz, _vp, _vp]),
     "daisy_b200_kda_varlen_workspace_bytes": (_sz, [_i] * 4),
     "daisy_b200_kda_chunk_fwd_varlen": (_i, [_vp] * 8 + [_i] * 5 + [_f, _u, _vp, _i, _vp, _i, _vp, _sz, _vp, _vp]),
+    "daisy_b200_kda_chunk_tables": (_i, [_vp, _i, _i, _i, _vp, _i, _vp, _vp]),
     "daisy_b200_kda_mask_rows": (_i, [_vp, _i, _i64, _i, _i] + [_vp] * 4),
     "daisy_b200_kda_pack_rows": (_i, [_vp] * 4 + [_i] * 3 + [_vp]),
     "daisy_b200_kda_unpack_rows": (_i, [_vp] * 4 + [_i] * 3 + [_vp]),

@@ -9,11 +9,11 @@
 // queue is full and packed lengths on the device wait for the stream: other Python threads go on, also the one whose launch
 // that stream may be waiting for.
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CUDAEvent.h>
 #include <ATen/cuda/CUDAGraphsUtils.cuh>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
-#include <functional>
 #include <list>
 #include <mutex>
 
@@ -565,10 +565,20 @@ Lengths lengths_of(const py::object& cu_seqlens) {
   return r;
 }
 
+void check_offsets(const std::vector<int64_t>& cu) {
+  bool ok = cu.size() >= 2 && cu[0] == 0;
+  for (size_t i = 1; ok && i < cu.size(); ++i) ok = cu[i] >= cu[i - 1];
+  TORCH_CHECK_VALUE(ok, "cu_seqlens must start at 0 and not decrease");
+}
+// The integers of a tensor that was copied to the host.
+std::vector<int64_t> to_list(const Tensor& c) {
+  if (c.scalar_type() == at::kInt) return {c.data_ptr<int32_t>(), c.data_ptr<int32_t>() + c.numel()};
+  return {c.data_ptr<int64_t>(), c.data_ptr<int64_t>() + c.numel()};
+}
+
 // Tables of a packed batch on the device (see kda_varlen_tables); tok only if asked for.
 struct Packed { Tensor chunks, ptr, tok, cu; int64_t n_chunks = 0, n_seq = 0, total = 0; };
-// `meanwhile(n_seq)` runs while lengths that lie on the device are on their way.
-Packed pack_tables(const Lengths& lengths, c10::Device dev, int64_t chunk, bool want_tok, const std::function<void(int64_t)>& meanwhile = {}) {
+Packed pack_tables(const Lengths& lengths, c10::Device dev, int64_t chunk, bool want_tok) {
   TORCH_CHECK_VALUE(chunk > 0, "chunk must be positive, got ", chunk);
   std::vector<int64_t> cu = lengths.list;
   if (const Tensor& t = lengths.t; t.defined()) {
@@ -577,18 +587,13 @@ Packed pack_tables(const Lengths& lengths, c10::Device dev, int64_t chunk, bool 
       c10::cuda::CUDAGuard guard(t.device());
       Tensor c = at::empty(t.sizes(), at::TensorOptions().dtype(t.scalar_type()).pinned_memory(true));
       c.copy_(t, /*non_blocking=*/true);
-      if (meanwhile) meanwhile(t.numel() - 1);
       at::cuda::getCurrentCUDAStream(t.get_device()).synchronize();
-      if (t.scalar_type() == at::kInt) cu.assign(c.data_ptr<int32_t>(), c.data_ptr<int32_t>() + c.numel());
-      else cu.assign(c.data_ptr<int64_t>(), c.data_ptr<int64_t>() + c.numel());
+      cu = to_list(c);
     } else {
-      Tensor c = t.to(at::kCPU, at::kLong).contiguous();
-      cu.assign(c.data_ptr<int64_t>(), c.data_ptr<int64_t>() + c.numel());
+      cu = to_list(t.to(at::kCPU, at::kLong).contiguous());
     }
   }
-  bool ok = cu.size() >= 2 && cu[0] == 0;
-  for (size_t i = 1; ok && i < cu.size(); ++i) ok = cu[i] >= cu[i - 1];
-  TORCH_CHECK_VALUE(ok, "cu_seqlens must start at 0 and not decrease");
+  check_offsets(cu);
   Packed p;
   p.n_seq = (int64_t)cu.size() - 1;
   p.total = cu.back();
@@ -615,20 +620,9 @@ Packed pack_tables(const Lengths& lengths, c10::Device dev, int64_t chunk, bool 
   return p;
 }
 
-// What a chunked call writes; made ahead of the call where there is a wait to fill.
-struct KdaOut { Tensor o, ws; OptTensor hT; };
-KdaOut kda_out(const Tensor& q, const Tensor& v, int64_t n, int64_t ws_bytes, bool want_state, bool out_fp32) {
-  const int64_t B = q.size(0), T = q.size(1), H = q.size(2), K = q.size(3), V = v.size(3);
-  KdaOut r;
-  r.o = at::empty({B, T, H, V}, q.options().dtype(out_fp32 ? at::kFloat : at::kBFloat16));
-  if (want_state) r.hT = at::empty({n, H, K, V}, q.options().dtype(at::kFloat));
-  r.ws = at::empty({std::max<int64_t>(ws_bytes, 16)}, q.options().dtype(at::kByte));
-  return r;
-}
-
 // chunked forward, dense ([B,T,H,K], packed == nullptr) or packed ([1,T_total,H,K])
 std::pair<Tensor, OptTensor> kda_chunk(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g_, const Tensor& beta_, std::optional<double> scale,
-                                       const OptTensor& h0_, bool want_state, bool l2norm, bool out_fp32, const Packed* pk, const KdaOut* made = nullptr) {
+                                       const OptTensor& h0_, bool want_state, bool l2norm, bool out_fp32, const Packed* pk) {
   const Tensor* in[] = {&q, &k, &v};
   const char* names[] = {"q", "k", "v"};
   for (int i = 0; i < 3; ++i) { req(*in[i], names[i]); TORCH_CHECK_VALUE(in[i]->is_contiguous(), names[i], " must be contiguous"); }
@@ -644,9 +638,9 @@ std::pair<Tensor, OptTensor> kda_chunk(const Tensor& q, const Tensor& k, const T
   }
   const int64_t need = pk ? (int64_t)daisy_b200_kda_varlen_workspace_bytes((int)pk->n_chunks, (int)H, (int)K, (int)V)
                           : (int64_t)daisy_b200_kda_workspace_bytes((int)B, (int)T, (int)H, (int)K, (int)V);
-  const KdaOut r = made && made->ws.defined() && made->ws.numel() >= need ? *made : kda_out(q, v, n, need, want_state, out_fp32);
-  const Tensor &o = r.o, &ws = r.ws;
-  const OptTensor& hT = r.hT;
+  Tensor o = at::empty({B, T, H, V}, q.options().dtype(out_fp32 ? at::kFloat : at::kBFloat16)), ws = at::empty({std::max<int64_t>(need, 16)}, q.options().dtype(at::kByte));
+  OptTensor hT;
+  if (want_state) hT = at::empty({n, H, K, V}, q.options().dtype(at::kFloat));
   if (pk && (T == 0 || pk->n_chunks == 0)) {
     if (want_state) { if (h0.defined()) hT->copy_(h0); else hT->zero_(); }
     return {o, hT};
@@ -699,14 +693,35 @@ std::pair<Tensor, OptTensor> chunk_kda(const Tensor& q_, const Tensor& k_, const
   Tensor g = g_.to(at::kFloat).contiguous(), beta = beta_.to(at::kFloat).contiguous();
   OptTensor h0;
   if (h0_.has_value()) h0 = h0_->to(at::kFloat).contiguous();
+  if (const Tensor& t = cu_seqlens.t; t.defined() && t.is_cuda() && t.device() == q.device() && t.dim() == 1 && t.is_contiguous() && t.numel() > 1 && t.numel() <= 1024 &&
+                                      (t.scalar_type() == at::kInt || t.scalar_type() == at::kLong) && q.dim() == 4 && q.size(0) == 1 && q.size(1) > 0) {
+    // Offsets on the device: the tables are made there, and the offsets are read and checked here while the kernels run.
+    c10::cuda::CUDAGuard guard(q.device());
+    const auto stream = at::cuda::getCurrentCUDAStream();
+    Tensor c = at::empty(t.sizes(), at::TensorOptions().dtype(t.scalar_type()).pinned_memory(true));
+    c.copy_(t, /*non_blocking=*/true);
+    at::cuda::CUDAEvent there;
+    there.record(stream);
+    Packed p;
+    p.n_seq = t.numel() - 1;
+    p.total = q.size(1);
+    p.n_chunks = p.total / 64 + p.n_seq;                                                   // every sequence may end in a short chunk
+    Tensor tabs = at::empty({2 * p.n_chunks + p.n_seq + 1}, q.options().dtype(at::kInt));
+    p.chunks = tabs.narrow(0, 0, 2 * p.n_chunks);
+    p.ptr = tabs.narrow(0, 2 * p.n_chunks, p.n_seq + 1);
+    check(daisy_b200_kda_chunk_tables(t.data_ptr(), (int)t.element_size(), (int)p.n_seq, (int)p.total, p.chunks.data_ptr<int32_t>(), (int)p.n_chunks,
+                                      p.ptr.data_ptr<int32_t>(), stream.stream()),
+          "daisy_b200_kda_chunk_tables");
+    std::pair<Tensor, OptTensor> r = kda_chunk(q, k, v, g, beta, scale, h0, want_state, l2norm, out_fp32, &p);
+    there.synchronize();
+    const std::vector<int64_t> cu = to_list(c);
+    check_offsets(cu);
+    TORCH_CHECK_VALUE(cu.back() == p.total, "cu_seqlens covers ", cu.back(), " tokens, the inputs hold ", p.total);
+    return r;
+  }
   if (cu_seqlens.given) {
-    KdaOut made;
-    Packed p = pack_tables(cu_seqlens, q.device(), 64, false, [&](int64_t n) {
-      if (q.dim() != 4 || v.dim() != 4 || q.size(0) != 1) return;                          // the call itself reports what is wrong
-      const int64_t most = q.size(1) / 64 + n;                                             // every sequence may end in a short chunk
-      made = kda_out(q, v, n, (int64_t)daisy_b200_kda_varlen_workspace_bytes((int)most, (int)q.size(2), (int)q.size(3), (int)v.size(3)), want_state, out_fp32);
-    });
-    return kda_chunk(q, k, v, g, beta, scale, h0, want_state, l2norm, out_fp32, &p, &made);
+    Packed p = pack_tables(cu_seqlens, q.device(), 64, false);
+    return kda_chunk(q, k, v, g, beta, scale, h0, want_state, l2norm, out_fp32, &p);
   }
   return q.size(1) <= RECURRENT_MAX_T ? kda_recurrent(q, k, v, g, beta, scale, h0, want_state, l2norm, out_fp32, false)
                                       : kda_chunk(q, k, v, g, beta, scale, h0, want_state, l2norm, out_fp32, nullptr);

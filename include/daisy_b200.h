@@ -425,6 +425,7 @@ int daisy_b200_kda_unpack_rows(const void* y, const int32_t* rank, const int32_t
  *     sequence, each sequence cut into 64-token chunks from its own first token;
  *   seq_ptr [n_seq + 1] int32 (device): sequence i owns chunks seq_ptr[i] .. seq_ptr[i+1]-1 (none for an empty
  *     sequence, whose final state is its initial state).
+ * A chunk of no tokens is left out; seq_ptr does not reach it.
  * workspace: daisy_b200_kda_varlen_workspace_bytes(n_chunks, H, K, V).  Other arguments and errors as above. */
 size_t daisy_b200_kda_varlen_workspace_bytes(int n_chunks, int H, int K, int V);
 int daisy_b200_kda_chunk_fwd_varlen(const void* q, const void* k, const void* v, const float* g,
@@ -432,6 +433,11 @@ int daisy_b200_kda_chunk_fwd_varlen(const void* q, const void* k, const void* v,
                                     int T_total, int H, int K, int V, int chunk, float scale, unsigned flags,
                                     const int32_t* chunk_tab, int n_chunks, const int32_t* seq_ptr, int n_seq,
                                     void* workspace, size_t workspace_bytes, int* status_word, void* stream);
+
+/* Both tables made on the device from cu [n_seq + 1] (int32 or int64 by elem_bytes, device), for 64-token chunks; n_seq <= 1023.
+ * chunk_tab has max_chunks >= T_total / 64 + n_seq entries, those behind the last chunk of no tokens.  Offsets that do not begin
+ * at 0, decrease or do not end at T_total give no chunk at all: the caller checks them. */
+int daisy_b200_kda_chunk_tables(const void* cu, int elem_bytes, int n_seq, int T_total, int32_t* chunk_tab, int max_chunks, int32_t* seq_ptr, void* stream);
 
 /* The same recurrence token by token, for short inputs (decode steps; the reference calls chunk_kda with
  * T = 1 and the cached state, models/daisy/attention_kimi.py:144-149,175-180).  The state of one (batch, head)

@@ -240,6 +240,36 @@ def test_kda_varlen_matches_per_sequence_recurrence(cu, with_state):
         assert not s[n].any()
 
 
+@pytest.mark.parametrize("n,T", [(1, 1), (1, 64), (3, 65), (33, 700), (700, 640), (1023, 5000)])
+@pytest.mark.parametrize("dtype", [torch.int32, torch.int64])
+def test_kda_tables_made_on_the_device(n, T, dtype):
+    """The tables of lengths that lie on the device are those the host makes, filled up with chunks of no tokens."""
+    from daisy_b200 import _lib, ops
+    cut = torch.randint(0, T + 1, (n - 1,), generator=torch.Generator().manual_seed(n)).sort().values
+    cu = torch.cat([torch.tensor([0]), cut, torch.tensor([T])])
+    chunks, ptr, _, n_chunks = ops.kda_varlen_tables(cu, "cuda")
+    most = T // 64 + n
+    got, got_ptr = torch.full((most, 2), -1, dtype=torch.int32, device="cuda"), torch.full((n + 1,), -1, dtype=torch.int32, device="cuda")
+    call = lambda c: _lib.check(_lib.lib().daisy_b200_kda_chunk_tables(c.data_ptr(), c.element_size(), n, T, got.data_ptr(), most, got_ptr.data_ptr(),
+                                                                       torch.cuda.current_stream().cuda_stream), "kda_chunk_tables")
+    call(cu.to("cuda", dtype))
+    assert torch.equal(got[:n_chunks], chunks) and torch.equal(got_ptr, ptr) and not got[n_chunks:].any()
+    for at, to in ((0, 1), (n, T - 1), (n, T + 1), (n // 2, -5)):                # offsets that are refused give no chunks
+        wrong = cu.clone()
+        wrong[at] = to
+        call(wrong.to("cuda", dtype))
+        assert not got.any() and not got_ptr.any()
+
+
+@pytest.mark.parametrize("cu", [[0, 5, 3, 70], [1, 70], [0, 69], [0, 71], [0, -1, 70], [0, 2 ** 40, 70], [70]])
+def test_kda_offsets_on_the_device_are_checked(cu):
+    from daisy_b200.kda import chunk_kda
+    q, k, v, g, beta = (t.cuda() for t in _inputs(1, 70, 2, seed=3))
+    with pytest.raises(ValueError, match="cu_seqlens"):
+        chunk_kda(q, k, v, g, beta, cu_seqlens=torch.tensor(cu, device="cuda"))
+    torch.cuda.synchronize()
+
+
 def test_kda_varlen_equals_dense_per_sequence():
     """A packed batch gives, sequence by sequence, the bits of the dense call on that sequence alone (the chunking
     starts at each sequence's own first token)."""

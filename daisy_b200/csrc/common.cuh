@@ -561,4 +561,12 @@ static inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, 
   return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
 
+// Two launches, one after the other, that do not depend on each other and leave room on the chip.  AHEAD: lets the next one in only
+// when it has waited for what the stream held before.  BEHIND, directly after an AHEAD one: waits for nothing at its start, and
+// its last CTA ends only after the launch before has, so that whoever waits for this one has both.
+enum { ORDER_AHEAD = 1, ORDER_BEHIND = 2 };
+// daisy_b200_gemm_nt_group with a place in such a pair; *order comes back as 0 if the kernel chosen has none.
+int gemm_group(const void* const* x, int64_t ldx, const void* const* w, int64_t ldw, void* const* c, int64_t ldc, int n, int M, int N, int K,
+               int* order, int* status_word, void* stream);
+
 }  // namespace daisy_host

@@ -74,6 +74,7 @@ struct GemmParams {
   void* ring[2];
   int64_t r_sb, r_sh, r_sr;
   int cap, ring_first, ring_f16;
+  int order;                     // narrow tiles only: ORDER_AHEAD, ORDER_BEHIND (common.cuh) or 0
   // training: 1 / rms of every row and head slot, [M][3 H], and v as normalised before the gate, [M, H, 128]; or null
   float* rstd;
   __nv_bfloat16* vn;
@@ -501,8 +502,9 @@ small_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p, con
   tc_fence_after();
   if (QKV) asm volatile("barrier.cluster.arrive.release;" ::: "memory");                 // (1) this CTA runs
   const uint32_t tmem_base = bars->tmem_base;
-  grid_dep_launch();
-  grid_dep_wait();
+  if (p.order == 0) grid_dep_launch();
+  if (p.order != daisy_host::ORDER_BEHIND) grid_dep_wait();
+  if (p.order != 0) grid_dep_launch();
 
   if (warp < 5) {
     // ------------------------------------------------------------------ TMA producers: a turn of the loop takes one thread some
@@ -672,6 +674,7 @@ small_gemm_kernel(const __grid_constant__ GemmMaps maps, const GemmParams p, con
     tc_fence_after();
     tmem_dealloc(tmem_base, BN);
   }
+  if (p.order == daisy_host::ORDER_BEHIND && blockIdx.x == gridDim.x - 1) grid_dep_wait();
 }
 
 }  // namespace daisy
@@ -809,6 +812,7 @@ static int gemm_common(const void* const* x, int64_t ldx, const void* const* w, 
   if (sms <= 0) return DAISY_ENODEV;
   cudaStream_t st = (cudaStream_t)stream;
   const int tile = gemm_tile(p, sms);
+  if (tile != TILE_32 && tile != TILE_64) p.order = 0;
   if (tile == TILE_32) return launch_small<32, false>(x, ldx, w, ldw, n, p, st);
   if (tile == TILE_64) return p.epi ? launch_small<64, true>(x, ldx, w, ldw, n, p, st) : launch_small<64, false>(x, ldx, w, ldw, n, p, st);
   GemmMaps maps;
@@ -818,8 +822,8 @@ static int gemm_common(const void* const* x, int64_t ldx, const void* const* w, 
   return p.epi ? launch_gemm<128, false, true>(maps, p, st) : launch_gemm<128, false, false>(maps, p, st);
 }
 
-extern "C" int daisy_b200_gemm_nt_group(const void* const* x, int64_t ldx, const void* const* w, int64_t ldw, void* const* c, int64_t ldc,
-                                        int n, int M, int N, int K, int* status_word, void* stream) {
+int daisy_host::gemm_group(const void* const* x, int64_t ldx, const void* const* w, int64_t ldw, void* const* c, int64_t ldc,
+                           int n, int M, int N, int K, int* order, int* status_word, void* stream) {
   if (!x || !w || !c || n < 1 || n > GROUP) return DAISY_EINVAL;
   GemmParams p{};
   p.M = M; p.per = N; p.K = K; p.epi = 0; p.ldc = ldc; p.status = status_word;
@@ -829,7 +833,16 @@ extern "C" int daisy_b200_gemm_nt_group(const void* const* x, int64_t ldx, const
     p.c[i] = (__nv_bfloat16*)c[i];
   }
   if ((ldc & 7) || ldc < N) return DAISY_EALIGN;
-  return gemm_common(x, ldx, w, ldw, n, p, stream);
+  p.order = *order;
+  const int rc = gemm_common(x, ldx, w, ldw, n, p, stream);
+  *order = p.order;
+  return rc;
+}
+
+extern "C" int daisy_b200_gemm_nt_group(const void* const* x, int64_t ldx, const void* const* w, int64_t ldw, void* const* c, int64_t ldc,
+                                        int n, int M, int N, int K, int* status_word, void* stream) {
+  int order = 0;
+  return daisy_host::gemm_group(x, ldx, w, ldw, c, ldc, n, M, N, K, &order, status_word, stream);
 }
 
 extern "C" int daisy_b200_kda_low_rank(const void* x, int64_t ldx, const void* f0_w, const void* g0_w, const void* b_w, void* f0, void* g0, float* beta,

@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(TK_CT, 1) kda_token_kernel(const __grid_consta
 }
 
 // ---------------------------------------------------------------------------------------------
-// The same step for batches that the launch above would take in several: projections by the GEMM, everything between by this
+// The same step for batches that are not the launch above's (kt_one_launch): projections by the GEMM, everything between by this
 // kernel, one CTA per (batch, head).  It is bound by the state, 64 KB in and out (12 heads x 54 rows: 85 MB, 13 us at copy
 // bandwidth); the gates' second projections are formed here (64 KB of weights a CTA, from L2) rather than as two more products.
 struct KdaBatchParams {
@@ -391,11 +391,21 @@ using namespace daisy;
 
 static inline size_t kt_align(size_t n) { return (n + 255) / 256 * 256; }
 
+// One launch, or four: the one gives each (batch, head) pair a CTA and has to take turns where there are more than SMs.  One launch
+// against four, us: 16 heads 9 rows (144 pairs) 23.1 / 26.4, 11 (176) 27.4 / 26.6, 16 (256) 32.7 / 27.1; 12 heads 13 rows (156)
+// 27.4 / 28.2, 16 (192) 29.4 / 28.4; 8 heads 16 rows (128) 23.2 / 26.0.
+constexpr int KT_ONE_PAIRS = 168;
+static bool kt_one_launch(int B, int H) { return B <= TK_MAX_B && B * H <= KT_ONE_PAIRS; }
+// the exchange's words, up to TK_MAX_B rows; scratch of the four launches lies behind them, so that a buffer serves both
+static size_t kt_words(size_t B, size_t dim) {
+  if (B > TK_MAX_B) return 0;
+  return 256 + kt_align(B * 3 * dim * 4) + kt_align(B * 128 * 8) + kt_align(B * 64) + TK_COPIES * kt_align(B * dim * 4);
+}
+
 extern "C" size_t daisy_b200_kda_token_workspace_bytes(int B, int H, int D) {
   if (B <= 0 || H <= 0 || D != 128 || H * D > TK_MAX_DIM) return 0;
   const size_t dim = (size_t)H * D;
-  if (B > TK_MAX_B) return 4 * kt_align(B * dim * 2) + 2 * kt_align((size_t)B * 128 * 2);   // q, k, v, o; f0, g0
-  return 256 + kt_align(B * 3 * dim * 4) + kt_align((size_t)B * 128 * 8) + kt_align((size_t)B * 64) + TK_COPIES * kt_align(B * dim * 4);
+  return kt_words(B, dim) + (kt_one_launch(B, H) ? 0 : 4 * kt_align(B * dim * 2) + 2 * kt_align((size_t)B * 128 * 2));   // q, k, v, o; f0, g0
 }
 
 template <int NB>
@@ -425,12 +435,12 @@ static int launch_kda_token(KdaTokenParams& p, int sms, cudaStream_t st) {
   return DAISY_OK;
 }
 
-// More rows than a launch of kda_token_kernel takes: four launches for all of them.
+// More rows or pairs than a launch of kda_token_kernel is for: four launches for all of them.
 static int kda_batch_step(const daisy_b200_kda_layer* ly, const void* x, int64_t x_sb, void* y, float* state, void* conv_q, void* conv_k, void* conv_v,
                           int B, int H, float eps, unsigned flags, void* workspace, int* status_word, void* stream) {
   const int dim = H * 128;
   if ((int64_t)B * H >= (int64_t)1 << 31) return DAISY_EUNSUPPORTED;
-  uint8_t* ws = (uint8_t*)workspace;
+  uint8_t* ws = (uint8_t*)workspace + kt_words(B, dim);
   void *pr[3], *o, *low[2];
   for (void*& c : pr) { c = ws; ws += kt_align((size_t)B * dim * 2); }
   o = ws; ws += kt_align((size_t)B * dim * 2);
@@ -476,7 +486,7 @@ extern "C" int daisy_b200_kda_token_step(const daisy_b200_kda_layer* ly, const v
   const int sms = daisy_host::sm_count_cached();
   if (sms <= 0) return DAISY_ENODEV;
   const int dim = H * D;
-  if (B > TK_MAX_B) return kda_batch_step(ly, x, x_sb, y, state, conv_q, conv_k, conv_v, B, H, eps, flags, workspace, status_word, stream);
+  if (!kt_one_launch(B, H)) return kda_batch_step(ly, x, x_sb, y, state, conv_q, conv_k, conv_v, B, H, eps, flags, workspace, status_word, stream);
   KdaTokenParams p;
   const void* w[7] = {ly->q_w, ly->k_w, ly->v_w, ly->f0_w, ly->g0_w, ly->b_w, ly->o_w};
   const int rows[7] = {dim, dim, dim, 128, 128, H, dim};

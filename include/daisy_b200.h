@@ -521,12 +521,12 @@ int daisy_b200_qkv_prep_grad(const void* q_p, const void* k_p, const void* v_n, 
                              const void* ve, const float* ve_gate_logit, void* d_ve, float* d_logit, float* partial,
                              int M, int T, int H, int D, void* stream);
 
-/* One decoded token through a Kimi-delta-attention layer, up to 16 rows in one launch (KimiLinearSelfAttention.step,
+/* One decoded token through a Kimi-delta-attention layer, up to 16 rows and 168 (row, head) pairs in one launch (KimiLinearSelfAttention.step,
  * models/daisy/attention_kimi.py:128-211): projections, short convolutions (four taps, SiLU with DAISY_KDA_CONV_SILU), decay
- * gate, recurrent update, gated norm, output projection.  dim = H * 128 <= 2048; above 16 rows four launches.  Weights bf16, row-major as their
+ * gate, recurrent update, gated norm, output projection.  dim = H * 128 <= 2048; above that four launches.  Weights bf16, row-major as their
  * Linear layers hold them; a_log [H] and dt_bias [dim] fp32.  state [B,H,128,128] fp32 and conv_q / conv_k / conv_v
- * [B,dim,4] bf16 are updated in place.  x [B,dim] (row stride x_sb elements), y [B,dim].  Up to 16 rows a cooperative launch and
- * a workspace as in daisy_b200_swa_token_step; above that the workspace is scratch. */
+ * [B,dim,4] bf16 are updated in place.  x [B,dim] (row stride x_sb elements), y [B,dim].  The one launch is a cooperative
+ * one.  Up to 16 rows the workspace is as in daisy_b200_swa_token_step, above that scratch. */
 typedef struct daisy_b200_kda_layer {
   const void *q_w, *k_w, *v_w;               /* [dim, dim] */
   const void *f0_w, *g0_w;                   /* [128, dim] */

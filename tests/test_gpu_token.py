@@ -155,3 +155,32 @@ def test_kimi_batch_step_matches_row_launches(B, H, bias):
     for a, b in zip(got[2:], ref[2:]):
         assert torch.equal(a[..., :3], b[..., :3])
         assert_close_bf16(a, b, "the new input")
+
+
+@pytest.mark.parametrize("B,H", [(11, 16), (16, 16), (15, 12), (10, 16), (14, 12)])
+def test_kimi_step_either_side_of_the_line_between_its_routes(B, H):
+    """The most (batch, head) pairs of the single launch and the fewest of the four, in turn with single launches of one row: they
+    share a workspace, whose words the four launches' scratch must leave alone."""
+    from daisy_b200 import B200KimiLinearSelfAttention, ops
+    torch.manual_seed(B)
+    layer = B200KimiLinearSelfAttention(H * D, H, 4096, D).cuda()
+    x = torch.randn(B, 30, H * D, device="cuda", dtype=torch.bfloat16)
+    with torch.inference_mode():
+        layer.prefill(x[:, :29])
+        rec, conv = layer._recurrent_state.clone(), [c.clone() for c in layer._conv_state]
+
+        def step(b, n):
+            layer._recurrent_state, layer._conv_state = rec[b:b + n].clone(), tuple(c[b:b + n].clone() for c in conv)
+            return (layer.step(x[b:b + n, 29:])[0], layer._recurrent_state, *layer._conv_state)
+        got, ys = step(0, B), []
+        for b in range(B):
+            ys.append(step(b, 1))
+            again = step(0, B)
+            assert all(torch.equal(a, g) for a, g in zip(again, got))
+    ops.check_device_status("cuda")
+    ref = [torch.cat(t) for t in zip(*ys)]
+    assert_close_bf16(got[0], ref[0], "y", max_tol=3e-2, mean_tol=3e-3)
+    assert ((got[1] - ref[1]).norm() / ref[1].norm()).item() < 5e-3
+    for a, b in zip(got[2:], ref[2:]):
+        assert torch.equal(a[..., :3], b[..., :3])
+        assert_close_bf16(a, b, "the new input")

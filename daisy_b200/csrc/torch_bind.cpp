@@ -451,18 +451,23 @@ struct AttnFunction : public torch::autograd::Function<AttnFunction> {
     }
     Tensor d_o = at::mm(dy, w.select(0, 3));
     const unsigned bwd_flags = d[4] ? DAISY_WINDOW_BLOCKS : 0;
-    const size_t ws_bytes = daisy_b200_swa_attend_bwd_workspace_bytes_full((int)B, (int)T, (int)H, (int)window, bwd_flags);
-    const int64_t row = Saved::up(M * dim * 2), ws_at = 6 * row, part_at = ws_at + Saved::up((int64_t)ws_bytes);
+    const int64_t row = Saved::up(M * dim * 2), part_at = 6 * row;
     const int64_t n_part = ve2.defined() ? daisy_b200_qkv_prep_grad_blocks((int)M, (int)H) : 0;
-    Tensor tmp = at::empty({(part_at + Saved::up(4 * n_part)) / 2}, buf.options());          // dqkv, dq, dk, dv, workspace, partial sums
+    Tensor tmp = at::empty({(part_at + Saved::up(4 * n_part)) / 2}, buf.options());          // dqkv, dq, dk, dv, partial sums
     char *g = (char*)tmp.data_ptr(), *dq = g + 3 * row, *dk = g + 4 * row, *dv = g + 5 * row;
     Tensor dqkv = tmp.narrow(0, 0, M * 3 * dim).view({M, 3 * dim}), d_ve, d_logit;
+    Tensor ws;
+    try {
+      ws = at::empty({(int64_t)daisy_b200_swa_attend_bwd_workspace_bytes_full((int)B, (int)T, (int)H, (int)window, bwd_flags)}, buf.options().dtype(at::kByte));
+    } catch (const c10::OutOfMemoryError&) {                                                // no room for the images: dQ from the scores
+      ws = at::empty({(int64_t)daisy_b200_swa_attend_bwd_workspace_bytes((int)B, (int)T, (int)H)}, buf.options().dtype(at::kByte));
+    }
     Doc dc = doc_arg(doc.defined() ? OptTensor(doc) : std::nullopt, B, T, buf);
     const int64_t sb = T * H * 128, st = H * 128, sh = 128;
     void* stream = stream_of(buf);
     check(daisy_b200_swa_attend_bwd(p + at_.q, p + at_.k, p + at_.v, p + at_.o, d_o.data_ptr(), sb, st, sh, sb, st, sh, sb, st, sh, sb, st, sh, sb, st, sh,
                                     (const float*)(p + at_.lse), dq, dk, dv, (int)B, (int)T, (int)H, 128, (int)window, scale, dc.ptr, dc.sb,
-                                    bwd_flags, g + ws_at, ws_bytes, status_ptr(buf), stream),
+                                    bwd_flags, ws.data_ptr(), (size_t)ws.numel(), status_ptr(buf), stream),
           "daisy_b200_swa_attend_bwd");
     if (ve2.defined()) {
       d_ve = at::empty({M, dim}, buf.options());

@@ -307,3 +307,34 @@ def test_training_layer_takes_any_alignment():
         ref = ref or got
         assert torch.equal(got[0], ref[0])
         assert all(((a.float() - b.float()).norm() / b.float().norm()).item() <= 2 ** -8 for a, b in zip(got[1:], ref[1:]))
+
+
+def test_backward_without_room_for_the_images():
+    """Where the allocator has no room for the dZ images (268 MB here) the layer's and the operator's backward take the workspace
+    without them: the same dK and dV bits, dQ from the scores formed again, one rounding of dZ to bf16 either way (2^-8)."""
+    from daisy_b200 import B200CausalSelfAttention, WindowMask, ops
+    os.environ["DISABLE_O_ZERO_INIT"] = "1"
+    torch.manual_seed(4)
+    H, T = 2, 8192
+    m = B200CausalSelfAttention(H * D, H, D, receives_ve=False, layer_idx=None, max_seq_len=T).cuda()
+    x = torch.randn(1, T, H * D, device="cuda").bfloat16().requires_grad_(True)
+    q, k, v, d_o = (torch.randn(1, T, H, D, device="cuda").bfloat16() for _ in range(4))
+    q, k = (t / t.float().square().mean(-1, keepdim=True).sqrt().to(t.dtype) for t in (q, k))
+    o, lse2 = ops.swa_attend(q, k, v, T, 0.12, return_lse=True)
+
+    def both():
+        y = m(x, None, attn_mask=WindowMask(T))
+        return [*torch.autograd.grad(y, [x, m.qkvo_w], torch.ones_like(y)), *ops.swa_attend_bwd(q, k, v, o, d_o, lse2, T, 0.12)]
+    ref = both()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    try:
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (200 << 20)) / total)
+        with pytest.raises(torch.cuda.OutOfMemoryError):
+            torch.empty(268 << 20, dtype=torch.uint8, device="cuda")
+        got = both()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    ops.check_device_status("cuda")
+    assert torch.equal(got[3], ref[3]) and torch.equal(got[4], ref[4])
+    assert all(((a.float() - b.float()).norm() / b.float().norm()).item() <= 2 ** -8 for a, b in zip(got, ref))

@@ -452,9 +452,9 @@ def run_prefill(cfg, steps, warmup, dist, rank, world, peaks, name, lean=False, 
 
 def run_prefill_bwd(cfg, steps, warmup, peaks):
     """Backward of the windowed attention at the headline shape (training form): row-wise delta, the
-    key-block-stationary dK/dV kernel and the query-block-stationary dQ kernel.  FLOPs are counted as 2.5 x the forward's
-    (five products over the admitted pairs against the forward's two; the two recomputed score products of the
-    second kernel are not credited)."""
+    key-block-stationary kernel (dK, dV and dZ as operand images) and dQ as a product over the images, the last two once a
+    round of (batch, head) pairs.  FLOPs are counted as 2.5 x the forward's (five products over the admitted pairs against
+    the forward's two)."""
     from daisy_b200 import ops
     from daisy_b200 import accounting as acct
     B, T, H, D, W = cfg["B"], cfg["T"], cfg["H"], cfg["D"], cfg["window"]
@@ -478,7 +478,7 @@ def run_prefill_bwd(cfg, steps, warmup, peaks):
     same = all(torch.equal(a, b) for a, b in zip(first, res["g"]))
     flops = 2.5 * acct.prefill_flops(B, T, H, D, W)
     tf = flops / (ms * 1e-3) / 1e12
-    return {"ms_per_step": ms, "tflops": tf, "value": tf, "unit": "TFLOP/s", "steps": steps, "launches_per_step": 3,
+    return {"ms_per_step": ms, "tflops": tf, "value": tf, "unit": "TFLOP/s", "steps": steps, "launches_per_step": 3,   # with one round; at least
             "flops_counted": "2.5 x forward (dP, dV, dK, dQ and one score product over the admitted pairs)",
             "frac_of_burst_peak": tf / peaks["bf16_tflops"], "finite": bool(all(torch.isfinite(t.float()).all() for t in res["g"])),
             "bitwise_reproducible": bool(same),
@@ -832,7 +832,8 @@ def run_kda(cfg, steps, warmup, dist, rank, world, peaks, lean=False):
     return {"name": "kda_c5", "ms_per_step": per, "value": th / (per * 1e-3), "unit": "token-heads/s",
             "hbm_gbs": world * gbs, "tflops": th * acct.kda_flops_per_token_head(K, K) / (per * 1e-3) / 1e12,
             "scaling": "strong", "strong": strong,
-            "steps": steps, "launches_per_step": 2, "finite": bool(torch.isfinite(res["o"].float()).all()),
+            "steps": steps, "launches_per_step": 2,             # for each part of a long row; at least
+            "finite": bool(torch.isfinite(res["o"].float()).all()),
             "roofline": {"bound": "hbm", "achieved": gbs, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                          "frac": gbs / peaks["hbm_gbs"], "traffic": (kt["bytes"] * th_rank) if kt else None,
                          "traffic_unit": "bytes per call, both kernels (ncu dram read+write on a reduced case, scaled by token-heads; transcribed, see traffic_source)",

@@ -190,9 +190,11 @@ __device__ __forceinline__ BalancedWalk prefill_walk(int nq, int BH, int window,
 // What an item costs beside its tiles, and what a partly visible tile costs, is what short windows and documents are bound by
 // (7 x 1009 x 16, window 249: 22500 cycles an item of four tiles).  So the producer works out the items ahead and hands them out,
 // the output leaves through the item's Q buffer as bulk copies, and a partial tile's 32-column pieces are masked, skipped or
-// taken whole as a warp's rows see them: 44.1 -> 32.1 us there, 8 x 8192 x 16 at window 2048 873 -> 833.  A thread's second 32
-// scores are fetched under its first 32: all 64 at once spilled in the tile loop (1 x 65536, window 8192: 3090 -> 3048; 3031 before
-// all this).
+// taken whole as a warp's rows see them: 44.1 -> 32.1 us there, 8 x 8192 x 16 at window 2048 873 -> 833.
+// Whole tiles have a loop of their own, which keeps what only partial tiles need out of its registers (no spills; 4 to 12 bytes
+// with one loop for both), and a thread's second 32 scores are fetched under its first 32.  1 x 65536 x 16, window 8192, with
+// nearly all tiles whole: 2932 us; one loop 2996, both halves fetched at once in one loop 3073; 2973 for the form without the
+// items handed out.
 template <bool QRAW, bool BOUNDED, int NSPLIT, int STREAMS>
 __global__ void __launch_bounds__(32 * (8 * NSPLIT + 2), 1)
 swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -422,47 +424,69 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       int f_lo = window > 0 ? max(q0 + BM + BN - 1 - window, 0) / BN : 0;
       const int f_hi = q0 / BN - 1;
       if (p.doc_start) f_lo = max(f_lo, (p.doc_start[item->b * p.doc_sb + min(q0 + BM - 1, T - 1)] + BN - 1) / BN);
-      for (int j = jlo; ok && j <= jhi; ++j) {
-        ok = __all_sync(0xffffffffu, mbar_wait(&bars->s_full[s], n_s & 1, abort_flag, p.status, 6));
-        if (!ok) break;
+      auto scores_there = [&]() -> bool {
+        const bool there = __all_sync(0xffffffffu, mbar_wait(&bars->s_full[s], n_s & 1, abort_flag, p.status, 6));
         ++n_s;
         tc_fence_after();
-        uint32_t r[64];
-        tmem_ld32(s_tmem, r);
-        tc_wait_ld();
-        // P of 32 columns and its share of the row sums
-        auto rebuild = [&](int c) {
-          uint32_t pk[16];
+        return there;
+      };
+      // P of 32 columns and its share of the row sums
+      auto rebuild = [&](uint32_t (&r)[64], int c) {
+        uint32_t pk[16];
 #pragma unroll
-          for (int i = 0; i < 32; i += 4) {
-            if (c == 0 && i == 16) tmem_ld32(s_tmem + 32, r + 32);       // the other half of the scores, under this one
-            const uint64_t xa = fmul2(pack2f(__uint_as_float(r[32 * c + i]), __uint_as_float(r[32 * c + i + 1])), c2p);
-            const uint64_t xb = fmul2(pack2f(__uint_as_float(r[32 * c + i + 2]), __uint_as_float(r[32 * c + i + 3])), c2p);
-            float x0, x1, p2, p3;
-            unpack2f(xa, x0, x1);
-            const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
-            uint64_t pb;
-            if (POLY_HALF || (POLY_MASK && (i & POLY_MASK) == POLY_MASK)) {                           // a share of the pairs goes to the FMA pipes
-              pb = exp2_poly2(xb);
-              unpack2f(pb, p2, p3);
-            } else {
-              float x2, x3;
-              unpack2f(xb, x2, x3);
-              p2 = fast_exp2(x2); p3 = fast_exp2(x3);
-              pb = pack2f(p2, p3);
-            }
-            sum_a = fadd2(sum_a, pack2f(p0, p1));
-            sum_b = fadd2(sum_b, pb);
-            pk[i >> 1] = pack_bf16(p0, p1);
-            pk[(i >> 1) + 1] = pack_bf16(p2, p3);
+        for (int i = 0; i < 32; i += 4) {
+          if (c == 0 && i == 16) tmem_ld32(s_tmem + 32, r + 32);       // the other half of the scores, under this one
+          const uint64_t xa = fmul2(pack2f(__uint_as_float(r[32 * c + i]), __uint_as_float(r[32 * c + i + 1])), c2p);
+          const uint64_t xb = fmul2(pack2f(__uint_as_float(r[32 * c + i + 2]), __uint_as_float(r[32 * c + i + 3])), c2p);
+          float x0, x1, p2, p3;
+          unpack2f(xa, x0, x1);
+          const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
+          uint64_t pb;
+          if (POLY_HALF || (POLY_MASK && (i & POLY_MASK) == POLY_MASK)) {                           // a share of the pairs goes to the FMA pipes
+            pb = exp2_poly2(xb);
+            unpack2f(pb, p2, p3);
+          } else {
+            float x2, x3;
+            unpack2f(xb, x2, x3);
+            p2 = fast_exp2(x2); p3 = fast_exp2(x3);
+            pb = pack2f(p2, p3);
           }
-          tmem_st16(s_tmem + 16 * c, pk);
-          if (c == 0) tc_wait_ld();
-        };
+          sum_a = fadd2(sum_a, pack2f(p0, p1));
+          sum_b = fadd2(sum_b, pb);
+          pk[i >> 1] = pack_bf16(p0, p1);
+          pk[(i >> 1) + 1] = pack_bf16(p2, p3);
+        }
+        tmem_st16(s_tmem + 16 * c, pk);
+        if (c == 0) tc_wait_ld();
+      };
+      auto weights_done = [&]() {
+        tc_wait_st();
+        tc_fence_before();
+        mbar_arrive(&bars->p_full[s]);
+      };
+      for (int j = jlo; ok && j <= jhi;) {
         if (j >= f_lo && j <= f_hi) {
-          rebuild(0);
-          rebuild(1);
+          // a run of whole tiles; raw-Q mode stops behind the item's second one
+          int run = min(f_hi, jhi) + 1 - j;
+          if (QRAW && j <= jlo + 1) run = min(run, jlo + 2 - j);
+          j += run;
+          for (; run > 0; --run) {
+            ok = scores_there();
+            if (!ok) break;
+            uint32_t r[64];
+            tmem_ld32(s_tmem, r);
+            tc_wait_ld();
+            rebuild(r, 0);
+            rebuild(r, 1);
+            weights_done();
+          }
+          if (!ok) break;
         } else {
+          ok = scores_there();
+          if (!ok) break;
+          uint32_t r[64];
+          tmem_ld32(s_tmem, r);
+          tc_wait_ld();
           // column i is visible iff lo < i <= hi.  Of a partly visible tile a warp's 32 x 32 piece is mostly all or nothing
           // (element-wise over all 64 columns: 2000 - 2500 cycles a tile against 1250 for a full one)
           const int hi = item->q0[s] + row - (j * BN + half * 64);
@@ -487,13 +511,12 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
               for (int i = 0; i < 32; ++i)
                 if (!((visible >> i) & 1u)) r[32 * c + i] = 0xff800000u;      // -inf -> weight 0
             }
-            rebuild(c);
+            rebuild(r, c);
           }
+          weights_done();
+          ++j;
         }
-        tc_wait_st();
-        tc_fence_before();
-        mbar_arrive(&bars->p_full[s]);
-        if (QRAW && half == 0 && next_valid && !q_prepared && j == jlo + 1) {   // next item's Q, inside this item
+        if (QRAW && half == 0 && next_valid && !q_prepared && j == jlo + 2) {   // next item's Q, inside this item
           ok = prepare_q_tile(bars, q_tiles, s, row, n_qs, q_row_next, p, abort_flag);
           if (!ok) break;
           q_prepared = true;

@@ -170,6 +170,24 @@ def _random_doc_starts(B, T, n_docs, seed, per_batch):
     return torch.stack(rows) if per_batch else rows[0]
 
 
+@pytest.mark.parametrize("B,T,H,window,n_docs", [(8, 700, 8, None, 0), (8, 900, 8, 300, 0), (4, 1300, 8, 512, 0), (8, 700, 8, None, 4), (5, 257, 40, 256, 0)])
+def test_runs_of_whole_tiles(B, T, H, window, n_docs):
+    """Whole tiles are taken in runs: from an item's first tile on, behind a window's edge, behind a document's start, runs of
+    one tile, with more items than SMs; the run ends behind the second tile where the next item's Q is prepared there."""
+    from daisy_b200 import ops, _lib
+    qkv = bf16_randn(B, T, 3 * H, D, seed=T)
+    q, k, v = qkv.chunk(3, dim=-2)
+    cos, sin = swa.rope_tables(D, T)
+    ds = _random_doc_starts(1, T, n_docs, T, False) if n_docs else None
+    doc = None if ds is None else ds.cuda()
+    y_ref, _, _ = swa.swa_prefill(q.float().cpu(), k.float().cpu(), v.float().cpu(), cos, sin, window, **({} if ds is None else {"doc_start": ds}))
+    for flags in (_lib.QKV_DEFAULT, _lib.QKV_DEFAULT | _lib.Q_IN_KERNEL):
+        out = torch.full((B, T, H, D), float("nan"), dtype=torch.bfloat16, device="cuda")
+        ops.swa_prefill(q, k, v, cos.cuda(), sin.cuda(), window, flags=flags, out=out, doc_start=doc)
+        ops.check_device_status(q.device)
+        assert_close_bf16(out, y_ref, f"T={T} W={window} flags={flags}")
+
+
 @pytest.mark.parametrize("T,window,n_docs,per_batch", [(9, 4, 2, False), (300, 64, 5, True), (520, None, 3, False),
                                                         (1300, 512, 4, True), (2100, 1024, 7, True),
                                                         (700, 300, 40, False)])

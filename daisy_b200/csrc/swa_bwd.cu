@@ -137,7 +137,7 @@ template <bool STORE>
 __global__ void __launch_bounds__(KV_THREADS, 1)
 swa_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do, const BwdParams p) {
-  extern __shared__ __align__(1024) uint8_t bwd_smem_raw[];          // (the tiles leave no room to align the start by hand)
+  extern __shared__ __align__(1024) uint8_t bwd_smem_raw[];          // (no room to align the start by hand: bwd_smem_attr asks)
   uint8_t* x_tiles = bwd_smem_raw;                                   // K_j, V_j
   uint8_t* q_tiles = x_tiles + 2 * W_TILE;
   uint8_t* o_tiles = q_tiles + KV_NQ * W_TILE;
@@ -145,10 +145,6 @@ swa_bwd_kv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   int* ends = reinterpret_cast<int*>(col_f + 2 * 2 * WB);            // each key's first query that no longer sees it
   KvBars* bars = reinterpret_cast<KvBars*>(ends + WB);
   volatile int* abort_flag = &bars->abort_flag;
-  if (smem_u32(x_tiles) & 1023) {                                    // never seen; swizzled tiles need it
-    if (threadIdx.x == 0 && p.status) *p.status = DAISY_EALIGN;
-    return;
-  }
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int T = p.T, nblk = (T + WB - 1) / WB;
@@ -1070,6 +1066,15 @@ static int bwd_smem_attr() {
       cudaFuncSetAttribute(swa_bwd_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DQ_SMEM) != cudaSuccess ||
       cudaFuncSetAttribute(swa_bwd_q_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_SMEM) != cudaSuccess)
     return DAISY_ECUDA;
+  // swa_bwd_kv_kernel's swizzled tiles lie at the start of its dynamic shared memory, behind what the system and the kernel's static
+  // variables take: where that is no multiple of 1024 bytes no kernel of the backward is launched
+  int reserved = 0;
+  if (cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev) != cudaSuccess) return DAISY_ECUDA;
+  for (const auto kernel : {swa_bwd_kv_kernel<false>, swa_bwd_kv_kernel<true>}) {
+    cudaFuncAttributes a;
+    if (cudaFuncGetAttributes(&a, kernel) != cudaSuccess) return DAISY_ECUDA;
+    if ((reserved + a.sharedSizeBytes) & 1023) return DAISY_EALIGN;
+  }
   done[dev] = true;
   return DAISY_OK;
 }

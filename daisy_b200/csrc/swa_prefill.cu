@@ -86,6 +86,8 @@ struct PrefillBarriers {
   uint64_t s_full[2];
   uint64_t p_full[2];
   uint64_t o_full[2];
+  uint64_t l_part[2], l_all[2];    // split form: a stream's upper partial row sums, its totals
+  uint64_t out_full[2][2];         // split form: a half's output lies in its Q buffer
   uint64_t i_full[NITEM], i_empty[NITEM];
   ItemGeom item[NITEM];            // as the producer hands them out
   uint32_t tmem_base;
@@ -219,6 +221,8 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       mbar_init(&bars->s_full[s], 1);
       mbar_init(&bars->p_full[s], 128 * NSPLIT);
       mbar_init(&bars->o_full[s], 1);
+      mbar_init(&bars->l_part[s], 4); mbar_init(&bars->l_all[s], 4);          // by warps
+      for (int hf = 0; hf < 2; ++hf) mbar_init(&bars->out_full[s][hf], 4);
     }
     for (int i = 0; i < NSTAGE; ++i) { mbar_init(&bars->kv_full[i], 1); mbar_init(&bars->kv_empty[i], 1); }
     for (int i = 0; i < NITEM; ++i) { mbar_init(&bars->i_full[i], 1); mbar_init(&bars->i_empty[i], 8 * NSPLIT + 1); }   // issuer, softmax warps
@@ -408,9 +412,8 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       bool next_valid = false;
       int q_row_next = 0;
       if (QRAW && half == 0) {
-        // a wait that ran out must not leave the item loop here: the stream's other half still comes to the two
-        // named barriers below, which need all 256 threads -- skip the tile loop and the epilogue instead
         if (!q_prepared) ok = prepare_q_tile(bars, q_tiles, s, row, n_qs, q_row, p, abort_flag);
+        if (!ok) break;
         q_prepared = false;
         const int item_next = walk.at(rd + 1);
         if (item_next >= 0) {
@@ -522,6 +525,7 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           q_prepared = true;
         }
       }
+      if (!ok) break;
       float l;
       {
         float a0, a1, b0, b1;
@@ -529,20 +533,31 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         unpack2f(sum_b, b0, b1);
         l = (a0 + a1) + (b0 + b1);
       }
-      // the upper half publishes its partial sum, the lower half replaces it by the total (one slot per row)
-      if (half == 1) *lsum = l;
-      if (s == 0) asm volatile("bar.sync 1, 256;" ::: "memory");       // the 256 threads of this stream
-      else        asm volatile("bar.sync 2, 256;" ::: "memory");
-      if (half == 0) { l += *lsum; *lsum = l; }
-      if (s == 0) asm volatile("bar.sync 1, 256;" ::: "memory");
-      else        asm volatile("bar.sync 2, 256;" ::: "memory");
-      if (half == 1) l = *lsum;
-      if (p.lse2 && half == 0 && q_row < T) p.lse2[((int64_t)item->b * p.H + item->h) * T + q_row] = __log2f(l);   // no reference maximum in this form
-      if (ok) {
-        ok = __all_sync(0xffffffffu, mbar_wait(&bars->o_full[s], n_o & 1, abort_flag, p.status, 7));
-        ++n_o;
+      // The upper half publishes its partial sum, the lower half replaces it by the total (one slot per row).  Warps give up on
+      // their own, so they wait for one another in bounded waits only: at a named barrier those that go on would wait for good.
+      auto all_wait = [&](uint64_t* bar) {
+        return __all_sync(0xffffffffu, mbar_wait(bar, n_o & 1, abort_flag, p.status, 15));
+      };
+      auto warp_arrive = [&](uint64_t* bar) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar);
+      };
+      if (half == 1) {
+        *lsum = l;
+        warp_arrive(&bars->l_part[s]);
+        ok = all_wait(&bars->l_all[s]);
+        l = *lsum;
+      } else {
+        ok = all_wait(&bars->l_part[s]);
+        l += *lsum;
+        *lsum = l;
+        warp_arrive(&bars->l_all[s]);
       }
-      if (ok) {
+      if (!ok) break;
+      if (p.lse2 && half == 0 && q_row < T) p.lse2[((int64_t)item->b * p.H + item->h) * T + q_row] = __log2f(l);   // no reference maximum in this form
+      ok = all_wait(&bars->o_full[s]);
+      if (!ok) break;
+      {
         tc_fence_after();
         const float inv = 1.0f / l;
         uint32_t r[64];
@@ -560,13 +575,18 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         }
         // out through this item's Q buffer, whose last product was over before O_s was: this half's 64 columns are one swizzled box
         // (stores from registers, transposed to whole row segments by shuffles, took 2200 cycles an item)
-        uint8_t* box = q_tiles + (((n_o - 1) % NQBUF) * 2 + s) * TILE_BYTES + half * HALF_BYTES;
+        uint8_t* box = q_tiles + ((n_o % NQBUF) * 2 + s) * TILE_BYTES + half * HALF_BYTES;
         const uint32_t dst = smem_u32(box) + row * 128;
 #pragma unroll
         for (int c = 0; c < 8; ++c)
           asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst + ((c ^ (row & 7)) << 4)), "r"(ch[c].x), "r"(ch[c].y), "r"(ch[c].z), "r"(ch[c].w) : "memory");
         fence_proxy_async();
-        named_bar(3 + 2 * s + half, 128);
+        warp_arrive(&bars->out_full[s][half]);
+        if ((warp & 3) == 0) {
+          ok = all_wait(&bars->out_full[s][half]);
+          if (!ok) break;
+        }
+        ++n_o;
         if (out_thread) {
           tma_store_4d(&tm_o, box, 64 * half, q0, item->h, item->b);       // rows past T stay out of it
           asm volatile("cp.async.bulk.commit_group;" ::: "memory");

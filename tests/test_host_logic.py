@@ -1,6 +1,7 @@
 """Host-side logic that needs no GPU: ring index arithmetic, mask descriptor parsing, module construction,
 and the sharding arithmetic of the multi-GPU bench (world_size-2 gloo)."""
 import os
+import re
 import socket
 
 import pytest
@@ -207,3 +208,15 @@ def test_kda_step_graph_without_states_raises():
         with pytest.raises(RuntimeError):
             m.step_graph(x)
     assert m._seen == 0
+
+
+def test_prefill_warps_wait_for_one_another_in_bounded_waits_only():
+    """A warp of the attention kernel leaves when a wait runs out, whether or not the others see the same: at a barrier without a
+    limit they would wait for it for good.  The two block-wide barriers left are those before the roles part and after they meet."""
+    import daisy_b200
+    src = open(os.path.join(os.path.dirname(daisy_b200.__file__), "csrc", "swa_prefill.cu")).read()
+    code = re.sub(r"//[^\n]*", "", src)
+    kernel = code[code.index("swa_prefill_kernel("):]
+    kernel = kernel[:kernel.index("__global__")]
+    assert not re.search(r"\bnamed_bar|\bbar\.(sync|red|arrive)|\bbarrier\.", kernel)
+    assert kernel.count("__syncthreads") == 2

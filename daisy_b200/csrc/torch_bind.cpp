@@ -364,6 +364,35 @@ Tensor attn_stack(const Tensor& x_, const std::vector<Tensor>& weights, const st
   return ya;
 }
 
+// Workspace of an attention backward: with room for the dZ images, up to 2 GB, where the allocator has it, else without (dQ from
+// the scores).  Before the allocator refuses it gives back every block it has cached, behind waits for the device: a size it refused
+// is not asked for again in the next REFUSED_CALLS calls on that device.
+constexpr int REFUSED_CALLS = 256;
+struct Refused { int64_t bytes = 0; int calls = 0; };
+Refused g_refused[MAX_DEV];
+
+Tensor bwd_workspace(const Tensor& like, int64_t B, int64_t T, int64_t H, int64_t window, bool in_blocks) {
+  const int64_t full = (int64_t)daisy_b200_swa_attend_bwd_workspace_bytes_full((int)B, (int)T, (int)H, (int)window, in_blocks ? DAISY_WINDOW_BLOCKS : 0);
+  const auto bytes = like.options().dtype(at::kByte);
+  const int dev = like.get_device();
+  TORCH_CHECK(dev >= 0 && dev < MAX_DEV, "device index out of range");
+  bool ask = true;
+  {
+    std::lock_guard<std::mutex> lock(g_mutex);
+    Refused& r = g_refused[dev];
+    if (r.calls > 0) { --r.calls; ask = full < r.bytes; }
+  }
+  if (ask) {
+    try {
+      return at::empty({full}, bytes);
+    } catch (const c10::OutOfMemoryError&) {
+      std::lock_guard<std::mutex> lock(g_mutex);
+      g_refused[dev] = {full, REFUSED_CALLS};
+    }
+  }
+  return at::empty({(int64_t)daisy_b200_swa_attend_bwd_workspace_bytes((int)B, (int)T, (int)H)}, bytes);
+}
+
 // ------------------------------------------------------------------ attention layer under autograd
 // Forward: the fused projection (which also leaves 1 / rms of every head row), attention with its log-sum-exp, output
 // projection.  Backward: two library products for each projection, the attention backward, and one row-wise pass that undoes
@@ -456,12 +485,7 @@ struct AttnFunction : public torch::autograd::Function<AttnFunction> {
     Tensor tmp = at::empty({(part_at + Saved::up(4 * n_part)) / 2}, buf.options());          // dqkv, dq, dk, dv, partial sums
     char *g = (char*)tmp.data_ptr(), *dq = g + 3 * row, *dk = g + 4 * row, *dv = g + 5 * row;
     Tensor dqkv = tmp.narrow(0, 0, M * 3 * dim).view({M, 3 * dim}), d_ve, d_logit;
-    Tensor ws;
-    try {
-      ws = at::empty({(int64_t)daisy_b200_swa_attend_bwd_workspace_bytes_full((int)B, (int)T, (int)H, (int)window, bwd_flags)}, buf.options().dtype(at::kByte));
-    } catch (const c10::OutOfMemoryError&) {                                                // no room for the images: dQ from the scores
-      ws = at::empty({(int64_t)daisy_b200_swa_attend_bwd_workspace_bytes((int)B, (int)T, (int)H)}, buf.options().dtype(at::kByte));
-    }
+    Tensor ws = bwd_workspace(buf, B, T, H, window, d[4]);
     Doc dc = doc_arg(doc.defined() ? OptTensor(doc) : std::nullopt, B, T, buf);
     const int64_t sb = T * H * 128, st = H * 128, sh = 128;
     void* stream = stream_of(buf);
@@ -905,6 +929,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                          const OptTensor& doc_start, bool in_blocks) {
     return swa_attend(q, k, v, window, scale, out, bounded, doc_start, in_blocks, false).first;
   }, nogil());
+  m.def("bwd_workspace", &bwd_workspace, nogil());
   m.def("swa_attend_lse", [](const Tensor& q, const Tensor& k, const Tensor& v, int64_t window, double scale, const OptTensor& out, bool bounded,
                              const OptTensor& doc_start, bool in_blocks) {
     return swa_attend(q, k, v, window, scale, out, bounded, doc_start, in_blocks, true);

@@ -170,10 +170,7 @@ def swa_attend_bwd(q, k, v, o, d_o, lse2, window: Optional[int], scale: float = 
     dq, dk, dv = (torch.empty(B, T, H, D, dtype=torch.bfloat16, device=q.device) for _ in range(3))
     L = _lib.lib()
     flags = _lib.WINDOW_BLOCKS if window_in_blocks else 0
-    try:
-        ws = torch.empty(L.daisy_b200_swa_attend_bwd_workspace_bytes_full(B, T, H, int(window or 0), flags), dtype=torch.uint8, device=q.device)
-    except torch.cuda.OutOfMemoryError:                       # no room for the images: dQ from the scores
-        ws = torch.empty(L.daisy_b200_swa_attend_bwd_workspace_bytes(B, T, H), dtype=torch.uint8, device=q.device)
+    ws = ext().bwd_workspace(q, B, T, H, int(window or 0), window_in_blocks)
     _doc, doc_ptr, doc_sb = _doc_arg(doc_start, B, T, q.device)
     st = lambda t: (t.stride(0), t.stride(1), t.stride(2))
     rc = L.daisy_b200_swa_attend_bwd(

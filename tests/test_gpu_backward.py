@@ -338,3 +338,41 @@ def test_backward_without_room_for_the_images():
     ops.check_device_status("cuda")
     assert torch.equal(got[3], ref[3]) and torch.equal(got[4], ref[4])
     assert all(((a.float() - b.float()).norm() / b.float().norm()).item() <= 2 ** -8 for a, b in zip(got, ref))
+
+
+def test_backward_asks_once_for_room_that_is_refused():
+    """A refused workspace costs the allocator its cached blocks and waits for the device: the operator and the layer, whose images
+    are of one size, ask for it once between them and not in every call, and go on asking for what is smaller."""
+    from daisy_b200 import B200CausalSelfAttention, WindowMask, ops
+    os.environ["DISABLE_O_ZERO_INIT"] = "1"
+    torch.manual_seed(5)
+    H, T = 2, 16384
+    m = B200CausalSelfAttention(H * D, H, D, receives_ve=False, layer_idx=None, max_seq_len=T).cuda()
+    x = torch.randn(1, T, H * D, device="cuda").bfloat16().requires_grad_(True)
+
+    def call(t):
+        q, k, v, o, d_o = (torch.zeros(1, t, H, D, device="cuda", dtype=torch.bfloat16) for _ in range(5))
+        return ops.swa_attend_bwd(q, k, v, o, d_o, torch.zeros(1, H, t, device="cuda"), None)
+
+    def layer():
+        y = m(x, None, attn_mask=WindowMask(T))
+        torch.autograd.grad(y, [x, m.qkvo_w], torch.ones_like(y))
+    layer()
+    call(1024)
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    refused = lambda: torch.cuda.memory_stats()["num_alloc_retries"]
+    try:
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (400 << 20)) / total)
+        before = refused()
+        for _ in range(4):
+            call(T)
+            layer()
+        assert refused() - before <= 1                           # none where a test before this one met the refusal
+        torch.cuda.reset_peak_memory_stats()
+        held = torch.cuda.memory_allocated()
+        call(1024)
+        assert torch.cuda.max_memory_allocated() - held > 6 << 20     # inputs and gradients are 4 MB; images 2 x 36 of 32 KB at least
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    ops.check_device_status("cuda")

@@ -259,3 +259,41 @@ def test_block_window_training_form_matches_oracle(T, wb, n_docs):
     if T // 128 > wb and n_docs <= 6:                             # differs from the token-exact window of wb * 128
         y_tok, _, _ = ops.swa_prefill(q, k, v, cos.cuda(), sin.cuda(), wb * 128, doc_start=dsc)
         assert (y_tok.float() - y.float()).abs().max().item() > 1e-3
+
+
+@pytest.mark.parametrize("T,window,bounded", [(1, None, True), (131, 100, True), (300, None, True), (1300, 512, True), (300, 64, False)])
+@pytest.mark.parametrize("layout", ["padded", "transposed", "batch_inside"])
+def test_output_of_any_layout(T, window, bounded, layout):
+    """Outputs with gaps between rows and heads or another order of dimensions: the bits of the contiguous one (the bounded form
+    writes through a tensor map, whole tiles with rows past T among them), and nothing written in the gaps."""
+    from daisy_b200 import ops
+    B, H = 2, 3
+    q, k, v = (bf16_randn(B, T, H, D, seed=30 + i) for i in range(3))
+    q, k = (t / t.float().square().mean(-1, keepdim=True).sqrt().to(t.dtype) for t in (q, k))
+    ref, lse_ref = ops.swa_attend(q, k, v, window, bounded_qk=bounded, return_lse=True)
+    shape, view = {"padded": ((B + 1, T + 3, H + 2, D + 8), lambda t: t[:B, 2:T + 2, 1:H + 1, :D]),
+                   "transposed": ((B, H, T + 130, D), lambda t: t[:, :, :T].transpose(1, 2)),
+                   "batch_inside": ((T + 1, B, H, D), lambda t: t[1:].transpose(0, 1))}[layout]
+    buf = torch.full(shape, 7.0, dtype=torch.bfloat16, device="cuda")
+    out, lse = ops.swa_attend(q, k, v, window, bounded_qk=bounded, out=view(buf), return_lse=True)
+    ops.check_device_status(q.device)
+    assert torch.equal(view(buf), ref) and torch.equal(lse, lse_ref)
+    view(buf).fill_(7.0)
+    assert bool((buf == 7).all())
+    assert torch.equal(ops.swa_attend(q, k, v, window, bounded_qk=bounded, out=view(buf)), ref)
+
+
+@pytest.mark.parametrize("lse", [False, True])
+def test_output_that_no_tensor_map_describes(lse):
+    """One row whose row stride is zero: the call takes the general form, whose bits are those without the bound."""
+    from daisy_b200 import ops
+    B, H = 3, 4
+    q, k, v = (bf16_randn(B, 1, H, D, seed=40 + i) for i in range(3))
+    q, k = (t / t.float().square().mean(-1, keepdim=True).sqrt().to(t.dtype) for t in (q, k))
+    buf = torch.full((B, H, D), 7.0, dtype=torch.bfloat16, device="cuda")
+    out = buf.as_strided((B, 1, H, D), (H * D, 0, D, 1))
+    got, ref = (ops.swa_attend(q, k, v, None, return_lse=lse, **kw) for kw in ({"bounded_qk": True, "out": out}, {}))
+    ops.check_device_status(q.device)
+    for a, b in zip(got if lse else (got,), ref if lse else (ref,)):
+        assert torch.equal(a, b)
+    assert torch.equal(buf, v[:, 0])                              # one key: its value

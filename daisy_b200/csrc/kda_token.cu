@@ -1,6 +1,7 @@
-// One decoded token through a Kimi-delta-attention layer in ONE launch: the projections, the short convolutions with their
+// One decoded token through a Kimi-delta-attention layer: the projections, the short convolutions with their
 // carried state, the decay gate, the recurrent state update, the gated norm and the output projection
-// (KimiLinearSelfAttention.step, models/daisy/attention_kimi.py:128-211 with T = 1 and the cached states).
+// (KimiLinearSelfAttention.step, models/daisy/attention_kimi.py:128-211 with T = 1 and the cached states).  One launch up to
+// TK_MAX_B rows and KT_ONE_PAIRS (row, head) pairs, four above (kda_batch_kernel).
 //
 // Bound: HBM and latency -- at dim 2048 and batch 1 the weights are 35 MB (5.4 us at copy bandwidth) and the state 2 MB, but
 // as seventeen dependent launches of 2-5 us the step took 79 us replayed as a graph and 278 us issued from Python.  As in

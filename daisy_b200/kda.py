@@ -180,8 +180,8 @@ class B200KimiLinearSelfAttention(torch.nn.Module):
         self._recurrent_state, self._conv_state, self._seen = None, None, 0
 
     def _token_step(self, x, out=None, workspace=None):
-        """The decode step as one native call (``csrc/kda_token.cu``; one launch up to 16 batch rows, four above), states updated
-        in place; None where the layer or its states are not of the form those kernels take."""
+        """The decode step as one native call (``csrc/kda_token.cu``; one launch up to 16 batch rows and 168 (row, head) pairs, four
+        above), states updated in place; None where the layer or its states are not of the form those kernels take."""
         rec, conv = self._recurrent_state, self._conv_state
         if (rec is None or conv is None or x.shape[1] != 1 or not x.is_cuda or self.hidden_size != self.key_dim
                 or self.head_dim != 128 or not ext().kda_token_supported(self.num_heads)
@@ -293,7 +293,7 @@ class B200KimiLinearSelfAttention(torch.nn.Module):
     @torch.inference_mode()
     def capture_step(self, batch: int = 1) -> None:
         """Prepare ``step_graph``: a single-token ``step`` (no value embedding) into a fixed output buffer.  Needs the states a
-        ``prefill`` leaves; they are updated in place.  Where the layer takes the single-launch step that launch is all of it;
+        ``prefill`` leaves; they are updated in place.  Where the layer takes the native step (one launch or four) that is all of it;
         otherwise the step is recorded into a CUDA graph, and ``step_graph(x)`` costs one copy and one graph launch."""
         if self._recurrent_state is None or (self.use_short_conv and self._conv_state is None):
             raise RuntimeError("capture_step needs the cached states of a prefill")
@@ -314,12 +314,12 @@ class B200KimiLinearSelfAttention(torch.nn.Module):
         side = torch.cuda.Stream(device=dev)
         side.wait_stream(torch.cuda.current_stream(dev))
         with torch.cuda.stream(side):                              # warm-up outside the capture (lazy initialisation)
-            one_launch = ext().kda_token_supported(self.num_heads) and self._token_step(self._gx, self._gy, self._gws) is not None
-            if not one_launch:
+            native = ext().kda_token_supported(self.num_heads) and self._token_step(self._gx, self._gy, self._gws) is not None
+            if not native:
                 self._forward_core(self._gx, None, None, None, use_cache=True)
         torch.cuda.current_stream(dev).wait_stream(side)
         restore()
-        if one_launch:
+        if native:
             return
         self._graph = torch.cuda.CUDAGraph()
         self._gstates = (self._recurrent_state, *(self._conv_state or ()))     # what the graph updates: kept as long as it is
@@ -330,7 +330,7 @@ class B200KimiLinearSelfAttention(torch.nn.Module):
     @torch.inference_mode()
     def step_graph(self, x):
         """``step`` into the fixed buffer: ``x [batch, 1, dim]`` -> ``y`` (overwritten by the next call).  ``x`` may lie on the
-        host or broadcast to that shape.  The states of the layer must be there: one launch takes them where they are (another
+        host or broadcast to that shape.  The states of the layer must be there: the native step takes them where they are (another
         ``prefill`` of the same batch may have made them), a graph only those ``capture_step`` saw."""
         if self._graph is None:
             if x.get_device() != self._gx.get_device() or x.shape != self._gx.shape:

@@ -133,8 +133,9 @@ def test_kimi_token_step_continues_a_prefill(B, H, bias):
 
 @pytest.mark.parametrize("B,H,bias", [(17, 1, True), (33, 3, False), (64, 16, True)])
 def test_kimi_batch_step_matches_row_launches(B, H, bias):
-    """Above 16 rows (kda_batch_kernel between GEMMs) against the single launch on 16 rows at a time: the convolution states bit
-    for bit but for the new input, everything else to the order of fp32 sums under bf16 roundings."""
+    """Above 16 rows (kda_batch_kernel between GEMMs) against the single launch on as many rows at a time as it takes (16, and 168
+    (row, head) pairs): the convolution states bit for bit but for the new input, everything else to the order of fp32 sums under
+    bf16 roundings."""
     from daisy_b200 import B200KimiLinearSelfAttention, ops
     torch.manual_seed(B)
     layer = B200KimiLinearSelfAttention(H * D, H, 4096, D, conv_bias=bias).cuda()
@@ -145,9 +146,10 @@ def test_kimi_batch_step_matches_row_launches(B, H, bias):
         y, _, _ = layer.step(x[:, 29:])
         got = (y, layer._recurrent_state, *layer._conv_state)
         ys = []
-        for b in range(0, B, 16):
-            layer._recurrent_state, layer._conv_state = rec[b:b + 16].clone(), tuple(c[b:b + 16].clone() for c in conv)
-            ys.append((layer.step(x[b:b + 16, 29:])[0], layer._recurrent_state, *layer._conv_state))
+        n = min(16, 168 // H)
+        for b in range(0, B, n):
+            layer._recurrent_state, layer._conv_state = rec[b:b + n].clone(), tuple(c[b:b + n].clone() for c in conv)
+            ys.append((layer.step(x[b:b + n, 29:])[0], layer._recurrent_state, *layer._conv_state))
     ops.check_device_status("cuda")
     ref = [torch.cat(t) for t in zip(*ys)]
     assert_close_bf16(got[0], ref[0], "y", max_tol=3e-2, mean_tol=3e-3)

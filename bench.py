@@ -455,7 +455,7 @@ def run_prefill_bwd(cfg, steps, warmup, peaks):
     key-block-stationary kernel (dK, dV and dZ as operand images) and dQ as a product over the images, the last two once a
     round of (batch, head) pairs.  FLOPs are counted as 2.5 x the forward's (five products over the admitted pairs against
     the forward's two)."""
-    from daisy_b200 import ops
+    from daisy_b200 import ops, _lib
     from daisy_b200 import accounting as acct
     B, T, H, D, W = cfg["B"], cfg["T"], cfg["H"], cfg["D"], cfg["window"]
     dev = torch.device("cuda", torch.cuda.current_device())
@@ -478,7 +478,9 @@ def run_prefill_bwd(cfg, steps, warmup, peaks):
     same = all(torch.equal(a, b) for a, b in zip(first, res["g"]))
     flops = 2.5 * acct.prefill_flops(B, T, H, D, W)
     tf = flops / (ms * 1e-3) / 1e12
-    return {"ms_per_step": ms, "tflops": tf, "value": tf, "unit": "TFLOP/s", "steps": steps, "launches_per_step": 3,   # with one round; at least
+    L = _lib.lib()
+    rounds = L.daisy_b200_swa_attend_bwd_rounds(B, T, H, W, 0, L.daisy_b200_swa_attend_bwd_workspace_bytes_full(B, T, H, W, 0))
+    return {"ms_per_step": ms, "tflops": tf, "value": tf, "unit": "TFLOP/s", "steps": steps, "launches_per_step": 1 + 2 * rounds,
             "flops_counted": "2.5 x forward (dP, dV, dK, dQ and one score product over the admitted pairs)",
             "frac_of_burst_peak": tf / peaks["bf16_tflops"], "finite": bool(all(torch.isfinite(t.float()).all() for t in res["g"])),
             "bitwise_reproducible": bool(same),
@@ -764,7 +766,7 @@ def kda_inputs(cfg, b_lo, b_hi, h_lo, h_hi, dev):
 def run_kda(cfg, steps, warmup, dist, rank, world, peaks, lean=False):
     """The B x H (batch, head) pairs are sharded over the ranks (one global problem, strong scaling); rank 0 also runs
     all of them alone for T(1) when there is more than one rank."""
-    from daisy_b200 import ops
+    from daisy_b200 import ops, _lib
     from daisy_b200 import accounting as acct
     B, T, H, K = cfg["B"], cfg["T"], cfg["H"], cfg["K"]
     dev = torch.device("cuda", torch.cuda.current_device())
@@ -785,9 +787,10 @@ def run_kda(cfg, steps, warmup, dist, rank, world, peaks, lean=False):
     th_rank = Bs * T * Hs
     byts = th_rank * acct.kda_bytes_per_token_head(K, K)
     gbs = byts / (per * 1e-3) / 1e9
+    launches = 2 * _lib.lib().daisy_b200_kda_parts(Bs, T, Hs)
     if lean:
         return {"name": "kda", "ms_per_step": per, "value": th / (per * 1e-3), "unit": "token-heads/s", "steps": steps,
-                "launches_per_step": 2, "roofline": None, "e2e": None,
+                "launches_per_step": launches, "roofline": None, "e2e": None,
                 "config": {"workload": f"kda: B={B} T={T} H={H} K=V={K} (profiler capture case)"}}
     # e2e: host tensors in, output back
     hq, hk, hv, hg, hb = (x.cpu().pin_memory() for x in (q, k, v, g, beta))
@@ -832,7 +835,7 @@ def run_kda(cfg, steps, warmup, dist, rank, world, peaks, lean=False):
     return {"name": "kda_c5", "ms_per_step": per, "value": th / (per * 1e-3), "unit": "token-heads/s",
             "hbm_gbs": world * gbs, "tflops": th * acct.kda_flops_per_token_head(K, K) / (per * 1e-3) / 1e12,
             "scaling": "strong", "strong": strong,
-            "steps": steps, "launches_per_step": 2,             # for each part of a long row; at least
+            "steps": steps, "launches_per_step": launches,
             "finite": bool(torch.isfinite(res["o"].float()).all()),
             "roofline": {"bound": "hbm", "achieved": gbs, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                          "frac": gbs / peaks["hbm_gbs"], "traffic": (kt["bytes"] * th_rank) if kt else None,

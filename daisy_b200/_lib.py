@@ -39,6 +39,7 @@ SIGNATURES = {
     "daisy_b200_swa_attend_lse": (_i, [_vp] * 3 + [_i64] * 9 + [_vp] + [_i64] * 3 + [_vp] + [_i] * 5 + [_f, _vp, _i64, _u, _vp, _vp]),
     "daisy_b200_swa_attend_bwd_workspace_bytes": (_sz, [_i] * 3),
     "daisy_b200_swa_attend_bwd_workspace_bytes_full": (_sz, [_i] * 4 + [_u]),
+    "daisy_b200_swa_attend_bwd_rounds": (_i, [_i] * 4 + [_u, _sz]),
     "daisy_b200_swa_attend_bwd": (_i, [_vp] * 5 + [_i64] * 15 + [_vp] * 4 + [_i] * 5 + [_f, _vp, _i64, _u, _vp, _sz, _vp, _vp]),
     "daisy_b200_qkv_prep_bwd": (_i, [_vp] * 3 + [_i64] * 9 + [_vp] * 2 + [_vp] * 6 + [_i] * 4 + [_f, _u, _vp]),
     "daisy_b200_swa_decode_splits": (_i, [_i] * 4),
@@ -69,6 +70,7 @@ SIGNATURES = {
                                           [_i, _vp, _vp]),
     "daisy_b200_ring_copy_rows": (_i, [_vp] + [_i64] * 3 + [_vp] + [_i64] * 3 + [_i] * 4 + [_i64] + [_i] * 3 + [_vp]),
     "daisy_b200_kda_workspace_bytes": (_sz, [_i] * 5),
+    "daisy_b200_kda_parts": (_i, [_i] * 3),
     "daisy_b200_kda_chunk_fwd": (_i, [_vp] * 8 + [_i] * 6 + [_f, _u, _vp, _sz, _vp, _vp]),
     "daisy_b200_kda_varlen_workspace_bytes": (_sz, [_i] * 4),
     "daisy_b200_kda_chunk_fwd_varlen": (_i, [_vp] * 8 + [_i] * 5 + [_f, _u, _vp, _i, _vp, _i, _vp, _sz, _vp, _vp]),

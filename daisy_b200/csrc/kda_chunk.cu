@@ -921,6 +921,13 @@ static int kda_split(int rows, int NC, int sms, int* end) {
   return best;
 }
 
+extern "C" int daisy_b200_kda_parts(int B, int T, int H) {
+  if (B <= 0 || T <= 0 || H <= 0) return DAISY_EINVAL;
+  const int sms = daisy_host::sm_count_cached();
+  int end[KDA_PARTS];
+  return sms > 0 ? kda_split(B * H, (T + KC - 1) / KC, sms, end) : DAISY_ENODEV;
+}
+
 // Shared launcher.  Dense: NC = ceil(T / 64) chunks per (batch, head) row, n_seq = B.  Packed variable-length (B = 1):
 // chunk_tab [NC][2] and seq_ptr [n_seq + 1] (both in device memory) say which tokens each chunk covers and which
 // chunks each sequence owns; h0 / hT are [n_seq, H, K, V].

@@ -1053,7 +1053,7 @@ __global__ void __launch_bounds__(1024) gate_grad_kernel(const float* partial, i
 using namespace daisy;
 
 // Most bytes of dZ images that a call asks room for (above that the (batch, head) pairs go in several rounds).  8 x 8192 tokens,
-// 16 heads, window 2048 are 4.3 GB: two rounds.
+// 16 heads are 4.6 GB at a window of 2048 tokens, three rounds, and 4.3 GB at one of 16 blocks of 128, two.
 static constexpr size_t BWD_TILES_MAX = (size_t)2 << 30;
 
 static int bwd_smem_attr() {
@@ -1099,6 +1099,23 @@ extern "C" size_t daisy_b200_swa_attend_bwd_workspace_bytes_full(int B, int T, i
   const size_t one = bwd_tiles_bytes(T, window, (flags & DAISY_WINDOW_BLOCKS) != 0), pairs = (size_t)B * H;
   const size_t n = BWD_TILES_MAX / one < pairs ? BWD_TILES_MAX / one : pairs;
   return n ? bwd_delta_bytes(B, T, H) + n * one : daisy_b200_swa_attend_bwd_workspace_bytes(B, T, H);
+}
+
+// (batch, head) pairs a round takes: rounds of equal size, as many as there is room for images; 0: no room for one pair's
+static int bwd_pairs_a_round(int B, int T, int H, int window, bool in_blocks, size_t workspace_bytes) {
+  const size_t delta_bytes = bwd_delta_bytes(B, T, H);
+  const int64_t room = workspace_bytes > delta_bytes ? (int64_t)((workspace_bytes - delta_bytes) / bwd_tiles_bytes(T, window, in_blocks)) : 0;
+  if (room == 0) return 0;
+  const int64_t pairs = (int64_t)B * H, rounds = (pairs + room - 1) / room;
+  return (int)((pairs + rounds - 1) / rounds);
+}
+
+extern "C" int daisy_b200_swa_attend_bwd_rounds(int B, int T, int H, int window, unsigned flags, size_t workspace_bytes) {
+  if (B <= 0 || T <= 0 || H <= 0 || (flags & ~DAISY_WINDOW_BLOCKS)) return DAISY_EINVAL;
+  if ((int64_t)B * T * H >= (int64_t)1 << 31) return DAISY_EUNSUPPORTED;
+  if (workspace_bytes < daisy_b200_swa_attend_bwd_workspace_bytes(B, T, H)) return DAISY_EWORKSPACE;
+  const int per = bwd_pairs_a_round(B, T, H, window, (flags & DAISY_WINDOW_BLOCKS) != 0, workspace_bytes);
+  return per ? (B * H + per - 1) / per : 1;
 }
 
 extern "C" int daisy_b200_swa_attend_bwd(const void* q, const void* k, const void* v, const void* o, const void* d_o,
@@ -1150,12 +1167,8 @@ extern "C" int daisy_b200_swa_attend_bwd(const void* q, const void* k, const voi
   const int sms = daisy_host::sm_count_cached();
   if (sms <= 0) return DAISY_ENODEV;
   const int nblk = (T + WB - 1) / WB;
-  const size_t one = bwd_tiles_bytes(T, window, in_blocks), delta_bytes = bwd_delta_bytes(B, T, H);
-  const size_t room = workspace_bytes > delta_bytes ? (workspace_bytes - delta_bytes) / one : 0;
-  const int pairs = B * H;
-  p.tiles = (uint8_t*)workspace + delta_bytes; p.tiles_row = (int)bwd_tiles_row(T, window, in_blocks);
-  // rounds of equal size, as many (batch, head) pairs at a time as there is room for images; without room for one pair's all in one
-  const int rounds = room ? (int)((pairs + room - 1) / room) : 1, per = (pairs + rounds - 1) / rounds;
+  const int room = bwd_pairs_a_round(B, T, H, window, in_blocks, workspace_bytes), pairs = B * H, per = room ? room : pairs;
+  p.tiles = (uint8_t*)workspace + bwd_delta_bytes(B, T, H); p.tiles_row = (int)bwd_tiles_row(T, window, in_blocks);
   for (p.bh0 = 0; p.bh0 < pairs; p.bh0 += per) {
     p.n_bh = pairs - p.bh0 < per ? pairs - p.bh0 : per;
     const int64_t items = (int64_t)nblk * p.n_bh;

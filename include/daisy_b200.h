@@ -250,6 +250,8 @@ int daisy_b200_swa_attend_lse(const void* q, const void* k, const void* v,
  * (batch, head) pairs as the workspace holds; no atomics: results are bitwise reproducible. */
 size_t daisy_b200_swa_attend_bwd_workspace_bytes(int B, int T, int H);
 size_t daisy_b200_swa_attend_bwd_workspace_bytes_full(int B, int T, int H, int window, unsigned flags);
+/* How many times the last two are launched with a workspace of that size (or an error). */
+int daisy_b200_swa_attend_bwd_rounds(int B, int T, int H, int window, unsigned flags, size_t workspace_bytes);
 int daisy_b200_swa_attend_bwd(const void* q, const void* k, const void* v, const void* o, const void* d_o,
                               int64_t q_sb, int64_t q_st, int64_t q_sh,
                               int64_t k_sb, int64_t k_st, int64_t k_sh,
@@ -392,6 +394,8 @@ int daisy_b200_ring_copy_rows(void* ring, int64_t r_sb, int64_t r_sh, int64_t r_
  *   scale <= 0 selects K^-1/2.
  */
 size_t daisy_b200_kda_workspace_bytes(int B, int T, int H, int K, int V);
+/* In how many parts the dense call goes on the current device, two launches each (or an error). */
+int daisy_b200_kda_parts(int B, int T, int H);
 int daisy_b200_kda_chunk_fwd(const void* q, const void* k, const void* v, const float* g,
                              const float* beta, const float* h0, void* o, float* hT,
                              int B, int T, int H, int K, int V, int chunk, float scale,

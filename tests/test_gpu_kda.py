@@ -338,10 +338,14 @@ def test_waiting_for_packed_lengths_leaves_other_threads_running():
         torch.cuda.synchronize()
 
 
-@pytest.mark.parametrize("B,T,H", [(1, 64 * 30 + 1, 4), (2, 64 * 47 - 7, 16), (1, 64 * 150, 12), (4, 64 * 60 + 33, 16), (1, 64 * 20, 112)])
-def test_kda_in_parts_has_the_bits_of_one_pass(B, T, H):
+@pytest.mark.parametrize("B,T,H,parts", [(1, 64 * 30 + 1, 4, 1), (1, 64 * 20, 112, 1), (2, 1000, 16, 2), (1, 64 * 40 + 5, 64, 2), (2, 64 * 47 - 7, 16, 3),
+                                         (1, 64 * 150, 12, 3), (4, 64 * 60 + 33, 16, 3), (2, 64 * 180 + 1, 8, 4)])
+def test_kda_in_parts_has_the_bits_of_one_pass(B, T, H, parts):
     """Long rows are cut into parts, the state's pass over one beside the intra-chunk pass over the next.  Packed sequences are
-    not cut, so a packed call on each row says what one pass gives."""
+    not cut, so a packed call on each row says what one pass gives.  (The first two go in one pass: too few chunks for a cut.)"""
+    from daisy_b200 import _lib
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert _lib.lib().daisy_b200_kda_parts(B, T, H) == parts
     q, k, v, g, beta = _inputs(B, T, H, seed=B * T + H)
     h0 = torch.randn(B, H, 128, 128, device="cuda", generator=torch.Generator("cuda").manual_seed(1)) * 0.1
     for _ in range(3):                                        # back to back: a call's first launch reuses the room of the last

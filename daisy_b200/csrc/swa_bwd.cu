@@ -1094,11 +1094,31 @@ static size_t bwd_tiles_bytes(int T, int window, bool in_blocks) {
 }
 static size_t bwd_delta_bytes(int B, int T, int H) { return (daisy_b200_swa_attend_bwd_workspace_bytes(B, T, H) + 1023) & ~(size_t)1023; }
 
+// Whether images of `room` (batch, head) pairs at a time are worth their rounds: a tile through them costs 0.78 of one whose
+// scores are formed again, but a round of few items lasts as long as its longest, while the other way all items share the SMs.  An
+// SM's tiles are taken as the mean and a quarter of the longest item, or as the longest.  Images against scores, us:
+// no window: 1 x 24576 x 8 (eight rounds of 192 items, the longest of 192 tiles where the mean of an SM is 125) 4424-4804 / 3880,
+// with eight documents 1190 / 787; 1 x 26000 x 8 4750 / 4336, 28000 5266 / 5233, 28700 5450 / 5520 (the rule's line: 28100), 30000 5697 / 6257; 1 x 24576 x 1
+// 610 / 840; 1 x 20480 x 8 (four rounds, 160 against 174) 2394 / 2992; 1 x 32000 x 4 2948 / 3365;
+// window 8192: 1 x 65536 x 4 3252-3373 / 3521; window 2048: 1 x 65536 x 16 3134 / 4667
+static bool bwd_images_pay(int B, int T, int H, int window, bool in_blocks, size_t room) {
+  const size_t pairs = (size_t)B * H, rounds = (pairs + room - 1) / room;
+  if (rounds == 1) return true;
+  const int sms = daisy_host::sm_count_cached();
+  const double nblk = (double)(((int64_t)T + WB - 1) / WB), longest = (double)bwd_tiles_row(T, window, in_blocks), tiles = longest * (nblk - (longest - 1) / 2);
+  const auto lasts = [&](size_t n) {
+    const double sm = n * tiles / (sms > 0 ? sms : 148) + longest / 4;
+    return sm > longest ? sm : longest;
+  };
+  return 0.78 * rounds * lasts((pairs + rounds - 1) / rounds) < lasts(pairs);
+}
+
 extern "C" size_t daisy_b200_swa_attend_bwd_workspace_bytes_full(int B, int T, int H, int window, unsigned flags) {
   if (B <= 0 || T <= 0 || H <= 0 || (flags & ~DAISY_WINDOW_BLOCKS)) return 0;
-  const size_t one = bwd_tiles_bytes(T, window, (flags & DAISY_WINDOW_BLOCKS) != 0), pairs = (size_t)B * H;
+  const bool in_blocks = (flags & DAISY_WINDOW_BLOCKS) != 0;
+  const size_t one = bwd_tiles_bytes(T, window, in_blocks), pairs = (size_t)B * H;
   const size_t n = BWD_TILES_MAX / one < pairs ? BWD_TILES_MAX / one : pairs;
-  return n ? bwd_delta_bytes(B, T, H) + n * one : daisy_b200_swa_attend_bwd_workspace_bytes(B, T, H);
+  return n && bwd_images_pay(B, T, H, window, in_blocks, n) ? bwd_delta_bytes(B, T, H) + n * one : daisy_b200_swa_attend_bwd_workspace_bytes(B, T, H);
 }
 
 // (batch, head) pairs a round takes: rounds of equal size, as many as there is room for images; 0: no room for one pair's

@@ -244,7 +244,8 @@ int daisy_b200_swa_attend_lse(const void* q, const void* k, const void* v,
  *   dq,dk,dv   gradients w.r.t. the prepared q, k, v: [B,T,H,D] bf16 contiguous
  *   workspace  daisy_b200_swa_attend_bwd_workspace_bytes(B,T,H) bytes at least; with
  *              daisy_b200_swa_attend_bwd_workspace_bytes_full(B,T,H,window,flags) bytes (2 GB and delta at most) dZ is kept between
- *              the kernel for dK, dV and the one for dQ instead of being formed again.  Any size between is used as far as it goes
+ *              the kernel for dK, dV and the one for dQ instead of being formed again (where that is slower, by the sizes, it is
+ *              the former).  Any size between is used as far as it goes
  *              (the dQ of both ways agree to bf16 rounding).
  * Launches: row-wise delta = sum_d dO O; a key-block-stationary kernel for dK, dV and a kernel for dQ, both once for as many
  * (batch, head) pairs as the workspace holds; no atomics: results are bitwise reproducible. */

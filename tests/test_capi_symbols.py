@@ -149,3 +149,23 @@ def test_token_step_rewrites_no_vector_that_may_still_be_read(lib):
                 assert readers <= owners | seen, (ctas, H, h, sorted(readers - owners - seen))
     assert lib.daisy_b200_swa_token_rows(148, 148, 256, 0, C.byref(first), C.byref(end)) < 0
     assert lib.daisy_b200_swa_token_rows(0, 148, 200, 0, C.byref(first), C.byref(end)) < 0
+
+
+@pytest.mark.parametrize("B,T,H,window,blocks,images", [(1, 1024, 6, 0, False, True), (8, 8192, 16, 2048, False, True), (8, 8192, 16, 16, True, True),
+                                                        (1, 20480, 8, 0, False, True), (1, 24576, 8, 0, False, False), (4, 25000, 16, 0, False, False),
+                                                        (1, 24576, 1, 0, False, True), (1, 32000, 4, 0, False, True), (1, 65536, 4, 8192, False, True),
+                                                        (1, 131072, 2, 8192, False, False)])
+def test_backward_asks_for_images_where_they_pay(lib, B, T, H, window, blocks, images):
+    """Rounds that leave most SMs waiting for their longest item (one pair's 192 key blocks, or too little room for any pair) are not
+    asked room for; the rounds of a size are those its room gives."""
+    from daisy_b200 import _lib
+    flags = _lib.WINDOW_BLOCKS if blocks else 0
+    delta, full = lib.daisy_b200_swa_attend_bwd_workspace_bytes(B, T, H), lib.daisy_b200_swa_attend_bwd_workspace_bytes_full(B, T, H, window, flags)
+    assert (full > delta) == images and full <= (2 << 30) + delta + 1024
+    rounds = lambda size: lib.daisy_b200_swa_attend_bwd_rounds(B, T, H, window, flags, size)
+    assert rounds(delta) == 1 and rounds(delta - 1) == _lib.EWORKSPACE
+    if images:
+        nblk = -(-T // 128)
+        one = nblk * min(nblk, (window if blocks else (window + 126) // 128 + 1) if window else nblk) * 32768
+        room = (full - delta) // one
+        assert 0 < room <= B * H and rounds(full) == -(-B * H // room)

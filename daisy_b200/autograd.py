@@ -2,7 +2,7 @@
 
 ``swa_attention(q, k, v, cos, sin, window, ...)`` takes the RAW projections ``[B,T,H,D]`` (views of the merged QKV
 projection are fine) and returns the attention output ``[B,T,H,D]``; its backward runs
-``daisy_b200_swa_attend_bwd`` (three launches, deterministic) and the norm / RoPE backward.  This is what the
+``daisy_b200_swa_attend_bwd`` (deterministic) and the norm / RoPE backward.  This is what the
 reference gets from autograd through ``F.rms_norm``, ``_apply_rope`` and ``scaled_dot_product_attention`` /
 ``flex_attention`` inside ``CausalSelfAttention.forward`` during training (models/daisy/attention.py:116-127,
 141-162).  The projections either side stay ordinary ``F.linear`` calls, so their weight and input gradients come

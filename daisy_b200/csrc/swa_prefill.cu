@@ -193,7 +193,7 @@ __device__ __forceinline__ BalancedWalk prefill_walk(int nq, int BH, int window,
 // (7 x 1009 x 16, window 249: 22500 cycles an item of four tiles).  So the producer works out the items ahead and hands them out,
 // the output leaves through the item's Q buffer as bulk copies, and a partial tile's 32-column pieces are masked, skipped or
 // taken whole as a warp's rows see them: 44.1 -> 32.1 us there, 8 x 8192 x 16 at window 2048 873 -> 833.
-// Whole tiles have a loop of their own, which keeps what only partial tiles need out of its registers (no spills; 4 to 12 bytes
+// Whole tiles have a loop of their own, which keeps what only partial tiles need out of its registers (4 bytes spilled; 4 to 20
 // with one loop for both), and a thread's second 32 scores are fetched under its first 32.  1 x 65536 x 16, window 8192, with
 // nearly all tiles whole: 2932 us; one loop 2996, both halves fetched at once in one loop 3073; 2973 for the form without the
 // items handed out.

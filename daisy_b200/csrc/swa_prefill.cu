@@ -37,7 +37,7 @@ constexpr int PREFILL_THREADS = 320;          // one softmax warpgroup per strea
 constexpr int PREFILL_THREADS_SPLIT = 576;    // two softmax warpgroups per stream (64 key columns each)
 constexpr int SMEM_TILES = (2 * NQBUF + NSTAGE) * TILE_BYTES;
 constexpr int PREFILL_BARS = 512;
-constexpr int PREFILL_SMEM = 1024 + SMEM_TILES + PREFILL_BARS + 2 * 128 * 4;   // alignment slack, tiles, barriers, row-sum exchange
+constexpr int PREFILL_SMEM = 1024 + SMEM_TILES + PREFILL_BARS;   // alignment slack, tiles, barriers
 static_assert(PREFILL_SMEM <= 232448, "over the 227 KB a CTA may use");
 constexpr float NEG_BIG = -1.0e30f;
 #ifndef POLY_MASK
@@ -86,8 +86,8 @@ struct PrefillBarriers {
   uint64_t s_full[2];
   uint64_t p_full[2];
   uint64_t o_full[2];
-  uint64_t l_part[2], l_all[2];    // split form: a stream's upper partial row sums, its totals
   uint64_t out_full[2][2];         // split form: a half's output lies in its Q buffer
+  uint64_t l_full[2][4];           // split form: the partial row sums of the two warps that share 32 rows of a stream
   uint64_t i_full[NITEM], i_empty[NITEM];
   ItemGeom item[NITEM];            // as the producer hands them out
   uint32_t tmem_base;
@@ -193,7 +193,7 @@ __device__ __forceinline__ BalancedWalk prefill_walk(int nq, int BH, int window,
 // (7 x 1009 x 16, window 249: 22500 cycles an item of four tiles).  So the producer works out the items ahead and hands them out,
 // the output leaves through the item's Q buffer as bulk copies, and a partial tile's 32-column pieces are masked, skipped or
 // taken whole as a warp's rows see them: 44.1 -> 32.1 us there, 8 x 8192 x 16 at window 2048 873 -> 833.
-// Whole tiles have a loop of their own, which keeps what only partial tiles need out of its registers (4 bytes spilled; 4 to 20
+// Whole tiles have a loop of their own, which keeps what only partial tiles need out of its registers (no spills; 4 to 12 bytes
 // with one loop for both), and a thread's second 32 scores are fetched under its first 32.  1 x 65536 x 16, window 8192, with
 // nearly all tiles whole: 2932 us; one loop 2996, both halves fetched at once in one loop 3073; 2973 for the form without the
 // items handed out.
@@ -221,8 +221,8 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       mbar_init(&bars->s_full[s], 1);
       mbar_init(&bars->p_full[s], 128 * NSPLIT);
       mbar_init(&bars->o_full[s], 1);
-      mbar_init(&bars->l_part[s], 4); mbar_init(&bars->l_all[s], 4);          // by warps
-      for (int hf = 0; hf < 2; ++hf) mbar_init(&bars->out_full[s][hf], 4);
+      for (int i = 0; i < 4; ++i) mbar_init(&bars->l_full[s][i], 2);
+      mbar_init(&bars->out_full[s][0], 4); mbar_init(&bars->out_full[s][1], 4);
     }
     for (int i = 0; i < NSTAGE; ++i) { mbar_init(&bars->kv_full[i], 1); mbar_init(&bars->kv_empty[i], 1); }
     for (int i = 0; i < NITEM; ++i) { mbar_init(&bars->i_full[i], 1); mbar_init(&bars->i_empty[i], 8 * NSPLIT + 1); }   // issuer, softmax warps
@@ -394,7 +394,6 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
     const uint32_t s_tmem = tmem_base + lane_off + s * 128 + half * 64;          // this thread's 64 S columns; P over the first 32
     const uint32_t o_tmem = tmem_base + lane_off + 256 + s * 128 + half * 64;    // and its 64 output columns in the epilogue
-    float* lsum = reinterpret_cast<float*>(smem + SMEM_TILES + PREFILL_BARS) + s * 128 + row;   // one exchange slot per row
     const uint64_t c2p = pack2f(p.scale_log2, p.scale_log2);
     uint32_t n_s = 0, n_o = 0, n_qs = 0;
     bool ok = true;
@@ -533,29 +532,20 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         unpack2f(sum_b, b0, b1);
         l = (a0 + a1) + (b0 + b1);
       }
-      // The upper half publishes its partial sum, the lower half replaces it by the total (one slot per row).  Warps give up on
-      // their own, so they wait for one another in bounded waits only: at a named barrier those that go on would wait for good.
-      auto all_wait = [&](uint64_t* bar) {
-        return __all_sync(0xffffffffu, mbar_wait(bar, n_o & 1, abort_flag, p.status, 15));
-      };
-      auto warp_arrive = [&](uint64_t* bar) {
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar);
-      };
-      if (half == 1) {
-        *lsum = l;
-        warp_arrive(&bars->l_part[s]);
-        ok = all_wait(&bars->l_all[s]);
-        l = *lsum;
-      } else {
-        ok = all_wait(&bars->l_part[s]);
-        l += *lsum;
-        *lsum = l;
-        warp_arrive(&bars->l_all[s]);
-      }
+      // The two warps that share rows exchange their partial sums through the item's Q buffer, which its last scores have left: each
+      // writes into the rows that the other's output will take.  Warps give up on their own, so they wait for one another in bounded
+      // waits only: at a named barrier those that go on would wait for good.  (131 tokens, 2 layers of 6 heads: 40.0 us; through a slot a row
+      // and the whole stream's warps twice 40.9, with a bulk copy for each warp's rows 41.6; named barriers 40.2, and agreed on by reductions 41.9.)
+      uint8_t* box = q_tiles + ((n_o % NQBUF) * 2 + s) * TILE_BYTES;
+      *reinterpret_cast<float*>(box + (1 - half) * HALF_BYTES + row * 128 + lane * 4) = l;
+      box += half * HALF_BYTES;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars->l_full[s][quarter]);
+      ok = __all_sync(0xffffffffu, mbar_wait(&bars->l_full[s][quarter], n_o & 1, abort_flag, p.status, 15));
       if (!ok) break;
+      l += *reinterpret_cast<const float*>(box + row * 128 + lane * 4);
       if (p.lse2 && half == 0 && q_row < T) p.lse2[((int64_t)item->b * p.H + item->h) * T + q_row] = __log2f(l);   // no reference maximum in this form
-      ok = all_wait(&bars->o_full[s]);
+      ok = __all_sync(0xffffffffu, mbar_wait(&bars->o_full[s], n_o & 1, abort_flag, p.status, 7));
       if (!ok) break;
       {
         tc_fence_after();
@@ -575,17 +565,15 @@ swa_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         }
         // out through this item's Q buffer, whose last product was over before O_s was: this half's 64 columns are one swizzled box
         // (stores from registers, transposed to whole row segments by shuffles, took 2200 cycles an item)
-        uint8_t* box = q_tiles + ((n_o % NQBUF) * 2 + s) * TILE_BYTES + half * HALF_BYTES;
         const uint32_t dst = smem_u32(box) + row * 128;
 #pragma unroll
         for (int c = 0; c < 8; ++c)
           asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst + ((c ^ (row & 7)) << 4)), "r"(ch[c].x), "r"(ch[c].y), "r"(ch[c].z), "r"(ch[c].w) : "memory");
         fence_proxy_async();
-        warp_arrive(&bars->out_full[s][half]);
-        if ((warp & 3) == 0) {
-          ok = all_wait(&bars->out_full[s][half]);
-          if (!ok) break;
-        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->out_full[s][half]);
+        if ((warp & 3) == 0) ok = __all_sync(0xffffffffu, mbar_wait(&bars->out_full[s][half], n_o & 1, abort_flag, p.status, 16));
+        if (!ok) break;
         ++n_o;
         if (out_thread) {
           tma_store_4d(&tm_o, box, 64 * half, q0, item->h, item->b);       // rows past T stay out of it
